@@ -79,6 +79,26 @@ def lib():
     return _lib
 
 
+class _Native(object):
+    """The compiled half of the Python layer (native/native.cc), loaded at first
+    use.  Functions are copied into the instance, so later calls find them
+    without a second lookup."""
+
+    def __getattr__(self, name):
+        lib()                    # torch's NCCL first, then libsgb.so; raises if that is missing
+        path = os.path.join(HERE, "_native.so")
+        if not os.path.exists(path):
+            raise ImportError(
+                "_native.so is not built (%s). Run `python -m singa_b200.build`; "
+                "there is no CPU fallback." % path)
+        from . import _native
+        self.__dict__.update((k, v) for k, v in vars(_native).items() if not k.startswith("__"))
+        return getattr(_native, name)
+
+
+native = _Native()
+
+
 def call(name, *args):
     """Calls an int-returning entry point and raises SgbError on failure."""
     handle = lib()

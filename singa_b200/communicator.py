@@ -11,6 +11,8 @@ import torch
 
 from . import _lib
 
+_n = _lib.native
+
 
 class NcclIdHolder(object):
     """Holds an ncclUniqueId (communicator.cc:49-51) as bytes."""
@@ -22,13 +24,6 @@ class NcclIdHolder(object):
             _lib.call("sgb_comm_get_unique_id", C.cast(buf, C.c_void_p))
             id_bytes = buf.raw
         self.id = bytes(id_bytes)
-
-
-def _table(tensors):
-    n = len(tensors)
-    ptrs = (C.c_void_p * n)(*[t.data_ptr() for t in tensors])
-    sizes = (C.c_size_t * n)(*[t.numel() for t in tensors])
-    return ptrs, sizes, n
 
 
 def _stream():
@@ -43,6 +38,10 @@ class Communicator(object):
     current (compute) stream wait for the communicator's side streams.
     """
 
+    # Staging (``send=False``) only records the tensors, the bytes move at the
+    # flush: a driver may hand a whole bucket over at once.
+    stages_lazily = True
+
     def __init__(self, local_rank, world_size, holder, buffSize=4194304, min_ctas=0, max_ctas=0):
         if not torch.cuda.is_available():
             raise RuntimeError("singa_b200.Communicator needs a CUDA device; there is no CPU path")
@@ -53,7 +52,7 @@ class Communicator(object):
         torch.cuda.current_stream().synchronize()   # context exists before NCCL init
         handle = C.c_void_p()
         idbuf = C.create_string_buffer(holder.id, len(holder.id))
-        self._h = None
+        self._h = self._ptr = None
         try:
             _lib.call("sgb_comm_create_ex", C.byref(handle), self.global_rank, self.world_size,
                       C.cast(idbuf, C.c_void_p), int(buffSize), int(min_ctas), int(max_ctas))
@@ -62,11 +61,12 @@ class Communicator(object):
                 _lib.lib().sgb_comm_destroy(handle)
             raise
         self._h = handle
+        self._ptr = handle.value          # what the native calls take
 
     def close(self):
         if self._h is not None:
             _lib.lib().sgb_comm_destroy(self._h)
-            self._h = None
+            self._h = self._ptr = None
 
     def __del__(self):
         try:
@@ -103,33 +103,22 @@ class Communicator(object):
 
     # -- reference API -------------------------------------------------------
     def synch(self, t):
-        _lib.call("sgb_comm_synch", self._h, t.data_ptr(), t.numel(),
-                  int(t.dtype == torch.float16), _stream())
+        _n.comm_synch(self._ptr, t)
 
     def fusedSynch(self, ts, send=True):
-        ptrs, sizes, n = _table(ts)
-        _lib.call("sgb_comm_fused_synch", self._h, ptrs, sizes, n,
-                  int(ts[0].dtype == torch.float16), int(send), _stream())
+        _n.comm_fused_synch(self._ptr, ts, send)
 
     def synchHalf(self, t):
-        assert t.dtype == torch.float32, \
-            "only available for 32-bit tensors, which are converted to 16 bits before transmit"
-        _lib.call("sgb_comm_synch_half", self._h, t.data_ptr(), t.numel(), _stream())
+        _n.comm_synch_half(self._ptr, t)
 
     def fusedSynchHalf(self, ts, send=True):
-        assert ts[0].dtype == torch.float32
-        ptrs, sizes, n = _table(ts)
-        _lib.call("sgb_comm_fused_synch_half", self._h, ptrs, sizes, n, int(send), _stream())
+        _n.comm_fused_synch_half(self._ptr, ts, send)
 
     def sparsification(self, t, accumulation, sparsThreshold, topK):
-        self.fusedSparsification([t], accumulation, sparsThreshold, topK)
+        _n.comm_sparsify(self._ptr, [t], accumulation, sparsThreshold, topK)
 
     def fusedSparsification(self, ts, accumulation, sparsThreshold, topK):
-        assert ts[0].dtype == torch.float32, "sparsification supports fp32 only"
-        ptrs, sizes, n = _table(ts)
-        acc = None if accumulation is None else accumulation.data_ptr()
-        _lib.call("sgb_comm_sparsification", self._h, ptrs, sizes, n, acc,
-                  float(sparsThreshold), int(bool(topK)), _stream())
+        _n.comm_sparsify(self._ptr, ts, accumulation, sparsThreshold, topK)
 
     def boundedSparsification(self, ts, accumulation, sparsThreshold, capacity):
         """Threshold sparsification with a fixed exchange of `capacity` slots per
@@ -137,7 +126,9 @@ class Communicator(object):
         whose fusedSparsification reads them back, communicator.cc:657-669).
         Entries a rank selects beyond `capacity` stay in `accumulation`."""
         assert ts[0].dtype == torch.float32, "sparsification supports fp32 only"
-        ptrs, sizes, n = _table(ts)
+        n = len(ts)
+        ptrs = (C.c_void_p * n)(*[t.data_ptr() for t in ts])
+        sizes = (C.c_size_t * n)(*[t.numel() for t in ts])
         acc = None if accumulation is None else accumulation.data_ptr()
         _lib.call("sgb_comm_sparsification_bounded", self._h, ptrs, sizes, n, acc, float(sparsThreshold),
                   int(capacity), _stream())
@@ -150,4 +141,4 @@ class Communicator(object):
         return int(out.value)
 
     def wait(self):
-        _lib.call("sgb_comm_wait", self._h, _stream())
+        _n.comm_wait(self._ptr)

@@ -3,6 +3,9 @@
 Owns the device tensors (torch is the allocator), turns every op into one
 pre-bound C-ABI call, replays DistOpt's bucket policy on the communicator as
 gradients become ready, and finishes with the fused multi-tensor SGD update.
+The calls of a step are recorded once as a native program; ``run_step`` is one
+call that issues them in order (2 us a call instead of 5: the arguments are
+already converted, and no interpreter runs between two launches).
 The whole step can be captured once into a CUDA graph and replayed, which is
 this implementation's counterpart of the reference's buffered-operation graph
 (``Device::EnableGraph`` / ``RunGraph``).
@@ -290,98 +293,97 @@ class HotPathGPU(object):
                 tot = sum(sizes[i] for i in ev[1])
                 self.residuals[ev[1][-1]] = torch.zeros(tot, device=self.device)
 
-    # --------------------------------------------------------------------- run
-    def _check(self, name, status):
-        if status != 0:
-            raise _lib.SgbError(name, status, self.lib.sgb_status_string(status).decode())
+        self._record_program()
 
-    def _on_grad_ready(self, idx, stream):
-        """opt.py:846-862 (plain), :885-912 (half), :1030-1090 (sparse)."""
-        c, L = self.comm, self.lib
-        if c is None:
+    # ----------------------------------------------------------------- program
+    def _record_program(self):
+        """The whole step as one native program: the compute calls, the exchange
+        and the update of every bucket at the place where its last gradient is
+        ready (opt.py:846-862 plain, :885-912 half, :1030-1090 sparse)."""
+        prog, self.calls_per_step = [], 0
+        order_index = {n: i for i, n in enumerate(self.plan["grad_order"])}
+        for name, args in self.calls:
+            if name == "grad_ready":
+                self.calls_per_step += self._record_exchange(prog, order_index[args])
+            elif name == "sync_and_update":
+                if self.comm is not None:
+                    prog.append(("sgb_comm_wait", (self.comm._h.value, "STREAM"), False))
+                if self.update_on_arrival:
+                    continue                  # every bucket was updated as it arrived
+                prog.append(self._sgd_call(self.sgd_tables, "STREAM"))
+                self.calls_per_step += 1
+            else:
+                prog.append((name, tuple(C.addressof(a) if isinstance(a, C.Array) else a for a in args), False))
+                self.calls_per_step += 1
+        self._program = _lib.native.program(prog, None if self.comm is None else self.comm._h.value)
+
+    def _sgd_call(self, tables, stream):
+        pp, gp, mp, sizes, n = tables
+        scale = float(np.float32(1.0) / np.float32(self.world))
+        return ("sgb_sgd_update_multi_f32", (C.addressof(pp), C.addressof(gp), C.addressof(mp), C.addressof(sizes), n,
+                                             "LR", "MOMENTUM", 0.0, "DECAY", 0, scale, stream), False)
+
+    def _record_exchange(self, prog, idx):
+        """Appends what happens when gradient `idx` is ready; returns how many
+        calls that counts for."""
+        if self.comm is None:
             return 0
-        n_calls = 0
+        h = self.comm._h.value
         ev = self.flush_after.get(idx)
         opt = self.dist_option
         is_direct = ev is not None and ev[0] == "direct"
-        if self.profile and ev is not None:
-            L.sgb_comm_profile_mark(c._h, b"bucket_ready", stream)
-        if opt in ("plain", "half"):
-            half = opt == "half"
-            if is_direct:
-                g = self.grads[idx]
-                if half:
-                    self._check("synch_half", L.sgb_comm_synch_half(c._h, g.data_ptr(), g.numel(), stream))
-                else:
-                    self._check("synch", L.sgb_comm_synch(c._h, g.data_ptr(), g.numel(), 0, stream))
-                self._sgd_bucket(idx)
-                return 1
-            ptrs, sizes, n = self.single_tables[idx]
-            if half:
-                self._check("stage_half", L.sgb_comm_fused_synch_half(c._h, ptrs, sizes, n, 0, stream))
-            else:
-                self._check("stage", L.sgb_comm_fused_synch(c._h, ptrs, sizes, n, 0, 0, stream))
-            n_calls += 1
-            if ev is not None:
-                ptrs, sizes, n = self.fused_tables[idx]
-                if half:
-                    self._check("flush_half", L.sgb_comm_fused_synch_half(c._h, ptrs, sizes, n, 1, stream))
-                else:
-                    self._check("flush", L.sgb_comm_fused_synch(c._h, ptrs, sizes, n, 0, 1, stream))
-                self._sgd_bucket(idx)
-                n_calls += 2
-            return n_calls
-        # sparse options: nothing is staged, the whole bucket is handed over at flush time
-        if ev is None:
-            return 0
-        topk = opt == "sparseTopK"
-        ptrs, sizes, n = self.single_tables[idx] if is_direct else self.fused_tables[idx]
-        self._check("sparsification", L.sgb_comm_sparsification(
-            c._h, ptrs, sizes, n, self.residuals[idx].data_ptr(), float(self.spars), int(topk), stream))
-        return 1
 
-    def _sgd_bucket(self, idx):
+        def addresses(tables):
+            ptrs, sizes, n = tables
+            return C.addressof(ptrs), C.addressof(sizes), n
+
+        if ev is not None:
+            prog.append(("sgb_comm_profile_mark", (h, b"bucket_ready", "STREAM"), True))
+        if opt not in ("plain", "half"):
+            # sparse options: nothing is staged, the whole bucket is handed over at flush time
+            if ev is None:
+                return 0
+            prog.append(("sgb_comm_sparsification",
+                         (h,) + addresses(self.single_tables[idx] if is_direct else self.fused_tables[idx]) +
+                         (self.residuals[idx].data_ptr(), float(self.spars), int(opt == "sparseTopK"), "STREAM"), False))
+            return 1
+        half = opt == "half"
+        if is_direct:
+            g = self.grads[idx]
+            prog.append(("sgb_comm_synch_half", (h, g.data_ptr(), g.numel(), "STREAM"), False) if half else
+                        ("sgb_comm_synch", (h, g.data_ptr(), g.numel(), 0, "STREAM"), False))
+            self._record_bucket_update(prog, idx)
+            return 1
+
+        def fused(tables, send):
+            mode = (send, "STREAM") if half else (0, send, "STREAM")
+            prog.append(("sgb_comm_fused_synch_half" if half else "sgb_comm_fused_synch",
+                         (h,) + addresses(tables) + mode, False))
+
+        fused(self.single_tables[idx], 0)
+        if ev is None:
+            return 1
+        fused(self.fused_tables[idx], 1)
+        self._record_bucket_update(prog, idx)
+        return 3
+
+    def _record_bucket_update(self, prog, idx):
         """The bucket's parameters are updated on the side stream on which its
         reduced gradients land (never on the NCCL stream: the next bucket's
         all-reduce does not wait for this update)."""
         if not self.update_on_arrival:
             return
-        L, h = self.lib, self.comm._h
-        side = L.sgb_comm_result_stream(h)
-        which = [L.sgb_comm_stream(h, w) for w in (0, 1, 2)].index(side)
-        pp, gp, mp, sizes, n = self.bucket_sgd[idx]
-        scale = float(np.float32(1.0) / np.float32(self.world))
-        L.sgb_comm_profile_range(h, b"sgd_update_bucket", which, 1)
-        self._check("sgd", L.sgb_sgd_update_multi_f32(pp, gp, mp, sizes, n, self.lr, self.momentum, 0.0,
-                                                       self.weight_decay, 0, scale, side))
-        L.sgb_comm_profile_range(h, b"sgd_update_bucket", which, 0)
+        h = self.comm._h.value
+        prog.append(("sgb_comm_profile_range", (h, b"sgd_update_bucket", "RESULT_INDEX", 1), False))
+        prog.append(self._sgd_call(self.bucket_sgd[idx], "RESULT_STREAM"))
+        prog.append(("sgb_comm_profile_range", (h, b"sgd_update_bucket", "RESULT_INDEX", 0), False))
 
+    # --------------------------------------------------------------------- run
     def run_step(self):
         """Enqueues one full step on the current stream (+ the communicator's
         side streams).  Returns the number of C-ABI calls issued."""
-        L = self.lib
-        stream = torch.cuda.current_stream().cuda_stream
-        order_index = {n: i for i, n in enumerate(self.plan["grad_order"])}
-        ncalls = 0
-        for name, args in self.calls:
-            if name == "grad_ready":
-                ncalls += self._on_grad_ready(order_index[args], stream)
-            elif name == "sync_and_update":
-                if self.comm is not None:
-                    self._check("wait", L.sgb_comm_wait(self.comm._h, stream))
-                if self.update_on_arrival:
-                    continue                  # every bucket was updated as it arrived
-                pp, gp, mp, sizes, n = self.sgd_tables
-                scale = float(np.float32(1.0) / np.float32(self.world))
-                self._check("sgd", L.sgb_sgd_update_multi_f32(pp, gp, mp, sizes, n, self.lr, self.momentum, 0.0,
-                                                               self.weight_decay, 0, scale, stream))
-                ncalls += 1
-            else:
-                st = getattr(L, name)(*[stream if a == "STREAM" else a for a in args])
-                if st != 0:
-                    self._check(name, st)
-                ncalls += 1
-        return ncalls
+        _lib.native.run_program(self._program, self.lr, self.momentum, self.weight_decay, self.profile)
+        return self.calls_per_step
 
     def capture(self):
         """Captures one step into a CUDA graph (after a warm-up step has run)."""

@@ -61,7 +61,13 @@ class SGD(object):
         self.apply_many([param_name], [param_value], [param_grad], grad_scale)
 
     def apply_many(self, names, params, grads, grad_scale=1.0):
-        moments = [self._moment(n, p) for n, p in zip(names, params)] if self.momentum != 0 else None
+        moments = None
+        if self.momentum != 0:
+            have = self.moments
+            try:
+                moments = [have[n] for n in names]
+            except KeyError:                              # first step of a parameter
+                moments = [self._moment(n, p) for n, p in zip(names, params)]
         sw.sgd_update_multi(params, grads, moments, self.lr, self.momentum, self.dampening,
                             self.weight_decay, self.nesterov, grad_scale)
 
@@ -118,24 +124,35 @@ class DistOpt(object):
 
     def _update_all(self, plist):
         scale = float(np.float32(1.0) / np.float32(self.world_size))
-        names = [n for n, _, _ in plist]
-        self.opt.apply_many(names, [p for _, p, _ in plist], [g for _, _, g in plist], scale)
+        if plist:
+            names, params, grads = zip(*plist)
+            self.opt.apply_many(names, params, grads, scale)
         self.opt.step()
 
     def _sync_dense(self, grad_stream, threshold, direct, fused):
+        # A communicator whose staging only takes note of the tensors gets each
+        # bucket in one piece; others are told of every gradient as it arrives.
+        whole = getattr(self.communicator, "stages_lazily", False)
         plist, glist, acc = [], [], 0
-        for name, p, g in grad_stream:
-            if g.numel() > threshold:
+        for triple in grad_stream:
+            g = triple[2]
+            n = g.numel()
+            if n > threshold:
                 direct(g)
             else:
                 glist.append(g)
-                fused([g], False)
-                acc += g.numel()
+                if not whole:
+                    fused([g], False)
+                acc += n
                 if acc > threshold:
+                    if whole:
+                        fused(glist, False)
                     fused(glist, True)
                     acc, glist = 0, []
-            plist.append((name, p, g))
+            plist.append(triple)
         if glist:
+            if whole:
+                fused(glist, False)
             fused(glist, True)
         self.wait()
         return plist
@@ -150,11 +167,10 @@ class DistOpt(object):
         """opt.py:867-920: fp16 transport of fp32 gradients."""
         def clipped(stream):
             for name, p, g in stream:
-                if clipping:
-                    sw.Clamp(g, -clip_Value, clip_Value, out=g)
+                sw.Clamp(g, -clip_Value, clip_Value, out=g)
                 yield name, p, g
-        self._update_all(self._sync_dense(clipped(grad_stream), threshold, self.all_reduce_half,
-                                          self.fused_all_reduce_half))
+        self._update_all(self._sync_dense(clipped(grad_stream) if clipping else grad_stream, threshold,
+                                          self.all_reduce_half, self.fused_all_reduce_half))
 
     def _divide_by_world(self, t):
         sw.DivFloatWithRet(t, self.world_size, t)
