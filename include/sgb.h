@@ -646,6 +646,18 @@ int sgb_comm_sparsification(sgb_comm *c, void *const *tensors,
                             const size_t *sizes, size_t count,
                             float *accumulation, float spars, int topk,
                             void *compute_stream);
+/* The same exchange in two halves, so that a driver with several buckets can
+ * have the next bucket's selection running while the host waits for this one's
+ * counts: _begin selects (on c1), _end waits for the counts (threshold form)
+ * and issues the all-gather and the dense sum of the OLDEST begun exchange.  At
+ * most two may be open; the tensors must stay allocated until their _end, and
+ * every rank issues the same sequence.  SGB_ERR_STATE: a third _begin, an _end
+ * without a _begin, or a wait / one-call sparsification while one is open. */
+int sgb_comm_sparsification_begin(sgb_comm *c, void *const *tensors,
+                                  const size_t *sizes, size_t count,
+                                  float *accumulation, float spars, int topk,
+                                  void *compute_stream);
+int sgb_comm_sparsification_end(sgb_comm *c, void *compute_stream);
 /* Threshold sparsification with a fixed exchange size: every rank sends
  * exactly `capacity` (index, value) slots, the true counts travel on the
  * device, and the host never waits for a count - so the call can sit inside a

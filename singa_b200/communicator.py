@@ -120,6 +120,15 @@ class Communicator(object):
     def fusedSparsification(self, ts, accumulation, sparsThreshold, topK):
         _n.comm_sparsify(self._ptr, ts, accumulation, sparsThreshold, topK)
 
+    def beginSparsification(self, ts, accumulation, sparsThreshold, topK):
+        """The selection half of fusedSparsification; endSparsification() issues
+        the exchange of the oldest begun one.  Two may be open, so the next
+        bucket's selection runs while the host waits for this one's counts."""
+        _n.comm_sparsify_begin(self._ptr, ts, accumulation, sparsThreshold, topK)
+
+    def endSparsification(self):
+        _n.comm_sparsify_end(self._ptr)
+
     def boundedSparsification(self, ts, accumulation, sparsThreshold, capacity):
         """Threshold sparsification with a fixed exchange of `capacity` slots per
         rank and no host wait for the counts (no counterpart in the reference,

@@ -65,19 +65,32 @@ struct sgb_comm {
   __half* dsend_h = nullptr;   // direct (unbucketed) fp16 synch: never aliases a half-filled bucket
   __half* drecv_h = nullptr;
   // sparse path (allocated at first use)
-  float* sum = nullptr;        // g + acc (backupBuff)
-  int* pay_send = nullptr;     // [idx | val], 2 * max_elems words
   int* pay_recv = nullptr;     // world * 2 * max_elems words
   void* ws = nullptr;
   size_t ws_bytes = 0;
-  int* nnz_dev = nullptr;      // [0] own count, [1 .. world] all ranks
-  int* nnz_host = nullptr;     // pinned, world entries
+  // A sparse exchange between its selection and its all-gather.  Two may be
+  // open at a time, so that the next bucket's selection runs while the host
+  // waits for this one's counts.
+  struct Sparse {
+    int* pay_send = nullptr;     // [idx | val], 2 * max_elems words
+    int* nnz_dev = nullptr;      // [0] own count, [1 .. world] all ranks
+    int* nnz_host = nullptr;     // pinned, world entries
+    cudaEvent_t selected = nullptr;  // behind the selection on c1
+    cudaEvent_t counted = nullptr;   // behind the counts' copy to the host
+    size_t n = 0, nnz_max = 0, capacity = 0;
+    int topk = 0;
+    const char* op_name = "";
+    std::vector<float*> tensors;
+    std::vector<size_t> sizes;
+  };
+  Sparse sparse[2];
+  unsigned sparse_begun = 0, sparse_ended = 0;
   unsigned long long* dropped_dev = nullptr;   // entries the bounded threshold form left for later calls
   int topk_mode = 1;           // 1 = the reference comparator's key, 0 = |value|
   cudaStream_t s = nullptr, c1 = nullptr, c2 = nullptr;
   bool own_streams = true;     // false after sgb_comm_use_streams: the caller's streams are not destroyed
   cudaEvent_t ev_compute = nullptr, ev_c1 = nullptr, ev_s = nullptr, ev_c2 = nullptr,
-              ev_c2_done = nullptr, ev_host = nullptr;
+              ev_c2_done = nullptr;
   size_t send_off = 0;         // elements staged since the last flush
   // Which side streams received work since the last wait() (only those are
   // joined, so a wait() issued while the compute stream is being captured
@@ -229,14 +242,20 @@ int half_init(sgb_comm* c) {
 }
 
 int sparse_init(sgb_comm* c) {
-  if (c->pay_send) return SGB_OK;
+  if (c->pay_recv) return SGB_OK;
   const size_t n = c->max_elems;
-  CU(cudaMalloc(&c->pay_send, 2 * n * sizeof(int)));
-  CU(cudaMalloc(&c->pay_recv, 2 * n * sizeof(int) * static_cast<size_t>(c->world)));
   c->ws_bytes = sgb_sparse_workspace_bytes(n);
   CU(cudaMalloc(&c->ws, c->ws_bytes));
-  CU(cudaMalloc(&c->nnz_dev, sizeof(int) * (c->world + 1)));
-  CU(cudaMallocHost(&c->nnz_host, sizeof(int) * c->world));
+  for (sgb_comm::Sparse& x : c->sparse) {
+    CU(cudaMalloc(&x.pay_send, 2 * n * sizeof(int)));
+    CU(cudaMalloc(&x.nnz_dev, sizeof(int) * (c->world + 1)));
+    CU(cudaMallocHost(&x.nnz_host, sizeof(int) * c->world));
+    // the host polls for the counts: it has the next calls to issue, and a
+    // blocking wait woke it 50-100 us late
+    CU(cudaEventCreateWithFlags(&x.selected, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&x.counted, cudaEventDisableTiming));
+  }
+  CU(cudaMalloc(&c->pay_recv, 2 * n * sizeof(int) * static_cast<size_t>(c->world)));
   CU(cudaMalloc(&c->dropped_dev, sizeof(unsigned long long)));
   CU(cudaMemset(c->dropped_dev, 0, sizeof(unsigned long long)));
   return SGB_OK;
@@ -319,7 +338,6 @@ int sgb_comm_create_ex(sgb_comm** out, int rank, int world, const void* unique_i
   CU(cudaStreamCreateWithPriority(&c->c2, cudaStreamNonBlocking, prio_hi));
   cudaEvent_t* evs[] = {&c->ev_compute, &c->ev_c1, &c->ev_s, &c->ev_c2, &c->ev_c2_done};
   for (cudaEvent_t* e : evs) CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-  CU(cudaEventCreateWithFlags(&c->ev_host, cudaEventDisableTiming | cudaEventBlockingSync));
   return SGB_OK;
 }
 
@@ -332,14 +350,19 @@ int sgb_comm_destroy(sgb_comm* c) {
     for (void* h : c->registered) ncclCommDeregister(c->nccl, h);
     ncclCommDestroy(c->nccl);
   }
-  void* bufs[] = {c->send, c->recv, c->send_h, c->recv_h, c->dsend_h, c->drecv_h, c->sum, c->pay_send,
-                  c->pay_recv, c->ws, c->nnz_dev};
+  void* bufs[] = {c->send, c->recv, c->send_h, c->recv_h, c->dsend_h, c->drecv_h, c->pay_recv, c->ws};
   for (void* b : bufs)
     if (b) cudaFree(b);
-  if (c->nnz_host) cudaFreeHost(c->nnz_host);
+  for (sgb_comm::Sparse& x : c->sparse) {
+    if (x.pay_send) cudaFree(x.pay_send);
+    if (x.nnz_dev) cudaFree(x.nnz_dev);
+    if (x.nnz_host) cudaFreeHost(x.nnz_host);
+    if (x.selected) cudaEventDestroy(x.selected);
+    if (x.counted) cudaEventDestroy(x.counted);
+  }
   if (c->dropped_dev) cudaFree(c->dropped_dev);
   drop_ranges(c);
-  cudaEvent_t evs[] = {c->ev_compute, c->ev_c1, c->ev_s, c->ev_c2, c->ev_c2_done, c->ev_host, c->prof_origin};
+  cudaEvent_t evs[] = {c->ev_compute, c->ev_c1, c->ev_s, c->ev_c2, c->ev_c2_done, c->prof_origin};
   for (cudaEvent_t e : evs)
     if (e) cudaEventDestroy(e);
   cudaStream_t ss[] = {c->s, c->c1, c->c2};
@@ -352,7 +375,9 @@ int sgb_comm_destroy(sgb_comm* c) {
 int sgb_comm_use_streams(sgb_comm* c, void* s, void* c1, void* c2) {
   if (!c || !s || !c1 || !c2) return SGB_ERR_NULL;
   if (s == c1 || s == c2 || c1 == c2) return SGB_ERR_UNSUPPORTED;
-  if (c->order.dirty_s || c->order.dirty_c1 || c->order.dirty_c2 || !c->pend_ptrs.empty()) return SGB_ERR_STATE;
+  if (c->order.dirty_s || c->order.dirty_c1 || c->order.dirty_c2 || !c->pend_ptrs.empty() ||
+      c->sparse_begun != c->sparse_ended)
+    return SGB_ERR_STATE;
   if (c->own_streams) {
     cudaStream_t ss[] = {c->s, c->c1, c->c2};
     for (cudaStream_t st : ss)
@@ -388,6 +413,7 @@ void* sgb_comm_stream(const sgb_comm* c, int which) {
 
 int sgb_comm_wait(sgb_comm* c, void* compute_stream) {
   if (!c) return SGB_ERR_NULL;
+  if (c->sparse_begun != c->sparse_ended) return SGB_ERR_STATE;   // an exchange is still to be ended
   return emit(c, plan_call(c, sgb::order::kWait).before, sgb::as_stream(compute_stream));
 }
 
@@ -624,100 +650,127 @@ int sgb_comm_fused_synch_half(sgb_comm* c, void* const* tensors, const size_t* s
   return emit(c, p.post, nullptr);
 }
 
-// capacity == 0: the reference's exchange (the payload is as long as the
-// largest count, which the host reads back).  capacity > 0 (threshold mode):
-// every rank sends exactly `capacity` slots, no host round trip.
-static int sparsify(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count,
-                    float* accumulation, float spars, int topk, size_t capacity, void* compute_stream) {
+// The selection half.  capacity == 0: the reference's exchange (the payload is
+// as long as the largest count, which the host reads back).  capacity > 0
+// (threshold mode): every rank sends exactly `capacity` slots, no host round trip.
+static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count,
+                        float* accumulation, float spars, int topk, size_t capacity, void* compute_stream) {
   if (!c) return SGB_ERR_NULL;
   OK(check_list(tensors, sizes, count));
   const size_t n = total_of(sizes, count);
   if (n > c->max_elems) return SGB_ERR_CAPACITY;
   if (capacity > c->max_elems) return SGB_ERR_CAPACITY;
-  if (n == 0) return SGB_OK;
+  if (c->sparse_begun - c->sparse_ended >= 2) return SGB_ERR_STATE;
   OK(sparse_init(c));
-  const int W = c->world;
-  const char* op_name = count > 1 ? "Dist_c1c2_fusedSparsification" : "Dist_c1c2_sparsification";
-  const sgb::order::Step p = plan_call(c, sgb::order::kSparse);
-  OK(emit(c, p.pre, sgb::as_stream(compute_stream)));
-  // One tensor, or tensors that lie back to back in memory (a gradient arena),
-  // are selected from and scattered into IN PLACE: no copy into the send
-  // buffer and none back (16 B/element saved).  The selection has finished
-  // reading the gradient before the dense result is written: c1 -> s -> c2.
-  bool in_place = sgb::aligned16(tensors[0]);
-  for (size_t i = 1; i < count && in_place; ++i)
-    in_place = static_cast<const float*>(tensors[i]) == static_cast<const float*>(tensors[i - 1]) + sizes[i - 1];
-  float* grad = in_place ? static_cast<float*>(tensors[0]) : c->send;
-  float* dense = in_place ? static_cast<float*>(tensors[0]) : c->recv;
-
-  size_t nnz_max = 0;
-  auto select = [&]() -> int {
-  Phase ph(c, op_name, sgb::order::kStreamC1);
-  if (!in_place) OK(sgb_pack_f32(tensors, sizes, count, c->send, 0, c->c1));
-  if (!topk && capacity) {
-    OK(sgb::sparse_threshold_count(grad, accumulation, n, spars, c->nnz_dev, c->ws,
-                                   c->ws_bytes, c->c1));
-    // the counts travel on the device only; receivers clamp them to the capacity
-    NC(ncclAllGather(c->nnz_dev, c->nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
-    OK(sgb::sparse_threshold_write_bounded(grad, accumulation, n, spars, c->pay_send, capacity, c->dropped_dev,
-                                           c->ws, c->c1));
-    nnz_max = capacity;
-  } else if (!topk) {
-    OK(sgb::sparse_threshold_count(grad, accumulation, n, spars, c->nnz_dev, c->ws,
-                                   c->ws_bytes, c->c1));
-    NC(ncclAllGather(c->nnz_dev, c->nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
-    CU(cudaMemcpyAsync(c->nnz_host, c->nnz_dev + 1, sizeof(int) * W, cudaMemcpyDeviceToHost, c->c1));
-    CU(cudaEventRecord(c->ev_host, c->c1));
-    // the compaction runs while the host waits for the counts
-    OK(sgb::sparse_threshold_write_packed(grad, accumulation, n, spars, c->pay_send, c->ws, c->c1));
-    CU(cudaEventSynchronize(c->ev_host));
-    for (int r = 0; r < W; ++r) {
-      if (c->nnz_host[r] < 0 || static_cast<size_t>(c->nnz_host[r]) > n) return SGB_ERR_STATE;
-      if (static_cast<size_t>(c->nnz_host[r]) > nnz_max) nnz_max = c->nnz_host[r];
-    }
-  } else {
-    nnz_max = static_cast<size_t>(sgb_topk_count(spars, n));
-    for (int r = 0; r < W; ++r) c->nnz_host[r] = static_cast<int>(nnz_max);
-    if (nnz_max)
-      OK(sgb_sparse_topk_f32(grad, accumulation, nullptr, n, nnz_max, c->topk_mode, c->pay_send,
-                             reinterpret_cast<float*>(c->pay_send) + nnz_max, c->ws, c->ws_bytes,
-                             c->c1));
+  sgb_comm::Sparse& x = c->sparse[c->sparse_begun & 1];
+  x.n = n;
+  x.nnz_max = 0;
+  x.capacity = capacity;
+  x.topk = topk;
+  x.op_name = count > 1 ? "Dist_c1c2_fusedSparsification" : "Dist_c1c2_sparsification";
+  x.tensors.clear();
+  x.sizes.clear();
+  for (size_t i = 0; i < count; ++i) {
+    x.tensors.push_back(static_cast<float*>(tensors[i]));
+    x.sizes.push_back(sizes[i]);
   }
+  if (n) {
+    OK(emit(c, plan_call(c, sgb::order::kSparseSelect).pre, sgb::as_stream(compute_stream)));
+    // One tensor, or tensors that lie back to back in memory (a gradient arena),
+    // are selected from IN PLACE: no copy into the send buffer.
+    bool in_place = sgb::aligned16(tensors[0]);
+    for (size_t i = 1; i < count && in_place; ++i)
+      in_place = static_cast<const float*>(tensors[i]) == static_cast<const float*>(tensors[i - 1]) + sizes[i - 1];
+    const float* grad = in_place ? static_cast<const float*>(tensors[0]) : c->send;
+    Phase ph(c, x.op_name, sgb::order::kStreamC1);
+    if (!in_place) OK(sgb_pack_f32(tensors, sizes, count, c->send, 0, c->c1));
+    if (topk) {
+      x.nnz_max = static_cast<size_t>(sgb_topk_count(spars, n));
+      for (int r = 0; r < c->world; ++r) x.nnz_host[r] = static_cast<int>(x.nnz_max);
+      if (x.nnz_max)
+        OK(sgb_sparse_topk_f32(grad, accumulation, nullptr, n, x.nnz_max, c->topk_mode, x.pay_send,
+                               reinterpret_cast<float*>(x.pay_send) + x.nnz_max, c->ws, c->ws_bytes, c->c1));
+    } else if (capacity) {
+      x.nnz_max = capacity;
+      OK(sgb::sparse_threshold_bounded(grad, accumulation, n, spars, x.pay_send, capacity, x.nnz_dev, c->dropped_dev,
+                                       c->ws, c->ws_bytes, c->c1));
+      // the counts travel on the device only; receivers clamp them to the capacity
+      NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
+    } else {
+      OK(sgb::sparse_threshold_packed(grad, accumulation, n, spars, x.pay_send, x.nnz_dev, c->ws, c->ws_bytes, c->c1));
+      NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
+      CU(cudaMemcpyAsync(x.nnz_host, x.nnz_dev + 1, sizeof(int) * c->world, cudaMemcpyDeviceToHost, c->c1));
+      CU(cudaEventRecord(x.counted, c->c1));
+    }
+    CU(cudaEventRecord(x.selected, c->c1));
+  }
+  ++c->sparse_begun;
   return SGB_OK;
-  };
-  OK(select());
+}
 
-  OK(emit(c, p.before, sgb::as_stream(compute_stream)));
-  if (nnz_max) {
+// The exchange half of the oldest exchange that is open.
+static int sparse_end(sgb_comm* c, void* compute_stream) {
+  if (!c) return SGB_ERR_NULL;
+  if (c->sparse_begun == c->sparse_ended) return SGB_ERR_STATE;
+  sgb_comm::Sparse& x = c->sparse[c->sparse_ended++ & 1];
+  if (x.n == 0) return SGB_OK;
+  const int W = c->world;
+  if (!x.topk && !x.capacity) {
+    CU(cudaEventSynchronize(x.counted));
+    for (int r = 0; r < W; ++r) {
+      if (x.nnz_host[r] < 0 || static_cast<size_t>(x.nnz_host[r]) > x.n) return SGB_ERR_STATE;
+      if (static_cast<size_t>(x.nnz_host[r]) > x.nnz_max) x.nnz_max = x.nnz_host[r];
+    }
+  }
+  const sgb::order::Step p = plan_call(c, sgb::order::kSparseExchange);
+  // s waits for this exchange's own selection, not for what c1 was given since
+  CU(cudaStreamWaitEvent(c->s, x.selected, 0));
+  OK(emit(c, p.before & ~static_cast<unsigned>(sgb::order::kC1ToS), sgb::as_stream(compute_stream)));
+  if (x.nnz_max) {
     Phase ph(c, "Dist_s_sparsification_allgather", sgb::order::kStreamS);
-    NC(ncclAllGather(c->pay_send, c->pay_recv, 2 * nnz_max, ncclFloat, c->nccl, c->s));
+    NC(ncclAllGather(x.pay_send, c->pay_recv, 2 * x.nnz_max, ncclFloat, c->nccl, c->s));
   }
   OK(emit(c, p.after, nullptr));
-  auto scatter = [&]() -> int {
-  Phase ph(c, op_name, sgb::order::kStreamC2);
-  CU(cudaMemsetAsync(dense, 0, n * sizeof(float), c->c2));
-  for (int r = 0; r < W && nnz_max; ++r) {  // ranks in ascending order, as the reference
-    const int* seg = c->pay_recv + static_cast<size_t>(r) * 2 * nnz_max;
-    if (capacity) {                                   // fixed layout; the rank's count is read on the device
-      OK(sgb_scatter_add_f32(seg, reinterpret_cast<const float*>(seg) + capacity, capacity, c->nnz_dev + 1 + r,
-                             dense, n, c->c2));
-      continue;
+  {
+    Phase ph(c, x.op_name, sgb::order::kStreamC2);
+    const size_t stride = 2 * x.nnz_max;
+    if (W <= sgb::kMaxDenseRanks) {
+      OK(sgb::sparse_dense_sum(c->pay_recv, stride, x.capacity, x.nnz_host, x.capacity ? x.nnz_dev + 1 : nullptr, W,
+                               x.tensors.data(), x.sizes.data(), x.tensors.size(), c->c2));
+    } else {
+      // more ranks than the dense kernel's table holds: fill, then add rank after rank
+      CU(cudaMemsetAsync(c->recv, 0, x.n * sizeof(float), c->c2));
+      for (int r = 0; r < W && x.nnz_max; ++r) {
+        const int* seg = c->pay_recv + static_cast<size_t>(r) * stride;
+        const size_t cnt = x.capacity ? x.capacity : static_cast<size_t>(x.nnz_host[r]);
+        OK(sgb_scatter_add_f32(seg, reinterpret_cast<const float*>(seg) + cnt, cnt,
+                               x.capacity ? x.nnz_dev + 1 + r : nullptr, c->recv, x.n, c->c2));
+      }
+      OK(sgb_unpack_f32(c->recv, 0, reinterpret_cast<void* const*>(x.tensors.data()), x.sizes.data(),
+                        x.tensors.size(), 1.0f, c->c2));
     }
-    const size_t cnt = static_cast<size_t>(c->nnz_host[r]);
-    OK(sgb_scatter_add_f32(seg, reinterpret_cast<const float*>(seg) + cnt, cnt, nullptr, dense,
-                           n, c->c2));
   }
-  if (!in_place) OK(sgb_unpack_f32(c->recv, 0, tensors, sizes, count, 1.0f, c->c2));
-  return SGB_OK;
-  };
-  OK(scatter());
   return emit(c, p.post, nullptr);
+}
+
+static int sparsify(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count, float* accumulation,
+                    float spars, int topk, size_t capacity, void* compute_stream) {
+  if (c && c->sparse_begun != c->sparse_ended) return SGB_ERR_STATE;
+  OK(sparse_begin(c, tensors, sizes, count, accumulation, spars, topk, capacity, compute_stream));
+  return sparse_end(c, compute_stream);
 }
 
 int sgb_comm_sparsification(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count,
                             float* accumulation, float spars, int topk, void* compute_stream) {
   return sparsify(c, tensors, sizes, count, accumulation, spars, topk, 0, compute_stream);
 }
+
+int sgb_comm_sparsification_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count,
+                                  float* accumulation, float spars, int topk, void* compute_stream) {
+  return sparse_begin(c, tensors, sizes, count, accumulation, spars, topk, 0, compute_stream);
+}
+
+int sgb_comm_sparsification_end(sgb_comm* c, void* compute_stream) { return sparse_end(c, compute_stream); }
 
 int sgb_comm_sparsification_bounded(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count,
                                     float* accumulation, float threshold, size_t capacity,

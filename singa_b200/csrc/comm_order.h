@@ -33,6 +33,10 @@ enum Call {
   kSparse = 5,        // select on c1, all-gather, scatter-add on c2
   kStageCopy = 6,     // copies into the staging buffer on c1 (no collective)
   kWait = 7,
+  // the two halves of kSparse, issued one after the other or with another
+  // exchange's half between them (not replayed through sgb_comm_order_plan)
+  kSparseSelect = 16,    // the selection on c1
+  kSparseExchange = 17,  // ordered behind that selection: all-gather on s, dense sum on c2
 };
 
 enum Edge : unsigned {
@@ -85,6 +89,19 @@ inline Step plan(State& st, int call) {
     case kSynchHalf:
     case kSparse:
       p.pre = kComputeToC1;
+      p.before = kC1ToS | (st.c2_reads_recv ? kC2DoneToS : 0u);
+      p.after = kSToC1 | kSToC2;
+      p.post = kMarkC2Done;
+      p.result_stream = kStreamC2;
+      st.c2_reads_recv = 1;
+      st.dirty_s = st.dirty_c1 = st.dirty_c2 = 1;
+      break;
+    case kSparseSelect:
+      p.pre = kComputeToC1;
+      p.result_stream = kStreamC1;
+      st.dirty_c1 = 1;
+      break;
+    case kSparseExchange:
       p.before = kC1ToS | (st.c2_reads_recv ? kC2DoneToS : 0u);
       p.after = kSToC1 | kSToC2;
       p.post = kMarkC2Done;

@@ -3,90 +3,137 @@
 //     compaction into a [1-based index | value] payload;
 //   * top-K selection by radix select on a 32-bit key (no sort), ties broken
 //     by lower index, with the same compaction;
-//   * scatter-add of a received payload into the dense sum buffer.
+//   * the dense sum of the received payloads.
 //
-// Compaction is the classic three-step form (per-tile counts, one-CTA scan of
-// the tile counts, per-tile write at the scanned offsets).  It has no waits
-// between CTAs, so nothing can spin.  All index arithmetic that reaches the
-// payload is 1-based int32, the reference's wire format.
-#include "common.cuh"
+// Each selection is ONE cooperative kernel.  The elements are split into chunks
+// of eight runs (one per warp) of one or four 512-element tiles; what a warp
+// selects in its run goes to a private list in the workspace in ascending index
+// order, so that after one device-wide barrier (all counts are known) the lists
+// are copied to their final place: no scan kernel, no second read of the
+// gradient.  A CTA draws its next chunk from a ticket counter while it works on
+// the current one: with a fixed share per CTA the slowest SMs finished 40 us
+// after the others at 1e8 elements (SMs do not get equal bandwidth).  Inside a
+// chunk warps do not wait for one another.  The device-wide barriers are
+// cooperative-launch grid barriers (all CTAs of the grid are co-resident by
+// construction).  A list that fills up (a run in which more than about one
+// element in six is selected) costs no correctness: the warp notes how many
+// tiles were listed and reads the others again.
+//
+// What bounds them: HBM.  g and the residual are read once, the residual is
+// written once (12 B/element); the top-K form reads the residual once more
+// (4 B/element) after the first radix digit is decided.  All index arithmetic
+// that reaches the payload is 1-based int32, the reference's wire format.
+#include <cooperative_groups.h>
+
+#include <atomic>
+
+#include "sparse.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace sgb {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kVecPerThread = 4;                       // float4 vectors per thread
-constexpr int kTile = kBlock * kVecPerThread * 4;      // 4096 elements per CTA
+constexpr int kWarps = kBlock / 32;
+constexpr int kRounds = 4;                             // float4 vectors per lane and tile
+constexpr int kTile = 32 * kRounds * 4;                // 512 elements, a warp's unit of work
 constexpr int kBins1 = 4096, kBins23 = 1024;           // 12 + 10 + 10 key bits
+// 4 CTAs per SM: 128 KB of loads in flight per SM already saturate HBM, and a
+// cooperative grid that does not need every slot can start beside the kernels
+// of another stream.
+constexpr int kCtasPerSm = 4;
+constexpr int kMaxGrid = 1024;
 
-// Device-resident selection state shared by the top-K passes.
-struct SelectState {
-  unsigned prefix;       // key bits decided so far (high bits), low bits zero
-  unsigned remaining;    // how many elements are still to be taken at/below prefix
-  unsigned threshold;    // final key T
-  unsigned quota;        // number of key == T elements to take (lowest indices)
-  int nnz;               // payload length (threshold mode: count; top-K: K)
-  unsigned max_key;      // largest key seen by pass 0 (zeroed with the histogram before every call)
-  unsigned skip1;        // 1: every key is below 2^10, pass 1 (bits 10..19) has nothing to decide
-  int pad;
+struct Counters {        // zeroed before a call that uses them
+  unsigned ticket[4];    // chunks drawn so far, one counter per pass
+  unsigned max_key;      // largest key of pass 0
+  unsigned pad[3];
+  unsigned hist0[kBins1], hist1[kBins23], hist2[kBins23];
 };
 
-// Workspace layout (all 256-byte aligned segments).
-struct Workspace {
-  unsigned* tile_counts;   // tiles entries (threshold) or packed gt<<16|eq... see below
-  unsigned* tile_gt;       // tiles
-  unsigned* tile_eq;       // tiles
-  unsigned* hist;          // kBins1
-  SelectState* state;
-};
 inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 inline size_t tiles_of(size_t n) { return ceil_div(n, kTile); }
-inline size_t workspace_bytes(size_t n) {
-  return 3 * align256(tiles_of(n) * sizeof(unsigned)) + align256(kBins1 * sizeof(unsigned)) +
-         align256(sizeof(SelectState));
+inline size_t max_grid() {
+  const size_t g = static_cast<size_t>(sm_count()) * kCtasPerSm;
+  return g < kMaxGrid ? g : kMaxGrid;
 }
-inline Workspace carve(void* ws, size_t n) {
+// How the tiles are cut.  One tile per warp and chunk until every CTA has four
+// chunks, then four: fewer counts to add up, less to draw.
+struct Work {
+  unsigned chunks, grid;
+  unsigned run;          // tiles per warp and chunk
+  unsigned capacity;     // list entries per warp and chunk
+  bool dynamic;          // chunks are drawn from the ticket counter
+};
+inline Work work_for(size_t n) {
+  const size_t tiles = tiles_of(n), g = max_grid();
+  Work w;
+  w.run = tiles > 4 * kWarps * g ? 4 : 1;
+  w.capacity = w.run == 4 ? 352 : 128;
+  w.chunks = static_cast<unsigned>(ceil_div(tiles, kWarps * w.run));
+  w.grid = static_cast<unsigned>(w.chunks < g ? w.chunks : g);
+  w.dynamic = w.chunks > 2 * w.grid;
+  return w;
+}
+
+struct Workspace {
+  Counters* counters;
+  unsigned* chunk_a;     // per chunk: selected, or keys above the threshold
+  unsigned* chunk_b;     //            keys equal to the threshold
+  unsigned* run_meta;    // per warp and chunk, see pack_meta
+  unsigned* run_counts;  // per warp and chunk: keys above / equal to the threshold (16 bits each)
+  int* list_idx;         // chunks * kWarps segments of `capacity` entries
+  float* list_val;
+};
+inline size_t workspace_bytes_exact(size_t n) {
+  const Work w = work_for(n);
+  const size_t runs = static_cast<size_t>(w.chunks) * kWarps;
+  return align256(sizeof(Counters)) + 2 * align256(w.chunks * sizeof(unsigned)) + 2 * align256(runs * sizeof(unsigned)) +
+         2 * align256(runs * w.capacity * sizeof(int));
+}
+// Monotonic in n (a workspace for n serves any smaller call): where the cut
+// changes from one tile to four, the shorter runs need the larger lists.
+inline size_t workspace_bytes(size_t n) {
+  const size_t turn = 4 * kWarps * max_grid() * static_cast<size_t>(kTile);
+  size_t b = workspace_bytes_exact(n);
+  if (n > turn && workspace_bytes_exact(turn) > b) b = workspace_bytes_exact(turn);
+  return b;
+}
+inline Workspace carve(void* ws, const Work& k) {
   char* p = static_cast<char*>(ws);
+  const size_t runs = static_cast<size_t>(k.chunks) * kWarps;
   Workspace w;
-  const size_t t = align256(tiles_of(n) * sizeof(unsigned));
-  w.tile_counts = reinterpret_cast<unsigned*>(p); p += t;
-  w.tile_gt = reinterpret_cast<unsigned*>(p); p += t;
-  w.tile_eq = reinterpret_cast<unsigned*>(p); p += t;
-  w.hist = reinterpret_cast<unsigned*>(p); p += align256(kBins1 * sizeof(unsigned));
-  w.state = reinterpret_cast<SelectState*>(p);
+  w.counters = reinterpret_cast<Counters*>(p); p += align256(sizeof(Counters));
+  w.chunk_a = reinterpret_cast<unsigned*>(p); p += align256(k.chunks * sizeof(unsigned));
+  w.chunk_b = reinterpret_cast<unsigned*>(p); p += align256(k.chunks * sizeof(unsigned));
+  w.run_meta = reinterpret_cast<unsigned*>(p); p += align256(runs * sizeof(unsigned));
+  w.run_counts = reinterpret_cast<unsigned*>(p); p += align256(runs * sizeof(unsigned));
+  w.list_idx = reinterpret_cast<int*>(p); p += align256(runs * k.capacity * sizeof(int));
+  w.list_val = reinterpret_cast<float*>(p);
   return w;
 }
 
 // ------------------------------------------------------------- tile helpers
-// Element order inside a tile: vector v = r * kBlock + t (round r, thread t),
-// elements 4v .. 4v+3.  Loads are fully coalesced; ranks below follow this
-// order, which is ascending element index.
-__device__ __forceinline__ float load_sum(const float* __restrict__ g,
-                                          const float* __restrict__ acc, size_t i) {
-  return acc ? g[i] + acc[i] : g[i];
+// Element order inside a tile: vector v = r * 32 + lane (round r), elements
+// 4v .. 4v+3.  Loads are fully coalesced; ranks below follow this order, which
+// is ascending element index.
+__device__ __forceinline__ size_t vec_at(size_t tile, int r) {
+  return tile * kTile + (r * 32 + (threadIdx.x & 31)) * 4;
 }
 
-// The four values s = g (+ acc) of elements i .. i+3; out-of-range lanes get 0.
-// `vec` (host-checked 16-byte alignment of g and acc) turns the eight scalar
-// loads into two 128-bit loads.
-__device__ __forceinline__ void load_sum4(const float* __restrict__ g,
-                                          const float* __restrict__ acc, size_t i, size_t n,
-                                          bool vec, float (&s)[4]) {
+// The values of elements i .. i+3; out-of-range lanes get 0.  `vec` (host-checked
+// 16-byte alignment of every operand) allows 128-bit accesses.
+__device__ __forceinline__ void load4(const float* p, size_t i, size_t n, bool vec, float (&s)[4]) {
   if (vec && i + 4 <= n) {
-    const float4 a = *reinterpret_cast<const float4*>(g + i);
+    const float4 a = *reinterpret_cast<const float4*>(p + i);
     s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w;
-    if (acc) {
-      const float4 b = *reinterpret_cast<const float4*>(acc + i);
-      s[0] += b.x; s[1] += b.y; s[2] += b.z; s[3] += b.w;
-    }
   } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) s[j] = i + j < n ? load_sum(g, acc, i + j) : 0.0f;
+    for (int j = 0; j < 4; ++j) s[j] = i + j < n ? p[i + j] : 0.0f;
   }
 }
-
-__device__ __forceinline__ void store4(float* __restrict__ p, size_t i, size_t n, bool vec,
-                                       const float (&v)[4]) {
+__device__ __forceinline__ void store4(float* p, size_t i, size_t n, bool vec, const float (&v)[4]) {
   if (vec && i + 4 <= n) {
     *reinterpret_cast<float4*>(p + i) = make_float4(v[0], v[1], v[2], v[3]);
   } else {
@@ -95,504 +142,871 @@ __device__ __forceinline__ void store4(float* __restrict__ p, size_t i, size_t n
       if (i + j < n) p[i + j] = v[j];
   }
 }
+// s = g + acc for one tile, all loads issued before the first use.
+__device__ __forceinline__ void load_tile(const float* g, const float* acc, size_t tile, size_t n, bool vec,
+                                          float (&s)[kRounds][4]) {
+  float b[kRounds][4];
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) load4(g, vec_at(tile, r), n, vec, s[r]);
+  if (!acc) return;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) load4(acc, vec_at(tile, r), n, vec, b[r]);
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[r][j] += b[r][j];
+}
 
-// Exclusive offsets, in element order, of per-thread per-round counts c[r].
-// Returns the tile total.  smem: 32 unsigned.
-__device__ __forceinline__ unsigned tile_exclusive(const unsigned (&c)[kVecPerThread],
-                                                   unsigned (&excl)[kVecPerThread],
-                                                   unsigned* smem) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;  // 8 warps
-  unsigned incl[kVecPerThread];
+// Exclusive offsets, in element order, of this lane's counts inside the tile:
+// `mine` holds the counts of the four rounds, one byte each (<= 4; a warp's
+// total of a round is at most 128), so one scan serves all rounds.  Returns
+// the tile total.
+__device__ __forceinline__ unsigned tile_exclusive(unsigned mine, unsigned (&excl)[kRounds]) {
+  static_assert(kRounds == 4, "one byte per round");
+  const int lane = threadIdx.x & 31;
+  unsigned incl = mine;
 #pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    unsigned v = c[r];
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  const unsigned totals = __shfl_sync(0xffffffffu, incl, 31);
+  const unsigned before = incl - mine;      // bytes cannot borrow: incl >= mine in each
+  unsigned base = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += u;
-    }
-    incl[r] = v;
-    if (lane == 31) smem[r * 8 + w] = v;  // warp total for (round r, warp w)
+  for (int r = 0; r < kRounds; ++r) {
+    excl[r] = base + ((before >> (8 * r)) & 0xffu);
+    base += (totals >> (8 * r)) & 0xffu;
+  }
+  return base;
+}
+// One bit per element of a tile (bit 4r + j) -> the four counts, one byte each.
+__device__ __forceinline__ unsigned round_counts(unsigned m) {
+  return __popc(m & 0xfu) | __popc(m & 0xf0u) << 8 | __popc(m & 0xf00u) << 16 | __popc(m & 0xf000u) << 24;
+}
+// The bits of elements below n (all of them except in the last tile).
+__device__ __forceinline__ unsigned in_range(size_t tile, size_t n) {
+  if ((tile + 1) * kTile <= n) return 0xffffu;
+  unsigned m = 0;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m |= vec_at(tile, r) + j < n ? 1u << (4 * r + j) : 0u;
+  return m;
+}
+
+// Writes a tile's selected elements (bit 4r + j of `m`) to list[at ...] in
+// element order.  They pass through the warp's shared-memory slots so that the
+// list is written in full sectors: straight from the lanes every store would
+// carry one or two of them.  A tile with more than `slots` goes straight.
+__device__ __forceinline__ void list_tile(const float (&s)[kRounds][4], unsigned m, const unsigned (&excl)[kRounds],
+                                          unsigned total, size_t tile, int* list_idx, float* list_val, int* slot_idx,
+                                          float* slot_val, unsigned slots) {
+  const bool staged = total <= slots;
+  int* const di = staged ? slot_idx : list_idx;
+  float* const dv = staged ? slot_val : list_val;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    unsigned pos = excl[r];
+    const int i1 = static_cast<int>(vec_at(tile, r) + 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (m >> (4 * r + j) & 1u) {
+        di[pos] = i1 + j;
+        dv[pos] = s[r][j];
+        ++pos;
+      }
+  }
+  if (!staged) return;
+  __syncwarp();
+  for (unsigned e = threadIdx.x & 31; e < total; e += 32) {
+    list_idx[e] = slot_idx[e];
+    list_val[e] = slot_val[e];
+  }
+  __syncwarp();
+}
+
+// Sum over the CTA of one unsigned per thread (two at once); valid in every thread.
+__device__ __forceinline__ uint2 cta_sum2(unsigned a, unsigned b, uint2* sm) {
+  a = __reduce_add_sync(0xffffffffu, a);
+  b = __reduce_add_sync(0xffffffffu, b);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = make_uint2(a, b);
+  __syncthreads();
+  uint2 t = make_uint2(0, 0);
+#pragma unroll
+  for (int k = 0; k < kWarps; ++k) {
+    t.x += sm[k].x;
+    t.y += sm[k].y;
+  }
+  return t;
+}
+
+// What one warp left behind for its run of a chunk: elements selected (<= 2048),
+// list entries written (<= 352) and tiles listed (the first ones of the run).
+__device__ __forceinline__ unsigned pack_meta(unsigned count, unsigned used, unsigned listed) {
+  return count | used << 12 | listed << 24;
+}
+__device__ __forceinline__ unsigned meta_count(unsigned m) { return m & 0xfffu; }
+__device__ __forceinline__ unsigned meta_used(unsigned m) { return m >> 12 & 0xfffu; }
+__device__ __forceinline__ unsigned meta_listed(unsigned m) { return m >> 24; }
+
+// This warp's tiles [lo, hi) of a chunk.
+__device__ __forceinline__ void run_tiles(const Work& k, unsigned chunk, size_t n, size_t& lo, size_t& hi) {
+  const size_t tiles = (n + kTile - 1) / kTile;
+  lo = (static_cast<size_t>(chunk) * kWarps + (threadIdx.x >> 5)) * k.run;
+  hi = lo + k.run < tiles ? lo + k.run : tiles;
+  if (lo > hi) lo = hi;
+}
+// Calls body(chunk) in all warps of the CTA for each of its chunks, and then,
+// behind a barrier, after(chunk, parity) in all warps; `parity` alternates, so
+// that what the warps hand to `after` in shared memory can be double-buffered.
+// Every CTA's first chunk is its own number; the counter hands out the rest.
+template <bool DESCENDING, typename Body, typename After>
+__device__ __forceinline__ void for_chunks(const Work& k, unsigned* ticket, unsigned* sm_next, Body body, After after) {
+  unsigned c = blockIdx.x, parity = 0;
+  while (c < k.chunks) {
+    unsigned next = c + gridDim.x;
+    if (k.dynamic && threadIdx.x == 0) next = gridDim.x + atomicAdd(ticket, 1u);
+    const unsigned chunk = DESCENDING ? k.chunks - 1 - c : c;
+    body(chunk, parity);
+    if (k.dynamic && threadIdx.x == 0) sm_next[parity] = next;
+    __syncthreads();
+    after(chunk, parity);
+    c = k.dynamic ? sm_next[parity] : next;
+    parity ^= 1;
   }
   __syncthreads();
-  if (w == 0) {  // scan the 32 (round, warp) totals in element order
-    unsigned v = smem[lane];
-    unsigned s = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned u = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += u;
-    }
-    smem[lane] = s - v;          // exclusive
-    if (lane == 31) smem[32] = s;  // tile total
+}
+// After a grid barrier the chunks are walked in contiguous shares: this CTA's
+// [first, last), and how much one or two counts per chunk add up to before it.
+__device__ __forceinline__ void my_chunks(const Work& k, unsigned& first, unsigned& last) {
+  first = static_cast<unsigned>(static_cast<unsigned long long>(k.chunks) * blockIdx.x / gridDim.x);
+  last = static_cast<unsigned>(static_cast<unsigned long long>(k.chunks) * (blockIdx.x + 1) / gridDim.x);
+}
+struct Before {
+  unsigned before, total;
+};
+__device__ __forceinline__ Before counts_before(const unsigned* counts, unsigned chunks, unsigned first, uint2* sm) {
+  unsigned b = 0, t = 0;
+#pragma unroll 8
+  for (unsigned k = threadIdx.x; k < chunks; k += kBlock) {
+    const unsigned v = __ldcg(counts + k);
+    t += v;
+    b += k < first ? v : 0u;
   }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) excl[r] = smem[r * 8 + w] + incl[r] - c[r];
-  const unsigned total = smem[32];
-  __syncthreads();
-  return total;
+  const uint2 s = cta_sum2(b, t, sm);
+  return Before{s.x, s.y};
 }
 
 // ------------------------------------------------------------ threshold mode
-// kept value of element i: s = g (+ acc); |s| >= thr ? s : 0; sent iff != 0.
-// With a residual buffer the count pass leaves s = g + acc IN acc, so that the
-// write pass reads 4 bytes per element instead of 8 and only has to zero the
-// entries it sends (the residual of every other element is s itself).
-__global__ void __launch_bounds__(kBlock)
-thr_count_kernel(const float* __restrict__ g, float* __restrict__ acc, size_t n,
-                 float thr, unsigned* __restrict__ tile_counts, bool vec) {
-  __shared__ unsigned sm[32];
-  const size_t base = static_cast<size_t>(blockIdx.x) * kTile;
-  unsigned cnt = 0;
-#pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    float s[4];
-    load_sum4(g, acc, i, n, vec, s);      // out-of-range lanes are 0 and never counted
-    if (acc) store4(acc, i, n, vec, s);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cnt += (fabsf(s[j]) >= thr && s[j] != 0.0f) ? 1u : 0u;
-  }
-  // block total (integer, order irrelevant)
-  cnt = __reduce_add_sync(0xffffffffu, cnt);
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = cnt;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned t = 0;
-    for (int k = 0; k < kBlock / 32; ++k) t += sm[k];
-    tile_counts[blockIdx.x] = t;
-  }
-}
+// s = g (+ acc); kept = |s| >= thr ? s : 0; sent iff kept != 0; acc = s - kept.
+// BOUNDED: the payload layout is fixed, [idx(cap) | val(cap)], and only the
+// first `cap` selected entries (index order) are sent; the others go back into
+// the residual (without one they are lost) and their number is added to
+// *dropped, so the caller knows the length of the exchange before the count.
+struct ThrArgs {
+  const float* g;
+  float* acc;
+  size_t n;
+  float thr;
+  Work work;
+  Workspace ws;
+  int* idx_out;
+  float* val_out;        // null: right behind the indices (packed payload)
+  int* nnz_dev;
+  unsigned cap;          // BOUNDED only
+  unsigned long long* dropped;
+  bool vec;
+};
 
-// One CTA: exclusive scan of the tile counts (two arrays at once), totals to
-// the state.  In place: counts become offsets.  Every thread owns a contiguous
-// chunk: it adds the chunk up, a block-wide scan of the 1024 chunk totals gives
-// its base, and a second walk over the chunk writes the offsets.
-__global__ void __launch_bounds__(1024)
-scan_tiles_kernel(unsigned* __restrict__ a, unsigned* __restrict__ b, size_t tiles,
-                  SelectState* __restrict__ st, int write_nnz) {
-  __shared__ unsigned sa[32], sb[32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const size_t chunk = (tiles + 1023) / 1024;
-  const size_t lo = threadIdx.x * chunk, hi = lo + chunk < tiles ? lo + chunk : tiles;
-  constexpr int kReg = 32;                 // chunks up to 32 entries live in registers
-  const bool in_regs = chunk <= kReg;
-  unsigned ra_[kReg], rb_[kReg];
-  unsigned ta = 0, tb = 0;
-  if (in_regs) {
+template <bool BOUNDED>
+__global__ void __launch_bounds__(kBlock, kCtasPerSm)
+thr_select_kernel(const ThrArgs a) {
+  constexpr unsigned kSlots = 192;
+  __shared__ int slot_idx[kWarps][kSlots];
+  __shared__ float slot_val[kWarps][kSlots];
+  __shared__ uint2 sm[kWarps];
+  __shared__ unsigned warp_counts[2][kWarps], next[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for_chunks<false>(
+      a.work, a.ws.counters->ticket, next,
+      [&](unsigned chunk, unsigned parity) {
+        size_t lo, hi;
+        run_tiles(a.work, chunk, a.n, lo, hi);
+        const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+        int* const list_idx = a.ws.list_idx + run * a.work.capacity;
+        float* const list_val = a.ws.list_val + run * a.work.capacity;
+        unsigned used = 0, count = 0;
+        size_t unlisted = hi;           // tiles [unlisted, hi) are counted only; acc keeps s there
+        for (size_t tile = lo; tile < hi; ++tile) {
+          float s[kRounds][4];
+          load_tile(a.g, a.acc, tile, a.n, a.vec, s);
+          unsigned m = 0, excl[kRounds];  // out-of-range lanes are 0 and never selected
 #pragma unroll
-    for (int j = 0; j < kReg; ++j) {       // independent loads, one round trip
-      const size_t i = lo + j;
-      ra_[j] = (j < static_cast<int>(chunk) && i < tiles) ? a[i] : 0u;
-      rb_[j] = (b && j < static_cast<int>(chunk) && i < tiles) ? b[i] : 0u;
-    }
+          for (int r = 0; r < kRounds; ++r)
 #pragma unroll
-    for (int j = 0; j < kReg; ++j) {
-      ta += ra_[j];
-      tb += rb_[j];
-    }
-  } else {
-    for (size_t i = lo; i < hi; ++i) {
-      ta += a[i];
-      if (b) tb += b[i];
-    }
-  }
-  unsigned xa = ta, xb = tb;
+            for (int j = 0; j < 4; ++j)
+              m |= (fabsf(s[r][j]) >= a.thr && s[r][j] != 0.0f) ? 1u << (4 * r + j) : 0u;
+          const unsigned total = tile_exclusive(round_counts(m), excl);
+          if (unlisted == hi && used + total > a.work.capacity) unlisted = tile;
+          const bool listed = unlisted == hi;
+          if (a.acc) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned ua = __shfl_up_sync(0xffffffffu, xa, o);
-    const unsigned ub = __shfl_up_sync(0xffffffffu, xb, o);
-    if (lane >= o) { xa += ua; xb += ub; }
-  }
-  if (lane == 31) { sa[w] = xa; sb[w] = xb; }
-  __syncthreads();
-  if (w == 0) {
-    const unsigned va = sa[lane], vb = sb[lane];
-    unsigned ya = va, yb = vb;
+            for (int r = 0; r < kRounds; ++r) {
+              float res[4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned ua = __shfl_up_sync(0xffffffffu, ya, o);
-      const unsigned ub = __shfl_up_sync(0xffffffffu, yb, o);
-      if (lane >= o) { ya += ua; yb += ub; }
-    }
-    sa[lane] = ya - va;
-    sb[lane] = yb - vb;
-    if (lane == 31 && write_nnz) st->nnz = static_cast<int>(ya);
-  }
-  __syncthreads();
-  unsigned ra = sa[w] + xa - ta, rb = sb[w] + xb - tb;   // exclusive base of this chunk
-  if (in_regs) {
-#pragma unroll
-    for (int j = 0; j < kReg; ++j) {
-      const size_t i = lo + j;
-      if (j < static_cast<int>(chunk) && i < tiles) {
-        a[i] = ra;
-        ra += ra_[j];
-        if (b) {
-          b[i] = rb;
-          rb += rb_[j];
+              for (int j = 0; j < 4; ++j)
+                res[j] = listed && fabsf(s[r][j]) >= a.thr ? s[r][j] - s[r][j] : s[r][j];
+              store4(a.acc, vec_at(tile, r), a.n, a.vec, res);
+            }
+          }
+          count += total;
+          if (!listed || !total) continue;
+          list_tile(s, m, excl, total, tile, list_idx + used, list_val + used, slot_idx[warp], slot_val[warp], kSlots);
+          used += total;
         }
-      }
-    }
-    return;
-  }
-  for (size_t i = lo; i < hi; ++i) {
-    const unsigned va = a[i];
-    a[i] = ra;
-    ra += va;
-    if (b) {
-      const unsigned vb = b[i];
-      b[i] = rb;
-      rb += vb;
-    }
-  }
-}
+        if (lane == 0) {
+          a.ws.run_meta[run] = pack_meta(count, used, static_cast<unsigned>(unlisted - lo));
+          warp_counts[parity][warp] = count;
+        }
+      },
+      [&](unsigned chunk, unsigned parity) {
+        if (threadIdx.x != 0) return;
+        unsigned t = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) t += warp_counts[parity][w];
+        a.ws.chunk_a[chunk] = t;
+      });
+  cg::this_grid().sync();
 
-// `sum` is acc after the count pass (or g when there is no residual buffer).
-__global__ void __launch_bounds__(kBlock)
-thr_write_kernel(const float* __restrict__ sum, float* __restrict__ acc, size_t n, float thr,
-                 const unsigned* __restrict__ tile_offsets, int* __restrict__ idx_out,
-                 float* __restrict__ val_out, const SelectState* __restrict__ st, bool vec) {
-  __shared__ unsigned sm[33];
-  // packed payload [idx(nnz) | val(nnz)]: values start right after the indices
-  if (!val_out) val_out = reinterpret_cast<float*>(idx_out) + st->nnz;
-  const size_t base = static_cast<size_t>(blockIdx.x) * kTile;
-  float kept[kVecPerThread][4];
-  unsigned c[kVecPerThread], excl[kVecPerThread];
+  unsigned first, last;
+  my_chunks(a.work, first, last);
+  const Before b = counts_before(a.ws.chunk_a, a.work.chunks, first, sm);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.nnz_dev = static_cast<int>(b.total);
+  float* const val_out = a.val_out ? a.val_out : reinterpret_cast<float*>(a.idx_out) + (BOUNDED ? a.cap : b.total);
+  const float* const sum = a.acc ? a.acc : a.g;
+  unsigned lost = 0, chunk_at = b.before;
+  for (unsigned chunk = first; chunk < last; ++chunk) {
+    const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+    const int* const list_idx = a.ws.list_idx + run * a.work.capacity;
+    const float* const list_val = a.ws.list_val + run * a.work.capacity;
+    const unsigned meta = lane < kWarps ? __ldcg(a.ws.run_meta + run - warp + lane) : 0u;
+    // the first 128 entries are fetched beside the count (they are inside the
+    // segment whatever it is): one round trip per chunk instead of two
+    int idx[4];
+    float val[4];
 #pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    c[r] = 0;
-    float s[4], res[4];
-    load_sum4(sum, nullptr, i, n, vec, s);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float k = fabsf(s[j]) >= thr ? s[j] : 0.0f;   // out-of-range lanes: s == 0 -> k == 0
-      res[j] = s[j] - k;                                  // residual kept locally
-      kept[r][j] = k;
-      c[r] += k != 0.0f ? 1u : 0u;
+    for (int q = 0; q < 4; ++q) {
+      idx[q] = __ldcg(list_idx + lane + 32 * q);
+      val[q] = __ldcg(list_val + lane + 32 * q);
     }
-    if (acc && c[r]) store4(acc, i, n, vec, res);         // untouched vectors already hold their residual
-  }
-  tile_exclusive(c, excl, sm);
-  const unsigned tile_off = tile_offsets[blockIdx.x];
+    const unsigned mine = __shfl_sync(0xffffffffu, meta, warp), used = meta_used(mine);
+    unsigned base = chunk_at + __reduce_add_sync(0xffffffffu, lane < warp ? meta_count(meta) : 0u);
+    chunk_at += __reduce_add_sync(0xffffffffu, meta_count(meta));
+    for (unsigned e0 = lane; e0 < used; e0 += 128) {
 #pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    unsigned pos = tile_off + excl[r];
+      for (int q = 0; q < 4; ++q)
+        if (e0 >= 128 && e0 + 32 * q < used) {
+          idx[q] = __ldcg(list_idx + e0 + 32 * q);
+          val[q] = __ldcg(list_val + e0 + 32 * q);
+        }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (kept[r][j] != 0.0f) {
-        idx_out[pos] = static_cast<int>(i + j + 1);
-        val_out[pos] = kept[r][j];
-        ++pos;
-      }
-  }
-}
-
-// Capacity-bounded form: the payload layout is fixed, [idx(cap) | val(cap)],
-// and only the first `cap` selected entries (index order) are written.  The
-// others stay in the residual (acc keeps s there), so they are sent by a later
-// call; their number is added to *dropped.  With this the length of the
-// exchange is known on the host before the count is, and the caller needs no
-// host round trip between selection and all-gather.
-__global__ void __launch_bounds__(kBlock)
-thr_write_bounded_kernel(const float* __restrict__ sum, float* __restrict__ acc, size_t n, float thr,
-                         const unsigned* __restrict__ tile_offsets, int* __restrict__ idx_out, unsigned cap,
-                         unsigned long long* __restrict__ dropped, bool vec) {
-  __shared__ unsigned sm[33];
-  float* val_out = reinterpret_cast<float*>(idx_out) + cap;
-  const size_t base = static_cast<size_t>(blockIdx.x) * kTile;
-  float sv[kVecPerThread][4];
-  unsigned c[kVecPerThread], excl[kVecPerThread];
-#pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    c[r] = 0;
-    load_sum4(sum, nullptr, i, n, vec, sv[r]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) c[r] += (fabsf(sv[r][j]) >= thr && sv[r][j] != 0.0f) ? 1u : 0u;
-  }
-  tile_exclusive(c, excl, sm);
-  const unsigned tile_off = tile_offsets[blockIdx.x];
-  unsigned lost = 0;
-#pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    if (!c[r]) continue;                                  // untouched vectors already hold their residual
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    unsigned pos = tile_off + excl[r];
-    bool sent = false;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (fabsf(sv[r][j]) >= thr && sv[r][j] != 0.0f) {
-        if (pos < cap) {
-          idx_out[pos] = static_cast<int>(i + j + 1);
-          val_out[pos] = sv[r][j];
-          sv[r][j] = 0.0f;                                // sent: leaves the residual
-          sent = true;
+      for (int q = 0; q < 4; ++q) {
+        if (e0 + 32 * q >= used) break;
+        const unsigned pos = base + e0 + 32 * q;
+        if (!BOUNDED || pos < a.cap) {
+          a.idx_out[pos] = idx[q];
+          val_out[pos] = val[q];
         } else {
-          ++lost;                                         // over capacity: stays in the residual
+          if (a.acc) a.acc[idx[q] - 1] = val[q];
+          ++lost;
         }
-        ++pos;
       }
-    if (acc && sent) store4(acc, i, n, vec, sv[r]);
+    }
+    // tiles that did not fit the list: acc (or g) still holds s
+    base += used;
+    size_t lo, hi;
+    run_tiles(a.work, chunk, a.n, lo, hi);
+    for (size_t tile = lo + meta_listed(mine); tile < hi; ++tile) {
+      float s[kRounds][4];
+      load_tile(sum, nullptr, tile, a.n, a.vec, s);
+      unsigned m = 0, excl[kRounds];
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          m |= (fabsf(s[r][j]) >= a.thr && s[r][j] != 0.0f) ? 1u << (4 * r + j) : 0u;
+      const unsigned total = tile_exclusive(round_counts(m), excl);
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const size_t i = vec_at(tile, r);
+        unsigned pos = base + excl[r];
+        bool sent = false;
+        float res[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          res[j] = s[r][j];
+          if (!(fabsf(s[r][j]) >= a.thr)) continue;
+          if (s[r][j] == 0.0f) {                     // thr == 0: not sent, s - kept is still +0
+            res[j] = 0.0f;
+            sent = true;
+            continue;
+          }
+          if (!BOUNDED || pos < a.cap) {
+            a.idx_out[pos] = static_cast<int>(i + j + 1);
+            val_out[pos] = s[r][j];
+            res[j] = s[r][j] - s[r][j];
+            sent = true;
+          } else {
+            ++lost;
+          }
+          ++pos;
+        }
+        if (a.acc && sent) store4(a.acc, i, a.n, a.vec, res);
+      }
+      base += total;
+    }
   }
-  if (lost) atomicAdd(dropped, static_cast<unsigned long long>(lost));
+  if (BOUNDED) {
+    lost = __reduce_add_sync(0xffffffffu, lost);
+    if (lane == 0 && lost) atomicAdd(a.dropped, static_cast<unsigned long long>(lost));
+  }
 }
 
 // ---------------------------------------------------------------- top-K mode
 // mode 0 "magnitude": key = bits of |s| (monotonic in |s| for non-NaN);
 // mode 1 "compat":    key = |(int)s|, the value the reference's comparator
 //                     actually compares (both operands truncated to int).
-__device__ __forceinline__ unsigned make_key(float s, int mode) {
-  if (mode == 0) return __float_as_uint(s) & 0x7fffffffu;
+template <int MODE>
+__device__ __forceinline__ unsigned make_key(float s) {
+  if (MODE == 0) return __float_as_uint(s) & 0x7fffffffu;
   const int t = static_cast<int>(s);  // saturating truncation toward zero
   return t < 0 ? 0u - static_cast<unsigned>(t) : static_cast<unsigned>(t);
 }
 
-// Pass p (0,1,2) histograms bits [20..31], [10..19], [0..9] of the keys whose
-// higher bits equal the prefix decided so far.  Pass 0 also materialises
-// s = g + acc into `sum` so later passes read 4 bytes per element.
-template <int PASS>
-__global__ void __launch_bounds__(kBlock)
-topk_hist_kernel(const float* __restrict__ g, const float* __restrict__ acc,
-                 float* __restrict__ sum, size_t n, int mode,
-                 const SelectState* __restrict__ st, unsigned* __restrict__ hist, bool vec) {
-  constexpr int kBins = PASS == 0 ? kBins1 : kBins23;
-  constexpr int kShift = PASS == 0 ? 20 : (PASS == 1 ? 10 : 0);
-  __shared__ unsigned sh[kBins];
-  if (PASS == 1 && st->skip1) return;               // uniform for the whole grid
-  for (int b = threadIdx.x; b < kBins; b += kBlock) sh[b] = 0;
-  __syncthreads();
-  unsigned top = 0;                                  // PASS 0: largest key of this thread
-  const unsigned prefix = PASS == 0 ? 0u : st->prefix;
-  const unsigned hi_mask = PASS == 0 ? 0u : (PASS == 1 ? 0xfff00000u : 0xfffffc00u);
-  for (size_t tile = blockIdx.x; tile * kTile < n; tile += gridDim.x) {
-    const size_t base = tile * kTile;
+// Adds the four keys of one vector to a shared-memory histogram.  Fast path:
+// every lane of the warp takes all four of its elements and they fall into one
+// bin (always true when every key ties): one atomic per warp for 128 elements.
+__device__ __forceinline__ void tally4(unsigned* sh, const unsigned (&bin)[4], const bool (&take)[4]) {
+  const bool mine_same = take[0] && take[1] && take[2] && take[3] && bin[0] == bin[1] && bin[1] == bin[2] &&
+                         bin[2] == bin[3];
+  const unsigned b0 = __shfl_sync(0xffffffffu, bin[0], 0);
+  if (__all_sync(0xffffffffu, mine_same && bin[0] == b0)) {
+    if ((threadIdx.x & 31) == 0) atomicAdd(&sh[b0], 128u);
+  } else {
 #pragma unroll
-    for (int r = 0; r < kVecPerThread; ++r) {
-      const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-      float s[4];
-      if (PASS == 0) {
-        load_sum4(g, acc, i, n, vec, s);
-        if (acc) store4(sum, i, n, vec, s);         // sum == acc: the residual buffer now holds g + acc
-      } else {
-        load_sum4(sum, nullptr, i, n, vec, s);
-      }
-      unsigned bin[4];
-      bool take[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const unsigned key = make_key(s[j], mode);
-        take[j] = i + j < n && (key & hi_mask) == prefix;
-        bin[j] = (key >> kShift) & (kBins - 1);
-        if (PASS == 0 && i + j < n) top = max(top, key);
-      }
-      // Fast path: every lane of the warp takes all four of its elements and
-      // they all fall into one bin (always true when every key ties): one
-      // shared-memory atomic per warp for 128 elements.
-      const bool mine_same = take[0] && take[1] && take[2] && take[3] && bin[0] == bin[1] &&
-                             bin[1] == bin[2] && bin[2] == bin[3];
-      const unsigned b0 = __shfl_sync(0xffffffffu, bin[0], 0);
-      if (__all_sync(0xffffffffu, mine_same && bin[0] == b0)) {
-        if ((threadIdx.x & 31) == 0) atomicAdd(&sh[b0], 128u);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (take[j]) atomicAdd(&sh[bin[j]], 1u);
-      }
-    }
-  }
-  __syncthreads();
-  for (int b = threadIdx.x; b < kBins; b += kBlock)
-    if (sh[b]) atomicAdd(&hist[b], sh[b]);
-  if (PASS == 0) {
-    top = __reduce_max_sync(0xffffffffu, top);
-    if ((threadIdx.x & 31) == 0 && top) atomicMax(const_cast<unsigned*>(&st->max_key), top);
+    for (int j = 0; j < 4; ++j)
+      if (take[j]) atomicAdd(&sh[bin[j]], 1u);
   }
 }
 
-// One CTA: find the bin, counted from the top, in which the cumulative count
-// reaches `remaining`, and fix that bin's bits into the prefix.  Each of the
-// 1024 threads owns kBins/1024 consecutive bins (descending), a block-wide
-// inclusive scan gives every thread the count of all higher bins, and exactly
-// one thread finds the crossing inside its own bins.  Clears the histogram for
-// the next pass.
-template <int PASS>
-__global__ void __launch_bounds__(1024)
-topk_pick_kernel(unsigned* __restrict__ hist, SelectState* __restrict__ st, unsigned k_total) {
-  constexpr int kBins = PASS == 0 ? kBins1 : kBins23;
-  constexpr int kShift = PASS == 0 ? 20 : (PASS == 1 ? 10 : 0);
-  constexpr int kPer = kBins / 1024;                 // 4 or 1 bins per thread
-  __shared__ unsigned warp_tot[32];
-  if (PASS == 1 && st->skip1) return;                // prefix and remaining stand; the histogram is still clear
+template <int BINS>
+__device__ __forceinline__ void clear_bins(unsigned* sh) {
+  for (int b = threadIdx.x; b < BINS; b += kBlock) sh[b] = 0;
+  __syncthreads();
+}
+template <int BINS>
+__device__ __forceinline__ void flush_bins(const unsigned* sh, unsigned* global) {
+  __syncthreads();
+  for (int b = threadIdx.x; b < BINS; b += kBlock)
+    if (sh[b]) atomicAdd(&global[b], sh[b]);
+}
+
+// The bin, counted from the top, in which the cumulative count reaches
+// `remaining`, and how many elements are still to be taken from it.  Every CTA
+// works it out for itself from the global histogram.  If the total is short
+// (cannot happen for k <= n) the lowest bin takes whatever is left.
+template <int BINS>
+__device__ __forceinline__ void pick_bin(const unsigned* hist, unsigned& remaining, unsigned& bin, unsigned* sm) {
+  constexpr int kPer = BINS / kBlock;                // consecutive bins per thread, descending
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  // thread t owns descending bins  kBins-1 - t*kPer - j,  j = 0 .. kPer-1
   unsigned mine[kPer], local = 0;
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int b = kBins - 1 - (threadIdx.x * kPer + j);
-    mine[j] = hist[b];
-    hist[b] = 0;
-    local += mine[j];
+  for (int j = 0; j < kPer; j += 4) {
+    // bins kBins-1 - (t*kPer + j) and the three below it: one aligned vector, reversed
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(hist + BINS - 4 - (threadIdx.x * kPer + j)));
+    mine[j] = v.w; mine[j + 1] = v.z; mine[j + 2] = v.y; mine[j + 3] = v.x;
   }
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) local += mine[j];
   unsigned incl = local;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += u;
   }
-  if (lane == 31) warp_tot[w] = incl;
+  if (lane == 31) sm[w] = incl;
   __syncthreads();
-  if (w == 0) {
-    const unsigned t = warp_tot[lane];
-    unsigned x = t;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned u = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += u;
-    }
-    warp_tot[lane] = x - t;                          // exclusive over warps
-  }
-  __syncthreads();
-  const unsigned remaining0 = PASS == 0 ? k_total : st->remaining;
-  const unsigned prefix0 = PASS == 0 ? 0u : st->prefix;
-  unsigned above = warp_tot[w] + incl - local;       // elements in bins above this thread's
-  __syncthreads();
-  // crossing thread: above < remaining0 <= above + local.  If the total is
-  // short (cannot happen for k <= n) the lowest bin takes whatever is left.
-  const bool last = threadIdx.x == 1023;
-  if (above < remaining0 && (remaining0 <= above + local || last)) {
-    unsigned remaining = remaining0 - above;
-    int b = kBins - 1 - threadIdx.x * kPer;
+  unsigned above = incl - local;
+  for (int k = 0; k < w; ++k) above += sm[k];
+  const bool last = threadIdx.x == kBlock - 1;
+  if (above < remaining && (remaining <= above + local || last)) {   // exactly one thread
+    unsigned left = remaining - above;
+    int b = BINS - 1 - threadIdx.x * kPer;
+    bool found = false;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
-      if (mine[j] >= remaining || (last && j == kPer - 1)) break;
-      remaining -= mine[j];
-      --b;
+      if (!found && (mine[j] >= left || (last && j == kPer - 1))) {
+        found = true;
+        b -= j;
+      }
+      if (!found) left -= mine[j];
     }
-    const unsigned prefix = prefix0 | (static_cast<unsigned>(b) << kShift);
-    st->prefix = prefix;
-    st->remaining = remaining;
-    // Keys that all fit in the lowest digit (the integer-truncated keys of small
-    // gradients) leave the middle digit zero everywhere: skip that pass.
-    if (PASS == 0) st->skip1 = st->max_key < (1u << 10) ? 1u : 0u;
-    if (PASS == 2) {
-      st->threshold = prefix;
-      st->quota = remaining;
-      st->nnz = static_cast<int>(k_total);
-    }
+    sm[kWarps] = static_cast<unsigned>(b);
+    sm[kWarps + 1] = left;
   }
+  __syncthreads();
+  bin = sm[kWarps];
+  remaining = sm[kWarps + 1];
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(kBlock)
-topk_count_kernel(const float* __restrict__ sum, size_t n, int mode,
-                  const SelectState* __restrict__ st, unsigned* __restrict__ tile_gt,
-                  unsigned* __restrict__ tile_eq, bool vec) {
-  __shared__ unsigned sg[8], se[8];
-  const unsigned T = st->threshold;
-  const size_t base = static_cast<size_t>(blockIdx.x) * kTile;
-  unsigned gt = 0, eq = 0;
+struct TopkArgs {
+  const float* g;
+  float* acc;
+  size_t n;
+  unsigned k;
+  Work work;
+  Workspace ws;
+  int* idx_out;
+  float* val_out;
+  bool vec;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(kBlock, kCtasPerSm)
+topk_select_kernel(const TopkArgs a) {
+  __shared__ unsigned sh[kBins1];
+  __shared__ uint2 sm2[kWarps];
+  __shared__ unsigned sm[kWarps + 2], next[2];
+  cg::grid_group grid = cg::this_grid();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // pass 1 needs 1024 of the 4096 bins: the rest are the warps' list slots
+  constexpr unsigned kSlots = (kBins1 - kBins23) / (2 * kWarps);
+  int* const slot_idx = reinterpret_cast<int*>(sh + kBins23) + warp * 2 * kSlots;
+  float* const slot_val = reinterpret_cast<float*>(slot_idx + kSlots);
+  Counters* const cnt = a.ws.counters;
+  const size_t n = a.n;
+  const unsigned capacity = a.work.capacity;
+  const float* const sum = a.acc ? a.acc : a.g;      // s after pass 0
+  auto nothing = [](unsigned, unsigned) {};
+
+  // pass 0: fold the gradient into the residual, histogram of the top 12 key bits
+  clear_bins<kBins1>(sh);
+  unsigned top = 0;
+  for_chunks<false>(
+      a.work, &cnt->ticket[0], next,
+      [&](unsigned chunk, unsigned) {
+        size_t lo, hi;
+        run_tiles(a.work, chunk, n, lo, hi);
+        for (size_t tile = lo; tile < hi; ++tile) {
+          float s[kRounds][4];
+          load_tile(a.g, a.acc, tile, n, a.vec, s);
+          const unsigned valid = in_range(tile, n);
 #pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    float s[4];
-    load_sum4(sum, nullptr, i, n, vec, s);
+          for (int r = 0; r < kRounds; ++r) {
+            if (a.acc) store4(a.acc, vec_at(tile, r), n, a.vec, s[r]);
+            unsigned bin[4];
+            bool take[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (i + j < n) {
-        const unsigned key = make_key(s[j], mode);
-        gt += key > T;
-        eq += key == T;
-      }
-  }
-  gt = __reduce_add_sync(0xffffffffu, gt);
-  eq = __reduce_add_sync(0xffffffffu, eq);
-  if ((threadIdx.x & 31) == 0) { sg[threadIdx.x >> 5] = gt; se[threadIdx.x >> 5] = eq; }
+            for (int j = 0; j < 4; ++j) {
+              const unsigned key = make_key<MODE>(s[r][j]);  // 0 outside the range
+              take[j] = valid >> (4 * r + j) & 1u;
+              top = max(top, key);
+              bin[j] = key >> 20;
+            }
+            tally4(sh, bin, take);
+          }
+        }
+      },
+      nothing);
+  flush_bins<kBins1>(sh, cnt->hist0);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) sm[warp] = top;
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned a = 0, b = 0;
-    for (int k = 0; k < 8; ++k) { a += sg[k]; b += se[k]; }
-    tile_gt[blockIdx.x] = a;
-    tile_eq[blockIdx.x] = b;
+    for (int k = 1; k < kWarps; ++k) top = max(top, sm[k]);
+    if (top) atomicMax(&cnt->max_key, top);
+  }
+  grid.sync();
+
+  unsigned remaining = a.k, bin;
+  pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
+  const unsigned max_key = __ldcg(&cnt->max_key);
+  if (max_key == 0) {
+    // every key is 0 (small gradients under integer-truncated keys): the first
+    // k elements are sent, and the whole grid shares the work
+    for (size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x; i < a.k;
+         i += static_cast<size_t>(gridDim.x) * kBlock) {
+      a.idx_out[i] = static_cast<int>(i + 1);
+      a.val_out[i] = __ldcg(sum + i);                // written by another CTA in pass 0
+      if (a.acc) a.acc[i] = 0.0f;
+    }
+    return;
+  }
+
+  // pass 1: list the keys at or above the chosen bin (chunks in descending
+  // order: what pass 0 touched last is still in L2) and take the histogram of
+  // the next digit inside the bin
+  const bool low_only = max_key < (1u << 10);        // the middle digit is zero everywhere
+  const int shift = low_only ? 0 : 10;
+  unsigned prefix = bin << 20;
+  // The lowest bin takes in everything: no use listing it, and its keys tend
+  // to tie, which is what tally4 is for.
+  const bool everything = prefix == 0;
+  clear_bins<kBins23>(sh);
+  for_chunks<true>(
+      a.work, &cnt->ticket[1], next,
+      [&](unsigned chunk, unsigned) {
+        size_t lo, hi;
+        run_tiles(a.work, chunk, n, lo, hi);
+        const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+        int* const list_idx = a.ws.list_idx + run * capacity;
+        float* const list_val = a.ws.list_val + run * capacity;
+        unsigned used = 0;
+        size_t unlisted = everything ? lo : hi;      // tiles [unlisted, hi) are not in the list
+        for (size_t tile = lo; tile < hi; ++tile) {
+          float s[kRounds][4];
+          load_tile(sum, nullptr, tile, n, a.vec, s);
+          if (everything) {
+            const unsigned valid = in_range(tile, n);
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r) {
+              unsigned digit[4];
+              bool take[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const unsigned key = make_key<MODE>(s[r][j]);
+                take[j] = (valid >> (4 * r + j) & 1u) && key >> 20 == 0;
+                digit[j] = (key >> shift) & (kBins23 - 1);
+              }
+              tally4(sh, digit, take);
+            }
+            continue;
+          }
+          unsigned m = 0;                            // out-of-range lanes have key 0 < prefix
+#pragma unroll
+          for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m |= make_key<MODE>(s[r][j]) >= prefix ? 1u << (4 * r + j) : 0u;
+          if (!__any_sync(0xffffffffu, m)) continue;
+          // Few candidates per lane (about one element in sixty): walk the set
+          // bits and fetch the value again (an L1 hit) instead of sixteen
+          // predicated blocks.
+          bool room = unlisted == hi;
+          unsigned excl[kRounds];
+          unsigned total = 0;
+          if (room) {
+            total = tile_exclusive(round_counts(m), excl);
+            if (used + total > capacity) {
+              unlisted = tile;
+              room = false;
+            }
+          }
+          const bool staged = total <= kSlots;
+          int* const di = staged ? slot_idx : list_idx + used;
+          float* const dv = staged ? slot_val : list_val + used;
+          unsigned long long at = 0;
+          if (room) {
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r) at |= static_cast<unsigned long long>(excl[r]) << (16 * r);
+          }
+          for (unsigned left = m; left; left &= left - 1) {
+            const int q = __ffs(left) - 1;
+            const size_t i = vec_at(tile, q >> 2) + (q & 3);
+            const float v = sum[i];
+            const unsigned key = make_key<MODE>(v);
+            if (key >> 20 == bin) atomicAdd(&sh[(key >> shift) & (kBins23 - 1)], 1u);
+            if (room) {
+              const unsigned pos = static_cast<unsigned>(at >> (16 * (q >> 2))) & 0xffffu;
+              at += 1ull << (16 * (q >> 2));
+              di[pos] = static_cast<int>(i + 1);
+              dv[pos] = v;
+            }
+          }
+          if (!room) continue;
+          if (staged) {
+            __syncwarp();
+            for (unsigned e = lane; e < total; e += 32) {
+              list_idx[used + e] = slot_idx[e];
+              list_val[used + e] = slot_val[e];
+            }
+            __syncwarp();
+          }
+          used += total;
+        }
+        if (lane == 0) a.ws.run_meta[run] = pack_meta(0, used, static_cast<unsigned>(unlisted - lo));
+      },
+      nothing);
+  flush_bins<kBins23>(sh, cnt->hist1);
+  grid.sync();
+  pick_bin<kBins23>(cnt->hist1, remaining, bin, sm);
+  prefix |= bin << shift;
+
+  // From here on only the lists are looked at, and the tiles that are not in
+  // one.  Calls entry(value) for each listed entry and tile_fn(values, tile)
+  // for each other tile of this warp's run.
+  unsigned first, last;
+  my_chunks(a.work, first, last);
+  auto visit = [&](unsigned chunk, auto entry, auto tile_fn) {
+    const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+    const float* const list_val = a.ws.list_val + run * capacity;
+    const float v0 = __ldcg(list_val + lane);          // inside the segment whatever the count: one round trip less
+    const unsigned meta = __ldcg(a.ws.run_meta + run), used = meta_used(meta);
+    if (lane < used) entry(v0);
+    for (unsigned e = lane + 32; e < used; e += 32) entry(__ldcg(list_val + e));
+    size_t lo, hi;
+    run_tiles(a.work, chunk, n, lo, hi);
+    for (size_t tile = lo + meta_listed(meta); tile < hi; ++tile) {
+      float s[kRounds][4];
+      load_tile(sum, nullptr, tile, n, a.vec, s);
+      tile_fn(s, tile);
+    }
+  };
+  if (!low_only) {
+    // pass 2: the last digit
+    clear_bins<kBins23>(sh);
+    for (unsigned chunk = first; chunk < last; ++chunk)
+      visit(
+          chunk,
+          [&](float v) {
+            const unsigned key = make_key<MODE>(v);
+            if ((key & ~(kBins23 - 1u)) == prefix) atomicAdd(&sh[key & (kBins23 - 1)], 1u);
+          },
+          [&](const float (&s)[kRounds][4], size_t tile) {
+            const unsigned valid = in_range(tile, n);
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r) {
+              unsigned digit[4];
+              bool take[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const unsigned key = make_key<MODE>(s[r][j]);
+                take[j] = (valid >> (4 * r + j) & 1u) && (key & ~(kBins23 - 1u)) == prefix;
+                digit[j] = key & (kBins23 - 1);
+              }
+              tally4(sh, digit, take);
+            }
+          });
+    flush_bins<kBins23>(sh, cnt->hist2);
+    grid.sync();
+    pick_bin<kBins23>(cnt->hist2, remaining, bin, sm);
+    prefix |= bin;
+  }
+
+  // T = prefix: keys above T are sent, and the first `quota` keys equal to T
+  const unsigned T = prefix, quota = remaining;
+  auto masks = [&](const float (&s)[kRounds][4], size_t tile, unsigned& mg, unsigned& me) {
+    mg = me = 0;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned key = make_key<MODE>(s[r][j]);
+        mg |= key > T ? 1u << (4 * r + j) : 0u;
+        me |= key == T ? 1u << (4 * r + j) : 0u;
+      }
+    me &= in_range(tile, n);                         // out-of-range lanes have key 0: never above T
+  };
+  // counts per warp and chunk, greater in the high half (a run has <= 2048
+  // elements), kept for the positions below; sums per chunk for the other CTAs
+  for (unsigned chunk = first; chunk < last; ++chunk) {
+    unsigned c = 0;
+    visit(
+        chunk,
+        [&](float v) {
+          const unsigned key = make_key<MODE>(v);
+          c += key > T ? 0x10000u : key == T ? 1u : 0u;
+        },
+        [&](const float (&s)[kRounds][4], size_t tile) {
+          unsigned mg, me;
+          masks(s, tile, mg, me);
+          c += __popc(mg) << 16 | __popc(me);
+        });
+    c = __reduce_add_sync(0xffffffffu, c);
+    __syncthreads();
+    if (lane == 0) {
+      sm[warp] = c;
+      a.ws.run_counts[static_cast<size_t>(chunk) * kWarps + warp] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned g = 0, e = 0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        g += sm[w] >> 16;
+        e += sm[w] & 0xffffu;
+      }
+      a.ws.chunk_a[chunk] = g;
+      a.ws.chunk_b[chunk] = e;
+    }
+  }
+  grid.sync();
+  unsigned g_chunk = counts_before(a.ws.chunk_a, a.work.chunks, first, sm2).before;
+  unsigned e_chunk = counts_before(a.ws.chunk_b, a.work.chunks, first, sm2).before;
+
+  // payload position = (#greater before) + min(#equal before, quota)
+  auto send = [&](size_t index1, float v, unsigned ng, unsigned ne) {
+    const unsigned pos = ng + (ne < quota ? ne : quota);
+    a.idx_out[pos] = static_cast<int>(index1);
+    a.val_out[pos] = v;
+    if (a.acc) a.acc[index1 - 1] = 0.0f;             // s - s
+  };
+  const unsigned below = (1u << lane) - 1u;
+  for (unsigned chunk = first; chunk < last; ++chunk) {
+    const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+    const int* const list_idx = a.ws.list_idx + run * capacity;
+    const float* const list_val = a.ws.list_val + run * capacity;
+    const unsigned c = lane < kWarps ? __ldcg(a.ws.run_counts + run - warp + lane) : 0u;
+    const unsigned meta = __ldcg(a.ws.run_meta + run), used = meta_used(meta);
+    const float v0 = __ldcg(list_val + lane);          // four loads, one round trip
+    const int i0 = __ldcg(list_idx + lane);
+    const unsigned mine = __shfl_sync(0xffffffffu, c, warp);
+    unsigned g_at = g_chunk + __reduce_add_sync(0xffffffffu, lane < warp ? c >> 16 : 0u);
+    unsigned e_at = e_chunk + __reduce_add_sync(0xffffffffu, lane < warp ? c & 0xffffu : 0u);
+    g_chunk += __reduce_add_sync(0xffffffffu, c >> 16);
+    e_chunk += __reduce_add_sync(0xffffffffu, c & 0xffffu);
+    if (mine >> 16 == 0 && ((mine & 0xffffu) == 0 || e_at >= quota)) continue;   // this run sends nothing
+    for (unsigned base = 0; base < used; base += 32) {   // the list, 32 entries at a time, in order
+      const bool in = base + lane < used;
+      const float v = !in ? 0.0f : base == 0 ? v0 : __ldcg(list_val + base + lane);
+      const int idx = !in ? 0 : base == 0 ? i0 : __ldcg(list_idx + base + lane);
+      const unsigned key = make_key<MODE>(v);
+      const bool is_gt = in && key > T, is_eq = in && key == T;
+      const unsigned mg = __ballot_sync(0xffffffffu, is_gt), me = __ballot_sync(0xffffffffu, is_eq);
+      const unsigned ng = g_at + __popc(mg & below), ne = e_at + __popc(me & below);
+      if (is_gt || (is_eq && ne < quota)) send(static_cast<size_t>(idx), v, ng, ne);
+      g_at += __popc(mg);
+      e_at += __popc(me);
+    }
+    size_t lo, hi;
+    run_tiles(a.work, chunk, n, lo, hi);
+    for (size_t tile = lo + meta_listed(meta); tile < hi; ++tile) {
+      float s[kRounds][4];
+      load_tile(sum, nullptr, tile, n, a.vec, s);
+      unsigned mg, me, xg[kRounds], xe[kRounds];
+      masks(s, tile, mg, me);
+      const unsigned tg = tile_exclusive(round_counts(mg), xg), te = tile_exclusive(round_counts(me), xe);
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const size_t i = vec_at(tile, r);
+        unsigned ng = g_at + xg[r], ne = e_at + xe[r];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const bool is_gt = mg >> (4 * r + j) & 1u, is_eq = me >> (4 * r + j) & 1u;
+          if (is_gt || (is_eq && ne < quota)) send(i + j + 1, s[r][j], ng, ne);
+          ng += is_gt;
+          ne += is_eq;
+        }
+      }
+      g_at += tg;
+      e_at += te;
+    }
   }
 }
 
-// Selected: key > T, or key == T and fewer than `quota` equal keys precede it.
-// Payload position = (#greater before) + min(#equal before, quota).
+// -------------------------------------------------------- dense sum of payloads
+// The dense gradient is built tile by tile in shared memory: zeros, plus each
+// rank's entries of that tile in ascending rank order (the additions of the
+// reference's scatter, rank after rank), then one coalesced store to the
+// tensors the tile overlaps.  It replaces a fill of the dense buffer, one
+// scatter pass per rank that re-reads and re-writes scattered sectors of it,
+// and the copy back into the tensors: 4 B/element written, the payload read.
+// Payloads are in ascending index order, so a CTA finds its start in each with
+// one search and then walks forward.
+constexpr int kDenseTargets = 72;
+constexpr int kDenseTile = 4096;   // elements: 16 KB of shared memory
+struct DenseArgs {
+  const int* payload;          // rank r: [idx | val] at payload + r * stride
+  size_t stride;
+  size_t val_off;              // 0: the values follow the rank's own count
+  const int* counts_dev;       // counts on the device, clamped to val_off; null: counts[]
+  int world;
+  int counts[kMaxDenseRanks];
+  size_t first, last;          // element range of this launch
+  int targets;
+  size_t off[kDenseTargets + 1];   // first element of each target tensor; off[targets] == last
+  float* ptr[kDenseTargets];
+};
+
+// First position whose index is >= want (1-based, ascending): one warp, 32-ary.
+__device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned count, long long want) {
+  const unsigned lane = threadIdx.x & 31;
+  unsigned lo = 0, hi = count;                       // the answer is in [lo, hi]
+  while (hi > lo) {
+    const unsigned step = (hi - lo + 31) / 32;
+    const unsigned at = lo + lane * step;
+    const bool less = at < hi && static_cast<long long>(idx[at]) < want;
+    const unsigned m = __ballot_sync(0xffffffffu, less);
+    if (m == 0) return lo;
+    const unsigned top = 31 - __clz(m);              // probes below the answer are a prefix of the lanes
+    const unsigned base = lo + top * step;
+    hi = base + step < hi ? base + step : hi;
+    lo = base + 1;
+  }
+  return lo;
+}
+
 __global__ void __launch_bounds__(kBlock)
-topk_write_kernel(const float* __restrict__ sum, float* __restrict__ acc, size_t n, int mode,
-                  const SelectState* __restrict__ st, const unsigned* __restrict__ gt_off,
-                  const unsigned* __restrict__ eq_off, int* __restrict__ idx_out,
-                  float* __restrict__ val_out, bool vec) {
-  __shared__ unsigned sm[33];
-  const unsigned T = st->threshold, quota = st->quota;
-  // A tile that holds no key above T and no key == T that is still within the
-  // quota sends nothing, and its residual (acc already holds g + acc) stays as
-  // it is: leave before reading a byte.  The counts are differences of the
-  // scanned offsets; the last tile has no successor and always runs.
-  if (blockIdx.x + 1 < gridDim.x) {
-    const unsigned g_lo = gt_off[blockIdx.x], e_lo = eq_off[blockIdx.x];
-    const unsigned n_gt = gt_off[blockIdx.x + 1] - g_lo, n_eq = eq_off[blockIdx.x + 1] - e_lo;
-    if (n_gt == 0 && (n_eq == 0 || e_lo >= quota)) return;
-  }
-  const size_t base = static_cast<size_t>(blockIdx.x) * kTile;
-  float s[kVecPerThread][4];
-  unsigned cg[kVecPerThread], ce[kVecPerThread], eg[kVecPerThread], ee[kVecPerThread];
-  unsigned char flag[kVecPerThread][4];  // 0 none, 1 greater, 2 equal
-#pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    cg[r] = 0; ce[r] = 0;
-    load_sum4(sum, nullptr, i, n, vec, s[r]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      flag[r][j] = 0;
-      if (i + j < n) {
-        const unsigned key = make_key(s[r][j], mode);
-        if (key > T) { flag[r][j] = 1; ++cg[r]; }
-        else if (key == T) { flag[r][j] = 2; ++ce[r]; }
-      }
+dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta) {
+  __shared__ __align__(16) float out[kDenseTile];
+  __shared__ unsigned cursor[kMaxDenseRanks], count[kMaxDenseRanks];
+  const size_t begin = a.first + static_cast<size_t>(blockIdx.x) * tiles_per_cta * kDenseTile;
+  const size_t end = begin + static_cast<size_t>(tiles_per_cta) * kDenseTile < a.last
+                         ? begin + static_cast<size_t>(tiles_per_cta) * kDenseTile : a.last;
+  for (int r = threadIdx.x >> 5; r < a.world; r += kWarps) {
+    int c = a.counts_dev ? a.counts_dev[r] : a.counts[r];
+    if (c < 0) c = 0;
+    if (a.counts_dev && static_cast<size_t>(c) > a.val_off) c = static_cast<int>(a.val_off);
+    const unsigned at = warp_lower_bound(a.payload + r * a.stride, static_cast<unsigned>(c),
+                                         static_cast<long long>(begin) + 1);
+    if ((threadIdx.x & 31) == 0) {
+      cursor[r] = at;
+      count[r] = static_cast<unsigned>(c);
     }
   }
-  {  // one scan for both counters: greater in the high half, equal in the low half (each <= 4096)
-    unsigned packed[kVecPerThread], excl[kVecPerThread];
+  int target = 0;
+  while (target + 1 < a.targets && a.off[target + 1] <= begin) ++target;
+  for (size_t base = begin; base < end; base += kDenseTile) {
+    const size_t stop = base + kDenseTile < end ? base + kDenseTile : end;
+    __syncthreads();                                 // cursors set; the previous tile has been stored
 #pragma unroll
-    for (int r = 0; r < kVecPerThread; ++r) packed[r] = (cg[r] << 16) | ce[r];
-    tile_exclusive(packed, excl, sm);
-#pragma unroll
-    for (int r = 0; r < kVecPerThread; ++r) {
-      eg[r] = excl[r] >> 16;
-      ee[r] = excl[r] & 0xffffu;
-    }
-  }
-  const unsigned g0 = gt_off[blockIdx.x], e0 = eq_off[blockIdx.x];
-#pragma unroll
-  for (int r = 0; r < kVecPerThread; ++r) {
-    const size_t i = base + (static_cast<size_t>(r) * kBlock + threadIdx.x) * 4;
-    unsigned ng = g0 + eg[r], ne = e0 + ee[r];
-    float res[4];
-    bool any = false;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      bool sel = false;
-      if (flag[r][j] == 1) {
-        sel = true;
-      } else if (flag[r][j] == 2) {
-        sel = ne < quota;
+    for (int r = 0; r < kDenseTile / (4 * kBlock); ++r)
+      reinterpret_cast<float4*>(out)[r * kBlock + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    for (int r = 0; r < a.world; ++r) {
+      const int* idx = a.payload + r * a.stride;
+      const unsigned cnt = count[r];
+      const float* val = reinterpret_cast<const float*>(idx) + (a.val_off ? a.val_off : cnt);
+      unsigned c = cursor[r];
+      for (int in_tile = kBlock; in_tile == kBlock;) {
+        const unsigned j = c + threadIdx.x;
+        const int i = j < cnt ? idx[j] : 0;
+        const bool mine = i > 0 && static_cast<size_t>(i) <= stop;
+        if (mine && static_cast<size_t>(i) > base) out[i - 1 - base] += val[j];   // indices are unique within a payload
+        in_tile = __syncthreads_count(mine);
+        c += static_cast<unsigned>(in_tile);
       }
-      if (sel) {
-        const unsigned pos = ng + (ne < quota ? ne : quota);
-        idx_out[pos] = static_cast<int>(i + j + 1);
-        val_out[pos] = s[r][j];
-      }
-      res[j] = sel ? 0.0f : s[r][j];  // s - s == 0 when sent
-      any = any || sel;
-      if (flag[r][j] == 1) ++ng;
-      if (flag[r][j] == 2) ++ne;
+      if (threadIdx.x == 0) cursor[r] = c;           // read again behind the next barrier
     }
-    if (acc && any) store4(acc, i, n, vec, res);     // acc already holds s everywhere else
+    // store the tile to the tensors it overlaps
+    for (size_t at = base; at < stop;) {
+      const size_t seg_end = a.off[target + 1] < stop ? a.off[target + 1] : stop;
+      float* dst = a.ptr[target] + (at - a.off[target]);
+      const float* src = out + (at - base);
+      const int len = static_cast<int>(seg_end - at);
+      if (((reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>((at - base) * 4)) & 15u) == 0) {
+        const int nv = len >> 2;
+        for (int v = threadIdx.x; v < nv; v += kBlock)
+          reinterpret_cast<float4*>(dst)[v] = reinterpret_cast<const float4*>(src)[v];
+        for (int v = (nv << 2) + threadIdx.x; v < len; v += kBlock) dst[v] = src[v];
+      } else {
+        for (int v = threadIdx.x; v < len; v += kBlock) dst[v] = src[v];
+      }
+      at = seg_end;
+      if (seg_end == a.off[target + 1] && target + 1 < a.targets) ++target;
+    }
   }
 }
 
@@ -617,54 +1031,100 @@ scatter_add_kernel(const int* __restrict__ idx, const float* __restrict__ val, s
   }
 }
 
-int check_common(const float* g, size_t n, const void* idx_out, const void* val_out, void* ws,
-                 size_t ws_bytes) {
-  if (!g || !idx_out || !val_out) return SGB_ERR_NULL;
+int check_common(const float* g, size_t n, const void* idx_out, void* ws, size_t ws_bytes) {
+  if (!g || !idx_out) return SGB_ERR_NULL;
   if (n > 0x7fffffffu) return SGB_ERR_SIZE;  // 1-based int32 indices on the wire
   if (!ws || ws_bytes < workspace_bytes(n) || (reinterpret_cast<uintptr_t>(ws) & 255u))
     return SGB_ERR_WORKSPACE;
   return SGB_OK;
 }
 
-}  // namespace
-
-// ---- two-phase form used by the communicator (declared in sparse.cuh) ------
-int sparse_threshold_count(const float* g, float* acc, size_t n, float thr, int* nnz_dev,
-                           void* ws, size_t ws_bytes, cudaStream_t s) {
-  if (n == 0) {
-    cudaError_t e = cudaMemsetAsync(nnz_dev, 0, sizeof(int), s);
-    return e == cudaSuccess ? SGB_OK : note_cuda_error(e);
-  }
-  if (n > 0x7fffffffu) return SGB_ERR_SIZE;
-  if (!ws || ws_bytes < workspace_bytes(n) || (reinterpret_cast<uintptr_t>(ws) & 255u))
-    return SGB_ERR_WORKSPACE;
-  Workspace w = carve(ws, n);
-  const unsigned tiles = static_cast<unsigned>(tiles_of(n));
-  thr_count_kernel<<<tiles, kBlock, 0, s>>>(g, acc, n, thr, w.tile_counts, aligned16(g) && (!acc || aligned16(acc)));
-  scan_tiles_kernel<<<1, 1024, 0, s>>>(w.tile_counts, nullptr, tiles, w.state, 1);
-  cudaError_t e = cudaMemcpyAsync(nnz_dev, &w.state->nnz, sizeof(int), cudaMemcpyDeviceToDevice, s);
+// A grid whose CTAs wait for one another: all of them are resident or the
+// launch fails.  work_for() asks for at most kCtasPerSm CTAs per SM, which the
+// launch bounds and the shared memory of both kernels allow.
+template <typename A>
+int launch_cooperative(void (*kernel)(A), unsigned grid, const A& args, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kBlock);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args);
   if (e != cudaSuccess) return note_cuda_error(e);
   return launch_status();
 }
 
-int sparse_threshold_write_packed(const float* g, float* acc, size_t n, float thr, int* payload,
-                                  void* ws, cudaStream_t s) {
-  if (n == 0) return SGB_OK;
-  Workspace w = carve(ws, n);
-  const unsigned tiles = static_cast<unsigned>(tiles_of(n));
-  thr_write_kernel<<<tiles, kBlock, 0, s>>>(acc ? acc : g, acc, n, thr, w.tile_counts, payload, nullptr, w.state, aligned16(g) && (!acc || aligned16(acc)));
-  return launch_status();
+int threshold_select(const float* g, float* acc, size_t n, float thr, int* idx_out, float* val_out, int* nnz_dev,
+                     size_t cap, unsigned long long* dropped, void* ws, size_t ws_bytes, cudaStream_t s) {
+  if (!nnz_dev) return SGB_ERR_NULL;
+  if (n == 0) {
+    cudaError_t e = cudaMemsetAsync(nnz_dev, 0, sizeof(int), s);
+    return e == cudaSuccess ? SGB_OK : note_cuda_error(e);
+  }
+  const int st = check_common(g, n, idx_out, ws, ws_bytes);
+  if (st != SGB_OK) return st;
+  const Work work = work_for(n);
+  ThrArgs a{g, acc, n, thr, work, carve(ws, work), idx_out, val_out, nnz_dev, static_cast<unsigned>(cap), dropped,
+            aligned16(g) && (!acc || aligned16(acc))};
+  if (work.dynamic) {
+    cudaError_t e = cudaMemsetAsync(a.ws.counters->ticket, 0, sizeof(a.ws.counters->ticket), s);
+    if (e != cudaSuccess) return note_cuda_error(e);
+  }
+  return cap ? launch_cooperative(thr_select_kernel<true>, work.grid, a, s)
+             : launch_cooperative(thr_select_kernel<false>, work.grid, a, s);
 }
 
-int sparse_threshold_write_bounded(const float* g, float* acc, size_t n, float thr, int* payload, size_t cap,
-                                   unsigned long long* dropped_dev, void* ws, cudaStream_t s) {
-  if (n == 0) return SGB_OK;
+}  // namespace
+
+// ---- forms used by the communicator (declared in sparse.cuh) ---------------
+int sparse_threshold_packed(const float* g, float* acc, size_t n, float thr, int* payload, int* nnz_dev, void* ws,
+                            size_t ws_bytes, cudaStream_t s) {
+  return threshold_select(g, acc, n, thr, payload, nullptr, nnz_dev, 0, nullptr, ws, ws_bytes, s);
+}
+
+int sparse_threshold_bounded(const float* g, float* acc, size_t n, float thr, int* payload, size_t cap, int* nnz_dev,
+                             unsigned long long* dropped_dev, void* ws, size_t ws_bytes, cudaStream_t s) {
   if (cap == 0 || cap > 0x7fffffffu || !dropped_dev) return SGB_ERR_SIZE;
-  Workspace w = carve(ws, n);
-  const unsigned tiles = static_cast<unsigned>(tiles_of(n));
-  thr_write_bounded_kernel<<<tiles, kBlock, 0, s>>>(acc ? acc : g, acc, n, thr, w.tile_counts, payload,
-                                                    static_cast<unsigned>(cap), dropped_dev,
-                                                    aligned16(g) && (!acc || aligned16(acc)));
+  return threshold_select(g, acc, n, thr, payload, nullptr, nnz_dev, cap, dropped_dev, ws, ws_bytes, s);
+}
+
+int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
+                     int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s) {
+  DenseArgs a;
+  if (world < 1 || world > kMaxDenseRanks) return SGB_ERR_UNSUPPORTED;
+  a.payload = payload;
+  a.stride = stride;
+  a.val_off = val_off;
+  a.counts_dev = counts_dev;
+  a.world = world;
+  for (int r = 0; r < world; ++r) a.counts[r] = counts_dev ? 0 : counts[r];
+  size_t at = 0;
+  for (size_t k = 0; k < ntensors;) {
+    a.first = at;
+    a.targets = 0;
+    while (k < ntensors && a.targets < kDenseTargets) {
+      if (sizes[k]) {
+        // tensors that lie back to back are one target
+        if (a.targets && a.ptr[a.targets - 1] + (at - a.off[a.targets - 1]) == tensors[k]) {
+        } else {
+          a.off[a.targets] = at;
+          a.ptr[a.targets++] = tensors[k];
+        }
+        at += sizes[k];
+      }
+      ++k;
+    }
+    if (!a.targets) continue;
+    a.last = at;
+    a.off[a.targets] = at;
+    const size_t tiles = ceil_div(a.last - a.first, kDenseTile);
+    const unsigned per = static_cast<unsigned>(ceil_div(tiles, static_cast<size_t>(sm_count()) * 8));
+    dense_from_payloads_kernel<<<static_cast<unsigned>(ceil_div(tiles, per)), kBlock, 0, s>>>(a, per);
+  }
   return launch_status();
 }
 
@@ -689,22 +1149,8 @@ int sgb_topk_count(float ratio, size_t n) {
 int sgb_sparse_threshold_f32(const float* g, float* acc, size_t n, float thr, int32_t* idx_out,
                              float* val_out, int32_t* nnz_dev, void* ws, size_t ws_bytes,
                              void* stream) {
-  if (!nnz_dev) return SGB_ERR_NULL;
-  cudaStream_t s = as_stream(stream);
-  if (n == 0) {
-    cudaError_t e = cudaMemsetAsync(nnz_dev, 0, sizeof(int), s);
-    return e == cudaSuccess ? SGB_OK : note_cuda_error(e);
-  }
-  int st = check_common(g, n, idx_out, val_out, ws, ws_bytes);
-  if (st != SGB_OK) return st;
-  Workspace w = carve(ws, n);
-  const unsigned tiles = static_cast<unsigned>(tiles_of(n));
-  thr_count_kernel<<<tiles, kBlock, 0, s>>>(g, acc, n, thr, w.tile_counts, aligned16(g) && (!acc || aligned16(acc)));
-  scan_tiles_kernel<<<1, 1024, 0, s>>>(w.tile_counts, nullptr, tiles, w.state, 1);
-  cudaError_t e = cudaMemcpyAsync(nnz_dev, &w.state->nnz, sizeof(int), cudaMemcpyDeviceToDevice, s);
-  if (e != cudaSuccess) return note_cuda_error(e);
-  thr_write_kernel<<<tiles, kBlock, 0, s>>>(acc ? acc : g, acc, n, thr, w.tile_counts, idx_out, val_out, w.state, aligned16(g) && (!acc || aligned16(acc)));
-  return launch_status();
+  if (n && !val_out) return SGB_ERR_NULL;
+  return threshold_select(g, acc, n, thr, idx_out, val_out, nnz_dev, 0, nullptr, ws, ws_bytes, as_stream(stream));
 }
 
 int sgb_sparse_topk_f32(const float* g, float* acc, float* sum_scratch, size_t n, size_t k,
@@ -713,29 +1159,18 @@ int sgb_sparse_topk_f32(const float* g, float* acc, float* sum_scratch, size_t n
   if (n == 0 || k == 0) return SGB_OK;
   if (mode != 0 && mode != 1) return SGB_ERR_UNSUPPORTED;
   (void)sum_scratch;   // kept in the signature; the sum lives in acc (or is g itself without a residual)
-  int st = check_common(g, n, idx_out, val_out, ws, ws_bytes);
+  if (!val_out) return SGB_ERR_NULL;
+  int st = check_common(g, n, idx_out, ws, ws_bytes);
   if (st != SGB_OK) return st;
   if (k > n) k = n;
   cudaStream_t s = as_stream(stream);
-  Workspace w = carve(ws, n);
-  const unsigned tiles = static_cast<unsigned>(tiles_of(n));
-  const unsigned hgrid = capped_grid(tiles, 1, 8);
-  const bool vec = aligned16(g) && (!acc || aligned16(acc));
-  float* sum = acc ? acc : const_cast<float*>(g);
-  // histogram and the selection state behind it (one contiguous region)
-  cudaError_t e = cudaMemsetAsync(w.hist, 0, align256(kBins1 * sizeof(unsigned)) + sizeof(SelectState), s);
+  const Work work = work_for(n);
+  TopkArgs a{g, acc, n, static_cast<unsigned>(k), work, carve(ws, work), idx_out, val_out,
+             aligned16(g) && (!acc || aligned16(acc))};
+  cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
   if (e != cudaSuccess) return note_cuda_error(e);
-  topk_hist_kernel<0><<<hgrid, kBlock, 0, s>>>(g, acc, sum, n, mode, w.state, w.hist, vec);
-  topk_pick_kernel<0><<<1, 1024, 0, s>>>(w.hist, w.state, static_cast<unsigned>(k));
-  topk_hist_kernel<1><<<hgrid, kBlock, 0, s>>>(g, acc, sum, n, mode, w.state, w.hist, vec);
-  topk_pick_kernel<1><<<1, 1024, 0, s>>>(w.hist, w.state, static_cast<unsigned>(k));
-  topk_hist_kernel<2><<<hgrid, kBlock, 0, s>>>(g, acc, sum, n, mode, w.state, w.hist, vec);
-  topk_pick_kernel<2><<<1, 1024, 0, s>>>(w.hist, w.state, static_cast<unsigned>(k));
-  topk_count_kernel<<<tiles, kBlock, 0, s>>>(sum, n, mode, w.state, w.tile_gt, w.tile_eq, vec);
-  scan_tiles_kernel<<<1, 1024, 0, s>>>(w.tile_gt, w.tile_eq, tiles, w.state, 0);
-  topk_write_kernel<<<tiles, kBlock, 0, s>>>(sum, acc, n, mode, w.state, w.tile_gt,
-                                             w.tile_eq, idx_out, val_out, vec);
-  return launch_status();
+  return mode == 0 ? launch_cooperative(topk_select_kernel<0>, work.grid, a, s)
+                   : launch_cooperative(topk_select_kernel<1>, work.grid, a, s);
 }
 
 int sgb_scatter_add_f32(const int32_t* idx, const float* val, size_t count,

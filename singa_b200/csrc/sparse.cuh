@@ -1,24 +1,28 @@
-// Internal two-phase interface of the threshold sparsifier, used by the
-// communicator so that the payload length can travel to the host while the
-// compaction kernel is already running.
+// Internal interface of the sparsifiers, used by the communicator.
 #pragma once
 #include "common.cuh"
 
 namespace sgb {
 
-// Phase 1: per-tile counts + scan; the payload length lands in *nnz_dev.
-int sparse_threshold_count(const float* g, float* acc, size_t n, float thr, int* nnz_dev,
-                           void* ws, size_t ws_bytes, cudaStream_t s);
+constexpr int kMaxDenseRanks = 64;
 
-// Phase 2: residual update and packed payload [idx(nnz) | val(nnz)] written to
-// `payload` (int32 view), using the offsets left in `ws` by phase 1.
-int sparse_threshold_write_packed(const float* g, float* acc, size_t n, float thr, int* payload,
-                                  void* ws, cudaStream_t s);
+// Threshold selection with residual update and packed payload [idx(nnz) | val(nnz)]
+// (int32 view); the payload length lands in *nnz_dev.
+int sparse_threshold_packed(const float* g, float* acc, size_t n, float thr, int* payload, int* nnz_dev, void* ws,
+                            size_t ws_bytes, cudaStream_t s);
 
-// Phase 2, capacity-bounded: payload [idx(cap) | val(cap)]; selected entries
-// beyond the first `cap` (index order) stay in the residual and are counted in
-// *dropped_dev (a device counter the caller owns).
-int sparse_threshold_write_bounded(const float* g, float* acc, size_t n, float thr, int* payload, size_t cap,
-                                   unsigned long long* dropped_dev, void* ws, cudaStream_t s);
+// Capacity-bounded form: payload [idx(cap) | val(cap)]; selected entries beyond
+// the first `cap` (index order) stay in the residual and are counted in
+// *dropped_dev (a device counter the caller owns).  *nnz_dev is the full count.
+int sparse_threshold_bounded(const float* g, float* acc, size_t n, float thr, int* payload, size_t cap, int* nnz_dev,
+                             unsigned long long* dropped_dev, void* ws, size_t ws_bytes, cudaStream_t s);
+
+// Dense sum of `world` payloads (ascending indices, rank r at payload + r *
+// stride words) into the tensors, which cover the index space in list order.
+// Values start val_off words behind the indices, or, with val_off == 0, right
+// behind the rank's own count.  counts: host array, or counts_dev on the device
+// (then clamped to val_off).
+int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
+                     int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s);
 
 }  // namespace sgb

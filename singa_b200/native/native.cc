@@ -638,6 +638,19 @@ PyObject* py_comm_sparsify(Args a, Py_ssize_t) {  // (communicator, tensors, acc
   ISSUE(sgb_comm_sparsification, comm(a[0]), l.ptrs.data(), l.sizes.data(), l.n(), acc, spars, topk, stream());
   Py_RETURN_NONE;
 }
+PyObject* py_comm_sparsify_begin(Args a, Py_ssize_t) {  // as comm_sparsify: the selection half
+  require(first_type(a[1]) == at::kFloat, "sparsification supports fp32 only");
+  const TensorList l(a[1], false);
+  float* acc = is_none(a[2]) ? nullptr : f32w(tensor(a[2]));
+  const float spars = static_cast<float>(real(a[3]));
+  const int topk = truth(a[4]);
+  ISSUE(sgb_comm_sparsification_begin, comm(a[0]), l.ptrs.data(), l.sizes.data(), l.n(), acc, spars, topk, stream());
+  Py_RETURN_NONE;
+}
+PyObject* py_comm_sparsify_end(Args a, Py_ssize_t) {
+  ISSUE(sgb_comm_sparsification_end, comm(a[0]), stream());
+  Py_RETURN_NONE;
+}
 PyObject* py_comm_wait(Args a, Py_ssize_t) {
   ISSUE(sgb_comm_wait, comm(a[0]), stream());
   Py_RETURN_NONE;
@@ -832,7 +845,7 @@ PyMethodDef kMethods[] = {
     METHOD(bn_backward, 9), METHOD(bn_add_relu_backward, 10), METHOD(pool_forward, 5), METHOD(pool_backward, 5),
     METHOD(pool_forward_argmax, 4), METHOD(pool_backward_argmax, 3), METHOD(sgd_multi, 9), METHOD(pack, 3), METHOD(unpack, 4),
     METHOD(comm_synch, 2), METHOD(comm_synch_half, 2), METHOD(comm_fused_synch, 3), METHOD(comm_fused_synch_half, 3),
-    METHOD(comm_sparsify, 5), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
+    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

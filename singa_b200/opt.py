@@ -235,21 +235,43 @@ class DistOpt(object):
                 self.gradAccumulation.append(torch.zeros(n, dtype=like.dtype, device=like.device))
             return self.gradAccumulation[k] if corr else None
 
-        for name, p, g in grad_stream:
-            if g.numel() > threshold:
+        # A communicator that offers the exchange in two halves has bucket k's
+        # selection issued before the host waits for the counts of bucket k-1.
+        begin = getattr(self.communicator, "beginSparsification", None)
+        opened = 0
+
+        def exchange(tensors, n, single):
+            nonlocal opened
+            if begin is not None:
+                begin(tensors, residual(n, tensors[0]), spars, topK)
+                opened += 1
+                if opened == 2:
+                    self.communicator.endSparsification()
+                    opened = 1
+            elif single:
+                self.sparsification(tensors[0], residual(n, tensors[0]), spars, topK)
+            else:
+                self.fused_sparsification(tensors, residual(n, tensors[0]), spars, topK)
+
+        for triple in grad_stream:
+            g = triple[2]
+            n = g.numel()
+            if n > threshold:
                 k += 1
-                self.sparsification(g, residual(g.numel(), g), spars, topK)
+                exchange([g], n, True)
             else:
                 glist.append(g)
-                acc += g.numel()
+                acc += n
                 if acc > threshold:
                     k += 1
-                    self.fused_sparsification(glist, residual(acc, g), spars, topK)
+                    exchange(glist, acc, False)
                     acc, glist = 0, []
-            plist.append((name, p, g))
+            plist.append(triple)
         if glist:
             k += 1
-            self.fused_sparsification(glist, residual(acc, glist[0]), spars, topK)
+            exchange(glist, acc, False)
+        if opened:
+            self.communicator.endSparsification()
         self.wait()
         self.sparsInit = True
         self._update_all(plist)
