@@ -63,6 +63,7 @@ __device__ __forceinline__ void sgd_one(float& p, float g, float& m, const SgdAr
 
 __global__ void __launch_bounds__(kBlock)
 sgd_multi_kernel(const __grid_constant__ Table t, const SgdArgs a) {
+  dependency_wait();
   const int k = find_tensor(t, blockIdx.x);
   const size_t n = t.n[k];
   const size_t base = static_cast<size_t>(blockIdx.x - t.first_tile[k]) * kTile;
@@ -77,6 +78,7 @@ sgd_multi_kernel(const __grid_constant__ Table t, const SgdArgs a) {
     vp.u = ld128(p + i);
     vg.u = ld128(g + i);
     if (a.use_momentum) vm.u = ld128(m + i);
+    release_dependents();
 #pragma unroll
     for (int j = 0; j < 4; ++j) sgd_one(vp.f[j], vg.f[j], vm.f[j], a);
     st128(p + i, vp.u);
@@ -97,6 +99,8 @@ template <int MODE>
 __global__ void __launch_bounds__(kBlock)
 pack_multi_kernel(const __grid_constant__ Table t, const __grid_constant__ Offsets o,
                   void* flat, float scale, int use_scale) {
+  dependency_wait();
+  release_dependents();
   const int k = find_tensor(t, blockIdx.x);
   const size_t n = t.n[k];
   const size_t i = static_cast<size_t>(blockIdx.x - t.first_tile[k]) * kTile + 4 * threadIdx.x;
@@ -217,12 +221,12 @@ int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t coun
     if (cnt == 0) continue;
     // offsets inside the chunk are contiguous because empty tensors add 0
     const unsigned tiles = fill_table(t, &o, ptrs, nullptr, nullptr, ns, 0, cnt, chunk_off);
-    switch (mode) {
-      case kPackF32: pack_multi_kernel<kPackF32><<<tiles, kBlock, 0, s>>>(t, o, flat, scale, use_scale); break;
-      case kPackF32ToF16: pack_multi_kernel<kPackF32ToF16><<<tiles, kBlock, 0, s>>>(t, o, flat, scale, use_scale); break;
-      case kUnpackF32: pack_multi_kernel<kUnpackF32><<<tiles, kBlock, 0, s>>>(t, o, flat, scale, use_scale); break;
-      default: pack_multi_kernel<kUnpackF16ToF32><<<tiles, kBlock, 0, s>>>(t, o, flat, scale, use_scale); break;
-    }
+    auto kernel = mode == kPackF32        ? pack_multi_kernel<kPackF32>
+                  : mode == kPackF32ToF16 ? pack_multi_kernel<kPackF32ToF16>
+                  : mode == kUnpackF32    ? pack_multi_kernel<kUnpackF32>
+                                          : pack_multi_kernel<kUnpackF16ToF32>;
+    const int st = launch_ex(kernel, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, o, flat, scale, use_scale);
+    if (st != SGB_OK) return st;
   }
   return launch_status();
 }
@@ -272,7 +276,8 @@ int sgb_sgd_update_multi_f32(void* const* params, void* const* grads, void* cons
     }
     if (cnt == 0) continue;
     const unsigned tiles = fill_table(t, nullptr, pa, pb, pc, ns, 0, cnt, 0);
-    sgd_multi_kernel<<<tiles, kBlock, 0, s>>>(t, a);
+    const int st = launch_ex(sgd_multi_kernel, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, a);
+    if (st != SGB_OK) return st;
   }
   return launch_status();
 }

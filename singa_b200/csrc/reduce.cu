@@ -5,68 +5,180 @@
 // All sums are formed in a fixed order (per-thread strided accumulation, warp
 // shuffles, then a fixed-order combine of per-CTA partials), so results are
 // identical from run to run; none uses atomics.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace sgb {
 namespace {
 
 constexpr int kBlock = 256;
+constexpr int kWarps = kBlock / 32;
+constexpr int kMaxCluster = 8;
 
 // ---------------------------------------------------------------- column sums
-// v[c] = sum_r M[r][c].  A CTA owns 32 adjacent columns (one per lane) and a
-// slice of the rows (blockIdx.y); its 8 warps stride over the rows, so every
-// warp-load is one coalesced 128-byte line.  With gridDim.y > 1 the CTA writes
-// a partial row to `partial` and the second kernel adds the slices in order.
-__global__ void __launch_bounds__(kBlock)
-colsum_kernel(const float* __restrict__ M, float* __restrict__ out, size_t nrow,
-              size_t ncol, size_t rows_per_slice) {
-  __shared__ float sm[8][33];
+// v[c] = sum_r M[r][c].  A CTA owns a block of adjacent columns and a slice of
+// the rows; its 8 warps stride over the rows.  A lane owns one column (or four
+// adjacent ones, VEC); matrices narrower than a warp put 32 / width rows side
+// by side in a warp (`shift` = log2 of the lanes per row).  Eight loads per
+// lane are in flight.  The slices of a column block are the CTAs of one
+// thread-block cluster: their partial sums meet in the first CTA's shared
+// memory and are added in rank order, so a call is one launch (it was two: the
+// problems here are a few microseconds, a launch is half of that).  With more
+// slices than a cluster holds, the CTAs leave partial rows in `out` and
+// colsum_finish_kernel adds them.
+template <bool VEC>
+__global__ void __launch_bounds__(kBlock, 4)
+colsum_kernel(const float* __restrict__ M, float* __restrict__ out, size_t nrow, size_t ncol, size_t rows_per_slice,
+              int slices, int shift, bool clustered) {
+  constexpr int kW = VEC ? 4 : 1;
+  __shared__ float sm[kWarps][32 * kW];
+  __shared__ float part[kMaxCluster][32 * kW];
+  dependency_wait();
+  release_dependents();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const size_t c = blockIdx.x * 32ull + lane;
-  const size_t r0 = blockIdx.y * rows_per_slice;
+  const size_t block = blockIdx.x / slices;
+  const int slice = static_cast<int>(blockIdx.x - block * slices);
+  const int lanes = 1 << shift, rows_abreast = 32 >> shift;
+  const size_t c = (block * lanes + (lane & (lanes - 1))) * kW;
+  const size_t r0 = slice * rows_per_slice;
   const size_t r1 = r0 + rows_per_slice < nrow ? r0 + rows_per_slice : nrow;
-  float acc = 0.f;
-  if (c < ncol)
-    for (size_t r = r0 + w; r < r1; r += 8) acc += M[r * ncol + c];
-  sm[w][lane] = acc;
-  __syncthreads();
-  if (w == 0 && c < ncol) {
-    float s = 0.f;
+  const size_t step = static_cast<size_t>(kWarps) * rows_abreast;
+  float acc[kW];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s += sm[k][lane];
-    out[blockIdx.y * ncol + c] = s;
+  for (int k = 0; k < kW; ++k) acc[k] = 0.f;
+  if (c < ncol) {
+    const float* p = M + c;
+    size_t r = r0 + w * rows_abreast + (lane >> shift);
+    for (; r + 7 * step < r1; r += 8 * step) {
+      if (VEC) {
+        float4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = *reinterpret_cast<const float4*>(p + (r + k * step) * ncol);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          acc[0] += v[k].x;
+          acc[1 % kW] += v[k].y;
+          acc[2 % kW] += v[k].z;
+          acc[3 % kW] += v[k].w;
+        }
+      } else {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = p[(r + k * step) * ncol];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[0] += v[k];
+      }
+    }
+#pragma unroll 4
+    for (; r < r1; r += step) {
+      if (VEC) {
+        const float4 v = *reinterpret_cast<const float4*>(p + r * ncol);
+        acc[0] += v.x;
+        acc[1 % kW] += v.y;
+        acc[2 % kW] += v.z;
+        acc[3 % kW] += v.w;
+      } else {
+        acc[0] += p[r * ncol];
+      }
+    }
+  }
+  if (!VEC)
+    for (int o = lanes; o < 32; o <<= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+#pragma unroll
+  for (int k = 0; k < kW; ++k) sm[w][lane * kW + k] = acc[k];
+  cg::cluster_group cluster = cg::this_cluster();
+  if (clustered) cluster.barrier_arrive();             // completed before the first remote store below
+  __syncthreads();
+  float s[kW];
+#pragma unroll
+  for (int k = 0; k < kW; ++k) {
+    s[k] = 0.f;
+    if (w == 0)
+#pragma unroll
+      for (int q = 0; q < kWarps; ++q) s[k] += sm[q][lane * kW + k];
+  }
+  if (clustered) {
+    cluster.barrier_wait();
+    if (w == 0) {
+      float* first = cluster.map_shared_rank(&part[slice][0], 0);
+#pragma unroll
+      for (int k = 0; k < kW; ++k) first[lane * kW + k] = s[k];
+    }
+    cluster.sync();
+    if (slice != 0) return;
+    if (w == 0)
+#pragma unroll
+      for (int k = 0; k < kW; ++k) {
+        s[k] = 0.f;
+        for (int q = 0; q < slices; ++q) s[k] += part[q][lane * kW + k];
+      }
+  }
+  if (w == 0 && c < ncol && lane < lanes) {
+    float* o = out + (clustered ? 0 : slice * ncol) + c;
+#pragma unroll
+    for (int k = 0; k < kW; ++k) o[k] = s[k];
   }
 }
 
 __global__ void __launch_bounds__(kBlock)
 colsum_finish_kernel(const float* __restrict__ partial, float* __restrict__ v,
                      size_t ncol, int slices) {
+  dependency_wait();
+  release_dependents();
   const size_t c = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x;
   if (c >= ncol) return;
   float s = 0.f;
+#pragma unroll 8
   for (int k = 0; k < slices; ++k) s += partial[k * ncol + c];
   v[c] = s;
 }
 
-int colsum_slices(size_t nrow, size_t ncol) {
-  const size_t col_blocks = ceil_div(ncol, 32);
-  const size_t target = static_cast<size_t>(sm_count()) * 4;
-  size_t s = col_blocks >= target ? 1 : ceil_div(target, col_blocks);
-  const size_t max_by_rows = ceil_div(nrow, 64);  // at least 64 rows per slice
-  if (s > max_by_rows) s = max_by_rows;
-  if (s > 256) s = 256;
-  return static_cast<int>(s < 1 ? 1 : s);
+struct ColsumPlan {
+  int shift, slices;
+  bool vec, clustered;
+  size_t blocks;
+};
+ColsumPlan colsum_plan(size_t nrow, size_t ncol, bool can_vec) {
+  ColsumPlan p;
+  p.shift = 5;
+  while (p.shift > 0 && (static_cast<size_t>(1) << (p.shift - 1)) >= ncol) --p.shift;
+  // four columns per lane once that still leaves a column block for most SMs
+  p.vec = can_vec && ncol >= 4096;
+  p.blocks = ceil_div(ncol, (p.vec ? 4u : 1u) << p.shift);
+  const size_t rows_per_pass = static_cast<size_t>(kWarps) << (5 - p.shift);   // rows a CTA reads with one load per lane
+  const size_t useful = ceil_div(nrow, rows_per_pass);                           // more slices than this have no row
+  const size_t target = ceil_div(static_cast<size_t>(sm_count()) * 4, p.blocks);
+  size_t s = useful < target ? useful : target;
+  // A cluster covers up to 8 slices; beyond 64 loads per lane a second launch
+  // with more slices is the faster way.
+  p.clustered = s <= kMaxCluster || useful <= kMaxCluster * 64;
+  if (p.clustered) {
+    size_t c = 1;
+    while (c * 2 <= kMaxCluster && c < s) c *= 2;
+    s = c;
+  } else if (s > 256) {
+    s = 256;
+  }
+  p.slices = static_cast<int>(s < 1 ? 1 : s);
+  if (p.slices == 1) p.clustered = true;      // a single CTA per column block: nothing to exchange
+  return p;
 }
 
 // ------------------------------------------------------------------- row sums
 // v[r] = sum_c M[r][c]; one warp per row, lanes stride over the columns.
 __global__ void __launch_bounds__(kBlock)
 rowsum_kernel(const float* __restrict__ M, float* __restrict__ v, size_t nrow, size_t ncol) {
+  dependency_wait();
+  release_dependents();
   const int lane = threadIdx.x & 31;
   const size_t r = (blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x) >> 5;
   if (r >= nrow) return;
   const float* row = M + r * ncol;
   float acc = 0.f;
+#pragma unroll 4
   for (size_t c = lane; c < ncol; c += 32) acc += row[c];
   acc = warp_sum(acc);
   if (lane == 0) v[r] = acc;
@@ -74,61 +186,98 @@ rowsum_kernel(const float* __restrict__ M, float* __restrict__ v, size_t nrow, s
 
 __global__ void __launch_bounds__(kBlock)
 rowmax_kernel(const float* __restrict__ M, float* __restrict__ v, size_t nrow, size_t ncol) {
+  dependency_wait();
+  release_dependents();
   const int lane = threadIdx.x & 31;
   const size_t r = (blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x) >> 5;
   if (r >= nrow) return;
   const float* row = M + r * ncol;
   float m = row[0];  // seeded with the first element, as the CUDA reference does
+#pragma unroll 4
   for (size_t c = lane; c < ncol; c += 32) m = fmaxf(m, row[c]);
   m = warp_max(m);
   if (lane == 0) v[r] = m;
 }
 
 // ---------------------------------------------------- per-channel NCHW reduce
-// db[c] = sum over n and the HW plane of dy[n][c][:].  grid = (slices, C); a
-// CTA walks the flattened (n, i) index space of its channel slice.
+// db[c] = sum over n and the HW plane of dy[n][c][:].  A CTA walks its slice of
+// the channel's flattened (n, i) index space; with up to eight slices per
+// channel they form a cluster and the call is one launch (see above), else the
+// partials are added by chansum_finish_kernel.
+template <bool VEC>
 __global__ void __launch_bounds__(kBlock)
 chansum_kernel(const float* __restrict__ dy, float* __restrict__ out, int N, int C,
-               int HW, int per_slice, int vec) {
+               int HW, int per_slice, int slices, bool clustered) {
   __shared__ float sm[32];
-  const int c = blockIdx.y, slice = blockIdx.x;
+  __shared__ float part[kMaxCluster];
+  dependency_wait();
+  release_dependents();
+  const int c = static_cast<int>(blockIdx.x / slices), slice = static_cast<int>(blockIdx.x - c * slices);
+  constexpr int kW = VEC ? 4 : 1;
+  const int hwu = HW / kW, total = N * hwu;
+  const int i0 = min(slice * per_slice, total), i1 = min(i0 + per_slice, total);
   float acc = 0.f;
-  if (vec) {
-    const int hw4 = HW >> 2, total = N * hw4;
-    int i0 = slice * per_slice, i1 = min(i0 + per_slice, total);
-    for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
-      const int n = i / hw4, q = i - n * hw4;
-      const float4 v = *reinterpret_cast<const float4*>(
-          dy + (static_cast<size_t>(n) * C + c) * HW + 4 * q);
+  // (sample, position) of the unit is advanced without a division per step
+  int n = (i0 + static_cast<int>(threadIdx.x)) / hwu, q = (i0 + static_cast<int>(threadIdx.x)) - n * hwu;
+  const int dn = kBlock / hwu, dq = kBlock - dn * hwu;
+#pragma unroll 4
+  for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
+    const float* p = dy + (static_cast<size_t>(n) * C + c) * HW + static_cast<size_t>(q) * kW;
+    if (VEC) {
+      const float4 v = *reinterpret_cast<const float4*>(p);
       acc += (v.x + v.y) + (v.z + v.w);
+    } else {
+      acc += *p;
     }
-  } else {
-    const int total = N * HW;
-    int i0 = slice * per_slice, i1 = min(i0 + per_slice, total);
-    for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
-      const int n = i / HW, q = i - n * HW;
-      acc += dy[(static_cast<size_t>(n) * C + c) * HW + q];
+    n += dn;
+    q += dq;
+    if (q >= hwu) {
+      q -= hwu;
+      ++n;
     }
   }
+  cg::cluster_group cluster = cg::this_cluster();
+  if (clustered) cluster.barrier_arrive();
   acc = block_sum(acc, sm);
-  if (threadIdx.x == 0) out[static_cast<size_t>(c) * gridDim.x + slice] = acc;
+  if (!clustered) {
+    if (threadIdx.x == 0) out[static_cast<size_t>(c) * slices + slice] = acc;
+    return;
+  }
+  cluster.barrier_wait();
+  if (threadIdx.x == 0) *cluster.map_shared_rank(&part[slice], 0) = acc;
+  cluster.sync();
+  if (slice == 0 && threadIdx.x == 0) {
+    float s = 0.f;
+    for (int k = 0; k < slices; ++k) s += part[k];
+    out[c] = s;
+  }
 }
 
 __global__ void chansum_finish_kernel(const float* __restrict__ partial,
                                       float* __restrict__ db, int C, int slices) {
+  dependency_wait();
+  release_dependents();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   float s = 0.f;
+#pragma unroll 8
   for (int k = 0; k < slices; ++k) s += partial[static_cast<size_t>(c) * slices + k];
   db[c] = s;
 }
 
-int chan_slices(int N, int C, int HW) {
+int chan_slices(int N, int C, int HW, bool* clustered) {
   const long long per_channel = static_cast<long long>(N) * HW;
   long long s = ceil_div(static_cast<size_t>(sm_count()) * 8, static_cast<size_t>(C));
   const long long max_s = (per_channel + 4095) / 4096;  // >= 4096 elements per slice
   if (s > max_s) s = max_s;
   if (s > 64) s = 64;
+  // eight slices of one cluster, unless that leaves more than 64K elements to each
+  *clustered = s <= kMaxCluster || per_channel <= kMaxCluster * 65536LL;
+  if (*clustered) {
+    int c = 1;
+    while (c * 2 <= kMaxCluster && c < s) c *= 2;
+    s = c;
+  }
   return static_cast<int>(s < 1 ? 1 : s);
 }
 
@@ -136,7 +285,10 @@ int chan_slices(int N, int C, int HW) {
 __global__ void __launch_bounds__(kBlock)
 sumall_partial_kernel(const float* __restrict__ x, float* __restrict__ partial, size_t n) {
   __shared__ float sm[32];
+  dependency_wait();
+  release_dependents();
   float acc = 0.f;
+#pragma unroll 8
   for (size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * kBlock)
     acc += x[i];
@@ -146,6 +298,8 @@ sumall_partial_kernel(const float* __restrict__ x, float* __restrict__ partial, 
 __global__ void __launch_bounds__(kBlock)
 sumall_finish_kernel(const float* __restrict__ partial, float* __restrict__ out, int parts) {
   __shared__ float sm[32];
+  dependency_wait();
+  release_dependents();
   float acc = 0.f;
   for (int i = threadIdx.x; i < parts; i += kBlock) acc += partial[i];
   acc = block_sum(acc, sm);
@@ -167,8 +321,14 @@ extern "C" {
 
 size_t sgb_sum_rows_workspace_bytes(size_t nrow, size_t ncol) {
   if (nrow == 0 || ncol == 0) return 0;
-  int s = colsum_slices(nrow, ncol);
-  return s > 1 ? static_cast<size_t>(s) * ncol * sizeof(float) : 0;
+  // what either alignment may need
+  size_t need = 0;
+  for (const bool can_vec : {false, true}) {
+    const ColsumPlan p = colsum_plan(nrow, ncol, can_vec);
+    if (!p.clustered && static_cast<size_t>(p.slices) * ncol * sizeof(float) > need)
+      need = static_cast<size_t>(p.slices) * ncol * sizeof(float);
+  }
+  return need;
 }
 
 int sgb_sum_rows_f32(const float* M, float* v, size_t nrow, size_t ncol, void* ws,
@@ -178,20 +338,20 @@ int sgb_sum_rows_f32(const float* M, float* v, size_t nrow, size_t ncol, void* w
   cudaStream_t s = as_stream(stream);
   if (nrow == 0) return sgb_set_f32(0.f, v, ncol, stream);
   if (!M) return SGB_ERR_NULL;
-  const int slices = colsum_slices(nrow, ncol);
-  const dim3 grid(static_cast<unsigned>(ceil_div(ncol, 32)), slices);
-  if (grid.x > 0x7fffffffu) return SGB_ERR_SIZE;
-  if (slices == 1) {
-    colsum_kernel<<<grid, kBlock, 0, s>>>(M, v, nrow, ncol, nrow);
-  } else {
-    if (!ws || ws_bytes < static_cast<size_t>(slices) * ncol * sizeof(float))
-      return SGB_ERR_WORKSPACE;
-    float* partial = static_cast<float*>(ws);
-    colsum_kernel<<<grid, kBlock, 0, s>>>(M, partial, nrow, ncol, ceil_div(nrow, slices));
-    colsum_finish_kernel<<<static_cast<unsigned>(ceil_div(ncol, kBlock)), kBlock, 0, s>>>(
-        partial, v, ncol, slices);
+  const ColsumPlan p = colsum_plan(nrow, ncol, ncol % 4 == 0 && aligned16(M));
+  if (p.blocks * p.slices > 0x7fffffffu) return SGB_ERR_SIZE;
+  const dim3 grid(static_cast<unsigned>(p.blocks * p.slices));
+  float* out = v;
+  if (!p.clustered) {
+    if (!ws || ws_bytes < static_cast<size_t>(p.slices) * ncol * sizeof(float)) return SGB_ERR_WORKSPACE;
+    out = static_cast<float*>(ws);
   }
-  return launch_status();
+  const int st = launch_ex(p.vec ? colsum_kernel<true> : colsum_kernel<false>, grid, dim3(kBlock), 0, s,
+                           p.clustered && p.slices > 1 ? p.slices : 0, true, M, out, nrow, ncol,
+                           ceil_div(nrow, p.slices), p.slices, p.shift, p.clustered && p.slices > 1);
+  if (st != SGB_OK || p.clustered) return st;
+  return launch_ex(colsum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(ncol, kBlock))), dim3(kBlock), 0, s, 0,
+                   true, static_cast<const float*>(out), v, ncol, p.slices);
 }
 
 int sgb_sum_columns_f32(const float* M, float* v, size_t nrow, size_t ncol, void* stream) {
@@ -199,23 +359,22 @@ int sgb_sum_columns_f32(const float* M, float* v, size_t nrow, size_t ncol, void
   if (!v) return SGB_ERR_NULL;
   if (ncol == 0) return sgb_set_f32(0.f, v, nrow, stream);
   if (!M) return SGB_ERR_NULL;
-  rowsum_kernel<<<static_cast<unsigned>(ceil_div(nrow * 32, kBlock)), kBlock, 0, as_stream(stream)>>>(
-      M, v, nrow, ncol);
-  return launch_status();
+  return launch_ex(rowsum_kernel, dim3(static_cast<unsigned>(ceil_div(nrow * 32, kBlock))), dim3(kBlock), 0,
+                   as_stream(stream), 0, true, M, v, nrow, ncol);
 }
 
 int sgb_row_max_f32(const float* M, float* v, size_t nrow, size_t ncol, void* stream) {
   if (nrow == 0) return SGB_OK;
   if (!M || !v) return SGB_ERR_NULL;
   if (ncol == 0) return SGB_ERR_SIZE;
-  rowmax_kernel<<<static_cast<unsigned>(ceil_div(nrow * 32, kBlock)), kBlock, 0, as_stream(stream)>>>(
-      M, v, nrow, ncol);
-  return launch_status();
+  return launch_ex(rowmax_kernel, dim3(static_cast<unsigned>(ceil_div(nrow * 32, kBlock))), dim3(kBlock), 0,
+                   as_stream(stream), 0, true, M, v, nrow, ncol);
 }
 
 size_t sgb_conv_bias_backward_workspace_bytes(int N, int C, int HW) {
   if (N <= 0 || C <= 0 || HW <= 0) return 0;
-  return static_cast<size_t>(chan_slices(N, C, HW)) * C * sizeof(float);
+  bool clustered;
+  return static_cast<size_t>(chan_slices(N, C, HW, &clustered)) * C * sizeof(float);
 }
 
 int sgb_conv_bias_backward_f32(const float* dy, float* db, int N, int C, int HW, void* ws,
@@ -226,16 +385,21 @@ int sgb_conv_bias_backward_f32(const float* dy, float* db, int N, int C, int HW,
   if (N == 0 || HW == 0) return sgb_set_f32(0.f, db, C, stream);
   if (!dy) return SGB_ERR_NULL;
   if (static_cast<long long>(N) * HW > 0x7fffffffLL || C > 65535) return SGB_ERR_SIZE;
-  const int slices = chan_slices(N, C, HW);
+  bool clustered;
+  const int slices = chan_slices(N, C, HW, &clustered);
   if (!ws || ws_bytes < static_cast<size_t>(slices) * C * sizeof(float)) return SGB_ERR_WORKSPACE;
-  const int vec = (HW % 4 == 0) && aligned16(dy);
+  const bool vec = (HW % 4 == 0) && aligned16(dy);
   const int total = vec ? N * (HW / 4) : N * HW;
   const int per_slice = static_cast<int>(ceil_div(total, slices));
   cudaStream_t s = as_stream(stream);
-  float* partial = static_cast<float*>(ws);
-  chansum_kernel<<<dim3(slices, C), kBlock, 0, s>>>(dy, partial, N, C, HW, per_slice, vec);
-  chansum_finish_kernel<<<static_cast<unsigned>(ceil_div(C, 128)), 128, 0, s>>>(partial, db, C, slices);
-  return launch_status();
+  if (slices == 1) clustered = false;     // the CTA's sum is the result
+  float* out = clustered || slices == 1 ? db : static_cast<float*>(ws);
+  const int st = launch_ex(vec ? chansum_kernel<true> : chansum_kernel<false>,
+                           dim3(static_cast<unsigned>(slices) * C), dim3(kBlock), 0, s, clustered ? slices : 0, true,
+                           dy, out, N, C, HW, per_slice, slices, clustered);
+  if (st != SGB_OK || out == db) return st;
+  return launch_ex(chansum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(C, 128))), dim3(128), 0, s, 0, true,
+                   static_cast<const float*>(out), db, C, slices);
 }
 
 size_t sgb_sum_all_workspace_bytes(size_t n) {
@@ -253,12 +417,12 @@ int sgb_sum_all_f32(const float* x, float* out, size_t n, void* ws, size_t ws_by
   if (parts == 1) {
     // one CTA covers everything: its block sum IS the result (adding the zeros
     // of a second pass would not change a bit), so write it straight to `out`
-    sumall_partial_kernel<<<1, kBlock, 0, s>>>(x, out, n);
-    return launch_status();
+    return launch_ex(sumall_partial_kernel, dim3(1), dim3(kBlock), 0, s, 0, true, x, out, n);
   }
-  sumall_partial_kernel<<<parts, kBlock, 0, s>>>(x, partial, n);
-  sumall_finish_kernel<<<1, kBlock, 0, s>>>(partial, out, parts);
-  return launch_status();
+  const int st = launch_ex(sumall_partial_kernel, dim3(parts), dim3(kBlock), 0, s, 0, true, x, partial, n);
+  if (st != SGB_OK) return st;
+  return launch_ex(sumall_finish_kernel, dim3(1), dim3(kBlock), 0, s, 0, true, static_cast<const float*>(partial), out,
+                   parts);
 }
 
 }  // extern "C"

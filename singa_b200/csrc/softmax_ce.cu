@@ -1,8 +1,17 @@
 // Row softmax, per-sample cross entropy and the softmax-cross-entropy gradient.
-// The problems on this path are tiny (batch x classes = 32x1000 ... 256x10), so
-// the point of these kernels is to be ONE launch each and to fold the 1/batch
-// scaling into the gradient instead of a clone + edit + scale sequence.
+// The problems on this path are small (batch x classes = 32x1000 ... 256x10),
+// so the point of these kernels is to be ONE launch each with few serial steps,
+// and to fold the 1/batch scaling into the gradient instead of a clone + edit +
+// scale sequence.
+//
+// A row is read from memory once and stays in registers: its maximum, its sum
+// of exponentials and the result come from there (three passes over the row and
+// two evaluations of exp per element before: 4.0 us at 256 x 1000).  32 to 1024
+// threads work on a row, each with at most 32 elements; short rows share a CTA.
+// Rows beyond 32768 elements are re-read instead.
 #include <float.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -11,24 +20,226 @@ namespace {
 
 constexpr int kBlock = 128;
 
-// One CTA per row: max, sum of exp(x - max), normalise.  expf and the division
-// are the full-precision forms (the "accurate" softmax mode).
-__global__ void __launch_bounds__(kBlock)
-softmax_rows_kernel(const float* __restrict__ x, float* __restrict__ y, size_t ncol) {
-  __shared__ float sm[32];
-  const float* xr = x + blockIdx.x * ncol;
-  float* yr = y + blockIdx.x * ncol;
-  float m = xr[0];
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) m = fmaxf(m, xr[c]);
-  m = warp_max(m);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sm[w] = m;
+__device__ __forceinline__ float as_float(float v) { return v; }
+__device__ __forceinline__ float as_float(__half v) { return __half2float(v); }
+__device__ __forceinline__ void put(float* p, float v) { *p = v; }
+__device__ __forceinline__ void put(__half* p, float v) { *p = __float2half_rn(v); }
+
+// Sum / maximum over the T threads that share a row; T = 32: a warp, else a CTA.
+template <int T, bool MAX>
+__device__ __forceinline__ float row_reduce(float v, float* sm) {
+  v = MAX ? warp_max(v) : warp_sum(v);
+  if (T == 32) return v;
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
   __syncthreads();
-  m = fmaxf(fmaxf(sm[0], sm[1]), fmaxf(sm[2], sm[3]));
+  constexpr int kWarps = T / 32;
+  const int lane = threadIdx.x & 31;
+  v = lane < kWarps ? sm[lane] : (MAX ? -INFINITY : 0.0f);
+  return MAX ? warp_max(v) : warp_sum(v);
+}
+
+// One row in registers: NV vectors of kL elements per thread.
+template <typename V, int T, int NV>
+struct Row {
+  static constexpr int kL = 16 / sizeof(V);
+  float v[NV][kL];
+  float sum;
+
+  // element index of vector k of thread t
+  __device__ __forceinline__ static size_t at(int k, int t) { return (static_cast<size_t>(k) * T + t) * kL; }
+
+  // Loads the row and turns it into exp(x - max); `vec`: 16-byte accesses.
+  __device__ __forceinline__ void softmax(const V* __restrict__ x, size_t ncol, bool vec, int t, float* sm) {
+    float m = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const size_t i = at(k, t);
+      union {
+        uint4 u;
+        V e[kL];
+      } q;
+      if (vec && i + kL <= ncol) {
+        q.u = ld128(x + i);
+#pragma unroll
+        for (int j = 0; j < kL; ++j) v[k][j] = as_float(q.e[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kL; ++j) v[k][j] = i + j < ncol ? as_float(x[i + j]) : -INFINITY;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int j = 0; j < kL; ++j) m = fmaxf(m, v[k][j]);
+    m = row_reduce<T, true>(m, sm);
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int j = 0; j < kL; ++j) {
+        v[k][j] = at(k, t) + j < ncol ? expf(v[k][j] - m) : 0.0f;
+        s += v[k][j];
+      }
+    sum = row_reduce<T, false>(s, sm + 32);
+  }
+  __device__ __forceinline__ static void store(V* __restrict__ y, size_t ncol, bool vec, size_t i, const float (&e)[kL]) {
+    if (vec && i + kL <= ncol) {
+      union {
+        uint4 u;
+        V e[kL];
+      } q;
+#pragma unroll
+      for (int j = 0; j < kL; ++j) put(&q.e[j], e[j]);
+      st128(y + i, q.u);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kL; ++j)
+        if (i + j < ncol) put(y + i + j, e[j]);
+    }
+  }
+};
+
+// expf and the division are the full-precision forms (the "accurate" softmax
+// mode); fp16 rows are computed in fp32 with one rounding on store.
+template <typename V, int T, int NV>
+__global__ void __launch_bounds__(T == 32 ? 128 : T, T == 32 ? 8 : 1024 / T)
+softmax_rows_kernel(const V* __restrict__ x, V* __restrict__ y, size_t nrow, size_t ncol, bool vec) {
+  __shared__ float sm[64];
+  dependency_wait();
+  release_dependents();
+  const size_t row = T == 32 ? blockIdx.x * 4ull + (threadIdx.x >> 5) : blockIdx.x;
+  const int t = T == 32 ? threadIdx.x & 31 : threadIdx.x;
+  if (row >= nrow) return;
+  Row<V, T, NV> r;
+  r.softmax(x + row * ncol, ncol, vec, t, sm);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+#pragma unroll
+    for (int j = 0; j < Row<V, T, NV>::kL; ++j) r.v[k][j] = r.v[k][j] / r.sum;
+    r.store(y + row * ncol, ncol, vec, r.at(k, t), r.v[k]);
+  }
+}
+
+// The whole loss head for integer targets in one launch: row softmax, the
+// sample's loss -log(max(p[t], FLT_MIN)) and the scaled gradient
+// (p - onehot) * scale.  Every value is formed by the same fp32 operations as
+// in the separate kernels, so results are identical bit for bit.
+template <int T, int NV>
+__global__ void __launch_bounds__(T == 32 ? 128 : T, T == 32 ? 8 : 1024 / T)
+softmax_ce_fused_kernel(const float* __restrict__ x, const int* __restrict__ tgt, float* __restrict__ prob,
+                        float* __restrict__ loss, float* __restrict__ grad, size_t nrow, size_t ncol, float scale,
+                        bool vec) {
+  __shared__ float sm[64];
+  dependency_wait();
+  release_dependents();
+  const size_t row = T == 32 ? blockIdx.x * 4ull + (threadIdx.x >> 5) : blockIdx.x;
+  const int t = T == 32 ? threadIdx.x & 31 : threadIdx.x;
+  if (row >= nrow) return;
+  const size_t hot = static_cast<size_t>(tgt[row]);
+  if (hot >= ncol && t == 0) loss[row] = __int_as_float(0x7fc00000);   // label out of range: NaN, not stale memory
+  Row<float, T, NV> r;
+  r.softmax(x + row * ncol, ncol, vec, t, sm);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const size_t i = r.at(k, t);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) r.v[k][j] = r.v[k][j] / r.sum;
+    if (prob) r.store(prob + row * ncol, ncol, vec, i, r.v[k]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float g = r.v[k][j];
+      if (i + j == hot) {
+        loss[row] = -logf(fmaxf(g, FLT_MIN));
+        g = g - 1.0f;
+      }
+      r.v[k][j] = g * scale;
+    }
+    r.store(grad + row * ncol, ncol, vec, i, r.v[k]);
+  }
+}
+
+// Rows too long for registers: three passes over the row.
+template <typename V>
+__global__ void __launch_bounds__(1024)
+softmax_long_kernel(const V* __restrict__ x, V* __restrict__ y, size_t ncol) {
+  __shared__ float sm[64];
+  dependency_wait();
+  release_dependents();
+  const V* xr = x + blockIdx.x * ncol;
+  V* yr = y + blockIdx.x * ncol;
+  float m = -INFINITY;
+  for (size_t c = threadIdx.x; c < ncol; c += 1024) m = fmaxf(m, as_float(xr[c]));
+  m = row_reduce<1024, true>(m, sm);
   float s = 0.f;
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) s += expf(xr[c] - m);
-  s = block_sum(s, sm);
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) yr[c] = expf(xr[c] - m) / s;
+  for (size_t c = threadIdx.x; c < ncol; c += 1024) s += expf(as_float(xr[c]) - m);
+  s = row_reduce<1024, false>(s, sm + 32);
+  for (size_t c = threadIdx.x; c < ncol; c += 1024) put(yr + c, expf(as_float(xr[c]) - m) / s);
+}
+__global__ void __launch_bounds__(1024)
+softmax_ce_long_kernel(const float* __restrict__ x, const int* __restrict__ t, float* __restrict__ prob,
+                       float* __restrict__ loss, float* __restrict__ grad, size_t ncol, float scale) {
+  __shared__ float sm[64];
+  dependency_wait();
+  release_dependents();
+  const size_t row = blockIdx.x;
+  const float* xr = x + row * ncol;
+  float m = -INFINITY;
+  for (size_t c = threadIdx.x; c < ncol; c += 1024) m = fmaxf(m, xr[c]);
+  m = row_reduce<1024, true>(m, sm);
+  float s = 0.f;
+  for (size_t c = threadIdx.x; c < ncol; c += 1024) s += expf(xr[c] - m);
+  s = row_reduce<1024, false>(s, sm + 32);
+  const size_t hot = static_cast<size_t>(t[row]);
+  if (hot >= ncol && threadIdx.x == 0) loss[row] = __int_as_float(0x7fc00000);
+  for (size_t c = threadIdx.x; c < ncol; c += 1024) {
+    const float p = expf(xr[c] - m) / s;
+    if (prob) prob[row * ncol + c] = p;
+    float g = p;
+    if (c == hot) {
+      g = g - 1.0f;
+      loss[row] = -logf(fmaxf(p, FLT_MIN));
+    }
+    grad[row * ncol + c] = g * scale;
+  }
+}
+
+// Threads per row and vectors per thread by row length: a warp up to 512
+// elements (no barrier at all), then the smallest CTA whose threads hold the
+// row with four vectors each.  F is called with the two constants.
+template <typename V, typename F>
+int by_length(size_t ncol, F f) {
+  constexpr size_t kL = 16 / sizeof(V);
+  const size_t vecs = ceil_div(ncol, kL);
+#define SGB_ROW(T, NV)                                                            \
+  if (vecs <= static_cast<size_t>(T) * (NV)) return f(std::integral_constant<int, T>{}, std::integral_constant<int, NV>{});
+  SGB_ROW(32, 1)
+  SGB_ROW(32, 2)
+  SGB_ROW(32, 4)
+  SGB_ROW(128, 2)
+  SGB_ROW(128, 4)
+  SGB_ROW(256, 4)
+  SGB_ROW(512, 4)
+  SGB_ROW(1024, 4)
+  if constexpr (kL == 4) { SGB_ROW(1024, 8) }
+#undef SGB_ROW
+  return -1000;          // longer
+}
+
+template <typename V>
+int softmax_rows(const V* x, V* y, size_t nrow, size_t ncol, void* stream) {
+  if (nrow == 0 || ncol == 0) return SGB_OK;
+  if (!x || !y) return SGB_ERR_NULL;
+  if (nrow > 0x7fffffffu) return SGB_ERR_SIZE;
+  const bool vec = ncol % (16 / sizeof(V)) == 0 && aligned16(x) && aligned16(y);
+  const int st = by_length<V>(ncol, [&](auto T, auto NV) {
+    constexpr int kT = decltype(T)::value, kNV = decltype(NV)::value;
+    const unsigned grid = static_cast<unsigned>(kT == 32 ? ceil_div(nrow, 4) : nrow);
+    return launch_ex(softmax_rows_kernel<V, kT, kNV>, dim3(grid), dim3(kT == 32 ? 128 : kT), 0, as_stream(stream), 0,
+                     true, x, y, nrow, ncol, vec);
+  });
+  if (st != -1000) return st;
+  return launch_ex(softmax_long_kernel<V>, dim3(static_cast<unsigned>(nrow)), dim3(1024), 0, as_stream(stream), 0, true,
+                   x, y, ncol);
 }
 
 // loss[i] = -log(max(p[i, t[i]], FLT_MIN)) or the weighted form for array
@@ -36,6 +247,8 @@ softmax_rows_kernel(const float* __restrict__ x, float* __restrict__ y, size_t n
 __global__ void ce_fwd_kernel(int int_target, size_t batch, size_t dim,
                               const float* __restrict__ p, const int* __restrict__ t,
                               float* __restrict__ loss) {
+  dependency_wait();
+  release_dependents();
   size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= batch) return;
   if (int_target) {
@@ -57,102 +270,91 @@ __global__ void ce_fwd_kernel(int int_target, size_t batch, size_t dim,
   }
 }
 
-// grad = (p - target) * scale, one CTA per sample row.  With SCALE == false the
-// multiply is skipped, so the values equal the reference's in-place kernel bit
-// for bit; with SCALE the extra multiply is the same fp32 product the
-// reference forms in its separate "dx /= batch" pass.
+// grad = (p - onehot) * scale over the flattened matrix, one 16-byte vector
+// per thread; with SCALE == false the multiply is skipped, so the values equal
+// the reference's in-place kernel bit for bit, with SCALE the extra multiply is
+// the same fp32 product the reference forms in its separate "dx /= batch" pass.
+// VEC: rows are a whole number of vectors and the pointers are aligned.
+__device__ __forceinline__ float less_one(float v) { return v - 1.0f; }
+__device__ __forceinline__ __half less_one(__half v) { return __hsub(v, __int2half_rn(1)); }
+template <typename V, bool SCALE, bool VEC>
+__global__ void __launch_bounds__(256)
+ce_bwd_int_kernel(size_t dim, size_t total, const V* __restrict__ p, const int* __restrict__ t, V* __restrict__ grad,
+                  float scale) {
+  constexpr int kL = VEC ? 16 / sizeof(V) : 1;
+  dependency_wait();
+  release_dependents();
+  const size_t i = (blockIdx.x * 256ull + threadIdx.x) * kL;
+  if (i >= total) return;
+  const size_t row = total <= 0xffffffffu ? static_cast<unsigned>(i) / static_cast<unsigned>(dim) : i / dim;
+  const size_t hot = static_cast<size_t>(t[row]), c = i - row * dim;
+  union {
+    uint4 u;
+    V e[kL];
+  } q;
+  if (VEC) q.u = ld128(p + i);
+  else q.e[0] = p[i];
+#pragma unroll
+  for (int j = 0; j < kL; ++j) {
+    if (c + j == hot) q.e[j] = less_one(q.e[j]);
+    if (SCALE) q.e[j] = static_cast<V>(static_cast<float>(q.e[j]) * scale);   // fp32 only
+  }
+  if (VEC) st128(grad + i, q.u);
+  else grad[i] = q.e[0];
+}
+template <typename V, bool SCALE>
+int ce_bwd_int(size_t batch, size_t dim, const V* p, const int* t, V* grad, float scale, void* stream) {
+  constexpr size_t kL = 16 / sizeof(V);
+  const bool vec = dim % kL == 0 && aligned16(p) && aligned16(grad);
+  const size_t total = batch * dim, work = vec ? total / kL : total;
+  if (ceil_div(work, 256) > 0x7fffffffu) return SGB_ERR_SIZE;
+  return launch_ex(vec ? ce_bwd_int_kernel<V, SCALE, true> : ce_bwd_int_kernel<V, SCALE, false>,
+                   dim3(static_cast<unsigned>(ceil_div(work, 256))), dim3(256), 0, as_stream(stream), 0, true, dim, total,
+                   p, t, grad, scale);
+}
+
+// The same for array targets (weights normalised per row), one CTA per sample row.
 template <bool SCALE>
 __global__ void __launch_bounds__(kBlock)
-ce_bwd_kernel(int int_target, size_t dim, const float* __restrict__ p,
-              const int* __restrict__ t, float* __restrict__ grad, float scale) {
+ce_bwd_array_kernel(size_t dim, const float* __restrict__ p, const int* __restrict__ t, float* __restrict__ grad,
+                    float scale) {
   __shared__ float sm[32];
+  dependency_wait();
+  release_dependents();
   const size_t row = blockIdx.x;
   const float* pr = p + row * dim;
   float* gr = grad + row * dim;
-  if (int_target) {
-    const size_t hot = static_cast<size_t>(t[row]);
-    for (size_t j = threadIdx.x; j < dim; j += kBlock) {
-      float g = pr[j];
-      if (j == hot) g = g - 1.0f;
-      gr[j] = SCALE ? g * scale : g;
-    }
-  } else {
-    const int* tr = t + row * dim;
-    // the reference adds the integer weights serially in fp32; sums of small
-    // integers are exact in any order
-    float part = 0.f;
-    for (size_t j = threadIdx.x; j < dim; j += kBlock) part += tr[j];
-    const float sum = block_sum(part, sm);
-    for (size_t j = threadIdx.x; j < dim; j += kBlock) {
-      float g = pr[j] - tr[j] / sum;
-      gr[j] = SCALE ? g * scale : g;
-    }
+  const int* tr = t + row * dim;
+  // the reference adds the integer weights serially in fp32; sums of small
+  // integers are exact in any order
+  float part = 0.f;
+  for (size_t j = threadIdx.x; j < dim; j += kBlock) part += tr[j];
+  const float sum = block_sum(part, sm);
+  for (size_t j = threadIdx.x; j < dim; j += kBlock) {
+    float g = pr[j] - tr[j] / sum;
+    gr[j] = SCALE ? g * scale : g;
   }
 }
-
-// The whole loss head for integer targets in one launch, one CTA per sample:
-// row softmax, the sample's loss -log(max(p[t], FLT_MIN)) and the scaled
-// gradient (p - onehot) * scale.  Every value is formed by the same fp32
-// operations as in the three separate kernels above, so results are identical
-// bit for bit.
-__global__ void __launch_bounds__(kBlock)
-softmax_ce_fused_kernel(const float* __restrict__ x, const int* __restrict__ t,
-                        float* __restrict__ prob, float* __restrict__ loss,
-                        float* __restrict__ grad, size_t ncol, float scale) {
-  __shared__ float sm[32];
-  const size_t row = blockIdx.x;
-  const float* xr = x + row * ncol;
-  float m = xr[0];
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) m = fmaxf(m, xr[c]);
-  m = warp_max(m);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sm[w] = m;
-  __syncthreads();
-  m = fmaxf(fmaxf(sm[0], sm[1]), fmaxf(sm[2], sm[3]));
-  float s = 0.f;
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) s += expf(xr[c] - m);
-  s = block_sum(s, sm);
-  const size_t hot = static_cast<size_t>(t[row]);
-  if (hot >= ncol && threadIdx.x == 0) loss[row] = __int_as_float(0x7fc00000);   // label out of range: NaN, not stale memory
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) {
-    const float p = expf(xr[c] - m) / s;
-    if (prob) prob[row * ncol + c] = p;
-    float g = p;
-    if (c == hot) {
-      g = g - 1.0f;
-      loss[row] = -logf(fmaxf(p, FLT_MIN));
-    }
-    grad[row * ncol + c] = g * scale;
-  }
+template <bool SCALE>
+int ce_bwd(int int_target, size_t batch, size_t dim, const float* p, const int32_t* t, float scale, float* grad,
+           void* stream) {
+  if (batch == 0 || dim == 0) return SGB_OK;
+  if (!p || !t || !grad) return SGB_ERR_NULL;
+  if (batch > 0x7fffffffu) return SGB_ERR_SIZE;
+  if (int_target) return ce_bwd_int<float, SCALE>(batch, dim, p, t, grad, scale, stream);
+  return launch_ex(ce_bwd_array_kernel<SCALE>, dim3(static_cast<unsigned>(batch)), dim3(kBlock), 0, as_stream(stream), 0,
+                   true, dim, p, t, grad, scale);
 }
 
 // ------------------------------------------------------------------- fp16
-// Row softmax on fp16 data: fp32 arithmetic inside, one rounding on store.
-__global__ void __launch_bounds__(kBlock)
-softmax_rows_f16_kernel(const __half* __restrict__ x, __half* __restrict__ y, size_t ncol) {
-  __shared__ float sm[32];
-  const __half* xr = x + blockIdx.x * ncol;
-  __half* yr = y + blockIdx.x * ncol;
-  float m = __half2float(xr[0]);
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) m = fmaxf(m, __half2float(xr[c]));
-  m = warp_max(m);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) sm[w] = m;
-  __syncthreads();
-  m = fmaxf(fmaxf(sm[0], sm[1]), fmaxf(sm[2], sm[3]));
-  float s = 0.f;
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock) s += expf(__half2float(xr[c]) - m);
-  s = block_sum(s, sm);
-  for (size_t c = threadIdx.x; c < ncol; c += kBlock)
-    yr[c] = __float2half_rn(expf(__half2float(xr[c]) - m) / s);
-}
-
 // fp16 cross entropy with the arithmetic of the fp16 kernel it replaces: all
 // steps in half precision, probabilities floored at half(1e-7), integer
 // weights converted with round-down, the per-sample sums formed serially.
 __global__ void ce_fwd_f16_kernel(int int_target, size_t batch, size_t dim,
                                   const __half* __restrict__ p, const int* __restrict__ t,
                                   __half* __restrict__ loss) {
+  dependency_wait();
+  release_dependents();
   size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= batch) return;
   const __half eps = __float2half_rn(0.0000001f);
@@ -176,31 +378,26 @@ __global__ void ce_fwd_f16_kernel(int int_target, size_t batch, size_t dim,
   }
 }
 
-// grad = p - target in half precision; one CTA per sample row.  The integer
-// weights of an array target are small, so their half sum is exact in any
-// order as long as it stays below 2048.
+// grad = p - target in half precision for array targets; one CTA per sample
+// row.  The integer weights are small, so their half sum is exact in any order
+// as long as it stays below 2048.
 __global__ void __launch_bounds__(kBlock)
-ce_bwd_f16_kernel(int int_target, size_t dim, const __half* __restrict__ p,
-                  const int* __restrict__ t, __half* __restrict__ grad) {
+ce_bwd_array_f16_kernel(size_t dim, const __half* __restrict__ p, const int* __restrict__ t, __half* __restrict__ grad) {
   __shared__ __half total;
+  dependency_wait();
+  release_dependents();
   const size_t row = blockIdx.x;
   const __half* pr = p + row * dim;
   __half* gr = grad + row * dim;
-  if (int_target) {
-    const size_t hot = static_cast<size_t>(t[row]);
-    for (size_t j = threadIdx.x; j < dim; j += kBlock)
-      gr[j] = j == hot ? __hsub(pr[j], __int2half_rn(1)) : pr[j];
-  } else {
-    const int* tr = t + row * dim;
-    if (threadIdx.x == 0) {
-      __half sum = __float2half_rn(0.f);
-      for (size_t j = 0; j < dim; ++j) sum = __hadd(sum, __int2half_rd(tr[j]));
-      total = sum;
-    }
-    __syncthreads();
-    for (size_t j = threadIdx.x; j < dim; j += kBlock)
-      gr[j] = __hsub(pr[j], __hdiv(__int2half_rd(tr[j]), total));
+  const int* tr = t + row * dim;
+  if (threadIdx.x == 0) {
+    __half sum = __float2half_rn(0.f);
+    for (size_t j = 0; j < dim; ++j) sum = __hadd(sum, __int2half_rd(tr[j]));
+    total = sum;
   }
+  __syncthreads();
+  for (size_t j = threadIdx.x; j < dim; j += kBlock)
+    gr[j] = __hsub(pr[j], __hdiv(__int2half_rd(tr[j]), total));
 }
 
 }  // namespace
@@ -211,11 +408,7 @@ using namespace sgb;
 extern "C" {
 
 int sgb_softmax_rows_f32(const float* x, float* y, size_t nrow, size_t ncol, void* stream) {
-  if (nrow == 0 || ncol == 0) return SGB_OK;
-  if (!x || !y) return SGB_ERR_NULL;
-  if (nrow > 0x7fffffffu) return SGB_ERR_SIZE;
-  softmax_rows_kernel<<<static_cast<unsigned>(nrow), kBlock, 0, as_stream(stream)>>>(x, y, ncol);
-  return launch_status();
+  return softmax_rows<float>(x, y, nrow, ncol, stream);
 }
 
 int sgb_cross_entropy_f32(int int_target, size_t batch, size_t dim, const float* p,
@@ -223,29 +416,18 @@ int sgb_cross_entropy_f32(int int_target, size_t batch, size_t dim, const float*
   if (batch == 0) return SGB_OK;
   if (!p || !t || !loss) return SGB_ERR_NULL;
   if (dim == 0) return SGB_ERR_SIZE;
-  ce_fwd_kernel<<<static_cast<unsigned>(ceil_div(batch, 128)), 128, 0, as_stream(stream)>>>(
-      int_target, batch, dim, p, t, loss);
-  return launch_status();
+  return launch_ex(ce_fwd_kernel, dim3(static_cast<unsigned>(ceil_div(batch, 128))), dim3(128), 0, as_stream(stream), 0,
+                   true, int_target, batch, dim, p, t, loss);
 }
 
 int sgb_softmax_cross_entropy_bwd_f32(int int_target, size_t batch, size_t dim, const float* p,
                                       const int32_t* t, float* grad, void* stream) {
-  if (batch == 0 || dim == 0) return SGB_OK;
-  if (!p || !t || !grad) return SGB_ERR_NULL;
-  if (batch > 0x7fffffffu) return SGB_ERR_SIZE;
-  ce_bwd_kernel<false><<<static_cast<unsigned>(batch), kBlock, 0, as_stream(stream)>>>(
-      int_target, dim, p, t, grad, 1.0f);
-  return launch_status();
+  return ce_bwd<false>(int_target, batch, dim, p, t, 1.0f, grad, stream);
 }
 
 int sgb_softmax_cross_entropy_grad_f32(int int_target, size_t batch, size_t dim, const float* p,
                                        const int32_t* t, float scale, float* grad, void* stream) {
-  if (batch == 0 || dim == 0) return SGB_OK;
-  if (!p || !t || !grad) return SGB_ERR_NULL;
-  if (batch > 0x7fffffffu) return SGB_ERR_SIZE;
-  ce_bwd_kernel<true><<<static_cast<unsigned>(batch), kBlock, 0, as_stream(stream)>>>(
-      int_target, dim, p, t, grad, scale);
-  return launch_status();
+  return ce_bwd<true>(int_target, batch, dim, p, t, scale, grad, stream);
 }
 
 int sgb_softmax_cross_entropy_fused_f32(const float* logits, const int32_t* t, size_t batch, size_t dim,
@@ -254,18 +436,20 @@ int sgb_softmax_cross_entropy_fused_f32(const float* logits, const int32_t* t, s
   if (batch == 0 || dim == 0) return SGB_OK;
   if (!logits || !t || !loss || !grad) return SGB_ERR_NULL;
   if (batch > 0x7fffffffu) return SGB_ERR_SIZE;
-  softmax_ce_fused_kernel<<<static_cast<unsigned>(batch), kBlock, 0, as_stream(stream)>>>(
-      logits, t, prob, loss, grad, dim, scale);
-  return launch_status();
+  const bool vec = dim % 4 == 0 && aligned16(logits) && (!prob || aligned16(prob)) && aligned16(grad);
+  const int st = by_length<float>(dim, [&](auto T, auto NV) {
+    constexpr int kT = decltype(T)::value, kNV = decltype(NV)::value;
+    const unsigned grid = static_cast<unsigned>(kT == 32 ? ceil_div(batch, 4) : batch);
+    return launch_ex(softmax_ce_fused_kernel<kT, kNV>, dim3(grid), dim3(kT == 32 ? 128 : kT), 0, as_stream(stream), 0,
+                     true, logits, t, prob, loss, grad, batch, dim, scale, vec);
+  });
+  if (st != -1000) return st;
+  return launch_ex(softmax_ce_long_kernel, dim3(static_cast<unsigned>(batch)), dim3(1024), 0, as_stream(stream), 0, true,
+                   logits, t, prob, loss, grad, dim, scale);
 }
 
 int sgb_softmax_rows_f16(const void* x, void* y, size_t nrow, size_t ncol, void* stream) {
-  if (nrow == 0 || ncol == 0) return SGB_OK;
-  if (!x || !y) return SGB_ERR_NULL;
-  if (nrow > 0x7fffffffu) return SGB_ERR_SIZE;
-  softmax_rows_f16_kernel<<<static_cast<unsigned>(nrow), kBlock, 0, as_stream(stream)>>>(
-      static_cast<const __half*>(x), static_cast<__half*>(y), ncol);
-  return launch_status();
+  return softmax_rows<__half>(static_cast<const __half*>(x), static_cast<__half*>(y), nrow, ncol, stream);
 }
 
 int sgb_cross_entropy_f16(int int_target, size_t batch, size_t dim, const void* p, const int32_t* t,
@@ -273,9 +457,9 @@ int sgb_cross_entropy_f16(int int_target, size_t batch, size_t dim, const void* 
   if (batch == 0) return SGB_OK;
   if (!p || !t || !loss) return SGB_ERR_NULL;
   if (dim == 0) return SGB_ERR_SIZE;
-  ce_fwd_f16_kernel<<<static_cast<unsigned>(ceil_div(batch, 128)), 128, 0, as_stream(stream)>>>(
-      int_target, batch, dim, static_cast<const __half*>(p), t, static_cast<__half*>(loss));
-  return launch_status();
+  return launch_ex(ce_fwd_f16_kernel, dim3(static_cast<unsigned>(ceil_div(batch, 128))), dim3(128), 0,
+                   as_stream(stream), 0, true, int_target, batch, dim, static_cast<const __half*>(p), t,
+                   static_cast<__half*>(loss));
 }
 
 int sgb_softmax_cross_entropy_bwd_f16(int int_target, size_t batch, size_t dim, const void* p,
@@ -283,9 +467,11 @@ int sgb_softmax_cross_entropy_bwd_f16(int int_target, size_t batch, size_t dim, 
   if (batch == 0 || dim == 0) return SGB_OK;
   if (!p || !t || !grad) return SGB_ERR_NULL;
   if (batch > 0x7fffffffu) return SGB_ERR_SIZE;
-  ce_bwd_f16_kernel<<<static_cast<unsigned>(batch), kBlock, 0, as_stream(stream)>>>(
-      int_target, dim, static_cast<const __half*>(p), t, static_cast<__half*>(grad));
-  return launch_status();
+  if (int_target)
+    return ce_bwd_int<__half, false>(batch, dim, static_cast<const __half*>(p), t, static_cast<__half*>(grad), 1.0f,
+                                     stream);
+  return launch_ex(ce_bwd_array_f16_kernel, dim3(static_cast<unsigned>(batch)), dim3(kBlock), 0, as_stream(stream), 0,
+                   true, dim, static_cast<const __half*>(p), t, static_cast<__half*>(grad));
 }
 
 }  // extern "C"

@@ -952,6 +952,8 @@ __global__ void __launch_bounds__(kBlock)
 dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta) {
   __shared__ __align__(16) float out[kDenseTile];
   __shared__ unsigned cursor[kMaxDenseRanks], count[kMaxDenseRanks];
+  dependency_wait();
+  release_dependents();
   const size_t begin = a.first + static_cast<size_t>(blockIdx.x) * tiles_per_cta * kDenseTile;
   const size_t end = begin + static_cast<size_t>(tiles_per_cta) * kDenseTile < a.last
                          ? begin + static_cast<size_t>(tiles_per_cta) * kDenseTile : a.last;
@@ -1123,7 +1125,9 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
     a.off[a.targets] = at;
     const size_t tiles = ceil_div(a.last - a.first, kDenseTile);
     const unsigned per = static_cast<unsigned>(ceil_div(tiles, static_cast<size_t>(sm_count()) * 8));
-    dense_from_payloads_kernel<<<static_cast<unsigned>(ceil_div(tiles, per)), kBlock, 0, s>>>(a, per);
+    const int st = launch_ex(dense_from_payloads_kernel, dim3(static_cast<unsigned>(ceil_div(tiles, per))),
+                             dim3(kBlock), 0, s, 0, true, a, per);
+    if (st != SGB_OK) return st;
   }
   return launch_status();
 }
