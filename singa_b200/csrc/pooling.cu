@@ -41,6 +41,8 @@ __device__ __forceinline__ void covering(int h, int pad, int k, int stride, int 
 template <bool MAX>
 __global__ void __launch_bounds__(kBlock)
 pool_fwd_kernel(const float* __restrict__ x, float* __restrict__ y, PoolShape p, size_t total) {
+  dependency_wait();
+  release_dependents();
   const size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x;
   if (i >= total) return;
   const int ow = static_cast<int>(i % p.OW);
@@ -90,6 +92,8 @@ maxpool_bwd_band_kernel(const float* __restrict__ x, const float* __restrict__ d
   extern __shared__ float smem[];
   float* xs = smem;                                            // max_xrows * W
   int* winner = reinterpret_cast<int*>(smem + bp.max_xrows * p.W);  // max_orows * OW
+  dependency_wait();
+  release_dependents();
   const size_t plane = blockIdx.x;
   const int h_lo = blockIdx.y * bp.rows, h_hi = min(h_lo + bp.rows, p.H);  // dx rows [h_lo, h_hi)
   int o_lo, o_hi, unused;
@@ -162,6 +166,8 @@ maxpool_bwd_band_fast_kernel(const float* __restrict__ x, const float* __restric
   float* xs = smem;
   int* winner = reinterpret_cast<int*>(xs + bp.max_xrows * p.W);
   float* gs = reinterpret_cast<float*>(winner + bp.max_orows * p.OW);
+  dependency_wait();
+  release_dependents();
   const size_t plane = blockIdx.x;
   const int H = p.H, W = p.W, OH = p.OH, OW = p.OW;
   const int h_lo = blockIdx.y * bp.rows, h_hi = min(h_lo + bp.rows, H);
@@ -238,108 +244,6 @@ maxpool_bwd_band_fast_kernel(const float* __restrict__ x, const float* __restric
   }
 }
 
-// 3x3 window, stride 2, padding 1 on even H and W % 4 == 0 (the ResNet stem):
-// the general scheme above with everything that can be decided at compile time
-// decided.  The staged x band carries a -FLT_MAX column on the left and, at the
-// top of the plane, a -FLT_MAX row, so the nine reads of a window need no
-// bounds tests; every thread then produces a 2 x 4 patch of dx from six parked
-// winners (two window rows x three window columns), whose raster-order sums
-// are written out explicitly.  ~30 instructions per dx element.
-struct StemPlan {
-  int rows;     // dx rows per band (even)
-  int bands;
-};
-
-// WC: plane width known at compile time (0 = use the run-time value); with a
-// constant width the row / column splits below compile to multiply-shift
-// sequences instead of integer divisions, a quarter of the kernel's instructions.
-template <int WC>
-__global__ void __launch_bounds__(kBlock)
-maxpool_bwd_k3s2p1_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                          float* __restrict__ dx, int H, int W_rt, int OH, int OW_rt, int rows) {
-  extern __shared__ float smem[];
-  const int W = WC ? WC : W_rt;
-  const int OW = WC ? WC / 2 : OW_rt;
-  const int pitch = W + 4;                       // xs[r][4 + c] = x[xr0 + r][c], xs[r][3] = -FLT_MAX
-  const int wp = OW + 1;                         // winner / dy pitch (one never-matching pad column)
-  const int h_lo = blockIdx.y * rows, h_hi = min(h_lo + rows, H);
-  const int o_lo = h_lo >> 1, o_hi = min(h_hi >> 1, OH - 1);     // window rows [o_lo, o_hi]
-  const int norow = o_hi - o_lo + 1;
-  const int xr0 = 2 * o_lo - 1;                                 // may be -1
-  const int xr1 = min(2 * o_hi + 2, H);                         // x rows [xr0, xr1)
-  const int nxr = xr1 - xr0;
-  float* xs = smem;
-  int* winner = reinterpret_cast<int*>(xs + (rows + 3) * pitch);
-  float* gs = reinterpret_cast<float*>(winner + ((rows >> 1) + 2) * wp);
-  const size_t plane = blockIdx.x;
-  const float* xp = x + plane * H * W;
-  const float* gp = dy + plane * OH * OW;
-  float* dp = dx + plane * H * W;
-
-  const int w4 = W >> 2;
-  for (int v = threadIdx.x; v < nxr * w4; v += kBlock) {
-    const int r = v / w4, c4 = v - r * w4, xr = xr0 + r;
-    float4 val = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX);
-    if (xr >= 0) val = *reinterpret_cast<const float4*>(xp + xr * W + 4 * c4);
-    *reinterpret_cast<float4*>(xs + r * pitch + 4 + 4 * c4) = val;
-  }
-  for (int r = threadIdx.x; r < nxr; r += kBlock) xs[r * pitch + 3] = -FLT_MAX;
-  // dy rows of the band's windows, plus a pad row / column of winners that match nothing
-  for (int o = threadIdx.x; o < (norow + 1) * wp; o += kBlock) {
-    const int r = o / wp, c = o - r * wp;
-    const bool real = r < norow && c < OW;
-    gs[o] = real ? gp[(o_lo + r) * OW + c] : 0.0f;
-    if (!real) winner[o] = -2;
-  }
-  __syncthreads();
-  for (int o = threadIdx.x; o < norow * OW; o += kBlock) {
-    const int r = o / OW, ow = o - r * OW;
-    const float* win = xs + (2 * r) * pitch + 2 * ow + 3;        // top-left cell of the window
-    const int g0 = (2 * (o_lo + r) - 1) * W + 2 * ow - 1;        // its flat plane index
-    float best = -FLT_MAX;
-    int bi = -1;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const float v = win[i * pitch + j];
-        if (v > best || (v != v && best == best)) {   // first maximum; a NaN wins and then sticks, as in cuDNN
-          best = v;
-          bi = g0 + i * W + j;
-        }
-      }
-    winner[r * wp + ow] = bi;
-  }
-  __syncthreads();
-  const int npatch = ((h_hi - h_lo) >> 1) * w4;
-  for (int t = threadIdx.x; t < npatch; t += kBlock) {
-    const int m = t / w4, q = t - m * w4;
-    const int* w0 = winner + m * wp + 2 * q;       // windows (m, 2q .. 2q+2)
-    const int* w1 = w0 + wp;                        // windows (m+1, ...)
-    const float* g0 = gs + m * wp + 2 * q;
-    const float* g1 = g0 + wp;
-    const int a0 = w0[0], a1 = w0[1], a2 = w0[2], b0 = w1[0], b1 = w1[1], b2 = w1[2];
-    const float ga0 = g0[0], ga1 = g0[1], ga2 = g0[2], gb0 = g1[0], gb1 = g1[1], gb2 = g1[2];
-    const int h = h_lo + 2 * m;
-    const int i0 = h * W + 4 * q, i1 = i0 + W;      // flat indices of the patch's two rows
-#define PICK(wv, gv, idx) ((wv) == (idx) ? (gv) : 0.0f)
-    float4 top, bot;
-    top.x = 0.0f + PICK(a0, ga0, i0);
-    top.y = (0.0f + PICK(a0, ga0, i0 + 1)) + PICK(a1, ga1, i0 + 1);
-    top.z = 0.0f + PICK(a1, ga1, i0 + 2);
-    top.w = (0.0f + PICK(a1, ga1, i0 + 3)) + PICK(a2, ga2, i0 + 3);
-    bot.x = (0.0f + PICK(a0, ga0, i1)) + PICK(b0, gb0, i1);
-    bot.y = (((0.0f + PICK(a0, ga0, i1 + 1)) + PICK(a1, ga1, i1 + 1)) + PICK(b0, gb0, i1 + 1)) +
-            PICK(b1, gb1, i1 + 1);
-    bot.z = (0.0f + PICK(a1, ga1, i1 + 2)) + PICK(b1, gb1, i1 + 2);
-    bot.w = (((0.0f + PICK(a1, ga1, i1 + 3)) + PICK(a2, ga2, i1 + 3)) + PICK(b1, gb1, i1 + 3)) +
-            PICK(b2, gb2, i1 + 3);
-#undef PICK
-    *reinterpret_cast<float4*>(dp + i0) = top;
-    *reinterpret_cast<float4*>(dp + i1) = bot;
-  }
-}
-
 // ------------------------------------------------ arg-max forward partner
 // Max-pool forward that also records, per window, WHERE its (first, in raster
 // order) maximum sits: one byte, row offset in the high nibble and column
@@ -349,6 +253,8 @@ maxpool_bwd_k3s2p1_kernel(const float* __restrict__ x, const float* __restrict__
 __global__ void __launch_bounds__(kBlock)
 maxpool_fwd_argmax_kernel(const float* __restrict__ x, float* __restrict__ y,
                           unsigned char* __restrict__ arg, PoolShape p, size_t total) {
+  dependency_wait();
+  release_dependents();
   const size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x;
   if (i >= total) return;
   const int ow = static_cast<int>(i % p.OW);
@@ -378,6 +284,8 @@ maxpool_fwd_argmax_kernel(const float* __restrict__ x, float* __restrict__ y,
 __global__ void __launch_bounds__(kBlock)
 maxpool_bwd_argmax_kernel(const float* __restrict__ dy, const unsigned char* __restrict__ arg,
                           float* __restrict__ dx, PoolShape p, size_t total) {
+  dependency_wait();
+  release_dependents();
   const size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x;
   if (i >= total) return;
   const int w = static_cast<int>(i % p.W);
@@ -398,69 +306,697 @@ maxpool_bwd_argmax_kernel(const float* __restrict__ dy, const unsigned char* __r
   dx[i] = acc;
 }
 
-// Backward from the record for 3x3 / stride 2 / pad 1 (ResNet stem): the same
-// band / 2x4-patch scheme as maxpool_bwd_k3s2p1_kernel without its x staging
-// and winner search - the parked winners come straight from the record.
-template <int WC>
-__global__ void __launch_bounds__(kBlock)
-maxpool_bwd_argmax_k3s2p1_kernel(const float* __restrict__ dy, const unsigned char* __restrict__ arg,
-                                 float* __restrict__ dx, int H, int W_rt, int OH, int OW_rt, int rows) {
-  extern __shared__ float smem[];
-  const int W = WC ? WC : W_rt;
-  const int OW = WC ? WC / 2 : OW_rt;
-  const int wp = OW + 1;                         // winner / dy pitch (one never-matching pad column)
-  const int h_lo = blockIdx.y * rows, h_hi = min(h_lo + rows, H);
-  const int o_lo = h_lo >> 1, o_hi = min(h_hi >> 1, OH - 1);     // window rows [o_lo, o_hi]
-  const int norow = o_hi - o_lo + 1;
-  int* winner = reinterpret_cast<int*>(smem);
-  float* gs = reinterpret_cast<float*>(winner + ((rows >> 1) + 2) * wp);
-  const size_t plane = blockIdx.x;
-  const float* gp = dy + plane * OH * OW;
-  const unsigned char* ap = arg + plane * OH * OW;
-  float* dp = dx + plane * H * W;
-  for (int o = threadIdx.x; o < (norow + 1) * wp; o += kBlock) {
-    const int r = o / wp, c = o - r * wp;
-    const bool real = r < norow && c < OW;
-    float g = 0.0f;
-    int win = -2;
-    if (real) {
-      const int oh = o_lo + r;
-      g = gp[oh * OW + c];
-      const int code = ap[oh * OW + c];
-      if (code != 0xff) win = (2 * oh - 1 + (code >> 4)) * W + 2 * c - 1 + (code & 15);
+// ------------------------------------------------ 3x3 / stride 2 / pad 1, all passes
+// The ResNet stem's geometry, any plane size.  A lane owns four adjacent input
+// columns, which are the two windows 2q and 2q + 1 (columns 4q-1 .. 4q+3); a
+// warp walks down the rows of one or more planes.  Everything is in registers:
+// the row above is kept from the step before, the column to the left comes
+// from the neighbour lane, and the first window of the lane to the right is
+// fetched with a shuffle where a gradient needs it.  No shared memory and no
+// barrier; the next two rows are in flight while the current ones are worked
+// on.  (The form with staged rows spent its time on shared-memory traffic and
+// index arithmetic: 67 us forward, 59 us backward at 32x64x112x112, where the
+// bytes take 20 and 35 us.)  Planes wider than 128 columns are cut into
+// segments of 30 lanes with one halo lane on each side.
+enum StripMode { kMaxFwd = 0, kMaxFwdRecord = 1, kMaxBwd = 2, kMaxBwdRecord = 3, kAvgFwd = 4, kAvgBwd = 5 };
+
+struct StripArgs {
+  const float* x;          // input planes (kMaxFwd*, kMaxBwd, kAvgFwd)
+  const float* dy;         // output gradient (backward modes)
+  float* out;              // y or dx
+  unsigned char* record;   // written by kMaxFwdRecord, read by kMaxBwdRecord
+  int planes, H, W, OH, OW;
+  int quads;               // lanes a row needs: ceil(W / 4)
+  int abreast;             // planes side by side in a warp
+  int segments;            // warps a row needs
+  int rows;                // window rows per band
+  int bands;
+};
+
+constexpr int kNoCell = -1;
+
+// Index 0..8 (raster order) of the window's first maximum; kNoCell if no cell
+// exceeds -FLT_MAX.  NANS: a NaN wins and then sticks, as in cuDNN.
+template <bool NANS>
+__device__ __forceinline__ int first_max(const float (&v)[9], float& best) {
+  best = -FLT_MAX;
+  int at = kNoCell;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const bool p = NANS ? v[k] > best || (v[k] != v[k] && best == best) : v[k] > best;
+    best = p ? v[k] : best;
+    at = p ? k : at;
+  }
+  return at;
+}
+
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(kBlock, 4)
+pool_k3s2p1_kernel(const StripArgs a) {
+  constexpr bool kBackward = MODE == kMaxBwd || MODE == kMaxBwdRecord || MODE == kAvgBwd;
+  constexpr bool kNeedsX = MODE != kMaxBwdRecord && MODE != kAvgBwd;
+  constexpr bool kMax = MODE <= kMaxBwdRecord;
+  constexpr unsigned kAll = 0xffffffffu;
+  dependency_wait();
+  release_dependents();
+  const int lane = threadIdx.x & 31;
+  const unsigned task = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+  const unsigned rest = task / a.bands;
+  const int band = static_cast<int>(task - rest * a.bands);
+  const int group = static_cast<int>(rest / a.segments), seg = static_cast<int>(rest - group * a.segments);
+  int q, plane;
+  bool active, owner;
+  if (a.segments > 1) {
+    q = seg * 30 - 1 + lane;
+    plane = group;
+    active = q >= 0 && q < a.quads && plane < a.planes;
+    owner = active && lane >= 1 && lane <= 30;
+  } else {
+    const int pl = lane / a.quads;
+    q = lane - pl * a.quads;
+    plane = group * a.abreast + pl;
+    active = pl < a.abreast && plane < a.planes;
+    owner = active;
+  }
+  if (!active) plane = 0;
+  const int H = a.H, W = a.W, OH = a.OH, OW = a.OW, c = 4 * q;
+  const float* xp = a.x + static_cast<size_t>(plane) * H * W + c;
+  const size_t window0 = static_cast<size_t>(plane) * OH * OW + 2 * q;   // window (row 0, column 2q)
+  float* dxp = a.out + static_cast<size_t>(plane) * H * W + c;
+  const bool has_left = q > 0, has_right = q + 1 < a.quads;
+  const bool w1_exists = 2 * q + 1 < OW;
+  const float kPad = kMax ? -FLT_MAX : 0.0f;
+
+  auto load_row = [&](int h, float (&v)[4]) {
+    const bool in = active && h >= 0 && h < H;
+    if (VEC) {
+      float4 t = make_float4(kPad, kPad, kPad, kPad);
+      if (in) t = *reinterpret_cast<const float4*>(xp + static_cast<size_t>(h) * W);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = in && c + j < W ? xp[static_cast<size_t>(h) * W + j] : kPad;
     }
-    gs[o] = g;
-    winner[o] = win;
+  };
+  auto load_windows = [&](int m, float (&g)[2], unsigned (&code)[2]) {
+    const size_t i = window0 + static_cast<size_t>(m) * OW;
+    if (VEC) {                                       // W % 4 == 0: both windows exist, i is even
+      if (kBackward) {
+        const float2 t = active ? *reinterpret_cast<const float2*>(a.dy + i) : make_float2(0.f, 0.f);
+        g[0] = t.x;
+        g[1] = t.y;
+      }
+      if (MODE == kMaxBwdRecord) {
+        const unsigned t = active ? *reinterpret_cast<const unsigned short*>(a.record + i) : 0xffffu;
+        code[0] = t & 0xffu;
+        code[1] = t >> 8;
+      }
+      return;
+    }
+    if (kBackward) {
+      g[0] = active ? a.dy[i] : 0.0f;
+      g[1] = active && w1_exists ? a.dy[i + 1] : 0.0f;
+    }
+    if (MODE == kMaxBwdRecord) {
+      code[0] = active ? a.record[i] : 0xffu;
+      code[1] = active && w1_exists ? a.record[i + 1] : 0xffu;
+    }
+  };
+  auto store_row = [&](int h, const float (&v)[4]) {
+    if (!owner || h >= H) return;
+    float* p = dxp + static_cast<size_t>(h) * W;
+    if (VEC) {
+      *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < W) p[j] = v[j];
+    }
+  };
+
+  const int m0 = band * a.rows, m1 = min(m0 + a.rows, OH);
+  // backward: the odd row above window row m1 also takes from it
+  const int last = kBackward ? min(m1, OH - 1) : m1 - 1;
+  float above[4], above_left = kPad, r0[4], r1[4], n0[4], n1[4], g[2] = {0.f, 0.f}, ng[2] = {0.f, 0.f};
+  unsigned code[2] = {0, 0}, ncode[2] = {0, 0};
+  bool odd_above = false;          // something in the row above that only the NaN-aware comparison may decide
+  auto unordered = [](const float (&v)[4]) {
+    const float s = (v[0] + v[1]) + (v[2] + v[3]);   // NaN, or inf - inf: rare enough
+    return s != s;
+  };
+  if (kNeedsX) {
+    load_row(2 * m0 - 1, above);
+    load_row(2 * m0, n0);
+    load_row(2 * m0 + 1, n1);
+    above_left = __shfl_up_sync(kAll, above[3], 1);
+    if (!has_left) above_left = kPad;
+    if (kMax) odd_above = __any_sync(kAll, unordered(above));
   }
-  __syncthreads();
-  const int w4 = W >> 2;
-  const int npatch = ((h_hi - h_lo) >> 1) * w4;
-  for (int t = threadIdx.x; t < npatch; t += kBlock) {
-    const int m = t / w4, q = t - m * w4;
-    const int* w0 = winner + m * wp + 2 * q;       // windows (m, 2q .. 2q+2)
-    const int* w1 = w0 + wp;                        // windows (m+1, ...)
-    const float* g0 = gs + m * wp + 2 * q;
-    const float* g1 = g0 + wp;
-    const int a0 = w0[0], a1 = w0[1], a2 = w0[2], b0 = w1[0], b1 = w1[1], b2 = w1[2];
-    const float ga0 = g0[0], ga1 = g0[1], ga2 = g0[2], gb0 = g1[0], gb1 = g1[1], gb2 = g1[2];
-    const int h = h_lo + 2 * m;
-    const int i0 = h * W + 4 * q, i1 = i0 + W;      // flat indices of the patch's two rows
-#define PICK(wv, gv, idx) ((wv) == (idx) ? (gv) : 0.0f)
-    float4 top, bot;
-    top.x = 0.0f + PICK(a0, ga0, i0);
-    top.y = (0.0f + PICK(a0, ga0, i0 + 1)) + PICK(a1, ga1, i0 + 1);
-    top.z = 0.0f + PICK(a1, ga1, i0 + 2);
-    top.w = (0.0f + PICK(a1, ga1, i0 + 3)) + PICK(a2, ga2, i0 + 3);
-    bot.x = (0.0f + PICK(a0, ga0, i1)) + PICK(b0, gb0, i1);
-    bot.y = (((0.0f + PICK(a0, ga0, i1 + 1)) + PICK(a1, ga1, i1 + 1)) + PICK(b0, gb0, i1 + 1)) +
-            PICK(b1, gb1, i1 + 1);
-    bot.z = (0.0f + PICK(a1, ga1, i1 + 2)) + PICK(b1, gb1, i1 + 2);
-    bot.w = (((0.0f + PICK(a1, ga1, i1 + 3)) + PICK(a2, ga2, i1 + 3)) + PICK(b1, gb1, i1 + 3)) +
-            PICK(b2, gb2, i1 + 3);
-#undef PICK
-    *reinterpret_cast<float4*>(dp + i0) = top;
-    *reinterpret_cast<float4*>(dp + i1) = bot;
+  load_windows(m0, ng, ncode);
+  float pend[4] = {0.f, 0.f, 0.f, 0.f};   // gradient of row 2m - 1 so far
+  for (int m = m0; m <= last; ++m) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      r0[j] = n0[j];
+      r1[j] = n1[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      g[j] = ng[j];
+      code[j] = ncode[j];
+    }
+    if (m < last) {
+      if (kNeedsX) {
+        load_row(2 * m + 2, n0);
+        load_row(2 * m + 3, n1);
+      }
+      load_windows(m + 1, ng, ncode);
+    }
+    int at0 = kNoCell, at1 = kNoCell;
+    float best0 = 0.f, best1 = 0.f;
+    if (kNeedsX) {
+      float l0 = __shfl_up_sync(kAll, r0[3], 1), l1 = __shfl_up_sync(kAll, r1[3], 1);
+      if (!has_left) l0 = l1 = kPad;
+      const float w0[9] = {above_left, above[0], above[1], l0, r0[0], r0[1], l1, r1[0], r1[1]};
+      const float w1[9] = {above[1], above[2], above[3], r0[1], r0[2], r0[3], r1[1], r1[2], r1[3]};
+      if (kMax) {
+        const bool odd0 = __any_sync(kAll, unordered(r0)), odd1 = __any_sync(kAll, unordered(r1));
+        if (odd_above || odd0 || odd1) {
+          at0 = first_max<true>(w0, best0);
+          at1 = first_max<true>(w1, best1);
+        } else {
+          at0 = first_max<false>(w0, best0);
+          at1 = first_max<false>(w1, best1);
+        }
+        odd_above = odd1;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+          best0 += w0[k];
+          best1 += w1[k];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) above[j] = r1[j];
+      above_left = l1;
+    }
+    if (MODE == kMaxBwdRecord) {
+      at0 = code[0] == 0xffu ? kNoCell : static_cast<int>(code[0] >> 4) * 3 + static_cast<int>(code[0] & 15u);
+      at1 = code[1] == 0xffu ? kNoCell : static_cast<int>(code[1] >> 4) * 3 + static_cast<int>(code[1] & 15u);
+    }
+    if (!kMax) {
+      // cells inside the plane: the divisor excludes the padding
+      const int rows_in = 3 - (m == 0) - (2 * m + 1 >= H);
+      const float n_0 = static_cast<float>(rows_in * (3 - (c == 0) - (c + 1 >= W)));
+      const float n_1 = static_cast<float>(rows_in * (3 - (c + 3 >= W)));
+      if (kBackward) {
+        g[0] = g[0] / n_0;
+        g[1] = w1_exists ? g[1] / n_1 : 0.0f;
+      } else {
+        best0 = best0 / n_0;
+        best1 = best1 / n_1;
+      }
+    }
+    if (!kBackward) {
+      if (owner) {
+        const size_t i = window0 + static_cast<size_t>(m) * OW;
+        if (VEC) {
+          *reinterpret_cast<float2*>(a.out + i) = make_float2(best0, best1);
+        } else {
+          a.out[i] = best0;
+          if (w1_exists) a.out[i + 1] = best1;
+        }
+        if (MODE == kMaxFwdRecord) {
+          const unsigned c0 = at0 < 0 ? 0xffu : static_cast<unsigned>((at0 / 3) << 4 | at0 % 3);
+          const unsigned c1 = at1 < 0 ? 0xffu : static_cast<unsigned>((at1 / 3) << 4 | at1 % 3);
+          if (VEC) {
+            *reinterpret_cast<unsigned short*>(a.record + i) = static_cast<unsigned short>(c0 | c1 << 8);
+          } else {
+            a.record[i] = static_cast<unsigned char>(c0);
+            if (w1_exists) a.record[i + 1] = static_cast<unsigned char>(c1);
+          }
+        }
+      }
+    } else {
+      if (!w1_exists) at1 = kNoCell;
+      int at2 = __shfl_down_sync(kAll, at0, 1);
+      float g2 = __shfl_down_sync(kAll, g[0], 1);
+      if (!has_right) {
+        at2 = kNoCell;
+        g2 = 0.0f;
+      }
+      // gradient of the four columns in window row DR of the three, windows in raster order
+      auto row_of = [&](int dr, float (&v)[4]) {
+        if (kMax) {
+          v[0] = v[0] + (at0 == 3 * dr + 1 ? g[0] : 0.0f);
+          v[1] = (v[1] + (at0 == 3 * dr + 2 ? g[0] : 0.0f)) + (at1 == 3 * dr ? g[1] : 0.0f);
+          v[2] = v[2] + (at1 == 3 * dr + 1 ? g[1] : 0.0f);
+          v[3] = (v[3] + (at1 == 3 * dr + 2 ? g[1] : 0.0f)) + (at2 == 3 * dr ? g2 : 0.0f);
+        } else {
+          v[0] = v[0] + g[0];
+          v[1] = (v[1] + g[0]) + g[1];
+          v[2] = v[2] + g[1];
+          v[3] = (v[3] + g[1]) + g2;
+        }
+      };
+      if (m > m0) {
+        row_of(0, pend);
+        store_row(2 * m - 1, pend);
+      }
+      if (m < m1) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        row_of(1, v);
+        store_row(2 * m, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pend[j] = 0.f;
+        row_of(2, pend);
+      }
+    }
   }
+  if (kBackward && m1 == OH) store_row(2 * OH - 1, pend);   // below it there is no further window
+}
+
+StripArgs strip_args(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p) {
+  StripArgs a;
+  a.x = x;
+  a.dy = dy;
+  a.out = out;
+  a.record = record;
+  a.planes = p.N * p.C;
+  a.H = p.H;
+  a.W = p.W;
+  a.OH = p.OH;
+  a.OW = p.OW;
+  a.quads = (p.W + 3) / 4;
+  a.abreast = a.quads <= 32 ? 32 / a.quads : 1;
+  a.segments = a.quads <= 32 ? 1 : (a.quads + 29) / 30;
+  // A band re-reads the row above it (and, backward, works out the window rows
+  // at its edges twice), so bands are as tall as leaves about three warps per
+  // slot of the machine (32 per SM), at least four window rows.
+  const long long strips = static_cast<long long>((a.planes + a.abreast - 1) / a.abreast) * a.segments;
+  const long long want = (static_cast<long long>(sm_count()) * 96 + strips - 1) / strips;   // bands wanted
+  long long rows = (p.OH + want - 1) / want;
+  if (rows < 4) rows = 4;
+  if (rows > p.OH) rows = p.OH;
+  a.bands = static_cast<int>((p.OH + rows - 1) / rows);
+  a.rows = (p.OH + a.bands - 1) / a.bands;       // even heights
+  a.bands = (p.OH + a.rows - 1) / a.rows;
+  return a;
+}
+long long strip_ctas(const StripArgs& a) {
+  const long long strips = static_cast<long long>((a.planes + a.abreast - 1) / a.abreast) * a.segments;
+  return (strips * a.bands + kBlock / 32 - 1) / (kBlock / 32);
+}
+template <int MODE>
+int launch_k3s2p1(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p, cudaStream_t s) {
+  const StripArgs a = strip_args(x, dy, out, record, p);
+  const long long ctas = strip_ctas(a);
+  if (ctas > 0x7fffffffLL) return SGB_ERR_SIZE;
+  const bool vec = p.W % 4 == 0 && (!x || aligned16(x)) && (!dy || aligned16(dy)) && aligned16(out) &&
+                   (reinterpret_cast<uintptr_t>(record) & 1u) == 0;
+  return launch_ex(vec ? pool_k3s2p1_kernel<MODE, true> : pool_k3s2p1_kernel<MODE, false>,
+                   dim3(static_cast<unsigned>(ctas)), dim3(kBlock), 0, s, 0, true, a);
+}
+inline bool is_k3s2p1(const PoolShape& p) {
+  return p.kh == 3 && p.kw == 3 && p.sh == 2 && p.sw == 2 && p.ph == 1 && p.pw == 1;
+}
+
+// ------------------------------------------------ 3x3 / stride 1 / pad 1, max passes
+// Same layout: a lane owns four columns and the four windows centred on them.
+// The first maximum of three adjacent cells of a row is worked out once and
+// serves the three windows it belongs to (6 comparisons per window instead of
+// 9; taking a row's winner only if it is strictly greater than the rows above
+// keeps the raster order).  Was 231 us forward and 276 us backward at
+// 32x64x112x112, where the bytes take 31 and 47 us.
+struct RowBest {
+  float v[4];
+  int at[4];               // column offset 0..2 of the winner, kNoCell if none
+};
+
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(kBlock, 4)
+pool_k3s1p1_kernel(const StripArgs a) {
+  constexpr bool kBackward = MODE == kMaxBwd || MODE == kMaxBwdRecord;
+  constexpr bool kNeedsX = MODE != kMaxBwdRecord;
+  constexpr unsigned kAll = 0xffffffffu;
+  dependency_wait();
+  release_dependents();
+  const int lane = threadIdx.x & 31;
+  const unsigned task = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+  const unsigned rest = task / a.bands;
+  const int band = static_cast<int>(task - rest * a.bands);
+  const int group = static_cast<int>(rest / a.segments), seg = static_cast<int>(rest - group * a.segments);
+  int q, plane;
+  bool active, owner;
+  if (a.segments > 1) {
+    q = seg * 30 - 1 + lane;
+    plane = group;
+    active = q >= 0 && q < a.quads && plane < a.planes;
+    owner = active && lane >= 1 && lane <= 30;
+  } else {
+    const int pl = lane / a.quads;
+    q = lane - pl * a.quads;
+    plane = group * a.abreast + pl;
+    active = pl < a.abreast && plane < a.planes;
+    owner = active;
+  }
+  if (!active) plane = 0;
+  const int H = a.H, W = a.W, c = 4 * q;
+  const size_t origin = static_cast<size_t>(plane) * H * W + c;      // input and output planes have one size
+  const bool has_left = q > 0, has_right = q + 1 < a.quads;
+
+  auto load4 = [&](const float* p, int h, float pad, float (&v)[4]) {
+    const bool in = active && h >= 0 && h < H;
+    const float* r = p + origin + static_cast<ptrdiff_t>(h) * W;
+    if (VEC) {
+      float4 t = make_float4(pad, pad, pad, pad);
+      if (in) t = *reinterpret_cast<const float4*>(r);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = in && c + j < W ? r[j] : pad;
+    }
+  };
+  auto store4 = [&](float* p, int h, const float (&v)[4]) {
+    if (!owner || h < 0 || h >= H) return;
+    float* r = p + origin + static_cast<size_t>(h) * W;
+    if (VEC) {
+      *reinterpret_cast<float4*>(r) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < W) r[j] = v[j];
+    }
+  };
+  auto better = [](bool nans, float v, float best) { return v > best || (nans && v != v && best == best); };
+  // the winner of each window's three cells in one row, and whether the row
+  // (of the whole warp) holds anything that needs the NaN-aware comparison
+  auto row_best = [&](const float (&v)[4], RowBest& b) -> bool {
+    float left = __shfl_up_sync(kAll, v[3], 1), right = __shfl_down_sync(kAll, v[0], 1);
+    if (!has_left) left = -FLT_MAX;
+    if (!has_right) right = -FLT_MAX;
+    const float s = (v[0] + v[1]) + (v[2] + v[3]) + (left + right);
+    const bool nans = __any_sync(kAll, s != s);
+    const float cell[6] = {left, v[0], v[1], v[2], v[3], right};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float best = -FLT_MAX;
+      int at = kNoCell;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const bool p = better(nans, cell[j + k], best);
+        best = p ? cell[j + k] : best;
+        at = p ? k : at;
+      }
+      b.v[j] = best;
+      b.at[j] = at;
+    }
+    return nans;
+  };
+
+  // forward: output rows [m0, m1); backward: window rows m0 - 1 .. m1 feed dx rows [m0, m1)
+  const int m0 = band * a.rows, m1 = min(m0 + a.rows, H);
+  const int first = kBackward ? max(m0 - 1, 0) : m0, last = kBackward ? min(m1, H - 1) : m1 - 1;
+  RowBest up, mid, low;
+  bool nan_up = false, nan_mid = false, nan_low = false;
+  float v[4], ahead[4], g[4], g_ahead[4];
+  unsigned code_ahead[4] = {0, 0, 0, 0}, code[4];
+  auto load_codes = [&](int m, unsigned (&k)[4]) {
+    const unsigned char* r = a.record + origin + static_cast<size_t>(m) * W;
+    if (VEC) {
+      const unsigned t = active ? *reinterpret_cast<const unsigned*>(r) : 0xffffffffu;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = t >> (8 * j) & 0xffu;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) k[j] = active && c + j < W ? r[j] : 0xffu;
+    }
+  };
+  if (kNeedsX) {
+    load4(a.x, first - 1, -FLT_MAX, v);
+    load4(a.x, first, -FLT_MAX, ahead);
+    nan_up = row_best(v, up);
+    nan_mid = row_best(ahead, mid);
+    load4(a.x, first + 1, -FLT_MAX, ahead);
+  }
+  if (kBackward) load4(a.dy, first, 0.0f, g_ahead);
+  if (MODE == kMaxBwdRecord) load_codes(first, code_ahead);
+  float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};   // dx rows m - 1 and m so far
+  for (int m = first; m <= last; ++m) {
+    int win[4];
+    float best[4];
+    if (kNeedsX) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = ahead[j];
+      if (m < last) load4(a.x, m + 2, -FLT_MAX, ahead);
+    }
+    if (kBackward) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) g[j] = g_ahead[j];
+      if (m < last) load4(a.dy, m + 1, 0.0f, g_ahead);
+    }
+    if (MODE == kMaxBwdRecord) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) code[j] = code_ahead[j];
+      if (m < last) load_codes(m + 1, code_ahead);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        win[j] = code[j] == 0xffu ? kNoCell : static_cast<int>(code[j] >> 4) * 3 + static_cast<int>(code[j] & 15u);
+    }
+    if (kNeedsX) {
+      nan_low = row_best(v, low);
+      const bool nans = nan_up || nan_mid || nan_low;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        best[j] = up.v[j];
+        win[j] = up.at[j];
+        bool p = better(nans, mid.v[j], best[j]);
+        best[j] = p ? mid.v[j] : best[j];
+        win[j] = p ? 3 + mid.at[j] : win[j];
+        p = better(nans, low.v[j], best[j]);
+        best[j] = p ? low.v[j] : best[j];
+        win[j] = p ? 6 + low.at[j] : win[j];
+        if (kBackward && c + j >= W) win[j] = kNoCell;
+      }
+      up = mid;
+      mid = low;
+      nan_up = nan_mid;
+      nan_mid = nan_low;
+    }
+    if (!kBackward) {
+      store4(a.out, m, best);
+      if (MODE == kMaxFwdRecord && owner) {
+        unsigned char* r = a.record + origin + static_cast<size_t>(m) * W;
+        unsigned packed = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const unsigned k = win[j] < 0 ? 0xffu : static_cast<unsigned>((win[j] / 3) << 4 | win[j] % 3);
+          packed |= k << (8 * j);
+          if (!VEC && c + j < W) r[j] = static_cast<unsigned char>(k);
+        }
+        if (VEC) *reinterpret_cast<unsigned*>(r) = packed;
+      }
+      continue;
+    }
+    // the windows centred on columns c-1 .. c+4
+    int w[6];
+    float gw[6];
+    w[0] = __shfl_up_sync(kAll, win[3], 1);
+    gw[0] = __shfl_up_sync(kAll, g[3], 1);
+    w[5] = __shfl_down_sync(kAll, win[0], 1);
+    gw[5] = __shfl_down_sync(kAll, g[0], 1);
+    if (!has_left) w[0] = kNoCell;
+    if (!has_right) w[5] = kNoCell;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w[j + 1] = win[j];
+      gw[j + 1] = g[j];
+    }
+    // column c + j lies in the windows j, j + 1, j + 2 of that list, at column offsets 2, 1, 0
+    auto add_row = [&](int dr, float (&t)[4]) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) t[j] += w[j + k] == 3 * dr + 2 - k ? gw[j + k] : 0.0f;
+    };
+    add_row(0, acc0);
+    if (m - 1 >= m0) store4(a.out, m - 1, acc0);
+    add_row(1, acc1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc0[j] = acc1[j];
+      acc1[j] = 0.f;
+    }
+    add_row(2, acc1);
+  }
+  if (kBackward && m1 == H) store4(a.out, H - 1, acc0);     // below it there is no further window row
+}
+
+template <int MODE>
+int launch_k3s1p1(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p, cudaStream_t s) {
+  const StripArgs a = strip_args(x, dy, out, record, p);
+  const long long ctas = strip_ctas(a);
+  if (ctas > 0x7fffffffLL) return SGB_ERR_SIZE;
+  const bool vec = p.W % 4 == 0 && (!x || aligned16(x)) && (!dy || aligned16(dy)) && aligned16(out) &&
+                   (reinterpret_cast<uintptr_t>(record) & 3u) == 0;
+  return launch_ex(vec ? pool_k3s1p1_kernel<MODE, true> : pool_k3s1p1_kernel<MODE, false>,
+                   dim3(static_cast<unsigned>(ctas)), dim3(kBlock), 0, s, 0, true, a);
+}
+
+// ------------------------------------------------ 2x2 / stride 2 / no padding
+// The windows do not overlap: a thread owns four columns of two rows, i.e. two
+// whole windows.  Rows and columns that no window covers (odd sizes) get zero
+// gradient.  One 16-byte access per row where the width allows it.
+struct FastDiv {           // n / d for n < 2^31 by multiplication with ceil(2^(31 + l) / d), l = ceil(log2 d)
+  unsigned d, mul, shift;
+  explicit FastDiv(unsigned div) : d(div) {
+    unsigned l = 0;
+    while ((1ull << l) < div) ++l;
+    shift = 31 + l;
+    mul = static_cast<unsigned>(((1ull << shift) + div - 1) / div);
+  }
+  __device__ __forceinline__ unsigned quot(unsigned n) const {
+    return static_cast<unsigned>((static_cast<unsigned long long>(n) * mul) >> shift);
+  }
+};
+
+struct PairArgs {
+  const float* x;
+  const float* dy;
+  float* out;
+  unsigned char* record;
+  unsigned work;           // planes * row pairs * quads, < 2^31
+  int H, W, OH, OW;
+  FastDiv quads, pairs;    // quads per row, row pairs per plane
+};
+
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(kBlock)
+pool_k2s2_kernel(const PairArgs a) {
+  constexpr bool kBackward = MODE == kMaxBwd || MODE == kMaxBwdRecord || MODE == kAvgBwd;
+  constexpr bool kNeedsX = MODE != kMaxBwdRecord && MODE != kAvgBwd;
+  constexpr bool kMax = MODE <= kMaxBwdRecord;
+  dependency_wait();
+  release_dependents();
+  const unsigned i = blockIdx.x * static_cast<unsigned>(kBlock) + threadIdx.x;
+  if (i >= a.work) return;
+  const unsigned line = a.quads.quot(i);
+  const int c = 4 * static_cast<int>(i - line * a.quads.d);
+  const unsigned plane = a.pairs.quot(line);
+  const int m = static_cast<int>(line - plane * a.pairs.d), h = 2 * m;
+  const size_t in0 = (static_cast<size_t>(plane) * a.H + h) * a.W + c;
+  const size_t win = (static_cast<size_t>(plane) * a.OH + m) * a.OW + c / 2;
+  const bool second_row = h + 1 < a.H;
+  const bool exists[2] = {second_row && c + 1 < a.W, second_row && c + 3 < a.W};
+  float v[2][4];
+  if (kNeedsX) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      if (VEC) {
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r == 0 || second_row) t = *reinterpret_cast<const float4*>(a.x + in0 + static_cast<size_t>(r) * a.W);
+        v[r][0] = t.x; v[r][1] = t.y; v[r][2] = t.z; v[r][3] = t.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[r][j] = (r == 0 || second_row) && c + j < a.W ? a.x[in0 + static_cast<size_t>(r) * a.W + j] : 0.0f;
+      }
+    }
+  }
+  float o[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    if (!exists[w]) continue;
+    int at = kNoCell;
+    float best = kMax ? -FLT_MAX : 0.0f;
+    if (kNeedsX) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float t = v[k >> 1][2 * w + (k & 1)];
+        if (kMax) {
+          if (t > best || (t != t && best == best)) {   // first maximum; a NaN wins and then sticks, as in cuDNN
+            best = t;
+            at = k;
+          }
+        } else {
+          best += t;
+        }
+      }
+    }
+    if (!kBackward) {
+      a.out[win + w] = kMax ? best : best / 4.0f;
+      if (MODE == kMaxFwdRecord)
+        a.record[win + w] = at < 0 ? 0xff : static_cast<unsigned char>((at >> 1) << 4 | (at & 1));
+      continue;
+    }
+    float g = a.dy[win + w];
+    if (MODE == kMaxBwdRecord) {
+      const unsigned code = a.record[win + w];
+      at = code == 0xffu ? kNoCell : static_cast<int>(code >> 4) * 2 + static_cast<int>(code & 15u);
+    }
+    if (MODE == kAvgBwd) g = g / 4.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k >> 1][2 * w + (k & 1)] = 0.0f + (!kMax || at == k ? g : 0.0f);
+  }
+  if (!kBackward) return;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if (r == 1 && !second_row) break;
+    float* p = a.out + in0 + static_cast<size_t>(r) * a.W;
+    if (VEC) {
+      *reinterpret_cast<float4*>(p) = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < a.W) p[j] = o[r][j];
+    }
+  }
+}
+
+inline bool is_k2s2(const PoolShape& p) {
+  const long long work = static_cast<long long>(p.N) * p.C * ((p.H + 1) / 2) * ((p.W + 3) / 4);
+  return p.kh == 2 && p.kw == 2 && p.sh == 2 && p.sw == 2 && p.ph == 0 && p.pw == 0 && work < 0x7fffffffLL;
+}
+template <int MODE>
+int launch_k2s2(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p, cudaStream_t s) {
+  const unsigned quads = (p.W + 3) / 4, pairs = (p.H + 1) / 2;
+  const unsigned work = static_cast<unsigned>(p.N) * p.C * pairs * quads;
+  const PairArgs a{x, dy, out, record, work, p.H, p.W, p.OH, p.OW, FastDiv(quads), FastDiv(pairs)};
+  const bool backward = MODE == kMaxBwd || MODE == kMaxBwdRecord || MODE == kAvgBwd;
+  const bool vec = p.W % 4 == 0 && (!x || aligned16(x)) && (!backward || aligned16(out));
+  return launch_ex(vec ? pool_k2s2_kernel<MODE, true> : pool_k2s2_kernel<MODE, false>,
+                   dim3(static_cast<unsigned>(ceil_div(work, kBlock))), dim3(kBlock), 0, s, 0, true, a);
+}
+
+// Global average (one window = the whole plane): a warp adds up one plane.
+__global__ void __launch_bounds__(kBlock)
+avgpool_fwd_global_kernel(const float* __restrict__ x, float* __restrict__ y, int planes, int hw) {
+  dependency_wait();
+  release_dependents();
+  const int plane = static_cast<int>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (plane >= planes) return;
+  const float* p = x + static_cast<size_t>(plane) * hw;
+  float s = 0.f;
+#pragma unroll 8
+  for (int i = lane; i < hw; i += 32) s += p[i];
+  s = warp_sum(s);
+  if (lane == 0) y[plane] = s / static_cast<float>(hw);
+}
+
+// The geometries above, if `p` is one of them; `done` tells.
+template <int MODE>
+int launch_known(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p, cudaStream_t s,
+                 bool* done) {
+  *done = true;
+  if (is_k3s2p1(p) && static_cast<long long>(p.N) * p.C <= 0x7fffffffLL)
+    return launch_k3s2p1<MODE>(x, dy, out, record, p, s);
+  if (is_k2s2(p)) return launch_k2s2<MODE>(x, dy, out, record, p, s);
+  if constexpr (MODE <= kMaxBwdRecord)
+    if (p.kh == 3 && p.kw == 3 && p.sh == 1 && p.sw == 1 && p.ph == 1 && p.pw == 1 &&
+        static_cast<long long>(p.N) * p.C <= 0x7fffffffLL)
+      return launch_k3s1p1<MODE>(x, dy, out, record, p, s);
+  *done = false;
+  return SGB_OK;
 }
 
 // Band height: the largest power-of-two-ish row count whose staging fits
@@ -488,6 +1024,8 @@ BandPlan plan_bands(const PoolShape& p, size_t budget) {
 __global__ void __launch_bounds__(kBlock)
 maxpool_bwd_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                    float* __restrict__ dx, PoolShape p) {
+  dependency_wait();
+  release_dependents();
   const size_t plane = blockIdx.x;
   const int i = blockIdx.y * kBlock + threadIdx.x;
   if (i >= p.H * p.W) return;
@@ -525,6 +1063,8 @@ maxpool_bwd_kernel(const float* __restrict__ x, const float* __restrict__ dy,
 __global__ void __launch_bounds__(kBlock)
 avgpool_bwd_kernel(const float* __restrict__ dy, float* __restrict__ dx, PoolShape p,
                    unsigned total) {
+  dependency_wait();
+  release_dependents();
   const unsigned i = blockIdx.x * static_cast<unsigned>(kBlock) + threadIdx.x;
   if (i >= total) return;
   const unsigned hw = static_cast<unsigned>(p.H * p.W);
@@ -550,6 +1090,8 @@ avgpool_bwd_kernel(const float* __restrict__ dy, float* __restrict__ dx, PoolSha
 __global__ void __launch_bounds__(kBlock)
 avgpool_bwd_global_kernel(const float* __restrict__ dy, float* __restrict__ dx, unsigned hw,
                           unsigned total4) {
+  dependency_wait();
+  release_dependents();
   const unsigned v = blockIdx.x * static_cast<unsigned>(kBlock) + threadIdx.x;
   if (v >= total4) return;
   const unsigned i = 4u * v;
@@ -607,16 +1149,26 @@ int sgb_maxpool_forward_f32(const float* x, float* y, int N, int C, int H, int W
                             int ph, int pw, int sh, int sw, void* stream) {
   POOL_PROLOGUE(1)
   if (!x || !y) return SGB_ERR_NULL;
-  pool_fwd_kernel<true><<<blocks_for(out_total), kBlock, 0, as_stream(stream)>>>(x, y, p, out_total);
-  return launch_status();
+  bool done;
+  const int r = launch_known<kMaxFwd>(x, nullptr, y, nullptr, p, as_stream(stream), &done);
+  if (done) return r;
+  return launch_ex(pool_fwd_kernel<true>, dim3(blocks_for(out_total)), dim3(kBlock), 0, as_stream(stream), 0, true, x, y,
+                   p, out_total);
 }
 
 int sgb_avgpool_forward_f32(const float* x, float* y, int N, int C, int H, int W, int kh, int kw,
                             int ph, int pw, int sh, int sw, void* stream) {
   POOL_PROLOGUE(1)
   if (!x || !y) return SGB_ERR_NULL;
-  pool_fwd_kernel<false><<<blocks_for(out_total), kBlock, 0, as_stream(stream)>>>(x, y, p, out_total);
-  return launch_status();
+  if (p.OH == 1 && p.OW == 1 && ph == 0 && pw == 0 && kh == H && kw == W &&
+      static_cast<long long>(N) * C <= 0x7fffffffLL && static_cast<long long>(H) * W <= 0x7fffffffLL)
+    return launch_ex(avgpool_fwd_global_kernel, dim3(static_cast<unsigned>(ceil_div(out_total, kBlock / 32))),
+                     dim3(kBlock), 0, as_stream(stream), 0, true, x, y, N * C, H * W);
+  bool done;
+  const int r = launch_known<kAvgFwd>(x, nullptr, y, nullptr, p, as_stream(stream), &done);
+  if (done) return r;
+  return launch_ex(pool_fwd_kernel<false>, dim3(blocks_for(out_total)), dim3(kBlock), 0, as_stream(stream), 0, true, x,
+                   y, p, out_total);
 }
 
 int sgb_maxpool_backward_f32(const float* x, const float* y, const float* dy, float* dx, int N,
@@ -627,54 +1179,27 @@ int sgb_maxpool_backward_f32(const float* x, const float* y, const float* dy, fl
   if (!x || !dy || !dx) return SGB_ERR_NULL;
   const size_t planes = static_cast<size_t>(N) * C;
   if (planes > 0x7fffffffu || static_cast<long long>(H) * W > 0x7fffffffLL) return SGB_ERR_SIZE;
+  cudaStream_t s = as_stream(stream);
+  bool done;
+  const int r = launch_known<kMaxBwd>(x, dy, dx, nullptr, p, s, &done);
+  if (done) return r;
   const BandPlan bp = plan_bands(p, 24 * 1024);
   if (bp.rows > 0 && bp.bands <= 65535) {
     const size_t smem = (static_cast<size_t>(bp.max_xrows) * W +
                          2 * static_cast<size_t>(bp.max_orows) * p.OW) * sizeof(float);
     const dim3 grid(static_cast<unsigned>(planes), bp.bands);
-    cudaStream_t s = as_stream(stream);
     const bool square = kh == kw && sh == sw && ph == pw && W % 4 == 0 && aligned16(x) && aligned16(dx);
-    if (square && kh == 3 && sh == 2 && ph == 1 && H % 2 == 0 && H >= 2) {
-      const int nb = (H + 31) / 32;
-      int rows = (H + nb - 1) / nb;
-      rows += rows & 1;
-      const int nbands = (H + rows - 1) / rows;
-      const size_t bytes = (static_cast<size_t>(rows + 3) * (W + 4) +
-                            2 * static_cast<size_t>((rows >> 1) + 2) * (p.OW + 1)) * sizeof(float);
-      if (bytes <= 48 * 1024 && nbands <= 65535) {
-        const dim3 g(static_cast<unsigned>(planes), nbands);
-#define SGB_STEM_W(WW)                                                                              \
-  if (W == WW && p.OW == WW / 2) {                                                                  \
-    maxpool_bwd_k3s2p1_kernel<WW><<<g, kBlock, bytes, s>>>(x, dy, dx, H, W, p.OH, p.OW, rows);      \
-    return launch_status();                                                                         \
-  }
-        SGB_STEM_W(112)
-        SGB_STEM_W(56)
-        SGB_STEM_W(32)
-#undef SGB_STEM_W
-        maxpool_bwd_k3s2p1_kernel<0><<<g, kBlock, bytes, s>>>(x, dy, dx, H, W, p.OH, p.OW, rows);
-        return launch_status();
-      }
-    }
 #define SGB_POOL_FAST(KK, SS, PP)                                                       \
-  if (square && kh == KK && sh == SS && ph == PP) {                                     \
-    maxpool_bwd_band_fast_kernel<KK, SS, PP><<<grid, kBlock, smem, s>>>(x, dy, dx, p, bp); \
-    return launch_status();                                                             \
-  }
-    SGB_POOL_FAST(3, 2, 1)
-    SGB_POOL_FAST(2, 2, 0)
+  if (square && kh == KK && sh == SS && ph == PP)                                       \
+    return launch_ex(maxpool_bwd_band_fast_kernel<KK, SS, PP>, grid, dim3(kBlock), smem, s, 0, true, x, dy, dx, p, bp);
     SGB_POOL_FAST(3, 2, 0)
-    SGB_POOL_FAST(3, 1, 1)
     SGB_POOL_FAST(2, 1, 0)
 #undef SGB_POOL_FAST
-    maxpool_bwd_band_kernel<<<grid, kBlock, smem, s>>>(x, dy, dx, p, bp);
-  } else {
-    const unsigned by = blocks_for(static_cast<size_t>(H) * W);
-    if (by > 65535) return SGB_ERR_SIZE;
-    maxpool_bwd_kernel<<<dim3(static_cast<unsigned>(planes), by), kBlock, 0, as_stream(stream)>>>(
-        x, dy, dx, p);
+    return launch_ex(maxpool_bwd_band_kernel, grid, dim3(kBlock), smem, s, 0, true, x, dy, dx, p, bp);
   }
-  return launch_status();
+  const unsigned by = blocks_for(static_cast<size_t>(H) * W);
+  if (by > 65535) return SGB_ERR_SIZE;
+  return launch_ex(maxpool_bwd_kernel, dim3(static_cast<unsigned>(planes), by), dim3(kBlock), 0, s, 0, true, x, dy, dx, p);
 }
 
 int sgb_maxpool_forward_argmax_f32(const float* x, float* y, unsigned char* argmax, int N, int C, int H,
@@ -682,8 +1207,11 @@ int sgb_maxpool_forward_argmax_f32(const float* x, float* y, unsigned char* argm
   POOL_PROLOGUE(1)
   if (!x || !y || !argmax) return SGB_ERR_NULL;
   if (kh > 15 || kw > 15) return SGB_ERR_UNSUPPORTED;           // offsets are stored in nibbles; 15|15 is "none"
-  maxpool_fwd_argmax_kernel<<<blocks_for(out_total), kBlock, 0, as_stream(stream)>>>(x, y, argmax, p, out_total);
-  return launch_status();
+  bool done;
+  const int r = launch_known<kMaxFwdRecord>(x, nullptr, y, argmax, p, as_stream(stream), &done);
+  if (done) return r;
+  return launch_ex(maxpool_fwd_argmax_kernel, dim3(blocks_for(out_total)), dim3(kBlock), 0, as_stream(stream), 0, true,
+                   x, y, argmax, p, out_total);
 }
 
 int sgb_maxpool_backward_argmax_f32(const float* dy, const unsigned char* argmax, float* dx, int N, int C,
@@ -692,32 +1220,12 @@ int sgb_maxpool_backward_argmax_f32(const float* dy, const unsigned char* argmax
   POOL_PROLOGUE(0)
   if (!dy || !argmax || !dx) return SGB_ERR_NULL;
   if (kh > 15 || kw > 15) return SGB_ERR_UNSUPPORTED;
-  const size_t planes = static_cast<size_t>(N) * C;
   cudaStream_t s = as_stream(stream);
-  if (kh == 3 && kw == 3 && sh == 2 && sw == 2 && ph == 1 && pw == 1 && W % 4 == 0 && H % 2 == 0 && H >= 2 &&
-      aligned16(dx) && planes <= 0x7fffffffu && static_cast<long long>(H) * W <= 0x7fffffffLL) {
-    const int nb = (H + 31) / 32;
-    int rows = (H + nb - 1) / nb;
-    rows += rows & 1;
-    const int nbands = (H + rows - 1) / rows;
-    const size_t bytes = 2 * static_cast<size_t>((rows >> 1) + 2) * (p.OW + 1) * sizeof(float);
-    if (bytes <= 48 * 1024 && nbands <= 65535) {
-      const dim3 g(static_cast<unsigned>(planes), nbands);
-#define SGB_STEM_W(WW)                                                                                  \
-  if (W == WW && p.OW == WW / 2) {                                                                      \
-    maxpool_bwd_argmax_k3s2p1_kernel<WW><<<g, kBlock, bytes, s>>>(dy, argmax, dx, H, W, p.OH, p.OW, rows); \
-    return launch_status();                                                                             \
-  }
-      SGB_STEM_W(112)
-      SGB_STEM_W(56)
-      SGB_STEM_W(32)
-#undef SGB_STEM_W
-      maxpool_bwd_argmax_k3s2p1_kernel<0><<<g, kBlock, bytes, s>>>(dy, argmax, dx, H, W, p.OH, p.OW, rows);
-      return launch_status();
-    }
-  }
-  maxpool_bwd_argmax_kernel<<<blocks_for(in_total), kBlock, 0, s>>>(dy, argmax, dx, p, in_total);
-  return launch_status();
+  bool done;
+  const int r = launch_known<kMaxBwdRecord>(nullptr, dy, dx, const_cast<unsigned char*>(argmax), p, s, &done);
+  if (done) return r;
+  return launch_ex(maxpool_bwd_argmax_kernel, dim3(blocks_for(in_total)), dim3(kBlock), 0, s, 0, true, dy, argmax, dx, p,
+                   in_total);
 }
 
 int sgb_avgpool_backward_f32(const float* dy, float* dx, int N, int C, int H, int W, int kh,
@@ -729,10 +1237,12 @@ int sgb_avgpool_backward_f32(const float* dy, float* dx, int N, int C, int H, in
   if (p.OH == 1 && p.OW == 1 && ph == 0 && pw == 0 && kh == H && kw == W && aligned16(dx) &&
       in_total % 4 == 0 && in_total < 0x7fffffffu) {
     const unsigned total4 = static_cast<unsigned>(in_total / 4);
-    avgpool_bwd_global_kernel<<<blocks_for(total4), kBlock, 0, as_stream(stream)>>>(
-        dy, dx, static_cast<unsigned>(H * W), total4);
-    return launch_status();
+    return launch_ex(avgpool_bwd_global_kernel, dim3(blocks_for(total4)), dim3(kBlock), 0, as_stream(stream), 0, true,
+                     dy, dx, static_cast<unsigned>(H * W), total4);
   }
+  bool done;
+  const int r = launch_known<kAvgBwd>(nullptr, dy, dx, nullptr, p, as_stream(stream), &done);
+  if (done) return r;
   // whole planes per launch, each launch below 2^31 elements
   const size_t hw = static_cast<size_t>(H) * W;
   const size_t planes_per_launch = (0x7fffffffu - kBlock) / hw;
@@ -740,8 +1250,9 @@ int sgb_avgpool_backward_f32(const float* dy, float* dx, int N, int C, int H, in
   for (size_t p0 = 0; p0 < planes; p0 += planes_per_launch) {
     const size_t np = planes - p0 < planes_per_launch ? planes - p0 : planes_per_launch;
     const unsigned total = static_cast<unsigned>(np * hw);
-    avgpool_bwd_kernel<<<blocks_for(total), kBlock, 0, as_stream(stream)>>>(
-        dy + p0 * p.OH * p.OW, dx + p0 * hw, p, total);
+    const int e = launch_ex(avgpool_bwd_kernel, dim3(blocks_for(total)), dim3(kBlock), 0, as_stream(stream), 0, true,
+                            dy + p0 * p.OH * p.OW, dx + p0 * hw, p, total);
+    if (e != SGB_OK) return e;
   }
   return launch_status();
 }
