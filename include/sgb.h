@@ -358,8 +358,10 @@ int sgb_bn_forward_training_f32(const float *x, const float *scale,
  * CTAs meet through counters in device memory with bounded waits: *flags
  * receives the sticky fault word of the current device (0 = none; bit 0 a
  * wait ran out, bit 1 a counter table was still in use by another launch - at
- * most eight such launches may be in flight per device).  A faulted launch
- * stops early and its outputs are undefined.  Synchronises the device. */
+ * most eight such launches may be in flight per device; bits 8 and 16 the same
+ * for the exchanges inside the backward and forward cluster kernels).  A
+ * faulted launch stops early and its outputs are undefined.  Synchronises the
+ * device. */
 int sgb_bn_backward_faults(unsigned *flags);
 /* How the streaming form would cut an (N, C, HW) problem (host arithmetic
  * only, no device work): returns 1 and fills plan6 = {pieces per plane, floats

@@ -34,101 +34,13 @@
 // The optional ReLU mask fuses "dy = relu_in > 0 ? dy : 0" (the backward of
 // the ReLU that follows the BN layer) into both passes, which removes one
 // full write + read of the intermediate gradient.
-#include <cooperative_groups.h>
-#include <stdlib.h>
-
-#include <atomic>
-
+#include "bn_common.cuh"
 #include "bn_stream.cuh"
-#include "bulk_copy.cuh"
-#include "common.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace sgb {
 namespace {
-
-constexpr int kBlock = 256;
-constexpr int kMaxSlices = 64;
-
-// Opts a kernel in to more than 48 KB of dynamic shared memory (and, for the
-// cluster kernels, to non-portable cluster sizes) once per device: the
-// attribute sticks to the function in that device's context, so later
-// launches - including launches under stream capture - issue no attribute
-// call.  `done` is one flag per device ordinal; ordinals beyond the table are
-// set every time.  Racing first calls from two host threads both set the
-// same attribute, which is harmless.
-template <typename K>
-int opt_in_once(K kernel, std::atomic<bool>* done, bool cluster) {
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
-  const bool tracked = dev >= 0 && dev < 64;
-  if (tracked && done[dev].load(std::memory_order_acquire)) return SGB_OK;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  if (e != cudaSuccess) return note_cuda_error(e);
-  if (cluster) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return note_cuda_error(e);
-  }
-  if (tracked) done[dev].store(true, std::memory_order_release);
-  return SGB_OK;
-}
-
-struct BnShape {
-  int N, C, HW;
-};
-
-// Walks the units u0 + tid, u0 + tid + T, ... of a share and keeps the
-// (plane n, position q) decomposition up to date without a division per step.
-struct UnitWalk {
-  int n, q, dn, dq, hwu;
-  __device__ __forceinline__ UnitWalk(int u, int step, int hwu_) : hwu(hwu_) {
-    n = u / hwu_;
-    q = u - n * hwu_;
-    dn = step / hwu_;
-    dq = step - dn * hwu_;
-  }
-  __device__ __forceinline__ void next() {
-    n += dn;
-    q += dq;
-    if (q >= hwu) {
-      q -= hwu;
-      ++n;
-    }
-  }
-};
-
-// How the fused ReLU backward learns which gradients to keep.  MASK 0: no ReLU.
-// MASK 1: from the ReLU's stored input (keep where it is > 0).  MASK 2: from the
-// forward partner's record, one bit per element in element order (bit i & 7 of
-// byte i >> 3; 1 = the input was > 0), passed through the same pointer.
-// `off` is the element offset; for the 4-wide forms it is a multiple of 4.
-template <int MASK>
-__device__ __forceinline__ unsigned keep4(const float* relu_in, size_t off) {
-  if (MASK == 2) {
-    const unsigned char b = reinterpret_cast<const unsigned char*>(relu_in)[off >> 3];
-    return (b >> (off & 4)) & 15u;
-  }
-  Vec4f v;
-  v.u = ld128(relu_in + off);
-  unsigned bits = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) bits |= (v.f[k] > 0 ? 1u : 0u) << k;
-  return bits;
-}
-template <int MASK>
-__device__ __forceinline__ bool keep1(const float* relu_in, size_t off) {
-  if (MASK == 2) return (reinterpret_cast<const unsigned char*>(relu_in)[off >> 3] >> (off & 7)) & 1u;
-  return relu_in[off] > 0;
-}
-
-__host__ __device__ inline int bn_slices_for(long long per_channel, int C, int sms) {
-  long long s = (static_cast<long long>(sms) * 16 + C - 1) / C;
-  const long long max_s = (per_channel + 2047) / 2048;  // >= 2048 elements per slice
-  if (s > max_s) s = max_s;
-  if (s > kMaxSlices) s = kMaxSlices;
-  return static_cast<int>(s < 1 ? 1 : s);
-}
 
 template <bool VEC, int MASK>
 __global__ void __launch_bounds__(kBlock)
@@ -275,24 +187,6 @@ bn_bwd_apply_kernel(const float* __restrict__ x, const float* __restrict__ dy,
 }
 
 // ----------------------------------------------------------- single pass
-__device__ __forceinline__ void cp_async16(float* smem_dst, const float* gmem_src) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Returns once at most PENDING of this thread's most recent copy groups are still in flight.
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait_pending() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-// A thread issues its copies in kCopyGroups groups, so that it can start adding
-// up the units of the first group while the later ones are still in flight
-// (a thread only ever reads back what it staged itself: no barrier needed).
-constexpr int kCopyGroups = 4;
-
 // CTA size of the single-pass kernel: 512 threads for large shares (fewer
 // serial iterations per thread), 256 for small ones.
 
@@ -717,6 +611,110 @@ bn_bwd_group_kernel(const float* __restrict__ x, const float* __restrict__ dy,
   }
 }
 
+// ------------------------------------------- single pass, channels in registers
+// Small channels (one sample of a 40x40 plane, a small batch of 10x10 or 5x5
+// planes): 32, 128 or 256 threads hold a channel's operands in registers, so
+// there is nothing between the loads and the stores but the reduction - no
+// staging, no cluster, for a warp (four channels per CTA) not even a barrier.
+// Such calls are latency, not bandwidth: what they cost is the length of this
+// chain.  3x1024x10x10: 5.3 -> 2.3 us, fused with ReLU 8.3 -> 3.8 us.
+// NV units (float4, or float when !VEC) per thread and operand.  MASK 3: the
+// incoming gradient is the join dy + dy_b, masked by the ReLU's input and also
+// written to `joined` (only with VEC).
+template <int MASK, int G, int NV, bool VEC>
+__global__ void __launch_bounds__(G == 32 ? 128 : G)
+bn_bwd_small_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ relu_in,
+                    const float* __restrict__ scale, const float* __restrict__ mean, const float* __restrict__ invstd,
+                    float* __restrict__ dx, float* __restrict__ dscale, float* __restrict__ dbias, BnShape sh,
+                    const float* __restrict__ dy_b, float* __restrict__ joined) {
+  constexpr int kW = VEC ? 4 : 1;
+  __shared__ float sm[2 * G / 32];
+  const int c = G == 32 ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
+  const int t = G == 32 ? threadIdx.x & 31 : threadIdx.x;
+  dependency_wait();
+  release_dependents();
+  if (c >= sh.C) return;
+  const int hwu = sh.HW / kW, total = sh.N * hwu;
+  const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
+  float vx[NV][kW], vg[NV][kW];
+  size_t off[NV];
+  UnitWalk w(t, G, hwu);
+#pragma unroll
+  for (int k = 0; k < NV; ++k, w.next()) {
+    off[k] = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * kW;
+    const bool in = t + k * G < total;
+    if (VEC) {
+      Vec4f a, b, m, e;
+      a.u = b.u = m.u = e.u = make_uint4(0, 0, 0, 0);
+      unsigned bits = 15u;
+      if (in) {
+        a.u = ld128(x + off[k]);
+        b.u = ld128(dy + off[k]);
+        if (MASK == 3) e.u = ld128(dy_b + off[k]);
+        if (MASK == 1 || MASK == 3) m.u = ld128(relu_in + off[k]);
+        if (MASK == 2) bits = keep4<2>(relu_in, off[k]);
+      }
+#pragma unroll
+      for (int j = 0; j < kW; ++j) {
+        vx[k][j] = a.f[j];
+        vg[k][j] = b.f[j];
+        if (MASK == 3) vg[k][j] = m.f[j] > 0 ? (b.f[j] + e.f[j]) : 0.0f;
+        if (MASK == 1) vg[k][j] = m.f[j] > 0 ? vg[k][j] : 0.0f;
+        if (MASK == 2) vg[k][j] = (bits >> j) & 1u ? vg[k][j] : 0.0f;
+      }
+    } else {
+      vx[k][0] = vg[k][0] = 0.0f;
+      if (in) {
+        vx[k][0] = x[off[k]];
+        vg[k][0] = dy[off[k]];
+        if (MASK) vg[k][0] = keep1<MASK>(relu_in, off[k]) ? vg[k][0] : 0.0f;
+      }
+    }
+  }
+  const float mu = mean[c], r = invstd[c], sc = scale[c];
+  float a = 0.f, b = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int j = 0; j < kW; ++j) {     // outside the channel both are 0 (a test here would split the loads above)
+      a += vg[k][j];
+      b += vg[k][j] * (vx[k][j] - mu);
+    }
+  channel_sums<G, true>(a, b, sm);
+  const float inv_m = 1.0f / (static_cast<float>(sh.N) * static_cast<float>(sh.HW));
+  const float ds = b * r, k_ = sc * r, am = a * inv_m, bm = ds * r * inv_m;
+  if (t == 0) {
+    dscale[c] = ds;
+    dbias[c] = a;
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    if (t + k * G >= total) break;
+    if (VEC) {
+      Vec4f o;
+#pragma unroll
+      for (int j = 0; j < kW; ++j) o.f[j] = k_ * (vg[k][j] - am - (vx[k][j] - mu) * bm);
+      st128(dx + off[k], o.u);
+      if (MASK == 3) {
+#pragma unroll
+        for (int j = 0; j < kW; ++j) o.f[j] = vg[k][j];
+        st128(joined + off[k], o.u);
+      }
+    } else {
+      dx[off[k]] = k_ * (vg[k][0] - am - (vx[k][0] - mu) * bm);
+    }
+  }
+}
+
+template <int MASK, int G, int NV, bool VEC>
+int launch_small(const float* x, const float* dy, const float* relu_in, const float* scale, const float* mean,
+                 const float* invstd, float* dx, float* dscale, float* dbias, BnShape sh, cudaStream_t s,
+                 const float* dy_b = nullptr, float* joined = nullptr) {
+  const unsigned grid = static_cast<unsigned>(G == 32 ? (sh.C + 3) / 4 : sh.C);
+  return launch_ex(bn_bwd_small_kernel<MASK, G, NV, VEC>, dim3(grid), dim3(G == 32 ? 128 : G), 0, s, 0, true, x, dy,
+                   relu_in, scale, mean, invstd, dx, dscale, dbias, sh, dy_b, joined);
+}
+
 template <int MASK, int G>
 int launch_group(const float* x, const float* dy, const float* relu_in, const float* scale,
                  const float* mean, const float* invstd, float* dx, float* dscale, float* dbias,
@@ -730,34 +728,351 @@ int launch_group(const float* x, const float* dy, const float* relu_in, const fl
                    dx, dscale, dbias, sh);
 }
 
-// Cluster size (1, 2, 4 or 8) and per-CTA share for the single-pass kernel;
-// returns 0 when a channel does not fit 8 CTAs' shared memory.
-int cluster_plan(long long units_per_channel, int unit_bytes, int* per_cta, int channels) {
-  constexpr int share_kb = 50;   // preferred staging per CTA
-  constexpr int max_cs = 8;      // portable cluster size (16-CTA clusters with 50 KB shares measured slower)
-  constexpr int fill = 0;        // >0 would split small channels further (measured slower on B200)
-  const long long kPreferred = share_kb * 1024LL, kLimit = 100 * 1024;
+// One warp: this CTA's pair of sums goes to the slot parts[rank] of all `cs`
+// CTAs of the cluster as asynchronous 8-byte stores that signal the receiver's
+// mbarrier: a CTA goes on as soon as its cs pairs are in.  The peers have
+// started (cluster barrier): their memory is addressable.
+__device__ __forceinline__ void exchange_pairs(int cs, int rank, float p0, float p1, float2* parts,
+                                               unsigned long long* pairs_in) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) mbar_arrive_expect(pairs_in, 8u * static_cast<unsigned>(cs));
+  if (lane < cs) {
+    unsigned remote_slot, remote_bar;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_slot) : "r"(smem_addr(&parts[rank])), "r"(lane));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_bar) : "r"(smem_addr(pairs_in)), "r"(lane));
+    const unsigned long long bits = (static_cast<unsigned long long>(__float_as_uint(p1)) << 32) |
+                                    static_cast<unsigned long long>(__float_as_uint(p0));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(remote_slot),
+                 "l"(bits), "r"(remote_bar)
+                 : "memory");
+  }
+}
+// All threads: the totals over the cluster, in rank order, once every pair has
+// landed (bounded wait; a run-out sets the sticky fault word).
+__device__ __forceinline__ void pair_totals(int cs, const float2* parts, unsigned long long* pairs_in, float& a,
+                                            float& b) {
+  bool in = false;
+  for (unsigned it = 0; it < (1u << 24) && !in; ++it) in = mbar_try_wait(pairs_in, 0);
+  if (!in) atomicOr(&g_cluster_faults, 1u);
+  a = b = 0.f;
+  for (int r = 0; r < cs; ++r) {
+    a += parts[r].x;
+    b += parts[r].y;
+  }
+}
 
-  for (int pass = 0; pass < 2; ++pass) {
-    const long long cap = pass == 0 ? kPreferred : kLimit;
-    for (int cs = 1; cs <= max_cs; cs *= 2) {
-      long long share = (units_per_channel + cs - 1) / cs;
-      if (share * unit_bytes * 2 <= cap && share <= 8192) {   // <= 16 units per thread of a 512-thread CTA
-        // Small tensors: a grid of C*cs CTAs that leaves SMs idle is latency
-        // bound; split the channel over more CTAs (shorter per-thread loops)
-        // while a share still keeps every thread of a 256-thread CTA busy.
-        const long long want = static_cast<long long>(sm_count()) * fill;
-        while (cs * 2 <= max_cs && static_cast<long long>(channels) * cs < want &&
-               (units_per_channel + 2 * cs - 1) / (2 * cs) >= 512) {
-          cs *= 2;
-          share = (units_per_channel + cs - 1) / cs;
+// ---------------------------------- planes that are not a multiple of four floats
+// The cluster scheme over the aligned vectors that touch a plane (RaggedUnit);
+// with one float per access the loads of a CTA were a quarter as wide.
+template <int MASK, int T>
+__global__ void __launch_bounds__(T)
+bn_bwd_ragged_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ relu_in,
+                     const float* __restrict__ scale, const float* __restrict__ mean, const float* __restrict__ invstd,
+                     float* __restrict__ dx, float* __restrict__ dscale, float* __restrict__ dbias, BnShape sh,
+                     int per_cta, size_t numel) {
+  extern __shared__ __align__(16) float stage[];
+  __shared__ unsigned long long pairs_in;
+  __shared__ float red[2 * T / 32];
+  __shared__ float2 parts[16];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = static_cast<int>(cluster.num_blocks());
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int c = blockIdx.x / cs;
+  if (threadIdx.x == 0) {
+    mbar_init(&pairs_in, 1);
+    fence_mbarrier_init();
+  }
+  cluster.barrier_arrive();
+  const int upp = ragged_units(sh.HW), total = sh.N * upp;
+  const int u0 = min(rank * per_cta, total), u1 = min(u0 + per_cta, total);
+  const int first = u0 + threadIdx.x;
+  float* sx = stage;
+  float* sg = stage + static_cast<size_t>(per_cta) * 4;
+  const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
+  dependency_wait();
+  const float mu = mean[c];
+  const int group_units = ((per_cta + T - 1) / T + kCopyGroups - 1) / kCopyGroups;
+  {
+    UnitWalk w(first, T, upp);
+    int u = first;
+#pragma unroll
+    for (int g = 0; g < kCopyGroups; ++g) {
+      for (int k = 0; k < group_units && u < u1; ++k, u += T, w.next()) {
+        const RaggedUnit r(w.n * plane_stride + chan_off, w.q, sh.HW);
+        const int l = (u - u0) * 4;
+        if (r.valid) {
+          ragged_copy(sx + l, x, r.off, numel);
+          ragged_copy(sg + l, dy, r.off, numel);
         }
-        *per_cta = static_cast<int>(share);
-        return cs;
+      }
+      cp_async_commit();
+    }
+  }
+  // ReLU decisions, 4 bits per unit (a share is at most 16 units per thread)
+  unsigned long long keep = 0;
+  if (MASK) {
+    UnitWalk w(first, T, upp);
+    int slot = 0;
+    for (int u = first; u < u1;) {
+      Vec4f vm[4];
+      unsigned bits[4];
+      int cnt = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        bits[j] = 0;
+        vm[j].u = make_uint4(0, 0, 0, 0);
+        if (u < u1) {
+          const RaggedUnit r(w.n * plane_stride + chan_off, w.q, sh.HW);
+          if (r.valid) {
+            if (MASK == 1) vm[j] = ragged_load(relu_in, r.off, numel);
+            else bits[j] = keep4<2>(relu_in, r.off);
+          }
+          u += T;
+          w.next();
+          cnt = j + 1;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j < cnt) {
+          if (MASK == 1)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) bits[j] |= (vm[j].f[k] > 0 ? 1u : 0u) << k;
+          keep |= static_cast<unsigned long long>(bits[j] & 15u) << slot;
+          slot += 4;
+        }
       }
     }
   }
-  return 0;
+  float s_dy = 0.f, s_dyx = 0.f;
+  {
+    UnitWalk w(first, T, upp);
+    int slot = 0, u = first;
+    auto sum_copy_group = [&]() {
+      for (int k = 0; k < group_units && u < u1; ++k, u += T, slot += 4, w.next()) {
+        const RaggedUnit r(w.n * plane_stride + chan_off, w.q, sh.HW);
+        if (!r.valid) continue;
+        const int l = (u - u0) * 4;
+        Vec4f vx, vg;
+        vx.u = *reinterpret_cast<const uint4*>(sx + l);
+        vg.u = *reinterpret_cast<const uint4*>(sg + l);
+        if (MASK) {
+          const unsigned bits = static_cast<unsigned>(keep >> slot);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) vg.f[q] = (bits >> q) & 1u ? vg.f[q] : 0.0f;
+          *reinterpret_cast<uint4*>(sg + l) = vg.u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (r.valid >> q & 1u) {
+            s_dy += vg.f[q];
+            s_dyx += vg.f[q] * (vx.f[q] - mu);
+          }
+      }
+    };
+    static_assert(kCopyGroups == 4, "the waits below are written out for four groups");
+    cp_async_wait_pending<3>();
+    sum_copy_group();
+    cp_async_wait_pending<2>();
+    sum_copy_group();
+    cp_async_wait_pending<1>();
+    sum_copy_group();
+    cp_async_wait_pending<0>();
+    sum_copy_group();
+  }
+  channel_sums<T, true>(s_dy, s_dyx, red);
+  cluster.barrier_wait();
+  if (threadIdx.x < 32) exchange_pairs(cs, rank, s_dy, s_dyx, parts, &pairs_in);
+  // no CTA writes to a peer after this and none exits before all pairs addressed to it have landed
+  float a, b;
+  pair_totals(cs, parts, &pairs_in, a, b);
+  const float r_ = invstd[c];
+  const float inv_m = 1.0f / (static_cast<float>(sh.N) * static_cast<float>(sh.HW));
+  const float ds = b * r_, k_ = scale[c] * r_, am = a * inv_m, bm = ds * r_ * inv_m;
+  if (rank == 0 && threadIdx.x == 0) {
+    dscale[c] = ds;
+    dbias[c] = a;
+  }
+  release_dependents();
+  UnitWalk w(first, T, upp);
+  for (int u = first; u < u1; u += T, w.next()) {
+    const RaggedUnit r(w.n * plane_stride + chan_off, w.q, sh.HW);
+    if (!r.valid) continue;
+    const int l = (u - u0) * 4;
+    Vec4f vx, vg, o;
+    vx.u = *reinterpret_cast<const uint4*>(sx + l);
+    vg.u = *reinterpret_cast<const uint4*>(sg + l);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.f[j] = k_ * (vg.f[j] - am - (vx.f[j] - mu) * bm);
+    ragged_store(dx, r, o);
+  }
+}
+
+// Two passes over the same units, for channels that no cluster holds.
+template <int MASK>
+__global__ void __launch_bounds__(kBlock, 4)
+bn_bwd_ragged_reduce_kernel(const float* __restrict__ x, const float* __restrict__ dy,
+                            const float* __restrict__ relu_in, const float* __restrict__ mean,
+                            float2* __restrict__ partial, BnShape sh, int per_slice, size_t numel) {
+  __shared__ float sm[2 * kBlock / 32];
+  constexpr int kFlight = MASK == 1 ? 2 : 4;         // units of each operand in flight
+  const int c = blockIdx.y, slice = blockIdx.x;
+  dependency_wait();
+  release_dependents();
+  const float mu = mean[c];
+  const int upp = ragged_units(sh.HW), total = sh.N * upp;
+  const int i0 = slice * per_slice, i1 = min(i0 + per_slice, total);
+  const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
+  float s_dy = 0.f, s_dyx = 0.f;
+  UnitWalk w(i0 + threadIdx.x, kBlock, upp);
+  for (int i = i0 + threadIdx.x; i < i1;) {
+    Vec4f vx[kFlight], vg[kFlight], vm[kFlight];
+    unsigned valid[kFlight], bits[kFlight];
+#pragma unroll
+    for (int k = 0; k < kFlight; ++k) {
+      valid[k] = 0;
+      bits[k] = 15u;
+      if (i < i1) {
+        const RaggedUnit r(w.n * plane_stride + chan_off, w.q, sh.HW);
+        valid[k] = r.valid;
+        if (r.valid) {
+          vx[k] = ragged_load(x, r.off, numel);
+          vg[k] = ragged_load(dy, r.off, numel);
+          if (MASK == 1) vm[k] = ragged_load(relu_in, r.off, numel);
+          if (MASK == 2) bits[k] = keep4<2>(relu_in, r.off);
+        }
+        i += kBlock;
+        w.next();
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kFlight; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (valid[k] >> j & 1u) {
+          float g = vg[k].f[j];
+          if (MASK == 1) g = vm[k].f[j] > 0 ? g : 0.0f;
+          if (MASK == 2) g = (bits[k] >> j) & 1u ? g : 0.0f;
+          s_dy += g;
+          s_dyx += g * (vx[k].f[j] - mu);
+        }
+  }
+  channel_sums<kBlock, true>(s_dy, s_dyx, sm);
+  if (threadIdx.x == 0) partial[static_cast<size_t>(c) * gridDim.x + slice] = make_float2(s_dy, s_dyx);
+}
+
+template <int MASK>
+__global__ void __launch_bounds__(kBlock, 4)
+bn_bwd_ragged_apply_kernel(const float* __restrict__ x, const float* __restrict__ dy,
+                           const float* __restrict__ relu_in, const float* __restrict__ scale,
+                           const float* __restrict__ mean, const float* __restrict__ invstd,
+                           const float2* __restrict__ partial, int slices, float* __restrict__ dx,
+                           float* __restrict__ dscale, float* __restrict__ dbias, BnShape sh, size_t numel) {
+  __shared__ float coef[4];
+  const int c = sh.C - 1 - blockIdx.y;               // descending: what the first pass touched last is still in L2
+  const int upp = ragged_units(sh.HW), total = sh.N * upp;
+  const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
+  const int unit0 = blockIdx.x * (kBlock * kApplyUnits) + threadIdx.x;
+  Vec4f vx[kApplyUnits], vg[kApplyUnits];
+  UnitWalk w(min(unit0, total - 1), kBlock, upp);
+  UnitWalk w2 = w;
+  dependency_wait();
+#pragma unroll
+  for (int j = 0; j < kApplyUnits; ++j) {
+    vx[j].u = vg[j].u = make_uint4(0, 0, 0, 0);
+    if (unit0 + j * kBlock < total) {
+      const RaggedUnit r(w.n * plane_stride + chan_off, w.q, sh.HW);
+      if (r.valid) {
+        vx[j] = ragged_load(x, r.off, numel);
+        vg[j] = ragged_load(dy, r.off, numel);
+        unsigned bits = 15u;
+        Vec4f vm;
+        if (MASK == 1) vm = ragged_load(relu_in, r.off, numel);
+        if (MASK == 2) bits = keep4<2>(relu_in, r.off);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (MASK == 1) vg[j].f[k] = vm.f[k] > 0 ? vg[j].f[k] : 0.0f;
+          if (MASK == 2) vg[j].f[k] = (bits >> k) & 1u ? vg[j].f[k] : 0.0f;
+        }
+      }
+      w.next();
+    }
+  }
+  if (threadIdx.x < 32) {
+    float a = 0.f, b = 0.f;
+    for (int k = threadIdx.x; k < slices; k += 32) {
+      const float2 p = partial[static_cast<size_t>(c) * slices + k];
+      a += p.x;
+      b += p.y;
+    }
+    a = warp_sum(a);
+    b = warp_sum(b);
+    if (threadIdx.x == 0) {
+      const float r = invstd[c];
+      const float inv_m = 1.0f / (static_cast<float>(sh.N) * static_cast<float>(sh.HW));
+      const float ds = b * r;
+      coef[0] = scale[c] * r;
+      coef[1] = a * inv_m;
+      coef[2] = ds * r * inv_m;
+      coef[3] = mean[c];
+      if (blockIdx.x == 0) {
+        dscale[c] = ds;
+        dbias[c] = a;
+      }
+    }
+  }
+  __syncthreads();
+  release_dependents();
+  const float k_ = coef[0], am = coef[1], bm = coef[2], mu = coef[3];
+#pragma unroll
+  for (int j = 0; j < kApplyUnits; ++j) {
+    if (unit0 + j * kBlock >= total) break;
+    const RaggedUnit r(w2.n * plane_stride + chan_off, w2.q, sh.HW);
+    w2.next();
+    if (!r.valid) continue;
+    Vec4f o;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o.f[i] = k_ * (vg[j].f[i] - am - (vx[j].f[i] - mu) * bm);
+    ragged_store(dx, r, o);
+  }
+}
+
+template <int MASK, int T>
+int launch_ragged_t(const float* x, const float* dy, const float* relu_in, const float* scale, const float* mean,
+                    const float* invstd, float* dx, float* dscale, float* dbias, BnShape sh, int cs, int per_cta,
+                    cudaStream_t s) {
+  auto kernel = bn_bwd_ragged_kernel<MASK, T>;
+  static std::atomic<bool> attr_set[64];
+  const int ready = opt_in_once(kernel, attr_set, true);
+  if (ready != SGB_OK) return ready;
+  return launch_ex(kernel, dim3(static_cast<unsigned>(sh.C) * cs), dim3(T), static_cast<size_t>(per_cta) * 32, s, cs,
+                   true, x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, per_cta,
+                   static_cast<size_t>(sh.N) * sh.C * sh.HW);
+}
+// One pass with a cluster where the channel fits one, else two passes.
+template <int MASK>
+int launch_ragged(const float* x, const float* dy, const float* relu_in, const float* scale, const float* mean,
+                  const float* invstd, float* dx, float* dscale, float* dbias, BnShape sh, void* ws, size_t ws_bytes,
+                  cudaStream_t s) {
+  const int total = sh.N * ragged_units(sh.HW);
+  int per_cta = 0;
+  const int cs = cluster_plan(total, 32, 8192, &per_cta, sh.C);
+  if (cs > 0 && static_cast<long long>(sh.C) * cs <= 0x7fffffffLL)
+    return per_cta > 2048 ? launch_ragged_t<MASK, 512>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, cs,
+                                                       per_cta, s)
+                          : launch_ragged_t<MASK, 256>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, cs,
+                                                       per_cta, s);
+  const size_t numel = static_cast<size_t>(sh.N) * sh.C * sh.HW;
+  const int slices = bn_slices_for(static_cast<long long>(sh.N) * sh.HW, sh.C, sm_count());
+  if (!ws || ws_bytes < static_cast<size_t>(slices) * sh.C * sizeof(float2) || !aligned16(ws)) return SGB_ERR_WORKSPACE;
+  float2* partial = static_cast<float2*>(ws);
+  const int st = launch_ex(bn_bwd_ragged_reduce_kernel<MASK>, dim3(slices, sh.C), dim3(kBlock), 0, s, 0, true, x, dy,
+                           relu_in, mean, partial, sh, static_cast<int>(ceil_div(total, slices)), numel);
+  if (st != SGB_OK) return st;
+  return launch_ex(bn_bwd_ragged_apply_kernel<MASK>,
+                   dim3(static_cast<unsigned>(ceil_div(total, kBlock * kApplyUnits)), sh.C), dim3(kBlock), 0, s, 0, true,
+                   x, dy, relu_in, scale, mean, invstd, static_cast<const float2*>(partial), slices, dx, dscale, dbias,
+                   sh, numel);
 }
 
 template <bool VEC, int MASK, int T, bool ADD = false>
@@ -840,18 +1155,38 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
   const bool vec = (HW % 4 == 0) && aligned16(x) && aligned16(dy) && aligned16(dx) &&
                    (MASK != 1 || aligned16(relu_in));
   const BnShape sh{N, C, HW};
-  if (!vec && HW > 1 && aligned16(x) && aligned16(dy) && aligned16(dx) && (MASK != 1 || aligned16(relu_in))) {
-    // odd planes: groups of adjacent channels make 16-byte runs (7x7 layers)
-    const int G = (HW % 2) ? 4 : 2;
-    if ((HW * G) % 4 == 0 && C % G == 0 && static_cast<long long>(G) * per_channel * 8 <= 100 * 1024) {
+  const bool bases_aligned = aligned16(x) && aligned16(dy) && aligned16(dx) && (MASK != 1 || aligned16(relu_in));
+  // groups of G adjacent channels make 16-byte runs of odd planes (7x7 layers)
+  const int G = (HW % 2) ? 4 : 2;
+  const bool groups = !vec && HW > 1 && bases_aligned && (HW * G) % 4 == 0 && C % G == 0 &&
+                      static_cast<long long>(G) * per_channel * 8 <= 100 * 1024;
+  // Channels that fit a CTA's registers need no staging.  Where that means
+  // scalar accesses, the group form still wins once the call is bound by bytes
+  // and not by latency and no mask has to be formed (32x2048x7x7: 12.9 against
+  // 13.3 us; 32x512x7x7: 5.7 against 4.5; with ReLU 16.8 against 13.7).
+  if (!(groups && MASK == 0 && per_channel * C > 2000000LL)) {
+    int st = SGB_OK;
+    auto go = [&](auto g, auto nv, auto v) {
+      st = launch_small<MASK, decltype(g)::value, decltype(nv)::value, decltype(v)::value>(
+          x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, s);
+    };
+    if (vec ? small_plan<true, 6>(per_channel / 4, [&](auto g, auto nv) { go(g, nv, std::true_type{}); })
+            : small_plan<false, 6>(per_channel, [&](auto g, auto nv) { go(g, nv, std::false_type{}); }))
+      return st;
+  }
+  if (!vec && HW > 1 && bases_aligned) {
+    if (groups) {
       if (G == 4)
         return launch_group<MASK, 4>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, s);
       return launch_group<MASK, 2>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, s);
     }
+    // below eight elements a plane has more edge units than whole ones
+    if (HW >= 8 && static_cast<long long>(N) * ragged_units(HW) <= 0x7fffffffLL)
+      return launch_ragged<MASK>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, ws, ws_bytes, s);
   }
   {
     int per_cta = 0;
-    const int cs = cluster_plan(vec ? per_channel / 4 : per_channel, vec ? 16 : 4, &per_cta, C);
+    const int cs = cluster_plan(vec ? per_channel / 4 : per_channel, vec ? 32 : 8, 8192, &per_cta, C);
     if (cs > 0 && static_cast<long long>(C) * cs <= 0x7fffffffLL) {
       return vec ? launch_cluster<true, MASK>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias,
                                               sh, cs, per_cta, s)
@@ -905,11 +1240,18 @@ int bn_add_relu_backward(const float* x, const float* dy_a, const float* dy_b, c
   const bool vec = (HW % 4 == 0) && aligned16(x) && aligned16(dy_a) && aligned16(dy_b) &&
                    aligned16(relu_in) && aligned16(joined) && aligned16(dx);
   if (vec) {
+    const BnShape sh{N, C, HW};
+    cudaStream_t s = as_stream(stream);
+    // the same forms as without the join (same sums, bit for bit)
+    int st = SGB_OK;
+    if (small_plan<true, 6>(per_channel / 4, [&](auto g, auto nv) {
+          st = launch_small<3, decltype(g)::value, decltype(nv)::value, true>(
+              x, dy_a, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, s, dy_b, joined);
+        }))
+      return st;
     int per_cta = 0;
-    const int cs = cluster_plan(per_channel / 4, 16, &per_cta, C);
+    const int cs = cluster_plan(per_channel / 4, 32, 8192, &per_cta, C);
     if (cs > 0 && static_cast<long long>(C) * cs <= 0x7fffffffLL) {
-      const BnShape sh{N, C, HW};
-      cudaStream_t s = as_stream(stream);
       if (per_cta > 2048)
         return launch_cluster_t<true, true, 512, true>(x, dy_a, relu_in, scale, mean, invstd, dx, dscale,
                                                        dbias, sh, cs, per_cta, s, dy_b, joined);
@@ -921,231 +1263,6 @@ int bn_add_relu_backward(const float* x, const float* dy_a, const float* dy_b, c
   if (st != SGB_OK) return st;
   return bn_backward<0>(x, joined, nullptr, scale, mean, invstd, dx, dscale, dbias, N, C, HW, ws,
                         ws_bytes, stream);
-}
-
-// ------------------------------------------------------------ forward (training)
-// Forward partner of the backward kernels: batch statistics, normalisation and
-// running-statistics update in one pass over x.  A cluster stages its channel
-// in shared memory once; mean and the centred sum of squares are two reductions
-// over the staged copy (no E[x^2]-E[x]^2 cancellation), each exchanged through
-// distributed shared memory.  Emits what the backward consumes: save_mean and
-// save_invstd = 1/sqrt(biased_var + eps).  Running statistics follow cuDNN:
-// r = (1-f)*r + f*batch_value, with the UNBIASED variance (M/(M-1)).
-template <bool VEC, int T>
-__global__ void __launch_bounds__(T)
-bn_fwd_cluster_kernel(const float* __restrict__ x, const float* __restrict__ scale,
-                      const float* __restrict__ bias, float* __restrict__ running_mean,
-                      float* __restrict__ running_var, float factor, float eps,
-                      float* __restrict__ y, float* __restrict__ save_mean,
-                      float* __restrict__ save_invstd, BnShape sh, int per_cta) {
-  extern __shared__ __align__(16) float stage[];
-  __shared__ float red[T / 32];
-  __shared__ float parts[2][16];
-  cg::cluster_group cluster = cg::this_cluster();
-  const int cs = static_cast<int>(cluster.num_blocks());
-  const int rank = static_cast<int>(cluster.block_rank());
-  const int c = blockIdx.x / cs;
-  cluster.barrier_arrive();
-  constexpr int kW = VEC ? 4 : 1;
-  const int hwu = sh.HW / kW, total = sh.N * hwu;
-  const int u0 = min(rank * per_cta, total), u1 = min(u0 + per_cta, total);
-  const int first = u0 + threadIdx.x;
-  const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW;
-  const size_t chan_off = static_cast<size_t>(c) * sh.HW;
-  {
-    UnitWalk w(first, T, hwu);
-    for (int u = first; u < u1; u += T, w.next()) {
-      const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * kW;
-      if (VEC) cp_async16(stage + (u - u0) * 4, x + off);
-      else stage[u - u0] = x[off];
-    }
-  }
-  if (VEC) cp_async_wait_all();
-  const float inv_m = 1.0f / (static_cast<float>(sh.N) * static_cast<float>(sh.HW));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int kWarps = T / 32;
-  auto cluster_total = [&](float v, int slot) -> float {
-    v = warp_sum(v);
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-      float p = lane < kWarps ? red[lane] : 0.0f;
-      p = warp_sum(p);
-      if (slot == 0) cluster.barrier_wait();      // first exchange: peers must have started
-      if (lane < cs) *cluster.map_shared_rank(&parts[slot][rank], lane) = p;
-    } else if (slot == 0) {
-      cluster.barrier_wait();
-    }
-    cluster.sync();
-    float t = 0.f;
-    for (int r = 0; r < cs; ++r) t += parts[slot][r];
-    return t;
-  };
-  float s = 0.f;
-  for (int u = first; u < u1; u += T) {
-    const int l = (u - u0) * kW;
-#pragma unroll
-    for (int k = 0; k < kW; ++k) s += stage[l + k];
-  }
-  const float mu = cluster_total(s, 0) * inv_m;
-  float q = 0.f;
-  for (int u = first; u < u1; u += T) {
-    const int l = (u - u0) * kW;
-#pragma unroll
-    for (int k = 0; k < kW; ++k) {
-      const float d = stage[l + k] - mu;
-      q += d * d;
-    }
-  }
-  const float var = cluster_total(q, 1) * inv_m;      // biased
-  const float invstd = 1.0f / sqrtf(var + eps);
-  if (rank == 0 && threadIdx.x == 0) {
-    save_mean[c] = mu;
-    save_invstd[c] = invstd;
-    const float m = static_cast<float>(sh.N) * static_cast<float>(sh.HW);
-    const float unbiased = m > 1.0f ? var * (m / (m - 1.0f)) : var;
-    running_mean[c] = (1.0f - factor) * running_mean[c] + factor * mu;
-    running_var[c] = (1.0f - factor) * running_var[c] + factor * unbiased;
-  }
-  const float g = scale[c] * invstd, b = bias[c];
-  {
-    UnitWalk w(first, T, hwu);
-    for (int u = first; u < u1; u += T, w.next()) {
-      const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * kW;
-      const int l = (u - u0) * kW;
-      if (VEC) {
-        Vec4f v, o;
-        v.u = *reinterpret_cast<const uint4*>(stage + l);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) o.f[k] = (v.f[k] - mu) * g + b;
-        st128(y + off, o.u);
-      } else {
-        y[off] = (stage[l] - mu) * g + b;
-      }
-    }
-  }
-}
-
-// Fallback for channels that do not fit a cluster: three streaming kernels
-// (mean partials, centred-square partials, normalise), partials in workspace.
-template <int PHASE>
-__global__ void __launch_bounds__(kBlock)
-bn_fwd_partial_kernel(const float* __restrict__ x, const float* __restrict__ mean_in,
-                      float* __restrict__ partial, BnShape sh, int per_slice) {
-  __shared__ float sm[32];
-  const int c = blockIdx.y, slice = blockIdx.x;
-  const int total = sh.N * sh.HW;
-  const int i0 = slice * per_slice, i1 = min(i0 + per_slice, total);
-  const float mu = PHASE == 1 ? mean_in[c] : 0.0f;
-  float acc = 0.f;
-  UnitWalk w(i0 + threadIdx.x, kBlock, sh.HW);
-  for (int i = i0 + threadIdx.x; i < i1; i += kBlock, w.next()) {
-    const float v = x[(static_cast<size_t>(w.n) * sh.C + c) * sh.HW + w.q];
-    acc += PHASE == 0 ? v : (v - mu) * (v - mu);
-  }
-  acc = block_sum(acc, sm);
-  if (threadIdx.x == 0) partial[static_cast<size_t>(c) * gridDim.x + slice] = acc;
-}
-
-__global__ void bn_fwd_finish_kernel(int phase, const float* __restrict__ partial, int slices,
-                                     float* __restrict__ save_mean, float* __restrict__ save_invstd,
-                                     float* __restrict__ running_mean, float* __restrict__ running_var,
-                                     float factor, float eps, BnShape sh) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= sh.C) return;
-  float t = 0.f;
-  for (int k = 0; k < slices; ++k) t += partial[static_cast<size_t>(c) * slices + k];
-  const float m = static_cast<float>(sh.N) * static_cast<float>(sh.HW);
-  if (phase == 0) {
-    save_mean[c] = t / m;
-  } else {
-    const float var = t / m;
-    save_invstd[c] = 1.0f / sqrtf(var + eps);
-    const float unbiased = m > 1.0f ? var * (m / (m - 1.0f)) : var;
-    running_mean[c] = (1.0f - factor) * running_mean[c] + factor * save_mean[c];
-    running_var[c] = (1.0f - factor) * running_var[c] + factor * unbiased;
-  }
-}
-
-__global__ void __launch_bounds__(kBlock)
-bn_fwd_normalize_kernel(const float* __restrict__ x, const float* __restrict__ scale,
-                        const float* __restrict__ bias, const float* __restrict__ mean,
-                        const float* __restrict__ invstd, float* __restrict__ y, BnShape sh) {
-  const int c = blockIdx.y;
-  const int i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= sh.N * sh.HW) return;
-  const int n = i / sh.HW, q = i - n * sh.HW;
-  const size_t off = (static_cast<size_t>(n) * sh.C + c) * sh.HW + q;
-  y[off] = (x[off] - mean[c]) * (scale[c] * invstd[c]) + bias[c];
-}
-
-template <bool VEC, int T>
-int launch_fwd_cluster(const float* x, const float* scale, const float* bias, float* rm, float* rv,
-                       float factor, float eps, float* y, float* sm_, float* si, BnShape sh, int cs,
-                       int per_cta, cudaStream_t s) {
-  auto kernel = bn_fwd_cluster_kernel<VEC, T>;
-  const size_t smem = static_cast<size_t>(per_cta) * (VEC ? 16 : 4);
-  static std::atomic<bool> attr_set[64];
-  const int ready = opt_in_once(kernel, attr_set, false);
-  if (ready != SGB_OK) return ready;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(sh.C) * cs);
-  cfg.blockDim = dim3(T);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cs;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, x, scale, bias, rm, rv, factor, eps, y, sm_, si, sh, per_cta);
-  if (e != cudaSuccess) return note_cuda_error(e);
-  return launch_status();
-}
-
-int bn_forward_training(const float* x, const float* scale, const float* bias, float* rm, float* rv,
-                        float factor, float eps, float* y, float* save_mean, float* save_invstd,
-                        int N, int C, int HW, void* ws, size_t ws_bytes, void* stream) {
-  if (N < 0 || C < 0 || HW < 0) return SGB_ERR_SIZE;
-  if (N == 0 || C == 0 || HW == 0) return SGB_OK;
-  if (!x || !scale || !bias || !rm || !rv || !y || !save_mean || !save_invstd) return SGB_ERR_NULL;
-  const long long per_channel = static_cast<long long>(N) * HW;
-  if (per_channel > 0x7fffffffLL || C > 65535) return SGB_ERR_SIZE;
-  cudaStream_t s = as_stream(stream);
-  const BnShape sh{N, C, HW};
-  const bool vec = (HW % 4 == 0) && aligned16(x) && aligned16(y);
-  // x only is staged: a share of `units` units costs units * unit_bytes
-  const long long units = vec ? per_channel / 4 : per_channel;
-  const int unit_bytes = vec ? 16 : 4;
-  for (int pass = 0; pass < 2; ++pass) {
-    const long long cap = pass == 0 ? 50 * 1024 : 100 * 1024;
-    for (int cs = 1; cs <= 8; cs *= 2) {
-      const long long share = (units + cs - 1) / cs;
-      if (share * unit_bytes <= cap) {
-        const int per_cta = static_cast<int>(share);
-        if (vec)
-          return share > 2048
-                     ? launch_fwd_cluster<true, 512>(x, scale, bias, rm, rv, factor, eps, y, save_mean, save_invstd, sh, cs, per_cta, s)
-                     : launch_fwd_cluster<true, 256>(x, scale, bias, rm, rv, factor, eps, y, save_mean, save_invstd, sh, cs, per_cta, s);
-        return launch_fwd_cluster<false, 256>(x, scale, bias, rm, rv, factor, eps, y, save_mean, save_invstd, sh, cs, per_cta, s);
-      }
-    }
-  }
-  const int slices = bn_slices_for(per_channel, C, sm_count());
-  if (!ws || ws_bytes < static_cast<size_t>(slices) * C * sizeof(float)) return SGB_ERR_WORKSPACE;
-  float* partial = static_cast<float*>(ws);
-  const int per_slice = static_cast<int>(ceil_div(static_cast<size_t>(per_channel), slices));
-  const dim3 g1(slices, C);
-  const unsigned fb = static_cast<unsigned>(ceil_div(C, 128));
-  bn_fwd_partial_kernel<0><<<g1, kBlock, 0, s>>>(x, nullptr, partial, sh, per_slice);
-  bn_fwd_finish_kernel<<<fb, 128, 0, s>>>(0, partial, slices, save_mean, save_invstd, rm, rv, factor, eps, sh);
-  bn_fwd_partial_kernel<1><<<g1, kBlock, 0, s>>>(x, save_mean, partial, sh, per_slice);
-  bn_fwd_finish_kernel<<<fb, 128, 0, s>>>(1, partial, slices, save_mean, save_invstd, rm, rv, factor, eps, sh);
-  bn_fwd_normalize_kernel<<<dim3(static_cast<unsigned>(ceil_div(static_cast<size_t>(per_channel), kBlock)), C),
-                            kBlock, 0, s>>>(x, scale, bias, save_mean, save_invstd, y, sh);
-  return launch_status();
 }
 
 // ------------------------------------------------ variant with built-in scratch
@@ -1235,7 +1352,10 @@ int sgb_bn_backward_faults(unsigned* flags) {
   if (st != SGB_OK) return st;
   cudaError_t e = cudaMemcpyFromSymbol(&cluster, g_cluster_faults, sizeof(unsigned));
   if (e != cudaSuccess) return note_cuda_error(e);
-  *flags = streaming | (cluster << 8);
+  unsigned forward = 0;
+  const int fs = bn_forward_faults(&forward);
+  if (fs != SGB_OK) return fs;
+  *flags = streaming | (cluster << 8) | (forward << 16);
   return SGB_OK;
 }
 
@@ -1266,14 +1386,6 @@ int sgb_bn_add_relu_backward_f32(const float* x, const float* dy_a, const float*
                                  void* stream) {
   return bn_add_relu_backward(x, dy_a, dy_b, relu_in, scale, mean, invstd, joined, dx, dscale, dbias, N,
                               C, HW, ws, ws_bytes, stream);
-}
-
-int sgb_bn_forward_training_f32(const float* x, const float* scale, const float* bias,
-                                float* running_mean, float* running_var, float factor, float eps,
-                                float* y, float* save_mean, float* save_invstd, int N, int C,
-                                int HW, void* ws, size_t ws_bytes, void* stream) {
-  return bn_forward_training(x, scale, bias, running_mean, running_var, factor, eps, y, save_mean,
-                             save_invstd, N, C, HW, ws, ws_bytes, stream);
 }
 
 int sgb_bn_backward_noalloc_f32(const float* x, const float* dy, const float* scale,
