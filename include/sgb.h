@@ -641,8 +641,8 @@ int sgb_comm_fused_synch_half(sgb_comm *c, void *const *tensors,
 /* Communicator::sparsification / fusedSparsification (communicator.cc:
  * 469-617) -> valSparsAllReduce / topKSparsAllReduce (:619-807).  count == 1
  * is the single-tensor form.  accumulation (device, total size) may be NULL.
- * topk == 0: spars is the magnitude threshold; the call blocks the host until
- * the per-rank counts have arrived (as the reference does).  topk != 0: spars
+ * topk == 0: spars is the magnitude threshold; with more than one rank the call
+ * blocks the host until the per-rank counts have arrived (as the reference does).  topk != 0: spars
  * is the fraction of elements sent; fully asynchronous. */
 int sgb_comm_sparsification(sgb_comm *c, void *const *tensors,
                             const size_t *sizes, size_t count,

@@ -77,6 +77,8 @@ struct sgb_comm {
     int* nnz_host = nullptr;     // pinned, world entries
     cudaEvent_t selected = nullptr;  // behind the selection on c1
     cudaEvent_t counted = nullptr;   // behind the counts' copy to the host
+    cudaEvent_t consumed = nullptr;  // behind the dense sum on c2 that read pay_send (one rank)
+    bool in_use = false;             // that sum has not been joined by a wait() yet
     size_t n = 0, nnz_max = 0, capacity = 0;
     int topk = 0;
     const char* op_name = "";
@@ -232,6 +234,15 @@ void defer(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count,
   }
 }
 
+// One rank, and the flush hands back exactly the tensors that were staged.
+bool alone(const sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count, size_t total, int half) {
+  if (c->world != 1 || c->pend_half != half || c->pend_off != 0 || c->pend_ptrs.size() != count || c->send_off != total)
+    return false;
+  for (size_t i = 0; i < count; ++i)
+    if (c->pend_ptrs[i] != tensors[i] || c->pend_sizes[i] != sizes[i]) return false;
+  return true;
+}
+
 int half_init(sgb_comm* c) {
   if (c->send_h) return SGB_OK;
   CU(cudaMalloc(&c->send_h, c->max_elems * sizeof(__half)));
@@ -242,7 +253,7 @@ int half_init(sgb_comm* c) {
 }
 
 int sparse_init(sgb_comm* c) {
-  if (c->pay_recv) return SGB_OK;
+  if (c->dropped_dev) return SGB_OK;
   const size_t n = c->max_elems;
   c->ws_bytes = sgb_sparse_workspace_bytes(n);
   CU(cudaMalloc(&c->ws, c->ws_bytes));
@@ -254,8 +265,9 @@ int sparse_init(sgb_comm* c) {
     // blocking wait woke it 50-100 us late
     CU(cudaEventCreateWithFlags(&x.selected, cudaEventDisableTiming));
     CU(cudaEventCreateWithFlags(&x.counted, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&x.consumed, cudaEventDisableTiming));
   }
-  CU(cudaMalloc(&c->pay_recv, 2 * n * sizeof(int) * static_cast<size_t>(c->world)));
+  if (c->world > 1) CU(cudaMalloc(&c->pay_recv, 2 * n * sizeof(int) * static_cast<size_t>(c->world)));
   CU(cudaMalloc(&c->dropped_dev, sizeof(unsigned long long)));
   CU(cudaMemset(c->dropped_dev, 0, sizeof(unsigned long long)));
   return SGB_OK;
@@ -359,6 +371,7 @@ int sgb_comm_destroy(sgb_comm* c) {
     if (x.nnz_host) cudaFreeHost(x.nnz_host);
     if (x.selected) cudaEventDestroy(x.selected);
     if (x.counted) cudaEventDestroy(x.counted);
+    if (x.consumed) cudaEventDestroy(x.consumed);
   }
   if (c->dropped_dev) cudaFree(c->dropped_dev);
   drop_ranges(c);
@@ -414,6 +427,7 @@ void* sgb_comm_stream(const sgb_comm* c, int which) {
 int sgb_comm_wait(sgb_comm* c, void* compute_stream) {
   if (!c) return SGB_ERR_NULL;
   if (c->sparse_begun != c->sparse_ended) return SGB_ERR_STATE;   // an exchange is still to be ended
+  for (sgb_comm::Sparse& x : c->sparse) x.in_use = false;          // c2 is joined here
   return emit(c, plan_call(c, sgb::order::kWait).before, sgb::as_stream(compute_stream));
 }
 
@@ -567,6 +581,19 @@ int sgb_comm_fused_synch(sgb_comm* c, void* const* tensors, const size_t* sizes,
   }
   const sgb::order::Step p = plan_call(c, sgb::order::kFlushPacked);
   OK(emit(c, p.pre, compute));
+  if (alone(c, tensors, sizes, count, total, 0)) {
+    // One rank: the tensors hold their sum already.  Streams, events and phases
+    // are those of any world size; nothing is packed, reduced or copied back.
+    c->pend_ptrs.clear();
+    c->pend_sizes.clear();
+    c->send_off = 0;
+    { Phase ph(c, "Dist_c1_fusedSynch_filling", sgb::order::kStreamC1); }
+    OK(emit(c, p.before, compute));
+    { Phase ph(c, "Dist_s_fusedSynch_allreduce", sgb::order::kStreamS); }
+    OK(emit(c, p.after, nullptr));
+    Phase ph(c, "Dist_c1_fusedSynch_copyBackToTensor", sgb::order::kStreamC1);
+    return SGB_OK;
+  }
   OK(pack_pending(c, "Dist_c1_fusedSynch_filling"));
   OK(emit(c, p.before, compute));
   if (c->send_off) {
@@ -598,20 +625,27 @@ int sgb_comm_synch_half(sgb_comm* c, float* data, size_t n, void* compute_stream
   OK(half_init(c));
   cudaStream_t compute = sgb::as_stream(compute_stream);
   const sgb::order::Step p = plan_call(c, sgb::order::kSynchHalf);
+  const bool one = c->world == 1;     // the sum of one rank's fp16 values is those values: round in place
   OK(emit(c, p.pre, compute));
   {
     Phase ph(c, "Dist_c1_synchHalf_float2half", sgb::order::kStreamC1);
-    OK(sgb_cast_f32_f16(data, c->dsend_h, n, c->c1));
+    if (one) {
+      void* const t[1] = {data};
+      const size_t sz[1] = {n};
+      OK(sgb::round_f16_multi(t, sz, 1, c->c1));
+    } else {
+      OK(sgb_cast_f32_f16(data, c->dsend_h, n, c->c1));
+    }
   }
   OK(emit(c, p.before, compute));
   {
     Phase ph(c, "Dist_s_synchHalf_allreduce", sgb::order::kStreamS);
-    NC(ncclAllReduce(c->dsend_h, c->drecv_h, n, ncclHalf, ncclSum, c->nccl, c->s));
+    if (!one) NC(ncclAllReduce(c->dsend_h, c->drecv_h, n, ncclHalf, ncclSum, c->nccl, c->s));
   }
   OK(emit(c, p.after, nullptr));
   {
     Phase ph(c, "Dist_c2_synchHalf_half2float", sgb::order::kStreamC2);
-    OK(sgb_cast_f16_f32(c->drecv_h, data, n, c->c2));
+    if (!one) OK(sgb_cast_f16_f32(c->drecv_h, data, n, c->c2));
   }
   return emit(c, p.post, nullptr);
 }
@@ -634,8 +668,18 @@ int sgb_comm_fused_synch_half(sgb_comm* c, void* const* tensors, const size_t* s
   }
   if (total > c->max_elems) return SGB_ERR_CAPACITY;
   const sgb::order::Step p = plan_call(c, sgb::order::kFlushHalf);
+  const bool one = alone(c, tensors, sizes, count, total, 1);
   OK(emit(c, p.pre, compute));
-  OK(pack_pending(c, "Dist_c1_fusedSynchHalf_float2half"));
+  if (one) {
+    // one rank: rounded where they are, see sgb_comm_synch_half
+    c->pend_ptrs.clear();
+    c->pend_sizes.clear();
+    c->send_off = 0;
+    Phase ph(c, "Dist_c1_fusedSynchHalf_float2half", sgb::order::kStreamC1);
+    OK(sgb::round_f16_multi(tensors, sizes, count, c->c1));
+  } else {
+    OK(pack_pending(c, "Dist_c1_fusedSynchHalf_float2half"));
+  }
   OK(emit(c, p.before, compute));
   if (c->send_off) {
     Phase ph(c, "Dist_s_fusedSynchHalf_allreduce", sgb::order::kStreamS);
@@ -645,7 +689,7 @@ int sgb_comm_fused_synch_half(sgb_comm* c, void* const* tensors, const size_t* s
   OK(emit(c, p.after, nullptr));
   {
     Phase ph(c, "Dist_c2_fusedSynchHalf_half2floatcopy", sgb::order::kStreamC2);
-    OK(sgb_unpack_f16_to_f32(c->recv_h, 0, tensors, sizes, count, 1.0f, c->c2));
+    if (!one) OK(sgb_unpack_f16_to_f32(c->recv_h, 0, tensors, sizes, count, 1.0f, c->c2));
   }
   return emit(c, p.post, nullptr);
 }
@@ -676,6 +720,7 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
   }
   if (n) {
     OK(emit(c, plan_call(c, sgb::order::kSparseSelect).pre, sgb::as_stream(compute_stream)));
+    if (x.in_use) CU(cudaStreamWaitEvent(c->c1, x.consumed, 0));
     // One tensor, or tensors that lie back to back in memory (a gradient arena),
     // are selected from IN PLACE: no copy into the send buffer.
     bool in_place = sgb::aligned16(tensors[0]);
@@ -695,7 +740,10 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
       OK(sgb::sparse_threshold_bounded(grad, accumulation, n, spars, x.pay_send, capacity, x.nnz_dev, c->dropped_dev,
                                        c->ws, c->ws_bytes, c->c1));
       // the counts travel on the device only; receivers clamp them to the capacity
-      NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
+      if (c->world > 1) NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
+    } else if (c->world == 1) {
+      // nobody to tell: the dense sum reads the payload and its count where they are
+      OK(sgb::sparse_threshold_packed(grad, accumulation, n, spars, x.pay_send, x.nnz_dev, c->ws, c->ws_bytes, c->c1));
     } else {
       OK(sgb::sparse_threshold_packed(grad, accumulation, n, spars, x.pay_send, x.nnz_dev, c->ws, c->ws_bytes, c->c1));
       NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
@@ -715,7 +763,7 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
   sgb_comm::Sparse& x = c->sparse[c->sparse_ended++ & 1];
   if (x.n == 0) return SGB_OK;
   const int W = c->world;
-  if (!x.topk && !x.capacity) {
+  if (!x.topk && !x.capacity && W > 1) {
     CU(cudaEventSynchronize(x.counted));
     for (int r = 0; r < W; ++r) {
       if (x.nnz_host[r] < 0 || static_cast<size_t>(x.nnz_host[r]) > x.n) return SGB_ERR_STATE;
@@ -726,15 +774,20 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
   // s waits for this exchange's own selection, not for what c1 was given since
   CU(cudaStreamWaitEvent(c->s, x.selected, 0));
   OK(emit(c, p.before & ~static_cast<unsigned>(sgb::order::kC1ToS), sgb::as_stream(compute_stream)));
-  if (x.nnz_max) {
+  {
     Phase ph(c, "Dist_s_sparsification_allgather", sgb::order::kStreamS);
-    NC(ncclAllGather(x.pay_send, c->pay_recv, 2 * x.nnz_max, ncclFloat, c->nccl, c->s));
+    if (W > 1 && x.nnz_max) NC(ncclAllGather(x.pay_send, c->pay_recv, 2 * x.nnz_max, ncclFloat, c->nccl, c->s));
   }
   OK(emit(c, p.after, nullptr));
   {
     Phase ph(c, x.op_name, sgb::order::kStreamC2);
     const size_t stride = 2 * x.nnz_max;
-    if (W <= sgb::kMaxDenseRanks) {
+    if (W == 1) {
+      OK(sgb::sparse_dense_sum(x.pay_send, 0, x.capacity, x.nnz_host, x.topk ? nullptr : x.nnz_dev, 1, x.tensors.data(),
+                               x.sizes.data(), x.tensors.size(), c->c2));
+      CU(cudaEventRecord(x.consumed, c->c2));
+      x.in_use = true;
+    } else if (W <= sgb::kMaxDenseRanks) {
       OK(sgb::sparse_dense_sum(c->pay_recv, stride, x.capacity, x.nnz_host, x.capacity ? x.nnz_dev + 1 : nullptr, W,
                                x.tensors.data(), x.sizes.data(), x.tensors.size(), c->c2));
     } else {

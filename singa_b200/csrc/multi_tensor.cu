@@ -93,7 +93,9 @@ sgd_multi_kernel(const __grid_constant__ Table t, const SgdArgs a) {
   }
 }
 
-enum PackMode { kPackF32 = 0, kPackF32ToF16 = 1, kUnpackF32 = 2, kUnpackF16ToF32 = 3 };
+// kRoundF16: the tensors are rounded to fp16 and widened again where they are
+// (what packing, a one-rank all-reduce and unpacking do to them).
+enum PackMode { kPackF32 = 0, kPackF32ToF16 = 1, kUnpackF32 = 2, kUnpackF16ToF32 = 3, kRoundF16 = 4 };
 
 template <int MODE>
 __global__ void __launch_bounds__(kBlock)
@@ -106,8 +108,20 @@ pack_multi_kernel(const __grid_constant__ Table t, const __grid_constant__ Offse
   const size_t i = static_cast<size_t>(blockIdx.x - t.first_tile[k]) * kTile + 4 * threadIdx.x;
   if (i >= n) return;
   float* tensor = static_cast<float*>(t.a[k]);
-  const size_t fo = o.off[k] + i;
   const bool full = i + 4 <= n;
+  if (MODE == kRoundF16) {
+    if (full && (reinterpret_cast<uintptr_t>(tensor + i) & 15u) == 0) {
+      Vec4f v;
+      v.u = ld128(tensor + i);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v.f[j] = __half2float(__float2half_rn(v.f[j]));
+      st128(tensor + i, v.u);
+    } else {
+      for (size_t j = 0; j < 4 && i + j < n; ++j) tensor[i + j] = __half2float(__float2half_rn(tensor[i + j]));
+    }
+    return;
+  }
+  const size_t fo = o.off[k] + i;
   if (MODE == kPackF32 || MODE == kUnpackF32) {
     float* fl = static_cast<float*>(flat) + fo;
     const bool vec = full && ((reinterpret_cast<uintptr_t>(tensor + i) |
@@ -186,7 +200,7 @@ unsigned fill_table(Table& t, Offsets* o, void* const* a, void* const* b, void* 
 int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t count, void* flat,
                 size_t flat_offset, float scale, int use_scale, void* stream) {
   if (count == 0) return SGB_OK;
-  if (!tensors || !sizes || !flat) return SGB_ERR_NULL;
+  if (!tensors || !sizes || (!flat && mode != kRoundF16)) return SGB_ERR_NULL;
   cudaStream_t s = as_stream(stream);
   size_t off = flat_offset;
   for (size_t first = 0; first < count;) {
@@ -224,6 +238,7 @@ int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t coun
     auto kernel = mode == kPackF32        ? pack_multi_kernel<kPackF32>
                   : mode == kPackF32ToF16 ? pack_multi_kernel<kPackF32ToF16>
                   : mode == kUnpackF32    ? pack_multi_kernel<kUnpackF32>
+                  : mode == kRoundF16     ? pack_multi_kernel<kRoundF16>
                                           : pack_multi_kernel<kUnpackF16ToF32>;
     const int st = launch_ex(kernel, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, o, flat, scale, use_scale);
     if (st != SGB_OK) return st;
@@ -232,6 +247,11 @@ int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t coun
 }
 
 }  // namespace
+
+int round_f16_multi(void* const* tensors, const size_t* sizes, size_t count, cudaStream_t s) {
+  return pack_common(kRoundF16, tensors, sizes, count, nullptr, 0, 1.f, 0, s);
+}
+
 }  // namespace sgb
 
 using namespace sgb;

@@ -921,7 +921,8 @@ struct DenseArgs {
   const int* payload;          // rank r: [idx | val] at payload + r * stride
   size_t stride;
   size_t val_off;              // 0: the values follow the rank's own count
-  const int* counts_dev;       // counts on the device, clamped to val_off; null: counts[]
+  const int* counts_dev;       // counts on the device, clamped to most; null: counts[]
+  unsigned most;
   int world;
   int counts[kMaxDenseRanks];
   size_t first, last;          // element range of this launch
@@ -960,7 +961,7 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
   for (int r = threadIdx.x >> 5; r < a.world; r += kWarps) {
     int c = a.counts_dev ? a.counts_dev[r] : a.counts[r];
     if (c < 0) c = 0;
-    if (a.counts_dev && static_cast<size_t>(c) > a.val_off) c = static_cast<int>(a.val_off);
+    if (static_cast<unsigned>(c) > a.most) c = static_cast<int>(a.most);
     const unsigned at = warp_lower_bound(a.payload + r * a.stride, static_cast<unsigned>(c),
                                          static_cast<long long>(begin) + 1);
     if ((threadIdx.x & 31) == 0) {
@@ -1102,6 +1103,9 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
   a.stride = stride;
   a.val_off = val_off;
   a.counts_dev = counts_dev;
+  size_t n = 0;
+  for (size_t k = 0; k < ntensors; ++k) n += sizes[k];
+  a.most = static_cast<unsigned>(val_off ? val_off : n);
   a.world = world;
   for (int r = 0; r < world; ++r) a.counts[r] = counts_dev ? 0 : counts[r];
   size_t at = 0;

@@ -21,8 +21,11 @@ int sparse_threshold_bounded(const float* g, float* acc, size_t n, float thr, in
 // stride words) into the tensors, which cover the index space in list order.
 // Values start val_off words behind the indices, or, with val_off == 0, right
 // behind the rank's own count.  counts: host array, or counts_dev on the device
-// (then clamped to val_off).
+// (then clamped to val_off, or to the size of the index space).
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
                      int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s);
+
+// Rounds the tensors to fp16 and back, in place (multi_tensor.cu).
+int round_f16_multi(void* const* tensors, const size_t* sizes, size_t count, cudaStream_t s);
 
 }  // namespace sgb
