@@ -100,6 +100,7 @@ def _link_native(obj):
     if _stale(NATIVE_LIB, [obj, LIB]):
         subprocess.check_call(["g++", "-shared", obj, "-o", NATIVE_LIB, "-L", os.path.join(_torch_dir(), "lib"),
                                "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+                               "-L", os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "lib64"), "-lcudart",
                                "-L", HERE, "-lsgb", "-Wl,-rpath,$ORIGIN"])
 
 

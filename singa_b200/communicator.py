@@ -38,10 +38,6 @@ class Communicator(object):
     current (compute) stream wait for the communicator's side streams.
     """
 
-    # Staging (``send=False``) only records the tensors, the bytes move at the
-    # flush: a driver may hand a whole bucket over at once.
-    stages_lazily = True
-
     def __init__(self, local_rank, world_size, holder, buffSize=4194304, min_ctas=0, max_ctas=0):
         if not torch.cuda.is_available():
             raise RuntimeError("singa_b200.Communicator needs a CUDA device; there is no CPU path")
@@ -119,6 +115,13 @@ class Communicator(object):
 
     def fusedSparsification(self, ts, accumulation, sparsThreshold, topK):
         _n.comm_sparsify(self._ptr, ts, accumulation, sparsThreshold, topK)
+
+    def syncDense(self, grad_stream, threshold, half=False):
+        """DistOpt's exchange of (name, param, grad) triples in one call: synch /
+        synchHalf of every gradient above ``threshold``, fusedSynch /
+        fusedSynchHalf of the buckets of smaller ones, each issued as soon as it
+        is complete.  Returns the names, parameters and gradients."""
+        return _n.comm_sync_dense(self._ptr, grad_stream, threshold, half)
 
     def beginSparsification(self, ts, accumulation, sparsThreshold, topK):
         """The selection half of fusedSparsification; endSparsification() issues

@@ -521,7 +521,7 @@ int sgb_comm_synch(sgb_comm* c, void* data, size_t n, int is_half, void* compute
   OK(emit(c, p.before, sgb::as_stream(compute_stream)));
   {
     Phase ph(c, "Dist_s_synch_allreduce", sgb::order::kStreamS);
-    NC(ncclAllReduce(data, data, n, is_half ? ncclHalf : ncclFloat, ncclSum, c->nccl, c->s));
+    if (c->world > 1) NC(ncclAllReduce(data, data, n, is_half ? ncclHalf : ncclFloat, ncclSum, c->nccl, c->s));
   }
   return emit(c, p.after, nullptr);
 }
@@ -574,7 +574,7 @@ int sgb_comm_fused_synch(sgb_comm* c, void* const* tensors, const size_t* sizes,
       OK(emit(c, p.before, compute));
       {
         Phase ph(c, "Dist_s_fusedSynch_allreduce", sgb::order::kStreamS);
-        NC(ncclAllReduce(tensors[0], tensors[0], total, ncclFloat, ncclSum, c->nccl, c->s));
+        if (c->world > 1) NC(ncclAllReduce(tensors[0], tensors[0], total, ncclFloat, ncclSum, c->nccl, c->s));
       }
       return emit(c, p.after, nullptr);
     }

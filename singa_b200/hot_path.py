@@ -5,7 +5,9 @@ pre-bound C-ABI call, replays DistOpt's bucket policy on the communicator as
 gradients become ready, and finishes with the fused multi-tensor SGD update.
 The calls of a step are recorded once as a native program; ``run_step`` is one
 call that issues them in order (2 us a call instead of 5: the arguments are
-already converted, and no interpreter runs between two launches).
+already converted, and no interpreter runs between two launches), or, for steps
+of small kernels repeated with the same hyper-parameters, launches them as one
+graph that it has captured itself.
 The whole step can be captured once into a CUDA graph and replayed, which is
 this implementation's counterpart of the reference's buffered-operation graph
 (``Device::EnableGraph`` / ``RunGraph``).
@@ -315,7 +317,17 @@ class HotPathGPU(object):
             else:
                 prog.append((name, tuple(C.addressof(a) if isinstance(a, C.Array) else a for a in args), False))
                 self.calls_per_step += 1
-        self._program = _lib.native.program(prog, None if self.comm is None else self.comm._h.value)
+        # The library may capture the program by itself unless the launches have to be
+        # made one by one: collectives (a graph that holds them keeps the communicator
+        # from closing), the sparse exchange (more ranks wait for counts on the host)
+        # and the streaming batch-norm form for channels that no cluster holds (each
+        # launch draws one of eight counter tables, a captured one would keep its own).
+        single = self.comm is not None and (self.comm.world_size > 1 or self.dist_option not in ("plain", "half"))
+        for op in self.plan["ops"]:
+            if "bn_" in op.kind:
+                n, _, h, w = self.t[op.args["x"]].shape
+                single = single or n * h * w * 8 > 8 * 100 * 1024
+        self._program = _lib.native.program(prog, None if self.comm is None else self.comm._h.value, not single)
 
     def _sgd_call(self, tables, stream):
         pp, gp, mp, sizes, n = tables

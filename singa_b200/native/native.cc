@@ -15,11 +15,13 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <array>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -651,6 +653,68 @@ PyObject* py_comm_sparsify_end(Args a, Py_ssize_t) {
   ISSUE(sgb_comm_sparsification_end, comm(a[0]), stream());
   Py_RETURN_NONE;
 }
+// The dense exchange of a stream of gradients (DistOpt's bucket policy): takes
+// (name, param, gradient) triples from an iterator, reduces a gradient above the
+// threshold at once and a bucket of smaller ones as soon as it holds more than
+// the threshold, while the iterator is still producing the next ones.  Returns
+// the names, parameters and gradients as three lists.
+PyObject* py_comm_sync_dense(Args a, Py_ssize_t) {   // (communicator, iterable, threshold, half)
+  sgb_comm* const c = comm(a[0]);
+  const double threshold = real(a[2]);
+  const bool half = truth(a[3]);
+  using Ref = std::unique_ptr<PyObject, void (*)(PyObject*)>;
+  auto drop = [](PyObject* p) { Py_XDECREF(p); };
+  const Ref it(PyObject_GetIter(a[1]), drop);
+  const Ref names(PyList_New(0), drop), params(PyList_New(0), drop), grads(PyList_New(0), drop);
+  if (!it || !names || !params || !grads) throw PyError{};
+  std::vector<void*> ptrs;
+  std::vector<size_t> sizes;
+  size_t held = 0;
+  auto need_f32 = [&](const Tensor& g) {
+    require(!half || g.scalar_type() == at::kFloat,
+            "only available for 32-bit tensors, which are converted to 16 bits before transmit");
+  };
+  bool bucket_f16 = false;
+  auto flush = [&] {
+    if (ptrs.empty()) return;
+    for (const int send : {0, 1}) {
+      if (half)
+        ISSUE(sgb_comm_fused_synch_half, c, ptrs.data(), sizes.data(), ptrs.size(), send, stream());
+      else
+        ISSUE(sgb_comm_fused_synch, c, ptrs.data(), sizes.data(), ptrs.size(), bucket_f16, send, stream());
+    }
+    ptrs.clear();
+    sizes.clear();
+    held = 0;
+  };
+  while (PyObject* item = PyIter_Next(it.get())) {
+    const Ref hold(item, drop);
+    const Ref triple(PySequence_Fast(item, "(name, param, grad) triples are expected"), drop);
+    if (!triple) throw PyError{};
+    if (PySequence_Fast_GET_SIZE(triple.get()) != 3) fail(PyExc_ValueError, "(name, param, grad) triples are expected");
+    PyObject** v = PySequence_Fast_ITEMS(triple.get());
+    if (PyList_Append(names.get(), v[0]) || PyList_Append(params.get(), v[1]) || PyList_Append(grads.get(), v[2]))
+      throw PyError{};
+    const Tensor& g = tensor(v[2]);
+    need_f32(g);
+    const size_t n = count(g);
+    if (static_cast<double>(n) > threshold) {
+      if (half) ISSUE(sgb_comm_synch_half, c, f32w(g), n, stream());
+      else ISSUE(sgb_comm_synch, c, raww(g), n, g.scalar_type() == at::kHalf, stream());
+      continue;
+    }
+    if (ptrs.empty()) bucket_f16 = g.scalar_type() == at::kHalf;
+    ptrs.push_back(raww(g));
+    sizes.push_back(n);
+    held += n;
+    if (static_cast<double>(held) > threshold) flush();
+  }
+  if (PyErr_Occurred()) throw PyError{};
+  flush();
+  PyObject* out = PyTuple_Pack(3, names.get(), params.get(), grads.get());
+  if (!out) throw PyError{};
+  return out;
+}
 PyObject* py_comm_wait(Args a, Py_ssize_t) {
   ISSUE(sgb_comm_wait, comm(a[0]), stream());
   Py_RETURN_NONE;
@@ -730,26 +794,50 @@ struct Call {
   std::vector<std::pair<size_t, int>> patches;
   bool profile_only;
 };
+// What a recorded step depends on besides its arguments: if this is the same as
+// in the run before, so are its launches.
+struct Settings {
+  double lr, momentum, decay;
+  int overlap;
+  int device;
+  bool operator==(const Settings& o) const {
+    return lr == o.lr && momentum == o.momentum && decay == o.decay && overlap == o.overlap && device == o.device;
+  }
+};
 struct Program {
   std::vector<Call> calls;
   sgb_comm* comm = nullptr;
   PyObject* keep = nullptr;   // the argument objects (names stay valid while it lives)
+  // A step of small kernels costs the host 1.9 us a launch and the GPU less than
+  // that per kernel, so once a program has run twice in a row with the same
+  // settings its launches are captured and a run is one graph launch (17 kernels:
+  // 32 us launched one by one, 10 us as a graph).  Off for programs whose
+  // launches must be made one by one (see HotPathGPU._record_program), while a
+  // caller captures, and while the communicator's phases are timed.
+  bool graphable = false;
+  Settings seen{};
+  unsigned streak = 0;        // runs in a row with `seen`
+  cudaGraphExec_t exec = nullptr;
+  std::mutex guard;           // of the four fields above
 };
+constexpr unsigned kEagerRuns = 2;
 const char kProgramTag[] = "singa_b200.program";
 
 void drop_program(PyObject* capsule) {
   auto* p = static_cast<Program*>(PyCapsule_GetPointer(capsule, kProgramTag));
   if (!p) return;
   Py_XDECREF(p->keep);
+  if (p->exec) cudaGraphExecDestroy(p->exec);
   delete p;
 }
 
-// (list of (function name, argument tuple, profile only), communicator | None) -> program
-PyObject* py_program(Args a, Py_ssize_t) {
+// (list of (function name, argument tuple, profile only), communicator | None[, graphable]) -> program
+PyObject* py_program(Args a, Py_ssize_t n) {
   PyObject* seq = PySequence_Fast(a[0], "a list of calls is expected");
   if (!seq) throw PyError{};
   auto prog = std::make_unique<Program>();
   prog->comm = comm(a[1]);
+  prog->graphable = n > 2 && truth(a[2]);
   const std::unique_ptr<PyObject, void (*)(PyObject*)> hold(seq, [](PyObject* p) { Py_DECREF(p); });
   for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(seq); ++k) {
     PyObject* item = PySequence_Fast_GET_ITEM(seq, k);
@@ -789,16 +877,8 @@ PyObject* py_program(Args a, Py_ssize_t) {
   return cap;
 }
 
-// (program, lr, momentum, weight decay, profile)
-PyObject* py_run_program(Args a, Py_ssize_t) {
-  auto* prog = static_cast<Program*>(PyCapsule_GetPointer(a[0], kProgramTag));
-  if (!prog) throw PyError{};
-  const double lr = real(a[1]), mom = real(a[2]), decay = real(a[3]);
-  const bool profile = truth(a[4]);
-  void* const st = stream();
-  int status = SGB_OK;
-  const char* where = "";
-  Py_BEGIN_ALLOW_THREADS;
+// Issues the calls in order on `st`; on a failure `where` names the call.
+int issue_calls(const Program* prog, const Settings& now, bool profile, void* st, const char** where) {
   Slot scratch_slots[kMaxArguments];
   for (const Call& c : prog->calls) {
     if (c.profile_only && !profile) continue;
@@ -816,19 +896,81 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
             scratch_slots[i].i = w;
             break;
           }
-          case kLr: scratch_slots[i].d = lr; break;
-          case kMomentum: scratch_slots[i].d = mom; break;
-          default: scratch_slots[i].d = decay;
+          case kLr: scratch_slots[i].d = now.lr; break;
+          case kMomentum: scratch_slots[i].d = now.momentum; break;
+          default: scratch_slots[i].d = now.decay;
         }
       }
       slots = scratch_slots;
     }
-    status = c.fn->invoke(slots);
+    const int status = c.fn->invoke(slots);
     if (status != SGB_OK) {
-      where = c.fn->name;
-      break;
+      *where = c.fn->name;
+      return status;
     }
   }
+  return SGB_OK;
+}
+
+// Captures one run on a stream of its own (nothing executes) and instantiates
+// it.  False: not possible here; the program then stays with single launches.
+bool capture_calls(Program* prog, const Settings& now) {
+  cudaStream_t side;
+  if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
+  cudaGraph_t graph = nullptr;
+  const char* where = "";
+  bool ok = cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  if (ok) {
+    ok = issue_calls(prog, now, false, side, &where) == SGB_OK;
+    ok = cudaStreamEndCapture(side, &graph) == cudaSuccess && ok && graph;
+  }
+  cudaGraphExec_t exec = nullptr;
+  if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  cudaStreamDestroy(side);
+  if (!ok) {
+    cudaGetLastError();      // a refused capture is not an error of the step
+    return false;
+  }
+  if (prog->exec) cudaGraphExecDestroy(prog->exec);
+  prog->exec = exec;
+  return true;
+}
+
+// (program, lr, momentum, weight decay, profile)
+PyObject* py_run_program(Args a, Py_ssize_t) {
+  auto* prog = static_cast<Program*>(PyCapsule_GetPointer(a[0], kProgramTag));
+  if (!prog) throw PyError{};
+  const bool profile = truth(a[4]);
+  const auto current = c10::cuda::getCurrentCUDAStream();
+  const Settings now{real(a[1]), real(a[2]), real(a[3]), sgb_get_option(SGB_OPT_OVERLAP_LAUNCHES),
+                     current.device_index()};
+  void* const st = current.stream();
+  const bool may_graph = prog->graphable && !profile &&
+                         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+  int status = SGB_OK;
+  const char* where = "";
+  Py_BEGIN_ALLOW_THREADS;
+  bool launched = false;
+  if (may_graph) {
+    const std::lock_guard<std::mutex> lock(prog->guard);
+    if (!(prog->streak && prog->seen == now)) {
+      prog->seen = now;
+      prog->streak = 0;
+    }
+    if (++prog->streak > kEagerRuns) {
+      if (prog->streak == kEagerRuns + 1 && !capture_calls(prog, now)) prog->graphable = false;
+      if (prog->graphable) {
+        launched = true;
+        if (cudaGraphLaunch(prog->exec, static_cast<cudaStream_t>(st)) != cudaSuccess) {
+          status = SGB_ERR_CUDA;
+          where = "cudaGraphLaunch";
+        }
+        if (prog->streak > 1u << 30) prog->streak = 1u << 30;
+      }
+    }
+  }
+  if (!launched) status = issue_calls(prog, now, profile, st, &where);
   Py_END_ALLOW_THREADS;
   if (status != SGB_OK) fail_status(where, status);
   Py_RETURN_NONE;
@@ -845,7 +987,7 @@ PyMethodDef kMethods[] = {
     METHOD(bn_backward, 9), METHOD(bn_add_relu_backward, 10), METHOD(pool_forward, 5), METHOD(pool_backward, 5),
     METHOD(pool_forward_argmax, 4), METHOD(pool_backward_argmax, 3), METHOD(sgd_multi, 9), METHOD(pack, 3), METHOD(unpack, 4),
     METHOD(comm_synch, 2), METHOD(comm_synch_half, 2), METHOD(comm_fused_synch, 3), METHOD(comm_fused_synch_half, 3),
-    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
+    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sync_dense, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

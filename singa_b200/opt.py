@@ -124,38 +124,37 @@ class DistOpt(object):
 
     def _update_all(self, plist):
         scale = float(np.float32(1.0) / np.float32(self.world_size))
-        if plist:
-            names, params, grads = zip(*plist)
+        names, params, grads = plist
+        if names:
             self.opt.apply_many(names, params, grads, scale)
         self.opt.step()
 
-    def _sync_dense(self, grad_stream, threshold, direct, fused):
-        # A communicator whose staging only takes note of the tensors gets each
-        # bucket in one piece; others are told of every gradient as it arrives.
-        whole = getattr(self.communicator, "stages_lazily", False)
-        plist, glist, acc = [], [], 0
-        for triple in grad_stream:
-            g = triple[2]
+    def _sync_dense(self, grad_stream, threshold, direct, fused, half=False):
+        """Names, parameters and (reduced) gradients of the stream."""
+        whole = getattr(self.communicator, "syncDense", None)
+        if whole is not None:
+            plist = whole(grad_stream, threshold, half)
+            self.wait()
+            return plist
+        names, params, grads, glist, acc = [], [], [], [], 0
+        for name, p, g in grad_stream:
             n = g.numel()
             if n > threshold:
                 direct(g)
             else:
                 glist.append(g)
-                if not whole:
-                    fused([g], False)
+                fused([g], False)
                 acc += n
                 if acc > threshold:
-                    if whole:
-                        fused(glist, False)
                     fused(glist, True)
                     acc, glist = 0, []
-            plist.append(triple)
+            names.append(name)
+            params.append(p)
+            grads.append(g)
         if glist:
-            if whole:
-                fused(glist, False)
             fused(glist, True)
         self.wait()
-        return plist
+        return names, params, grads
 
     def backward_and_update(self, grad_stream, threshold=2097152):
         """opt.py:826-865 over (name, param, grad) triples."""
@@ -170,7 +169,7 @@ class DistOpt(object):
                 sw.Clamp(g, -clip_Value, clip_Value, out=g)
                 yield name, p, g
         self._update_all(self._sync_dense(clipped(grad_stream) if clipping else grad_stream, threshold,
-                                          self.all_reduce_half, self.fused_all_reduce_half))
+                                          self.all_reduce_half, self.fused_all_reduce_half, half=True))
 
     def _divide_by_world(self, t):
         sw.DivFloatWithRet(t, self.world_size, t)
@@ -228,7 +227,7 @@ class DistOpt(object):
         if not hasattr(self, "sparsInit") and corr:
             self.gradAccumulation = []
             self.sparsInit = False
-        plist, glist, acc, k = [], [], 0, -1
+        names, params, grads, glist, acc, k = [], [], [], [], 0, -1
 
         def residual(n, like):
             if corr and not self.sparsInit:
@@ -253,8 +252,7 @@ class DistOpt(object):
             else:
                 self.fused_sparsification(tensors, residual(n, tensors[0]), spars, topK)
 
-        for triple in grad_stream:
-            g = triple[2]
+        for name, p, g in grad_stream:
             n = g.numel()
             if n > threshold:
                 k += 1
@@ -266,7 +264,9 @@ class DistOpt(object):
                     k += 1
                     exchange(glist, acc, False)
                     acc, glist = 0, []
-            plist.append(triple)
+            names.append(name)
+            params.append(p)
+            grads.append(g)
         if glist:
             k += 1
             exchange(glist, acc, False)
@@ -274,4 +274,4 @@ class DistOpt(object):
             self.communicator.endSparsification()
         self.wait()
         self.sparsInit = True
-        self._update_all(plist)
+        self._update_all((names, params, grads))

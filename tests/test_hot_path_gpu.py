@@ -288,3 +288,37 @@ def test_relu_forward_record_layout(n):
         bits = np.unpackbits(rec.cpu().numpy(), bitorder="little")[:n]
         assert np.array_equal(bits.astype(bool), (x > 0).cpu().numpy())
         assert torch.equal(dx, torch.where(x > 0, dy, torch.zeros_like(dy)))
+
+
+def test_repeated_steps_follow_their_hyper_parameters_and_stream():
+    """run_step may replay launches it has captured itself: many steps in a row,
+    a change of the learning rate in between, a caller's stream, a caller's own
+    capture in the middle - the parameters must be those of the oracle's steps."""
+    from oracle.path import OraclePath
+    from singa_b200.hot_path import HotPathGPU
+    from singa_b200.resnet50_path import build_cnn_plan, fuse_plan
+    plan = fuse_plan(build_cnn_plan(batch=3, channels=8))
+    gpu = HotPathGPU(plan, communicator=None, world=1, seed=2, lr=0.01, momentum=0.9, weight_decay=1e-5)
+    host = gpu.host_copy()
+    steps = [0.01] * 6 + [0.02] + [0.03] * 5 + [0.01] * 2
+    for lr in steps:
+        OraclePath(plan, host, lr=lr, momentum=0.9, weight_decay=1e-5).run_step()
+    side = torch.cuda.Stream()
+    calls = set()
+    for i, lr in enumerate(steps):
+        gpu.lr = lr
+        if i == 4:                            # a caller's own capture: one replay is this step
+            gpu.capture().replay()
+        elif i in (3, 9, 10):
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                calls.add(gpu.run_step())
+            torch.cuda.current_stream().wait_stream(side)
+        else:
+            calls.add(gpu.run_step())
+    torch.cuda.synchronize()
+    assert len(calls) == 1
+    got = gpu.host_copy()
+    for p in plan["params"]:
+        close(got[p], host[p], 2e-6, "param " + p)
+        close(got["m:" + p], host["m:" + p], 4e-5, "moment " + p)
