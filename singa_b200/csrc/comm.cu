@@ -667,19 +667,18 @@ int sgb_comm_fused_synch_half(sgb_comm* c, void* const* tensors, const size_t* s
     return SGB_OK;
   }
   if (total > c->max_elems) return SGB_ERR_CAPACITY;
-  const sgb::order::Step p = plan_call(c, sgb::order::kFlushHalf);
-  const bool one = alone(c, tensors, sizes, count, total, 1);
-  OK(emit(c, p.pre, compute));
-  if (one) {
-    // one rank: rounded where they are, see sgb_comm_synch_half
+  if (alone(c, tensors, sizes, count, total, 1)) {
+    // one rank: rounded where they are (see sgb_comm_synch_half), all of it on c1
     c->pend_ptrs.clear();
     c->pend_sizes.clear();
     c->send_off = 0;
+    OK(emit(c, plan_call(c, sgb::order::kStageCopy).pre, compute));
     Phase ph(c, "Dist_c1_fusedSynchHalf_float2half", sgb::order::kStreamC1);
-    OK(sgb::round_f16_multi(tensors, sizes, count, c->c1));
-  } else {
-    OK(pack_pending(c, "Dist_c1_fusedSynchHalf_float2half"));
+    return sgb::round_f16_multi(tensors, sizes, count, c->c1);
   }
+  const sgb::order::Step p = plan_call(c, sgb::order::kFlushHalf);
+  OK(emit(c, p.pre, compute));
+  OK(pack_pending(c, "Dist_c1_fusedSynchHalf_float2half"));
   OK(emit(c, p.before, compute));
   if (c->send_off) {
     Phase ph(c, "Dist_s_fusedSynchHalf_allreduce", sgb::order::kStreamS);
@@ -689,7 +688,7 @@ int sgb_comm_fused_synch_half(sgb_comm* c, void* const* tensors, const size_t* s
   OK(emit(c, p.after, nullptr));
   {
     Phase ph(c, "Dist_c2_fusedSynchHalf_half2floatcopy", sgb::order::kStreamC2);
-    if (!one) OK(sgb_unpack_f16_to_f32(c->recv_h, 0, tensors, sizes, count, 1.0f, c->c2));
+    OK(sgb_unpack_f16_to_f32(c->recv_h, 0, tensors, sizes, count, 1.0f, c->c2));
   }
   return emit(c, p.post, nullptr);
 }
@@ -721,31 +720,37 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
   if (n) {
     OK(emit(c, plan_call(c, sgb::order::kSparseSelect).pre, sgb::as_stream(compute_stream)));
     if (x.in_use) CU(cudaStreamWaitEvent(c->c1, x.consumed, 0));
-    // One tensor, or tensors that lie back to back in memory (a gradient arena),
-    // are selected from IN PLACE: no copy into the send buffer.
-    bool in_place = sgb::aligned16(tensors[0]);
-    for (size_t i = 1; i < count && in_place; ++i)
-      in_place = static_cast<const float*>(tensors[i]) == static_cast<const float*>(tensors[i - 1]) + sizes[i - 1];
-    const float* grad = in_place ? static_cast<const float*>(tensors[0]) : c->send;
     Phase ph(c, x.op_name, sgb::order::kStreamC1);
-    if (!in_place) OK(sgb_pack_f32(tensors, sizes, count, c->send, 0, c->c1));
+    // The selection reads the tensors where they are; only a long list, or one
+    // without a residual buffer, is copied together first.
+    float* const* grads = x.tensors.data();
+    const size_t* grad_sizes = x.sizes.data();
+    size_t ngrads = count;
+    if (!sgb::sparse_selects_from(grads, grad_sizes, ngrads, accumulation)) {
+      OK(sgb_pack_f32(tensors, sizes, count, c->send, 0, c->c1));
+      grads = &c->send;
+      grad_sizes = &x.n;
+      ngrads = 1;
+    }
     if (topk) {
       x.nnz_max = static_cast<size_t>(sgb_topk_count(spars, n));
       for (int r = 0; r < c->world; ++r) x.nnz_host[r] = static_cast<int>(x.nnz_max);
       if (x.nnz_max)
-        OK(sgb_sparse_topk_f32(grad, accumulation, nullptr, n, x.nnz_max, c->topk_mode, x.pay_send,
-                               reinterpret_cast<float*>(x.pay_send) + x.nnz_max, c->ws, c->ws_bytes, c->c1));
+        OK(sgb::sparse_topk(grads, grad_sizes, ngrads, accumulation, x.nnz_max, c->topk_mode, x.pay_send,
+                            reinterpret_cast<float*>(x.pay_send) + x.nnz_max, c->ws, c->ws_bytes, c->c1));
     } else if (capacity) {
       x.nnz_max = capacity;
-      OK(sgb::sparse_threshold_bounded(grad, accumulation, n, spars, x.pay_send, capacity, x.nnz_dev, c->dropped_dev,
-                                       c->ws, c->ws_bytes, c->c1));
+      OK(sgb::sparse_threshold_bounded(grads, grad_sizes, ngrads, accumulation, spars, x.pay_send, capacity, x.nnz_dev,
+                                       c->dropped_dev, c->ws, c->ws_bytes, c->c1));
       // the counts travel on the device only; receivers clamp them to the capacity
       if (c->world > 1) NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
     } else if (c->world == 1) {
       // nobody to tell: the dense sum reads the payload and its count where they are
-      OK(sgb::sparse_threshold_packed(grad, accumulation, n, spars, x.pay_send, x.nnz_dev, c->ws, c->ws_bytes, c->c1));
+      OK(sgb::sparse_threshold_packed(grads, grad_sizes, ngrads, accumulation, spars, x.pay_send, x.nnz_dev, c->ws,
+                                      c->ws_bytes, c->c1));
     } else {
-      OK(sgb::sparse_threshold_packed(grad, accumulation, n, spars, x.pay_send, x.nnz_dev, c->ws, c->ws_bytes, c->c1));
+      OK(sgb::sparse_threshold_packed(grads, grad_sizes, ngrads, accumulation, spars, x.pay_send, x.nnz_dev, c->ws,
+                                      c->ws_bytes, c->c1));
       NC(ncclAllGather(x.nnz_dev, x.nnz_dev + 1, 1, ncclInt, c->nccl, c->c1));
       CU(cudaMemcpyAsync(x.nnz_host, x.nnz_dev + 1, sizeof(int) * c->world, cudaMemcpyDeviceToHost, c->c1));
       CU(cudaEventRecord(x.counted, c->c1));
@@ -763,7 +768,18 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
   sgb_comm::Sparse& x = c->sparse[c->sparse_ended++ & 1];
   if (x.n == 0) return SGB_OK;
   const int W = c->world;
-  if (!x.topk && !x.capacity && W > 1) {
+  if (W == 1) {
+    // The payload is read where it lies: no all-gather, no count on the host.
+    plan_call(c, sgb::order::kSparseLocal);
+    CU(cudaStreamWaitEvent(c->c2, x.selected, 0));
+    Phase ph(c, x.op_name, sgb::order::kStreamC2);
+    OK(sgb::sparse_dense_sum(x.pay_send, 0, x.capacity, x.nnz_host, x.topk ? nullptr : x.nnz_dev, 1, x.tensors.data(),
+                             x.sizes.data(), x.tensors.size(), c->c2));
+    CU(cudaEventRecord(x.consumed, c->c2));
+    x.in_use = true;
+    return SGB_OK;
+  }
+  if (!x.topk && !x.capacity) {
     CU(cudaEventSynchronize(x.counted));
     for (int r = 0; r < W; ++r) {
       if (x.nnz_host[r] < 0 || static_cast<size_t>(x.nnz_host[r]) > x.n) return SGB_ERR_STATE;
@@ -776,18 +792,13 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
   OK(emit(c, p.before & ~static_cast<unsigned>(sgb::order::kC1ToS), sgb::as_stream(compute_stream)));
   {
     Phase ph(c, "Dist_s_sparsification_allgather", sgb::order::kStreamS);
-    if (W > 1 && x.nnz_max) NC(ncclAllGather(x.pay_send, c->pay_recv, 2 * x.nnz_max, ncclFloat, c->nccl, c->s));
+    if (x.nnz_max) NC(ncclAllGather(x.pay_send, c->pay_recv, 2 * x.nnz_max, ncclFloat, c->nccl, c->s));
   }
   OK(emit(c, p.after, nullptr));
   {
     Phase ph(c, x.op_name, sgb::order::kStreamC2);
     const size_t stride = 2 * x.nnz_max;
-    if (W == 1) {
-      OK(sgb::sparse_dense_sum(x.pay_send, 0, x.capacity, x.nnz_host, x.topk ? nullptr : x.nnz_dev, 1, x.tensors.data(),
-                               x.sizes.data(), x.tensors.size(), c->c2));
-      CU(cudaEventRecord(x.consumed, c->c2));
-      x.in_use = true;
-    } else if (W <= sgb::kMaxDenseRanks) {
+    if (W <= sgb::kMaxDenseRanks) {
       OK(sgb::sparse_dense_sum(c->pay_recv, stride, x.capacity, x.nnz_host, x.capacity ? x.nnz_dev + 1 : nullptr, W,
                                x.tensors.data(), x.sizes.data(), x.tensors.size(), c->c2));
     } else {

@@ -37,6 +37,7 @@ enum Call {
   // exchange's half between them (not replayed through sgb_comm_order_plan)
   kSparseSelect = 16,    // the selection on c1
   kSparseExchange = 17,  // ordered behind that selection: all-gather on s, dense sum on c2
+  kSparseLocal = 18,     // the same with one rank: the dense sum on c2 waits for the selection's own event
 };
 
 enum Edge : unsigned {
@@ -108,6 +109,10 @@ inline Step plan(State& st, int call) {
       p.result_stream = kStreamC2;
       st.c2_reads_recv = 1;
       st.dirty_s = st.dirty_c1 = st.dirty_c2 = 1;
+      break;
+    case kSparseLocal:
+      p.result_stream = kStreamC2;
+      st.dirty_c1 = st.dirty_c2 = 1;
       break;
     case kStageCopy:
       p.pre = kComputeToC1;

@@ -7,7 +7,10 @@
 //     in and the fp16->fp32 cast (+ scale) on the way out.
 // The tensor table (pointers, sizes, first-tile index) travels in the kernel
 // argument buffer, so there is no host-to-device table copy and no
-// allocation; lists longer than kMaxTensors are split into several launches.
+// allocation.  Two table sizes: lists of up to 72 tensors stay below 4 KB of
+// arguments, longer ones use the large buffer of this architecture (448
+// tensors, 18 KB: all 161 of ResNet-50 in one launch instead of three), and
+// only beyond that are several launches made.
 // Every CTA handles one 1024-element tile and finds its tensor with a binary
 // search over the table.
 #include "common.cuh"
@@ -17,22 +20,26 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr int kTile = 1024;       // elements per CTA (one float4 per thread)
-constexpr int kMaxTensors = 72;   // 72 * 40 B + header < 4 KB of kernel arguments
+constexpr int kSmallTable = 72, kLargeTable = 448;
 
+template <int N>
 struct Table {
+  static constexpr int kMost = N;
   int count;
-  unsigned first_tile[kMaxTensors + 1];
-  unsigned long long n[kMaxTensors];
-  void* a[kMaxTensors];  // param            | packed tensor
-  void* b[kMaxTensors];  // grad             | (unused)
-  void* c[kMaxTensors];  // momentum buffer  | (unused)
+  unsigned first_tile[N + 1];
+  unsigned long long n[N];
+  void* a[N];  // param            | packed tensor
+  void* b[N];  // grad             | (unused)
+  void* c[N];  // momentum buffer  | (unused)
 };
 // flat-buffer element offset of tensor k (pack / unpack)
+template <int N>
 struct Offsets {
-  unsigned long long off[kMaxTensors];
+  unsigned long long off[N];
 };
 
-__device__ __forceinline__ int find_tensor(const Table& t, unsigned tile) {
+template <int N>
+__device__ __forceinline__ int find_tensor(const Table<N>& t, unsigned tile) {
   int lo = 0, hi = t.count - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -61,8 +68,9 @@ __device__ __forceinline__ void sgd_one(float& p, float g, float& m, const SgdAr
   p = fmaf(0.0f - a.lr, step, p);
 }
 
+template <int N>
 __global__ void __launch_bounds__(kBlock)
-sgd_multi_kernel(const __grid_constant__ Table t, const SgdArgs a) {
+sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
   dependency_wait();
   const int k = find_tensor(t, blockIdx.x);
   const size_t n = t.n[k];
@@ -97,9 +105,9 @@ sgd_multi_kernel(const __grid_constant__ Table t, const SgdArgs a) {
 // (what packing, a one-rank all-reduce and unpacking do to them).
 enum PackMode { kPackF32 = 0, kPackF32ToF16 = 1, kUnpackF32 = 2, kUnpackF16ToF32 = 3, kRoundF16 = 4 };
 
-template <int MODE>
+template <int MODE, int N>
 __global__ void __launch_bounds__(kBlock)
-pack_multi_kernel(const __grid_constant__ Table t, const __grid_constant__ Offsets o,
+pack_multi_kernel(const __grid_constant__ Table<N> t, const __grid_constant__ Offsets<N> o,
                   void* flat, float scale, int use_scale) {
   dependency_wait();
   release_dependents();
@@ -178,7 +186,8 @@ pack_multi_kernel(const __grid_constant__ Table t, const __grid_constant__ Offse
 }
 
 // Fills a table with tensors [first, first+count) and returns the tile count.
-unsigned fill_table(Table& t, Offsets* o, void* const* a, void* const* b, void* const* c,
+template <int N>
+unsigned fill_table(Table<N>& t, Offsets<N>* o, void* const* a, void* const* b, void* const* c,
                     const size_t* sizes, size_t first, int count, size_t flat_off0) {
   t.count = count;
   unsigned tiles = 0;
@@ -197,22 +206,23 @@ unsigned fill_table(Table& t, Offsets* o, void* const* a, void* const* b, void* 
   return tiles;
 }
 
-int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t count, void* flat,
-                size_t flat_offset, float scale, int use_scale, void* stream) {
+template <int N>
+int pack_list(int mode, void* const* tensors, const size_t* sizes, size_t count, void* flat,
+              size_t flat_offset, float scale, int use_scale, void* stream) {
   if (count == 0) return SGB_OK;
   if (!tensors || !sizes || (!flat && mode != kRoundF16)) return SGB_ERR_NULL;
   cudaStream_t s = as_stream(stream);
   size_t off = flat_offset;
   for (size_t first = 0; first < count;) {
     // take as many tensors as fit the table, skipping empty ones
-    Table t;
-    Offsets o;
-    void* ptrs[kMaxTensors];
-    size_t ns[kMaxTensors];
+    Table<N> t;
+    Offsets<N> o;
+    void* ptrs[N];
+    size_t ns[N];
     int cnt = 0;
     size_t chunk_off = off;
     unsigned long long tiles64 = 0;
-    while (first < count && cnt < kMaxTensors) {
+    while (first < count && cnt < N) {
       const size_t n = sizes[first];
       if (n && !tensors[first]) return SGB_ERR_NULL;
       const unsigned long long tl = ceil_div(n, kTile);
@@ -234,13 +244,57 @@ int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t coun
     }
     if (cnt == 0) continue;
     // offsets inside the chunk are contiguous because empty tensors add 0
-    const unsigned tiles = fill_table(t, &o, ptrs, nullptr, nullptr, ns, 0, cnt, chunk_off);
-    auto kernel = mode == kPackF32        ? pack_multi_kernel<kPackF32>
-                  : mode == kPackF32ToF16 ? pack_multi_kernel<kPackF32ToF16>
-                  : mode == kUnpackF32    ? pack_multi_kernel<kUnpackF32>
-                  : mode == kRoundF16     ? pack_multi_kernel<kRoundF16>
-                                          : pack_multi_kernel<kUnpackF16ToF32>;
+    const unsigned tiles = fill_table<N>(t, &o, ptrs, nullptr, nullptr, ns, 0, cnt, chunk_off);
+    auto kernel = mode == kPackF32        ? pack_multi_kernel<kPackF32, N>
+                  : mode == kPackF32ToF16 ? pack_multi_kernel<kPackF32ToF16, N>
+                  : mode == kUnpackF32    ? pack_multi_kernel<kUnpackF32, N>
+                  : mode == kRoundF16     ? pack_multi_kernel<kRoundF16, N>
+                                          : pack_multi_kernel<kUnpackF16ToF32, N>;
     const int st = launch_ex(kernel, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, o, flat, scale, use_scale);
+    if (st != SGB_OK) return st;
+  }
+  return launch_status();
+}
+
+int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t count, void* flat,
+                size_t flat_offset, float scale, int use_scale, void* stream) {
+  return count <= kSmallTable
+             ? pack_list<kSmallTable>(mode, tensors, sizes, count, flat, flat_offset, scale, use_scale, stream)
+             : pack_list<kLargeTable>(mode, tensors, sizes, count, flat, flat_offset, scale, use_scale, stream);
+}
+
+// One launch for as many tensors as the table holds.
+template <int N>
+int sgd_list(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
+             const SgdArgs& a, cudaStream_t s) {
+  const bool use_m = a.use_momentum;
+  for (size_t first = 0; first < count;) {
+    Table<N> t;
+    void *pa[N], *pb[N], *pc[N];
+    size_t ns[N];
+    int cnt = 0;
+    unsigned long long tiles64 = 0;
+    while (first < count && cnt < N) {
+      const size_t n = sizes[first];
+      if (n) {
+        if (!params[first] || !grads[first] || (use_m && !moments[first])) return SGB_ERR_NULL;
+        const unsigned long long tl = ceil_div(n, kTile);
+        if (tiles64 + tl > 0x7fffffffull) {
+          if (cnt == 0) return SGB_ERR_SIZE;
+          break;
+        }
+        pa[cnt] = params[first];
+        pb[cnt] = grads[first];
+        pc[cnt] = use_m ? moments[first] : nullptr;
+        ns[cnt] = n;
+        ++cnt;
+        tiles64 += tl;
+      }
+      ++first;
+    }
+    if (cnt == 0) continue;
+    const unsigned tiles = fill_table<N>(t, nullptr, pa, pb, pc, ns, 0, cnt, 0);
+    const int st = launch_ex(sgd_multi_kernel<N>, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, a);
     if (st != SGB_OK) return st;
   }
   return launch_status();
@@ -270,36 +324,8 @@ int sgb_sgd_update_multi_f32(void* const* params, void* const* grads, void* cons
   SgdArgs a{lr, momentum, dampening, weight_decay, grad_scale, use_m, nesterov != 0,
             weight_decay != 0.0f, grad_scale != 1.0f};
   cudaStream_t s = as_stream(stream);
-  for (size_t first = 0; first < count;) {
-    Table t;
-    void *pa[kMaxTensors], *pb[kMaxTensors], *pc[kMaxTensors];
-    size_t ns[kMaxTensors];
-    int cnt = 0;
-    unsigned long long tiles64 = 0;
-    while (first < count && cnt < kMaxTensors) {
-      const size_t n = sizes[first];
-      if (n) {
-        if (!params[first] || !grads[first] || (use_m && !moments[first])) return SGB_ERR_NULL;
-        const unsigned long long tl = ceil_div(n, kTile);
-        if (tiles64 + tl > 0x7fffffffull) {
-          if (cnt == 0) return SGB_ERR_SIZE;
-          break;
-        }
-        pa[cnt] = params[first];
-        pb[cnt] = grads[first];
-        pc[cnt] = use_m ? moments[first] : nullptr;
-        ns[cnt] = n;
-        ++cnt;
-        tiles64 += tl;
-      }
-      ++first;
-    }
-    if (cnt == 0) continue;
-    const unsigned tiles = fill_table(t, nullptr, pa, pb, pc, ns, 0, cnt, 0);
-    const int st = launch_ex(sgd_multi_kernel, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, a);
-    if (st != SGB_OK) return st;
-  }
-  return launch_status();
+  return count <= kSmallTable ? sgd_list<kSmallTable>(params, grads, moments, sizes, count, a, s)
+                              : sgd_list<kLargeTable>(params, grads, moments, sizes, count, a, s);
 }
 
 int sgb_sgd_update_f32(float* param, const float* grad, float* moment, size_t n, float lr,

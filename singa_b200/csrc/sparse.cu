@@ -67,7 +67,8 @@ struct Work {
   bool dynamic;          // chunks are drawn from the ticket counter
 };
 inline Work work_for(size_t n) {
-  const size_t tiles = tiles_of(n), g = max_grid();
+  const size_t tiles = tiles_of(n);
+  const size_t g = max_grid();
   Work w;
   w.run = tiles > 4 * kWarps * g ? 4 : 1;
   w.capacity = w.run == 4 ? 352 : 128;
@@ -155,6 +156,51 @@ __device__ __forceinline__ void load_tile(const float* g, const float* acc, size
   for (int r = 0; r < kRounds; ++r)
 #pragma unroll
     for (int j = 0; j < 4; ++j) s[r][j] += b[r][j];
+}
+
+// The gradient as a list of tensors that need not lie back to back: element i
+// of the bucket is ptr[k][i - off[k]] for the k with off[k] <= i < off[k + 1].
+// Selecting straight from the list saves the copy into one buffer (8 B/element
+// and a launch per bucket).
+constexpr int kPieces = 256;
+struct Pieces {
+  int count;
+  unsigned off[kPieces + 1];
+  const float* ptr[kPieces];
+};
+struct NoPieces {};
+__device__ __forceinline__ void load_tile(const NoPieces&, const float* g, const float* acc, size_t tile, size_t n,
+                                          bool vec, float (&s)[kRounds][4]) {
+  load_tile(g, acc, tile, n, vec, s);
+}
+// s = gradient + acc for one tile.  A tile inside one tensor is loaded as above,
+// one that crosses an end element by element.  acc is there and aligned.
+__device__ __forceinline__ void load_tile(const Pieces& p, const float*, const float* acc, size_t tile, size_t n, bool,
+                                          float (&s)[kRounds][4]) {
+  const unsigned e0 = static_cast<unsigned>(tile * kTile), e1 = e0 + kTile;
+  int lo = 0, hi = p.count - 1;
+  while (lo < hi) {                                    // the same in all lanes
+    const int mid = (lo + hi + 1) >> 1;
+    if (p.off[mid] <= e0) lo = mid; else hi = mid - 1;
+  }
+  const float* base = p.ptr[lo] - p.off[lo];           // only used where it points into the tensor
+  if (e1 <= p.off[lo + 1] && (reinterpret_cast<uintptr_t>(base + e0) & 15u) == 0) {
+    load_tile(base, acc, tile, n, true, s);
+    return;
+  }
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const unsigned i = static_cast<unsigned>(vec_at(tile, r));
+    int k = lo;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s[r][j] = 0.0f;
+      if (i + j < n) {
+        while (i + j >= p.off[k + 1]) ++k;
+        s[r][j] = p.ptr[k][i + j - p.off[k]] + acc[i + j];
+      }
+    }
+  }
 }
 
 // Exclusive offsets, in element order, of this lane's counts inside the tile:
@@ -320,9 +366,9 @@ struct ThrArgs {
   bool vec;
 };
 
-template <bool BOUNDED>
+template <bool BOUNDED, typename Source>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
-thr_select_kernel(const ThrArgs a) {
+thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
   constexpr unsigned kSlots = 192;
   __shared__ int slot_idx[kWarps][kSlots];
   __shared__ float slot_val[kWarps][kSlots];
@@ -341,7 +387,7 @@ thr_select_kernel(const ThrArgs a) {
         size_t unlisted = hi;           // tiles [unlisted, hi) are counted only; acc keeps s there
         for (size_t tile = lo; tile < hi; ++tile) {
           float s[kRounds][4];
-          load_tile(a.g, a.acc, tile, a.n, a.vec, s);
+          load_tile(source, a.g, a.acc, tile, a.n, a.vec, s);
           unsigned m = 0, excl[kRounds];  // out-of-range lanes are 0 and never selected
 #pragma unroll
           for (int r = 0; r < kRounds; ++r)
@@ -574,9 +620,9 @@ struct TopkArgs {
   bool vec;
 };
 
-template <int MODE>
+template <int MODE, typename Source>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
-topk_select_kernel(const TopkArgs a) {
+topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   __shared__ unsigned sh[kBins1];
   __shared__ uint2 sm2[kWarps];
   __shared__ unsigned sm[kWarps + 2], next[2];
@@ -602,7 +648,7 @@ topk_select_kernel(const TopkArgs a) {
         run_tiles(a.work, chunk, n, lo, hi);
         for (size_t tile = lo; tile < hi; ++tile) {
           float s[kRounds][4];
-          load_tile(a.g, a.acc, tile, n, a.vec, s);
+          load_tile(source, a.g, a.acc, tile, n, a.vec, s);
           const unsigned valid = in_range(tile, n);
 #pragma unroll
           for (int r = 0; r < kRounds; ++r) {
@@ -915,7 +961,7 @@ topk_select_kernel(const TopkArgs a) {
 // and the copy back into the tensors: 4 B/element written, the payload read.
 // Payloads are in ascending index order, so a CTA finds its start in each with
 // one search and then walks forward.
-constexpr int kDenseTargets = 72;
+constexpr int kDenseTargets = 200;   // below 4 KB of kernel arguments
 constexpr int kDenseTile = 4096;   // elements: 16 KB of shared memory
 struct DenseArgs {
   const int* payload;          // rank r: [idx | val] at payload + r * stride
@@ -1045,8 +1091,8 @@ int check_common(const float* g, size_t n, const void* idx_out, void* ws, size_t
 // A grid whose CTAs wait for one another: all of them are resident or the
 // launch fails.  work_for() asks for at most kCtasPerSm CTAs per SM, which the
 // launch bounds and the shared memory of both kernels allow.
-template <typename A>
-int launch_cooperative(void (*kernel)(A), unsigned grid, const A& args, cudaStream_t s) {
+template <typename A, typename S>
+int launch_cooperative(void (*kernel)(A, S), unsigned grid, const A& args, const S& source, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kBlock);
@@ -1056,13 +1102,50 @@ int launch_cooperative(void (*kernel)(A), unsigned grid, const A& args, cudaStre
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args, source);
   if (e != cudaSuccess) return note_cuda_error(e);
   return launch_status();
 }
 
-int threshold_select(const float* g, float* acc, size_t n, float thr, int* idx_out, float* val_out, int* nnz_dev,
+// The gradient behind a selection: one array, or a list of tensors.
+struct Gradient {
+  const float* flat = nullptr;
+  Pieces pieces;
+  size_t n = 0;
+};
+// Fills in `g` from a tensor list; false where the list has to be packed first
+// (too many tensors, or no residual buffer to hold their sum).
+bool gather(Gradient* g, float* const* tensors, const size_t* sizes, size_t count, const float* acc) {
+  g->flat = nullptr;
+  g->n = 0;
+  g->pieces.count = 0;
+  bool joined = true;                                  // back to back in memory
+  for (size_t k = 0; k < count; ++k) {
+    if (!sizes[k]) continue;
+    Pieces& p = g->pieces;
+    if (p.count && p.ptr[p.count - 1] + (g->n - p.off[p.count - 1]) == tensors[k]) {
+      g->n += sizes[k];
+      continue;
+    }
+    if (p.count) joined = false;
+    if (p.count == kPieces) return false;
+    p.off[p.count] = static_cast<unsigned>(g->n);
+    p.ptr[p.count++] = tensors[k];
+    g->n += sizes[k];
+  }
+  if (g->n > 0x7fffffffu) return false;
+  g->pieces.off[g->pieces.count] = static_cast<unsigned>(g->n);
+  if (joined) {
+    g->flat = g->pieces.count ? g->pieces.ptr[0] : nullptr;
+    return true;
+  }
+  return acc && aligned16(acc);
+}
+
+int threshold_select(const Gradient& source, float* acc, float thr, int* idx_out, float* val_out, int* nnz_dev,
                      size_t cap, unsigned long long* dropped, void* ws, size_t ws_bytes, cudaStream_t s) {
+  const size_t n = source.n;
+  const float* g = source.flat ? source.flat : acc;
   if (!nnz_dev) return SGB_ERR_NULL;
   if (n == 0) {
     cudaError_t e = cudaMemsetAsync(nnz_dev, 0, sizeof(int), s);
@@ -1077,22 +1160,64 @@ int threshold_select(const float* g, float* acc, size_t n, float thr, int* idx_o
     cudaError_t e = cudaMemsetAsync(a.ws.counters->ticket, 0, sizeof(a.ws.counters->ticket), s);
     if (e != cudaSuccess) return note_cuda_error(e);
   }
-  return cap ? launch_cooperative(thr_select_kernel<true>, work.grid, a, s)
-             : launch_cooperative(thr_select_kernel<false>, work.grid, a, s);
+  if (!source.flat)
+    return cap ? launch_cooperative(thr_select_kernel<true, Pieces>, work.grid, a, source.pieces, s)
+               : launch_cooperative(thr_select_kernel<false, Pieces>, work.grid, a, source.pieces, s);
+  return cap ? launch_cooperative(thr_select_kernel<true, NoPieces>, work.grid, a, NoPieces{}, s)
+             : launch_cooperative(thr_select_kernel<false, NoPieces>, work.grid, a, NoPieces{}, s);
+}
+
+int topk_select(const Gradient& source, float* acc, size_t k, int mode, int* idx_out, float* val_out, void* ws,
+                size_t ws_bytes, cudaStream_t s) {
+  const size_t n = source.n;
+  if (n == 0 || k == 0) return SGB_OK;
+  if (mode != 0 && mode != 1) return SGB_ERR_UNSUPPORTED;
+  if (!val_out) return SGB_ERR_NULL;
+  const float* g = source.flat ? source.flat : acc;
+  const int st = check_common(g, n, idx_out, ws, ws_bytes);
+  if (st != SGB_OK) return st;
+  if (k > n) k = n;
+  const Work work = work_for(n);
+  TopkArgs a{g, acc, n, static_cast<unsigned>(k), work, carve(ws, work), idx_out, val_out,
+             aligned16(g) && (!acc || aligned16(acc))};
+  cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
+  if (e != cudaSuccess) return note_cuda_error(e);
+  if (!source.flat)
+    return mode == 0 ? launch_cooperative(topk_select_kernel<0, Pieces>, work.grid, a, source.pieces, s)
+                     : launch_cooperative(topk_select_kernel<1, Pieces>, work.grid, a, source.pieces, s);
+  return mode == 0 ? launch_cooperative(topk_select_kernel<0, NoPieces>, work.grid, a, NoPieces{}, s)
+                   : launch_cooperative(topk_select_kernel<1, NoPieces>, work.grid, a, NoPieces{}, s);
 }
 
 }  // namespace
 
 // ---- forms used by the communicator (declared in sparse.cuh) ---------------
-int sparse_threshold_packed(const float* g, float* acc, size_t n, float thr, int* payload, int* nnz_dev, void* ws,
-                            size_t ws_bytes, cudaStream_t s) {
-  return threshold_select(g, acc, n, thr, payload, nullptr, nnz_dev, 0, nullptr, ws, ws_bytes, s);
+bool sparse_selects_from(float* const* tensors, const size_t* sizes, size_t count, const float* acc) {
+  Gradient g;
+  return gather(&g, tensors, sizes, count, acc);
 }
 
-int sparse_threshold_bounded(const float* g, float* acc, size_t n, float thr, int* payload, size_t cap, int* nnz_dev,
-                             unsigned long long* dropped_dev, void* ws, size_t ws_bytes, cudaStream_t s) {
+int sparse_threshold_packed(float* const* tensors, const size_t* sizes, size_t count, float* acc, float thr,
+                            int* payload, int* nnz_dev, void* ws, size_t ws_bytes, cudaStream_t s) {
+  Gradient g;
+  if (!gather(&g, tensors, sizes, count, acc)) return SGB_ERR_UNSUPPORTED;
+  return threshold_select(g, acc, thr, payload, nullptr, nnz_dev, 0, nullptr, ws, ws_bytes, s);
+}
+
+int sparse_threshold_bounded(float* const* tensors, const size_t* sizes, size_t count, float* acc, float thr,
+                             int* payload, size_t cap, int* nnz_dev, unsigned long long* dropped_dev, void* ws,
+                             size_t ws_bytes, cudaStream_t s) {
   if (cap == 0 || cap > 0x7fffffffu || !dropped_dev) return SGB_ERR_SIZE;
-  return threshold_select(g, acc, n, thr, payload, nullptr, nnz_dev, cap, dropped_dev, ws, ws_bytes, s);
+  Gradient g;
+  if (!gather(&g, tensors, sizes, count, acc)) return SGB_ERR_UNSUPPORTED;
+  return threshold_select(g, acc, thr, payload, nullptr, nnz_dev, cap, dropped_dev, ws, ws_bytes, s);
+}
+
+int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float* acc, size_t k, int mode, int* idx_out,
+                float* val_out, void* ws, size_t ws_bytes, cudaStream_t s) {
+  Gradient g;
+  if (!gather(&g, tensors, sizes, count, acc)) return SGB_ERR_UNSUPPORTED;
+  return topk_select(g, acc, k, mode, idx_out, val_out, ws, ws_bytes, s);
 }
 
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
@@ -1157,28 +1282,22 @@ int sgb_topk_count(float ratio, size_t n) {
 int sgb_sparse_threshold_f32(const float* g, float* acc, size_t n, float thr, int32_t* idx_out,
                              float* val_out, int32_t* nnz_dev, void* ws, size_t ws_bytes,
                              void* stream) {
-  if (n && !val_out) return SGB_ERR_NULL;
-  return threshold_select(g, acc, n, thr, idx_out, val_out, nnz_dev, 0, nullptr, ws, ws_bytes, as_stream(stream));
+  if (n && (!g || !val_out)) return SGB_ERR_NULL;
+  Gradient source;
+  source.flat = g;
+  source.n = n;
+  return threshold_select(source, acc, thr, idx_out, val_out, nnz_dev, 0, nullptr, ws, ws_bytes, as_stream(stream));
 }
 
 int sgb_sparse_topk_f32(const float* g, float* acc, float* sum_scratch, size_t n, size_t k,
                         int mode, int32_t* idx_out, float* val_out, void* ws, size_t ws_bytes,
                         void* stream) {
-  if (n == 0 || k == 0) return SGB_OK;
-  if (mode != 0 && mode != 1) return SGB_ERR_UNSUPPORTED;
   (void)sum_scratch;   // kept in the signature; the sum lives in acc (or is g itself without a residual)
-  if (!val_out) return SGB_ERR_NULL;
-  int st = check_common(g, n, idx_out, ws, ws_bytes);
-  if (st != SGB_OK) return st;
-  if (k > n) k = n;
-  cudaStream_t s = as_stream(stream);
-  const Work work = work_for(n);
-  TopkArgs a{g, acc, n, static_cast<unsigned>(k), work, carve(ws, work), idx_out, val_out,
-             aligned16(g) && (!acc || aligned16(acc))};
-  cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
-  if (e != cudaSuccess) return note_cuda_error(e);
-  return mode == 0 ? launch_cooperative(topk_select_kernel<0>, work.grid, a, s)
-                   : launch_cooperative(topk_select_kernel<1>, work.grid, a, s);
+  if (n && k && !g) return SGB_ERR_NULL;
+  Gradient source;
+  source.flat = g;
+  source.n = n;
+  return topk_select(source, acc, k, mode, idx_out, val_out, ws, ws_bytes, as_stream(stream));
 }
 
 int sgb_scatter_add_f32(const int32_t* idx, const float* val, size_t count,

@@ -6,16 +6,25 @@ namespace sgb {
 
 constexpr int kMaxDenseRanks = 64;
 
+// Whether the selectors can read this bucket from its tensors: they lie back to
+// back, or there are at most 256 runs of them and an aligned residual buffer.
+bool sparse_selects_from(float* const* tensors, const size_t* sizes, size_t count, const float* acc);
+
 // Threshold selection with residual update and packed payload [idx(nnz) | val(nnz)]
 // (int32 view); the payload length lands in *nnz_dev.
-int sparse_threshold_packed(const float* g, float* acc, size_t n, float thr, int* payload, int* nnz_dev, void* ws,
-                            size_t ws_bytes, cudaStream_t s);
+int sparse_threshold_packed(float* const* tensors, const size_t* sizes, size_t count, float* acc, float thr,
+                            int* payload, int* nnz_dev, void* ws, size_t ws_bytes, cudaStream_t s);
 
 // Capacity-bounded form: payload [idx(cap) | val(cap)]; selected entries beyond
 // the first `cap` (index order) stay in the residual and are counted in
 // *dropped_dev (a device counter the caller owns).  *nnz_dev is the full count.
-int sparse_threshold_bounded(const float* g, float* acc, size_t n, float thr, int* payload, size_t cap, int* nnz_dev,
-                             unsigned long long* dropped_dev, void* ws, size_t ws_bytes, cudaStream_t s);
+int sparse_threshold_bounded(float* const* tensors, const size_t* sizes, size_t count, float* acc, float thr,
+                             int* payload, size_t cap, int* nnz_dev, unsigned long long* dropped_dev, void* ws,
+                             size_t ws_bytes, cudaStream_t s);
+
+// Top-K selection (see sgb_sparse_topk_f32) from a tensor list.
+int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float* acc, size_t k, int mode, int* idx_out,
+                float* val_out, void* ws, size_t ws_bytes, cudaStream_t s);
 
 // Dense sum of `world` payloads (ascending indices, rank r at payload + r *
 // stride words) into the tensors, which cover the index space in list order.
