@@ -1075,6 +1075,171 @@ int launch_ragged(const float* x, const float* dy, const float* relu_in, const f
                    sh, numel);
 }
 
+// ------------------------ single pass, gradient in registers, x in shared memory
+// For shares of which shared memory alone holds only two CTAs' worth per SM:
+// the first kRegUnits units per thread of the gradient stay in registers, so
+// THREE CTAs of 256 threads fit an SM and half as many bytes again are staged.
+// (A CTA spends 3.3 us taking its share in and 4.2 us on reduction, exchange
+// and dx; with two CTAs the SM's input idles part of the time.)  32x256x56x56:
+// 68.8 -> 60.4 us (0.78 of the copy bandwidth).
+// All loads have to be issued at once: a second, dependent batch waits behind
+// everything that is queued already (gradient after x: 62.7 us).  That is why
+// there is no form with a ReLU's input, which would need more registers than
+// three CTAs have (111 us with batches of four, against 88).
+// The sums are formed exactly as by bn_bwd_cluster_kernel with 512 threads
+// (thread t stands in for its threads t and t + 256), so that a fused call and
+// its unfused parts agree bit for bit whichever kernels they take.
+constexpr int kRegUnits = 8;
+constexpr int kHybridT = 256;
+
+__global__ void __launch_bounds__(kHybridT, 3)
+bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ scale,
+                     const float* __restrict__ mean, const float* __restrict__ invstd, float* __restrict__ dx,
+                     float* __restrict__ dscale, float* __restrict__ dbias, BnShape sh, int per_cta) {
+  constexpr int T = kHybridT, R = kRegUnits;
+  extern __shared__ __align__(16) float stage[];
+  __shared__ unsigned long long pairs_in;
+  __shared__ float red[2][2 * T / 32];
+  __shared__ float2 parts[16];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = static_cast<int>(cluster.num_blocks());
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int c = blockIdx.x / cs;
+  if (threadIdx.x == 0) {
+    mbar_init(&pairs_in, 1);
+    fence_mbarrier_init();
+  }
+  cluster.barrier_arrive();
+  const int hwu = sh.HW >> 2, total = sh.N * hwu;
+  const int u0 = min(rank * per_cta, total), u1 = min(u0 + per_cta, total);
+  const int first = u0 + threadIdx.x;
+  float* const sx = stage + static_cast<size_t>(threadIdx.x) * 4;                             // unit k at k * T * 4
+  float* const sg = stage + static_cast<size_t>(per_cta) * 4 + static_cast<size_t>(threadIdx.x) * 4;   // k >= R, at (k - R) * T * 4
+  const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
+  dependency_wait();
+  const float mu = mean[c];
+  Vec4f g[R];
+  {
+    UnitWalk w(first, T, hwu);
+#pragma unroll
+    for (int k = 0; k < R; ++k, w.next()) {
+      g[k].u = make_uint4(0, 0, 0, 0);
+      if (first + k * T < u1) {
+        const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4;
+        g[k].u = ld128(dy + off);
+        cp_async16(sx + k * (T * 4), x + off);
+      }
+      if (k == R / 2 - 1) cp_async_commit();
+    }
+    cp_async_commit();
+    int k = R;
+    for (int u = first + R * T; u < u1; u += T, w.next(), ++k) {
+      const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4;
+      cp_async16(sx + k * (T * 4), x + off);
+      cp_async16(sg + (k - R) * (T * 4), dy + off);
+    }
+    cp_async_commit();
+  }
+  // sums, in the order of the units; [0]: even units (thread t), [1]: odd ones (thread t + 256)
+  float s_dy[2] = {0.f, 0.f}, s_dyx[2] = {0.f, 0.f};
+  auto add = [&](int half, const Vec4f& vx, const Vec4f& vg) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      s_dy[half] += vg.f[q];
+      s_dyx[half] += vg.f[q] * (vx.f[q] - mu);
+    }
+  };
+  cp_async_wait_pending<2>();
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    if (k == R / 2) cp_async_wait_pending<1>();
+    if (first + k * T < u1) {
+      Vec4f vx;
+      vx.u = *reinterpret_cast<const uint4*>(sx + k * (T * 4));
+      add(k & 1, vx, g[k]);
+    }
+  }
+  cp_async_wait_pending<0>();
+#pragma unroll
+  for (int k = R; k < 16; ++k) {
+    if (first + k * T >= u1) break;
+    Vec4f vx, vg;
+    vx.u = *reinterpret_cast<const uint4*>(sx + k * (T * 4));
+    vg.u = *reinterpret_cast<const uint4*>(sg + (k - R) * (T * 4));
+    add(k & 1, vx, vg);
+  }
+  {
+    constexpr int kWarps = 2 * T / 32;                 // of the 512 threads
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const float p0 = warp_sum(s_dy[half]), p1 = warp_sum(s_dyx[half]);
+      if (lane == 0) {
+        red[0][half * (T / 32) + wid] = p0;
+        red[1][half * (T / 32) + wid] = p1;
+      }
+    }
+    __syncthreads();
+    cluster.barrier_wait();
+    if (wid == 0) {
+      const float p0 = warp_sum(lane < kWarps ? red[0][lane] : 0.0f);
+      const float p1 = warp_sum(lane < kWarps ? red[1][lane] : 0.0f);
+      exchange_pairs(cs, rank, p0, p1, parts, &pairs_in);
+    }
+  }
+  const float r_ = invstd[c], sc = scale[c];
+  float a, b;
+  pair_totals(cs, parts, &pairs_in, a, b);
+  const float inv_m = 1.0f / (static_cast<float>(sh.N) * static_cast<float>(sh.HW));
+  const float ds = b * r_, k_ = sc * r_, am = a * inv_m, bm = ds * r_ * inv_m;
+  if (rank == 0 && threadIdx.x == 0) {
+    dscale[c] = ds;
+    dbias[c] = a;
+  }
+  release_dependents();
+  auto emit = [&](size_t off, const Vec4f& vx, const Vec4f& vg) {
+    Vec4f o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.f[j] = k_ * (vg.f[j] - am - (vx.f[j] - mu) * bm);
+    st128(dx + off, o.u);
+  };
+  UnitWalk w(first, T, hwu);
+#pragma unroll
+  for (int k = 0; k < R; ++k, w.next()) {
+    if (first + k * T < u1) {
+      Vec4f vx;
+      vx.u = *reinterpret_cast<const uint4*>(sx + k * (T * 4));
+      emit(w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4, vx, g[k]);
+    }
+  }
+  int k = R;
+  for (int u = first + R * T; u < u1; u += T, w.next(), ++k) {
+    Vec4f vx, vg;
+    vx.u = *reinterpret_cast<const uint4*>(sx + k * (T * 4));
+    vg.u = *reinterpret_cast<const uint4*>(sg + (k - R) * (T * 4));
+    emit(w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4, vx, vg);
+  }
+}
+
+inline size_t hybrid_smem(long long units) {
+  const long long rest = units - kRegUnits * kHybridT;
+  return (static_cast<size_t>(units) + (rest > 0 ? rest : 0)) * 16;
+}
+// A share that the cluster kernel would give 512 threads, and that fits three
+// times into an SM this way.
+inline bool hybrid_share(int units) {
+  return units > 2048 && units <= 16 * kHybridT && hybrid_smem(units) <= 74 * 1024;
+}
+int launch_hybrid(const float* x, const float* dy, const float* scale, const float* mean, const float* invstd,
+                  float* dx, float* dscale, float* dbias, BnShape sh, int cs, int per_cta, cudaStream_t s) {
+  auto kernel = bn_bwd_hybrid_kernel;
+  static std::atomic<bool> attr_set[64];
+  const int ready = opt_in_once(kernel, attr_set, true);
+  if (ready != SGB_OK) return ready;
+  return launch_ex(kernel, dim3(static_cast<unsigned>(sh.C) * cs), dim3(kHybridT), hybrid_smem(per_cta), s, cs, true, x,
+                   dy, scale, mean, invstd, dx, dscale, dbias, sh, per_cta);
+}
+
 template <bool VEC, int MASK, int T, bool ADD = false>
 int launch_cluster_t(const float* x, const float* dy, const float* relu_in, const float* scale,
                      const float* mean, const float* invstd, float* dx, float* dscale,
@@ -1188,6 +1353,9 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
     int per_cta = 0;
     const int cs = cluster_plan(vec ? per_channel / 4 : per_channel, vec ? 32 : 8, 8192, &per_cta, C);
     if (cs > 0 && static_cast<long long>(C) * cs <= 0x7fffffffLL) {
+      // two CTAs' worth of work per SM at least, or there is nothing for a third to overlap with
+      if (vec && MASK == 0 && hybrid_share(per_cta) && static_cast<long long>(C) * cs >= 2LL * sm_count())
+        return launch_hybrid(x, dy, scale, mean, invstd, dx, dscale, dbias, sh, cs, per_cta, s);
       return vec ? launch_cluster<true, MASK>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias,
                                               sh, cs, per_cta, s)
                  : launch_cluster<false, MASK>(x, dy, relu_in, scale, mean, invstd, dx, dscale,
