@@ -161,6 +161,42 @@ bn_fwd_small_kernel(const FwdArgs a) {
   }
 }
 
+// The CTAs of a cluster exchange (sum, m2, count) of their shares, once, as
+// 16-byte asynchronous stores that signal the receivers' mbarriers, and every
+// thread merges them in rank order: mean and biased variance of the channel.
+// The peers have started (cluster barrier): their memory is addressable.
+__device__ __forceinline__ void exchange_moments(const FwdArgs& a, int cs, int rank, float s, float q, float n,
+                                                 float4* parts, unsigned long long* parts_in, float& mu, float& var) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    if (lane == 0) mbar_arrive_expect(parts_in, 16u * static_cast<unsigned>(cs));
+    if (lane < cs) {
+      unsigned slot, bar;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(slot) : "r"(smem_addr(&parts[rank])), "r"(lane));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_addr(parts_in)), "r"(lane));
+      asm volatile(
+          "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(slot),
+          "r"(__float_as_uint(s)), "r"(__float_as_uint(q)), "r"(__float_as_uint(n)), "r"(0u), "r"(bar)
+          : "memory");
+    }
+  }
+  bool in = false;
+  for (unsigned it = 0; it < (1u << 24) && !in; ++it) in = mbar_try_wait(parts_in, 0);
+  if (!in) atomicOr(&g_forward_faults, 1u);
+  const float inv_m = 1.0f / (static_cast<float>(a.sh.N) * static_cast<float>(a.sh.HW));
+  float sum = 0.f, m2 = 0.f;
+  for (int r = 0; r < cs; ++r) sum += parts[r].x;
+  mu = sum * inv_m;
+  for (int r = 0; r < cs; ++r) {
+    const float4 p = parts[r];
+    if (p.z > 0.f) {
+      const float d = p.x / p.z - mu;
+      m2 += p.y + p.z * (d * d);
+    }
+  }
+  var = m2 * inv_m;
+}
+
 // ------------------------------------------------------------- in a cluster
 // The CTAs of a cluster share channel blockIdx.x / cs.  x is staged in shared
 // memory by 16-byte asynchronous copies; sum and squared differences of the
@@ -271,36 +307,9 @@ bn_fwd_cluster_kernel(const FwdArgs a, int per_cta) {
   }
   channel_sums<T, false>(q, unused, sm[1]);
   cluster.barrier_wait();                              // peers have started: their memory is addressable
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    if (lane == 0) mbar_arrive_expect(&parts_in, 16u * static_cast<unsigned>(cs));
-    if (lane < cs) {
-      unsigned slot, bar;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(slot) : "r"(smem_addr(&parts[rank])), "r"(lane));
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_addr(&parts_in)), "r"(lane));
-      asm volatile(
-          "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(slot),
-          "r"(__float_as_uint(s)), "r"(__float_as_uint(q)), "r"(__float_as_uint(n)), "r"(0u), "r"(bar)
-          : "memory");
-    }
-  }
-  {
-    bool in = false;
-    for (unsigned it = 0; it < (1u << 24) && !in; ++it) in = mbar_try_wait(&parts_in, 0);
-    if (!in) atomicOr(&g_forward_faults, 1u);
-  }
-  const float inv_m = 1.0f / (static_cast<float>(a.sh.N) * static_cast<float>(a.sh.HW));
-  float sum = 0.f, m2 = 0.f;
-  for (int r = 0; r < cs; ++r) sum += parts[r].x;      // rank order: same totals in every CTA
-  const float mu = sum * inv_m;
-  for (int r = 0; r < cs; ++r) {
-    const float4 p = parts[r];
-    if (p.z > 0.f) {
-      const float d = p.x / p.z - mu;
-      m2 += p.y + p.z * (d * d);
-    }
-  }
-  const float var = m2 * inv_m, invstd = 1.0f / sqrtf(var + a.eps), g = sc * invstd;
+  float mu, var;
+  exchange_moments(a, cs, rank, s, q, n, parts, &parts_in, mu, var);
+  const float invstd = 1.0f / sqrtf(var + a.eps), g = sc * invstd;
   if (rank == 0 && threadIdx.x == 0) finish_channel(a, c, mu, var, invstd);
   release_dependents();
   UnitWalk w(first, T, upp);
@@ -314,6 +323,107 @@ bn_fwd_cluster_kernel(const FwdArgs a, int per_cta) {
 #pragma unroll
     for (int j = 0; j < kW; ++j) o.f[j] = (v.f[j] - mu) * g + b;
     r.store(a.y, o);
+  }
+}
+
+// The same with the first kRegUnits units per thread in registers: three CTAs of
+// 256 threads keep 290 KB of an SM's registers and shared memory in flight
+// instead of 200 KB.  All loads are issued at once.
+constexpr int kRegUnits = 8;
+constexpr int kHybridT = 256;
+__global__ void __launch_bounds__(kHybridT, 3)
+bn_fwd_hybrid_kernel(const FwdArgs a, int per_cta) {
+  constexpr int T = kHybridT, R = kRegUnits;
+  extern __shared__ __align__(16) float stage[];
+  __shared__ unsigned long long parts_in;
+  __shared__ __align__(16) float4 parts[16];
+  __shared__ float sm[2][2 * T / 32];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = static_cast<int>(cluster.num_blocks());
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int c = blockIdx.x / cs;
+  if (threadIdx.x == 0) {
+    mbar_init(&parts_in, 1);
+    fence_mbarrier_init();
+  }
+  cluster.barrier_arrive();
+  const int hwu = a.sh.HW >> 2, total = a.sh.N * hwu;
+  const int u0 = min(rank * per_cta, total), u1 = min(u0 + per_cta, total);
+  const int first = u0 + threadIdx.x;
+  float* const sx = stage + static_cast<size_t>(threadIdx.x) * 4;      // unit k >= R at (k - R) * T * 4
+  const size_t plane_stride = static_cast<size_t>(a.sh.C) * a.sh.HW, chan_off = static_cast<size_t>(c) * a.sh.HW;
+  dependency_wait();
+  Vec4f v[R];
+  {
+    UnitWalk w(first, T, hwu);
+#pragma unroll
+    for (int k = 0; k < R; ++k, w.next()) {
+      v[k].u = make_uint4(0, 0, 0, 0);
+      if (first + k * T < u1) v[k].u = ld128(a.x + w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4);
+    }
+    float* dst = sx;
+    for (int u = first + R * T; u < u1; u += T, w.next(), dst += T * 4)
+      cp_async16(dst, a.x + w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4);
+    cp_async_commit();
+  }
+  const float sc = a.scale[c], b = a.bias[c];
+  float s = 0.f, q = 0.f, unused = 0.f;
+#pragma unroll
+  for (int k = 0; k < R; ++k) s += (v[k].f[0] + v[k].f[1]) + (v[k].f[2] + v[k].f[3]);
+  cp_async_wait_pending<0>();
+  {
+    const float* src = sx;
+    for (int u = first + R * T; u < u1; u += T, src += T * 4) {
+      Vec4f t;
+      t.u = *reinterpret_cast<const uint4*>(src);
+      s += (t.f[0] + t.f[1]) + (t.f[2] + t.f[3]);
+    }
+  }
+  channel_sums<T, false>(s, unused, sm[0]);
+  const float n = static_cast<float>((u1 - u0) * 4), mine = n > 0.f ? s / n : 0.f;
+#pragma unroll
+  for (int k = 0; k < R; ++k)
+    if (first + k * T < u1) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float d = v[k].f[j] - mine;
+        q += d * d;
+      }
+    }
+  {
+    const float* src = sx;
+    for (int u = first + R * T; u < u1; u += T, src += T * 4) {
+      Vec4f t;
+      t.u = *reinterpret_cast<const uint4*>(src);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float d = t.f[j] - mine;
+        q += d * d;
+      }
+    }
+  }
+  channel_sums<T, false>(q, unused, sm[1]);
+  cluster.barrier_wait();
+  float mu, var;
+  exchange_moments(a, cs, rank, s, q, n, parts, &parts_in, mu, var);
+  const float invstd = 1.0f / sqrtf(var + a.eps), g = sc * invstd;
+  if (rank == 0 && threadIdx.x == 0) finish_channel(a, c, mu, var, invstd);
+  release_dependents();
+  UnitWalk w(first, T, hwu);
+  auto emit = [&](const Vec4f& x) {
+    Vec4f o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o.f[j] = (x.f[j] - mu) * g + b;
+    st128(a.y + w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4, o.u);
+  };
+#pragma unroll
+  for (int k = 0; k < R; ++k, w.next())
+    if (first + k * T < u1) emit(v[k]);
+  const float* src = sx;
+  for (int u = first + R * T; u < u1; u += T, w.next(), src += T * 4) {
+    Vec4f t;
+    t.u = *reinterpret_cast<const uint4*>(src);
+    emit(t);
   }
 }
 
@@ -469,6 +579,20 @@ template <int KIND>
 int launch_large(const FwdArgs& a, void* ws, size_t ws_bytes, cudaStream_t s) {
   const int total = a.sh.N * units_per_plane(KIND, a.sh.HW);
   int per_cta = 0;
+  if (KIND == kVec) {
+    // registers and shared memory together, where that still leaves two CTAs for
+    // every SM (32x256x56x56: 47.4 -> 44.4 us, 32x512x28x28 26.0 -> 24.8)
+    for (int hcs = 1; hcs <= 8; hcs *= 2) {
+      const int share = (total + hcs - 1) / hcs, rest = share - kRegUnits * kHybridT;
+      if (rest * 16 > 74 * 1024) continue;
+      if (rest < 0 || static_cast<long long>(a.sh.C) * hcs < 2LL * sm_count()) break;
+      static std::atomic<bool> attr_set[64];
+      const int ready = opt_in_once(bn_fwd_hybrid_kernel, attr_set, true);
+      if (ready != SGB_OK) return ready;
+      return launch_ex(bn_fwd_hybrid_kernel, dim3(static_cast<unsigned>(a.sh.C) * hcs), dim3(kHybridT),
+                       static_cast<size_t>(rest) * 16, s, hcs, true, a, share);
+    }
+  }
   const int cs = cluster_plan(total, Unit<KIND>::kW * 4, 8192, &per_cta, a.sh.C);
   if (cs > 0 && static_cast<long long>(a.sh.C) * cs <= 0x7fffffffLL)
     return per_cta > 2048 ? launch_cluster_t<KIND, 512>(a, cs, per_cta, s) : launch_cluster_t<KIND, 256>(a, cs, per_cta, s);
