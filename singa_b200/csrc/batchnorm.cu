@@ -1083,18 +1083,21 @@ int launch_ragged(const float* x, const float* dy, const float* relu_in, const f
 // and dx; with two CTAs the SM's input idles part of the time.)  32x256x56x56:
 // 68.8 -> 60.4 us (0.78 of the copy bandwidth).
 // All loads have to be issued at once: a second, dependent batch waits behind
-// everything that is queued already (gradient after x: 62.7 us).  That is why
-// there is no form with a ReLU's input, which would need more registers than
-// three CTAs have (111 us with batches of four, against 88).
+// everything that is queued already (gradient after x: 62.7 us).  A ReLU's input
+// has no registers left to go to, so it passes through the place of x and leaves
+// four bits per unit behind; x follows it unit by unit.  32x256x56x56 with the
+// ReLU's input: 87.7 -> 79.9 us (0.79 of the copy bandwidth); in batches of four
+// registers it was 111 us.
 // The sums are formed exactly as by bn_bwd_cluster_kernel with 512 threads
 // (thread t stands in for its threads t and t + 256), so that a fused call and
 // its unfused parts agree bit for bit whichever kernels they take.
 constexpr int kRegUnits = 8;
 constexpr int kHybridT = 256;
 
+template <bool RELU>
 __global__ void __launch_bounds__(kHybridT, 3)
-bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ scale,
-                     const float* __restrict__ mean, const float* __restrict__ invstd, float* __restrict__ dx,
+bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ relu_in,
+                     const float* __restrict__ scale, const float* __restrict__ mean, const float* __restrict__ invstd, float* __restrict__ dx,
                      float* __restrict__ dscale, float* __restrict__ dbias, BnShape sh, int per_cta) {
   constexpr int T = kHybridT, R = kRegUnits;
   extern __shared__ __align__(16) float stage[];
@@ -1119,6 +1122,16 @@ bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, 
   dependency_wait();
   const float mu = mean[c];
   Vec4f g[R];
+  unsigned long long keep = 0;       // RELU: 4 bits per unit
+  if (RELU) {
+    // The ReLU's input passes through the place of x, also by asynchronous copies:
+    // loads to registers would share the 28 KB that the staging leaves to L1.
+    UnitWalk w(first, T, hwu);
+    int k = 0;
+    for (int u = first; u < u1; u += T, w.next(), ++k)
+      cp_async16(sx + k * (T * 4), relu_in + w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4);
+    cp_async_commit();
+  }
   {
     UnitWalk w(first, T, hwu);
 #pragma unroll
@@ -1127,18 +1140,40 @@ bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, 
       if (first + k * T < u1) {
         const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4;
         g[k].u = ld128(dy + off);
-        cp_async16(sx + k * (T * 4), x + off);
+        if (!RELU) cp_async16(sx + k * (T * 4), x + off);
       }
-      if (k == R / 2 - 1) cp_async_commit();
+      if (!RELU && k == R / 2 - 1) cp_async_commit();
     }
-    cp_async_commit();
+    if (!RELU) cp_async_commit();
     int k = R;
     for (int u = first + R * T; u < u1; u += T, w.next(), ++k) {
       const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4;
-      cp_async16(sx + k * (T * 4), x + off);
+      if (!RELU) cp_async16(sx + k * (T * 4), x + off);
       cp_async16(sg + (k - R) * (T * 4), dy + off);
     }
     cp_async_commit();
+  }
+  if (RELU) {
+    cp_async_wait_pending<1>();
+    UnitWalk w(first, T, hwu);
+#pragma unroll
+    for (int k = 0; k < 16; ++k, w.next()) {
+      if (first + k * T < u1) {
+        Vec4f m;
+        m.u = *reinterpret_cast<const uint4*>(sx + k * (T * 4));
+        unsigned bits = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) bits |= (m.f[q] > 0 ? 1u : 0u) << q;
+        keep |= static_cast<unsigned long long>(bits) << (4 * k);
+        cp_async16(sx + k * (T * 4), x + w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4);
+      }
+      if (k == R / 2 - 1 || k == R - 1) cp_async_commit();
+    }
+    cp_async_commit();
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) g[k].f[q] = (keep >> (4 * k + q)) & 1u ? g[k].f[q] : 0.0f;
   }
   // sums, in the order of the units; [0]: even units (thread t), [1]: odd ones (thread t + 256)
   float s_dy[2] = {0.f, 0.f}, s_dyx[2] = {0.f, 0.f};
@@ -1166,6 +1201,11 @@ bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, 
     Vec4f vx, vg;
     vx.u = *reinterpret_cast<const uint4*>(sx + k * (T * 4));
     vg.u = *reinterpret_cast<const uint4*>(sg + (k - R) * (T * 4));
+    if (RELU) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) vg.f[q] = (keep >> (4 * k + q)) & 1u ? vg.f[q] : 0.0f;
+      *reinterpret_cast<uint4*>(sg + (k - R) * (T * 4)) = vg.u;
+    }
     add(k & 1, vx, vg);
   }
   {
@@ -1230,14 +1270,16 @@ inline size_t hybrid_smem(long long units) {
 inline bool hybrid_share(int units) {
   return units > 2048 && units <= 16 * kHybridT && hybrid_smem(units) <= 74 * 1024;
 }
-int launch_hybrid(const float* x, const float* dy, const float* scale, const float* mean, const float* invstd,
-                  float* dx, float* dscale, float* dbias, BnShape sh, int cs, int per_cta, cudaStream_t s) {
-  auto kernel = bn_bwd_hybrid_kernel;
+template <bool RELU>
+int launch_hybrid(const float* x, const float* dy, const float* relu_in, const float* scale, const float* mean,
+                  const float* invstd, float* dx, float* dscale, float* dbias, BnShape sh, int cs, int per_cta,
+                  cudaStream_t s) {
+  auto kernel = bn_bwd_hybrid_kernel<RELU>;
   static std::atomic<bool> attr_set[64];
   const int ready = opt_in_once(kernel, attr_set, true);
   if (ready != SGB_OK) return ready;
   return launch_ex(kernel, dim3(static_cast<unsigned>(sh.C) * cs), dim3(kHybridT), hybrid_smem(per_cta), s, cs, true, x,
-                   dy, scale, mean, invstd, dx, dscale, dbias, sh, per_cta);
+                   dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, per_cta);
 }
 
 template <bool VEC, int MASK, int T, bool ADD = false>
@@ -1354,8 +1396,8 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
     const int cs = cluster_plan(vec ? per_channel / 4 : per_channel, vec ? 32 : 8, 8192, &per_cta, C);
     if (cs > 0 && static_cast<long long>(C) * cs <= 0x7fffffffLL) {
       // two CTAs' worth of work per SM at least, or there is nothing for a third to overlap with
-      if (vec && MASK == 0 && hybrid_share(per_cta) && static_cast<long long>(C) * cs >= 2LL * sm_count())
-        return launch_hybrid(x, dy, scale, mean, invstd, dx, dscale, dbias, sh, cs, per_cta, s);
+      if (vec && MASK != 2 && hybrid_share(per_cta) && static_cast<long long>(C) * cs >= 2LL * sm_count())
+        return launch_hybrid<MASK == 1>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, cs, per_cta, s);
       return vec ? launch_cluster<true, MASK>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias,
                                               sh, cs, per_cta, s)
                  : launch_cluster<false, MASK>(x, dy, relu_in, scale, mean, invstd, dx, dscale,

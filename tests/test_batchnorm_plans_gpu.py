@@ -16,7 +16,8 @@ pytestmark = pytest.mark.gpu
 #         n, c, h, w
 SHAPES = [(1, 1, 1, 1), (1, 5, 4, 32), (1, 5, 4, 33), (4, 7, 8, 8), (4, 7, 8, 16), (4, 6, 16, 16), (4, 6, 16, 36),
           (8, 5, 32, 32), (1, 9, 64, 96), (1, 9, 64, 97), (4, 3, 46, 46), (33, 8, 7, 7), (33, 6, 7, 7), (9, 5, 2, 3),
-          (16, 10, 27, 27), (17, 48, 35, 29), (40, 3, 57, 57), (65, 2, 111, 113), (64, 2, 112, 112), (2, 300, 13, 13)]
+          (16, 10, 27, 27), (17, 48, 35, 29), (40, 3, 57, 57), (65, 2, 111, 113), (64, 2, 112, 112), (2, 300, 13, 13),
+          (32, 75, 56, 56), (7, 300, 44, 44), (11, 299, 28, 28)]
 
 
 def rel(got, want):
