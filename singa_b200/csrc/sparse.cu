@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include <atomic>
+#include <cmath>
 
 #include "sparse.cuh"
 
@@ -38,7 +39,7 @@ constexpr int kBlock = 256;
 constexpr int kWarps = kBlock / 32;
 constexpr int kRounds = 4;                             // float4 vectors per lane and tile
 constexpr int kTile = 32 * kRounds * 4;                // 512 elements, a warp's unit of work
-constexpr int kBins1 = 4096, kBins23 = 1024;           // 12 + 10 + 10 key bits
+constexpr int kBins1 = 3072, kBins23 = 1024;           // 12 + 10 + 10 key bits; no key is above 2^31, bin 2048
 // 4 CTAs per SM: 128 KB of loads in flight per SM already saturate HBM, and a
 // cooperative grid that does not need every slot can start beside the kernels
 // of another stream.
@@ -49,7 +50,7 @@ struct Counters {        // zeroed before a call that uses them
   unsigned ticket[4];    // chunks drawn so far, one counter per pass
   unsigned max_key;      // largest key of pass 0
   unsigned pad[3];
-  unsigned hist0[kBins1], hist1[kBins23], hist2[kBins23];
+  unsigned hist0[kBins1], hist1[kBins23], hist2[kBins23], sample[kBins1];
 };
 
 inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
@@ -613,6 +614,7 @@ struct TopkArgs {
   float* acc;
   size_t n;
   unsigned k;
+  unsigned sample_target;  // rank in the sample that bounds the k-th key from below; 0: no sample
   Work work;
   Workspace ws;
   int* idx_out;
@@ -620,23 +622,131 @@ struct TopkArgs {
   bool vec;
 };
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// s of one element.
+__device__ __forceinline__ float element(const NoPieces&, const float* g, const float* acc, size_t i) {
+  return acc ? g[i] + acc[i] : g[i];
+}
+__device__ __forceinline__ float element(const Pieces& p, const float*, const float* acc, size_t i) {
+  int lo = 0, hi = p.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (p.off[mid] <= i) lo = mid; else hi = mid - 1;
+  }
+  return p.ptr[lo][i - p.off[lo]] + acc[i];
+}
+
+// One warp's list while it goes through the tiles of a run.
+struct RunList {
+  int* idx;
+  float* val;
+  unsigned capacity, used;
+  size_t unlisted;       // tiles from here on are not in the list
+};
+// Appends the tile's elements of mask `m` while there is room, and calls
+// tally(value) for each of them in any case.  Few per lane (about one element
+// in sixty): walking the set bits, with the value picked from the registers,
+// beats sixteen predicated blocks.
+template <typename Tally>
+__device__ __forceinline__ void list_keys(const float (&s)[kRounds][4], unsigned m, size_t tile, size_t hi,
+                                          RunList& list, int* slot_idx, float* slot_val, unsigned slots, Tally tally) {
+  if (!__any_sync(0xffffffffu, m)) return;
+  const int lane = threadIdx.x & 31;
+  bool room = list.unlisted == hi;
+  unsigned excl[kRounds], total = 0;
+  if (room) {
+    total = tile_exclusive(round_counts(m), excl);
+    if (list.used + total > list.capacity) {
+      list.unlisted = tile;
+      room = false;
+    }
+  }
+  const bool staged = total <= slots;
+  int* const di = staged ? slot_idx : list.idx + list.used;
+  float* const dv = staged ? slot_val : list.val + list.used;
+  unsigned long long at = 0;                           // next position of each round, 16 bits each
+  if (room) {
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) at |= static_cast<unsigned long long>(excl[r]) << (16 * r);
+  }
+  for (unsigned left = m; left; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    float v = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 4 * kRounds; ++e) v = e == q ? s[e >> 2][e & 3] : v;
+    tally(v);
+    if (room) {
+      const unsigned pos = static_cast<unsigned>(at >> (16 * (q >> 2))) & 0xffffu;
+      at += 1ull << (16 * (q >> 2));
+      di[pos] = static_cast<int>(vec_at(tile, q >> 2) + (q & 3) + 1);
+      dv[pos] = v;
+    }
+  }
+  if (!room) return;
+  if (staged) {
+    __syncwarp();
+    for (unsigned e = lane; e < total; e += 32) {
+      list.idx[list.used + e] = slot_idx[e];
+      list.val[list.used + e] = slot_val[e];
+    }
+    __syncwarp();
+  }
+  list.used += total;
+}
+
+// Radix selection over 12 + 10 + 10 key bits, one cooperative launch:
+//   sample  128 elements per warp bound the k-th key from below (large n only)
+//   pass 0  s = g + acc; histogram of the top digit; with a bound, the keys at
+//           or above it go to the lists, and only they are counted
+//   pass 1  the middle digit inside the chosen bin: from the lists, or without
+//           a bound (or if it turned out too high) from s, which fills the lists
+//   pass 2  the last digit, from the lists; then count and copy out.
+// HBM-bound: pass 0 moves 12 B/element, pass 1 over s another 4, of which the
+// sample (8 us) saves the most and four in five of the shared-memory atomics.
 template <int MODE, typename Source>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
 topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
+  constexpr unsigned kSlots = 96;
   __shared__ unsigned sh[kBins1];
+  __shared__ int slot_idx_all[kWarps][kSlots];
+  __shared__ float slot_val_all[kWarps][kSlots];
   __shared__ uint2 sm2[kWarps];
   __shared__ unsigned sm[kWarps + 2], next[2];
   cg::grid_group grid = cg::this_grid();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // pass 1 needs 1024 of the 4096 bins: the rest are the warps' list slots
-  constexpr unsigned kSlots = (kBins1 - kBins23) / (2 * kWarps);
-  int* const slot_idx = reinterpret_cast<int*>(sh + kBins23) + warp * 2 * kSlots;
-  float* const slot_val = reinterpret_cast<float*>(slot_idx + kSlots);
+  int* const slot_idx = slot_idx_all[warp];
+  float* const slot_val = slot_val_all[warp];
   Counters* const cnt = a.ws.counters;
   const size_t n = a.n;
   const unsigned capacity = a.work.capacity;
   const float* const sum = a.acc ? a.acc : a.g;      // s after pass 0
   auto nothing = [](unsigned, unsigned) {};
+  auto run_list = [&](size_t run, size_t hi) {
+    return RunList{a.ws.list_idx + run * capacity, a.ws.list_val + run * capacity, capacity, 0, hi};
+  };
+
+  unsigned floor_bin = 0;                            // bins from here on are listed in pass 0; 0: none
+  if (MODE == 0 && a.sample_target) {
+    clear_bins<kBins1>(sh);
+    const unsigned warps = gridDim.x * kWarps;
+    const size_t e0 = n / warps * (blockIdx.x * kWarps + warp) + lane;   // n / warps >= 128: see the host's rule
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = element(source, a.g, a.acc, e0 + 32 * q);
+    unsigned bin[4];
+    const bool take[4] = {true, true, true, true};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) bin[q] = make_key<MODE>(v[q]) >> 20;
+    tally4(sh, bin, take);
+    flush_bins<kBins1>(sh, cnt->sample);
+    grid.sync();
+    unsigned left = a.sample_target, b;
+    pick_bin<kBins1>(cnt->sample, left, b, sm);
+    // more than an eighth at or above the bound (ties, a crowded bin) would not fit the lists
+    const unsigned taken = a.sample_target - left + __ldcg(&cnt->sample[b]);
+    if (taken <= warps * (128 / 8)) floor_bin = b;
+  }
 
   // pass 0: fold the gradient into the residual, histogram of the top 12 key bits
   clear_bins<kBins1>(sh);
@@ -646,13 +756,28 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
       [&](unsigned chunk, unsigned) {
         size_t lo, hi;
         run_tiles(a.work, chunk, n, lo, hi);
+        const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+        RunList list = run_list(run, hi);
         for (size_t tile = lo; tile < hi; ++tile) {
           float s[kRounds][4];
           load_tile(source, a.g, a.acc, tile, n, a.vec, s);
+          if (a.acc) {
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r) store4(a.acc, vec_at(tile, r), n, a.vec, s[r]);
+          }
+          if (floor_bin) {
+            unsigned m = 0;                          // out-of-range lanes have key 0
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) m |= make_key<MODE>(s[r][j]) >> 20 >= floor_bin ? 1u << (4 * r + j) : 0u;
+            list_keys(s, m, tile, hi, list, slot_idx, slot_val, kSlots,
+                      [&](float v) { atomicAdd(&sh[make_key<MODE>(v) >> 20], 1u); });
+            continue;
+          }
           const unsigned valid = in_range(tile, n);
 #pragma unroll
           for (int r = 0; r < kRounds; ++r) {
-            if (a.acc) store4(a.acc, vec_at(tile, r), n, a.vec, s[r]);
             unsigned bin[4];
             bool take[4];
 #pragma unroll
@@ -665,6 +790,8 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
             tally4(sh, bin, take);
           }
         }
+        if (floor_bin && lane == 0)
+          a.ws.run_meta[run] = pack_meta(0, list.used, static_cast<unsigned>(list.unlisted - lo));
       },
       nothing);
   flush_bins<kBins1>(sh, cnt->hist0);
@@ -679,7 +806,40 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
 
   unsigned remaining = a.k, bin;
   pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
-  const unsigned max_key = __ldcg(&cnt->max_key);
+  const bool listed = floor_bin && bin >= floor_bin;
+  if (floor_bin && !listed) {
+    // fewer than k keys at or above the bound: count the others as well
+    clear_bins<kBins1>(sh);
+    for_chunks<true>(
+        a.work, &cnt->ticket[2], next,
+        [&](unsigned chunk, unsigned) {
+          size_t lo, hi;
+          run_tiles(a.work, chunk, n, lo, hi);
+          for (size_t tile = lo; tile < hi; ++tile) {
+            float s[kRounds][4];
+            load_tile(sum, nullptr, tile, n, a.vec, s);
+            const unsigned valid = in_range(tile, n);
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r) {
+              unsigned low[4];
+              bool take[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                low[j] = make_key<MODE>(s[r][j]) >> 20;
+                take[j] = (valid >> (4 * r + j) & 1u) && low[j] < floor_bin;
+              }
+              tally4(sh, low, take);
+            }
+          }
+        },
+        nothing);
+    flush_bins<kBins1>(sh, cnt->hist0);
+    grid.sync();
+    remaining = a.k;
+    pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
+  }
+  // the sample has seen a key of floor_bin
+  const unsigned max_key = floor_bin ? floor_bin << 20 : __ldcg(&cnt->max_key);
   if (max_key == 0) {
     // every key is 0 (small gradients under integer-truncated keys): the first
     // k elements are sent, and the whole grid shares the work
@@ -692,9 +852,44 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
     return;
   }
 
-  // pass 1: list the keys at or above the chosen bin (chunks in descending
-  // order: what pass 0 touched last is still in L2) and take the histogram of
-  // the next digit inside the bin
+  // Once there are lists only they are looked at, and the tiles that are not in
+  // one: calls entry(value) for each listed entry and tile_fn(values, tile) for
+  // each other tile of this warp's runs, and done(run) after each run.  The
+  // next run's count and first 64 entries are fetched ahead (they are inside
+  // the segment whatever the count).
+  unsigned first, last;
+  my_chunks(a.work, first, last);
+  auto visit = [&](auto entry, auto tile_fn, auto done) {
+    unsigned meta = 0;
+    float v0 = 0.0f, v1 = 0.0f;
+    auto fetch = [&](unsigned chunk) {
+      const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+      meta = __ldcg(a.ws.run_meta + run);
+      v0 = __ldcg(a.ws.list_val + run * capacity + lane);
+      v1 = __ldcg(a.ws.list_val + run * capacity + lane + 32);
+    };
+    if (first < last) fetch(first);
+    for (unsigned chunk = first; chunk < last; ++chunk) {
+      const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+      const float* const list_val = a.ws.list_val + run * capacity;
+      const unsigned now = meta, used = meta_used(now);
+      const float w0 = v0, w1 = v1;
+      if (chunk + 1 < last) fetch(chunk + 1);
+      if (lane < used) entry(w0);
+      if (lane + 32 < used) entry(w1);
+      for (unsigned e = lane + 64; e < used; e += 32) entry(__ldcg(list_val + e));
+      size_t lo, hi;
+      run_tiles(a.work, chunk, n, lo, hi);
+      for (size_t tile = lo + meta_listed(now); tile < hi; ++tile) {
+        float s[kRounds][4];
+        load_tile(sum, nullptr, tile, n, a.vec, s);
+        tile_fn(s, tile);
+      }
+      done(run);
+    }
+  };
+  auto no_done = [](size_t) {};
+  // pass 1: the histogram of the next digit inside the bin
   const bool low_only = max_key < (1u << 10);        // the middle digit is zero everywhere
   const int shift = low_only ? 0 : 10;
   unsigned prefix = bin << 20;
@@ -702,120 +897,74 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   // to tie, which is what tally4 is for.
   const bool everything = prefix == 0;
   clear_bins<kBins23>(sh);
-  for_chunks<true>(
-      a.work, &cnt->ticket[1], next,
-      [&](unsigned chunk, unsigned) {
-        size_t lo, hi;
-        run_tiles(a.work, chunk, n, lo, hi);
-        const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
-        int* const list_idx = a.ws.list_idx + run * capacity;
-        float* const list_val = a.ws.list_val + run * capacity;
-        unsigned used = 0;
-        size_t unlisted = everything ? lo : hi;      // tiles [unlisted, hi) are not in the list
-        for (size_t tile = lo; tile < hi; ++tile) {
-          float s[kRounds][4];
-          load_tile(sum, nullptr, tile, n, a.vec, s);
-          if (everything) {
-            const unsigned valid = in_range(tile, n);
+  auto tally_tile = [&](const float (&s)[kRounds][4], size_t tile) {
+    const unsigned valid = in_range(tile, n);
 #pragma unroll
-            for (int r = 0; r < kRounds; ++r) {
-              unsigned digit[4];
-              bool take[4];
+    for (int r = 0; r < kRounds; ++r) {
+      unsigned digit[4];
+      bool take[4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const unsigned key = make_key<MODE>(s[r][j]);
-                take[j] = (valid >> (4 * r + j) & 1u) && key >> 20 == 0;
-                digit[j] = (key >> shift) & (kBins23 - 1);
-              }
-              tally4(sh, digit, take);
+      for (int j = 0; j < 4; ++j) {
+        const unsigned key = make_key<MODE>(s[r][j]);
+        take[j] = (valid >> (4 * r + j) & 1u) && key >> 20 == bin;
+        digit[j] = (key >> shift) & (kBins23 - 1);
+      }
+      tally4(sh, digit, take);
+    }
+  };
+  auto tally_key = [&](float v) {
+    const unsigned key = make_key<MODE>(v);
+    if (key >> 20 == bin) atomicAdd(&sh[(key >> shift) & (kBins23 - 1)], 1u);
+  };
+  if (listed) {
+    // pass 0 has streamed the lists out of L2: ask for all of them at once
+    for (unsigned chunk = first + lane; chunk < last; chunk += 32) {
+      const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+      prefetch_l2(a.ws.run_meta + run);
+      prefetch_l2(a.ws.list_val + run * capacity);
+      prefetch_l2(a.ws.list_val + run * capacity + 32);
+      prefetch_l2(a.ws.list_idx + run * capacity);
+      prefetch_l2(a.ws.list_idx + run * capacity + 32);
+    }
+    visit(tally_key, tally_tile, no_done);
+  } else {
+    // chunks in descending order: what pass 0 touched last is still in L2
+    for_chunks<true>(
+        a.work, &cnt->ticket[1], next,
+        [&](unsigned chunk, unsigned) {
+          size_t lo, hi;
+          run_tiles(a.work, chunk, n, lo, hi);
+          const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+          RunList list = run_list(run, hi);
+          if (everything) list.unlisted = lo;
+          for (size_t tile = lo; tile < hi; ++tile) {
+            float s[kRounds][4];
+            load_tile(sum, nullptr, tile, n, a.vec, s);
+            if (everything) {
+              tally_tile(s, tile);
+              continue;
             }
-            continue;
-          }
-          unsigned m = 0;                            // out-of-range lanes have key 0 < prefix
+            unsigned m = 0;                          // out-of-range lanes have key 0 < prefix
 #pragma unroll
-          for (int r = 0; r < kRounds; ++r)
+            for (int r = 0; r < kRounds; ++r)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) m |= make_key<MODE>(s[r][j]) >= prefix ? 1u << (4 * r + j) : 0u;
-          if (!__any_sync(0xffffffffu, m)) continue;
-          // Few candidates per lane (about one element in sixty): walk the set
-          // bits and fetch the value again (an L1 hit) instead of sixteen
-          // predicated blocks.
-          bool room = unlisted == hi;
-          unsigned excl[kRounds];
-          unsigned total = 0;
-          if (room) {
-            total = tile_exclusive(round_counts(m), excl);
-            if (used + total > capacity) {
-              unlisted = tile;
-              room = false;
-            }
+              for (int j = 0; j < 4; ++j) m |= make_key<MODE>(s[r][j]) >= prefix ? 1u << (4 * r + j) : 0u;
+            list_keys(s, m, tile, hi, list, slot_idx, slot_val, kSlots, tally_key);
           }
-          const bool staged = total <= kSlots;
-          int* const di = staged ? slot_idx : list_idx + used;
-          float* const dv = staged ? slot_val : list_val + used;
-          unsigned long long at = 0;
-          if (room) {
-#pragma unroll
-            for (int r = 0; r < kRounds; ++r) at |= static_cast<unsigned long long>(excl[r]) << (16 * r);
-          }
-          for (unsigned left = m; left; left &= left - 1) {
-            const int q = __ffs(left) - 1;
-            const size_t i = vec_at(tile, q >> 2) + (q & 3);
-            const float v = sum[i];
-            const unsigned key = make_key<MODE>(v);
-            if (key >> 20 == bin) atomicAdd(&sh[(key >> shift) & (kBins23 - 1)], 1u);
-            if (room) {
-              const unsigned pos = static_cast<unsigned>(at >> (16 * (q >> 2))) & 0xffffu;
-              at += 1ull << (16 * (q >> 2));
-              di[pos] = static_cast<int>(i + 1);
-              dv[pos] = v;
-            }
-          }
-          if (!room) continue;
-          if (staged) {
-            __syncwarp();
-            for (unsigned e = lane; e < total; e += 32) {
-              list_idx[used + e] = slot_idx[e];
-              list_val[used + e] = slot_val[e];
-            }
-            __syncwarp();
-          }
-          used += total;
-        }
-        if (lane == 0) a.ws.run_meta[run] = pack_meta(0, used, static_cast<unsigned>(unlisted - lo));
-      },
-      nothing);
+          if (lane == 0)
+            a.ws.run_meta[run] = pack_meta(0, list.used, static_cast<unsigned>(list.unlisted - lo));
+        },
+        nothing);
+  }
   flush_bins<kBins23>(sh, cnt->hist1);
   grid.sync();
   pick_bin<kBins23>(cnt->hist1, remaining, bin, sm);
   prefix |= bin << shift;
 
-  // From here on only the lists are looked at, and the tiles that are not in
-  // one.  Calls entry(value) for each listed entry and tile_fn(values, tile)
-  // for each other tile of this warp's run.
-  unsigned first, last;
-  my_chunks(a.work, first, last);
-  auto visit = [&](unsigned chunk, auto entry, auto tile_fn) {
-    const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
-    const float* const list_val = a.ws.list_val + run * capacity;
-    const float v0 = __ldcg(list_val + lane);          // inside the segment whatever the count: one round trip less
-    const unsigned meta = __ldcg(a.ws.run_meta + run), used = meta_used(meta);
-    if (lane < used) entry(v0);
-    for (unsigned e = lane + 32; e < used; e += 32) entry(__ldcg(list_val + e));
-    size_t lo, hi;
-    run_tiles(a.work, chunk, n, lo, hi);
-    for (size_t tile = lo + meta_listed(meta); tile < hi; ++tile) {
-      float s[kRounds][4];
-      load_tile(sum, nullptr, tile, n, a.vec, s);
-      tile_fn(s, tile);
-    }
-  };
   if (!low_only) {
     // pass 2: the last digit
     clear_bins<kBins23>(sh);
-    for (unsigned chunk = first; chunk < last; ++chunk)
-      visit(
-          chunk,
+    visit(
           [&](float v) {
             const unsigned key = make_key<MODE>(v);
             if ((key & ~(kBins23 - 1u)) == prefix) atomicAdd(&sh[key & (kBins23 - 1)], 1u);
@@ -834,7 +983,8 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
               }
               tally4(sh, digit, take);
             }
-          });
+          },
+          no_done);
     flush_bins<kBins23>(sh, cnt->hist2);
     grid.sync();
     pick_bin<kBins23>(cnt->hist2, remaining, bin, sm);
@@ -855,42 +1005,36 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
       }
     me &= in_range(tile, n);                         // out-of-range lanes have key 0: never above T
   };
-  // counts per warp and chunk, greater in the high half (a run has <= 2048
-  // elements), kept for the positions below; sums per chunk for the other CTAs
-  for (unsigned chunk = first; chunk < last; ++chunk) {
-    unsigned c = 0;
-    visit(
-        chunk,
-        [&](float v) {
-          const unsigned key = make_key<MODE>(v);
-          c += key > T ? 0x10000u : key == T ? 1u : 0u;
-        },
-        [&](const float (&s)[kRounds][4], size_t tile) {
-          unsigned mg, me;
-          masks(s, tile, mg, me);
-          c += __popc(mg) << 16 | __popc(me);
-        });
-    c = __reduce_add_sync(0xffffffffu, c);
-    __syncthreads();
-    if (lane == 0) {
-      sm[warp] = c;
-      a.ws.run_counts[static_cast<size_t>(chunk) * kWarps + warp] = c;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned g = 0, e = 0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        g += sm[w] >> 16;
-        e += sm[w] & 0xffffu;
-      }
-      a.ws.chunk_a[chunk] = g;
-      a.ws.chunk_b[chunk] = e;
-    }
+  // counts per run, greater in the high half (a run has <= 2048 elements), kept
+  // for the positions below; sums per CTA for the other CTAs
+  unsigned c = 0, c_gt = 0, c_eq = 0;
+  visit(
+      [&](float v) {
+        const unsigned key = make_key<MODE>(v);
+        c += key > T ? 0x10000u : key == T ? 1u : 0u;
+      },
+      [&](const float (&s)[kRounds][4], size_t tile) {
+        unsigned mg, me;
+        masks(s, tile, mg, me);
+        c += __popc(mg) << 16 | __popc(me);
+      },
+      [&](size_t run) {
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) {
+          a.ws.run_counts[run] = c;
+          c_gt += c >> 16;
+          c_eq += c & 0xffffu;
+        }
+        c = 0;
+      });
+  const uint2 mine_all = cta_sum2(c_gt, c_eq, sm2);
+  if (threadIdx.x == 0) {
+    a.ws.chunk_a[blockIdx.x] = mine_all.x;
+    a.ws.chunk_b[blockIdx.x] = mine_all.y;
   }
   grid.sync();
-  unsigned g_chunk = counts_before(a.ws.chunk_a, a.work.chunks, first, sm2).before;
-  unsigned e_chunk = counts_before(a.ws.chunk_b, a.work.chunks, first, sm2).before;
+  unsigned g_chunk = counts_before(a.ws.chunk_a, gridDim.x, blockIdx.x, sm2).before;
+  unsigned e_chunk = counts_before(a.ws.chunk_b, gridDim.x, blockIdx.x, sm2).before;
 
   // payload position = (#greater before) + min(#equal before, quota)
   auto send = [&](size_t index1, float v, unsigned ng, unsigned ne) {
@@ -900,14 +1044,25 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
     if (a.acc) a.acc[index1 - 1] = 0.0f;             // s - s
   };
   const unsigned below = (1u << lane) - 1u;
+  unsigned next_c = 0, next_meta = 0;
+  float next_v = 0.0f;
+  int next_i = 0;
+  auto fetch = [&](unsigned chunk) {
+    const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
+    next_c = lane < kWarps ? __ldcg(a.ws.run_counts + run - warp + lane) : 0u;
+    next_meta = __ldcg(a.ws.run_meta + run);
+    next_v = __ldcg(a.ws.list_val + run * capacity + lane);
+    next_i = __ldcg(a.ws.list_idx + run * capacity + lane);
+  };
+  if (first < last) fetch(first);
   for (unsigned chunk = first; chunk < last; ++chunk) {
     const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
     const int* const list_idx = a.ws.list_idx + run * capacity;
     const float* const list_val = a.ws.list_val + run * capacity;
-    const unsigned c = lane < kWarps ? __ldcg(a.ws.run_counts + run - warp + lane) : 0u;
-    const unsigned meta = __ldcg(a.ws.run_meta + run), used = meta_used(meta);
-    const float v0 = __ldcg(list_val + lane);          // four loads, one round trip
-    const int i0 = __ldcg(list_idx + lane);
+    const unsigned c = next_c, meta = next_meta, used = meta_used(meta);
+    float v_now = next_v;
+    int i_now = next_i;
+    if (chunk + 1 < last) fetch(chunk + 1);
     const unsigned mine = __shfl_sync(0xffffffffu, c, warp);
     unsigned g_at = g_chunk + __reduce_add_sync(0xffffffffu, lane < warp ? c >> 16 : 0u);
     unsigned e_at = e_chunk + __reduce_add_sync(0xffffffffu, lane < warp ? c & 0xffffu : 0u);
@@ -916,8 +1071,12 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
     if (mine >> 16 == 0 && ((mine & 0xffffu) == 0 || e_at >= quota)) continue;   // this run sends nothing
     for (unsigned base = 0; base < used; base += 32) {   // the list, 32 entries at a time, in order
       const bool in = base + lane < used;
-      const float v = !in ? 0.0f : base == 0 ? v0 : __ldcg(list_val + base + lane);
-      const int idx = !in ? 0 : base == 0 ? i0 : __ldcg(list_idx + base + lane);
+      const float v = v_now;
+      const int idx = i_now;
+      if (base + 32 + lane < used) {
+        v_now = __ldcg(list_val + base + 32 + lane);
+        i_now = __ldcg(list_idx + base + 32 + lane);
+      }
       const unsigned key = make_key<MODE>(v);
       const bool is_gt = in && key > T, is_eq = in && key == T;
       const unsigned mg = __ballot_sync(0xffffffffu, is_gt), me = __ballot_sync(0xffffffffu, is_eq);
@@ -977,11 +1136,14 @@ struct DenseArgs {
   float* ptr[kDenseTargets];
 };
 
-// First position whose index is >= want (1-based, ascending): one warp, 32-ary.
-__device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned count, long long want) {
+// A position at most `slack` before the first whose index is >= want (1-based,
+// ascending): one warp, 32-ary.  The last rounds of a search cost as much as the
+// first (0.7 us each) and save less than one window.
+__device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned count, long long want,
+                                                     unsigned slack) {
   const unsigned lane = threadIdx.x & 31;
   unsigned lo = 0, hi = count;                       // the answer is in [lo, hi]
-  while (hi > lo) {
+  while (hi - lo > slack) {
     const unsigned step = (hi - lo + 31) / 32;
     const unsigned at = lo + lane * step;
     const bool less = at < hi && static_cast<long long>(idx[at]) < want;
@@ -995,8 +1157,15 @@ __device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned co
   return lo;
 }
 
+// Entries pass through windows of 1024, four per thread, indices and values
+// fetched together: with 256 at a time a tile of a dense payload was a chain of
+// three to four round trips.  A single rank's window stays in registers over the
+// tiles that it serves.  11 buckets of 2.3e6 elements, 15 % of them sent:
+// 5.4 us each; 1e8 elements, 1 % sent: 81 us.
+template <bool ALONE>
 __global__ void __launch_bounds__(kBlock)
 dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta) {
+  constexpr unsigned kPer = 4, kWindow = kPer * kBlock;
   __shared__ __align__(16) float out[kDenseTile];
   __shared__ unsigned cursor[kMaxDenseRanks], count[kMaxDenseRanks];
   dependency_wait();
@@ -1009,7 +1178,7 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
     if (c < 0) c = 0;
     if (static_cast<unsigned>(c) > a.most) c = static_cast<int>(a.most);
     const unsigned at = warp_lower_bound(a.payload + r * a.stride, static_cast<unsigned>(c),
-                                         static_cast<long long>(begin) + 1);
+                                         static_cast<long long>(begin) + 1, kBlock);
     if ((threadIdx.x & 31) == 0) {
       cursor[r] = at;
       count[r] = static_cast<unsigned>(c);
@@ -1017,6 +1186,9 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
   }
   int target = 0;
   while (target + 1 < a.targets && a.off[target + 1] <= begin) ++target;
+  unsigned wi[kPer];
+  float wv[kPer];
+  bool have = false;                                 // ALONE: the window at cursor[0] is in wi, wv
   for (size_t base = begin; base < end; base += kDenseTile) {
     const size_t stop = base + kDenseTile < end ? base + kDenseTile : end;
     __syncthreads();                                 // cursors set; the previous tile has been stored
@@ -1024,20 +1196,30 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
     for (int r = 0; r < kDenseTile / (4 * kBlock); ++r)
       reinterpret_cast<float4*>(out)[r * kBlock + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    for (int r = 0; r < a.world; ++r) {
+    for (int r = 0; r < (ALONE ? 1 : a.world); ++r) {
       const int* idx = a.payload + r * a.stride;
       const unsigned cnt = count[r];
       const float* val = reinterpret_cast<const float*>(idx) + (a.val_off ? a.val_off : cnt);
       unsigned c = cursor[r];
-      for (int in_tile = kBlock; in_tile == kBlock;) {
-        const unsigned j = c + threadIdx.x;
-        const int i = j < cnt ? idx[j] : 0;
-        const bool mine = i > 0 && static_cast<size_t>(i) <= stop;
-        if (mine && static_cast<size_t>(i) > base) out[i - 1 - base] += val[j];   // indices are unique within a payload
-        in_tile = __syncthreads_count(mine);
-        c += static_cast<unsigned>(in_tile);
+      for (;;) {
+        if (!ALONE || !have) {
+#pragma unroll
+          for (unsigned q = 0; q < kPer; ++q) {
+            const unsigned j = c + q * kBlock + threadIdx.x;
+            const int i = j < cnt ? idx[j] : 0;
+            wv[q] = j < cnt ? val[j] : 0.0f;
+            wi[q] = i > 0 ? static_cast<unsigned>(i) : 0xffffffffu;     // padding is beyond every tile
+          }
+          have = true;
+        }
+#pragma unroll
+        for (unsigned q = 0; q < kPer; ++q)          // indices are unique within a payload
+          if (wi[q] > base && wi[q] <= stop) out[wi[q] - 1 - base] += wv[q];
+        if (__syncthreads_or(wi[kPer - 1] > stop)) break;               // the window reaches past the tile
+        c += kWindow;
+        have = false;
+        if (threadIdx.x == 0) cursor[r] = c;         // read again behind a barrier
       }
-      if (threadIdx.x == 0) cursor[r] = c;           // read again behind the next barrier
     }
     // store the tile to the tensors it overlaps
     for (size_t at = base; at < stop;) {
@@ -1178,7 +1360,17 @@ int topk_select(const Gradient& source, float* acc, size_t k, int mode, int* idx
   if (st != SGB_OK) return st;
   if (k > n) k = n;
   const Work work = work_for(n);
-  TopkArgs a{g, acc, n, static_cast<unsigned>(k), work, carve(ws, work), idx_out, val_out,
+  // The sample takes 8 us, and pass 1 over s 16 us per 10^7 elements: it pays
+  // from there on, where every warp has two KB or more of elements to sample
+  // from.  k up to n / 12, so that bound and margin stay inside the lists (352
+  // entries per 2048 elements).  Margin: an eighth and four standard deviations.
+  // Not for integer keys, which are mostly 0 or tied.
+  double target = 0;
+  if (mode == 0 && work.run == 4 && k <= n / 12) {
+    target = static_cast<double>(k) / static_cast<double>(n) * (work.grid * kWarps * 128.0);
+    target += target / 8 + 4 * std::sqrt(target) + 16;
+  }
+  TopkArgs a{g, acc, n, static_cast<unsigned>(k), static_cast<unsigned>(target), work, carve(ws, work), idx_out, val_out,
              aligned16(g) && (!acc || aligned16(acc))};
   cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
   if (e != cudaSuccess) return note_cuda_error(e);
@@ -1254,7 +1446,7 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
     a.off[a.targets] = at;
     const size_t tiles = ceil_div(a.last - a.first, kDenseTile);
     const unsigned per = static_cast<unsigned>(ceil_div(tiles, static_cast<size_t>(sm_count()) * 8));
-    const int st = launch_ex(dense_from_payloads_kernel, dim3(static_cast<unsigned>(ceil_div(tiles, per))),
+    const int st = launch_ex(world == 1 ? dense_from_payloads_kernel<true> : dense_from_payloads_kernel<false>, dim3(static_cast<unsigned>(ceil_div(tiles, per))),
                              dim3(kBlock), 0, s, 0, true, a, per);
     if (st != SGB_OK) return st;
   }

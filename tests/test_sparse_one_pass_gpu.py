@@ -46,6 +46,33 @@ def test_selection_where_the_plan_changes(n, shape):
         assert torch.equal(got_acc, left)
 
 
+@pytest.mark.parametrize("n", [2 * TURN + 1, 2 * TURN + 4099])
+@pytest.mark.parametrize("shape", ["gaussian", "heavy", "planted", "alike"])
+def test_top_k_with_a_sampled_bound(n, shape):
+    """`planted`: one sampled warp in twelve sees large keys that are nowhere
+    else, so the bound is too high and the full count has to take over."""
+    from singa_b200 import singa_wrap as sw
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    g = torch.randn(n, device="cuda", generator=gen)
+    if shape == "heavy":
+        g = g ** 7
+    elif shape == "planted":
+        warps = 148 * 4 * 8
+        starts = torch.arange(0, warps, 12, device="cuda") * (n // warps)
+        g[(starts[:, None] + torch.arange(128, device="cuda")).flatten()] = 1000.0
+    elif shape == "alike":
+        g.fill_(0.25)
+        g[n // 2:n // 2 + 500] = 0.5
+    for k in (1, 499, 501, n // 100, n // 12, n // 12 + 1):
+        acc = torch.zeros(n, device="cuda")
+        idx, val = sw.sparse_topk(g, acc, k, "magnitude")
+        want = largest(g, k, "magnitude")
+        assert torch.equal(idx.long() - 1, want) and torch.equal(val, g[want])
+        left = g.clone()
+        left[want] = 0
+        assert torch.equal(acc, left)
+
+
 def test_two_halves_equal_one_call_and_keep_their_order():
     from singa_b200 import _lib
     from singa_b200.communicator import Communicator, NcclIdHolder
