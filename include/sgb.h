@@ -638,6 +638,14 @@ int sgb_comm_synch_half(sgb_comm *c, float *data, size_t n,
 int sgb_comm_fused_synch_half(sgb_comm *c, void *const *tensors,
                               const size_t *sizes, size_t count, int send,
                               void *compute_stream);
+/* synch_half / fused_synch_half of a whole list of gradients that all exist, on
+ * one rank: the sum of one rank's fp16 values is those values, so the list is
+ * rounded in place by as few launches as its length allows, on c1.
+ * SGB_ERR_UNSUPPORTED (nothing done) with more ranks, with staged tensors
+ * pending, while profiling (whose phases are per bucket), and for a bucket
+ * (`largest` elements) above the communicator's capacity. */
+int sgb_comm_round_half(sgb_comm *c, void *const *tensors, const size_t *sizes, size_t count, size_t largest,
+                        void *compute_stream);
 /* Communicator::sparsification / fusedSparsification (communicator.cc:
  * 469-617) -> valSparsAllReduce / topKSparsAllReduce (:619-807).  count == 1
  * is the single-tensor form.  accumulation (device, total size) may be NULL.

@@ -693,6 +693,18 @@ int sgb_comm_fused_synch_half(sgb_comm* c, void* const* tensors, const size_t* s
   return emit(c, p.post, nullptr);
 }
 
+int sgb_comm_round_half(sgb_comm* c, void* const* tensors, const size_t* sizes, size_t count, size_t largest,
+                        void* compute_stream) {
+  if (!c) return SGB_ERR_NULL;
+  OK(check_list(tensors, sizes, count));
+  if (c->world != 1 || c->profiling || c->send_off || !c->pend_ptrs.empty() || largest > c->max_elems)
+    return SGB_ERR_UNSUPPORTED;
+  if (count == 0) return SGB_OK;
+  OK(emit(c, plan_call(c, sgb::order::kStageCopy).pre, sgb::as_stream(compute_stream)));
+  Phase ph(c, "Dist_c1_fusedSynchHalf_float2half", sgb::order::kStreamC1);
+  return sgb::round_f16_multi(tensors, sizes, count, c->c1);
+}
+
 // The selection half.  capacity == 0: the reference's exchange (the payload is
 // as long as the largest count, which the host reads back).  capacity > 0
 // (threshold mode): every rank sends exactly `capacity` slots, no host round trip.
