@@ -668,6 +668,16 @@ int sgb_comm_sparsification_begin(sgb_comm *c, void *const *tensors,
                                   float *accumulation, float spars, int topk,
                                   void *compute_stream);
 int sgb_comm_sparsification_end(sgb_comm *c, void *compute_stream);
+/* Threshold sparsification of several buckets whose gradients all exist, on one
+ * rank: tensors and sizes hold the buckets one behind the other, counts[k] of
+ * them in bucket k, whose residual is accumulations[k].  Results as by one call
+ * per bucket.  SGB_ERR_UNSUPPORTED (nothing done) where that is what it takes:
+ * more ranks, profiling on, an exchange open, a bucket above the capacity or of
+ * more than 2^25 elements or 256 runs of tensors, a residual that is missing or
+ * not on a 16-byte boundary. */
+int sgb_comm_sparsification_buckets(sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
+                                    float *const *accumulations, size_t nbuckets, float threshold,
+                                    void *compute_stream);
 /* Threshold sparsification with a fixed exchange size: every rank sends
  * exactly `capacity` (index, value) slots, the true counts travel on the
  * device, and the host never waits for a count - so the call can sit inside a

@@ -132,6 +132,12 @@ class Communicator(object):
     def endSparsification(self):
         _n.comm_sparsify_end(self._ptr)
 
+    def sparsifyBuckets(self, buckets, residuals, threshold):
+        """Threshold sparsification of several buckets that all exist, as one
+        selection and one write-back.  False (nothing done) where it takes a call
+        per bucket: more ranks, profiling, a bucket beyond the limits."""
+        return _n.comm_sparsify_buckets(self._ptr, buckets, residuals, threshold)
+
     def boundedSparsification(self, ts, accumulation, sparsThreshold, capacity):
         """Threshold sparsification with a fixed exchange of `capacity` slots per
         rank and no host wait for the counts (no counterpart in the reference,

@@ -27,6 +27,7 @@
 
 #include <atomic>
 #include <cmath>
+#include <vector>
 
 #include "sparse.cuh"
 
@@ -202,6 +203,38 @@ __device__ __forceinline__ void load_tile(const Pieces& p, const float*, const f
       }
     }
   }
+}
+
+// Several buckets, each with its own residual, as one index space in which
+// every bucket starts on a tile (the gaps are beyond its end and never selected).
+constexpr int kBuckets = 32;
+struct Buckets {
+  int count;
+  unsigned tile[kBuckets];       // first tile
+  unsigned end[kBuckets];        // one past the last element
+  float* acc[kBuckets];
+  Pieces pieces;                 // offsets in the joint space; a bucket's last piece takes in the gap
+};
+__device__ __forceinline__ void load_tile(const Buckets& b, const float* g, const float* acc, size_t tile, size_t n,
+                                          bool vec, float (&s)[kRounds][4]) {
+  load_tile(b.pieces, g, acc, tile, n, vec, s);
+}
+// The residual (indexed like the elements) and the end of what a tile belongs to.
+struct View {
+  float* acc;
+  size_t n;
+};
+template <typename Source>
+__device__ __forceinline__ View view(const Source&, float* acc, size_t n, size_t) {
+  return View{acc, n};
+}
+__device__ __forceinline__ View view(const Buckets& b, float*, size_t, size_t tile) {
+  int lo = 0, hi = b.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (b.tile[mid] <= tile) lo = mid; else hi = mid - 1;
+  }
+  return View{b.acc[lo] - static_cast<size_t>(b.tile[lo]) * kTile, b.end[lo]};
 }
 
 // Exclusive offsets, in element order, of this lane's counts inside the tile:
@@ -388,7 +421,8 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
         size_t unlisted = hi;           // tiles [unlisted, hi) are counted only; acc keeps s there
         for (size_t tile = lo; tile < hi; ++tile) {
           float s[kRounds][4];
-          load_tile(source, a.g, a.acc, tile, a.n, a.vec, s);
+          const View v = view(source, a.acc, a.n, tile);
+          load_tile(source, a.g, v.acc, tile, v.n, a.vec, s);
           unsigned m = 0, excl[kRounds];  // out-of-range lanes are 0 and never selected
 #pragma unroll
           for (int r = 0; r < kRounds; ++r)
@@ -398,14 +432,14 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
           const unsigned total = tile_exclusive(round_counts(m), excl);
           if (unlisted == hi && used + total > a.work.capacity) unlisted = tile;
           const bool listed = unlisted == hi;
-          if (a.acc) {
+          if (v.acc) {
 #pragma unroll
             for (int r = 0; r < kRounds; ++r) {
               float res[4];
 #pragma unroll
               for (int j = 0; j < 4; ++j)
                 res[j] = listed && fabsf(s[r][j]) >= a.thr ? s[r][j] - s[r][j] : s[r][j];
-              store4(a.acc, vec_at(tile, r), a.n, a.vec, res);
+              store4(v.acc, vec_at(tile, r), v.n, a.vec, res);
             }
           }
           count += total;
@@ -432,7 +466,6 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
   const Before b = counts_before(a.ws.chunk_a, a.work.chunks, first, sm);
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.nnz_dev = static_cast<int>(b.total);
   float* const val_out = a.val_out ? a.val_out : reinterpret_cast<float*>(a.idx_out) + (BOUNDED ? a.cap : b.total);
-  const float* const sum = a.acc ? a.acc : a.g;
   unsigned lost = 0, chunk_at = b.before;
   for (unsigned chunk = first; chunk < last; ++chunk) {
     const size_t run = static_cast<size_t>(chunk) * kWarps + warp;
@@ -477,7 +510,8 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
     run_tiles(a.work, chunk, a.n, lo, hi);
     for (size_t tile = lo + meta_listed(mine); tile < hi; ++tile) {
       float s[kRounds][4];
-      load_tile(sum, nullptr, tile, a.n, a.vec, s);
+      const View v = view(source, a.acc, a.n, tile);
+      load_tile(v.acc ? v.acc : a.g, nullptr, tile, v.n, a.vec, s);
       unsigned m = 0, excl[kRounds];
 #pragma unroll
       for (int r = 0; r < kRounds; ++r)
@@ -510,7 +544,7 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
           }
           ++pos;
         }
-        if (a.acc && sent) store4(a.acc, i, a.n, a.vec, res);
+        if (v.acc && sent) store4(v.acc, i, v.n, a.vec, res);
       }
       base += total;
     }
@@ -1227,7 +1261,8 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
       float* dst = a.ptr[target] + (at - a.off[target]);
       const float* src = out + (at - base);
       const int len = static_cast<int>(seg_end - at);
-      if (((reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>((at - base) * 4)) & 15u) == 0) {
+      if (!a.ptr[target]) {                            // a gap between buckets
+      } else if (((reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>((at - base) * 4)) & 15u) == 0) {
         const int nv = len >> 2;
         for (int v = threadIdx.x; v < nv; v += kBlock)
           reinterpret_cast<float4*>(dst)[v] = reinterpret_cast<const float4*>(src)[v];
@@ -1349,6 +1384,31 @@ int threshold_select(const Gradient& source, float* acc, float thr, int* idx_out
              : launch_cooperative(thr_select_kernel<false, NoPieces>, work.grid, a, NoPieces{}, s);
 }
 
+bool gather_buckets(Buckets* b, const SparseBucket* buckets, size_t count, size_t* span) {
+  size_t at = 0;
+  b->count = 0;
+  b->pieces.count = 0;
+  Gradient g;
+  for (size_t k = 0; k < count; ++k) {
+    const SparseBucket& from = buckets[k];
+    // (a bucket that lies back to back is one piece, with or without a residual)
+    if (!from.acc || !aligned16(from.acc) || !gather(&g, from.tensors, from.sizes, from.count, from.acc)) return false;
+    if (g.n == 0) continue;
+    if (b->count == kBuckets || b->pieces.count + g.pieces.count > kPieces || at + g.n > kMaxBucketSpan) return false;
+    b->tile[b->count] = static_cast<unsigned>(at / kTile);
+    b->end[b->count] = static_cast<unsigned>(at + g.n);
+    b->acc[b->count++] = from.acc;
+    for (int p = 0; p < g.pieces.count; ++p) {
+      b->pieces.off[b->pieces.count] = static_cast<unsigned>(at) + g.pieces.off[p];
+      b->pieces.ptr[b->pieces.count++] = g.pieces.ptr[p];
+    }
+    at = (at + g.n + kTile - 1) / kTile * kTile;
+  }
+  b->pieces.off[b->pieces.count] = static_cast<unsigned>(at);
+  *span = at;
+  return at > 0;
+}
+
 int topk_select(const Gradient& source, float* acc, size_t k, int mode, int* idx_out, float* val_out, void* ws,
                 size_t ws_bytes, cudaStream_t s) {
   const size_t n = source.n;
@@ -1384,6 +1444,46 @@ int topk_select(const Gradient& source, float* acc, size_t k, int mode, int* idx
 }  // namespace
 
 // ---- forms used by the communicator (declared in sparse.cuh) ---------------
+size_t sparse_buckets_span(const SparseBucket* buckets, size_t count) {
+  Buckets b;
+  size_t span = 0;
+  return gather_buckets(&b, buckets, count, &span) ? span : 0;
+}
+
+int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float thr, int* payload, int* nnz_dev, void* ws,
+                             size_t ws_bytes, cudaStream_t s) {
+  Buckets b;
+  size_t n = 0;
+  if (!gather_buckets(&b, buckets, count, &n)) return SGB_ERR_UNSUPPORTED;
+  const int st = check_common(b.acc[0], n, payload, ws, ws_bytes);
+  if (st != SGB_OK) return st;
+  const Work work = work_for(n);
+  ThrArgs a{nullptr, nullptr, n, thr, work, carve(ws, work), payload, nullptr, nnz_dev, 0, nullptr, true};
+  if (work.dynamic) {
+    cudaError_t e = cudaMemsetAsync(a.ws.counters->ticket, 0, sizeof(a.ws.counters->ticket), s);
+    if (e != cudaSuccess) return note_cuda_error(e);
+  }
+  return launch_cooperative(thr_select_kernel<false, Buckets>, work.grid, a, b, s);
+}
+
+int sparse_dense_buckets(const int* payload, const int* nnz_dev, const SparseBucket* buckets, size_t count,
+                         cudaStream_t s) {
+  std::vector<float*> tensors;
+  std::vector<size_t> sizes;
+  const int none[1] = {0};
+  for (size_t k = 0; k < count; ++k) {
+    size_t n = 0;
+    for (size_t t = 0; t < buckets[k].count; ++t) {
+      tensors.push_back(buckets[k].tensors[t]);
+      sizes.push_back(buckets[k].sizes[t]);
+      n += buckets[k].sizes[t];
+    }
+    tensors.push_back(nullptr);                        // the gap up to the next tile
+    sizes.push_back((kTile - n % kTile) % kTile);
+  }
+  return sparse_dense_sum(payload, 0, 0, none, nnz_dev, 1, tensors.data(), sizes.data(), tensors.size(), s);
+}
+
 bool sparse_selects_from(float* const* tensors, const size_t* sizes, size_t count, const float* acc) {
   Gradient g;
   return gather(&g, tensors, sizes, count, acc);
@@ -1432,7 +1532,7 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
     while (k < ntensors && a.targets < kDenseTargets) {
       if (sizes[k]) {
         // tensors that lie back to back are one target
-        if (a.targets && a.ptr[a.targets - 1] + (at - a.off[a.targets - 1]) == tensors[k]) {
+        if (a.targets && a.ptr[a.targets - 1] && a.ptr[a.targets - 1] + (at - a.off[a.targets - 1]) == tensors[k]) {
         } else {
           a.off[a.targets] = at;
           a.ptr[a.targets++] = tensors[k];

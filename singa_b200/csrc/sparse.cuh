@@ -22,6 +22,25 @@ int sparse_threshold_bounded(float* const* tensors, const size_t* sizes, size_t 
                              int* payload, size_t cap, int* nnz_dev, unsigned long long* dropped_dev, void* ws,
                              size_t ws_bytes, cudaStream_t s);
 
+// Several buckets at once, each with an aligned residual, as one selection: the
+// payload's indices are in a joint space of sparse_buckets_span() elements in
+// which bucket k starts at the next multiple of 512 behind bucket k - 1.  The
+// span is 0 where the list has to be cut (more than 32 buckets, 256 runs of
+// tensors or kMaxBucketSpan elements).
+struct SparseBucket {
+  float* const* tensors;
+  const size_t* sizes;
+  size_t count;
+  float* acc;
+};
+constexpr size_t kMaxBucketSpan = size_t{1} << 25;
+size_t sparse_buckets_span(const SparseBucket* buckets, size_t count);
+int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float thr, int* payload, int* nnz_dev, void* ws,
+                             size_t ws_bytes, cudaStream_t s);
+// The dense gradients of that payload, back into the buckets' tensors.
+int sparse_dense_buckets(const int* payload, const int* nnz_dev, const SparseBucket* buckets, size_t count,
+                         cudaStream_t s);
+
 // Top-K selection (see sgb_sparse_topk_f32) from a tensor list.
 int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float* acc, size_t k, int mode, int* idx_out,
                 float* val_out, void* ws, size_t ws_bytes, cudaStream_t s);

@@ -650,6 +650,33 @@ PyObject* py_comm_sparsify_begin(Args a, Py_ssize_t) {  // as comm_sparsify: the
   ISSUE(sgb_comm_sparsification_begin, comm(a[0]), l.ptrs.data(), l.sizes.data(), l.n(), acc, spars, topk, stream());
   Py_RETURN_NONE;
 }
+PyObject* py_comm_sparsify_buckets(Args a, Py_ssize_t) {  // (communicator, buckets, residuals, threshold) -> done?
+  std::vector<void*> ptrs;
+  std::vector<size_t> sizes, counts;
+  const Py_ssize_t n = PySequence_Size(a[1]);
+  if (n < 0) throw PyError{};
+  for (Py_ssize_t k = 0; k < n; ++k) {
+    const std::unique_ptr<PyObject, void (*)(PyObject*)> bucket(PySequence_GetItem(a[1], k),
+                                                                [](PyObject* p) { Py_XDECREF(p); });
+    if (!bucket) throw PyError{};
+    require(first_type(bucket.get()) == at::kFloat, "sparsification supports fp32 only");
+    const TensorList l(bucket.get(), false);
+    ptrs.insert(ptrs.end(), l.ptrs.begin(), l.ptrs.end());
+    sizes.insert(sizes.end(), l.sizes.begin(), l.sizes.end());
+    counts.push_back(l.n());
+  }
+  const TensorList acc(a[2], false);
+  require(acc.n() == counts.size(), "one residual per bucket");
+  const float threshold = static_cast<float>(real(a[3]));
+  int st = SGB_OK;
+  issue("sgb_comm_sparsification_buckets", [&] {
+    st = sgb_comm_sparsification_buckets(comm(a[0]), ptrs.data(), sizes.data(), counts.data(),
+                                         reinterpret_cast<float* const*>(acc.ptrs.data()), counts.size(), threshold,
+                                         stream());
+    return st == SGB_ERR_UNSUPPORTED ? SGB_OK : st;
+  });
+  return PyBool_FromLong(st == SGB_OK);
+}
 PyObject* py_comm_sparsify_end(Args a, Py_ssize_t) {
   ISSUE(sgb_comm_sparsification_end, comm(a[0]), stream());
   Py_RETURN_NONE;
@@ -1024,7 +1051,7 @@ PyMethodDef kMethods[] = {
     METHOD(bn_backward, 9), METHOD(bn_add_relu_backward, 10), METHOD(pool_forward, 5), METHOD(pool_backward, 5),
     METHOD(pool_forward_argmax, 4), METHOD(pool_backward_argmax, 3), METHOD(sgd_multi, 9), METHOD(pack, 3), METHOD(unpack, 4),
     METHOD(comm_synch, 2), METHOD(comm_synch_half, 2), METHOD(comm_fused_synch, 3), METHOD(comm_fused_synch_half, 3),
-    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sync_dense, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
+    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

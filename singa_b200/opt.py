@@ -227,7 +227,25 @@ class DistOpt(object):
         if not hasattr(self, "sparsInit") and corr:
             self.gradAccumulation = []
             self.sparsInit = False
-        names, params, grads, glist, acc, k = [], [], [], [], 0, -1
+        names, params, grads, k = [], [], [], -1
+
+        def buckets():
+            glist, acc = [], 0
+            for name, p, g in grad_stream:
+                names.append(name)
+                params.append(p)
+                grads.append(g)
+                n = g.numel()
+                if n > threshold:
+                    yield [g], n, True
+                    continue
+                glist.append(g)
+                acc += n
+                if acc > threshold:
+                    yield glist, acc, False
+                    acc, glist = 0, []
+            if glist:
+                yield glist, acc, False
 
         def residual(n, like):
             if corr and not self.sparsInit:
@@ -239,37 +257,34 @@ class DistOpt(object):
         begin = getattr(self.communicator, "beginSparsification", None)
         opened = 0
 
-        def exchange(tensors, n, single):
+        def exchange(tensors, res, single):
             nonlocal opened
             if begin is not None:
-                begin(tensors, residual(n, tensors[0]), spars, topK)
+                begin(tensors, res, spars, topK)
                 opened += 1
                 if opened == 2:
                     self.communicator.endSparsification()
                     opened = 1
             elif single:
-                self.sparsification(tensors[0], residual(n, tensors[0]), spars, topK)
+                self.sparsification(tensors[0], res, spars, topK)
             else:
-                self.fused_sparsification(tensors, residual(n, tensors[0]), spars, topK)
+                self.fused_sparsification(tensors, res, spars, topK)
 
-        for name, p, g in grad_stream:
-            n = g.numel()
-            if n > threshold:
+        # On one rank, gradients that all exist already go through one selection.
+        joint = getattr(self.communicator, "sparsifyBuckets", None)
+        if (joint is not None and corr and not topK and self.world_size == 1 and
+                type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
+            ready = []
+            for tensors, n, single in buckets():
                 k += 1
-                exchange([g], n, True)
-            else:
-                glist.append(g)
-                acc += n
-                if acc > threshold:
-                    k += 1
-                    exchange(glist, acc, False)
-                    acc, glist = 0, []
-            names.append(name)
-            params.append(p)
-            grads.append(g)
-        if glist:
-            k += 1
-            exchange(glist, acc, False)
+                ready.append((tensors, residual(n, tensors[0]), single))
+            if not ready or not joint([b[0] for b in ready], [b[1] for b in ready], spars):
+                for b in ready:
+                    exchange(*b)
+        else:
+            for tensors, n, single in buckets():
+                k += 1
+                exchange(tensors, residual(n, tensors[0]), single)
         if opened:
             self.communicator.endSparsification()
         self.wait()
