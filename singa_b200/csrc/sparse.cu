@@ -1195,9 +1195,11 @@ __device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned co
 // fetched together: with 256 at a time a tile of a dense payload was a chain of
 // three to four round trips.  A single rank's window stays in registers over the
 // tiles that it serves.  11 buckets of 2.3e6 elements, 15 % of them sent:
-// 5.4 us each; 1e8 elements, 1 % sent: 81 us.
+// 5.4 us each; 2.56e7 at once: 31.4 -> 24.9 us with the window, the binary
+// search for the first target and all 8 CTAs of an SM resident; 1e8 elements,
+// 1 % sent: 81.4 -> 80.0 us.
 template <bool ALONE>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 8)
 dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta) {
   constexpr unsigned kPer = 4, kWindow = kPer * kBlock;
   __shared__ __align__(16) float out[kDenseTile];
@@ -1219,7 +1221,10 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
     }
   }
   int target = 0;
-  while (target + 1 < a.targets && a.off[target + 1] <= begin) ++target;
+  for (int hi = a.targets - 1; target < hi;) {
+    const int mid = (target + hi + 1) >> 1;
+    if (a.off[mid] <= begin) target = mid; else hi = mid - 1;
+  }
   unsigned wi[kPer];
   float wv[kPer];
   bool have = false;                                 // ALONE: the window at cursor[0] is in wi, wv
