@@ -960,9 +960,10 @@ def kernel_launches(path):
            "sgb_avgpool_backward_f32": 1, "sgb_softmax_rows_f32": 1, "sgb_cross_entropy_f32": 1,
            "sgb_sum_all_f32": 1, "sgb_softmax_cross_entropy_bwd_f32": 1,
            "sgb_softmax_cross_entropy_grad_f32": 1, "sgb_softmax_cross_entropy_fused_f32": 1,
-           "sgb_scalar_f32": 1, "sgb_sum_rows_f32": 1, "sgb_set_f32": 1}
+           "sgb_scalar_f32": 1, "sgb_sum_rows_f32": 1, "sgb_set_f32": 1, "sgb_conv_bias_backward_f32": 1,
+           "sgb_relu_backward_sum_rows_f32": 1, "sgb_relu_backward_conv_bias_f32": 1}
     n = 0
-    for name, args in path.calls:
+    for name, args in path.launched:
         if name in ("sgb_bn_backward_f32", "sgb_bn_relu_backward_f32", "sgb_bn_relu_backward_mask_f32",
                     "sgb_bn_add_relu_backward_f32"):
             N, _, HW = args[-6:-3]          # (..., N, C, HW, workspace, workspace bytes, stream)

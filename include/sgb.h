@@ -242,6 +242,11 @@ int sgb_generateindex_i32(int32_t *out, size_t n, void *stream);
 size_t sgb_sum_rows_workspace_bytes(size_t nrow, size_t ncol);
 int sgb_sum_rows_f32(const float *M, float *v, size_t nrow, size_t ncol,
                      void *ws, size_t ws_bytes, void *stream);
+/* relu_backward and sum_rows of its result in one pass (the gradient of a ReLU
+ * in front of a linear layer's output and that layer's bias gradient): dx and v
+ * are the bits of the two calls. */
+int sgb_relu_backward_sum_rows_f32(const float *dy, const float *x, float *dx, float *v, size_t nrow, size_t ncol,
+                                   void *ws, size_t ws_bytes, void *stream);
 /* SumColumns: v[r] = sum over columns of M[r][c] (tensor.cc:1508-1522). */
 int sgb_sum_columns_f32(const float *M, float *v, size_t nrow, size_t ncol,
                         void *stream);
@@ -255,6 +260,9 @@ int sgb_row_max_f32(const float *M, float *v, size_t nrow, size_t ncol,
 size_t sgb_conv_bias_backward_workspace_bytes(int N, int C, int HW);
 int sgb_conv_bias_backward_f32(const float *dy, float *db, int N, int C, int HW,
                                void *ws, size_t ws_bytes, void *stream);
+/* The same for a convolution: relu_backward and conv_bias_backward of its result. */
+int sgb_relu_backward_conv_bias_f32(const float *dy, const float *x, float *dx, float *db, int N, int C, int HW,
+                                    void *ws, size_t ws_bytes, void *stream);
 /* SumAll: out[0] = sum of x (device scalar).  Replaces SumAll
  * (tensor.cc:1242-1254: ones tensor + Dot<float, lang::Cuda>,
  * tensor_math_cuda.h:1084-1094). */

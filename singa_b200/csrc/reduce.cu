@@ -29,9 +29,15 @@ constexpr int kMaxCluster = 8;
 // problems here are a few microseconds, a launch is half of that).  With more
 // slices than a cluster holds, the CTAs leave partial rows in `out` and
 // colsum_finish_kernel adds them.
-template <bool VEC>
+//
+// RELU: M is the gradient behind a ReLU with input `x`; what is summed is the
+// gradient in front of it, which is also written to `dx` (every element passes
+// through exactly one lane).  The terms and their order are those of the two
+// calls it stands for, so the sums are the same bits.  256x4096: 6.9 us in two
+// calls, 4.6 in one; 64x32x24x24 (channels): 5.3 and 4.0.
+template <bool VEC, bool RELU>
 __global__ void __launch_bounds__(kBlock, 4)
-colsum_kernel(const float* __restrict__ M, float* __restrict__ out, size_t nrow, size_t ncol, size_t rows_per_slice,
+colsum_kernel(const float* __restrict__ M, const float* __restrict__ x, float* __restrict__ dx, float* __restrict__ out, size_t nrow, size_t ncol, size_t rows_per_slice,
               int slices, int shift, bool clustered) {
   constexpr int kW = VEC ? 4 : 1;
   __shared__ float sm[kWarps][32 * kW];
@@ -46,42 +52,67 @@ colsum_kernel(const float* __restrict__ M, float* __restrict__ out, size_t nrow,
   const size_t r0 = slice * rows_per_slice;
   const size_t r1 = r0 + rows_per_slice < nrow ? r0 + rows_per_slice : nrow;
   const size_t step = static_cast<size_t>(kWarps) * rows_abreast;
+  constexpr int kBatch = RELU ? 4 : 8;                 // two operands: half the loads of each
   float acc[kW];
 #pragma unroll
   for (int k = 0; k < kW; ++k) acc[k] = 0.f;
+  auto keep4 = [&](float4& v, const float4& m, size_t at) {
+    v.x = m.x > 0.f ? v.x : 0.f;
+    v.y = m.y > 0.f ? v.y : 0.f;
+    v.z = m.z > 0.f ? v.z : 0.f;
+    v.w = m.w > 0.f ? v.w : 0.f;
+    *reinterpret_cast<float4*>(dx + at) = v;
+  };
+  auto keep1 = [&](float& v, float m, size_t at) {
+    v = m > 0.f ? v : 0.f;
+    dx[at] = v;
+  };
   if (c < ncol) {
     const float* p = M + c;
     size_t r = r0 + w * rows_abreast + (lane >> shift);
-    for (; r + 7 * step < r1; r += 8 * step) {
+    for (; r + (kBatch - 1) * step < r1; r += kBatch * step) {
       if (VEC) {
-        float4 v[8];
+        float4 v[kBatch], m[kBatch];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = *reinterpret_cast<const float4*>(p + (r + k * step) * ncol);
+        for (int k = 0; k < kBatch; ++k) {
+          v[k] = *reinterpret_cast<const float4*>(p + (r + k * step) * ncol);
+          if (RELU) m[k] = *reinterpret_cast<const float4*>(x + c + (r + k * step) * ncol);
+        }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < kBatch; ++k) {
+          if (RELU) keep4(v[k], m[k], c + (r + k * step) * ncol);
           acc[0] += v[k].x;
           acc[1 % kW] += v[k].y;
           acc[2 % kW] += v[k].z;
           acc[3 % kW] += v[k].w;
         }
       } else {
-        float v[8];
+        float v[kBatch], m[kBatch];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = p[(r + k * step) * ncol];
+        for (int k = 0; k < kBatch; ++k) {
+          v[k] = p[(r + k * step) * ncol];
+          if (RELU) m[k] = x[c + (r + k * step) * ncol];
+        }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[0] += v[k];
+        for (int k = 0; k < kBatch; ++k) {
+          if (RELU) keep1(v[k], m[k], c + (r + k * step) * ncol);
+          acc[0] += v[k];
+        }
       }
     }
 #pragma unroll 4
     for (; r < r1; r += step) {
       if (VEC) {
-        const float4 v = *reinterpret_cast<const float4*>(p + r * ncol);
+        float4 v = *reinterpret_cast<const float4*>(p + r * ncol);
+        if (RELU) keep4(v, *reinterpret_cast<const float4*>(x + c + r * ncol), c + r * ncol);
         acc[0] += v.x;
         acc[1 % kW] += v.y;
         acc[2 % kW] += v.z;
         acc[3 % kW] += v.w;
       } else {
-        acc[0] += p[r * ncol];
+        float v = p[r * ncol];
+        if (RELU) keep1(v, x[c + r * ncol], c + r * ncol);
+        acc[0] += v;
       }
     }
   }
@@ -203,10 +234,11 @@ rowmax_kernel(const float* __restrict__ M, float* __restrict__ v, size_t nrow, s
 // db[c] = sum over n and the HW plane of dy[n][c][:].  A CTA walks its slice of
 // the channel's flattened (n, i) index space; with up to eight slices per
 // channel they form a cluster and the call is one launch (see above), else the
-// partials are added by chansum_finish_kernel.
-template <bool VEC>
+// partials are added by chansum_finish_kernel.  RELU as in colsum_kernel.
+template <bool VEC, bool RELU>
 __global__ void __launch_bounds__(kBlock)
-chansum_kernel(const float* __restrict__ dy, float* __restrict__ out, int N, int C,
+chansum_kernel(const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx,
+               float* __restrict__ out, int N, int C,
                int HW, int per_slice, int slices, bool clustered) {
   __shared__ float sm[32];
   __shared__ float part[kMaxCluster];
@@ -222,12 +254,25 @@ chansum_kernel(const float* __restrict__ dy, float* __restrict__ out, int N, int
   const int dn = kBlock / hwu, dq = kBlock - dn * hwu;
 #pragma unroll 4
   for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
-    const float* p = dy + (static_cast<size_t>(n) * C + c) * HW + static_cast<size_t>(q) * kW;
+    const size_t at = (static_cast<size_t>(n) * C + c) * HW + static_cast<size_t>(q) * kW;
     if (VEC) {
-      const float4 v = *reinterpret_cast<const float4*>(p);
+      float4 v = *reinterpret_cast<const float4*>(dy + at);
+      if (RELU) {
+        const float4 m = *reinterpret_cast<const float4*>(x + at);
+        v.x = m.x > 0.f ? v.x : 0.f;
+        v.y = m.y > 0.f ? v.y : 0.f;
+        v.z = m.z > 0.f ? v.z : 0.f;
+        v.w = m.w > 0.f ? v.w : 0.f;
+        *reinterpret_cast<float4*>(dx + at) = v;
+      }
       acc += (v.x + v.y) + (v.z + v.w);
     } else {
-      acc += *p;
+      float v = dy[at];
+      if (RELU) {
+        v = x[at] > 0.f ? v : 0.f;
+        dx[at] = v;
+      }
+      acc += v;
     }
     n += dn;
     q += dq;
@@ -317,6 +362,49 @@ int sumall_parts(size_t n) {
 
 using namespace sgb;
 
+namespace {
+// The column sums of M, or (RELU) of dx = x > 0 ? M : 0, which is written as well.
+template <bool RELU>
+int column_sums(const float* M, const float* x, float* dx, float* v, size_t nrow, size_t ncol, void* ws,
+                size_t ws_bytes, cudaStream_t s) {
+  const ColsumPlan p = colsum_plan(nrow, ncol, ncol % 4 == 0 && aligned16(RELU ? dx : M));
+  if (p.blocks * p.slices > 0x7fffffffu) return SGB_ERR_SIZE;
+  const dim3 grid(static_cast<unsigned>(p.blocks * p.slices));
+  float* out = v;
+  if (!p.clustered) {
+    if (!ws || ws_bytes < static_cast<size_t>(p.slices) * ncol * sizeof(float)) return SGB_ERR_WORKSPACE;
+    out = static_cast<float*>(ws);
+  }
+  const int st = launch_ex(p.vec ? colsum_kernel<true, RELU> : colsum_kernel<false, RELU>, grid, dim3(kBlock), 0, s,
+                           p.clustered && p.slices > 1 ? p.slices : 0, true, M, x, dx, out, nrow, ncol,
+                           ceil_div(nrow, p.slices), p.slices, p.shift, p.clustered && p.slices > 1);
+  if (st != SGB_OK || p.clustered) return st;
+  return launch_ex(colsum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(ncol, kBlock))), dim3(kBlock), 0, s, 0,
+                   true, static_cast<const float*>(out), v, ncol, p.slices);
+}
+
+// The same over the channels of an NCHW tensor.
+template <bool RELU>
+int channel_sums(const float* dy, const float* x, float* dx, float* db, int N, int C, int HW, void* ws,
+                 size_t ws_bytes, cudaStream_t s) {
+  if (static_cast<long long>(N) * HW > 0x7fffffffLL || C > 65535) return SGB_ERR_SIZE;
+  bool clustered;
+  const int slices = chan_slices(N, C, HW, &clustered);
+  if (!ws || ws_bytes < static_cast<size_t>(slices) * C * sizeof(float)) return SGB_ERR_WORKSPACE;
+  const bool vec = (HW % 4 == 0) && aligned16(RELU ? dx : dy);
+  const int total = vec ? N * (HW / 4) : N * HW;
+  const int per_slice = static_cast<int>(ceil_div(total, slices));
+  if (slices == 1) clustered = false;     // the CTA's sum is the result
+  float* out = clustered || slices == 1 ? db : static_cast<float*>(ws);
+  const int st = launch_ex(vec ? chansum_kernel<true, RELU> : chansum_kernel<false, RELU>,
+                           dim3(static_cast<unsigned>(slices) * C), dim3(kBlock), 0, s, clustered ? slices : 0, true,
+                           dy, x, dx, out, N, C, HW, per_slice, slices, clustered);
+  if (st != SGB_OK || out == db) return st;
+  return launch_ex(chansum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(C, 128))), dim3(128), 0, s, 0, true,
+                   static_cast<const float*>(out), db, C, slices);
+}
+}  // namespace
+
 extern "C" {
 
 size_t sgb_sum_rows_workspace_bytes(size_t nrow, size_t ncol) {
@@ -335,23 +423,20 @@ int sgb_sum_rows_f32(const float* M, float* v, size_t nrow, size_t ncol, void* w
                      size_t ws_bytes, void* stream) {
   if (ncol == 0) return SGB_OK;
   if (!v) return SGB_ERR_NULL;
-  cudaStream_t s = as_stream(stream);
   if (nrow == 0) return sgb_set_f32(0.f, v, ncol, stream);
   if (!M) return SGB_ERR_NULL;
-  const ColsumPlan p = colsum_plan(nrow, ncol, ncol % 4 == 0 && aligned16(M));
-  if (p.blocks * p.slices > 0x7fffffffu) return SGB_ERR_SIZE;
-  const dim3 grid(static_cast<unsigned>(p.blocks * p.slices));
-  float* out = v;
-  if (!p.clustered) {
-    if (!ws || ws_bytes < static_cast<size_t>(p.slices) * ncol * sizeof(float)) return SGB_ERR_WORKSPACE;
-    out = static_cast<float*>(ws);
+  return column_sums<false>(M, nullptr, nullptr, v, nrow, ncol, ws, ws_bytes, as_stream(stream));
+}
+
+int sgb_relu_backward_sum_rows_f32(const float* dy, const float* x, float* dx, float* v, size_t nrow, size_t ncol,
+                                   void* ws, size_t ws_bytes, void* stream) {
+  if (nrow && ncol && (!dy || !x || !dx)) return SGB_ERR_NULL;
+  // vectors or not is decided by dx, as when it is summed by itself
+  if (nrow == 0 || ncol == 0 || !v || (aligned16(dx) && !(aligned16(dy) && aligned16(x)))) {
+    const int st = sgb_relu_backward_f32(dy, x, dx, nrow * ncol, stream);
+    return st != SGB_OK ? st : sgb_sum_rows_f32(dx, v, nrow, ncol, ws, ws_bytes, stream);
   }
-  const int st = launch_ex(p.vec ? colsum_kernel<true> : colsum_kernel<false>, grid, dim3(kBlock), 0, s,
-                           p.clustered && p.slices > 1 ? p.slices : 0, true, M, out, nrow, ncol,
-                           ceil_div(nrow, p.slices), p.slices, p.shift, p.clustered && p.slices > 1);
-  if (st != SGB_OK || p.clustered) return st;
-  return launch_ex(colsum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(ncol, kBlock))), dim3(kBlock), 0, s, 0,
-                   true, static_cast<const float*>(out), v, ncol, p.slices);
+  return column_sums<true>(dy, x, dx, v, nrow, ncol, ws, ws_bytes, as_stream(stream));
 }
 
 int sgb_sum_columns_f32(const float* M, float* v, size_t nrow, size_t ncol, void* stream) {
@@ -384,22 +469,19 @@ int sgb_conv_bias_backward_f32(const float* dy, float* db, int N, int C, int HW,
   if (!db) return SGB_ERR_NULL;
   if (N == 0 || HW == 0) return sgb_set_f32(0.f, db, C, stream);
   if (!dy) return SGB_ERR_NULL;
-  if (static_cast<long long>(N) * HW > 0x7fffffffLL || C > 65535) return SGB_ERR_SIZE;
-  bool clustered;
-  const int slices = chan_slices(N, C, HW, &clustered);
-  if (!ws || ws_bytes < static_cast<size_t>(slices) * C * sizeof(float)) return SGB_ERR_WORKSPACE;
-  const bool vec = (HW % 4 == 0) && aligned16(dy);
-  const int total = vec ? N * (HW / 4) : N * HW;
-  const int per_slice = static_cast<int>(ceil_div(total, slices));
-  cudaStream_t s = as_stream(stream);
-  if (slices == 1) clustered = false;     // the CTA's sum is the result
-  float* out = clustered || slices == 1 ? db : static_cast<float*>(ws);
-  const int st = launch_ex(vec ? chansum_kernel<true> : chansum_kernel<false>,
-                           dim3(static_cast<unsigned>(slices) * C), dim3(kBlock), 0, s, clustered ? slices : 0, true,
-                           dy, out, N, C, HW, per_slice, slices, clustered);
-  if (st != SGB_OK || out == db) return st;
-  return launch_ex(chansum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(C, 128))), dim3(128), 0, s, 0, true,
-                   static_cast<const float*>(out), db, C, slices);
+  return channel_sums<false>(dy, nullptr, nullptr, db, N, C, HW, ws, ws_bytes, as_stream(stream));
+}
+
+int sgb_relu_backward_conv_bias_f32(const float* dy, const float* x, float* dx, float* db, int N, int C, int HW,
+                                    void* ws, size_t ws_bytes, void* stream) {
+  if (N < 0 || C < 0 || HW < 0) return SGB_ERR_SIZE;
+  const size_t n = static_cast<size_t>(N) * C * HW;
+  if (n && (!dy || !x || !dx)) return SGB_ERR_NULL;
+  if (n == 0 || !db || (aligned16(dx) && !(aligned16(dy) && aligned16(x)))) {
+    const int st = sgb_relu_backward_f32(dy, x, dx, n, stream);
+    return st != SGB_OK ? st : sgb_conv_bias_backward_f32(dx, db, N, C, HW, ws, ws_bytes, stream);
+  }
+  return channel_sums<true>(dy, x, dx, db, N, C, HW, ws, ws_bytes, as_stream(stream));
 }
 
 size_t sgb_sum_all_workspace_bytes(size_t n) {

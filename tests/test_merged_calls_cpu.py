@@ -1,0 +1,32 @@
+"""Which neighbours of a bound call list are merged (host logic only)."""
+from singa_b200.hot_path import merge_calls
+
+
+def test_pairs_merge_only_when_one_feeds_the_other():
+    S = "STREAM"
+    relu = ("sgb_relu_backward_f32", (1, 2, 3, 12, S))
+    rows = ("sgb_sum_rows_f32", (3, 4, 3, 4, 5, 6, S))
+    chan = ("sgb_conv_bias_backward_f32", (3, 4, 2, 3, 2, 5, 6, S))
+    assert merge_calls([relu, rows]) == [("sgb_relu_backward_sum_rows_f32", (1, 2, 3, 4, 3, 4, 5, 6, S))]
+    assert merge_calls([relu, chan]) == [("sgb_relu_backward_conv_bias_f32", (1, 2, 3, 4, 2, 3, 2, 5, 6, S))]
+    for other in ([("sgb_relu_backward_f32", (1, 2, 9, 12, S)), rows], [relu, ("grad_ready", "w"), rows],
+                  [relu, ("sgb_sum_rows_f32", (3, 4, 3, 3, 5, 6, S))]):
+        assert merge_calls(other) == other
+    join = ("sgb_add_relu_backward_f32", (1, 2, 3, 4, 24, S))
+    bn = ("sgb_bn_backward_f32", (10, 4, 11, 12, 13, 14, 15, 16, 2, 3, 4, 17, 18, S))
+    assert merge_calls([join, bn]) == [
+        ("sgb_bn_add_relu_backward_f32", (10, 1, 2, 3, 11, 12, 13, 4, 14, 15, 16, 2, 3, 4, 17, 18, S))]
+    wide = [("sgb_add_relu_backward_f32", (1, 2, 3, 4, 1 << 24, S)),
+            ("sgb_bn_backward_f32", (10, 4, 11, 12, 13, 14, 15, 16, 1 << 10, 1 << 10, 16, 17, 18, S))]
+    assert merge_calls(wide) == wide
+
+
+def test_the_loss_head_becomes_one_call():
+    S = "STREAM"
+    head = [("sgb_softmax_rows_f32", (1, 2, 8, 10, S)), ("sgb_cross_entropy_f32", (1, 8, 10, 2, 3, 4, S)),
+            ("sgb_sum_all_f32", (4, 5, 8, 6, 7, S)), ("sgb_softmax_cross_entropy_bwd_f32", (1, 8, 10, 2, 3, 9, S)),
+            ("sgb_scalar_f32", (1, 9, 0.125, 9, 80, S))]
+    assert merge_calls(head) == [("sgb_softmax_cross_entropy_fused_f32", (1, 3, 8, 10, 0.125, 2, 4, 9, S)), head[2]]
+    other = list(head)
+    other[3] = ("sgb_softmax_cross_entropy_bwd_f32", (1, 8, 10, 12, 3, 9, S))    # another tensor's probabilities
+    assert merge_calls(other)[:3] == other[:3]
