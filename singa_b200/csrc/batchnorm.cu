@@ -201,6 +201,19 @@ __device__ unsigned g_cluster_faults;
 // the ReLU input; it is formed while staging, kept in shared memory for the
 // two later phases and ALSO written to `joined` for the other consumers of the
 // join (the shortcut branch), which replaces a separate join+ReLU kernel.
+// This thread's units of a share, for L2 (see prefetch_l2): x and, where there
+// is one, the ReLU's input.
+__device__ __forceinline__ void prefetch_share(const float* x, const float* relu_in, int first, int u1, int threads,
+                                               int hwu, size_t plane_stride, size_t chan_off) {
+
+  UnitWalk w(first, threads, hwu);
+  for (int u = first; u < u1; u += threads, w.next()) {
+    const size_t off = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * 4;
+    prefetch_l2(x + off);
+    if (relu_in) prefetch_l2(relu_in + off);
+  }
+}
+
 template <bool VEC, int MASK, int T, bool ADD = false>
 __global__ void __launch_bounds__(T)
 bn_bwd_cluster_kernel(const float* __restrict__ x, const float* __restrict__ dy,
@@ -231,6 +244,7 @@ bn_bwd_cluster_kernel(const float* __restrict__ x, const float* __restrict__ dy,
   float* sg = stage + static_cast<size_t>(per_cta) * kW;
   const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW;
   const size_t chan_off = static_cast<size_t>(c) * sh.HW;
+  if (VEC && first_wave(2)) prefetch_share(x, MASK == 1 || ADD ? relu_in : nullptr, first, u1, T, hwu, plane_stride, chan_off);
   dependency_wait();                                  // first access to global memory follows
   const float mu = mean[c];
   // units of one copy group per thread (the same in every thread: kCopyGroups * group_units covers a share)
@@ -631,9 +645,6 @@ bn_bwd_small_kernel(const float* __restrict__ x, const float* __restrict__ dy, c
   __shared__ float sm[2 * G / 32];
   const int c = G == 32 ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
   const int t = G == 32 ? threadIdx.x & 31 : threadIdx.x;
-  dependency_wait();
-  release_dependents();
-  if (c >= sh.C) return;
   const int hwu = sh.HW / kW, total = sh.N * hwu;
   const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
   float vx[NV][kW], vg[NV][kW];
@@ -642,6 +653,18 @@ bn_bwd_small_kernel(const float* __restrict__ x, const float* __restrict__ dy, c
 #pragma unroll
   for (int k = 0; k < NV; ++k, w.next()) {
     off[k] = w.n * plane_stride + chan_off + static_cast<size_t>(w.q) * kW;
+    if (c < sh.C && t + k * G < total) {
+      prefetch_l2(x + off[k]);
+      if (MASK == 1 || MASK == 3) prefetch_l2(relu_in + off[k]);
+      if (MASK == 3) prefetch_l2(dy_b + off[k]);
+    }
+  }
+  if (c < sh.C && t < 3) prefetch_l2((t == 0 ? mean : t == 1 ? invstd : scale) + c);
+  dependency_wait();
+  release_dependents();
+  if (c >= sh.C) return;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
     const bool in = t + k * G < total;
     if (VEC) {
       Vec4f a, b, m, e;
@@ -1121,6 +1144,7 @@ bn_bwd_hybrid_kernel(const float* __restrict__ x, const float* __restrict__ dy, 
   float* const sx = stage + static_cast<size_t>(threadIdx.x) * 4;                             // unit k at k * T * 4
   float* const sg = stage + static_cast<size_t>(per_cta) * 4 + static_cast<size_t>(threadIdx.x) * 4;   // k >= R, at (k - R) * T * 4
   const size_t plane_stride = static_cast<size_t>(sh.C) * sh.HW, chan_off = static_cast<size_t>(c) * sh.HW;
+  if (first_wave(1)) prefetch_share(x, RELU ? relu_in : nullptr, first, u1, T, hwu, plane_stride, chan_off);
   dependency_wait();
   const float mu = mean[c];
   Vec4f g[R];

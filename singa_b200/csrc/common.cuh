@@ -92,6 +92,19 @@ inline unsigned capped_grid(size_t work_items, size_t per_cta, int ctas_per_sm) 
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Before dependency_wait() a kernel may still ask for lines to be brought into
+// L2: that reads no value, so it cannot see a stale one, and whatever an earlier
+// kernel of the stream writes goes through the same L2.  The CTAs of the first
+// wave ask for the operands that no running kernel is likely to produce
+// (activations, parameters, momentum) and so wait for DRAM while the previous
+// kernel drains.  Later waves find that kernel finished and load at once.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ bool first_wave(unsigned ctas_per_sm) {
+  unsigned sms;
+  asm("mov.u32 %0, %%nsmid;" : "=r"(sms));
+  return blockIdx.x < sms * ctas_per_sm;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

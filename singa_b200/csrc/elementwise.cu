@@ -39,6 +39,16 @@ ew_vec_kernel(F f, const uint4* __restrict__ a, const uint4* __restrict__ b, con
               uint4* __restrict__ out, size_t nvec, int rest) {
   constexpr int lanes = 16 / sizeof(TO);
   const size_t tile = static_cast<size_t>(kBlock) * kUnroll;
+  if (IN >= 2 && first_wave(8)) {                      // the first operand is the gradient that just came out
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const size_t i = blockIdx.x * tile + u * kBlock + threadIdx.x;
+      if (i < nvec) {
+        prefetch_l2(b + i);
+        if (IN >= 3) prefetch_l2(c + i);
+      }
+    }
+  }
   dependency_wait();
   for (size_t base = blockIdx.x * tile; base < nvec; base += gridDim.x * tile) {
     uint4 va[kUnroll], vb[kUnroll], vc[kUnroll];

@@ -71,7 +71,6 @@ __device__ __forceinline__ void sgd_one(float& p, float g, float& m, const SgdAr
 template <int N>
 __global__ void __launch_bounds__(kBlock)
 sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
-  dependency_wait();
   const int k = find_tensor(t, blockIdx.x);
   const size_t n = t.n[k];
   const size_t base = static_cast<size_t>(blockIdx.x - t.first_tile[k]) * kTile;
@@ -81,6 +80,11 @@ sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                      (a.use_momentum ? reinterpret_cast<uintptr_t>(m) : 0)) & 15u) == 0;
   const size_t i = base + 4 * threadIdx.x;
+  if (vec && i + 4 <= n && first_wave(8)) {
+    prefetch_l2(p + i);
+    if (a.use_momentum) prefetch_l2(m + i);
+  }
+  dependency_wait();
   if (vec && i + 4 <= n) {
     Vec4f vp, vg, vm;
     vp.u = ld128(p + i);

@@ -876,10 +876,7 @@ pool_k2s2_kernel(const PairArgs a) {
   constexpr bool kBackward = MODE == kMaxBwd || MODE == kMaxBwdRecord || MODE == kAvgBwd;
   constexpr bool kNeedsX = MODE != kMaxBwdRecord && MODE != kAvgBwd;
   constexpr bool kMax = MODE <= kMaxBwdRecord;
-  dependency_wait();
-  release_dependents();
   const unsigned i = blockIdx.x * static_cast<unsigned>(kBlock) + threadIdx.x;
-  if (i >= a.work) return;
   const unsigned line = a.quads.quot(i);
   const int c = 4 * static_cast<int>(i - line * a.quads.d);
   const unsigned plane = a.pairs.quot(line);
@@ -888,6 +885,13 @@ pool_k2s2_kernel(const PairArgs a) {
   const size_t win = (static_cast<size_t>(plane) * a.OH + m) * a.OW + c / 2;
   const bool second_row = h + 1 < a.H;
   const bool exists[2] = {second_row && c + 1 < a.W, second_row && c + 3 < a.W};
+  if (kBackward && kNeedsX && i < a.work) {
+    prefetch_l2(a.x + in0);
+    if (second_row) prefetch_l2(a.x + in0 + a.W);
+  }
+  dependency_wait();
+  release_dependents();
+  if (i >= a.work) return;
   float v[2][4];
   if (kNeedsX) {
 #pragma unroll

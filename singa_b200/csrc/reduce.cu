@@ -42,8 +42,6 @@ colsum_kernel(const float* __restrict__ M, const float* __restrict__ x, float* _
   constexpr int kW = VEC ? 4 : 1;
   __shared__ float sm[kWarps][32 * kW];
   __shared__ float part[kMaxCluster][32 * kW];
-  dependency_wait();
-  release_dependents();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const size_t block = blockIdx.x / slices;
   const int slice = static_cast<int>(blockIdx.x - block * slices);
@@ -67,6 +65,14 @@ colsum_kernel(const float* __restrict__ M, const float* __restrict__ x, float* _
     v = m > 0.f ? v : 0.f;
     dx[at] = v;
   };
+  if (RELU && c < ncol) {
+    size_t r = r0 + w * rows_abreast + (lane >> shift);
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+      if (r + k * step < r1) prefetch_l2(x + c + (r + k * step) * ncol);
+  }
+  dependency_wait();
+  release_dependents();
   if (c < ncol) {
     const float* p = M + c;
     size_t r = r0 + w * rows_abreast + (lane >> shift);
@@ -242,8 +248,6 @@ chansum_kernel(const float* __restrict__ dy, const float* __restrict__ x, float*
                int HW, int per_slice, int slices, bool clustered) {
   __shared__ float sm[32];
   __shared__ float part[kMaxCluster];
-  dependency_wait();
-  release_dependents();
   const int c = static_cast<int>(blockIdx.x / slices), slice = static_cast<int>(blockIdx.x - c * slices);
   constexpr int kW = VEC ? 4 : 1;
   const int hwu = HW / kW, total = N * hwu;
@@ -252,6 +256,20 @@ chansum_kernel(const float* __restrict__ dy, const float* __restrict__ x, float*
   // (sample, position) of the unit is advanced without a division per step
   int n = (i0 + static_cast<int>(threadIdx.x)) / hwu, q = (i0 + static_cast<int>(threadIdx.x)) - n * hwu;
   const int dn = kBlock / hwu, dq = kBlock - dn * hwu;
+  if (RELU && first_wave(8)) {
+    int pn = n, pq = q;
+    for (int k = 0, i = i0 + threadIdx.x; k < 4 && i < i1; ++k, i += kBlock) {
+      prefetch_l2(x + (static_cast<size_t>(pn) * C + c) * HW + static_cast<size_t>(pq) * kW);
+      pn += dn;
+      pq += dq;
+      if (pq >= hwu) {
+        pq -= hwu;
+        ++pn;
+      }
+    }
+  }
+  dependency_wait();
+  release_dependents();
 #pragma unroll 4
   for (int i = i0 + threadIdx.x; i < i1; i += kBlock) {
     const size_t at = (static_cast<size_t>(n) * C + c) * HW + static_cast<size_t>(q) * kW;

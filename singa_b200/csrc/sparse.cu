@@ -656,8 +656,6 @@ struct TopkArgs {
   bool vec;
 };
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 // s of one element.
 __device__ __forceinline__ float element(const NoPieces&, const float* g, const float* acc, size_t i) {
   return acc ? g[i] + acc[i] : g[i];
