@@ -21,7 +21,8 @@
 //
 // What bounds them: HBM.  g and the residual are read once, the residual is
 // written once (12 B/element); the top-K form reads the residual once more
-// (4 B/element) after the first radix digit is decided.  All index arithmetic
+// (4 B/element) after the first radix digit is decided, unless a sample has
+// bounded the k-th key before (large gradients).  All index arithmetic
 // that reaches the payload is 1-based int32, the reference's wire format.
 #include <cooperative_groups.h>
 
