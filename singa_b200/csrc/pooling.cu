@@ -576,7 +576,8 @@ pool_k3s2p1_kernel(const StripArgs a) {
   if (kBackward && m1 == OH) store_row(2 * OH - 1, pend);   // below it there is no further window
 }
 
-StripArgs strip_args(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p) {
+StripArgs strip_args(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p,
+                     long long warps_per_sm = 96) {
   StripArgs a;
   a.x = x;
   a.dy = dy;
@@ -592,9 +593,10 @@ StripArgs strip_args(const float* x, const float* dy, float* out, unsigned char*
   a.segments = a.quads <= 32 ? 1 : (a.quads + 29) / 30;
   // A band re-reads the row above it (and, backward, works out the window rows
   // at its edges twice), so bands are as tall as leaves about three warps per
-  // slot of the machine (32 per SM), at least four window rows.
+  // slot of the machine (32 per SM), at least four window rows.  Where the extra
+  // rows cost the most (`warps_per_sm`, see launch_k3s1p1) they are taller.
   const long long strips = static_cast<long long>((a.planes + a.abreast - 1) / a.abreast) * a.segments;
-  const long long want = (static_cast<long long>(sm_count()) * 96 + strips - 1) / strips;   // bands wanted
+  const long long want = (static_cast<long long>(sm_count()) * warps_per_sm + strips - 1) / strips;   // bands wanted
   long long rows = (p.OH + want - 1) / want;
   if (rows < 4) rows = 4;
   if (rows > p.OH) rows = p.OH;
@@ -834,7 +836,12 @@ pool_k3s1p1_kernel(const StripArgs a) {
 
 template <int MODE>
 int launch_k3s1p1(const float* x, const float* dy, float* out, unsigned char* record, const PoolShape& p, cudaStream_t s) {
-  const StripArgs a = strip_args(x, dy, out, record, p);
+  // Backward, a band works out two window rows more than it owns, and comparisons
+  // are what bounds it: bands twice as tall (1.5 warps per slot) were as fast or
+  // faster on each of ten shapes: 32x64x112x112 115.0 -> 104.8 us, 16x128x56x56
+  // 43.5 -> 38.1, 64x512x14x14 44.8 -> 34.7; fewer warps than that idle the machine.
+  constexpr bool kBackward = MODE == kMaxBwd || MODE == kMaxBwdRecord;
+  const StripArgs a = strip_args(x, dy, out, record, p, kBackward ? 48 : 96);
   const long long ctas = strip_ctas(a);
   if (ctas > 0x7fffffffLL) return SGB_ERR_SIZE;
   const bool vec = p.W % 4 == 0 && (!x || aligned16(x)) && (!dy || aligned16(dy)) && aligned16(out) &&
