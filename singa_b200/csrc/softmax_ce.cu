@@ -147,8 +147,11 @@ softmax_ce_fused_kernel(const float* __restrict__ x, const int* __restrict__ tgt
   const size_t row = T == 32 ? blockIdx.x * 4ull + (threadIdx.x >> 5) : blockIdx.x;
   const int t = T == 32 ? threadIdx.x & 31 : threadIdx.x;
   if (row >= nrow) return;
-  const size_t hot = static_cast<size_t>(tgt[row]);
-  if (hot >= ncol && t == 0) loss[row] = __int_as_float(0x7fc00000);   // label out of range: NaN, not stale memory
+  // a label out of range is no slot's number: the threads hold more slots than the row has elements
+  const int label = tgt[row];
+  const bool known = label >= 0 && static_cast<size_t>(label) < ncol;
+  const size_t hot = known ? static_cast<size_t>(label) : ~size_t{0};
+  if (!known && t == 0) loss[row] = __int_as_float(0x7fc00000);        // NaN, not stale memory
   Row<float, T, NV> r;
   r.softmax(x + row * ncol, ncol, vec, t, sm);
 #pragma unroll
