@@ -682,7 +682,9 @@ int sgb_comm_sparsification_end(sgb_comm *c, void *compute_stream);
  * per bucket.  SGB_ERR_UNSUPPORTED (nothing done) where that is what it takes:
  * more ranks, profiling on, an exchange open, a bucket above the capacity or of
  * more than 2^25 elements or 256 runs of tensors, a residual that is missing or
- * not on a 16-byte boundary. */
+ * not on a 16-byte boundary, and while the compute stream is being captured if
+ * the communicator has not selected as wide a list before (its buffers for this
+ * form grow outside captures only, and stay valid for graphs that hold them). */
 int sgb_comm_sparsification_buckets(sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
                                     float *const *accumulations, size_t nbuckets, float threshold,
                                     void *compute_stream);

@@ -86,11 +86,12 @@ struct sgb_comm {
     std::vector<size_t> sizes;
   };
   Sparse sparse[2];
-  // One rank's joint selection over several buckets; grows to the largest span
+  // One rank's joint selection over several buckets; grows with the largest span
   // that was asked for (at most kMaxBucketSpan), freed with the communicator.
   int *joint_pay = nullptr, *joint_nnz = nullptr;
   void* joint_ws = nullptr;
   size_t joint_elems = 0, joint_ws_bytes = 0;
+  std::vector<void*> joint_retired;
   unsigned sparse_begun = 0, sparse_ended = 0;
   unsigned long long* dropped_dev = nullptr;   // entries the bounded threshold form left for later calls
   int topk_mode = 1;           // 1 = the reference comparator's key, 0 = |value|
@@ -382,6 +383,7 @@ int sgb_comm_destroy(sgb_comm* c) {
   if (c->joint_pay) cudaFree(c->joint_pay);
   if (c->joint_nnz) cudaFree(c->joint_nnz);
   if (c->joint_ws) cudaFree(c->joint_ws);
+  for (void* b : c->joint_retired) cudaFree(b);
   drop_ranges(c);
   cudaEvent_t evs[] = {c->ev_compute, c->ev_c1, c->ev_s, c->ev_c2, c->ev_c2_done, c->prof_origin};
   for (cudaEvent_t e : evs)
@@ -837,21 +839,36 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
   return emit(c, p.post, nullptr);
 }
 
-static int joint_reserve(sgb_comm* c, size_t span) {
+// Room for a joint selection over `span` elements, ahead of any work of the call
+// (c1 has not joined a capture of the compute stream yet).  Outgrown buffers are
+// kept until the communicator goes: their addresses may sit in a captured graph
+// or in queued work.  Doubling keeps their sum below twice the size of the last one.
+static int joint_reserve(sgb_comm* c, size_t span, cudaStream_t compute) {
   if (span <= c->joint_elems) return SGB_OK;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c->c1, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return SGB_ERR_UNSUPPORTED;
-  CU(cudaStreamSynchronize(c->c1));                    // the old buffers may be in use there
-  CU(cudaFree(c->joint_pay));
-  CU(cudaFree(c->joint_ws));
-  c->joint_pay = nullptr;
-  c->joint_ws = nullptr;
-  c->joint_elems = 0;
-  c->joint_ws_bytes = sgb_sparse_workspace_bytes(span);
+  for (cudaStream_t st : {compute, c->c1}) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
+      cudaGetLastError();          // the default stream beside another stream's capture: no place to allocate either
+      return SGB_ERR_UNSUPPORTED;
+    }
+    if (capturing != cudaStreamCaptureStatusNone) return SGB_ERR_UNSUPPORTED;
+  }
+  size_t elems = 2 * c->joint_elems;
+  if (elems > sgb::kMaxBucketSpan) elems = sgb::kMaxBucketSpan;
+  if (elems < span) elems = span;
+  const size_t ws_bytes = sgb_sparse_workspace_bytes(elems);
+  int* pay = nullptr;
+  void* ws = nullptr;
   if (!c->joint_nnz) CU(cudaMalloc(&c->joint_nnz, sizeof(int)));
-  CU(cudaMalloc(&c->joint_pay, 2 * span * sizeof(int)));
-  CU(cudaMalloc(&c->joint_ws, c->joint_ws_bytes));
-  c->joint_elems = span;
+  CU(cudaMalloc(&pay, 2 * elems * sizeof(int)));
+  if (c->joint_pay) c->joint_retired.push_back(c->joint_pay);
+  c->joint_pay = pay;
+  c->joint_elems = 0;              // until the workspace is there as well
+  CU(cudaMalloc(&ws, ws_bytes));
+  if (c->joint_ws) c->joint_retired.push_back(c->joint_ws);
+  c->joint_ws = ws;
+  c->joint_ws_bytes = ws_bytes;
+  c->joint_elems = elems;
   return SGB_OK;
 }
 
@@ -888,7 +905,7 @@ int sgb_comm_sparsification_buckets(sgb_comm* c, void* const* tensors, const siz
     widest = span > widest ? span : widest;
     k = end;
   }
-  OK(joint_reserve(c, widest));
+  OK(joint_reserve(c, widest, sgb::as_stream(compute_stream)));
   OK(emit(c, plan_call(c, sgb::order::kStageCopy).pre, sgb::as_stream(compute_stream)));
   Phase ph(c, "Dist_c1c2_fusedSparsification", sgb::order::kStreamC1);
   size_t k = 0;
