@@ -224,7 +224,9 @@ class DistOpt(object):
                                    corr=True):
         """opt.py:994-1094: sparsified synchronisation with local residuals."""
         import torch
-        if not hasattr(self, "sparsInit") and corr:
+        if corr and not getattr(self, "sparsInit", False):
+            # also when an earlier first pass was cut short: a part of the list would
+            # hand each bucket another bucket's residual
             self.gradAccumulation = []
             self.sparsInit = False
         names, params, grads, k = [], [], [], -1
@@ -263,8 +265,8 @@ class DistOpt(object):
                 begin(tensors, res, spars, topK)
                 opened += 1
                 if opened == 2:
-                    self.communicator.endSparsification()
                     opened = 1
+                    self.communicator.endSparsification()
             elif single:
                 self.sparsification(tensors[0], res, spars, topK)
             else:
@@ -272,21 +274,26 @@ class DistOpt(object):
 
         # On one rank, gradients that all exist already go through one selection.
         joint = getattr(self.communicator, "sparsifyBuckets", None)
-        if (joint is not None and corr and not topK and self.world_size == 1 and
-                type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
-            ready = []
-            for tensors, n, single in buckets():
-                k += 1
-                ready.append((tensors, residual(n, tensors[0]), single))
-            if not ready or not joint([b[0] for b in ready], [b[1] for b in ready], spars):
-                for b in ready:
-                    exchange(*b)
-        else:
-            for tensors, n, single in buckets():
-                k += 1
-                exchange(tensors, residual(n, tensors[0]), single)
-        if opened:
-            self.communicator.endSparsification()
-        self.wait()
+        try:
+            if (joint is not None and corr and not topK and self.world_size == 1 and
+                    type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
+                ready = []
+                for tensors, n, single in buckets():
+                    k += 1
+                    ready.append((tensors, residual(n, tensors[0]), single))
+                if not ready or not joint([b[0] for b in ready], [b[1] for b in ready], spars):
+                    for b in ready:
+                        exchange(*b)
+            else:
+                for tensors, n, single in buckets():
+                    k += 1
+                    exchange(tensors, residual(n, tensors[0]), single)
+        finally:
+            # Whatever the stream or an exchange raised: one left open would refuse every
+            # later call, and without wait() the side streams could still be reading
+            # tensors that the unwinding frees.
+            if opened:
+                self.communicator.endSparsification()
+            self.wait()
         self.sparsInit = True
         self._update_all((names, params, grads))
