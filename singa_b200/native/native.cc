@@ -333,12 +333,23 @@ PyObject* py_sum_columns(Args a, Py_ssize_t) {   // (M, v | None)
   ISSUE(sgb_sum_columns_f32, f32(M), f32w(v), r, c, stream());
   return made.defined() ? wrap(std::move(made)) : same(a[1]);
 }
+// The first two sizes, whatever else the shape holds (IndexError below two).
+void leading_sizes(const Tensor& t, int64_t* n, int64_t* c) {
+  if (t.dim() < 2) fail(PyExc_IndexError, "a tensor of at least two dimensions is expected");
+  *n = t.size(0);
+  *c = t.size(1);
+}
+// a / b as Python's a // b answers it: an empty batch is an error of the caller
+int64_t divide(int64_t a, int64_t b) {
+  if (b == 0) fail(PyExc_ZeroDivisionError, "an empty batch has no size per sample");
+  return a / b;
+}
 PyObject* py_row_max(Args a, Py_ssize_t) {
   const Tensor& M = dev(a[0]);
-  size_t r, c;
-  rows_cols(M, &r, &c);
-  Tensor v = fresh({M.size(0)}, at::kFloat, M);
-  ISSUE(sgb_row_max_f32, f32(M), f32w(v), r, c, stream());
+  int64_t r, c;
+  leading_sizes(M, &r, &c);
+  Tensor v = fresh({r}, at::kFloat, M);
+  ISSUE(sgb_row_max_f32, f32(M), f32w(v), static_cast<size_t>(r), static_cast<size_t>(c), stream());
   return wrap(std::move(v));
 }
 PyObject* py_sum_all(Args a, Py_ssize_t) {
@@ -382,8 +393,10 @@ PyObject* py_dgmm(Args a, Py_ssize_t) {          // (right, M, v)
 }
 PyObject* py_conv_bias_backward(Args a, Py_ssize_t) {
   const Tensor& dy = dev(a[0]);
-  const int n = static_cast<int>(dy.size(0)), c = static_cast<int>(dy.size(1));
-  const int hw = static_cast<int>(dy.numel() / (static_cast<int64_t>(n) * c));
+  int64_t batch, channels;
+  leading_sizes(dy, &batch, &channels);
+  const int n = static_cast<int>(batch), c = static_cast<int>(channels);
+  const int hw = static_cast<int>(divide(dy.numel(), batch * channels));
   Tensor db = fresh({c}, at::kFloat, dy);
   const Ws ws(dy, sgb_conv_bias_backward_workspace_bytes(n, c, hw));
   ISSUE(sgb_conv_bias_backward_f32, f32(dy), f32w(db), n, c, hw, ws.ptr, ws.bytes, stream());
@@ -405,7 +418,7 @@ struct CeDims {
   int int_target;
   CeDims(const Tensor& p, const Tensor& t) {
     batch = p.dim() == 2 ? static_cast<size_t>(p.size(0)) : 1;
-    dim = batch ? count(p) / batch : 0;
+    dim = static_cast<size_t>(divide(p.numel(), static_cast<int64_t>(batch)));
     require(t.scalar_type() == at::kInt, "targets are int32 (kInt) tensors");
     int_target = count(t) == batch;
   }
