@@ -609,6 +609,8 @@ int sgb_comm_order_plan(unsigned char *state4, int call, unsigned *edges4,
  * and switches timing off; *count receives the number of recorded phases.
  * Not usable while a stream is being captured (phases are then not timed). */
 int sgb_comm_profile_begin(sgb_comm *c, void *compute_stream);
+/* 1 between begin and end, else 0. */
+int sgb_comm_profiling(const sgb_comm *c);
 int sgb_comm_profile_range(sgb_comm *c, const char *name, int which, int begin);
 /* A named point in time on any stream (start == end in the rows). */
 int sgb_comm_profile_mark(sgb_comm *c, const char *name, void *stream);

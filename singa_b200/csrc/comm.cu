@@ -167,6 +167,15 @@ sgb::order::Step plan_call(sgb_comm* c, int call) {
   return p;
 }
 
+// True also if the question fails (the default stream beside another stream's
+// capture): no place for a timing event or an allocation either.
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 // A named phase on one of the side streams: an NVTX range around the enqueue
 // and, while profiling is on, an event pair on that stream.
 struct Phase {
@@ -176,9 +185,7 @@ struct Phase {
   size_t slot = 0;
   Phase(sgb_comm* comm, const char* name, int which) : c(comm), stream(side(comm, which)) {
     nvtxRangePushA(name);
-    if (!c->profiling) return;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return;
+    if (!c->profiling || capturing(stream)) return;
     sgb_comm::Range r;
     r.name = name;
     if (cudaEventCreate(&r.start) != cudaSuccess) return;
@@ -473,10 +480,12 @@ int sgb_comm_profile_begin(sgb_comm* c, void* compute_stream) {
   return SGB_OK;
 }
 
+int sgb_comm_profiling(const sgb_comm* c) { return c && c->profiling ? 1 : 0; }
+
 int sgb_comm_profile_range(sgb_comm* c, const char* name, int which, int begin) {
   if (!c || !name) return SGB_ERR_NULL;
   if (which < 0 || which > 2) return SGB_ERR_UNSUPPORTED;
-  if (!c->profiling) return SGB_OK;
+  if (!c->profiling || capturing(side(c, which))) return SGB_OK;
   if (begin) {
     sgb_comm::Range r;
     r.name = name;
@@ -493,7 +502,7 @@ int sgb_comm_profile_range(sgb_comm* c, const char* name, int which, int begin) 
 
 int sgb_comm_profile_mark(sgb_comm* c, const char* name, void* stream) {
   if (!c || !name) return SGB_ERR_NULL;
-  if (!c->profiling) return SGB_OK;
+  if (!c->profiling || capturing(sgb::as_stream(stream))) return SGB_OK;
   sgb_comm::Range r;
   r.name = name;
   CU(cudaEventCreate(&r.start));
@@ -845,14 +854,7 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
 // or in queued work.  Doubling keeps their sum below twice the size of the last one.
 static int joint_reserve(sgb_comm* c, size_t span, cudaStream_t compute) {
   if (span <= c->joint_elems) return SGB_OK;
-  for (cudaStream_t st : {compute, c->c1}) {
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
-      cudaGetLastError();          // the default stream beside another stream's capture: no place to allocate either
-      return SGB_ERR_UNSUPPORTED;
-    }
-    if (capturing != cudaStreamCaptureStatusNone) return SGB_ERR_UNSUPPORTED;
-  }
+  if (capturing(compute) || capturing(c->c1)) return SGB_ERR_UNSUPPORTED;
   size_t elems = 2 * c->joint_elems;
   if (elems > sgb::kMaxBucketSpan) elems = sgb::kMaxBucketSpan;
   if (elems < span) elems = span;

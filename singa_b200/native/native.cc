@@ -1024,7 +1024,7 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
   const Settings now{real(a[1]), real(a[2]), real(a[3]), sgb_get_option(SGB_OPT_OVERLAP_LAUNCHES),
                      current.device_index()};
   void* const st = current.stream();
-  const bool may_graph = prog->graphable && !profile &&
+  const bool may_graph = prog->graphable && !profile && !sgb_comm_profiling(prog->comm) &&
                          c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
   int status = SGB_OK;
   const char* where = "";
