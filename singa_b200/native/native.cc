@@ -892,13 +892,22 @@ struct Program {
   // 32 us launched one by one, 10 us as a graph).  Off for programs whose
   // launches must be made one by one (see HotPathGPU._record_program), while a
   // caller captures, and while the communicator's phases are timed.
+  //
+  // The settings are part of the launches, so a capture serves only as long as
+  // they last, and it costs about as much as kPaysAfter of its replays save (MLP
+  // of 8 kernels: 220 us against 6 us a run).  One that was replayed less than
+  // that has the next one wait for as many runs, and four times as many each time
+  // it happens again: a rate that changes every third run took 85-97 us a run,
+  // 14 us launched one by one.
   bool graphable = false;
   Settings seen{};
   unsigned streak = 0;        // runs in a row with `seen`
+  unsigned eager = 2;         // of which so many are launched one by one
+  unsigned captures = 0;
   cudaGraphExec_t exec = nullptr;
-  std::mutex guard;           // of the four fields above
+  std::mutex guard;           // of the five fields above
 };
-constexpr unsigned kEagerRuns = 2;
+constexpr unsigned kEagerRuns = 2, kPaysAfter = 40, kMostEagerRuns = 1u << 16;
 const char kProgramTag[] = "singa_b200.program";
 
 void drop_program(PyObject* capsule) {
@@ -1033,11 +1042,18 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
   if (may_graph) {
     const std::lock_guard<std::mutex> lock(prog->guard);
     if (!(prog->streak && prog->seen == now)) {
+      if (prog->streak > prog->eager) {                // there was a capture: did it pay?
+        const bool paid = prog->streak - prog->eager >= kPaysAfter;
+        prog->eager = paid ? kEagerRuns : std::min(std::max(kPaysAfter, 4 * prog->eager), kMostEagerRuns);
+      }
       prog->seen = now;
       prog->streak = 0;
     }
-    if (++prog->streak > kEagerRuns) {
-      if (prog->streak == kEagerRuns + 1 && !capture_calls(prog, now)) prog->graphable = false;
+    if (++prog->streak > prog->eager) {
+      if (prog->streak == prog->eager + 1) {
+        if (capture_calls(prog, now)) ++prog->captures;
+        else prog->graphable = false;
+      }
       if (prog->graphable) {
         launched = true;
         if (cudaGraphLaunch(prog->exec, static_cast<cudaStream_t>(st)) != cudaSuccess) {
@@ -1054,6 +1070,13 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
   Py_RETURN_NONE;
 }
 
+PyObject* py_program_captures(Args a, Py_ssize_t) {   // how often the library has captured the program
+  auto* prog = static_cast<Program*>(PyCapsule_GetPointer(a[0], kProgramTag));
+  if (!prog) throw PyError{};
+  const std::lock_guard<std::mutex> lock(prog->guard);
+  return PyLong_FromUnsignedLong(prog->captures);
+}
+
 // ------------------------------------------------------------------- module
 #define METHOD(name, least) \
   { #name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<py_##name, least>)), METH_FASTCALL, nullptr }
@@ -1065,7 +1088,7 @@ PyMethodDef kMethods[] = {
     METHOD(bn_backward, 9), METHOD(bn_add_relu_backward, 10), METHOD(pool_forward, 5), METHOD(pool_backward, 5),
     METHOD(pool_forward_argmax, 4), METHOD(pool_backward_argmax, 3), METHOD(sgd_multi, 9), METHOD(pack, 3), METHOD(unpack, 4),
     METHOD(comm_synch, 2), METHOD(comm_synch_half, 2), METHOD(comm_fused_synch, 3), METHOD(comm_fused_synch_half, 3),
-    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5),
+    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5), METHOD(program_captures, 1),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -39,3 +39,45 @@ def test_phases_are_timed_when_a_step_has_been_replayed(comm, dist_option):
         assert all(t1 >= t0 >= 0 for _, t0, t1 in rows)
         for _ in range(4):
             hp.run_step()
+
+
+def parameters(hp):
+    torch.cuda.synchronize()
+    return [hp.t[p].clone() for p in hp.plan["params"]]
+
+
+@pytest.mark.parametrize("every, most", [(0, 1), (1, 0), (2, 0), (3, 2), (4, 2), (50, 2)])
+def test_captures_are_few_when_the_rate_keeps_changing(every, most):
+    """A rate that changes every few runs makes one short-lived capture, and the
+    next one only after 40 runs, and then 160; 48 replays pay for a capture."""
+    from singa_b200 import _lib
+    hp, one_by_one = small_step(), small_step()
+    one_by_one.profile = True                   # never captured
+    for i in range(100):
+        if every and i % every == 0:
+            hp.lr = one_by_one.lr = 0.1 / (i + 1)
+        hp.run_step()
+        one_by_one.run_step()
+    assert _lib.native.program_captures(hp._program) <= most
+    assert _lib.native.program_captures(one_by_one._program) == 0
+    for a, b in zip(parameters(hp), parameters(one_by_one)):
+        assert torch.equal(a, b)
+    if every:                                   # settings that last are captured in the end
+        before = _lib.native.program_captures(hp._program)
+        for _ in range(170):
+            hp.run_step()
+        assert _lib.native.program_captures(hp._program) == before + (every not in (50,))
+
+
+def test_a_step_captured_by_its_owner_while_phases_are_timed(comm):
+    hp = small_step(comm)
+    hp.run_step()
+    torch.cuda.synchronize()
+    comm.profile_begin()
+    g = hp.capture()                            # no timing event goes into the graph
+    g.replay()
+    hp.run_step()
+    rows = comm.profile_end()
+    assert sum(n == "sgd_update_bucket" for n, _, _ in rows) == len(hp.events)
+    hp.release_graph()
+    del g
