@@ -339,7 +339,18 @@ class HotPathGPU(object):
                 tot = sum(sizes[i] for i in ev[1])
                 self.residuals[ev[1][-1]] = torch.zeros(tot, device=self.device)
 
+        self._recorded = self._exchange_settings()
         self._record_program()
+
+    def _exchange_settings(self):
+        """What the recorded program holds of its owner's attributes (the rates are
+        passed at every run).  The communicator counts as long as it is open: its
+        address stands in the program."""
+        c = self.comm
+        if c is not None and c._h is None:
+            raise _lib.SgbError("sgb_comm", -1, "the communicator is closed")
+        return (None if c is None else c._h.value, self.world, self.dist_option, self.spars,
+                self.update_on_arrival)
 
     # ----------------------------------------------------------------- program
     def _record_program(self):
@@ -439,6 +450,10 @@ class HotPathGPU(object):
     def run_step(self):
         """Enqueues one full step on the current stream (+ the communicator's
         side streams).  Returns the number of C-ABI calls issued."""
+        now = self._exchange_settings()
+        if now != self._recorded:
+            self._record_program()
+            self._recorded = now
         _lib.native.run_program(self._program, self.lr, self.momentum, self.weight_decay, self.profile)
         return self.calls_per_step
 

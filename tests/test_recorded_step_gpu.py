@@ -81,3 +81,50 @@ def test_a_step_captured_by_its_owner_while_phases_are_timed(comm):
     assert sum(n == "sgd_update_bucket" for n, _, _ in rows) == len(hp.events)
     hp.release_graph()
     del g
+
+
+def test_world_size_and_exchange_may_change_between_runs(comm):
+    a, b = small_step(), small_step(world=4)
+    for _ in range(4):                          # `a` has been captured by now
+        a.run_step()
+    a.world = 4
+    for hp in (a, b):
+        for p in hp.plan["params"]:
+            hp.t[p].fill_(0.5)
+            hp.moments[p].zero_()
+        hp.grad_arena.fill_(0.25)
+    assert a.run_step() == b.run_step()
+    for x, y in zip(parameters(a), parameters(b)):
+        assert torch.equal(x, y)
+    alone, at_the_end = small_step(comm), small_step(comm, update_on_arrival=False)
+    alone.run_step()
+    alone.update_on_arrival = False             # from here on one update behind the last exchange
+    at_the_end.run_step()
+    assert alone.run_step() == at_the_end.run_step()
+    for x, y in zip(parameters(alone), parameters(at_the_end)):
+        assert torch.equal(x, y)
+    top = small_step(comm, dist_option="sparseTopK", spars=0.5)
+    top.run_step()
+    top.spars = 0.01
+    top.run_step()
+    torch.cuda.synchronize()
+    largest_bucket = max(r.numel() for r in top.residuals.values())
+    kept = sum(int((r != 0).sum()) for r in top.residuals.values())
+    assert kept > 0.9 * largest_bucket          # nearly everything stays behind
+
+
+def test_a_closed_communicator_is_an_error():
+    from singa_b200 import _lib
+    from singa_b200.communicator import Communicator, NcclIdHolder
+    c = Communicator(torch.cuda.current_device(), 1, NcclIdHolder(), buffSize=1 << 20)
+    hp = small_step(c)
+    for _ in range(4):
+        hp.run_step()
+    torch.cuda.synchronize()
+    c.close()
+    with pytest.raises(_lib.SgbError, match="closed"):
+        hp.run_step()
+    hp.comm = None                              # without an exchange the step still runs
+    hp.update_on_arrival = False
+    assert hp.run_step() > 0
+    torch.cuda.synchronize()
