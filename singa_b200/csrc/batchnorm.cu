@@ -1384,6 +1384,15 @@ int bn_add_relu_backward(const float* x, const float* dy_a, const float* dy_b, c
                          float* dx, float* dscale, float* dbias, int N, int C, int HW, void* ws,
                          size_t ws_bytes, void* stream);
 
+// The cluster size of the single-pass kernel for a channel, 0 if none holds it
+// (what the registers hold, a cluster holds too).
+int takes_cluster(long long per_channel, bool vec, int C, int* per_cta) {
+  int share = 0;
+  const int cs = cluster_plan(vec ? per_channel / 4 : per_channel, vec ? 32 : 8, 8192, &share, C);
+  if (per_cta) *per_cta = share;
+  return static_cast<long long>(C) * cs <= 0x7fffffffLL ? cs : 0;
+}
+
 template <int MASK>
 int bn_backward(const float* x, const float* dy, const float* relu_in, const float* scale,
                 const float* mean, const float* invstd, float* dx, float* dscale,
@@ -1435,8 +1444,8 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
   }
   {
     int per_cta = 0;
-    const int cs = cluster_plan(vec ? per_channel / 4 : per_channel, vec ? 32 : 8, 8192, &per_cta, C);
-    if (cs > 0 && static_cast<long long>(C) * cs <= 0x7fffffffLL) {
+    const int cs = takes_cluster(per_channel, vec, C, &per_cta);
+    if (cs > 0) {
       // two CTAs' worth of work per SM at least, or there is nothing for a third to overlap with
       if (vec && MASK != 2 && hybrid_share(per_cta) && static_cast<long long>(C) * cs >= 2LL * sm_count())
         return launch_hybrid<MASK == 1>(x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, cs, per_cta, s);
@@ -1502,8 +1511,8 @@ int bn_add_relu_backward(const float* x, const float* dy_a, const float* dy_b, c
         }))
       return st;
     int per_cta = 0;
-    const int cs = cluster_plan(per_channel / 4, 32, 8192, &per_cta, C);
-    if (cs > 0 && static_cast<long long>(C) * cs <= 0x7fffffffLL) {
+    const int cs = takes_cluster(per_channel, true, C, &per_cta);
+    if (cs > 0) {
       if (per_cta > 2048)
         return launch_cluster_t<true, true, 512, true>(x, dy_a, relu_in, scale, mean, invstd, dx, dscale,
                                                        dbias, sh, cs, per_cta, s, dy_b, joined);
@@ -1620,6 +1629,14 @@ int sgb_bn_backward_faults(unsigned* flags) {
   if (fs != SGB_OK) return fs;
   *flags = streaming | (cluster << 8) | (forward << 16);
   return SGB_OK;
+}
+
+int sgb_bn_backward_streams(int N, int C, int HW, int mask) {
+  if (N <= 0 || C <= 0 || HW <= 0 || HW % 4 != 0 || mask < 0 || mask > 2) return 0;
+  const long long per_channel = static_cast<long long>(N) * HW;
+  if (per_channel > 0x7fffffffLL || takes_cluster(per_channel, true, C, nullptr)) return 0;
+  BnStreamPlan plan;
+  return bn_stream_plan(N, C, HW, mask, &plan) ? 1 : 0;
 }
 
 int sgb_bn_backward_stream_plan(int N, int C, int HW, int mask, int* plan6) {

@@ -1,0 +1,36 @@
+"""Which batch-norm backward calls take the streaming kernel (host arithmetic):
+a recorded step asks, because a captured streaming launch would keep its
+counter table.  A channel streams when the x and dy of its N planes do not fit
+the shared memory of eight CTAs, 100 KB each, and its planes can be cut."""
+import ctypes
+import itertools
+
+import pytest
+
+from singa_b200 import _lib
+
+
+def expected(N, C, HW, mask):
+    if HW % 4:
+        return 0
+    units = N * HW // 4
+    if -(-units // 8) * 32 <= 100 * 1024:
+        return 0
+    return _lib.lib().sgb_bn_backward_stream_plan(N, C, HW, mask, (ctypes.c_int * 6)())
+
+
+def test_the_query_follows_the_capacity_of_a_cluster():
+    lib = _lib.lib()
+    shapes = [(32, 64, 112 * 112), (32, 256, 56 * 56), (33, 256, 56 * 56), (1, 3, 102400), (1, 3, 102404), (1, 3, 102432),
+              (16, 8, 80 * 80), (17, 8, 80 * 80), (32, 64, 111 * 111), (32, 5000, 12544), (2, 4, 1)]
+    shapes += itertools.product((1, 7, 32, 65), (1, 64, 2048), (49, 196, 784, 3136, 12544, 50176))
+    for N, C, HW in shapes:
+        for mask in (0, 1, 2):
+            assert lib.sgb_bn_backward_streams(N, C, HW, mask) == expected(N, C, HW, mask), (N, C, HW, mask)
+    assert lib.sgb_bn_backward_streams(32, 64, 112 * 112, 0) == 1
+    assert lib.sgb_bn_backward_streams(32, 256, 56 * 56, 0) == 0
+
+
+@pytest.mark.parametrize("args", [(0, 4, 16, 0), (4, 0, 16, 0), (4, 4, 0, 0), (32, 64, 12544, 3), (32, 64, 12544, -1)])
+def test_no_call_no_stream(args):
+    assert _lib.lib().sgb_bn_backward_streams(*args) == 0
