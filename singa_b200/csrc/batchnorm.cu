@@ -221,7 +221,7 @@ bn_bwd_cluster_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                       const float* __restrict__ mean, const float* __restrict__ invstd,
                       float* __restrict__ dx, float* __restrict__ dscale,
                       float* __restrict__ dbias, BnShape sh, int per_cta,
-                      const float* __restrict__ dy_b = nullptr, float* __restrict__ joined = nullptr) {
+                      bool early, const float* __restrict__ dy_b = nullptr, float* __restrict__ joined = nullptr) {
   extern __shared__ __align__(16) float stage[];
   __shared__ unsigned long long pairs_in;          // mbarrier: counts the peers' pairs as they land
   __shared__ float red[2 * T / 32];
@@ -246,10 +246,7 @@ bn_bwd_cluster_kernel(const float* __restrict__ x, const float* __restrict__ dy,
   const size_t chan_off = static_cast<size_t>(c) * sh.HW;
   if (VEC && first_wave(2)) prefetch_share(x, MASK == 1 || ADD ? relu_in : nullptr, first, u1, T, hwu, plane_stride, chan_off);
   dependency_wait();                                  // first access to global memory follows
-  // A grid of small shares leaves room on the SMs from the start: the next
-  // kernel's CTAs may come in and prefetch (ResNet-50 at batch 32, eleven layers
-  // of 14x14: 1683 -> 1673 us; letting larger shares go early costs 20 us).
-  const bool early = per_cta <= 800;
+  // see leaves_room()
   if (early) release_dependents();
   const float mu = mean[c];
   // units of one copy group per thread (the same in every thread: kCopyGroups * group_units covers a share)
@@ -1324,6 +1321,21 @@ int launch_hybrid(const float* x, const float* dy, const float* relu_in, const f
                    dy, relu_in, scale, mean, invstd, dx, dscale, dbias, sh, per_cta);
 }
 
+// Whether a grid lets the next kernel's CTAs in, to prefetch, as soon as all of
+// its own have started, and not only when it has nothing left to do but store:
+// if it takes at most half of the slots that the SMs have for it by shared memory
+// and threads.  With more, the waiting CTAs take the places of kernels behind
+// them.  A ResNet-50 step in us, never / this rule / one full wave / always:
+//   batch 4   398.2  397.9  415.0  415.0      batch 32  1695.9  1692.1  1702.8  1725.6
+//   batch 8   598.2  587.4  592.3  596.6      batch 33  1905.1  1897.7  1899.8  1940.7
+//   batch 16  974.9  969.4  974.3  983.0      batch 40  2240.5  2241.6  2231.8  2270.5
+//   batch 24 1331.4 1326.9 1318.6 1339.3      batch 64  3443.3  3443.6  3462.3  3502.0
+// and on images of 160 at batch 16: 613.7  602.9  609.1  613.6.
+inline bool leaves_room(long long ctas, size_t smem, int threads) {
+  const long long by_smem = 227 * 1024 / (static_cast<long long>(smem) + 2048), by_threads = 2048 / threads;
+  return 2 * ctas <= (by_smem < by_threads ? by_smem : by_threads) * sm_count();
+}
+
 template <bool VEC, int MASK, int T, bool ADD = false>
 int launch_cluster_t(const float* x, const float* dy, const float* relu_in, const float* scale,
                      const float* mean, const float* invstd, float* dx, float* dscale,
@@ -1335,7 +1347,8 @@ int launch_cluster_t(const float* x, const float* dy, const float* relu_in, cons
   const int ready = opt_in_once(kernel, attr_set, true);
   if (ready != SGB_OK) return ready;
   return launch_ex(kernel, dim3(static_cast<unsigned>(sh.C) * cs), dim3(T), smem, s, cs, true, x, dy, relu_in,
-                   scale, mean, invstd, dx, dscale, dbias, sh, per_cta, dy_b, joined);
+                   scale, mean, invstd, dx, dscale, dbias, sh, per_cta,
+                   leaves_room(static_cast<long long>(sh.C) * cs, smem, T), dy_b, joined);
 }
 
 template <bool VEC, int MASK>
