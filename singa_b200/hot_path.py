@@ -28,11 +28,29 @@ def _table(tensors):
             (C.c_size_t * n)(*[t.numel() for t in tensors]), n)
 
 
-# A batch-norm backward takes a join into itself where both are short (their
-# launches and latencies are what they cost: 3x512x20x20 4.8 -> 3.0 us); where
-# they are bound by bytes the streaming join is the faster place for them
-# (16x1024x14x14, 3.2e6 elements: 16.4 us apart, 16.7 together).
-_JOIN_ELEMENTS = 1 << 21
+def join_pays(n, c, hw):
+    """Whether a batch-norm backward takes the join in front of it into itself:
+    where both are short, one launch and one latency less is worth more than
+    what the streaming join does better.  The lines follow whole ResNet-50 steps
+    (us with all such joins apart -> merged, three captures of each):
+
+      up to 2^21 elements, as a rule: 1x224^2 285.7 -> 275, 4x224^2 400.5 -> 395.3,
+        2x256x56x56 alone 355.4 -> 347.6; beyond, where a cluster shares a
+        channel: 8x512x28x28 585.8 -> 597.8, 16x512x20x20 595.7 -> 606.0;
+      not where a warp holds a channel in nearly all of its four vectors
+        (32x1024x4x4 386.2 -> 390.7, 24x1024x4x4 342.3 -> 344.2) nor, above 2^20,
+        where a thread holds more than four (24x256x16x16 344 -> 350,
+        8x256x24x24 317.5 -> 321.6, 3x256x40x40 317.3 -> 322.5);
+      planes that are no multiple of four, one float an access: up to 2^17
+        elements, or 2^18 where a channel has no more than 128 (3x2048x5x5
+        319.6 -> 317.9, 1x2048x7x7 285.7 -> 283.3; but 4x512x25x25 423 -> 451,
+        10x1024x13x13 649 -> 669, 3x1024x7x7 271.1 -> 273.1)."""
+    channel, elements = n * hw, n * c * hw
+    if hw % 4:
+        return elements <= 1 << 17 or (elements <= 1 << 18 and channel <= 128)
+    if 320 < channel <= 512 or (4096 < channel <= 6144 and elements > 1 << 20):
+        return False
+    return elements <= 1 << 21
 
 
 def merge_calls(calls):
@@ -50,7 +68,7 @@ def merge_calls(calls):
     for name, a in calls:
         last, b = out[-1] if out else ("", None)
         if name == "sgb_bn_backward_f32" and last == "sgb_add_relu_backward_f32" and a[1] == b[3] and \
-                b[4] == a[8] * a[9] * a[10] <= _JOIN_ELEMENTS:
+                b[4] == a[8] * a[9] * a[10] and join_pays(*a[8:11]):
             out[-1] = ("sgb_bn_add_relu_backward_f32", (a[0],) + b[:3] + a[2:5] + (a[1],) + a[5:])
         elif name == "sgb_sum_rows_f32" and last == "sgb_relu_backward_f32" and a[0] == b[2] and b[3] == a[2] * a[3]:
             out[-1] = ("sgb_relu_backward_sum_rows_f32", b[:3] + a[1:])
