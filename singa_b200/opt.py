@@ -122,6 +122,20 @@ class DistOpt(object):
         scale = float(np.float32(1.0) / np.float32(self.world_size))
         self.opt.apply(name if name is not None else id(param), param, grad, grad_scale=scale)
 
+    def _whole(self, name, forwards, calls):
+        """The communicator's method `name`, which stands for a sequence of its
+        `calls`: None where the communicator has none, or where a subclass or an
+        instance has its own version of one of them or of this class's `forwards`,
+        which then has to be called."""
+        c = self.communicator
+        whole = getattr(c, name, None)
+        if whole is None or any(f in vars(self) or getattr(type(self), f) is not getattr(DistOpt, f) for f in forwards):
+            return None
+        owner = next((k for k in type(c).__mro__ if name in vars(k)), None)
+        if owner is None or any(f in vars(c) or getattr(type(c), f, None) is not getattr(owner, f, None) for f in calls):
+            return None
+        return whole
+
     def _update_all(self, plist):
         scale = float(np.float32(1.0) / np.float32(self.world_size))
         names, params, grads = plist
@@ -131,7 +145,8 @@ class DistOpt(object):
 
     def _sync_dense(self, grad_stream, threshold, direct, fused, half=False):
         """Names, parameters and (reduced) gradients of the stream."""
-        whole = getattr(self.communicator, "syncDense", None)
+        whole = self._whole("syncDense", ("all_reduce_half", "fused_all_reduce_half"), ("synchHalf", "fusedSynchHalf")) \
+            if half else self._whole("syncDense", ("all_reduce", "fused_all_reduce"), ("synch", "fusedSynch"))
         if whole is not None:
             plist = whole(grad_stream, threshold, half)
             self.wait()
@@ -256,7 +271,8 @@ class DistOpt(object):
 
         # A communicator that offers the exchange in two halves has bucket k's
         # selection issued before the host waits for the counts of bucket k-1.
-        begin = getattr(self.communicator, "beginSparsification", None)
+        parts = ("sparsification", "fused_sparsification"), ("sparsification", "fusedSparsification")
+        begin = self._whole("beginSparsification", *parts)
         opened = 0
 
         def exchange(tensors, res, single):
@@ -273,7 +289,7 @@ class DistOpt(object):
                 self.fused_sparsification(tensors, res, spars, topK)
 
         # On one rank, gradients that all exist already go through one selection.
-        joint = getattr(self.communicator, "sparsifyBuckets", None)
+        joint = self._whole("sparsifyBuckets", *parts)
         try:
             if (joint is not None and corr and not topK and self.world_size == 1 and
                     type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
