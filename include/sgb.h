@@ -589,15 +589,21 @@ void *sgb_comm_stream(const sgb_comm *c, int which);
  * Work put there is joined to the compute stream by the next sgb_comm_wait. */
 void *sgb_comm_result_stream(const sgb_comm *c);
 /* The communicator's cross-stream ordering rules as a pure host function (no
- * GPU needed): given the state {dirty_s, dirty_c1, dirty_c2, c2_reads_recv}
- * and a call kind (0 synch, 1 flush in place, 2 flush packed, 3 flush half,
- * 4 synch half, 5 sparsification, 6 stage copy, 7 wait) it updates the state
- * and returns the edge masks recorded before the pre-processing kernel,
- * before the collective, behind it, and behind the post-processing kernel
- * (bits: 1 compute->c1, 2 compute->s, 4 c1->s, 8 c2(done)->s, 16 s->c1,
- * 32 s->c2, 64 s->compute, 128 c1->compute, 256 c2->compute, 512 mark c2
- * done).  The communicator emits exactly these edges; the reference records
- * its compute-stream event before every stage and flush
+ * GPU needed): given the state {dirty_s, dirty_c1, dirty_c2, c2_reads_recv |
+ * sparse << 1} and a call kind (0 synch, 1 flush in place, 2 flush packed,
+ * 3 flush half, 4 synch half, 6 stage copy, 7 wait; a sparse exchange: 16 its
+ * selection, 17 its exchange half, 18 that half on one rank, 5 the first two
+ * one behind the other) it updates the state and returns the edge masks
+ * recorded before the pre-processing kernel, before the collective, behind it,
+ * and behind the post-processing kernel - for 16, which has no collective,
+ * behind the selection - (bits: 1 compute->c1, 2 compute->s, 4 c1->s, 8
+ * c2(done)->s, 16 s->c1, 32 s->c2, 64 s->compute, 128 c1->compute, 256
+ * c2->compute, 512 mark c2 done; with the events of the exchange's slot: 1024
+ * mark selected, 2048 selected->s, 4096 selected->c2, 8192 mark consumed, 16384
+ * consumed->c1).  sparse: bits 0 and 1 the slot of the next selection and of the
+ * next exchange half, bits 2 and 3 whether the payload in slot 0, 1 is read on
+ * c2.  The communicator emits exactly these edges; the reference records its
+ * compute-stream event before every stage and flush
  * (src/io/communicator.cc:227-233, 255-271, 313-319). */
 int sgb_comm_order_plan(unsigned char *state4, int call, unsigned *edges4,
                         int *result_stream);

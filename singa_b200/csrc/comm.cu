@@ -78,7 +78,6 @@ struct sgb_comm {
     cudaEvent_t selected = nullptr;  // behind the selection on c1
     cudaEvent_t counted = nullptr;   // behind the counts' copy to the host
     cudaEvent_t consumed = nullptr;  // behind the dense sum on c2 that read pay_send (one rank)
-    bool in_use = false;             // that sum has not been joined by a wait() yet
     size_t n = 0, nnz_max = 0, capacity = 0;
     int topk = 0;
     const char* op_name = "";
@@ -143,7 +142,7 @@ cudaStream_t side(const sgb_comm* c, int which) {
 // Emits the edges of one phase of a planned call (see comm_order.h), in a
 // fixed order.  Every edge re-records its event; a wait takes the state of the
 // event at the time of the wait, so an event can serve many edges in a row.
-int emit(sgb_comm* c, unsigned edges, cudaStream_t compute) {
+int emit(sgb_comm* c, unsigned edges, cudaStream_t compute, int slot = 0) {
   using namespace sgb::order;
   if (edges & kComputeToC1) OK(edge(c->ev_compute, compute, c->c1));
   if (edges & kComputeToS) OK(edge(c->ev_compute, compute, c->s));
@@ -155,6 +154,12 @@ int emit(sgb_comm* c, unsigned edges, cudaStream_t compute) {
     if (edges & kSToC2) CU(cudaStreamWaitEvent(c->c2, c->ev_s, 0));
   }
   if (edges & kMarkC2Done) CU(cudaEventRecord(c->ev_c2_done, c->c2));
+  const sgb_comm::Sparse& x = c->sparse[slot];
+  if (edges & kConsumedToC1) CU(cudaStreamWaitEvent(c->c1, x.consumed, 0));
+  if (edges & kMarkSelected) CU(cudaEventRecord(x.selected, c->c1));
+  if (edges & kSelectedToS) CU(cudaStreamWaitEvent(c->s, x.selected, 0));
+  if (edges & kSelectedToC2) CU(cudaStreamWaitEvent(c->c2, x.selected, 0));
+  if (edges & kMarkConsumed) CU(cudaEventRecord(x.consumed, c->c2));
   if (edges & kSToCompute) OK(edge(c->ev_s, c->s, compute));
   if (edges & kC1ToCompute) OK(edge(c->ev_c1, c->c1, compute));
   if (edges & kC2ToCompute) OK(edge(c->ev_c2, c->c2, compute));
@@ -444,25 +449,33 @@ void* sgb_comm_stream(const sgb_comm* c, int which) {
 int sgb_comm_wait(sgb_comm* c, void* compute_stream) {
   if (!c) return SGB_ERR_NULL;
   if (c->sparse_begun != c->sparse_ended) return SGB_ERR_STATE;   // an exchange is still to be ended
-  for (sgb_comm::Sparse& x : c->sparse) x.in_use = false;          // c2 is joined here
   return emit(c, plan_call(c, sgb::order::kWait).before, sgb::as_stream(compute_stream));
 }
 
 void* sgb_comm_result_stream(const sgb_comm* c) { return c ? side(c, c->result_stream) : nullptr; }
 
 int sgb_comm_order_plan(unsigned char* state, int call, unsigned* edges, int* result_stream) {
+  using namespace sgb::order;
   if (!state || !edges) return SGB_ERR_NULL;
-  if (call < sgb::order::kSynch || call > sgb::order::kWait) return SGB_ERR_UNSUPPORTED;
-  sgb::order::State st;
+  const bool both = call == 5;     // the two halves of a sparse exchange, one behind the other
+  if (!both && !(call >= kSynch && call <= kWait) && !(call >= kSparseSelect && call <= kSparseLocal))
+    return SGB_ERR_UNSUPPORTED;
+  State st;
   st.dirty_s = state[0];
   st.dirty_c1 = state[1];
   st.dirty_c2 = state[2];
-  st.c2_reads_recv = state[3];
-  const sgb::order::Step p = sgb::order::plan(st, call);
+  st.c2_reads_recv = state[3] & 1;
+  st.sparse = state[3] >> 1;
+  Step p = plan(st, both ? kSparseSelect : call);
+  if (both) {
+    const unsigned pre = p.pre, selected = p.post;
+    p = plan(st, kSparseExchange);
+    p.pre = pre | selected;        // recorded behind the selection, ahead of the exchange half
+  }
   state[0] = st.dirty_s;
   state[1] = st.dirty_c1;
   state[2] = st.dirty_c2;
-  state[3] = st.c2_reads_recv;
+  state[3] = static_cast<unsigned char>(st.c2_reads_recv | st.sparse << 1);
   edges[0] = p.pre;
   edges[1] = p.before;
   edges[2] = p.after;
@@ -736,7 +749,9 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
   if (capacity > c->max_elems) return SGB_ERR_CAPACITY;
   if (c->sparse_begun - c->sparse_ended >= 2) return SGB_ERR_STATE;
   OK(sparse_init(c));
-  sgb_comm::Sparse& x = c->sparse[c->sparse_begun & 1];
+  const unsigned char slots = c->order.sparse;
+  const sgb::order::Step p = plan_call(c, sgb::order::kSparseSelect);
+  sgb_comm::Sparse& x = c->sparse[p.slot];
   x.n = n;
   x.nnz_max = 0;
   x.capacity = capacity;
@@ -748,9 +763,9 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
     x.tensors.push_back(static_cast<float*>(tensors[i]));
     x.sizes.push_back(sizes[i]);
   }
-  if (n) {
-    OK(emit(c, plan_call(c, sgb::order::kSparseSelect).pre, sgb::as_stream(compute_stream)));
-    if (x.in_use) CU(cudaStreamWaitEvent(c->c1, x.consumed, 0));
+  const int st = [&] {
+    OK(emit(c, p.pre, sgb::as_stream(compute_stream), p.slot));
+    if (n == 0) return emit(c, p.post, nullptr, p.slot);
     Phase ph(c, x.op_name, sgb::order::kStreamC1);
     // The selection reads the tensors where they are; only a long list, or one
     // without a residual buffer, is copied together first.
@@ -786,7 +801,11 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
       CU(cudaMemcpyAsync(x.nnz_host, x.nnz_dev + 1, sizeof(int) * c->world, cudaMemcpyDeviceToHost, c->c1));
       CU(cudaEventRecord(x.counted, c->c1));
     }
-    CU(cudaEventRecord(x.selected, c->c1));
+    return emit(c, p.post, nullptr, p.slot);
+  }();
+  if (st != SGB_OK) {
+    c->order.sparse = slots;         // not begun: the slot stays free
+    return st;
   }
   ++c->sparse_begun;
   return SGB_OK;
@@ -796,37 +815,33 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
 static int sparse_end(sgb_comm* c, void* compute_stream) {
   if (!c) return SGB_ERR_NULL;
   if (c->sparse_begun == c->sparse_ended) return SGB_ERR_STATE;
-  sgb_comm::Sparse& x = c->sparse[c->sparse_ended++ & 1];
-  if (x.n == 0) return SGB_OK;
+  ++c->sparse_ended;
   const int W = c->world;
+  const sgb::order::Step p = plan_call(c, W == 1 ? sgb::order::kSparseLocal : sgb::order::kSparseExchange);
+  sgb_comm::Sparse& x = c->sparse[p.slot];
   if (W == 1) {
     // The payload is read where it lies: no all-gather, no count on the host.
-    plan_call(c, sgb::order::kSparseLocal);
-    CU(cudaStreamWaitEvent(c->c2, x.selected, 0));
+    OK(emit(c, p.before, sgb::as_stream(compute_stream), p.slot));
+    if (x.n == 0) return emit(c, p.post, nullptr, p.slot);
     Phase ph(c, x.op_name, sgb::order::kStreamC2);
     OK(sgb::sparse_dense_sum(x.pay_send, 0, x.capacity, x.nnz_host, x.topk ? nullptr : x.nnz_dev, 1, x.tensors.data(),
                              x.sizes.data(), x.tensors.size(), c->c2));
-    CU(cudaEventRecord(x.consumed, c->c2));
-    x.in_use = true;
-    return SGB_OK;
+    return emit(c, p.post, nullptr, p.slot);
   }
-  if (!x.topk && !x.capacity) {
+  if (x.n && !x.topk && !x.capacity) {
     CU(cudaEventSynchronize(x.counted));
     for (int r = 0; r < W; ++r) {
       if (x.nnz_host[r] < 0 || static_cast<size_t>(x.nnz_host[r]) > x.n) return SGB_ERR_STATE;
       if (static_cast<size_t>(x.nnz_host[r]) > x.nnz_max) x.nnz_max = x.nnz_host[r];
     }
   }
-  const sgb::order::Step p = plan_call(c, sgb::order::kSparseExchange);
-  // s waits for this exchange's own selection, not for what c1 was given since
-  CU(cudaStreamWaitEvent(c->s, x.selected, 0));
-  OK(emit(c, p.before & ~static_cast<unsigned>(sgb::order::kC1ToS), sgb::as_stream(compute_stream)));
+  OK(emit(c, p.before, sgb::as_stream(compute_stream), p.slot));
   {
     Phase ph(c, "Dist_s_sparsification_allgather", sgb::order::kStreamS);
     if (x.nnz_max) NC(ncclAllGather(x.pay_send, c->pay_recv, 2 * x.nnz_max, ncclFloat, c->nccl, c->s));
   }
   OK(emit(c, p.after, nullptr));
-  {
+  if (x.n) {
     Phase ph(c, x.op_name, sgb::order::kStreamC2);
     const size_t stride = 2 * x.nnz_max;
     if (W <= sgb::kMaxDenseRanks) {

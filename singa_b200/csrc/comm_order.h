@@ -18,6 +18,11 @@
 //     right behind that kernel, so later work on c2 does not delay NCCL);
 //   * the stream that post-processes, or on which a caller may consume the
 //     result, waits for the collective (s -> c1 / s -> c2);
+//   * a sparse exchange has two halves, and two exchanges may be open at a time:
+//     the exchange half of one is ordered behind ITS selection (an event of the
+//     slot it occupies), not behind what c1 was given since; where its payload is
+//     read in place on c2 (one rank), the next selection into that slot waits for
+//     that reader;
 //   * wait() joins every stream that received work back to the compute stream.
 #pragma once
 
@@ -30,14 +35,12 @@ enum Call {
   kFlushPacked = 2,   // pack on c1, all-reduce send -> recv, unpack on c1
   kFlushHalf = 3,     // pack + cast on c1, fp16 all-reduce, cast + unpack on c2
   kSynchHalf = 4,     // cast on c1, fp16 all-reduce, cast back on c2
-  kSparse = 5,        // select on c1, all-gather, scatter-add on c2
+  // (5: both halves of a sparse exchange, see sgb_comm_order_plan)
   kStageCopy = 6,     // copies into the staging buffer on c1 (no collective)
   kWait = 7,
-  // the two halves of kSparse, issued one after the other or with another
-  // exchange's half between them (not replayed through sgb_comm_order_plan)
-  kSparseSelect = 16,    // the selection on c1
-  kSparseExchange = 17,  // ordered behind that selection: all-gather on s, dense sum on c2
-  kSparseLocal = 18,     // the same with one rank: the dense sum on c2 waits for the selection's own event
+  kSparseSelect = 16,    // the selection on c1, into the next slot
+  kSparseExchange = 17,  // of the oldest open exchange: all-gather on s, dense sum on c2
+  kSparseLocal = 18,     // the same with one rank: the dense sum on c2 reads the payload in place
 };
 
 enum Edge : unsigned {
@@ -51,6 +54,12 @@ enum Edge : unsigned {
   kC1ToCompute = 1u << 7,
   kC2ToCompute = 1u << 8,
   kMarkC2Done = 1u << 9,  // record that event on c2
+  // events of the exchange's slot
+  kMarkSelected = 1u << 10,  // record behind the selection on c1
+  kSelectedToS = 1u << 11,
+  kSelectedToC2 = 1u << 12,
+  kMarkConsumed = 1u << 13,  // record on c2 behind the kernel that read the slot's payload
+  kConsumedToC1 = 1u << 14,
 };
 
 enum { kStreamS = 0, kStreamC1 = 1, kStreamC2 = 2 };
@@ -58,6 +67,9 @@ enum { kStreamS = 0, kStreamC1 = 1, kStreamC2 = 2 };
 struct State {
   unsigned char dirty_s = 0, dirty_c1 = 0, dirty_c2 = 0;  // received work since the last wait()
   unsigned char c2_reads_recv = 0;  // a kernel on c2 read a receive buffer since s last waited for c2
+  // bit 0: slot of the next selection, bit 1: slot of the next exchange half,
+  // bits 2, 3: the payload in slot 0, 1 is read on c2 since the last wait()
+  unsigned char sparse = 0;
 };
 
 struct Step {
@@ -66,6 +78,7 @@ struct Step {
   unsigned after = 0;   // behind the collective
   unsigned post = 0;    // behind the post-processing kernel
   int result_stream = kStreamS;  // where the reduced values can be consumed
+  int slot = 0;         // of a sparse exchange
 };
 
 inline Step plan(State& st, int call) {
@@ -88,7 +101,6 @@ inline Step plan(State& st, int call) {
       break;
     case kFlushHalf:
     case kSynchHalf:
-    case kSparse:
       p.pre = kComputeToC1;
       p.before = kC1ToS | (st.c2_reads_recv ? kC2DoneToS : 0u);
       p.after = kSToC1 | kSToC2;
@@ -98,20 +110,30 @@ inline Step plan(State& st, int call) {
       st.dirty_s = st.dirty_c1 = st.dirty_c2 = 1;
       break;
     case kSparseSelect:
-      p.pre = kComputeToC1;
+      p.slot = st.sparse & 1;
+      p.pre = kComputeToC1 | (st.sparse >> (2 + p.slot) & 1 ? kConsumedToC1 : 0u);
+      p.post = kMarkSelected;
       p.result_stream = kStreamC1;
+      st.sparse ^= 1;
       st.dirty_c1 = 1;
       break;
     case kSparseExchange:
-      p.before = kC1ToS | (st.c2_reads_recv ? kC2DoneToS : 0u);
+      p.slot = st.sparse >> 1 & 1;
+      p.before = kSelectedToS | (st.c2_reads_recv ? kC2DoneToS : 0u);
       p.after = kSToC1 | kSToC2;
       p.post = kMarkC2Done;
       p.result_stream = kStreamC2;
+      st.sparse ^= 2;
       st.c2_reads_recv = 1;
       st.dirty_s = st.dirty_c1 = st.dirty_c2 = 1;
       break;
     case kSparseLocal:
+      p.slot = st.sparse >> 1 & 1;
+      p.before = kSelectedToC2;
+      p.post = kMarkConsumed;
       p.result_stream = kStreamC2;
+      st.sparse ^= 2;
+      st.sparse |= 4u << p.slot;
       st.dirty_c1 = st.dirty_c2 = 1;
       break;
     case kStageCopy:
