@@ -90,7 +90,22 @@ def merge_calls(calls):
     return out
 
 
+def _recorded(name):
+    """An attribute that the recorded program of a step holds (the communicator by
+    its address): setting it has the program recorded anew at the next run."""
+    def read(self):
+        return getattr(self, "_" + name)
+
+    def write(self, value):
+        setattr(self, "_" + name, value)
+        self._program = None
+    return property(read, write)
+
+
 class HotPathGPU(object):
+    comm, world, dist_option = _recorded("comm"), _recorded("world"), _recorded("dist_option")
+    spars, update_on_arrival = _recorded("spars"), _recorded("update_on_arrival")
+
     def __init__(self, plan, communicator=None, world=1, seed=0, lr=0.1, momentum=0.9,
                  weight_decay=1e-5, threshold=2097152, dist_option="plain", spars=0.05,
                  device=None, update_on_arrival=True, pool_argmax=False):
@@ -357,18 +372,7 @@ class HotPathGPU(object):
                 tot = sum(sizes[i] for i in ev[1])
                 self.residuals[ev[1][-1]] = torch.zeros(tot, device=self.device)
 
-        self._recorded = self._exchange_settings()
         self._record_program()
-
-    def _exchange_settings(self):
-        """What the recorded program holds of its owner's attributes (the rates are
-        passed at every run).  The communicator counts as long as it is open: its
-        address stands in the program."""
-        c = self.comm
-        if c is not None and c._h is None:
-            raise _lib.SgbError("sgb_comm", -1, "the communicator is closed")
-        return (None if c is None else c._h.value, self.world, self.dist_option, self.spars,
-                self.update_on_arrival)
 
     # ----------------------------------------------------------------- program
     def _record_program(self):
@@ -469,10 +473,11 @@ class HotPathGPU(object):
     def run_step(self):
         """Enqueues one full step on the current stream (+ the communicator's
         side streams).  Returns the number of C-ABI calls issued."""
-        now = self._exchange_settings()
-        if now != self._recorded:
+        comm = self._comm
+        if comm is not None and comm._h is None:
+            raise _lib.SgbError("sgb_comm", -1, "the communicator is closed")
+        if self._program is None:
             self._record_program()
-            self._recorded = now
         _lib.native.run_program(self._program, self.lr, self.momentum, self.weight_decay, self.profile)
         return self.calls_per_step
 
