@@ -1,4 +1,4 @@
-"""Build recipes for the checker libraries.
+"""Build recipes for the oracle library.
 
 ``build_oracle()`` compiles ``oracle.c`` into ``oracle/liboracle.so`` with gcc.
 ``build_ref()`` (see ``oracle/ref_build.py``) compiles objects straight from an

@@ -125,7 +125,7 @@ def make_tensors(plan, seed=0):
         elif k in ("pgrad", "wsyn"):
             t[name] = rng.standard_normal(spec.shape, dtype=np.float32) * np.float32(1e-3)
         elif k == "mask":
-            continue                              # the CPU checker recomputes the decisions from the input
+            continue                              # the oracle recomputes the decisions from the input
         else:
             t[name] = np.zeros(spec.shape, np.float32)
     for name in list(T):

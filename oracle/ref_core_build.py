@@ -13,7 +13,7 @@ is replaced by three authored shims under ``oracle/ref_shims/``:
   cblas.h + ref_cblas.c  the eight CBLAS routines the back end calls, OpenMP loops
                          (no CBLAS library here)
 
-``ref_core_doors.cc`` adds extern "C" doors for the checker: the MLP training
+``ref_core_doors.cc`` adds extern "C" doors for the comparator: the MLP training
 step of benchmark configuration 1 on ``singa::Tensor`` objects, and single
 operations for cross-checks.  TEST INFRASTRUCTURE ONLY: the library is the
 CPU comparator / baseline; nothing under ``singa_b200/`` loads it.

@@ -2,7 +2,7 @@
 // lang::Cpp (CPU) back end (oracle/ref_core_build.py).  TEST INFRASTRUCTURE
 // ONLY: everything below runs on singa::Tensor objects through the reference's
 // public C++ functions, in the order its Python autograd issues them, so the
-// checker can (a) time the reference's CPU path on the MLP training step of
+// comparator can (a) time the reference's CPU path on the MLP training step of
 // benchmark configuration 1 and (b) pin the CPU restatement in oracle.c against
 // the code it restates.
 //

@@ -1,6 +1,6 @@
 // Stand-in for NVIDIA's cnmem library (an external, un-vendored dependency of
 // apache/singa: include/singa/core/memory.h:29, src/core/memory/memory.cc) for
-// builds of the reference's CUDA device classes in the checker.  The seven
+// builds of the reference's CUDA device classes in the comparator.  The seven
 // entry points the reference calls are provided over cudaMalloc with a
 // size-keyed free list: a freed block is handed to the next request of the
 // same size without a cudaFree, which keeps the property the reference's graph

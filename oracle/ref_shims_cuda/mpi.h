@@ -1,7 +1,7 @@
 /* Stand-in for <mpi.h>: apache/singa's communicator includes it
  * (include/singa/io/communicator.h:26) and calls six MPI routines from the
  * constructor that bootstraps through MPI (src/io/communicator.cc:79-98, 191).
- * No MPI is installed where the comparator is built, and the checker only
+ * No MPI is installed where the comparator is built, and it only
  * uses the constructor that receives an NCCL id, so the routines below exist
  * to satisfy the compiler and fail when called.  TEST INFRASTRUCTURE ONLY. */
 #ifndef SGB_REF_MPI_H_

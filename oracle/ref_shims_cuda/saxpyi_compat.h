@@ -1,7 +1,7 @@
 // cusparseSaxpyi (y[xInd[i] - base] += alpha * xVal[i]) was removed from
 // cuSPARSE in CUDA 12; apache/singa's communicator still calls it
 // (src/io/communicator.cc:715, 753, 803).  This header, force-included when
-// that file is compiled for the checker, declares a stand-in with the removed
+// that file is compiled for the comparator, declares a stand-in with the removed
 // routine's signature; saxpyi_compat.cu implements it with one scatter-add
 // kernel on the handle's stream.  TEST INFRASTRUCTURE ONLY.
 #ifndef SGB_REF_SAXPYI_COMPAT_H_

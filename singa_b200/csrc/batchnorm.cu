@@ -6,33 +6,44 @@
 //               (dy - dbias[c]/M - (x - mean[c]) * invstd[c] * dscale[c] / M)
 // M = N*H*W (spatial mode, NCHW) or N (per-activation mode, N x D).
 //
-// Single-pass scheme (12 bytes of HBM traffic per element), used whenever one
-// channel's x and dy (N*H*W*8 bytes) fit the shared memory of a thread-block
-// cluster of at most 8 CTAs: the cluster stages its channel in shared memory
-// with 16-byte asynchronous copies (cp.async, no register staging), every CTA
-// reduces its share with warp shuffles, the CTAs exchange their two partial
-// sums through distributed shared memory, and dx is computed from the staged
-// copy.  Shares are sized so that two to four CTAs are resident per SM and
-// the load phase of one overlaps the store phase of another.
+// One pass over HBM (12 bytes per element) wherever a channel can be held while
+// its two sums form, in this order of preference:
+//   registers  a warp or a CTA holds a channel of up to a few thousand elements
+//              (bn_bwd_small_kernel);
+//   groups     planes that are no multiple of four floats: a CTA stages the 2 or
+//              4 adjacent channels that make an aligned run (bn_bwd_group_kernel;
+//              also ahead of the registers for larger calls without a mask, see
+//              bn_backward);
+//   ragged     such planes when a channel needs a cluster: the aligned vectors
+//              that touch a plane, ends masked (bn_bwd_ragged_kernel);
+//   hybrid     a cluster of up to 8 CTAs shares a channel, part of the gradient
+//              stays in registers: three CTAs per SM where shared memory alone
+//              would leave two (bn_bwd_hybrid_kernel);
+//   cluster    the same with all of x and dy staged in shared memory by 16-byte
+//              asynchronous copies (cp.async, no register staging): every CTA
+//              reduces its share with warp shuffles, the CTAs exchange their two
+//              partial sums through distributed shared memory, and dx is computed
+//              from the staged copy; two to four CTAs per SM, so that the load
+//              phase of one overlaps the store phase of another
+//              (bn_bwd_cluster_kernel);
+//   streaming  channels too large for a cluster (e.g. 32 x 112 x 112): persistent
+//              small CTAs take 50 KB items of a channel from a ticket counter and
+//              meet through counters in global memory (bn_stream.cu).
 //
-// Channels too large for a cluster (e.g. 32 x 112 x 112) are also done in one
-// pass, by the streaming kernel of bn_stream.cu: persistent small CTAs take
-// 50 KB items of a channel from a ticket counter and meet through counters in
-// global memory.
-//
-// Two-pass scheme, 20 bytes of HBM traffic per element when the tensor does
-// not fit L2; the fallback for planes that are not a multiple of four floats,
-// misaligned operands, more than 4096 channels, and the entry point without
-// workspace:
+// Two passes (20 bytes of HBM traffic per element when the tensor does not fit
+// L2) for what is left: ragged planes too large for a cluster, misaligned
+// operands or planes below eight floats too large for one, channels that the
+// streaming kernel cannot cut or more than 4096 of them, and the entry point
+// without workspace:
 //   pass 1  grid (slices, C): a CTA walks its slice of the channel's flattened
-//           (n, hw) space with 128-bit loads and leaves two partial sums in the
-//           workspace (no atomics, fixed order -> run-to-run identical);
+//           (n, hw) space, with 128-bit loads where it can, and leaves two partial
+//           sums in the workspace (no atomics, fixed order -> run-to-run identical);
 //   pass 2  grid (tiles, C): every CTA first adds the channel's <= 64 partials
 //           in one warp (the same order in every CTA), then streams
-//           dx for its 1024-element tile.  CTAs with blockIdx.x == 0 also store
+//           dx for its 1024-unit tile.  CTAs with blockIdx.x == 0 also store
 //           dscale/dbias.
 // The optional ReLU mask fuses "dy = relu_in > 0 ? dy : 0" (the backward of
-// the ReLU that follows the BN layer) into both passes, which removes one
+// the ReLU that follows the BN layer) into every form, which removes one
 // full write + read of the intermediate gradient.
 #include "bn_common.cuh"
 #include "bn_stream.cuh"
@@ -1118,14 +1129,13 @@ int launch_ragged(const float* x, const float* dy, const float* relu_in, const f
 // the first kRegUnits units per thread of the gradient stay in registers, so
 // THREE CTAs of 256 threads fit an SM and half as many bytes again are staged.
 // (A CTA spends 3.3 us taking its share in and 4.2 us on reduction, exchange
-// and dx; with two CTAs the SM's input idles part of the time.)  32x256x56x56:
-// 68.8 -> 60.4 us (0.78 of the copy bandwidth).
+// and dx; with two CTAs the SM's input idles part of the time.)  32x256x56x56,
+// cluster form / this one: 67.0 / 56.7 us, 0.83 of the copy bandwidth.
 // All loads have to be issued at once: a second, dependent batch waits behind
-// everything that is queued already (gradient after x: 62.7 us).  A ReLU's input
+// everything that is queued already (gradient after x: 4 % slower).  A ReLU's input
 // has no registers left to go to, so it passes through the place of x and leaves
-// four bits per unit behind; x follows it unit by unit.  32x256x56x56 with the
-// ReLU's input: 87.7 -> 79.9 us (0.79 of the copy bandwidth); in batches of four
-// registers it was 111 us.
+// four bits per unit behind; x follows it unit by unit.  With the ReLU's input:
+// 88.3 / 75.0 us (0.84); in batches of four registers it was 40 % slower.
 // The sums are formed exactly as by bn_bwd_cluster_kernel with 512 threads
 // (thread t stands in for its threads t and t + 256), so that a fused call and
 // its unfused parts agree bit for bit whichever kernels they take.
@@ -1431,10 +1441,20 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
   const int G = (HW % 2) ? 4 : 2;
   const bool groups = !vec && HW > 1 && bases_aligned && (HW * G) % 4 == 0 && C % G == 0 &&
                       static_cast<long long>(G) * per_channel * 8 <= 100 * 1024;
-  // Channels that fit a CTA's registers need no staging.  Where that means
-  // scalar accesses, the group form still wins once the call is bound by bytes
-  // and not by latency and no mask has to be formed (32x2048x7x7: 12.9 against
-  // 13.3 us; 32x512x7x7: 5.7 against 4.5; with ReLU 16.8 against 13.7).
+  // Channels that fit a CTA's registers need no staging.  Where that means scalar
+  // accesses and no mask has to be formed, the group form takes over above 2e6
+  // elements, where the call is bound by bytes and no longer by latency.  Time in
+  // groups over time in registers (odd planes of 9 to 225, cold inputs), by how
+  // many of the threads' 1024, 2048 or 3072 slots a channel fills:
+  //   elements of a channel   1.5e6      2.2e6      4.5e6      12e6
+  //   1125-1215 (of 2048)    .95-1.01   .89-.95    .80-.83    .67-.70
+  //   567-605 (of 1024)     1.07-1.17   .99-1.09   .89-.96    -
+  //   1450-1575 (of 2048)   1.11-1.18  1.03-1.11   .93-1.01   .82-.87
+  //   2050-2110 (of 3072)   1.23-1.27   .98-1.00   .93-.96    .82-.85
+  //   845-900, 1780-2030, 2475-3040 (nearly all)
+  //                         1.12-1.46  1.18-1.55  1.08-1.37   .93-1.21
+  // So the line is right for channels that leave a quarter of the slots empty, and
+  // on the group form's side by up to half of the time for those that fill them.
   if (!(groups && MASK == 0 && per_channel * C > 2000000LL)) {
     int st = SGB_OK;
     auto go = [&](auto g, auto nv, auto v) {

@@ -155,9 +155,10 @@ maxpool_bwd_band_kernel(const float* __restrict__ x, const float* __restrict__ d
 // Same scheme with the geometry (square kernel K, stride S, padding P) known
 // at compile time: window loops unroll, the divisions by the stride become
 // shifts, dy rows are staged in shared memory as well, and every thread
-// produces four consecutive dx values of one row (one 128-bit store).  This is
-// the form the ResNet stem (3x3 / 2 / 1) and the small CNN (2x2 / 2 / 0) hit;
-// it needs W % 4 == 0.  About 60 instructions per dx element instead of ~200.
+// produces four consecutive dx values of one row (one 128-bit store).  For the
+// square windows that have no form of their own further down (3x3 / 2 / 0 and
+// 2x2 / 1 / 0); it needs W % 4 == 0.  About 60 instructions per dx element
+// instead of ~200.
 template <int K, int S, int P>
 __global__ void __launch_bounds__(kBlock)
 maxpool_bwd_band_fast_kernel(const float* __restrict__ x, const float* __restrict__ dy,
@@ -854,7 +855,9 @@ int launch_k3s1p1(const float* x, const float* dy, float* out, unsigned char* re
 // The windows do not overlap: a thread owns four columns of two rows, i.e. two
 // whole windows.  Rows and columns that no window covers (odd sizes) get zero
 // gradient.  One 16-byte access per row where the width allows it.
-struct FastDiv {           // n / d for n < 2^31 by multiplication with ceil(2^(31 + l) / d), l = ceil(log2 d)
+// n / d for n < 2^31 by multiplication with ceil(2^(31 + l) / d), l = ceil(log2 d):
+// division by invariant integers (T. Granlund, P. L. Montgomery, 1994).
+struct FastDiv {
   unsigned d, mul, shift;
   explicit FastDiv(unsigned div) : d(div) {
     unsigned l = 0;

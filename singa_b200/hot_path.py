@@ -230,7 +230,7 @@ class HotPathGPU(object):
         torch.cuda.synchronize()
 
     def host_copy(self):
-        """numpy copies of every tensor + moments (inputs for the CPU checker)."""
+        """numpy copies of every tensor + moments (inputs for the oracle)."""
         out = {k: v.detach().cpu().numpy().copy() for k, v in self.t.items() if k != "grad_arena"}
         out.update({"m:" + k: v.detach().cpu().numpy().copy() for k, v in self.moments.items()})
         return out

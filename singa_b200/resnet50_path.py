@@ -17,7 +17,7 @@ softmax-cross-entropy forward/backward, the bias-gradient reduction, the
 gradient synchronisation and the optimizer - is computed.
 
 ``build_plan`` is pure python (no device): it returns tensor specs and an op
-list that an executor (GPU: ``HotPathGPU`` below; CPU checker: the oracle
+list that an executor (GPU: ``HotPathGPU`` below; CPU: the oracle
 executor in bench.py/tests) walks in order.
 """
 from collections import namedtuple
@@ -377,7 +377,7 @@ def mask_plan(plan):
     backward) to consume the forward partner's one-bit-per-element record
     "mask:<relu input>" instead of the stored ReLU input.  Opt-in: it changes
     what the backward pass consumes.  The ops keep the name of the original
-    input under "x_ref" so that a checker can recompute the decisions."""
+    input under "x_ref" so that the oracle can recompute the decisions."""
     T = dict(plan["tensors"])
     rename = {"relu_bwd": ("relu_mask_bwd", "x"), "add_relu_bwd": ("add_relu_mask_bwd", "x"),
               "bn_relu_bwd": ("bn_relu_mask_bwd", "relu_x")}
