@@ -129,11 +129,24 @@ class DistOpt(object):
         which then has to be called."""
         c = self.communicator
         whole = getattr(c, name, None)
-        if whole is None or any(f in vars(self) or getattr(type(self), f) is not getattr(DistOpt, f) for f in forwards):
+        if whole is None:
             return None
-        owner = next((k for k in type(c).__mro__ if name in vars(k)), None)
-        if owner is None or any(f in vars(c) or getattr(type(c), f, None) is not getattr(owner, f, None) for f in calls):
-            return None
+        mine, own, theirs, kind = self.__dict__, type(self), getattr(c, "__dict__", ()), type(c)
+        for f in forwards:
+            if f in mine or (own is not DistOpt and getattr(own, f) is not getattr(DistOpt, f)):
+                return None
+        for f in calls:
+            if f in theirs:
+                return None
+        if name not in kind.__dict__:                     # inherited: whose calls does it stand for?
+            for owner in kind.__mro__:
+                if name in owner.__dict__:
+                    break
+            else:
+                return None
+            for f in calls:
+                if getattr(kind, f, None) is not getattr(owner, f, None):
+                    return None
         return whole
 
     def _update_all(self, plist):
