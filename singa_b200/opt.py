@@ -285,7 +285,7 @@ class DistOpt(object):
         # A communicator that offers the exchange in two halves has bucket k's
         # selection issued before the host waits for the counts of bucket k-1.
         parts = ("sparsification", "fused_sparsification"), ("sparsification", "fusedSparsification")
-        begin = self._whole("beginSparsification", *parts)
+        begin = None
         opened = 0
 
         def exchange(tensors, res, single):
@@ -302,18 +302,22 @@ class DistOpt(object):
                 self.fused_sparsification(tensors, res, spars, topK)
 
         # On one rank, gradients that all exist already go through one selection.
-        joint = self._whole("sparsifyBuckets", *parts)
+        joint = None
+        if (corr and not topK and self.world_size == 1 and
+                type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
+            joint = self._whole("sparsifyBuckets", *parts)
         try:
-            if (joint is not None and corr and not topK and self.world_size == 1 and
-                    type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
+            if joint is not None:
                 ready = []
                 for tensors, n, single in buckets():
                     k += 1
                     ready.append((tensors, residual(n, tensors[0]), single))
                 if not ready or not joint([b[0] for b in ready], [b[1] for b in ready], spars):
+                    begin = self._whole("beginSparsification", *parts)
                     for b in ready:
                         exchange(*b)
             else:
+                begin = self._whole("beginSparsification", *parts)
                 for tensors, n, single in buckets():
                     k += 1
                     exchange(tensors, residual(n, tensors[0]), single)
