@@ -5,6 +5,8 @@ The reference builds gradients with its autograd generator; this module takes
 any iterable of ``(param, grad)`` pairs in the order gradients are produced
 (what ``autograd.backward(loss)`` yields, python/singa/autograd.py:128-224).
 """
+import functools
+
 import numpy as np
 
 from . import singa_wrap as sw
@@ -75,6 +77,34 @@ class SGD(object):
         self.step_counter += 1
 
 
+# exchange: (the communicator's method for all of it, DistOpt's forwards and the
+# communicator's calls that it stands for)
+_WHOLE = {
+    "plain": ("syncDense", ("all_reduce", "fused_all_reduce"), ("synch", "fusedSynch")),
+    "half": ("syncDense", ("all_reduce_half", "fused_all_reduce_half"), ("synchHalf", "fusedSynchHalf")),
+    "sparse": ("beginSparsification", ("sparsification", "fused_sparsification"),
+               ("sparsification", "fusedSparsification")),
+    "joint": ("sparsifyBuckets", ("sparsification", "fused_sparsification"), ("sparsification", "fusedSparsification")),
+}
+
+
+@functools.lru_cache(maxsize=64)
+def _inverse(world_size):
+    """1 / world_size as fp32 forms it."""
+    return float(np.float32(1.0) / np.float32(world_size))
+
+
+@functools.lru_cache(maxsize=64)
+def _stands(own, kind, exchange):
+    """Whether the method of communicators of class `kind` does what `own` (DistOpt
+    or a subclass) would do call by call: nobody below the class that defines it
+    has a version of its own of a call."""
+    name, forwards, calls = _WHOLE[exchange]
+    owner = next((k for k in kind.__mro__ if name in vars(k)), None)
+    return owner is not None and all(getattr(own, f) is getattr(DistOpt, f) for f in forwards) and \
+        all(getattr(kind, f, None) is getattr(owner, f, None) for f in calls)
+
+
 class DistOpt(object):
     """Data-parallel wrapper of an optimizer (opt.py:686-1094).
 
@@ -119,38 +149,22 @@ class DistOpt(object):
 
     def update(self, param, grad, name=None):
         """grad /= world_size, then the wrapped optimizer's update."""
-        scale = float(np.float32(1.0) / np.float32(self.world_size))
+        scale = _inverse(self.world_size)
         self.opt.apply(name if name is not None else id(param), param, grad, grad_scale=scale)
 
-    def _whole(self, name, forwards, calls):
-        """The communicator's method `name`, which stands for a sequence of its
-        `calls`: None where the communicator has none, or where a subclass or an
-        instance has its own version of one of them or of this class's `forwards`,
-        which then has to be called."""
+    def _whole(self, exchange):
+        """The communicator's method that does the whole `exchange` (_WHOLE): None
+        where it has none, or where a subclass or an instance has its own version
+        of one of the calls that it stands for, which then has to be called."""
         c = self.communicator
-        whole = getattr(c, name, None)
-        if whole is None:
+        name, (f, g), (x, y) = _WHOLE[exchange]
+        mine, theirs = self.__dict__, getattr(c, "__dict__", ())
+        if f in mine or g in mine or x in theirs or y in theirs or not _stands(type(self), type(c), exchange):
             return None
-        mine, own, theirs, kind = self.__dict__, type(self), getattr(c, "__dict__", ()), type(c)
-        for f in forwards:
-            if f in mine or (own is not DistOpt and getattr(own, f) is not getattr(DistOpt, f)):
-                return None
-        for f in calls:
-            if f in theirs:
-                return None
-        if name not in kind.__dict__:                     # inherited: whose calls does it stand for?
-            for owner in kind.__mro__:
-                if name in owner.__dict__:
-                    break
-            else:
-                return None
-            for f in calls:
-                if getattr(kind, f, None) is not getattr(owner, f, None):
-                    return None
-        return whole
+        return getattr(c, name)
 
     def _update_all(self, plist):
-        scale = float(np.float32(1.0) / np.float32(self.world_size))
+        scale = _inverse(self.world_size)
         names, params, grads = plist
         if names:
             self.opt.apply_many(names, params, grads, scale)
@@ -158,8 +172,7 @@ class DistOpt(object):
 
     def _sync_dense(self, grad_stream, threshold, direct, fused, half=False):
         """Names, parameters and (reduced) gradients of the stream."""
-        whole = self._whole("syncDense", ("all_reduce_half", "fused_all_reduce_half"), ("synchHalf", "fusedSynchHalf")) \
-            if half else self._whole("syncDense", ("all_reduce", "fused_all_reduce"), ("synch", "fusedSynch"))
+        whole = self._whole("half" if half else "plain")
         if whole is not None:
             plist = whole(grad_stream, threshold, half)
             self.wait()
@@ -284,7 +297,6 @@ class DistOpt(object):
 
         # A communicator that offers the exchange in two halves has bucket k's
         # selection issued before the host waits for the counts of bucket k-1.
-        parts = ("sparsification", "fused_sparsification"), ("sparsification", "fusedSparsification")
         begin = None
         opened = 0
 
@@ -305,7 +317,7 @@ class DistOpt(object):
         joint = None
         if (corr and not topK and self.world_size == 1 and
                 type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
-            joint = self._whole("sparsifyBuckets", *parts)
+            joint = self._whole("joint")
         try:
             if joint is not None:
                 ready = []
@@ -313,11 +325,11 @@ class DistOpt(object):
                     k += 1
                     ready.append((tensors, residual(n, tensors[0]), single))
                 if not ready or not joint([b[0] for b in ready], [b[1] for b in ready], spars):
-                    begin = self._whole("beginSparsification", *parts)
+                    begin = self._whole("sparse")
                     for b in ready:
                         exchange(*b)
             else:
-                begin = self._whole("beginSparsification", *parts)
+                begin = self._whole("sparse")
                 for tensors, n, single in buckets():
                     k += 1
                     exchange(tensors, residual(n, tensors[0]), single)
