@@ -367,7 +367,8 @@ int sgb_bn_forward_training_f32(const float *x, const float *scale,
  * receives the sticky fault word of the current device (0 = none; bit 0 a
  * wait ran out, bit 1 a counter table was still in use by another launch - at
  * most eight such launches may be in flight per device; bits 8 and 16 the same
- * for the exchanges inside the backward and forward cluster kernels).  A
+ * for the exchanges inside the backward and forward cluster kernels, bit 24 for
+ * the kernels that visit their data twice).  A
  * faulted launch stops early and its outputs are undefined.  Synchronises the
  * device. */
 int sgb_bn_backward_faults(unsigned *flags);

@@ -26,9 +26,12 @@
 //              from the staged copy; two to four CTAs per SM, so that the load
 //              phase of one overlaps the store phase of another
 //              (bn_bwd_cluster_kernel);
-//   streaming  channels too large for a cluster (e.g. 32 x 112 x 112): persistent
+//   streaming  channels too large for a cluster (e.g. 32 x 112 x 112) and calls
+//              whose workspace is too small for the form below: persistent
 //              small CTAs take 50 KB items of a channel from a ticket counter and
 //              meet through counters in global memory (bn_stream.cu).
+// Ahead of them all, for large calls (revisit_pays): two visits to the data in one
+// kernel, the second out of L2 (bn_revisit.cu).
 //
 // Two passes (20 bytes of HBM traffic per element when the tensor does not fit
 // L2) for what is left: ragged planes too large for a cluster, misaligned
@@ -46,6 +49,7 @@
 // the ReLU that follows the BN layer) into every form, which removes one
 // full write + read of the intermediate gradient.
 #include "bn_common.cuh"
+#include "bn_revisit.cuh"
 #include "bn_stream.cuh"
 
 namespace cg = cooperative_groups;
@@ -1416,6 +1420,27 @@ int takes_cluster(long long per_channel, bool vec, int C, int* per_cta) {
   return static_cast<long long>(C) * cs <= 0x7fffffffLL ? cs : 0;
 }
 
+// Whether a call takes the form that visits its data twice (bn_revisit.cu).  It
+// overlaps everything but its first loads and last stores, which a call has to be
+// large enough for; the line is the same whatever the mask, so that a fused call
+// and its parts agree bit for bit.  Time of the forms below / of this one, with and
+// without a ReLU:
+//   32x128x28x28  (3.2e6 elements)  14.0 / 11.9    9.9 / 10.2
+//   12x48x80x80   (3.7e6)           14.0 / 13.3   10.1 / 11.3
+//   32x40x56x56   (4.0e6)           16.2 / 13.9   11.3 / 11.3
+//   8x512x32x32   (4.2e6)           18.3 / 15.6   13.8 / 13.2
+//   32x1024x14x14 (6.4e6)           24.1 / 22.0   18.3 / 18.5
+//   12x200x50x50  (6.0e6)           25.4 / 20.0   17.4 / 16.1
+// Planes that are no multiple of four pay for their masked ends twice:
+//   24x64x71x71   (7.7e6)           40.0 / 28.1   27.6 / 23.7
+//   18x256x33x33  (5.0e6)           25.4 / 19.8   16.1 / 17.0
+//   24x1024x15x15 (5.5e6)           28.6 / 22.6   17.9 / 20.2
+inline bool revisit_pays(int N, int C, int HW, bool aligned, bool groups) {
+  const long long elements = static_cast<long long>(N) * C * HW;
+  if (HW % 4) return aligned && !groups && HW >= 2500 && elements >= 6000000;
+  return aligned && HW >= 8 && elements >= 4000000;
+}
+
 template <int MASK>
 int bn_backward(const float* x, const float* dy, const float* relu_in, const float* scale,
                 const float* mean, const float* invstd, float* dx, float* dscale,
@@ -1441,6 +1466,11 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
   const int G = (HW % 2) ? 4 : 2;
   const bool groups = !vec && HW > 1 && bases_aligned && (HW * G) % 4 == 0 && C % G == 0 &&
                       static_cast<long long>(G) * per_channel * 8 <= 100 * 1024;
+  if (revisit_pays(N, C, HW, bases_aligned, groups)) {
+    const int st = bn_revisit_backward(MASK, x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, N, C, HW, ws,
+                                       ws_bytes, s);
+    if (st != SGB_ERR_WORKSPACE) return st;            // a smaller workspace: the forms below
+  }
   // Channels that fit a CTA's registers need no staging.  Where that means scalar
   // accesses and no mask has to be formed, the group form takes over above 2e6
   // elements, where the call is bound by bytes and no longer by latency.  Time in
@@ -1533,7 +1563,7 @@ int bn_add_relu_backward(const float* x, const float* dy_a, const float* dy_b, c
   if (per_channel > 0x7fffffffLL || C > 65535) return SGB_ERR_SIZE;
   const bool vec = (HW % 4 == 0) && aligned16(x) && aligned16(dy_a) && aligned16(dy_b) &&
                    aligned16(relu_in) && aligned16(joined) && aligned16(dx);
-  if (vec) {
+  if (vec && !revisit_pays(N, C, HW, true, false)) {
     const BnShape sh{N, C, HW};
     cudaStream_t s = as_stream(stream);
     // the same forms as without the join (same sums, bit for bit)
@@ -1647,7 +1677,11 @@ extern "C" {
 
 size_t sgb_bn_backward_workspace_bytes(int N, int C, int HW) {
   if (N <= 0 || C <= 0 || HW <= 0) return 0;
-  return static_cast<size_t>(kMaxSlices) * C * sizeof(float2);
+  size_t need = static_cast<size_t>(kMaxSlices) * C * sizeof(float2);
+  const size_t backward = revisit_pays(N, C, HW, true, false) ? bn_revisit_workspace_bytes(N, C, HW) : 0;
+  const size_t forward = bn_forward_workspace_bytes(N, C, HW);
+  if (backward > need) need = backward;
+  return forward > need ? forward : need;
 }
 
 int sgb_bn_backward_faults(unsigned* flags) {
@@ -1660,7 +1694,10 @@ int sgb_bn_backward_faults(unsigned* flags) {
   unsigned forward = 0;
   const int fs = bn_forward_faults(&forward);
   if (fs != SGB_OK) return fs;
-  *flags = streaming | (cluster << 8) | (forward << 16);
+  unsigned revisit = 0;
+  const int rs = revisit_faults(&revisit);
+  if (rs != SGB_OK) return rs;
+  *flags = streaming | (cluster << 8) | (forward << 16) | (revisit << 24);
   return SGB_OK;
 }
 

@@ -14,6 +14,8 @@ namespace sgb {
 
 // Sticky fault word of the forward cluster kernel (0: none), see batchnorm.cu.
 int bn_forward_faults(unsigned* flags);
+// What the forward form needs beyond the partial sums of two passes.
+size_t bn_forward_workspace_bytes(int N, int C, int HW);
 
 namespace {
 

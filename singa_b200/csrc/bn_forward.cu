@@ -9,16 +9,18 @@
 //   n = na + nb,  mean = ma + d nb/n,  m2 = m2a + m2b + d^2 na nb/n,  d = mb - ma:
 // T. F. Chan, G. H. Golub, R. J. LeVeque, 1983), never E[x^2] - E[x]^2.
 //
-// Three forms, by the size of a channel:
+// Four forms, by the size of a channel and of the call:
 //   registers   up to 8192 floats: one CTA (or a warp) per channel, one pass;
 //   cluster     up to 8 CTAs' shared memory: one pass; every CTA works out the
 //               moments of its share and the CTAs exchange them ONCE (sum, m2
 //               and count in one asynchronous store per pair of CTAs);
-//   two passes  anything larger: per-slice moments, then normalisation, which
+//   two visits  large channels of large calls (fwd_revisit_pays): one kernel that
+//               reads its data twice, the second time out of L2;
+//   two passes  anything else: per-slice moments, then normalisation, which
 //               adds the slices up itself (2 launches; 5 before).
 // Units are 16-byte vectors, also where planes are not a multiple of four
 // floats (RaggedUnit); single floats only for misaligned tensors and tiny planes.
-#include "bn_common.cuh"
+#include "bn_revisit.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -427,7 +429,6 @@ bn_fwd_hybrid_kernel(const FwdArgs a, int per_cta) {
   }
 }
 
-// -------------------------------------------------------------- in two passes
 struct Moments {
   float n, mean, m2;
 };
@@ -451,6 +452,145 @@ __device__ __forceinline__ Moments warp_merge(Moments v) {
   return v;              // valid in lane 0
 }
 
+// ------------------------------------------------------------ in two visits
+// See bn_revisit.cuh.  An item leaves its mean and its sum of squared differences.
+// One operand only, so a CTA takes more units: of 3 to 6 vectors and 192 to 288
+// threads these were the best (32x256x56x56 42.4 us against 43.8-47.6,
+// 32x128x57x57 28.7 against 30.2-37.9).
+template <bool VEC>
+constexpr RevisitShape kFwd = VEC ? RevisitShape{6, 256, 4} : RevisitShape{3, 256, 5};
+
+// Elements of channel c ahead of unit u.
+template <bool VEC>
+__device__ __forceinline__ unsigned elements_before(const Revisit& r, unsigned c, unsigned u) {
+  if (VEC) return 4 * u;
+  const unsigned n = r.upp.quot(u), q = u - n * r.upp.d, lead = (n * r.plane_stride + c * r.hw) & 3u;
+  return n * r.hw + (4 * q > lead ? min(4 * q - lead, r.hw) : 0u);
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kFwd<VEC>.threads + 32, kFwd<VEC>.per_sm)
+bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__ Revisit r) {
+  constexpr int NV = kFwd<VEC>.units, kWarps = kFwd<VEC>.threads / 32;
+  __shared__ float sm[2][kWarps];
+  __shared__ float coef[3];
+  const unsigned item = blockIdx.x, mine = item - r.delay, threads = blockDim.x - 32;
+  const bool summing = static_cast<int>(item) < r.items, finishing = static_cast<int>(item) >= r.delay;
+  const unsigned numel = static_cast<unsigned>(a.numel);
+  if (threadIdx.x >= threads) {
+    dependency_wait();
+    release_dependents();
+    if (!finishing) return;
+    const unsigned c = r.parts.quot(mine);
+    const float sc = a.scale[c], b = a.bias[c];
+    Moments m{0.f, 0.f, 0.f};
+    revisit_gather(r, c, [&](unsigned k, float mean, float m2) {
+      const unsigned e0 = elements_before<VEC>(r, c, k * r.per), e1 = elements_before<VEC>(r, c, min((k + 1) * r.per, r.total));
+      m = merge(m, Moments{static_cast<float>(e1 - e0), mean, m2});
+    });
+    m = warp_merge(m);
+    if ((threadIdx.x & 31) == 0) {
+      const float var = m.m2 / (static_cast<float>(a.sh.N) * static_cast<float>(a.sh.HW));
+      const float invstd = 1.0f / sqrtf(var + a.eps);
+      coef[0] = m.mean;
+      coef[1] = sc * invstd;
+      coef[2] = b;
+      if (mine == c * r.parts.d) finish_channel(a, c, m.mean, var, invstd);
+    }
+    revisit_arrive(2, blockDim.x);
+    revisit_leave(r, c);
+    return;
+  }
+  Vec4f v[NV];
+  // Sum over the summing threads; every thread adds the warps' sums up itself.
+  auto total = [&](float x, float (&s)[kWarps]) {
+    x = warp_sum(x);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = x;
+    revisit_sync(1, threads);
+    x = 0.f;
+    for (unsigned w = 0; w < threads / 32; ++w) x += s[w];
+    return x;
+  };
+  if (summing) {
+    const RevisitUnits<VEC, NV> u(r, item, threads);
+    if (first_wave(kFwd<VEC>.per_sm)) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (u.valid[k] && (VEC || u.off[k] < numel)) prefetch_l2(a.x + u.off[k]);
+    }
+    dependency_wait();
+    const unsigned long long keep = keep_policy();
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (u.valid[k]) v[k] = u.load(a.x, k, numel, keep);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (u.valid[k] >> j & 1u) s += v[k].f[j];
+    const unsigned e0 = elements_before<VEC>(r, u.c, u.part * r.per),
+                   e1 = elements_before<VEC>(r, u.c, min((u.part + 1) * r.per, r.total));
+    const float mean = e1 > e0 ? total(s, sm[0]) / static_cast<float>(e1 - e0) : total(s, sm[0]);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (u.valid[k] >> j & 1u) {
+          const float d = v[k].f[j] - mean;
+          q += d * d;
+        }
+    q = total(q, sm[1]);
+    if (threadIdx.x == 0) revisit_publish(r, item, u.c, u.part, mean, q);
+  } else {
+    dependency_wait();
+  }
+  if (!finishing) return;
+  const RevisitUnits<VEC, NV> u(r, mine, threads);
+  const unsigned long long ease = ease_policy();
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (u.valid[k]) v[k] = u.load(a.x, k, numel, ease);
+  revisit_sync(2, blockDim.x);
+  const float mu = coef[0], g = coef[1], b = coef[2];
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (u.valid[k]) {
+      Vec4f o;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o.f[j] = (v[k].f[j] - mu) * g + b;
+      u.store(a.y, k, o);
+    }
+}
+
+// One operand is little to overlap with, so only channels that leave clusters with
+// large shares or no place at all gain (us, the forms above and below / this one):
+//   32x64x112x112 61.5 / 41.3   32x256x56x56 44.5 / 42.4   32x64x56x56 14.9 / 14.2
+//   64x100x40x40  19.4 / 19.6   32x512x28x28 25.3 / 26.6   10x256x52x52 15.3 / 15.9
+//   32x64x111x111 99.1 / 53.1   32x128x57x57 37.3 / 28.7   24x64x71x71 24.4 / 18.8
+//   16x1024x13x13 14.1 / 14.5 (2.8e6 elements)
+inline bool fwd_revisit_pays(int N, int C, int HW) {
+  const long long channel = static_cast<long long>(N) * HW;
+  if (HW % 4) return HW >= 2500 && channel * C >= 6000000;
+  return HW >= 2500 && channel >= 65536 && channel * C >= 6000000;
+}
+
+// SGB_ERR_WORKSPACE and nothing done where the workspace is too small or the problem too large.
+template <bool VEC>
+int launch_revisit(const FwdArgs& a, void* ws, size_t ws_bytes, cudaStream_t s) {
+  const int upp = units_per_plane(VEC ? kVec : kRagged, a.sh.HW);
+  const long long units = static_cast<long long>(a.sh.N) * upp;
+  RevisitPlan p;
+  if (!ws || !aligned16(ws) || !revisit_plan(kFwd<VEC>, units, upp, a.sh.C, &p) || ws_bytes < p.bytes)
+    return SGB_ERR_WORKSPACE;
+  int st = SGB_OK;
+  unsigned* faults = revisit_fault_word(&st);
+  if (!faults) return st;
+  return launch_ex(bn_fwd_revisit_kernel<VEC>, dim3(static_cast<unsigned>(p.items + p.delay)), dim3(p.threads + 32), 0,
+                   s, 0, true, a, revisit_args(p, units, upp, a.sh.C, a.sh.HW, ws, faults));
+}
+
+// ------------------------------------------------------------- in two passes
 // Pass 1, grid (slices, C): moments of a slice.  A thread works out those of
 // four units at a time (in registers) and merges them into its own.
 template <int KIND>
@@ -611,6 +751,13 @@ int launch_large(const FwdArgs& a, void* ws, size_t ws_bytes, cudaStream_t s) {
 
 }  // namespace
 
+size_t bn_forward_workspace_bytes(int N, int C, int HW) {
+  const int upp = units_per_plane(HW % 4 ? kRagged : kVec, HW);
+  RevisitPlan p;
+  if (!fwd_revisit_pays(N, C, HW)) return 0;
+  return revisit_plan(HW % 4 ? kFwd<false> : kFwd<true>, static_cast<long long>(N) * upp, upp, C, &p) ? p.bytes : 0;
+}
+
 int bn_forward_faults(unsigned* flags) {
   const cudaError_t e = cudaMemcpyFromSymbol(flags, g_forward_faults, sizeof(unsigned));
   return e == cudaSuccess ? SGB_OK : note_cuda_error(e);
@@ -636,6 +783,11 @@ int sgb_bn_forward_training_f32(const float* x, const float* scale, const float*
                   BnShape{N, C, HW}, static_cast<size_t>(per_channel) * C};
   const bool bases = aligned16(x) && aligned16(y), vec = HW % 4 == 0 && bases;
   int st = SGB_OK;
+  if (bases && fwd_revisit_pays(N, C, HW)) {
+    st = vec ? launch_revisit<true>(a, ws, ws_bytes, s) : launch_revisit<false>(a, ws, ws_bytes, s);
+    if (st != SGB_ERR_WORKSPACE) return st;
+    st = SGB_OK;
+  }
   auto small = [&](auto g, auto nv, auto v) {
     constexpr int kG = decltype(g)::value, kNV = decltype(nv)::value;
     st = launch_ex(bn_fwd_small_kernel<kG, kNV, decltype(v)::value>,
