@@ -951,9 +951,9 @@ def main():
 
 def kernel_launches(path):
     """Kernels of this library launched per step (NCCL's own are not counted).
-    Batch-norm backward is one launch, except when a channel (x and dy of all
-    samples) exceeds what a cluster of eight CTAs can stage (8 x 100 KB): then
-    it is the reduce + apply pair."""
+    Batch-norm backward is one launch, except for ragged planes of small calls
+    when a channel (x and dy of all samples) exceeds what a cluster of eight CTAs
+    can stage (8 x 100 KB): then it is the reduce + apply pair."""
     per = {"sgb_relu_backward_f32": 1, "sgb_add_relu_backward_f32": 1, "sgb_binary_f32": 1,
            "sgb_relu_backward_mask_f32": 1, "sgb_add_relu_backward_mask_f32": 1,
            "sgb_maxpool_backward_f32": 1, "sgb_maxpool_backward_argmax_f32": 1,
@@ -961,13 +961,14 @@ def kernel_launches(path):
            "sgb_sum_all_f32": 1, "sgb_softmax_cross_entropy_bwd_f32": 1,
            "sgb_softmax_cross_entropy_grad_f32": 1, "sgb_softmax_cross_entropy_fused_f32": 1,
            "sgb_scalar_f32": 1, "sgb_sum_rows_f32": 1, "sgb_set_f32": 1, "sgb_conv_bias_backward_f32": 1,
-           "sgb_relu_backward_sum_rows_f32": 1, "sgb_relu_backward_conv_bias_f32": 1}
+           "sgb_relu_backward_sum_rows_f32": 1, "sgb_relu_backward_conv_bias_f32": 1,
+           "sgb_maxpool_relu_backward_conv_bias_f32": 1, "sgb_loss_head_f32": 2}
     n = 0
     for name, args in path.launched:
         if name in ("sgb_bn_backward_f32", "sgb_bn_relu_backward_f32", "sgb_bn_relu_backward_mask_f32",
                     "sgb_bn_add_relu_backward_f32"):
-            N, _, HW = args[-6:-3]          # (..., N, C, HW, workspace, workspace bytes, stream)
-            n += 2 if N * HW * 8 > 8 * 100 * 1024 else 1
+            N, c, HW = args[-6:-3]          # (..., N, C, HW, workspace, workspace bytes, stream)
+            n += 2 if N * HW * 8 > 8 * 100 * 1024 and HW % 4 and (HW < 2500 or N * c * HW < 6000000) else 1
         elif name == "sgb_unpack_f32":       # stand-in weight gradients: one launch per 72 tensors
             n += (args[4] + 71) // 72
         else:

@@ -263,6 +263,13 @@ int sgb_conv_bias_backward_f32(const float *dy, float *db, int N, int C, int HW,
 /* The same for a convolution: relu_backward and conv_bias_backward of its result. */
 int sgb_relu_backward_conv_bias_f32(const float *dy, const float *x, float *dx, float *db, int N, int C, int HW,
                                     void *ws, size_t ws_bytes, void *stream);
+/* The same behind a max pooling: sgb_maxpool_backward_f32(pool_x, pool_y, dy ->
+ * pool_dx), whose result goes through the call above; one launch for windows of
+ * 2x2 with stride 2 and no padding. */
+int sgb_maxpool_relu_backward_conv_bias_f32(const float *pool_x, const float *pool_y, const float *dy, float *pool_dx,
+                                            int N, int C, int H, int W, int kh, int kw, int ph, int pw, int sh, int sw,
+                                            const float *x, float *dx, float *db, void *ws, size_t ws_bytes,
+                                            void *stream);
 /* SumAll: out[0] = sum of x (device scalar).  Replaces SumAll
  * (tensor.cc:1242-1254: ones tensor + Dot<float, lang::Cuda>,
  * tensor_math_cuda.h:1084-1094). */
@@ -306,6 +313,12 @@ int sgb_softmax_cross_entropy_fused_f32(const float *logits, const int32_t *t,
                                         size_t batch, size_t dim, float scale,
                                         float *prob, float *loss, float *grad,
                                         void *stream);
+/* The same, then *total = the sum of the losses (sgb_sum_all_f32) and bias_grad =
+ * the column sums of grad (sgb_sum_rows_f32): one or two launches, the same bits
+ * as the three calls.  Workspace: what either sum needs. */
+int sgb_loss_head_f32(const float *logits, const int32_t *t, size_t batch, size_t dim,
+                      float scale, float *prob, float *loss, float *grad, float *total,
+                      float *bias_grad, void *ws, size_t ws_bytes, void *stream);
 
 /* fp16 forms.  Softmax computes in fp32 and rounds once on store.  The two
  * cross-entropy kernels keep the half-precision arithmetic of the overloads

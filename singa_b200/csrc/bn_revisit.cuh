@@ -80,38 +80,22 @@ inline bool revisit_plan(const RevisitShape& shape, long long units, int upp, in
   return true;
 }
 
-// n / d for n < 2^31 by a multiplication and a shift: mul = ceil(2^(31+l) / d) with
-// 2^l >= d exceeds 2^(31+l) / d by less than 1, so the error of the product is below
-// n / 2^(31+l) < 1 / d (the method of T. Granlund and P. L. Montgomery, 1994).
-struct Divisor {
-  unsigned d, mul, shift;
-  explicit Divisor(unsigned div) : d(div) {
-    unsigned l = 0;
-    while ((1ull << l) < div) ++l;
-    shift = 31 + l;
-    mul = static_cast<unsigned>(((1ull << shift) + div - 1) / div);
-  }
-  __device__ __forceinline__ unsigned quot(unsigned n) const {
-    return static_cast<unsigned>((static_cast<unsigned long long>(n) * mul) >> shift);
-  }
-};
-
 struct Revisit {
   RevisitEntry* entries;               // one per item
   unsigned* readers;                   // per channel: items finished
   unsigned long long tag;
   unsigned* faults;
-  Divisor parts;
+  FastDiv parts;
   unsigned per, total;                 // units per item, per channel
   int items, delay;
-  Divisor upp;                         // units per plane
+  FastDiv upp;                         // units per plane
   unsigned hw, plane_stride;           // plane_stride: elements per sample
 };
 inline Revisit revisit_args(const RevisitPlan& p, long long units, int upp, int C, int HW, void* ws, unsigned* faults) {
   char* const base = static_cast<char*>(ws);
   return Revisit{reinterpret_cast<RevisitEntry*>(base), reinterpret_cast<unsigned*>(base + p.readers), revisit_tag(),
-                 faults, Divisor(static_cast<unsigned>(p.parts)), static_cast<unsigned>(p.per),
-                 static_cast<unsigned>(units), p.items, p.delay, Divisor(static_cast<unsigned>(upp)),
+                 faults, FastDiv(static_cast<unsigned>(p.parts)), static_cast<unsigned>(p.per),
+                 static_cast<unsigned>(units), p.items, p.delay, FastDiv(static_cast<unsigned>(upp)),
                  static_cast<unsigned>(HW), static_cast<unsigned>(C) * static_cast<unsigned>(HW)};
 }
 

@@ -82,6 +82,21 @@ inline unsigned capped_grid(size_t work_items, size_t per_cta, int ctas_per_sm) 
   return static_cast<unsigned>(need < cap ? need : cap);
 }
 
+// n / d for n < 2^31 by multiplication with ceil(2^(31 + l) / d), l = ceil(log2 d):
+// division by invariant integers (T. Granlund, P. L. Montgomery, 1994).
+struct FastDiv {
+  unsigned d, mul, shift;
+  explicit FastDiv(unsigned div) : d(div) {
+    unsigned l = 0;
+    while ((1ull << l) < div) ++l;
+    shift = 31 + l;
+    mul = static_cast<unsigned>(((1ull << shift) + div - 1) / div);
+  }
+  __device__ __forceinline__ unsigned quot(unsigned n) const {
+    return static_cast<unsigned>((static_cast<unsigned long long>(n) * mul) >> shift);
+  }
+};
+
 // ---------------------------------------------------------------- device side
 // Programmatic dependent launch.  dependency_wait: returns once every kernel
 // this grid depends on has completed and its writes are visible (a no-op for

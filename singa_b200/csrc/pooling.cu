@@ -855,21 +855,6 @@ int launch_k3s1p1(const float* x, const float* dy, float* out, unsigned char* re
 // The windows do not overlap: a thread owns four columns of two rows, i.e. two
 // whole windows.  Rows and columns that no window covers (odd sizes) get zero
 // gradient.  One 16-byte access per row where the width allows it.
-// n / d for n < 2^31 by multiplication with ceil(2^(31 + l) / d), l = ceil(log2 d):
-// division by invariant integers (T. Granlund, P. L. Montgomery, 1994).
-struct FastDiv {
-  unsigned d, mul, shift;
-  explicit FastDiv(unsigned div) : d(div) {
-    unsigned l = 0;
-    while ((1ull << l) < div) ++l;
-    shift = 31 + l;
-    mul = static_cast<unsigned>(((1ull << shift) + div - 1) / div);
-  }
-  __device__ __forceinline__ unsigned quot(unsigned n) const {
-    return static_cast<unsigned>((static_cast<unsigned long long>(n) * mul) >> shift);
-  }
-};
-
 struct PairArgs {
   const float* x;
   const float* dy;

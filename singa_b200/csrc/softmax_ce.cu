@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "reduce.cuh"
 
 namespace sgb {
 namespace {
@@ -478,6 +479,16 @@ int sgb_softmax_cross_entropy_fused_f32(const float* logits, const int32_t* t, s
   if (st != -1000) return st;
   return launch_ex(softmax_ce_long_kernel, dim3(static_cast<unsigned>(batch)), dim3(1024), 0, as_stream(stream), 0, true,
                    logits, t, prob, loss, grad, dim, scale);
+}
+
+int sgb_loss_head_f32(const float* logits, const int32_t* t, size_t batch, size_t dim, float scale, float* prob,
+                      float* loss, float* grad, float* total, float* bias_grad, void* ws, size_t ws_bytes, void* stream) {
+  int st = sgb_softmax_cross_entropy_fused_f32(logits, t, batch, dim, scale, prob, loss, grad, stream);
+  if (st != SGB_OK) return st;
+  if (batch && dim && total && bias_grad)
+    return sum_rows_beside_total(grad, bias_grad, batch, dim, loss, total, ws, ws_bytes, stream);
+  st = sgb_sum_all_f32(loss, total, batch, ws, ws_bytes, stream);
+  return st != SGB_OK ? st : sgb_sum_rows_f32(grad, bias_grad, batch, dim, ws, ws_bytes, stream);
 }
 
 int sgb_softmax_rows_f16(const void* x, void* y, size_t nrow, size_t ncol, void* stream) {

@@ -61,8 +61,12 @@ def merge_calls(calls):
       relu_backward(-> t) ; sum_rows(t)                 =>  relu_backward_sum_rows
       relu_backward(-> t) ; conv_bias_backward(t)       =>  relu_backward_conv_bias
       cross_entropy_bwd(-> g) ; g *= c                  =>  cross_entropy_grad
+      maxpool_backward(-> s) ; relu_backward(s -> t) ; conv_bias_backward(t)
+                                                        =>  maxpool_relu_backward_conv_bias
       softmax(-> p) ; cross_entropy(p -> l) ; sum of l ; cross_entropy_grad(p)
                                                         =>  softmax_cross_entropy_fused ; sum of l
+      softmax_cross_entropy_fused(-> l, g) ; sum of l ; sum_rows(g)
+                                                        =>  loss_head
     """
     out = []
     for name, a in calls:
@@ -75,6 +79,10 @@ def merge_calls(calls):
         elif name == "sgb_conv_bias_backward_f32" and last == "sgb_relu_backward_f32" and a[0] == b[2] and \
                 b[3] == a[2] * a[3] * a[4]:
             out[-1] = ("sgb_relu_backward_conv_bias_f32", b[:3] + a[1:])
+            before, p = out[-2] if len(out) > 1 else ("", None)
+            # (pooling: x, y, dy, dx, n, c, h, w, windows, S; the pair: dy, x, dx, db, n, c, hw, ws, ws bytes, S)
+            if before == "sgb_maxpool_backward_f32" and p[3] == b[0] and p[4:6] == a[2:4] and p[6] * p[7] == a[4]:
+                out[-2:] = [("sgb_maxpool_relu_backward_conv_bias_f32", p[:-1] + b[1:3] + a[1:2] + a[5:])]
         elif name == "sgb_scalar_f32" and last == "sgb_softmax_cross_entropy_bwd_f32" and a[0] == 1 and \
                 a[1] == a[3] == b[5] and a[4] == b[1] * b[2]:
             out[-1] = ("sgb_softmax_cross_entropy_grad_f32", b[:5] + (a[2],) + b[5:])
@@ -87,6 +95,12 @@ def merge_calls(calls):
             if fwd[:5] == grd[:5] == (1,) + sm[2:4] + (sm[1], fwd[4]) and total[1][0] == fwd[5] and grd[6] != sm[0]:
                 out[-4:] = [("sgb_softmax_cross_entropy_fused_f32",
                              (sm[0], fwd[4]) + sm[2:4] + (grd[5], sm[1], fwd[5], grd[6]) + sm[4:]), total]
+        # (fused: x, t, rows, columns, scale, p, l, g, S; sum: l, out, n, ws, ws bytes, S; rows: g, v, rows, columns, ...)
+        if [n for n, _ in out[-3:]] == ["sgb_softmax_cross_entropy_fused_f32", "sgb_sum_all_f32", "sgb_sum_rows_f32"]:
+            (_, f), (_, total), (_, rows) = out[-3:]
+            if total[0] == f[6] and total[2] == f[2] and rows[0] == f[7] and rows[2:4] == f[2:4] and \
+                    total[3:5] == rows[4:6]:
+                out[-3:] = [("sgb_loss_head_f32", f[:8] + total[1:2] + rows[1:2] + rows[4:])]
     return out
 
 

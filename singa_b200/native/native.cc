@@ -856,6 +856,7 @@ const Callable kCallables[] = {
     CALLABLE(sgb_softmax_cross_entropy_grad_f32), CALLABLE(sgb_softmax_cross_entropy_fused_f32),
     CALLABLE(sgb_sum_all_f32), CALLABLE(sgb_sum_rows_f32), CALLABLE(sgb_conv_bias_backward_f32),
     CALLABLE(sgb_relu_backward_sum_rows_f32), CALLABLE(sgb_relu_backward_conv_bias_f32),
+    CALLABLE(sgb_maxpool_relu_backward_conv_bias_f32), CALLABLE(sgb_loss_head_f32),
     CALLABLE(sgb_unpack_f32), CALLABLE(sgb_sgd_update_multi_f32), CALLABLE(sgb_comm_synch),
     CALLABLE(sgb_comm_synch_half), CALLABLE(sgb_comm_fused_synch), CALLABLE(sgb_comm_fused_synch_half),
     CALLABLE(sgb_comm_sparsification), CALLABLE(sgb_comm_wait), CALLABLE(sgb_comm_profile_mark),

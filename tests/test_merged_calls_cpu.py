@@ -30,3 +30,19 @@ def test_the_loss_head_becomes_one_call():
     other = list(head)
     other[3] = ("sgb_softmax_cross_entropy_bwd_f32", (1, 8, 10, 12, 3, 9, S))    # another tensor's probabilities
     assert merge_calls(other)[:3] == other[:3]
+
+
+def test_three_calls_become_one():
+    S = "STREAM"
+    pool = ("sgb_maxpool_backward_f32", (20, 21, 22, 1, 2, 3, 4, 6, 2, 2, 0, 0, 2, 2, S))
+    relu = ("sgb_relu_backward_f32", (1, 2, 3, 144, S))
+    bias = ("sgb_conv_bias_backward_f32", (3, 4, 2, 3, 24, 5, 6, S))
+    assert merge_calls([pool, relu, bias]) == [
+        ("sgb_maxpool_relu_backward_conv_bias_f32", (20, 21, 22, 1, 2, 3, 4, 6, 2, 2, 0, 0, 2, 2, 2, 3, 4, 5, 6, S))]
+    other = ("sgb_maxpool_backward_f32", (20, 21, 22, 9, 2, 3, 4, 6, 2, 2, 0, 0, 2, 2, S))       # not what the ReLU reads
+    assert merge_calls([other, relu, bias])[0] == other
+    fused = ("sgb_softmax_cross_entropy_fused_f32", (1, 3, 8, 10, 0.125, 2, 4, 9, S))
+    total, rows = ("sgb_sum_all_f32", (4, 5, 8, 6, 7, S)), ("sgb_sum_rows_f32", (9, 11, 8, 10, 6, 7, S))
+    assert merge_calls([fused, total, rows]) == [("sgb_loss_head_f32", (1, 3, 8, 10, 0.125, 2, 4, 9, 5, 11, 6, 7, S))]
+    for apart in (("sgb_sum_rows_f32", (12, 11, 8, 10, 6, 7, S)), ("sgb_sum_rows_f32", (9, 11, 10, 8, 6, 7, S))):
+        assert merge_calls([fused, total, apart]) == [fused, total, apart]
