@@ -714,6 +714,21 @@ int sgb_comm_sparsification_end(sgb_comm *c, void *compute_stream);
 int sgb_comm_sparsification_buckets(sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
                                     float *const *accumulations, size_t nbuckets, float threshold,
                                     void *compute_stream);
+/* The same, threshold or (topk) the largest share, with the SGD update of the
+ * buckets' parameters (sgb_sgd_update_multi_f32, in the tensors' order) in the
+ * kernel that writes the dense gradients.  The update has to run on the
+ * communicator's stream, so it is complete behind sgb_comm_wait.  One rank;
+ * SGB_ERR_UNSUPPORTED, and nothing done, where it takes separate calls. */
+int sgb_comm_sparse_update(sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
+                           float *const *accumulations, size_t nbuckets, float spars, int topk, void *const *params,
+                           void *const *moments, float lr, float momentum, float dampening, float weight_decay,
+                           int nesterov, float grad_scale, void *compute_stream);
+/* sgb_comm_round_half and the SGD update behind it in one pass over gradient,
+ * parameter and momentum, on the caller's stream.  One rank; SGB_ERR_UNSUPPORTED,
+ * and nothing done, where sgb_comm_round_half answers so. */
+int sgb_comm_update_half(sgb_comm *c, void *const *params, void *const *grads, void *const *moments,
+                         const size_t *sizes, size_t count, size_t largest, float lr, float momentum, float dampening,
+                         float weight_decay, int nesterov, float grad_scale, void *compute_stream);
 /* Threshold sparsification with a fixed exchange size: every rank sends
  * exactly `capacity` (index, value) slots, the true counts travel on the
  * device, and the host never waits for a count - so the call can sit inside a

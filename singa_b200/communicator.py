@@ -138,6 +138,19 @@ class Communicator(object):
         per bucket: more ranks, profiling, a bucket beyond the limits."""
         return _n.comm_sparsify_buckets(self._ptr, buckets, residuals, threshold)
 
+    def updateHalf(self, params, grads, moments, threshold, hyper):
+        """syncDense in half precision of gradients that all exist, and the SGD
+        update behind it (``hyper``: rate, momentum, dampening, weight decay,
+        Nesterov, gradient scale), in one pass.  False (nothing done) where it
+        takes separate calls: more ranks, profiling, other types."""
+        return _n.comm_update_half(self._ptr, params, grads, moments, threshold, hyper)
+
+    def sparseUpdate(self, buckets, residuals, params, moments, spars, topK, hyper):
+        """Sparsification of buckets that all exist, and the SGD update of their
+        parameters in the kernel that writes the dense gradients; complete behind
+        wait().  False (nothing done) where it takes separate calls."""
+        return _n.comm_sparse_update(self._ptr, buckets, residuals, params, moments, spars, topK, hyper)
+
     def boundedSparsification(self, ts, accumulation, sparsThreshold, capacity):
         """Threshold sparsification with a fixed exchange of `capacity` slots per
         rank and no host wait for the counts (no counterpart in the reference,

@@ -41,6 +41,7 @@ enum Call {
   kSparseSelect = 16,    // the selection on c1, into the next slot
   kSparseExchange = 17,  // of the oldest open exchange: all-gather on s, dense sum on c2
   kSparseLocal = 18,     // the same with one rank: the dense sum on c2 reads the payload in place
+  kSparseUpdate = 20,    // one rank, selections and what reads them one after the other on c1, in one slot
 };
 
 enum Edge : unsigned {
@@ -135,6 +136,13 @@ inline Step plan(State& st, int call) {
       st.sparse ^= 2;
       st.sparse |= 4u << p.slot;
       st.dirty_c1 = st.dirty_c2 = 1;
+      break;
+    case kSparseUpdate:
+      p.slot = st.sparse & 1;
+      p.pre = kComputeToC1 | (st.sparse >> (2 + p.slot) & 1 ? kConsumedToC1 : 0u);
+      p.result_stream = kStreamC1;
+      st.sparse ^= 3;
+      st.dirty_c1 = 1;
       break;
     case kStageCopy:
       p.pre = kComputeToC1;

@@ -13,7 +13,7 @@
 // only beyond that are several launches made.
 // Every CTA handles one 1024-element tile and finds its tensor with a binary
 // search over the table.
-#include "common.cuh"
+#include "sgd.cuh"
 
 namespace sgb {
 namespace {
@@ -48,34 +48,17 @@ __device__ __forceinline__ int find_tensor(const Table<N>& t, unsigned tile) {
   return lo;
 }
 
-struct SgdArgs {
-  float lr, mom, damp, decay, grad_scale;
-  int use_momentum, nesterov, use_decay, use_scale;
-};
-
-__device__ __forceinline__ void sgd_one(float& p, float g, float& m, const SgdArgs& a) {
-  // the reference's chain, one rounding per BLAS-1 step (python/singa/opt.py):
-  //   g *= 1/world ; g += decay*p ; m = m*mom ; m += (1-damp)*g ; p += -lr*m
-  if (a.use_scale) g = g * a.grad_scale;
-  if (a.use_decay) g = fmaf(a.decay, p, g);
-  float step = g;
-  if (a.use_momentum) {
-    float b = m * a.mom;
-    b = fmaf(1.0f - a.damp, g, b);
-    m = b;
-    step = a.nesterov ? fmaf(a.mom, b, g) : b;
-  }
-  p = fmaf(0.0f - a.lr, step, p);
-}
-
-template <int N>
+// ROUND: the gradient is rounded to fp16 and widened again on the way, and written
+// back: what a one-rank exchange in half precision does to it.  One pass over p, g
+// and m (24 B/element) instead of one over g and one over all three (28).
+template <int N, bool ROUND>
 __global__ void __launch_bounds__(kBlock)
 sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
   const int k = find_tensor(t, blockIdx.x);
   const size_t n = t.n[k];
   const size_t base = static_cast<size_t>(blockIdx.x - t.first_tile[k]) * kTile;
   float* p = static_cast<float*>(t.a[k]);
-  const float* g = static_cast<const float*>(t.b[k]);
+  float* g = static_cast<float*>(t.b[k]);
   float* m = static_cast<float*>(t.c[k]);
   const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                      (a.use_momentum ? reinterpret_cast<uintptr_t>(m) : 0)) & 15u) == 0;
@@ -91,14 +74,20 @@ sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
     vg.u = ld128(g + i);
     if (a.use_momentum) vm.u = ld128(m + i);
     release_dependents();
+    if (ROUND) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) vg.f[j] = __half2float(__float2half_rn(vg.f[j]));
+      st128(g + i, vg.u);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) sgd_one(vp.f[j], vg.f[j], vm.f[j], a);
     st128(p + i, vp.u);
     if (a.use_momentum) st128(m + i, vm.u);
   } else {
     for (size_t j = i; j < n && j < i + 4; ++j) {
-      float pv = p[j], mv = a.use_momentum ? m[j] : 0.f;
-      sgd_one(pv, g[j], mv, a);
+      float pv = p[j], gv = g[j], mv = a.use_momentum ? m[j] : 0.f;
+      if (ROUND) g[j] = gv = __half2float(__float2half_rn(gv));
+      sgd_one(pv, gv, mv, a);
       p[j] = pv;
       if (a.use_momentum) m[j] = mv;
     }
@@ -268,7 +257,7 @@ int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t coun
 }
 
 // One launch for as many tensors as the table holds.
-template <int N>
+template <int N, bool ROUND>
 int sgd_list(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
              const SgdArgs& a, cudaStream_t s) {
   const bool use_m = a.use_momentum;
@@ -298,13 +287,25 @@ int sgd_list(void* const* params, void* const* grads, void* const* moments, cons
     }
     if (cnt == 0) continue;
     const unsigned tiles = fill_table<N>(t, nullptr, pa, pb, pc, ns, 0, cnt, 0);
-    const int st = launch_ex(sgd_multi_kernel<N>, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, a);
+    const int st = launch_ex(sgd_multi_kernel<N, ROUND>, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, a);
     if (st != SGB_OK) return st;
   }
   return launch_status();
 }
 
+template <bool ROUND>
+int sgd_any(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
+            const SgdArgs& a, cudaStream_t s) {
+  return count <= kSmallTable ? sgd_list<kSmallTable, ROUND>(params, grads, moments, sizes, count, a, s)
+                              : sgd_list<kLargeTable, ROUND>(params, grads, moments, sizes, count, a, s);
+}
+
 }  // namespace
+
+int sgd_round_f16_multi(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
+                        const SgdArgs& a, cudaStream_t s) {
+  return sgd_any<true>(params, grads, moments, sizes, count, a, s);
+}
 
 int round_f16_multi(void* const* tensors, const size_t* sizes, size_t count, cudaStream_t s) {
   return pack_common(kRoundF16, tensors, sizes, count, nullptr, 0, 1.f, 0, s);
@@ -322,14 +323,10 @@ int sgb_sgd_update_multi_f32(void* const* params, void* const* grads, void* cons
                              void* stream) {
   if (count == 0) return SGB_OK;
   if (!params || !grads || !sizes) return SGB_ERR_NULL;
-  const int use_m = momentum != 0.0f;
-  if (use_m && !moments) return SGB_ERR_NULL;
-  if (nesterov && (!use_m || dampening != 0.0f)) return SGB_ERR_UNSUPPORTED;
-  SgdArgs a{lr, momentum, dampening, weight_decay, grad_scale, use_m, nesterov != 0,
-            weight_decay != 0.0f, grad_scale != 1.0f};
-  cudaStream_t s = as_stream(stream);
-  return count <= kSmallTable ? sgd_list<kSmallTable>(params, grads, moments, sizes, count, a, s)
-                              : sgd_list<kLargeTable>(params, grads, moments, sizes, count, a, s);
+  SgdArgs a;
+  const int st = sgd_args(&a, moments, lr, momentum, dampening, weight_decay, nesterov, grad_scale);
+  if (st != SGB_OK) return st;
+  return sgd_any<false>(params, grads, moments, sizes, count, a, as_stream(stream));
 }
 
 int sgb_sgd_update_f32(float* param, const float* grad, float* moment, size_t n, float lr,

@@ -30,6 +30,9 @@
 #include <cmath>
 #include <vector>
 
+#include <type_traits>
+
+#include "sgd.cuh"
 #include "sparse.cuh"
 
 namespace cg = cooperative_groups;
@@ -1208,6 +1211,13 @@ struct DenseArgs {
   size_t off[kDenseTargets + 1];   // first element of each target tensor; off[targets] == last
   float* ptr[kDenseTargets];
 };
+// Parameter and momentum of each target, for the form that ends in the update.
+struct DenseUpdate {
+  SgdArgs sgd;
+  float* p[kDenseTargets];
+  float* m[kDenseTargets];
+};
+struct NoUpdate {};
 
 // A position at most `slack` before the first whose index is >= want (1-based,
 // ascending): one warp, 32-ary.  The last rounds of a search cost as much as the
@@ -1230,6 +1240,44 @@ __device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned co
   return lo;
 }
 
+// g = src (in shared memory, at the same offset modulo 16 bytes as `at` in the tile),
+// and the update of p and m with it; by all threads of the CTA.
+__device__ __forceinline__ void update_run(const SgdArgs& a, float* p, float* g, float* m, const float* src, int len) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
+                        static_cast<uintptr_t>(__cvta_generic_to_shared(src));
+  const int nv = (all & 15u) == 0 ? len >> 2 : 0;
+  constexpr int kVecs = 2;                             // loads of two vectors in flight
+  for (int v0 = threadIdx.x; v0 < nv; v0 += kVecs * kBlock) {
+    Vec4f vp[kVecs], vm[kVecs];
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      if (v0 + k * kBlock < nv) {
+        vp[k].u = ld128(p + 4 * (v0 + k * kBlock));
+        if (a.use_momentum) vm[k].u = ld128(m + 4 * (v0 + k * kBlock));
+      }
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) {
+      const int i = 4 * (v0 + k * kBlock);
+      if (v0 + k * kBlock >= nv) break;
+      Vec4f vg;
+      vg.u = *reinterpret_cast<const uint4*>(src + i);
+      st128(g + i, vg.u);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sgd_one(vp[k].f[j], vg.f[j], vm[k].f[j], a);
+      st128(p + i, vp[k].u);
+      if (a.use_momentum) st128(m + i, vm[k].u);
+    }
+  }
+  for (int i = 4 * nv + threadIdx.x; i < len; i += kBlock) {
+    float pv = p[i], mv = a.use_momentum ? m[i] : 0.f;
+    const float gv = src[i];
+    g[i] = gv;
+    sgd_one(pv, gv, mv, a);
+    p[i] = pv;
+    if (a.use_momentum) m[i] = mv;
+  }
+}
+
 // Entries pass through windows of 1024, four per thread, indices and values
 // fetched together: with 256 at a time a tile of a dense payload was a chain of
 // three to four round trips.  A single rank's window stays in registers over the
@@ -1237,10 +1285,15 @@ __device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned co
 // 5.4 us each; 2.56e7 at once: 31.4 -> 24.9 us with the window, the binary
 // search for the first target and all 8 CTAs of an SM resident; 1e8 elements,
 // 1 % sent: 81.4 -> 80.0 us.
-template <bool ALONE>
-__global__ void __launch_bounds__(kBlock, 8)
-dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta) {
+//
+// Update: the tile's parameters and momentum are updated with it on the way, so
+// that the dense gradient is not read back (a pass of 1e8 elements, 1 % sent:
+// 652 -> 644 us; of 3.6e6 62 -> 56, of 4.4e5 34 -> 30).
+template <bool ALONE, typename Update>
+__global__ void __launch_bounds__(kBlock, std::is_same_v<Update, NoUpdate> ? 8 : 5)
+dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta, const __grid_constant__ Update u) {
   constexpr unsigned kPer = 4, kWindow = kPer * kBlock;
+  constexpr bool kUpdate = std::is_same_v<Update, DenseUpdate>;
   __shared__ __align__(16) float out[kDenseTile];
   __shared__ unsigned cursor[kMaxDenseRanks], count[kMaxDenseRanks];
   dependency_wait();
@@ -1306,6 +1359,9 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
       const float* src = out + (at - base);
       const int len = static_cast<int>(seg_end - at);
       if (!a.ptr[target]) {                            // a gap between buckets
+      } else if constexpr (kUpdate) {
+        const size_t in = at - a.off[target];
+        update_run(u.sgd, u.p[target] + in, dst, u.sgd.use_momentum ? u.m[target] + in : nullptr, src, len);
       } else if (((reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>((at - base) * 4)) & 15u) == 0) {
         const int nv = len >> 2;
         for (int v = threadIdx.x; v < nv; v += kBlock)
@@ -1511,21 +1567,28 @@ int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float th
 }
 
 int sparse_dense_buckets(const int* payload, const int* nnz_dev, const SparseBucket* buckets, size_t count,
-                         cudaStream_t s) {
-  std::vector<float*> tensors;
+                         cudaStream_t s, const SparseUpdate* update) {
+  std::vector<float*> tensors, params, moments;
   std::vector<size_t> sizes;
   const int none[1] = {0};
+  size_t at = 0;
   for (size_t k = 0; k < count; ++k) {
     size_t n = 0;
-    for (size_t t = 0; t < buckets[k].count; ++t) {
+    for (size_t t = 0; t < buckets[k].count; ++t, ++at) {
       tensors.push_back(buckets[k].tensors[t]);
       sizes.push_back(buckets[k].sizes[t]);
+      if (update) params.push_back(update->params[at]);
+      if (update) moments.push_back(update->moments ? update->moments[at] : nullptr);
       n += buckets[k].sizes[t];
     }
     tensors.push_back(nullptr);                        // the gap up to the next tile
+    params.push_back(nullptr);
+    moments.push_back(nullptr);
     sizes.push_back((kTile - n % kTile) % kTile);
   }
-  return sparse_dense_sum(payload, 0, 0, none, nnz_dev, 1, tensors.data(), sizes.data(), tensors.size(), s);
+  const SparseUpdate joint{update ? update->sgd : nullptr, params.data(), moments.data()};
+  return sparse_dense_sum(payload, 0, 0, none, nnz_dev, 1, tensors.data(), sizes.data(), tensors.size(), s,
+                          update ? &joint : nullptr);
 }
 
 bool sparse_selects_from(float* const* tensors, const size_t* sizes, size_t count, const float* acc) {
@@ -1557,8 +1620,12 @@ int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float*
 }
 
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
-                     int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s) {
+                     int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s,
+                     const SparseUpdate* update) {
   DenseArgs a;
+  DenseUpdate u;
+  if (update && world != 1) return SGB_ERR_UNSUPPORTED;
+  if (update) u.sgd = *update->sgd;
   if (world < 1 || world > kMaxDenseRanks) return SGB_ERR_UNSUPPORTED;
   a.payload = payload;
   a.stride = stride;
@@ -1576,8 +1643,16 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
     while (k < ntensors && a.targets < kDenseTargets) {
       if (sizes[k]) {
         // tensors that lie back to back are one target
-        if (a.targets && a.ptr[a.targets - 1] && a.ptr[a.targets - 1] + (at - a.off[a.targets - 1]) == tensors[k]) {
-        } else {
+        const int last = a.targets - 1;
+        const size_t run = a.targets ? at - a.off[last] : 0;
+        const bool joined = a.targets && a.ptr[last] && a.ptr[last] + run == tensors[k] &&
+                            (!update || (u.p[last] + run == update->params[k] &&
+                                         (!u.sgd.use_momentum || u.m[last] + run == update->moments[k])));
+        if (!joined) {
+          if (update) {
+            u.p[a.targets] = update->params[k];
+            u.m[a.targets] = u.sgd.use_momentum ? update->moments[k] : nullptr;
+          }
           a.off[a.targets] = at;
           a.ptr[a.targets++] = tensors[k];
         }
@@ -1589,9 +1664,12 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
     a.last = at;
     a.off[a.targets] = at;
     const size_t tiles = ceil_div(a.last - a.first, kDenseTile);
-    const unsigned per = static_cast<unsigned>(ceil_div(tiles, static_cast<size_t>(sm_count()) * 8));
-    const int st = launch_ex(world == 1 ? dense_from_payloads_kernel<true> : dense_from_payloads_kernel<false>, dim3(static_cast<unsigned>(ceil_div(tiles, per))),
-                             dim3(kBlock), 0, s, 0, true, a, per);
+    const unsigned per = static_cast<unsigned>(ceil_div(tiles, static_cast<size_t>(sm_count()) * (update ? 5 : 8)));
+    const dim3 grid(static_cast<unsigned>(ceil_div(tiles, per)));
+    const int st = update ? launch_ex(dense_from_payloads_kernel<true, DenseUpdate>, grid, dim3(kBlock), 0, s, 0, true, a, per, u)
+                          : launch_ex(world == 1 ? dense_from_payloads_kernel<true, NoUpdate>
+                                                 : dense_from_payloads_kernel<false, NoUpdate>,
+                                      grid, dim3(kBlock), 0, s, 0, true, a, per, NoUpdate{});
     if (st != SGB_OK) return st;
   }
   return launch_status();

@@ -1,6 +1,6 @@
 // Internal interface of the sparsifiers, used by the communicator.
 #pragma once
-#include "common.cuh"
+#include "sgd.cuh"
 
 namespace sgb {
 
@@ -37,9 +37,16 @@ constexpr size_t kMaxBucketSpan = size_t{1} << 25;
 size_t sparse_buckets_span(const SparseBucket* buckets, size_t count);
 int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float thr, int* payload, int* nnz_dev, void* ws,
                              size_t ws_bytes, cudaStream_t s);
+// The SGD update that a dense sum ends in: parameters (and momentum buffers) of the
+// tensors, in their order.
+struct SparseUpdate {
+  const SgdArgs* sgd;
+  float* const* params;
+  float* const* moments;   // null without momentum
+};
 // The dense gradients of that payload, back into the buckets' tensors.
 int sparse_dense_buckets(const int* payload, const int* nnz_dev, const SparseBucket* buckets, size_t count,
-                         cudaStream_t s);
+                         cudaStream_t s, const SparseUpdate* update = nullptr);
 
 // Top-K selection (see sgb_sparse_topk_f32) from a tensor list.
 int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float* acc, size_t k, int mode, int* idx_out,
@@ -49,9 +56,10 @@ int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float*
 // stride words) into the tensors, which cover the index space in list order.
 // Values start val_off words behind the indices, or, with val_off == 0, right
 // behind the rank's own count.  counts: host array, or counts_dev on the device
-// (then clamped to val_off, or to the size of the index space).
+// (then clamped to val_off, or to the size of the index space).  update: one rank only.
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
-                     int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s);
+                     int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s,
+                     const SparseUpdate* update = nullptr);
 
 // Rounds the tensors to fp16 and back, in place (multi_tensor.cu).
 int round_f16_multi(void* const* tensors, const size_t* sizes, size_t count, cudaStream_t s);

@@ -690,6 +690,102 @@ PyObject* py_comm_sparsify_buckets(Args a, Py_ssize_t) {  // (communicator, buck
   });
   return PyBool_FromLong(st == SGB_OK);
 }
+// Tensors that a kernel may take as they are; false otherwise, and the separate
+// calls give their own answer.
+bool plain_f32(PyObject* seq, const TensorList& l) {
+  const Py_ssize_t n = PySequence_Size(seq);
+  if (n < 0) throw PyError{};
+  if (static_cast<size_t>(n) != l.n()) return false;
+  for (Py_ssize_t k = 0; k < n; ++k) {
+    PyObject* item = PyList_Check(seq) ? PyList_GET_ITEM(seq, k) : PyTuple_Check(seq) ? PyTuple_GET_ITEM(seq, k) : nullptr;
+    if (!item || !THPVariable_Check(item)) return false;
+    const Tensor& t = THPVariable_Unpack(item);
+    if (t.scalar_type() != at::kFloat || !t.is_cuda() || !t.is_contiguous()) return false;
+  }
+  return true;
+}
+struct Hyper {                         // lr, momentum, dampening, weight decay, nesterov, grad scale
+  float lr, mom, damp, decay, scale;
+  int nesterov;
+  explicit Hyper(PyObject* t) {
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 6) fail(PyExc_TypeError, "six hyper-parameters are expected");
+    auto v = [&](int k) { return static_cast<float>(real(PyTuple_GET_ITEM(t, k))); };
+    lr = v(0);
+    mom = v(1);
+    damp = v(2);
+    decay = v(3);
+    nesterov = truth(PyTuple_GET_ITEM(t, 4));
+    scale = v(5);
+  }
+};
+// (communicator, params, grads, moments | None, threshold, hyper) -> done?
+PyObject* py_comm_update_half(Args a, Py_ssize_t) {
+  const TensorList p(a[1], false), g(a[2], false);
+  const Hyper h(a[5]);
+  std::unique_ptr<TensorList> m;
+  if (h.mom != 0.0f) m = std::make_unique<TensorList>(a[3], false);
+  bool ok = plain_f32(a[1], p) && plain_f32(a[2], g) && p.sizes == g.sizes && p.n() != 0;
+  ok = ok && (!m || (plain_f32(a[3], *m) && m->sizes == p.sizes));
+  if (!ok) Py_RETURN_FALSE;
+  const double threshold = real(a[4]);
+  size_t largest = 0, held = 0;        // of the buckets that a call each would make
+  for (const size_t n : g.sizes) {
+    if (static_cast<double>(n) > threshold) {
+      largest = std::max(largest, n);
+      continue;
+    }
+    held += n;
+    largest = std::max(largest, held);
+    if (static_cast<double>(held) > threshold) held = 0;
+  }
+  int st = SGB_OK;
+  issue("sgb_comm_update_half", [&] {
+    st = sgb_comm_update_half(comm(a[0]), p.ptrs.data(), g.ptrs.data(), m ? m->ptrs.data() : nullptr, g.sizes.data(), g.n(),
+                              largest, h.lr, h.mom, h.damp, h.decay, h.nesterov, h.scale, stream());
+    return st == SGB_ERR_UNSUPPORTED ? SGB_OK : st;
+  });
+  return PyBool_FromLong(st == SGB_OK);
+}
+// (communicator, buckets, residuals, params, moments | None, spars, topk, hyper) -> done?
+PyObject* py_comm_sparse_update(Args a, Py_ssize_t) {
+  std::vector<void*> ptrs;
+  std::vector<size_t> sizes, counts;
+  const Py_ssize_t n = PySequence_Size(a[1]);
+  if (n < 0) throw PyError{};
+  for (Py_ssize_t k = 0; k < n; ++k) {
+    const std::unique_ptr<PyObject, void (*)(PyObject*)> bucket(PySequence_GetItem(a[1], k),
+                                                                [](PyObject* p) { Py_XDECREF(p); });
+    if (!bucket) throw PyError{};
+    const TensorList l(bucket.get(), false);
+    if (!plain_f32(bucket.get(), l)) Py_RETURN_FALSE;
+    ptrs.insert(ptrs.end(), l.ptrs.begin(), l.ptrs.end());
+    sizes.insert(sizes.end(), l.sizes.begin(), l.sizes.end());
+    counts.push_back(l.n());
+  }
+  const TensorList acc(a[2], false), p(a[3], false);
+  const float spars = static_cast<float>(real(a[5]));
+  const int topk = truth(a[6]);
+  const Hyper h(a[7]);
+  std::unique_ptr<TensorList> m;
+  if (h.mom != 0.0f) m = std::make_unique<TensorList>(a[4], false);
+  bool ok = !counts.empty() && acc.n() == counts.size() && plain_f32(a[2], acc) && plain_f32(a[3], p) && p.sizes == sizes;
+  ok = ok && (!m || (plain_f32(a[4], *m) && m->sizes == sizes));
+  for (size_t k = 0, at = 0; ok && k < counts.size(); ++k) {
+    size_t total = 0;
+    for (size_t i = 0; i < counts[k]; ++i) total += sizes[at++];
+    ok = acc.sizes[k] == total;
+  }
+  if (!ok) Py_RETURN_FALSE;
+  int st = SGB_OK;
+  issue("sgb_comm_sparse_update", [&] {
+    st = sgb_comm_sparse_update(comm(a[0]), ptrs.data(), sizes.data(), counts.data(),
+                                reinterpret_cast<float* const*>(acc.ptrs.data()), counts.size(), spars, topk,
+                                p.ptrs.data(), m ? m->ptrs.data() : nullptr, h.lr, h.mom, h.damp, h.decay, h.nesterov,
+                                h.scale, stream());
+    return st == SGB_ERR_UNSUPPORTED ? SGB_OK : st;
+  });
+  return PyBool_FromLong(st == SGB_OK);
+}
 PyObject* py_comm_sparsify_end(Args a, Py_ssize_t) {
   ISSUE(sgb_comm_sparsification_end, comm(a[0]), stream());
   Py_RETURN_NONE;
@@ -1089,7 +1185,7 @@ PyMethodDef kMethods[] = {
     METHOD(bn_backward, 9), METHOD(bn_add_relu_backward, 10), METHOD(pool_forward, 5), METHOD(pool_backward, 5),
     METHOD(pool_forward_argmax, 4), METHOD(pool_backward_argmax, 3), METHOD(sgd_multi, 9), METHOD(pack, 3), METHOD(unpack, 4),
     METHOD(comm_synch, 2), METHOD(comm_synch_half, 2), METHOD(comm_fused_synch, 3), METHOD(comm_fused_synch_half, 3),
-    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5), METHOD(program_captures, 1),
+    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_update_half, 6), METHOD(comm_sparse_update, 8), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5), METHOD(program_captures, 1),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

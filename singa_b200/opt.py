@@ -62,14 +62,17 @@ class SGD(object):
                                                        param_grad.shape)
         self.apply_many([param_name], [param_value], [param_grad], grad_scale)
 
+    def _moments_of(self, names, params):
+        if self.momentum == 0:
+            return None
+        have = self.moments
+        try:
+            return [have[n] for n in names]
+        except KeyError:                                  # first step of a parameter
+            return [self._moment(n, p) for n, p in zip(names, params)]
+
     def apply_many(self, names, params, grads, grad_scale=1.0):
-        moments = None
-        if self.momentum != 0:
-            have = self.moments
-            try:
-                moments = [have[n] for n in names]
-            except KeyError:                              # first step of a parameter
-                moments = [self._moment(n, p) for n, p in zip(names, params)]
+        moments = self._moments_of(names, params)
         sw.sgd_update_multi(params, grads, moments, self.lr, self.momentum, self.dampening,
                             self.weight_decay, self.nesterov, grad_scale)
 
@@ -88,6 +91,13 @@ _WHOLE = {
 }
 
 
+# the communicator's method that does an exchange and the update behind it
+# (and what else of the communicator it stands for)
+_WITH_UPDATE = {"half": ("updateHalf", ("syncDense", "wait")),
+                "sparse": ("sparseUpdate", ("beginSparsification", "endSparsification", "sparsifyBuckets", "wait"))}
+_LISTS = (list, tuple, type(iter([])), type(iter(())))
+
+
 @functools.lru_cache(maxsize=64)
 def _inverse(world_size):
     """1 / world_size as fp32 forms it."""
@@ -103,6 +113,17 @@ def _stands(own, kind, exchange):
     owner = next((k for k in kind.__mro__ if name in vars(k)), None)
     return owner is not None and all(getattr(own, f) is getattr(DistOpt, f) for f in forwards) and \
         all(getattr(kind, f, None) is getattr(owner, f, None) for f in calls)
+
+
+@functools.lru_cache(maxsize=64)
+def _stands_with_update(own, kind, exchange):
+    """Whether the method of communicators of class `kind` that also updates does what
+    the exchange, wait() and the update of `own` would do one after the other."""
+    def owner(name):
+        return next((k for k in kind.__mro__ if name in vars(k)), None)
+    name, calls = _WITH_UPDATE[exchange]
+    return owner(name) is not None and all(owner(x) in (None, owner(name)) for x in calls) and \
+        all(getattr(own, f) is getattr(DistOpt, f) for f in ("wait", "_update_all", "_sync_dense"))
 
 
 class DistOpt(object):
@@ -163,6 +184,24 @@ class DistOpt(object):
             return None
         return getattr(c, name)
 
+    def _with_update(self, exchange, grad_stream):
+        """The communicator's method that does the whole `exchange` of gradients that
+        exist already and the update behind it (_WITH_UPDATE), on one rank.  None
+        where it has none, or where something that it stands for has been replaced."""
+        c, opt = self.communicator, self.opt
+        if self.world_size != 1 or type(grad_stream) not in _LISTS or type(opt) is not SGD or \
+                not _stands_with_update(type(self), type(c), exchange) or self._whole(exchange) is None:
+            return None
+        (name, calls), mine, theirs = _WITH_UPDATE[exchange], self.__dict__, c.__dict__
+        if "apply_many" in opt.__dict__ or "wait" in mine or "_update_all" in mine or "_sync_dense" in mine or \
+                name in theirs or any(x in theirs for x in calls):
+            return None
+        return getattr(c, name)
+
+    def _hyper(self):
+        o = self.opt
+        return o.lr, o.momentum, o.dampening, o.weight_decay, o.nesterov, _inverse(self.world_size)
+
     def _update_all(self, plist):
         scale = _inverse(self.world_size)
         names, params, grads = plist
@@ -205,6 +244,15 @@ class DistOpt(object):
     def backward_and_update_half(self, grad_stream, threshold=2097152, clipping=False,
                                  clip_Value=100):
         """opt.py:867-920: fp16 transport of fp32 gradients."""
+        update = None if clipping else self._with_update("half", grad_stream)
+        if update is not None:
+            grad_stream = list(grad_stream)
+            if grad_stream and all(len(t) == 3 for t in grad_stream):
+                names, params, grads = map(list, zip(*grad_stream))
+                if update(params, grads, self.opt._moments_of(names, params), threshold, self._hyper()):
+                    self.opt.step()
+                    return
+
         def clipped(stream):
             for name, p, g in stream:
                 sw.Clamp(g, -clip_Value, clip_Value, out=g)
@@ -313,18 +361,29 @@ class DistOpt(object):
             else:
                 self.fused_sparsification(tensors, res, spars, topK)
 
-        # On one rank, gradients that all exist already go through one selection.
-        joint = None
-        if (corr and not topK and self.world_size == 1 and
-                type(grad_stream) in (list, tuple, type(iter([])), type(iter(())))):
-            joint = self._whole("joint")
+        # On one rank, gradients that all exist already go through one selection,
+        # and are updated as they are written.
+        joint = update = None
+        if corr and self.world_size == 1 and type(grad_stream) in _LISTS:
+            joint = None if topK else self._whole("joint")
+            update = self._with_update("sparse", grad_stream)
+        updated = False
         try:
-            if joint is not None:
+            if joint is not None or update is not None:
                 ready = []
                 for tensors, n, single in buckets():
                     k += 1
                     ready.append((tensors, residual(n, tensors[0]), single))
-                if not ready or not joint([b[0] for b in ready], [b[1] for b in ready], spars):
+                lists, residuals = [b[0] for b in ready], [b[1] for b in ready]
+                if update is not None and ready:
+                    # in bucket order: a large tensor's bucket may come before an open one's
+                    place = {id(g): i for i, g in enumerate(grads)}
+                    order = [place[id(g)] for b in lists for g in b]
+                    moments = self.opt._moments_of(names, params)
+                    updated = len(place) == len(grads) and update(
+                        lists, residuals, [params[i] for i in order],
+                        None if moments is None else [moments[i] for i in order], spars, topK, self._hyper())
+                if not updated and (joint is None or not ready or not joint(lists, residuals, spars)):
                     begin = self._whole("sparse")
                     for b in ready:
                         exchange(*b)
@@ -341,4 +400,7 @@ class DistOpt(object):
                 self.communicator.endSparsification()
             self.wait()
         self.sparsInit = True
-        self._update_all((names, params, grads))
+        if updated:
+            self.opt.step()
+        else:
+            self._update_all((names, params, grads))
