@@ -868,13 +868,14 @@ static int sparse_end(sgb_comm* c, void* compute_stream) {
 // (c1 has not joined a capture of the compute stream yet).  Outgrown buffers are
 // kept until the communicator goes: their addresses may sit in a captured graph
 // or in queued work.  Doubling keeps their sum below twice the size of the last one.
-static int joint_reserve(sgb_comm* c, size_t span, cudaStream_t compute) {
-  if (span <= c->joint_elems) return SGB_OK;
+static int joint_reserve(sgb_comm* c, size_t span, cudaStream_t compute, size_t ws_least = 0) {
+  if (span <= c->joint_elems && ws_least <= c->joint_ws_bytes) return SGB_OK;
   if (capturing(compute) || capturing(c->c1)) return SGB_ERR_UNSUPPORTED;
   size_t elems = 2 * c->joint_elems;
   if (elems > sgb::kMaxBucketSpan) elems = sgb::kMaxBucketSpan;
   if (elems < span) elems = span;
-  const size_t ws_bytes = sgb_sparse_workspace_bytes(elems);
+  size_t ws_bytes = sgb_sparse_workspace_bytes(elems);
+  if (ws_bytes < ws_least) ws_bytes = ws_least;
   int* pay = nullptr;
   void* ws = nullptr;
   if (!c->joint_nnz) CU(cudaMalloc(&c->joint_nnz, sizeof(int)));
@@ -921,7 +922,7 @@ static int threshold_buckets(sgb_comm* c, const std::vector<sgb::SparseBucket>& 
     sgb::SparseUpdate part{};
     if (update)
       part = {update->sgd, update->params + tensor, update->moments ? update->moments + tensor : nullptr};
-    OK(sgb::sparse_dense_buckets(c->joint_pay, c->joint_nnz, list.data() + k, end - k, c->c1, update ? &part : nullptr));
+    OK(sgb::sparse_dense_buckets(c->joint_pay, 0, c->joint_nnz, list.data() + k, end - k, c->c1, update ? &part : nullptr));
     for (; k < end; ++k) tensor += list[k].count;
   }
   return SGB_OK;
@@ -974,11 +975,29 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
   // 2.56e7 in 11 buckets 180.4 -> 181.4).
   if (!topk && elements > 16000000) return SGB_ERR_UNSUPPORTED;
   if (!topk) return threshold_buckets(c, list, spars, &update, compute);
-  // one bucket; several would follow one another on c1, without the overlap that
-  // separate calls have (25 buckets: 547 us a pass, 591 this way)
-  if (list.size() != 1) return SGB_ERR_UNSUPPORTED;
   for (const sgb::SparseBucket& b : list)
     if (!sgb::sparse_selects_from(b.tensors, b.sizes, b.count, b.acc)) return SGB_ERR_UNSUPPORTED;
+  // all buckets by one launch where they are few and small enough
+  std::vector<size_t> ks;
+  size_t span = 0;
+  for (const sgb::SparseBucket& b : list) {
+    const size_t n = total_of(b.sizes, b.count);
+    ks.push_back(static_cast<size_t>(sgb_topk_count(spars, n)));
+    span += n + 512;
+  }
+  const size_t ws_bytes = sgb::sparse_topk_buckets_bytes(list.data(), ks.data(), list.size(), c->topk_mode);
+  if (ws_bytes) {
+    OK(joint_reserve(c, span, compute, ws_bytes));
+    OK(emit(c, plan_call(c, sgb::order::kStageCopy).pre, compute));
+    Phase ph(c, "Dist_c1c2_fusedSparsification", sgb::order::kStreamC1);
+    int sent = 0;
+    OK(sgb::sparse_topk_buckets(list.data(), ks.data(), list.size(), c->topk_mode, c->joint_pay, &sent, c->joint_ws,
+                                c->joint_ws_bytes, c->c1));
+    return sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data(), list.size(), c->c1, &update);
+  }
+  // one bucket; several would follow one another on c1, without the overlap that
+  // separate calls have (72 buckets: 620 us a pass, 867 this way)
+  if (list.size() != 1) return SGB_ERR_UNSUPPORTED;
   if (!c->dropped_dev && (capturing(compute) || capturing(c->c1))) return SGB_ERR_UNSUPPORTED;
   OK(sparse_init(c));
   const sgb::order::Step p = plan_call(c, sgb::order::kSparseUpdate);

@@ -54,11 +54,12 @@ constexpr int kMaxGrid = 1024;
 struct Counters {        // zeroed before a call that uses them
   unsigned ticket[4];    // chunks drawn so far, one counter per pass
   unsigned max_key;      // largest key of pass 0
-  unsigned pad[3];
+  unsigned arrived;      // at the barriers of a part of the grid
+  unsigned pad[2];
   unsigned hist0[kBins1], hist1[kBins23], hist2[kBins23], sample[kBins1];
 };
 
-inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
+__host__ __device__ inline size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 inline size_t tiles_of(size_t n) { return ceil_div(n, kTile); }
 inline size_t max_grid() {
   const size_t g = static_cast<size_t>(sm_count()) * kCtasPerSm;
@@ -72,9 +73,8 @@ struct Work {
   unsigned capacity;     // list entries per warp and chunk
   bool dynamic;          // chunks are drawn from the ticket counter
 };
-inline Work work_for(size_t n) {
+inline Work work_for(size_t n, size_t g = max_grid()) {
   const size_t tiles = tiles_of(n);
-  const size_t g = max_grid();
   Work w;
   w.run = tiles > 4 * kWarps * g ? 4 : 1;
   w.capacity = w.run == 4 ? 352 : 128;
@@ -93,11 +93,13 @@ struct Workspace {
   int* list_idx;         // chunks * kWarps segments of `capacity` entries
   float* list_val;
 };
-inline size_t workspace_bytes_exact(size_t n) {
-  const Work w = work_for(n);
+inline size_t lists_bytes(const Work& w) {
   const size_t runs = static_cast<size_t>(w.chunks) * kWarps;
-  return align256(sizeof(Counters)) + 2 * align256(w.chunks * sizeof(unsigned)) + 2 * align256(runs * sizeof(unsigned)) +
+  return 2 * align256(w.chunks * sizeof(unsigned)) + 2 * align256(runs * sizeof(unsigned)) +
          2 * align256(runs * w.capacity * sizeof(int));
+}
+inline size_t workspace_bytes_exact(size_t n) {
+  return align256(sizeof(Counters)) + lists_bytes(work_for(n));
 }
 // Monotonic in n (a workspace for n serves any smaller call): where the cut
 // changes from one tile to four, the shorter runs need the larger lists.
@@ -107,11 +109,12 @@ inline size_t workspace_bytes(size_t n) {
   if (n > turn && workspace_bytes_exact(turn) > b) b = workspace_bytes_exact(turn);
   return b;
 }
-inline Workspace carve(void* ws, const Work& k) {
-  char* p = static_cast<char*>(ws);
+// The counters at `counters`, the rest from `lists` on.
+__host__ __device__ inline Workspace carve_at(char* counters, char* lists, const Work& k) {
+  char* p = lists;
   const size_t runs = static_cast<size_t>(k.chunks) * kWarps;
   Workspace w;
-  w.counters = reinterpret_cast<Counters*>(p); p += align256(sizeof(Counters));
+  w.counters = reinterpret_cast<Counters*>(counters);
   w.chunk_a = reinterpret_cast<unsigned*>(p); p += align256(k.chunks * sizeof(unsigned));
   w.chunk_b = reinterpret_cast<unsigned*>(p); p += align256(k.chunks * sizeof(unsigned));
   w.run_meta = reinterpret_cast<unsigned*>(p); p += align256(runs * sizeof(unsigned));
@@ -120,7 +123,10 @@ inline Workspace carve(void* ws, const Work& k) {
   w.list_val = reinterpret_cast<float*>(p);
   return w;
 }
-
+inline Workspace carve(void* ws, const Work& k) {
+  char* p = static_cast<char*>(ws);
+  return carve_at(p, p + align256(sizeof(Counters)), k);
+}
 // ------------------------------------------------------------- tile helpers
 // Element order inside a tile: vector v = r * 32 + lane (round r), elements
 // 4v .. 4v+3.  Loads are fully coalesced; ranks below follow this order, which
@@ -174,6 +180,12 @@ struct Pieces {
   unsigned off[kPieces + 1];
   const float* ptr[kPieces];
 };
+// A part of such a list that lies elsewhere in the kernel's arguments.
+struct PieceView {
+  int count;
+  const unsigned* off;
+  const float* const* ptr;
+};
 struct NoPieces {};
 // Where a tile lies in the lists: searched for once per run of tiles, then
 // walked.  (A search is up to thirteen dependent loads ahead of the tile's own.)
@@ -182,7 +194,8 @@ struct Cursor {
 };
 __device__ __forceinline__ void seek(const NoPieces&, Cursor&, size_t) {}
 __device__ __forceinline__ void advance(const NoPieces&, Cursor&, size_t) {}
-__device__ __forceinline__ void seek(const Pieces& p, Cursor& c, size_t tile) {
+template <typename P>
+__device__ __forceinline__ void seek_piece(const P& p, Cursor& c, size_t tile) {
   const unsigned e0 = static_cast<unsigned>(tile * kTile);
   int lo = 0, hi = p.count - 1;
   while (lo < hi) {                                    // the same in all lanes
@@ -191,18 +204,24 @@ __device__ __forceinline__ void seek(const Pieces& p, Cursor& c, size_t tile) {
   }
   c.piece = lo;
 }
-__device__ __forceinline__ void advance(const Pieces& p, Cursor& c, size_t tile) {
+template <typename P>
+__device__ __forceinline__ void advance_piece(const P& p, Cursor& c, size_t tile) {
   const unsigned e0 = static_cast<unsigned>(tile * kTile);
   while (c.piece + 1 < p.count && p.off[c.piece + 1] <= e0) ++c.piece;
 }
+__device__ __forceinline__ void seek(const Pieces& p, Cursor& c, size_t tile) { seek_piece(p, c, tile); }
+__device__ __forceinline__ void advance(const Pieces& p, Cursor& c, size_t tile) { advance_piece(p, c, tile); }
+__device__ __forceinline__ void seek(const PieceView& p, Cursor& c, size_t tile) { seek_piece(p, c, tile); }
+__device__ __forceinline__ void advance(const PieceView& p, Cursor& c, size_t tile) { advance_piece(p, c, tile); }
 __device__ __forceinline__ void load_tile(const NoPieces&, const Cursor&, const float* g, const float* acc, size_t tile,
                                           size_t n, bool vec, float (&s)[kRounds][4]) {
   load_tile(g, acc, tile, n, vec, s);
 }
 // s = gradient + acc for one tile.  A tile inside one tensor is loaded as above,
 // one that crosses an end element by element.  acc is there and aligned.
-__device__ __forceinline__ void load_tile(const Pieces& p, const Cursor& c, const float*, const float* acc, size_t tile,
-                                          size_t n, bool, float (&s)[kRounds][4]) {
+template <typename P>
+__device__ __forceinline__ void load_pieces(const P& p, const Cursor& c, const float* acc, size_t tile, size_t n,
+                                            float (&s)[kRounds][4]) {
   const unsigned e0 = static_cast<unsigned>(tile * kTile), e1 = e0 + kTile;
   const int lo = c.piece;
   const float* base = p.ptr[lo] - p.off[lo];           // only used where it points into the tensor
@@ -223,6 +242,15 @@ __device__ __forceinline__ void load_tile(const Pieces& p, const Cursor& c, cons
       }
     }
   }
+}
+
+__device__ __forceinline__ void load_tile(const Pieces& p, const Cursor& c, const float*, const float* acc, size_t tile,
+                                          size_t n, bool, float (&s)[kRounds][4]) {
+  load_pieces(p, c, acc, tile, n, s);
+}
+__device__ __forceinline__ void load_tile(const PieceView& p, const Cursor& c, const float*, const float* acc, size_t tile,
+                                          size_t n, bool, float (&s)[kRounds][4]) {
+  load_pieces(p, c, acc, tile, n, s);
 }
 
 // Several buckets, each with its own residual, as one index space in which
@@ -371,11 +399,12 @@ __device__ __forceinline__ void run_tiles(const Work& k, unsigned chunk, size_t 
 // that what the warps hand to `after` in shared memory can be double-buffered.
 // Every CTA's first chunk is its own number; the counter hands out the rest.
 template <bool DESCENDING, typename Body, typename After>
-__device__ __forceinline__ void for_chunks(const Work& k, unsigned* ticket, unsigned* sm_next, Body body, After after) {
-  unsigned c = blockIdx.x, parity = 0;
+__device__ __forceinline__ void for_chunks(const Work& k, unsigned rank, unsigned* ticket, unsigned* sm_next, Body body,
+                                           After after) {
+  unsigned c = rank, parity = 0;
   while (c < k.chunks) {
-    unsigned next = c + gridDim.x;
-    if (k.dynamic && threadIdx.x == 0) next = gridDim.x + atomicAdd(ticket, 1u);
+    unsigned next = c + k.grid;
+    if (k.dynamic && threadIdx.x == 0) next = k.grid + atomicAdd(ticket, 1u);
     const unsigned chunk = DESCENDING ? k.chunks - 1 - c : c;
     body(chunk, parity);
     if (k.dynamic && threadIdx.x == 0) sm_next[parity] = next;
@@ -388,9 +417,9 @@ __device__ __forceinline__ void for_chunks(const Work& k, unsigned* ticket, unsi
 }
 // After a grid barrier the chunks are walked in contiguous shares: this CTA's
 // [first, last), and how much one or two counts per chunk add up to before it.
-__device__ __forceinline__ void my_chunks(const Work& k, unsigned& first, unsigned& last) {
-  first = static_cast<unsigned>(static_cast<unsigned long long>(k.chunks) * blockIdx.x / gridDim.x);
-  last = static_cast<unsigned>(static_cast<unsigned long long>(k.chunks) * (blockIdx.x + 1) / gridDim.x);
+__device__ __forceinline__ void my_chunks(const Work& k, unsigned rank, unsigned& first, unsigned& last) {
+  first = static_cast<unsigned>(static_cast<unsigned long long>(k.chunks) * rank / k.grid);
+  last = static_cast<unsigned>(static_cast<unsigned long long>(k.chunks) * (rank + 1) / k.grid);
 }
 struct Before {
   unsigned before, total;
@@ -438,7 +467,7 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
   __shared__ unsigned warp_counts[2][kWarps], next[2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for_chunks<false>(
-      a.work, a.ws.counters->ticket, next,
+      a.work, blockIdx.x, a.ws.counters->ticket, next,
       [&](unsigned chunk, unsigned parity) {
         size_t lo, hi;
         run_tiles(a.work, chunk, a.n, lo, hi);
@@ -502,7 +531,7 @@ thr_select_kernel(const ThrArgs a, const __grid_constant__ Source source) {
   cg::this_grid().sync();
 
   unsigned first, last;
-  my_chunks(a.work, first, last);
+  my_chunks(a.work, blockIdx.x, first, last);
   const Before b = counts_before(a.ws.chunk_a, a.work.chunks, first, sm);
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.nnz_dev = static_cast<int>(b.total);
   float* const val_out = a.val_out ? a.val_out : reinterpret_cast<float*>(a.idx_out) + (BOUNDED ? a.cap : b.total);
@@ -696,13 +725,15 @@ struct TopkArgs {
   int* idx_out;
   float* val_out;
   bool vec;
+  unsigned index_base;     // added to the indices that are sent
 };
 
 // s of one element.
 __device__ __forceinline__ float element(const NoPieces&, const float* g, const float* acc, size_t i) {
   return acc ? g[i] + acc[i] : g[i];
 }
-__device__ __forceinline__ float element(const Pieces& p, const float*, const float* acc, size_t i) {
+template <typename P>
+__device__ __forceinline__ float element(const P& p, const float*, const float* acc, size_t i) {
   int lo = 0, hi = p.count - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -778,16 +809,18 @@ __device__ __forceinline__ void list_keys(const float (&s)[kRounds][4], unsigned
 //   pass 2  the last digit, from the lists; then count and copy out.
 // HBM-bound: pass 0 moves 12 B/element, pass 1 over s another 4, of which the
 // sample (8 us) saves the most and four in five of the shared-memory atomics.
-template <int MODE, typename Source>
-__global__ void __launch_bounds__(kBlock, kCtasPerSm)
-topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
+//
+// `rank` of a.work.grid CTAs, which sync() brings together: the whole grid, or the
+// part of it that works on one of several buckets.
+template <int MODE, typename Source, typename Sync>
+__device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& source, const unsigned rank, Sync sync) {
   constexpr unsigned kSlots = 96;
   __shared__ unsigned sh[kBins1];
   __shared__ int slot_idx_all[kWarps][kSlots];
   __shared__ float slot_val_all[kWarps][kSlots];
   __shared__ uint2 sm2[kWarps];
   __shared__ unsigned sm[kWarps + 2], next[2];
-  cg::grid_group grid = cg::this_grid();
+  const unsigned ranks = a.work.grid;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* const slot_idx = slot_idx_all[warp];
   float* const slot_val = slot_val_all[warp];
@@ -803,8 +836,8 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   unsigned floor_bin = 0;                            // bins from here on are listed in pass 0; 0: none
   if (MODE == 0 && a.sample_target) {
     clear_bins<kBins1>(sh);
-    const unsigned warps = gridDim.x * kWarps;
-    const size_t e0 = n / warps * (blockIdx.x * kWarps + warp) + lane;   // n / warps >= 128: see the host's rule
+    const unsigned warps = ranks * kWarps;
+    const size_t e0 = n / warps * (rank * kWarps + warp) + lane;   // n / warps >= 128: see the host's rule
     float v[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) v[q] = element(source, a.g, a.acc, e0 + 32 * q);
@@ -814,7 +847,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
     for (int q = 0; q < 4; ++q) bin[q] = make_key<MODE>(v[q]) >> 20;
     tally4(sh, bin, take);
     flush_bins<kBins1>(sh, cnt->sample);
-    grid.sync();
+    sync();
     unsigned left = a.sample_target, b;
     pick_bin<kBins1>(cnt->sample, left, b, sm);
     // more than an eighth at or above the bound (ties, a crowded bin) would not fit the lists
@@ -826,7 +859,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   clear_bins<kBins1>(sh);
   unsigned top = 0;
   for_chunks<false>(
-      a.work, &cnt->ticket[0], next,
+      a.work, rank, &cnt->ticket[0], next,
       [&](unsigned chunk, unsigned) {
         size_t lo, hi;
         run_tiles(a.work, chunk, n, lo, hi);
@@ -878,7 +911,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
     for (int k = 1; k < kWarps; ++k) top = max(top, sm[k]);
     if (top) atomicMax(&cnt->max_key, top);
   }
-  grid.sync();
+  sync();
 
   unsigned remaining = a.k, bin;
   pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
@@ -887,7 +920,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
     // fewer than k keys at or above the bound: count the others as well
     clear_bins<kBins1>(sh);
     for_chunks<true>(
-        a.work, &cnt->ticket[2], next,
+        a.work, rank, &cnt->ticket[2], next,
         [&](unsigned chunk, unsigned) {
           size_t lo, hi;
           run_tiles(a.work, chunk, n, lo, hi);
@@ -910,7 +943,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
         },
         nothing);
     flush_bins<kBins1>(sh, cnt->hist0);
-    grid.sync();
+    sync();
     remaining = a.k;
     pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
   }
@@ -919,9 +952,9 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   if (max_key == 0) {
     // every key is 0 (small gradients under integer-truncated keys): the first
     // k elements are sent, and the whole grid shares the work
-    for (size_t i = blockIdx.x * static_cast<size_t>(kBlock) + threadIdx.x; i < a.k;
-         i += static_cast<size_t>(gridDim.x) * kBlock) {
-      a.idx_out[i] = static_cast<int>(i + 1);
+    for (size_t i = rank * static_cast<size_t>(kBlock) + threadIdx.x; i < a.k;
+         i += static_cast<size_t>(ranks) * kBlock) {
+      a.idx_out[i] = static_cast<int>(i + 1 + a.index_base);
       a.val_out[i] = __ldcg(sum + i);                // written by another CTA in pass 0
       if (a.acc) a.acc[i] = 0.0f;
     }
@@ -934,7 +967,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   // next run's count and first 64 entries are fetched ahead (they are inside
   // the segment whatever the count).
   unsigned first, last;
-  my_chunks(a.work, first, last);
+  my_chunks(a.work, rank, first, last);
   auto visit = [&](auto entry, auto tile_fn, auto done) {
     unsigned meta = 0;
     float v0 = 0.0f, v1 = 0.0f;
@@ -1006,7 +1039,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
   } else {
     // chunks in descending order: what pass 0 touched last is still in L2
     for_chunks<true>(
-        a.work, &cnt->ticket[1], next,
+        a.work, rank, &cnt->ticket[1], next,
         [&](unsigned chunk, unsigned) {
           size_t lo, hi;
           run_tiles(a.work, chunk, n, lo, hi);
@@ -1033,7 +1066,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
         nothing);
   }
   flush_bins<kBins23>(sh, cnt->hist1);
-  grid.sync();
+  sync();
   pick_bin<kBins23>(cnt->hist1, remaining, bin, sm);
   prefix |= bin << shift;
 
@@ -1062,7 +1095,7 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
           },
           no_done);
     flush_bins<kBins23>(sh, cnt->hist2);
-    grid.sync();
+    sync();
     pick_bin<kBins23>(cnt->hist2, remaining, bin, sm);
     prefix |= bin;
   }
@@ -1105,17 +1138,17 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
       });
   const uint2 mine_all = cta_sum2(c_gt, c_eq, sm2);
   if (threadIdx.x == 0) {
-    a.ws.chunk_a[blockIdx.x] = mine_all.x;
-    a.ws.chunk_b[blockIdx.x] = mine_all.y;
+    a.ws.chunk_a[rank] = mine_all.x;
+    a.ws.chunk_b[rank] = mine_all.y;
   }
-  grid.sync();
-  unsigned g_chunk = counts_before(a.ws.chunk_a, gridDim.x, blockIdx.x, sm2).before;
-  unsigned e_chunk = counts_before(a.ws.chunk_b, gridDim.x, blockIdx.x, sm2).before;
+  sync();
+  unsigned g_chunk = counts_before(a.ws.chunk_a, ranks, rank, sm2).before;
+  unsigned e_chunk = counts_before(a.ws.chunk_b, ranks, rank, sm2).before;
 
   // payload position = (#greater before) + min(#equal before, quota)
   auto send = [&](size_t index1, float v, unsigned ng, unsigned ne) {
     const unsigned pos = ng + (ne < quota ? ne : quota);
-    a.idx_out[pos] = static_cast<int>(index1);
+    a.idx_out[pos] = static_cast<int>(index1 + a.index_base);
     a.val_out[pos] = v;
     if (a.acc) a.acc[index1 - 1] = 0.0f;             // s - s
   };
@@ -1185,6 +1218,66 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
       e_at += te;
     }
   }
+}
+
+template <int MODE, typename Source>
+__global__ void __launch_bounds__(kBlock, kCtasPerSm)
+topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
+  topk_select<MODE>(a, source, blockIdx.x, [] { cg::this_grid().sync(); });
+}
+
+// Several buckets at once, each by its own part of a cooperative grid: a bucket of
+// 2e5 elements keeps 54 CTAs busy for a tenth of the 14 us that its barriers take
+// (2.56e7 elements in 11 buckets: 547 -> 210 us a pass, in 25: 727 -> 206; 2e6 in
+// four: 93 -> 42).
+// The parts do not wait for one another.  Their barrier counts arrivals; all CTAs
+// are resident, and the wait is bounded (run out: the sticky fault word).
+struct TopkBuckets {
+  int count;
+  unsigned first_cta[kBuckets + 1];
+  unsigned n[kBuckets], k[kBuckets], sample_target[kBuckets], at[kBuckets], index_base[kBuckets];   // at: in the payload
+  Work work[kBuckets];
+  size_t ws_off[kBuckets];         // of a bucket's lists in the workspace, behind the counters of all
+  float* acc[kBuckets];
+  int first_piece[kBuckets + 1];   // a bucket's offsets start at first_piece + its number (one more than pieces)
+  unsigned off[kPieces + kBuckets];
+  const float* ptr[kPieces];
+  char* ws;
+  int* idx_out;
+  float* val_out;
+};
+__device__ unsigned g_topk_faults;
+template <int MODE>
+__global__ void __launch_bounds__(kBlock, kCtasPerSm)
+topk_buckets_kernel(const __grid_constant__ TopkBuckets b) {
+  int g = 0;
+  for (int hi = b.count - 1; g < hi;) {
+    const int mid = (g + hi + 1) >> 1;
+    if (b.first_cta[mid] <= blockIdx.x) g = mid; else hi = mid - 1;
+  }
+  const PieceView source{b.first_piece[g + 1] - b.first_piece[g], b.off + b.first_piece[g] + g, b.ptr + b.first_piece[g]};
+  const TopkArgs a{nullptr, b.acc[g], b.n[g], b.k[g], b.sample_target[g], b.work[g],
+                   carve_at(b.ws + g * align256(sizeof(Counters)), b.ws + b.ws_off[g], b.work[g]), b.idx_out + b.at[g],
+                   b.val_out + b.at[g], true, b.index_base[g]};
+  unsigned* const arrived = &a.ws.counters->arrived;
+  unsigned target = 0;
+  topk_select<MODE>(a, source, blockIdx.x - b.first_cta[g], [&] {
+    target += a.work.grid;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(arrived, 1u);
+      bool in = false;
+      for (unsigned q = 0; q < (1u << 22) && !in; ++q) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+        in = v >= target;
+      }
+      if (!in) atomicOr(&g_topk_faults, 1u);
+      __threadfence();
+    }
+    __syncthreads();
+  });
 }
 
 // -------------------------------------------------------- dense sum of payloads
@@ -1509,7 +1602,19 @@ bool gather_buckets(Buckets* b, const SparseBucket* buckets, size_t count, size_
   return at > 0;
 }
 
-int topk_select(const Gradient& source, float* acc, size_t k, int mode, int* idx_out, float* val_out, void* ws,
+// The sample takes 8 us, and pass 1 over s 16 us per 10^7 elements: it pays
+// from there on, where every warp has two KB or more of elements to sample
+// from.  k up to n / 12, so that bound and margin stay inside the lists (352
+// entries per 2048 elements).  Margin: an eighth and four standard deviations.
+// Not for integer keys, which are mostly 0 or tied.
+inline unsigned sample_target(size_t n, size_t k, int mode, const Work& work) {
+  if (mode != 0 || work.run != 4 || k > n / 12) return 0;
+  double target = static_cast<double>(k) / static_cast<double>(n) * (work.grid * kWarps * 128.0);
+  target += target / 8 + 4 * std::sqrt(target) + 16;
+  return static_cast<unsigned>(target);
+}
+
+int topk_launch(const Gradient& source, float* acc, size_t k, int mode, int* idx_out, float* val_out, void* ws,
                 size_t ws_bytes, cudaStream_t s) {
   const size_t n = source.n;
   if (n == 0 || k == 0) return SGB_OK;
@@ -1520,18 +1625,8 @@ int topk_select(const Gradient& source, float* acc, size_t k, int mode, int* idx
   if (st != SGB_OK) return st;
   if (k > n) k = n;
   const Work work = work_for(n);
-  // The sample takes 8 us, and pass 1 over s 16 us per 10^7 elements: it pays
-  // from there on, where every warp has two KB or more of elements to sample
-  // from.  k up to n / 12, so that bound and margin stay inside the lists (352
-  // entries per 2048 elements).  Margin: an eighth and four standard deviations.
-  // Not for integer keys, which are mostly 0 or tied.
-  double target = 0;
-  if (mode == 0 && work.run == 4 && k <= n / 12) {
-    target = static_cast<double>(k) / static_cast<double>(n) * (work.grid * kWarps * 128.0);
-    target += target / 8 + 4 * std::sqrt(target) + 16;
-  }
-  TopkArgs a{g, acc, n, static_cast<unsigned>(k), static_cast<unsigned>(target), work, carve(ws, work), idx_out, val_out,
-             aligned16(g) && (!acc || aligned16(acc))};
+  TopkArgs a{g, acc, n, static_cast<unsigned>(k), sample_target(n, k, mode, work), work, carve(ws, work), idx_out, val_out,
+             aligned16(g) && (!acc || aligned16(acc)), 0};
   cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
   if (e != cudaSuccess) return note_cuda_error(e);
   if (!source.flat)
@@ -1566,11 +1661,99 @@ int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float th
   return launch_cooperative(thr_select_kernel<false, Buckets>, work.grid, a, b, s);
 }
 
-int sparse_dense_buckets(const int* payload, const int* nnz_dev, const SparseBucket* buckets, size_t count,
+// The plan of a joint top-K selection; false where it takes a launch per bucket.
+static bool topk_plan(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, TopkBuckets* b, size_t* bytes,
+                      size_t* sent) {
+  if (count < 2 || count > kBuckets) return false;
+  size_t total = 0;
+  std::vector<size_t> sizes;
+  for (size_t k = 0; k < count; ++k) {
+    size_t n = 0;
+    for (size_t t = 0; t < buckets[k].count; ++t) n += buckets[k].sizes[t];
+    sizes.push_back(n);
+    total += n;
+  }
+  if (total == 0) return false;
+  const size_t most = max_grid();
+  size_t index = 0, lists = 0, payload = 0, ctas = 0, pieces = 0;
+  Gradient g;
+  b->count = 0;
+  for (size_t k = 0; k < count; ++k) {
+    const size_t n = sizes[k];
+    if (n && ks[k]) {
+      if (!buckets[k].acc || !aligned16(buckets[k].acc) ||
+          !gather(&g, buckets[k].tensors, buckets[k].sizes, buckets[k].count, buckets[k].acc) ||
+          pieces + g.pieces.count > kPieces)
+        return false;
+      const int i = b->count++;
+      size_t share = (most - count) * n / total;       // (each gets at least one)
+      if (share < 1) share = 1;
+      b->work[i] = work_for(n, share);
+      b->first_cta[i] = static_cast<unsigned>(ctas);
+      ctas += b->work[i].grid;
+      b->n[i] = static_cast<unsigned>(n);
+      b->k[i] = static_cast<unsigned>(ks[k] < n ? ks[k] : n);
+      b->sample_target[i] = sample_target(n, b->k[i], mode, b->work[i]);
+      b->at[i] = static_cast<unsigned>(payload);
+      b->index_base[i] = static_cast<unsigned>(index);
+      b->ws_off[i] = lists;
+      b->acc[i] = buckets[k].acc;
+      b->first_piece[i] = static_cast<int>(pieces);
+      for (int p = 0; p <= g.pieces.count; ++p) b->off[pieces + i + p] = g.pieces.off[p];
+      for (int p = 0; p < g.pieces.count; ++p) b->ptr[pieces + p] = g.pieces.ptr[p];
+      pieces += g.pieces.count;
+      b->first_piece[i + 1] = static_cast<int>(pieces);
+      lists += lists_bytes(b->work[i]);
+      payload += b->k[i];
+    }
+    index = (index + n + kTile - 1) / kTile * kTile;
+  }
+  if (index > kMaxBucketSpan || ctas > most) return false;
+  b->first_cta[b->count] = static_cast<unsigned>(ctas);
+  const size_t counters = b->count * align256(sizeof(Counters));
+  for (int i = 0; i < b->count; ++i) b->ws_off[i] += counters;
+  *bytes = counters + lists;
+  *sent = payload;
+  return true;
+}
+
+size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode) {
+  TopkBuckets b;
+  size_t bytes = 0, sent = 0;
+  return topk_plan(buckets, ks, count, mode, &b, &bytes, &sent) ? bytes + 256 : 0;
+}
+
+int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
+                        void* ws, size_t ws_bytes, cudaStream_t s) {
+  TopkBuckets b;
+  size_t bytes = 0, total = 0;
+  if (!topk_plan(buckets, ks, count, mode, &b, &bytes, &total)) return SGB_ERR_UNSUPPORTED;
+  if (!ws || ws_bytes < bytes || (reinterpret_cast<uintptr_t>(ws) & 255u)) return SGB_ERR_WORKSPACE;
+  *sent = static_cast<int>(total);
+  if (b.count == 0) return SGB_OK;
+  b.ws = static_cast<char*>(ws);
+  b.idx_out = payload;
+  b.val_out = reinterpret_cast<float*>(payload) + total;
+  cudaError_t e = cudaMemsetAsync(ws, 0, b.count * align256(sizeof(Counters)), s);
+  if (e != cudaSuccess) return note_cuda_error(e);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(b.first_cta[b.count]);
+  cfg.blockDim = dim3(kBlock);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;       // all CTAs are resident, or the launch fails
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = mode == 0 ? cudaLaunchKernelEx(&cfg, topk_buckets_kernel<0>, b) : cudaLaunchKernelEx(&cfg, topk_buckets_kernel<1>, b);
+  return e == cudaSuccess ? launch_status() : note_cuda_error(e);
+}
+
+int sparse_dense_buckets(const int* payload, int known, const int* nnz_dev, const SparseBucket* buckets, size_t count,
                          cudaStream_t s, const SparseUpdate* update) {
   std::vector<float*> tensors, params, moments;
   std::vector<size_t> sizes;
-  const int none[1] = {0};
+  const int none[1] = {known};
   size_t at = 0;
   for (size_t k = 0; k < count; ++k) {
     size_t n = 0;
@@ -1616,7 +1799,7 @@ int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float*
                 float* val_out, void* ws, size_t ws_bytes, cudaStream_t s) {
   Gradient g;
   if (!gather(&g, tensors, sizes, count, acc)) return SGB_ERR_UNSUPPORTED;
-  return topk_select(g, acc, k, mode, idx_out, val_out, ws, ws_bytes, s);
+  return topk_launch(g, acc, k, mode, idx_out, val_out, ws, ws_bytes, s);
 }
 
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
@@ -1711,7 +1894,7 @@ int sgb_sparse_topk_f32(const float* g, float* acc, float* sum_scratch, size_t n
   Gradient source;
   source.flat = g;
   source.n = n;
-  return topk_select(source, acc, k, mode, idx_out, val_out, ws, ws_bytes, as_stream(stream));
+  return topk_launch(source, acc, k, mode, idx_out, val_out, ws, ws_bytes, as_stream(stream));
 }
 
 int sgb_scatter_add_f32(const int32_t* idx, const float* val, size_t count,

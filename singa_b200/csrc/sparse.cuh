@@ -44,8 +44,15 @@ struct SparseUpdate {
   float* const* params;
   float* const* moments;   // null without momentum
 };
-// The dense gradients of that payload, back into the buckets' tensors.
-int sparse_dense_buckets(const int* payload, const int* nnz_dev, const SparseBucket* buckets, size_t count,
+// Top-K of several buckets (the first ks[k] of bucket k by size) by one launch, into
+// a payload of the same joint space; *sent: its length.  sparse_topk_buckets_bytes:
+// of workspace, 0 where it takes a launch per bucket (fewer than two, more than 32).
+size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode);
+int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
+                        void* ws, size_t ws_bytes, cudaStream_t s);
+// The dense gradients of such a payload, back into the buckets' tensors; its length
+// is on the device, or (nnz_dev null) `known`.
+int sparse_dense_buckets(const int* payload, int known, const int* nnz_dev, const SparseBucket* buckets, size_t count,
                          cudaStream_t s, const SparseUpdate* update = nullptr);
 
 // Top-K selection (see sgb_sparse_topk_f32) from a tensor list.
