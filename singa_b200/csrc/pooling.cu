@@ -388,6 +388,9 @@ pool_k3s2p1_kernel(const StripArgs a) {
   const bool w1_exists = 2 * q + 1 < OW;
   const float kPad = kMax ? -FLT_MAX : 0.0f;
 
+  const int m0 = band * a.rows, m1 = min(m0 + a.rows, OH);
+  // backward: the odd row above window row m1 also takes from it
+  const int last = kBackward ? min(m1, OH - 1) : m1 - 1;
   auto load_row = [&](int h, float (&v)[4]) {
     const bool in = active && h >= 0 && h < H;
     if (VEC) {
@@ -423,6 +426,22 @@ pool_k3s2p1_kernel(const StripArgs a) {
       code[1] = active && w1_exists ? a.record[i + 1] : 0xffu;
     }
   };
+  // What window row m needs, into L2: the registers hold one row pair ahead, which is
+  // 29 KB in flight per SM where the rate takes 47.  32x64x112x112: forward 27.5 ->
+  // 25.7 us, backward 48.1 -> 46.1, with the record 31.9 -> 28.7, average backward
+  // 39.8 -> 32.7; two rows further ahead it is 26.7 and more.  The backward pass that
+  // finds its winners again has no registers to spare: not on small problems (8x64x
+  // 112x112 14.9 -> 15.2, 16x512x14x14 7.7 -> 8.2) and odd rows (111x111 49.8 -> 50.9).
+  const bool far = MODE != kMaxBwd || (VEC && static_cast<long long>(a.planes) * H * W >= 16000000);
+  auto ahead = [&](int m) {
+    if (!far || !active || m > last) return;
+    if (kNeedsX) {
+      const float* p = xp + static_cast<size_t>(2 * m) * W;
+      if (2 * m < H) prefetch_l2(p);
+      if (2 * m + 1 < H) prefetch_l2(p + W);
+    }
+    if (kBackward) prefetch_l2(a.dy + window0 + static_cast<size_t>(m) * OW);
+  };
   auto store_row = [&](int h, const float (&v)[4]) {
     if (!owner || h >= H) return;
     float* p = dxp + static_cast<size_t>(h) * W;
@@ -435,9 +454,6 @@ pool_k3s2p1_kernel(const StripArgs a) {
     }
   };
 
-  const int m0 = band * a.rows, m1 = min(m0 + a.rows, OH);
-  // backward: the odd row above window row m1 also takes from it
-  const int last = kBackward ? min(m1, OH - 1) : m1 - 1;
   float above[4], above_left = kPad, r0[4], r1[4], n0[4], n1[4], g[2] = {0.f, 0.f}, ng[2] = {0.f, 0.f};
   unsigned code[2] = {0, 0}, ncode[2] = {0, 0};
   bool odd_above = false;          // something in the row above that only the NaN-aware comparison may decide
@@ -454,6 +470,7 @@ pool_k3s2p1_kernel(const StripArgs a) {
     if (kMax) odd_above = __any_sync(kAll, unordered(above));
   }
   load_windows(m0, ng, ncode);
+  ahead(m0 + 1);
   float pend[4] = {0.f, 0.f, 0.f, 0.f};   // gradient of row 2m - 1 so far
   for (int m = m0; m <= last; ++m) {
 #pragma unroll
@@ -472,6 +489,7 @@ pool_k3s2p1_kernel(const StripArgs a) {
         load_row(2 * m + 3, n1);
       }
       load_windows(m + 1, ng, ncode);
+      ahead(m + 2);
     }
     int at0 = kNoCell, at1 = kNoCell;
     float best0 = 0.f, best1 = 0.f;
