@@ -55,7 +55,9 @@ def join_pays(n, c, hw):
 
 def merge_calls(calls):
     """The bound calls with neighbours merged that one kernel does together.
-    Every tensor that the separate calls write is written, with the same bits:
+    Every tensor that the separate calls write is written, with the same bits.  Calls
+    stay apart where one writes over what an earlier one has read (its operands are
+    not needed any more by then, but one kernel still reads them):
 
       add_relu_backward(-> t) ; bn_backward(dy=t)       =>  bn_add_relu_backward
       relu_backward(-> t) ; sum_rows(t)                 =>  relu_backward_sum_rows
@@ -74,14 +76,16 @@ def merge_calls(calls):
         if name == "sgb_bn_backward_f32" and last == "sgb_add_relu_backward_f32" and a[1] == b[3] and \
                 b[4] == a[8] * a[9] * a[10] and join_pays(*a[8:11]):
             out[-1] = ("sgb_bn_add_relu_backward_f32", (a[0],) + b[:3] + a[2:5] + (a[1],) + a[5:])
-        elif name == "sgb_sum_rows_f32" and last == "sgb_relu_backward_f32" and a[0] == b[2] and b[3] == a[2] * a[3]:
+        elif name == "sgb_sum_rows_f32" and last == "sgb_relu_backward_f32" and a[0] == b[2] and \
+                b[3] == a[2] * a[3] and a[1] not in b[:2]:
             out[-1] = ("sgb_relu_backward_sum_rows_f32", b[:3] + a[1:])
         elif name == "sgb_conv_bias_backward_f32" and last == "sgb_relu_backward_f32" and a[0] == b[2] and \
-                b[3] == a[2] * a[3] * a[4]:
+                b[3] == a[2] * a[3] * a[4] and a[1] not in b[:2]:
             out[-1] = ("sgb_relu_backward_conv_bias_f32", b[:3] + a[1:])
             before, p = out[-2] if len(out) > 1 else ("", None)
             # (pooling: x, y, dy, dx, n, c, h, w, windows, S; the pair: dy, x, dx, db, n, c, hw, ws, ws bytes, S)
-            if before == "sgb_maxpool_backward_f32" and p[3] == b[0] and p[4:6] == a[2:4] and p[6] * p[7] == a[4]:
+            if before == "sgb_maxpool_backward_f32" and p[3] == b[0] and p[4:6] == a[2:4] and p[6] * p[7] == a[4] and \
+                    not {b[2], a[1]} & {p[0], p[2]}:
                 out[-2:] = [("sgb_maxpool_relu_backward_conv_bias_f32", p[:-1] + b[1:3] + a[1:2] + a[5:])]
         elif name == "sgb_scalar_f32" and last == "sgb_softmax_cross_entropy_bwd_f32" and a[0] == 1 and \
                 a[1] == a[3] == b[5] and a[4] == b[1] * b[2]:
@@ -99,7 +103,7 @@ def merge_calls(calls):
         if [n for n, _ in out[-3:]] == ["sgb_softmax_cross_entropy_fused_f32", "sgb_sum_all_f32", "sgb_sum_rows_f32"]:
             (_, f), (_, total), (_, rows) = out[-3:]
             if total[0] == f[6] and total[2] == f[2] and rows[0] == f[7] and rows[2:4] == f[2:4] and \
-                    total[3:5] == rows[4:6]:
+                    total[3:5] == rows[4:6] and total[1] not in (f[6], f[7]) and rows[1] not in (f[6], f[7]):
                 out[-3:] = [("sgb_loss_head_f32", f[:8] + total[1:2] + rows[1:2] + rows[4:])]
     return out
 

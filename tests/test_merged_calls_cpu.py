@@ -46,3 +46,21 @@ def test_three_calls_become_one():
     assert merge_calls([fused, total, rows]) == [("sgb_loss_head_f32", (1, 3, 8, 10, 0.125, 2, 4, 9, 5, 11, 6, 7, S))]
     for apart in (("sgb_sum_rows_f32", (12, 11, 8, 10, 6, 7, S)), ("sgb_sum_rows_f32", (9, 11, 10, 8, 6, 7, S))):
         assert merge_calls([fused, total, apart]) == [fused, total, apart]
+
+
+def test_results_over_earlier_operands_stay_apart():
+    S = "STREAM"
+    pool = lambda x, dy: ("sgb_maxpool_backward_f32", (x, 21, dy, 1, 2, 3, 4, 6, 2, 2, 0, 0, 2, 2, S))   # noqa: E731
+    relu, bias = ("sgb_relu_backward_f32", (1, 2, 3, 144, S)), ("sgb_conv_bias_backward_f32", (3, 4, 2, 3, 24, 5, 6, S))
+    for first in (pool(3, 22), pool(20, 3), pool(4, 22), pool(20, 4)):     # the ReLU's result, then the sums
+        assert merge_calls([first, relu, bias])[0] == first
+    over = ("sgb_relu_backward_f32", (1, 2, 1, 144, S)), ("sgb_conv_bias_backward_f32", (1, 4, 2, 3, 24, 5, 6, S))
+    assert len(merge_calls([pool(20, 22), *over])) == 1                    # over the pooling's result: element by element
+    for over in (1, 2):                                                    # the sums over what the ReLU has read
+        for sums in (("sgb_conv_bias_backward_f32", (3, over, 2, 3, 24, 5, 6, S)), ("sgb_sum_rows_f32", (3, over, 6, 24, 5, 6, S))):
+            assert merge_calls([relu, sums]) == [relu, sums]
+    fused = ("sgb_softmax_cross_entropy_fused_f32", (1, 3, 8, 10, 0.125, 2, 4, 9, S))
+    total, rows = ("sgb_sum_all_f32", (4, 5, 8, 6, 7, S)), ("sgb_sum_rows_f32", (9, 11, 8, 10, 6, 7, S))
+    for apart in ([fused, total, ("sgb_sum_rows_f32", (9, 4, 8, 10, 6, 7, S))],        # the sums over the losses
+                  [fused, ("sgb_sum_all_f32", (4, 4, 8, 6, 7, S)), rows]):             # the total over them
+        assert merge_calls(apart) == apart
