@@ -192,7 +192,7 @@ class DistOpt(object):
         if self.world_size != 1 or type(grad_stream) not in _LISTS or type(opt) is not SGD or \
                 not _stands_with_update(type(self), type(c), exchange) or self._whole(exchange) is None:
             return None
-        (name, calls), mine, theirs = _WITH_UPDATE[exchange], self.__dict__, c.__dict__
+        (name, calls), mine, theirs = _WITH_UPDATE[exchange], self.__dict__, getattr(c, "__dict__", ())
         if "apply_many" in opt.__dict__ or "wait" in mine or "_update_all" in mine or "_sync_dense" in mine or \
                 name in theirs or any(x in theirs for x in calls):
             return None

@@ -125,3 +125,22 @@ def test_the_sparse_form_waits_for_the_reader_of_its_slot():
     assert plan(update)[0] == 1 | 1 << 14
     plan(7)
     assert list(state) == [0, 0, 0, 0] and plan(update)[0] == 1
+
+
+def test_a_communicator_without_attributes_of_its_own():
+    class Slots(object):
+        __slots__ = ("world_size", "local_rank", "global_rank", "synchHalf", "fusedSynchHalf")
+
+        def syncDense(self, stream, threshold, half=False):
+            raise AssertionError("updateHalf is there")
+
+        def updateHalf(self, params, grads, moments, threshold, hyper):
+            return True
+
+        def wait(self):
+            pass
+    comm = Slots()
+    comm.world_size, comm.local_rank, comm.global_rank = 1, 0, 0
+    opt = DistOpt(SGD(lr=0.5), communicator=comm)
+    opt.backward_and_update_half(triples(), threshold=20)
+    assert opt.opt.step_counter == 1
