@@ -173,3 +173,6 @@ class Communicator(object):
 
     def wait(self):
         _n.comm_wait(self._ptr)
+
+
+Communicator._defined = dict(vars(Communicator))       # see opt._as_defined

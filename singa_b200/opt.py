@@ -95,6 +95,7 @@ _WHOLE = {
 # (and what else of the communicator it stands for)
 _WITH_UPDATE = {"half": ("updateHalf", ("syncDense", "wait")),
                 "sparse": ("sparseUpdate", ("beginSparsification", "endSparsification", "sparsifyBuckets", "wait"))}
+_AROUND = ("wait", "_update_all", "_sync_dense")     # of DistOpt: what lies between the two
 _LISTS = (list, tuple, type(iter([])), type(iter(())))
 
 
@@ -104,26 +105,37 @@ def _inverse(world_size):
     return float(np.float32(1.0) / np.float32(world_size))
 
 
+def _as_defined(cls, names):
+    """Whether the class still has the functions that it was defined with (classes
+    that keep those in ``_defined``; others are taken as they are)."""
+    defined = vars(cls).get("_defined", {})
+    return all(vars(cls).get(f) is defined[f] for f in names if f in defined)
+
+
+# The last argument of these two: what the classes have in place of the functions that
+# the answer is about, so that a remembered answer is not given for others.
 @functools.lru_cache(maxsize=64)
-def _stands(own, kind, exchange):
+def _stands(own, kind, exchange, functions):
     """Whether the method of communicators of class `kind` does what `own` (DistOpt
     or a subclass) would do call by call: nobody below the class that defines it
-    has a version of its own of a call."""
+    has a version of its own of a call, and nobody has put one into that class."""
     name, forwards, calls = _WHOLE[exchange]
     owner = next((k for k in kind.__mro__ if name in vars(k)), None)
     return owner is not None and all(getattr(own, f) is getattr(DistOpt, f) for f in forwards) and \
-        all(getattr(kind, f, None) is getattr(owner, f, None) for f in calls)
+        all(getattr(kind, f, None) is getattr(owner, f, None) for f in calls) and \
+        _as_defined(DistOpt, forwards) and _as_defined(owner, calls)
 
 
 @functools.lru_cache(maxsize=64)
-def _stands_with_update(own, kind, exchange):
+def _stands_with_update(own, kind, exchange, functions):
     """Whether the method of communicators of class `kind` that also updates does what
     the exchange, wait() and the update of `own` would do one after the other."""
     def owner(name):
         return next((k for k in kind.__mro__ if name in vars(k)), None)
     name, calls = _WITH_UPDATE[exchange]
     return owner(name) is not None and all(owner(x) in (None, owner(name)) for x in calls) and \
-        all(getattr(own, f) is getattr(DistOpt, f) for f in ("wait", "_update_all", "_sync_dense"))
+        all(getattr(own, f) is getattr(DistOpt, f) for f in _AROUND) and \
+        _as_defined(DistOpt, _AROUND) and _as_defined(owner(name), calls) and _as_defined(SGD, ("apply_many",))
 
 
 class DistOpt(object):
@@ -179,8 +191,10 @@ class DistOpt(object):
         of one of the calls that it stands for, which then has to be called."""
         c = self.communicator
         name, (f, g), (x, y) = _WHOLE[exchange]
-        mine, theirs = self.__dict__, getattr(c, "__dict__", ())
-        if f in mine or g in mine or x in theirs or y in theirs or not _stands(type(self), type(c), exchange):
+        mine, theirs, own, kind = self.__dict__, getattr(c, "__dict__", ()), type(self), type(c)
+        if f in mine or g in mine or x in theirs or y in theirs or \
+                not _stands(own, kind, exchange, (getattr(own, f), getattr(own, g), getattr(kind, x, None),
+                                                  getattr(kind, y, None), getattr(kind, name, None))):
             return None
         return getattr(c, name)
 
@@ -189,10 +203,14 @@ class DistOpt(object):
         exist already and the update behind it (_WITH_UPDATE), on one rank.  None
         where it has none, or where something that it stands for has been replaced."""
         c, opt = self.communicator, self.opt
-        if self.world_size != 1 or type(grad_stream) not in _LISTS or type(opt) is not SGD or \
-                not _stands_with_update(type(self), type(c), exchange) or self._whole(exchange) is None:
+        if self.world_size != 1 or type(grad_stream) not in _LISTS or type(opt) is not SGD:
             return None
+        own, kind = type(self), type(c)
         (name, calls), mine, theirs = _WITH_UPDATE[exchange], self.__dict__, getattr(c, "__dict__", ())
+        functions = (SGD.apply_many, own.wait, own._update_all, own._sync_dense, getattr(kind, name, None),
+                     *[getattr(kind, x, None) for x in calls])
+        if not _stands_with_update(own, kind, exchange, functions) or self._whole(exchange) is None:
+            return None
         if "apply_many" in opt.__dict__ or "wait" in mine or "_update_all" in mine or "_sync_dense" in mine or \
                 name in theirs or any(x in theirs for x in calls):
             return None
@@ -404,3 +422,6 @@ class DistOpt(object):
             self.opt.step()
         else:
             self._update_all((names, params, grads))
+
+
+SGD._defined, DistOpt._defined = dict(vars(SGD)), dict(vars(DistOpt))

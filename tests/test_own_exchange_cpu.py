@@ -130,3 +130,29 @@ def test_a_communicator_without_whole_calls():
         seen = []
         synch, fusedSynch, wait = Comm.synch, Comm.fusedSynch, Comm.wait
     assert run(DistOpt(Opt(), communicator=Plain()), "backward_and_update") == DENSE
+
+
+@pytest.mark.parametrize("where", ["communicator", "driver"])
+def test_a_call_put_into_the_class_is_called(where, monkeypatch):
+    """Also after the same classes have been looked at without it, and no longer than it is there."""
+    class Traced(Comm):
+        pass
+    Traced.synch = Comm.synch
+    Traced.syncDense = Comm.syncDense
+    Traced._defined = dict(vars(Traced))
+    opt = DistOpt(Opt(), communicator=Traced())
+    stream = lambda: [("p%d" % i, torch.zeros(n), torch.ones(n)) for i, n in enumerate(SIZES)]   # noqa: E731
+
+    def seen():
+        opt.communicator.seen.clear()
+        opt.backward_and_update(stream(), threshold=20)
+        return list(opt.communicator.seen)
+    whole = [("syncDense", False)]
+    assert seen() == whole
+    with monkeypatch.context() as m:
+        if where == "communicator":
+            m.setattr(Traced, "synch", lambda self, t: self.seen.append(("traced",)))
+        else:
+            m.setattr(DistOpt, "all_reduce", lambda self, t: self.communicator.seen.append(("traced",)))
+        assert seen() == [("traced",)] + DENSE[1:]
+    assert seen() == whole

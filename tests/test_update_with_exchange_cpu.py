@@ -144,3 +144,18 @@ def test_a_communicator_without_attributes_of_its_own():
     opt = DistOpt(SGD(lr=0.5), communicator=comm)
     opt.backward_and_update_half(triples(), threshold=20)
     assert opt.opt.step_counter == 1
+
+
+@pytest.mark.parametrize("owner, name", [(SGD, "apply_many"), (DistOpt, "_update_all"), (DistOpt, "wait")])
+def test_a_function_put_into_the_class_is_called(owner, name, monkeypatch):
+    opt, called = DistOpt(SGD(lr=0.5), communicator=Comm()), []
+    for method, kw in (("backward_and_update_half", {}), ("backward_and_sparse_update", dict(spars=0.1))):
+        both = run(opt, method, **kw)
+        assert isinstance(both[0], tuple)
+        with monkeypatch.context() as m:
+            m.setattr(SGD, "apply_many", lambda self, *a: None)          # CPU tensors: not applied
+            m.setattr(owner, name, lambda self, *a: called.append(name))
+            seen = run(opt, method, **kw)
+        assert called and not any(isinstance(s, tuple) for s in seen)
+        called.clear()
+        assert run(opt, method, **kw) == both
