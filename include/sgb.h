@@ -12,7 +12,9 @@
  *  - Calls only enqueue work; none synchronises unless documented.
  *  - No entry point allocates device memory.  Kernels that need scratch take
  *    a workspace pointer + size; the matching *_workspace_bytes() query gives
- *    the requirement.  (The communicator owns its staging buffers, allocated
+ *    the requirement.  A workspace serves one call at a time: calls that may
+ *    overlap (two streams, a replayed graph beside them) need one each, since
+ *    kernels exchange sums through it.  (The communicator owns its staging buffers, allocated
  *    once at creation, as the reference's does.)
  *  - Sizes are size_t element counts.  n == 0 is legal and a no-op.
  *  - Each declaration cites the reference interface (file:line inside

@@ -20,7 +20,9 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -157,42 +159,120 @@ void issue(const char* name, F&& f) {
 #define ISSUE(fn, ...) issue(#fn, [&] { return fn(__VA_ARGS__); })
 
 // ---------------------------------------------------------------- workspace
-// One scratch buffer per device, owned here (the C ABI never allocates).  When
-// a larger request arrives a new buffer takes over and the old one is kept
-// alive: its address may sit in a captured graph or in work queued on another
-// stream.  Growing while a capture is under way is refused.
+// Scratch buffers, owned here (the C ABI never allocates).  Kernels exchange sums
+// through them while they run, so calls that may overlap never share one: there is
+// one per device, stream and host thread (a call of several kernels is not cut in
+// two by another thread's on the same stream), and one per capture, which its graph
+// keeps for its own replays.  A buffer that a call still holds outlives its place
+// here, and what is given back goes to its stream's part of torch's allocator.
 struct Scratch {
-  std::vector<Tensor> current, retired;
+  cudaStream_t stream;
+  unsigned long long thread;
+  Tensor buffer;
 };
-Scratch& scratch() {
-  static Scratch* s = new Scratch;   // never destroyed: the CUDA context may be gone by then
-  return *s;
+struct CapturedScratch {
+  unsigned long long capture;
+  cudaStream_t stream;
+  unsigned long long thread;
+  Tensor buffer;
+};
+constexpr size_t kMostScratch = 32;          // per device; beyond it the one used least recently goes
+constexpr size_t kLeastScratch = size_t{1} << 20;
+
+// Most recently used first.  Never destroyed: the CUDA context may be gone by then.
+std::vector<Scratch>& scratch_of(size_t device) {
+  static auto* all = new std::vector<std::vector<Scratch>>;
+  if (all->size() <= device) all->resize(device + 1);
+  return (*all)[device];
 }
-const Tensor& workspace(const Tensor& like, size_t bytes) {
-  const size_t d = static_cast<size_t>(like.device().index());
-  auto& cur = scratch().current;
-  if (cur.size() <= d) cur.resize(d + 1);
-  Tensor& buf = cur[d];
-  if (!buf.defined() || count(buf) < bytes) {
-    if (buf.defined()) {
-      if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-        fail(PyExc_RuntimeError, "workspace of " + std::to_string(bytes) + " bytes needed during stream capture (have " +
-                                     std::to_string(count(buf)) + "): run the call once before capturing");
-      scratch().retired.push_back(buf);
-    }
-    const size_t want = bytes > (1u << 20) ? bytes : (1u << 20);
-    buf = fresh({static_cast<int64_t>(want)}, at::kByte, like);
+void cuda_ok(cudaError_t e, const char* what) {
+  if (e == cudaSuccess) return;
+  cudaGetLastError();
+  fail(PyExc_RuntimeError, std::string(what) + ": " + cudaGetErrorString(e));
+}
+// Captured buffers by number, and the numbers of those whose graph, with all that was
+// made of it, is gone.
+std::map<unsigned long long, CapturedScratch>& captured_scratch() {
+  static auto* m = new std::map<unsigned long long, CapturedScratch>;
+  return *m;
+}
+struct Gone {
+  std::mutex guard;
+  std::atomic<bool> any{false};
+  std::vector<unsigned long long> numbers;
+};
+Gone& gone() {
+  static auto* g = new Gone;
+  return *g;
+}
+void give_back() {
+  if (!gone().any.load(std::memory_order_relaxed)) return;
+  std::vector<unsigned long long> numbers;
+  {
+    const std::lock_guard<std::mutex> lock(gone().guard);
+    numbers.swap(gone().numbers);
+    gone().any = false;
   }
-  return buf;
+  for (const auto n : numbers) captured_scratch().erase(n);
 }
-struct Ws {
+// Buffer of a capture under way: a new one for a request that the capture's others are too small for.
+Tensor capture_workspace(const Tensor& like, size_t bytes, unsigned long long capture, cudaGraph_t graph,
+                         cudaStream_t stream, unsigned long long thread) {
+  static unsigned long long last = 0;
+  for (const auto& [n, c] : captured_scratch())
+    if (c.capture == capture && c.stream == stream && c.thread == thread && c.buffer.device() == like.device() &&
+        count(c.buffer) >= bytes)
+      return c.buffer;
+  const Tensor buffer = fresh({static_cast<int64_t>(bytes)}, at::kByte, like);
+  const auto destroy = [](void* number) {      // may call nothing of CUDA
+    const std::lock_guard<std::mutex> lock(gone().guard);
+    gone().numbers.push_back(reinterpret_cast<uintptr_t>(number));
+    gone().any = true;
+  };
+  cudaUserObject_t owner;
+  cuda_ok(cudaUserObjectCreate(&owner, reinterpret_cast<void*>(static_cast<uintptr_t>(++last)), destroy, 1,
+                               cudaUserObjectNoDestructorSync), "cudaUserObjectCreate");
+  captured_scratch().emplace(last, CapturedScratch{capture, stream, thread, buffer});
+  const cudaError_t kept = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+  if (kept != cudaSuccess) cudaUserObjectRelease(owner, 1);
+  cuda_ok(kept, "cudaGraphRetainUserObject");
+  return buffer;
+}
+Tensor workspace(const Tensor& like, size_t bytes) {
+  static std::atomic<unsigned long long> threads{0};
+  thread_local const unsigned long long thread = ++threads;
+  const cudaStream_t s = c10::cuda::getCurrentCUDAStream().stream();
+  unsigned long long capture = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  cuda_ok(cudaStreamGetCaptureInfo(s, &status, &capture, &graph, nullptr, nullptr), "cudaStreamGetCaptureInfo");
+  give_back();
+  if (status != cudaStreamCaptureStatusNone) return capture_workspace(like, bytes, capture, graph, s, thread);
+  auto& list = scratch_of(static_cast<size_t>(like.device().index()));
+  size_t k = 0;
+  while (k < list.size() && !(list[k].stream == s && list[k].thread == thread)) ++k;
+  if (k == list.size()) {
+    if (k == kMostScratch) list.pop_back();
+    list.insert(list.begin(), Scratch{s, thread, Tensor()});
+  } else if (k) {
+    std::rotate(list.begin(), list.begin() + k, list.begin() + k + 1);
+  }
+  Tensor& buffer = list[0].buffer;
+  if (!buffer.defined() || count(buffer) < bytes) {
+    buffer = Tensor();
+    buffer = fresh({static_cast<int64_t>(std::max(bytes, kLeastScratch))}, at::kByte, like);
+  }
+  return buffer;
+}
+struct Ws {                                  // keeps the buffer until its call has been launched
+  Tensor held;
   void* ptr = nullptr;
   size_t bytes = 0;
   Ws(const Tensor& like, size_t need) {
     if (!need) return;
-    const Tensor& b = workspace(like, need);
-    ptr = raww(b);
-    bytes = count(b);
+    held = workspace(like, need);
+    ptr = raww(held);
+    bytes = count(held);
   }
 };
 PyObject* py_workspace(Args a, Py_ssize_t) {   // (tensor on the device, bytes)

@@ -148,13 +148,11 @@ def Transform(t_storage, shape, stride):
 
 # ------------------------------------------------------------------ workspace
 def _workspace(like, nbytes):
-    """A per-device scratch buffer owned by the host layer (the C ABI never
-    allocates); 256-byte aligned by the torch allocator.  When a larger request
-    arrives a new buffer takes over and the old one is RETIRED, not freed: its
-    address may sit in a captured CUDA graph or in work queued on another
-    stream, and must not be handed to someone else by the caching allocator.
-    A graph captured through these wrappers therefore pins the workspace it saw.
-    Growth during a stream capture is refused (it would allocate inside it)."""
+    """A scratch buffer owned by the host layer (the C ABI never allocates), 256-byte
+    aligned by the torch allocator.  Kernels exchange sums through it while they run,
+    so calls that may overlap never get the same one: it belongs to the current
+    stream and host thread or, during a capture, to the graph that is being made,
+    whose replays keep it to themselves for as long as they can run."""
     return _n.workspace(like, nbytes)
 
 
