@@ -384,8 +384,8 @@ int sgb_bn_forward_training_f32(const float *x, const float *scale,
  * most eight such launches may be in flight per device; bits 8 and 16 the same
  * for the exchanges inside the backward and forward cluster kernels, bit 24 for
  * the kernels that visit their data twice).  A
- * faulted launch stops early and its outputs are undefined.  Synchronises the
- * device. */
+ * faulted launch stops early and its outputs are undefined, and so are those of
+ * a graph that holds it from then on.  Synchronises the device. */
 int sgb_bn_backward_faults(unsigned *flags);
 /* How the streaming form would cut an (N, C, HW) problem (host arithmetic
  * only, no device work): returns 1 and fills plan6 = {pieces per plane, floats

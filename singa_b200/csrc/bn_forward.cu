@@ -474,6 +474,7 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
   constexpr int NV = kFwd<VEC>.units, kWarps = kFwd<VEC>.threads / 32;
   __shared__ float sm[2][kWarps];
   __shared__ float coef[3];
+  __shared__ bool stopped;
   const unsigned item = blockIdx.x, mine = item - r.delay, threads = blockDim.x - 32;
   const bool summing = static_cast<int>(item) < r.items, finishing = static_cast<int>(item) >= r.delay;
   const unsigned numel = static_cast<unsigned>(a.numel);
@@ -484,21 +485,22 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
     const unsigned c = r.parts.quot(mine);
     const float sc = a.scale[c], b = a.bias[c];
     Moments m{0.f, 0.f, 0.f};
-    revisit_gather(r, c, [&](unsigned k, float mean, float m2) {
+    const bool got = revisit_gather(r, c, [&](unsigned k, float mean, float m2) {
       const unsigned e0 = elements_before<VEC>(r, c, k * r.per), e1 = elements_before<VEC>(r, c, min((k + 1) * r.per, r.total));
       m = merge(m, Moments{static_cast<float>(e1 - e0), mean, m2});
     });
     m = warp_merge(m);
     if ((threadIdx.x & 31) == 0) {
+      stopped = !got;
       const float var = m.m2 / (static_cast<float>(a.sh.N) * static_cast<float>(a.sh.HW));
       const float invstd = 1.0f / sqrtf(var + a.eps);
       coef[0] = m.mean;
       coef[1] = sc * invstd;
       coef[2] = b;
-      if (mine == c * r.parts.d) finish_channel(a, c, m.mean, var, invstd);
+      if (got && mine == c * r.parts.d) finish_channel(a, c, m.mean, var, invstd);
     }
     revisit_arrive(2, blockDim.x);
-    revisit_leave(r, c);
+    if (got) revisit_leave(r, c);
     return;
   }
   Vec4f v[NV];
@@ -552,6 +554,7 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
   for (int k = 0; k < NV; ++k)
     if (u.valid[k]) v[k] = u.load(a.x, k, numel, ease);
   revisit_sync(2, blockDim.x);
+  if (stopped) return;
   const float mu = coef[0], g = coef[1], b = coef[2];
 #pragma unroll
   for (int k = 0; k < NV; ++k)
@@ -584,10 +587,10 @@ int launch_revisit(const FwdArgs& a, void* ws, size_t ws_bytes, cudaStream_t s) 
   if (!ws || !aligned16(ws) || !revisit_plan(kFwd<VEC>, units, upp, a.sh.C, &p) || ws_bytes < p.bytes)
     return SGB_ERR_WORKSPACE;
   int st = SGB_OK;
-  unsigned* faults = revisit_fault_word(&st);
-  if (!faults) return st;
+  RevisitState* state = revisit_state(&st);
+  if (!state) return st;
   return launch_ex(bn_fwd_revisit_kernel<VEC>, dim3(static_cast<unsigned>(p.items + p.delay)), dim3(p.threads + 32), 0,
-                   s, 0, true, a, revisit_args(p, units, upp, a.sh.C, a.sh.HW, ws, faults));
+                   s, 0, true, a, revisit_args(p, units, upp, a.sh.C, a.sh.HW, ws, state));
 }
 
 // ------------------------------------------------------------- in two passes

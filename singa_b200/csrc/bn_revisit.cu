@@ -21,7 +21,7 @@ unsigned long long revisit_tag() {
 
 namespace {
 
-__device__ unsigned g_revisit_faults;
+__device__ RevisitState g_revisit_state;
 
 // Four vectors of x, dy and the ReLU's input are 48 registers, and four CTAs of
 // 256 threads fill an SM; the masked ends of ragged planes need registers for
@@ -51,6 +51,7 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
   constexpr int NV = kBwd<VEC>.units;
   __shared__ float2 sm[kBwd<VEC>.threads / 32];
   __shared__ float4 coef;
+  __shared__ bool stopped;
   const unsigned item = blockIdx.x, mine = item - a.r.delay, threads = blockDim.x - 32;
   const bool summing = static_cast<int>(item) < a.r.items, finishing = static_cast<int>(item) >= a.r.delay;
   if (threadIdx.x >= threads) {
@@ -60,22 +61,23 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
     const unsigned c = a.r.parts.quot(mine);
     const float sc = a.scale[c], r = a.invstd[c], mu = a.mean[c];
     float s = 0.f, t = 0.f;
-    revisit_gather(a.r, c, [&](unsigned, float p, float q) {
+    const bool got = revisit_gather(a.r, c, [&](unsigned, float p, float q) {
       s += p;
       t += q;
     });
     s = warp_sum(s);
     t = warp_sum(t);
     if ((threadIdx.x & 31) == 0) {
+      stopped = !got;
       const float ds = t * r;
       coef = make_float4(sc * r, s * a.inv_m, ds * r * a.inv_m, mu);
-      if (mine == c * a.r.parts.d) {
+      if (got && mine == c * a.r.parts.d) {
         a.dscale[c] = ds;
         a.dbias[c] = s;
       }
     }
     revisit_arrive(2, blockDim.x);
-    revisit_leave(a.r, c);
+    if (got) revisit_leave(a.r, c);
     return;
   }
   // loads of all units at once; what is not there is 0
@@ -141,6 +143,7 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
   const RevisitUnits<VEC, NV> u(a.r, mine, threads);
   load(u, drop_policy());
   revisit_sync(2, blockDim.x);
+  if (stopped) return;
   const float k_ = coef.x, am = coef.y, bm = coef.z, mu = coef.w;
 #pragma unroll
   for (int k = 0; k < NV; ++k)
@@ -154,8 +157,8 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
 
 }  // namespace
 
-unsigned* revisit_fault_word(int* status) {
-  static std::atomic<unsigned*> cached[64];
+RevisitState* revisit_state(int* status) {
+  static std::atomic<RevisitState*> cached[64];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= 64) {
@@ -163,20 +166,20 @@ unsigned* revisit_fault_word(int* status) {
     return nullptr;
   }
   *status = SGB_OK;
-  unsigned* p = cached[dev].load(std::memory_order_acquire);
+  RevisitState* p = cached[dev].load(std::memory_order_acquire);
   if (p) return p;
   void* q = nullptr;
-  e = cudaGetSymbolAddress(&q, g_revisit_faults);
+  e = cudaGetSymbolAddress(&q, g_revisit_state);
   if (e != cudaSuccess) {
     *status = note_cuda_error(e);
     return nullptr;
   }
-  cached[dev].store(static_cast<unsigned*>(q), std::memory_order_release);
-  return static_cast<unsigned*>(q);
+  cached[dev].store(static_cast<RevisitState*>(q), std::memory_order_release);
+  return static_cast<RevisitState*>(q);
 }
 
 int revisit_faults(unsigned* flags) {
-  const cudaError_t e = cudaMemcpyFromSymbol(flags, g_revisit_faults, sizeof(unsigned));
+  const cudaError_t e = cudaMemcpyFromSymbol(flags, g_revisit_state, sizeof(unsigned));
   return e == cudaSuccess ? SGB_OK : note_cuda_error(e);
 }
 
@@ -195,12 +198,12 @@ int bn_revisit_backward(int mask, const float* x, const float* dy, const float* 
   RevisitPlan p;
   if (!ws || !aligned16(ws) || !revisit_plan(vec ? kBwd<true> : kBwd<false>, units, upp, C, &p) || ws_bytes < p.bytes) return SGB_ERR_WORKSPACE;
   int st = SGB_OK;
-  unsigned* faults = revisit_fault_word(&st);
-  if (!faults) return st;
+  RevisitState* state = revisit_state(&st);
+  if (!state) return st;
   const BwdArgs a{x, dy, relu, scale, mean, invstd, dx, dscale, dbias,
                   static_cast<unsigned>(N) * static_cast<unsigned>(C) * static_cast<unsigned>(HW),
                   1.0f / (static_cast<float>(N) * static_cast<float>(HW)),
-                  revisit_args(p, units, upp, C, HW, ws, faults)};
+                  revisit_args(p, units, upp, C, HW, ws, state)};
   auto kernel = mask == 0   ? (vec ? bn_bwd_revisit_kernel<0, true> : bn_bwd_revisit_kernel<0, false>)
                 : mask == 1 ? (vec ? bn_bwd_revisit_kernel<1, true> : bn_bwd_revisit_kernel<1, false>)
                             : (vec ? bn_bwd_revisit_kernel<2, true> : bn_bwd_revisit_kernel<2, false>);

@@ -16,15 +16,19 @@
 // were all slower by 10 to 40 %.
 //
 // The exchange is in the caller's workspace, whose contents are unknown when the
-// kernel starts.  An item's two sums and the launch's tag, a 64-bit number that no
-// other launch of the process has, travel in one 16-byte access: an entry counts
-// once it shows the tag.  A graph replays a launch with the same tag, so the last
-// reader of a channel takes the tags away again.
+// kernel starts and which serves one launch at a time.  An item's two sums and the
+// launch's tag, a 64-bit number that no other launch of the process has, travel in
+// one 16-byte access: an entry counts once it shows the tag.  A graph replays a launch
+// with the same tag, so the last reader of a channel takes the tags away again.
 //
 // Progress: a CTA waits for CTAs with lower numbers only, and for a part of them
 // that waits for nobody.  CTAs are started in order, so however few are resident,
-// the lowest one can always go on.  The waits are bounded all the same: a run-out
-// sets the sticky fault word and voids that launch's outputs.
+// the lowest one can always go on.  (CUDA does not promise that order.  As the CTAs
+// that are waited for lie a full wave behind, more than a wave of disorder would be
+// needed for all resident CTAs to wait for ones that have no place.)  The waits are
+// bounded all the same: a CTA whose wait runs out sets the sticky fault word and names
+// the launch as stopped; the launch's other CTAs see that while they poll, and none
+// of them finishes its item.
 #pragma once
 #include "bn_common.cuh"
 
@@ -32,8 +36,12 @@ namespace sgb {
 
 // A number that no other launch of this process has, and that data do not show by chance.
 unsigned long long revisit_tag();
-// Address of the sticky fault word on the current device; null on an error.
-unsigned* revisit_fault_word(int* status);
+struct RevisitState {                  // one per device
+  unsigned faults;                     // sticky fault word
+  unsigned long long stopped;          // tag of the last launch whose wait ran out
+};
+// Its address on the current device; null on an error.
+RevisitState* revisit_state(int* status);
 int revisit_faults(unsigned* flags);
 
 // Backward: planes of any size from eight floats on, all pointers 16-byte aligned.
@@ -84,17 +92,18 @@ struct Revisit {
   RevisitEntry* entries;               // one per item
   unsigned* readers;                   // per channel: items finished
   unsigned long long tag;
-  unsigned* faults;
+  RevisitState* state;
   FastDiv parts;
   unsigned per, total;                 // units per item, per channel
   int items, delay;
   FastDiv upp;                         // units per plane
   unsigned hw, plane_stride;           // plane_stride: elements per sample
 };
-inline Revisit revisit_args(const RevisitPlan& p, long long units, int upp, int C, int HW, void* ws, unsigned* faults) {
+inline Revisit revisit_args(const RevisitPlan& p, long long units, int upp, int C, int HW, void* ws,
+                            RevisitState* state) {
   char* const base = static_cast<char*>(ws);
   return Revisit{reinterpret_cast<RevisitEntry*>(base), reinterpret_cast<unsigned*>(base + p.readers), revisit_tag(),
-                 faults, FastDiv(static_cast<unsigned>(p.parts)), static_cast<unsigned>(p.per),
+                 state, FastDiv(static_cast<unsigned>(p.parts)), static_cast<unsigned>(p.per),
                  static_cast<unsigned>(units), p.items, p.delay, FastDiv(static_cast<unsigned>(upp)),
                  static_cast<unsigned>(HW), static_cast<unsigned>(C) * static_cast<unsigned>(HW)};
 }
@@ -148,37 +157,50 @@ __device__ __forceinline__ bool get_entry(const RevisitEntry* p, unsigned long l
 __device__ __forceinline__ void revisit_publish(const Revisit& r, unsigned item, unsigned c, unsigned part, float a,
                                                 float b) {
   if (part == 0) {
+    // a graph's launches share a tag: an earlier one's stop is not this one's
+    if (item == 0 && *static_cast<volatile unsigned long long*>(&r.state->stopped) == r.tag) r.state->stopped = 0;
     r.readers[c] = 0;
     __threadfence();                   // who has seen the entry sees the 0
   }
   put_entry(r.entries + item, a, b, r.tag);
 }
 
-constexpr unsigned kMostPolls = 1u << 21;   // of half a microsecond and more
+constexpr unsigned kMostPolls = 1u << 20;   // of half a microsecond and more
 
 // One warp: calls fold(k, a, b) with the channel's entries k = lane, lane + 32, ...;
-// all entries of a batch are asked for at once.
+// all entries of a batch are asked for at once.  False (in all lanes): the launch has
+// been stopped.
 template <typename F>
-__device__ __forceinline__ void revisit_gather(const Revisit& r, unsigned c, F fold) {
+__device__ __forceinline__ bool revisit_gather(const Revisit& r, unsigned c, F fold) {
   constexpr int kBatch = 4;
   const unsigned parts = r.parts.d;
   const RevisitEntry* const e = r.entries + static_cast<size_t>(c) * parts;
-  for (unsigned k0 = threadIdx.x & 31; k0 < parts; k0 += 32 * kBatch) {
+  bool got = true;
+  for (unsigned k0 = threadIdx.x & 31; got && k0 < parts; k0 += 32 * kBatch) {
     float a[kBatch], b[kBatch];
     unsigned missing = 0;
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
       if (k0 + 32 * q < parts && !get_entry(e + k0 + 32 * q, r.tag, a[q], b[q])) missing |= 1u << q;
-    for (unsigned n = 0; missing && n < kMostPolls; ++n)
+    for (unsigned n = 1; missing && got; ++n) {
 #pragma unroll
       for (int q = 0; q < kBatch; ++q)
         if (missing >> q & 1u && get_entry(e + k0 + 32 * q, r.tag, a[q], b[q])) missing &= ~(1u << q);
-    if (missing) atomicOr(r.faults, 1u);
+      if (n % 256 == 0 && missing) {
+        got = *static_cast<volatile unsigned long long*>(&r.state->stopped) != r.tag;
+        if (got && n >= kMostPolls) {
+          r.state->stopped = r.tag;
+          atomicOr(&r.state->faults, 1u);
+          got = false;
+        }
+      }
+    }
+    if (!got) break;
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
       if (k0 + 32 * q < parts) fold(k0 + 32 * q, a[q], b[q]);
   }
-  __syncwarp();
+  return __all_sync(0xffffffffu, got);
 }
 // The same warp, once it has the sums: the last reader takes the channel's tags away.
 __device__ __forceinline__ void revisit_leave(const Revisit& r, unsigned c) {
