@@ -516,6 +516,11 @@ int sgb_unpack_f16_to_f32(const void *flat_f16, size_t flat_offset,
 /* ------------------------------------------------- sparsification kernels */
 /* Workspace (256-byte aligned) for the two selectors below. */
 size_t sgb_sparse_workspace_bytes(size_t n);
+/* Diagnostic: the sticky fault word of the current device's joint top-K selections
+ * (sgb_comm_sparse_update), whose CTAs meet with bounded waits: 0 = none, 1 a wait
+ * ran out.  Such a launch stops early; its gradients, parameters, momenta and
+ * residuals are undefined.  Synchronises the device. */
+int sgb_sparse_faults(unsigned *flags);
 /* K of the top-K variant: (int)ceil(ratio * n) evaluated in fp32 exactly as
  * Communicator::topKSparsAllReduce does (src/io/communicator.cc:744). */
 int sgb_topk_count(float ratio, size_t n);

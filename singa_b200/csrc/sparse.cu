@@ -811,7 +811,8 @@ __device__ __forceinline__ void list_keys(const float (&s)[kRounds][4], unsigned
 // sample (8 us) saves the most and four in five of the shared-memory atomics.
 //
 // `rank` of a.work.grid CTAs, which sync() brings together: the whole grid, or the
-// part of it that works on one of several buckets.
+// part of it that works on one of several buckets.  Where sync() says false the others
+// did not come: what they should have written is not there, and the CTA leaves.
 template <int MODE, typename Source, typename Sync>
 __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& source, const unsigned rank, Sync sync) {
   constexpr unsigned kSlots = 96;
@@ -847,7 +848,7 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
     for (int q = 0; q < 4; ++q) bin[q] = make_key<MODE>(v[q]) >> 20;
     tally4(sh, bin, take);
     flush_bins<kBins1>(sh, cnt->sample);
-    sync();
+    if (!sync()) return;
     unsigned left = a.sample_target, b;
     pick_bin<kBins1>(cnt->sample, left, b, sm);
     // more than an eighth at or above the bound (ties, a crowded bin) would not fit the lists
@@ -911,7 +912,7 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
     for (int k = 1; k < kWarps; ++k) top = max(top, sm[k]);
     if (top) atomicMax(&cnt->max_key, top);
   }
-  sync();
+  if (!sync()) return;
 
   unsigned remaining = a.k, bin;
   pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
@@ -943,7 +944,7 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
         },
         nothing);
     flush_bins<kBins1>(sh, cnt->hist0);
-    sync();
+    if (!sync()) return;
     remaining = a.k;
     pick_bin<kBins1>(cnt->hist0, remaining, bin, sm);
   }
@@ -1066,7 +1067,7 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
         nothing);
   }
   flush_bins<kBins23>(sh, cnt->hist1);
-  sync();
+  if (!sync()) return;
   pick_bin<kBins23>(cnt->hist1, remaining, bin, sm);
   prefix |= bin << shift;
 
@@ -1095,7 +1096,7 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
           },
           no_done);
     flush_bins<kBins23>(sh, cnt->hist2);
-    sync();
+    if (!sync()) return;
     pick_bin<kBins23>(cnt->hist2, remaining, bin, sm);
     prefix |= bin;
   }
@@ -1141,7 +1142,7 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
     a.ws.chunk_a[rank] = mine_all.x;
     a.ws.chunk_b[rank] = mine_all.y;
   }
-  sync();
+  if (!sync()) return;
   unsigned g_chunk = counts_before(a.ws.chunk_a, ranks, rank, sm2).before;
   unsigned e_chunk = counts_before(a.ws.chunk_b, ranks, rank, sm2).before;
 
@@ -1223,7 +1224,10 @@ __device__ __forceinline__ void topk_select(const TopkArgs& a, const Source& sou
 template <int MODE, typename Source>
 __global__ void __launch_bounds__(kBlock, kCtasPerSm)
 topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
-  topk_select<MODE>(a, source, blockIdx.x, [] { cg::this_grid().sync(); });
+  topk_select<MODE>(a, source, blockIdx.x, [] {
+    cg::this_grid().sync();
+    return true;
+  });
 }
 
 // Several buckets at once, each by its own part of a cooperative grid: a bucket of
@@ -1231,7 +1235,8 @@ topk_select_kernel(const TopkArgs a, const __grid_constant__ Source source) {
 // (2.56e7 elements in 11 buckets: 547 -> 210 us a pass, in 25: 727 -> 206; 2e6 in
 // four: 93 -> 42).
 // The parts do not wait for one another.  Their barrier counts arrivals; all CTAs
-// are resident, and the wait is bounded (run out: the sticky fault word).
+// are resident, and the wait is bounded: one that runs out sets the sticky fault word
+// (sgb_sparse_faults) and marks the barrier, and the part's CTAs leave.
 struct TopkBuckets {
   int count;
   unsigned first_cta[kBuckets + 1];
@@ -1262,21 +1267,24 @@ topk_buckets_kernel(const __grid_constant__ TopkBuckets b) {
   unsigned* const arrived = &a.ws.counters->arrived;
   unsigned target = 0;
   topk_select<MODE>(a, source, blockIdx.x - b.first_cta[g], [&] {
+    constexpr unsigned kLeft = 1u << 31, kMostPolls = 1u << 21;   // polls of half a microsecond and more
     target += a.work.grid;
     __syncthreads();
+    bool in = false;
     if (threadIdx.x == 0) {
       __threadfence();
       atomicAdd(arrived, 1u);
-      bool in = false;
-      for (unsigned q = 0; q < (1u << 22) && !in; ++q) {
-        unsigned v;
+      unsigned v = 0;
+      for (unsigned q = 0; q < kMostPolls && v < target; ++q)
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
-        in = v >= target;
+      in = v >= target && v < kLeft;
+      if (v < target) {
+        atomicOr(arrived, kLeft);
+        atomicOr(&g_topk_faults, 1u);
       }
-      if (!in) atomicOr(&g_topk_faults, 1u);
       __threadfence();
     }
-    __syncthreads();
+    return __syncthreads_or(in) != 0;
   });
 }
 
@@ -1774,6 +1782,11 @@ int sparse_dense_buckets(const int* payload, int known, const int* nnz_dev, cons
                           update ? &joint : nullptr);
 }
 
+int sparse_faults(unsigned* flags) {
+  const cudaError_t e = cudaMemcpyFromSymbol(flags, g_topk_faults, sizeof(unsigned));
+  return e == cudaSuccess ? SGB_OK : note_cuda_error(e);
+}
+
 bool sparse_selects_from(float* const* tensors, const size_t* sizes, size_t count, const float* acc) {
   Gradient g;
   return gather(&g, tensors, sizes, count, acc);
@@ -1896,6 +1909,8 @@ int sgb_sparse_topk_f32(const float* g, float* acc, float* sum_scratch, size_t n
   source.n = n;
   return topk_launch(source, acc, k, mode, idx_out, val_out, ws, ws_bytes, as_stream(stream));
 }
+
+int sgb_sparse_faults(unsigned* flags) { return flags ? sparse_faults(flags) : SGB_ERR_NULL; }
 
 int sgb_scatter_add_f32(const int32_t* idx, const float* val, size_t count,
                         const int32_t* count_dev, float* dst, size_t n, void* stream) {

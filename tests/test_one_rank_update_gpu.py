@@ -3,6 +3,8 @@ in one pass (half precision), or in the kernel that writes the dense gradients
 (sparse): the same bits in gradients, parameters, momentum and residuals as the
 call-by-call path, which a generator takes; and that path wherever an optimizer
 or a call of its own is to be used."""
+import ctypes
+
 import pytest
 import torch
 
@@ -101,3 +103,70 @@ def test_a_captured_update(comm):
         torch.cuda.synchronize()
         assert same(live, want), (method, kw)
         del graph
+
+
+# Larger lists: chunks drawn from a part's ticket (6e6 elements in all), runs of four
+# tiles and the sampled bound (from 9.7e6), one bucket a fifth of the others.
+WIDE = [([190003, 1900001, 333] * 3, 500000), ([2100000, 57000, 1] * 11, 1 << 21), ([4100000, 4100000, 500000, 400000, 4100000], 1 << 19)]
+
+
+def bucket_sizes(sizes, threshold):
+    out, held = [], 0
+    for n in sizes:
+        if n > threshold:
+            out.append(n)
+            continue
+        held += n
+        if held > threshold:
+            out.append(held)
+            held = 0
+    return out + [held] * (held > 0)
+
+
+def gradients(values, sizes, threshold, g):
+    n, dev = sum(sizes), torch.device("cuda")
+    flat = torch.randn(n, device=dev, generator=g)
+    if values == "small":                        # every integer-truncated key is 0
+        flat.mul_(1e-2)
+    if values == "ties":                         # a crowded bin
+        flat.round_()
+    out = list(flat.split(sizes))
+    if values == "misleading":
+        # large where the sample looks (128 elements at the start of each warp's share of the bucket) and
+        # nowhere else: fewer than k lie above the bound that it gives
+        ctas, total = 4 * torch.cuda.get_device_properties(0).multi_processor_count, sum(sizes)
+        for i, size in enumerate(sizes):
+            if size > threshold:
+                share = max(1, (ctas - len(bucket_sizes(sizes, threshold))) * size // total)
+                at = torch.arange(size, device=dev) % (size // (8 * share)) < 128
+                out[i] = torch.where(at, out[i] * 100, out[i] * 0.01)
+    return [t.clone() for t in out]
+
+
+@pytest.mark.parametrize("sizes,threshold", WIDE)
+@pytest.mark.parametrize("spars", [0.003, 0.04, 0.2])           # the sample is for shares up to a twelfth
+@pytest.mark.parametrize("mode", ["magnitude", "compat"])
+@pytest.mark.parametrize("values", ["normal", "small", "ties", "misleading"])
+def test_joint_selection_of_large_lists(comm, sizes, threshold, spars, mode, values):
+    from singa_b200 import _lib
+    from singa_b200.opt import SGD, DistOpt
+    comm.set_topk_mode(mode)
+    try:
+        sides = []
+        for as_list in (True, False):
+            g = torch.Generator(device="cuda").manual_seed(3)
+            opt = DistOpt(SGD(**OPTIONS[0]), communicator=comm)
+            params, grads = [torch.zeros(n, device="cuda") for n in sizes], []
+            for _ in range(2):
+                grads = gradients(values, sizes, threshold, g)
+                triples = [("p%d" % i, p, d) for i, (p, d) in enumerate(zip(params, grads))]
+                opt.backward_and_sparse_update(triples if as_list else (t for t in triples), threshold=threshold,
+                                               spars=spars, topK=True)
+            sides.append(grads + params + [opt.opt.moments["p%d" % i] for i in range(len(sizes))] + opt.gradAccumulation)
+        torch.cuda.synchronize()
+        assert same(*sides)
+        faults = ctypes.c_uint(1)
+        _lib.call("sgb_sparse_faults", ctypes.byref(faults))
+        assert faults.value == 0
+    finally:
+        comm.set_topk_mode("magnitude")
