@@ -270,7 +270,7 @@ rowmax_kernel(const float* __restrict__ M, float* __restrict__ v, size_t nrow, s
 // written to pool_dx as well.  Windows do not overlap: an element finds its
 // window's first maximum in the window's two rows (the other row's vector is a
 // neighbour's, so it comes from L1).  Same values and order as the three calls.
-template <bool VEC>
+// Planes whose width is a multiple of four only.
 struct Pool22 {
   int W, OH, OW;
   FastDiv width;
@@ -287,7 +287,7 @@ struct Pool22 {
       }
     return at;
   }
-  // Gradient of the unit at element `pos` of plane `plane`, whose offset is plane0.
+  // Gradient of the vector at element `pos` of plane `plane`, whose offset is plane0.
   __device__ __forceinline__ float4 unit(const float* __restrict__ px, const float* __restrict__ dy, size_t plane,
                                          size_t plane0, int pos) const {
     const int h = static_cast<int>(width.quot(static_cast<unsigned>(pos))), w = pos - h * W, oh = h >> 1, r = h & 1;
@@ -295,19 +295,13 @@ struct Pool22 {
     if (oh >= OH) return g;                          // a last row that no window covers
     const float* row = px + plane0 + static_cast<size_t>(h - r) * W + w;
     const float* gp = dy + (plane * OH + oh) * OW + (w >> 1);
-    if (VEC) {
-      const float4 a = *reinterpret_cast<const float4*>(row), b = *reinterpret_cast<const float4*>(row + W);
-      const float g0 = gp[0], g1 = gp[1];
-      const int at0 = winner(a.x, a.y, b.x, b.y), at1 = winner(a.z, a.w, b.z, b.w);
-      g.x = 0.0f + (at0 == 2 * r ? g0 : 0.0f);
-      g.y = 0.0f + (at0 == 2 * r + 1 ? g0 : 0.0f);
-      g.z = 0.0f + (at1 == 2 * r ? g1 : 0.0f);
-      g.w = 0.0f + (at1 == 2 * r + 1 ? g1 : 0.0f);
-    } else if ((w >> 1) < OW) {
-      const int k = w & 1;
-      const float* cell = row - k;
-      g.x = 0.0f + (winner(cell[0], cell[1], cell[W], cell[W + 1]) == 2 * r + k ? gp[0] : 0.0f);
-    }
+    const float4 a = *reinterpret_cast<const float4*>(row), b = *reinterpret_cast<const float4*>(row + W);
+    const float g0 = gp[0], g1 = gp[1];
+    const int at0 = winner(a.x, a.y, b.x, b.y), at1 = winner(a.z, a.w, b.z, b.w);
+    g.x = 0.0f + (at0 == 2 * r ? g0 : 0.0f);
+    g.y = 0.0f + (at0 == 2 * r + 1 ? g0 : 0.0f);
+    g.z = 0.0f + (at1 == 2 * r ? g1 : 0.0f);
+    g.w = 0.0f + (at1 == 2 * r + 1 ? g1 : 0.0f);
     return g;
   }
 };
@@ -315,7 +309,7 @@ template <bool VEC, bool RELU, bool POOL = false>
 __global__ void __launch_bounds__(kBlock)
 chansum_kernel(const float* __restrict__ dy, const float* __restrict__ x, float* __restrict__ dx,
                float* __restrict__ out, int N, int C,
-               int HW, int per_slice, int slices, bool clustered, const Pool22<VEC> pool,
+               int HW, int per_slice, int slices, bool clustered, const Pool22 pool,
                const float* __restrict__ pool_x, float* __restrict__ pool_dx) {
   __shared__ float sm[32];
   __shared__ float part[kMaxCluster];
@@ -362,9 +356,7 @@ chansum_kernel(const float* __restrict__ dy, const float* __restrict__ x, float*
       }
       acc += (v.x + v.y) + (v.z + v.w);
     } else {
-      float v;
-      if (POOL) pool_dx[at] = v = pooled.x;
-      else v = dy[at];
+      float v = dy[at];
       if (RELU) {
         v = x[at] > 0.f ? v : 0.f;
         dx[at] = v;
@@ -493,13 +485,12 @@ int channel_sums(const float* dy, const float* x, float* dx, float* db, int N, i
   const int per_slice = static_cast<int>(ceil_div(total, slices));
   if (slices == 1) clustered = false;     // the CTA's sum is the result
   float* out = clustered || slices == 1 ? db : static_cast<float*>(ws);
-  auto go = [&](auto v) {
-    constexpr bool kVec = decltype(v)::value;
-    const Pool22<kVec> p{pool.W, HW / pool.W / 2, pool.W / 2, FastDiv(static_cast<unsigned>(pool.W))};
-    return launch_ex(chansum_kernel<kVec, RELU, POOL>, dim3(static_cast<unsigned>(slices) * C), dim3(kBlock), 0, s,
-                     clustered ? slices : 0, true, dy, x, dx, out, N, C, HW, per_slice, slices, clustered, p, pool.x, pool.dx);
+  const Pool22 p{pool.W, HW / pool.W / 2, pool.W / 2, FastDiv(static_cast<unsigned>(pool.W))};
+  auto go = [&](auto kernel) {
+    return launch_ex(kernel, dim3(static_cast<unsigned>(slices) * C), dim3(kBlock), 0, s, clustered ? slices : 0, true,
+                     dy, x, dx, out, N, C, HW, per_slice, slices, clustered, p, pool.x, pool.dx);
   };
-  const int st = vec ? go(std::true_type{}) : go(std::false_type{});
+  const int st = POOL || vec ? go(chansum_kernel<true, RELU, POOL>) : go(chansum_kernel<false, RELU>);
   if (st != SGB_OK || out == db) return st;
   return launch_ex(chansum_finish_kernel, dim3(static_cast<unsigned>(ceil_div(C, 128))), dim3(128), 0, s, 0, true,
                    static_cast<const float*>(out), db, C, slices);
@@ -602,15 +593,28 @@ int sgb_maxpool_relu_backward_conv_bias_f32(const float* pool_x, const float* po
                                             const float* x, float* dx, float* db, void* ws, size_t ws_bytes,
                                             void* stream) {
   const int HW = H > 0 && W > 0 && static_cast<long long>(H) * W <= 0x7fffffffLL ? H * W : 0;
-  const bool vec = HW % 4 == 0 && aligned16(dx);       // how the sums are formed
-  // One launch and one read of the pooling's gradient less: 64x32x24x24 7.5 -> 6.0 us,
-  // 128x32x24x24 13.2 -> 9.1, 512x64x8x8 10.1 -> 8.2, 512x8x24x24 (2.4e6) 26.3 -> 24.1;
-  // but the pooling's own kernel reads whole rows, channel after channel, which
-  // counts from there on: 256x64x24x24 (9.4e6 elements) 33.3 -> 36.3.
-  const bool pays = static_cast<long long>(N) * C * HW <= 4000000;
-  if (pays && kh == 2 && kw == 2 && sh == 2 && sw == 2 && ph == 0 && pw == 0 && N > 0 && C > 0 && H >= 2 && W >= 2 && HW &&
-      pool_x && dy && pool_dx && x && dx && db &&
-      (!vec || (W % 4 == 0 && aligned16(pool_x) && aligned16(pool_dx) && aligned16(x))))
+  // One launch and one read of the pooling's gradient less, for the winners found
+  // twice and in the order of the channel sums, where the pooling's own kernel reads
+  // whole rows.  It pays while a CTA's threads have their few vectors in flight at once
+  // and the grid is one wave (elements per CTA, CTAs: the two calls / one, with the
+  // operands in L2, as a step of small layers has them, and from DRAM):
+  //   1024, 64     16x64x8x8     3.0 / 2.2    2.9 / 2.0
+  //   2304, 256    32x32x24x24   5.8 / 4.8    6.3 / 6.4
+  //   4608, 256    64x32x24x24   7.7 / 6.5    8.9 / 9.5
+  //   4608, 512    256x64x12x12 11.6 / 9.5   11.9 / 11.7
+  //   2304, 1024   32x128x24x24  9.0 / 11.8   9.9 / 14.2
+  //   9216, 64     128x8x24x24   7.7 / 8.0    9.4 / 13.6
+  //   9216, 256    128x32x24x24 13.7 / 9.5   13.7 / 16.3
+  //   36864, 96    512x12x24x24 19.1 / 25.6  29.4 / 49.8
+  // and not with single accesses (64x32x13x13 8.1 / 10.2, 256x8x15x15 13.5 / 21.9).
+  bool clustered, pays = kh == 2 && kw == 2 && sh == 2 && sw == 2 && ph == 0 && pw == 0 && N > 0 && C > 0 && H >= 2 &&
+                         HW && W % 4 == 0 && pool_x && dy && pool_dx && x && dx && db && aligned16(pool_x) &&
+                         aligned16(pool_dx) && aligned16(x) && aligned16(dx) && C <= 65535;
+  if (pays) {
+    const long long slices = chan_slices(N, C, HW, &clustered);
+    pays = static_cast<long long>(N) * HW <= 4608 * slices && slices * C <= 4LL * sm_count();
+  }
+  if (pays)
     return channel_sums<true, true>(dy, x, dx, db, N, C, HW, ws, ws_bytes, as_stream(stream), PoolOf{pool_x, pool_dx, W});
   const int st = sgb_maxpool_backward_f32(pool_x, pool_y, dy, pool_dx, N, C, H, W, kh, kw, ph, pw, sh, sw, stream);
   return st != SGB_OK ? st : sgb_relu_backward_conv_bias_f32(pool_dx, x, dx, db, N, C, H * W, ws, ws_bytes, stream);
