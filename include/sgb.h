@@ -726,6 +726,9 @@ int sgb_comm_sparsification_buckets(sgb_comm *c, void *const *tensors, const siz
  * kernel that writes the dense gradients.  The update has to run on the
  * communicator's stream, so it is complete behind sgb_comm_wait.  One rank;
  * SGB_ERR_UNSUPPORTED, and nothing done, where it takes separate calls. */
+/* (0 of the next call: it would not take such a list, by sizes and places alone.) */
+int sgb_comm_sparse_update_takes(const sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
+                                 size_t nbuckets, int topk);
 int sgb_comm_sparse_update(sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
                            float *const *accumulations, size_t nbuckets, float spars, int topk, void *const *params,
                            void *const *moments, float lr, float momentum, float dampening, float weight_decay,

@@ -145,6 +145,11 @@ class Communicator(object):
         takes separate calls: more ranks, profiling, other types."""
         return _n.comm_update_half(self._ptr, params, grads, moments, threshold, hyper)
 
+    def takesSparseUpdate(self, triples, threshold, topK):
+        """Whether sparseUpdate would take the buckets of these (name, param, grad)
+        triples, by sizes and places alone: asked before they are prepared for it."""
+        return _n.comm_sparse_update_takes(self._ptr, triples, threshold, topK)
+
     def sparseUpdate(self, buckets, residuals, params, moments, spars, topK, hyper):
         """Sparsification of buckets that all exist, and the SGD update of their
         parameters in the kernel that writes the dense gradients; complete behind

@@ -952,6 +952,22 @@ int sgb_comm_sparsification_buckets(sgb_comm* c, void* const* tensors, const siz
   return threshold_buckets(c, list, threshold, nullptr, sgb::as_stream(compute_stream));
 }
 
+// Which lists of one rank the joint call takes.  Beyond that many elements by threshold
+// the update has enough to read to cover its own latency, and gains nothing from the
+// dense sum's tiles (2.2e6 elements 27.9 -> 23.2 us a pass, 2.56e7 in 11 buckets
+// 180.4 -> 181.4).
+static bool sparse_update_pays(size_t elements, size_t, size_t, int topk) { return topk || elements <= 16000000; }
+
+int sgb_comm_sparse_update_takes(const sgb_comm* c, void* const* tensors, const size_t* sizes, const size_t* counts,
+                                 size_t nbuckets, int topk) {
+  if (!c || !tensors || !sizes || !counts || c->world != 1 || c->profiling) return 0;
+  size_t count = 0;
+  for (size_t k = 0; k < nbuckets; ++k) count += counts[k];
+  return sparse_update_pays(total_of(sizes, count), count, nbuckets, topk) &&
+         (!topk || nbuckets == 1 ||
+          sgb::sparse_topk_buckets_may(reinterpret_cast<float* const*>(tensors), sizes, counts, nbuckets));
+}
+
 int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* sizes, const size_t* counts,
                            float* const* accumulations, size_t nbuckets, float spars, int topk, void* const* params,
                            void* const* moments, float lr, float momentum, float dampening, float weight_decay,
@@ -968,12 +984,7 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
   cudaStream_t compute = sgb::as_stream(compute_stream);
   const sgb::SparseUpdate update{&sgd, reinterpret_cast<float* const*>(params),
                                  sgd.use_momentum ? reinterpret_cast<float* const*>(moments) : nullptr};
-  size_t elements = 0;
-  for (size_t k = 0; k < total; ++k) elements += sizes[k];
-  // Beyond that the update has enough to read to cover its own latency, and gains
-  // nothing from the dense sum's tiles (2.2e6 elements 27.9 -> 23.2 us a pass,
-  // 2.56e7 in 11 buckets 180.4 -> 181.4).
-  if (!topk && elements > 16000000) return SGB_ERR_UNSUPPORTED;
+  if (!sparse_update_pays(total_of(sizes, total), total, nbuckets, topk)) return SGB_ERR_UNSUPPORTED;
   if (!topk) return threshold_buckets(c, list, spars, &update, compute);
   for (const sgb::SparseBucket& b : list)
     if (!sgb::sparse_selects_from(b.tensors, b.sizes, b.count, b.acc)) return SGB_ERR_UNSUPPORTED;

@@ -1725,6 +1725,22 @@ static bool topk_plan(const SparseBucket* buckets, const size_t* ks, size_t coun
   return true;
 }
 
+bool sparse_topk_buckets_may(float* const* tensors, const size_t* sizes, const size_t* counts, size_t nbuckets) {
+  if (nbuckets < 2 || nbuckets > kBuckets) return false;
+  size_t span = 0, pieces = 0, t = 0;
+  for (size_t k = 0; k < nbuckets; ++k) {
+    const float* end = nullptr;
+    for (const size_t last = t + counts[k]; t < last; ++t) {
+      if (!sizes[t]) continue;
+      pieces += tensors[t] != end;                     // back to back with the one before: the same piece
+      end = tensors[t] + sizes[t];
+      span += sizes[t];
+    }
+    span = (span + kTile - 1) / kTile * kTile;
+  }
+  return span <= kMaxBucketSpan && pieces <= kPieces;
+}
+
 size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode) {
   TopkBuckets b;
   size_t bytes = 0, sent = 0;

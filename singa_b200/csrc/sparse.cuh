@@ -47,6 +47,8 @@ struct SparseUpdate {
 // Top-K of several buckets (the first ks[k] of bucket k by size) by one launch, into
 // a payload of the same joint space; *sent: its length.  sparse_topk_buckets_bytes:
 // of workspace, 0 where it takes a launch per bucket (fewer than two, more than 32).
+// sparse_topk_buckets_may: by sizes and places alone, before anything is prepared.
+bool sparse_topk_buckets_may(float* const* tensors, const size_t* sizes, const size_t* counts, size_t nbuckets);
 size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode);
 int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
                         void* ws, size_t ws_bytes, cudaStream_t s);

@@ -826,6 +826,42 @@ PyObject* py_comm_update_half(Args a, Py_ssize_t) {
   });
   return PyBool_FromLong(st == SGB_OK);
 }
+// (communicator, list of (name, param, grad), bucket threshold, topk) -> worth preparing?
+PyObject* py_comm_sparse_update_takes(Args a, Py_ssize_t) {
+  if (!PyList_Check(a[1])) Py_RETURN_FALSE;
+  const double threshold = real(a[2]);
+  const int topk = truth(a[3]);
+  std::vector<void*> ptrs, open;
+  std::vector<size_t> sizes, counts, open_sizes;
+  size_t held = 0;
+  auto flush = [&] {                   // large tensors come before a bucket that is still open
+    ptrs.insert(ptrs.end(), open.begin(), open.end());
+    sizes.insert(sizes.end(), open_sizes.begin(), open_sizes.end());
+    counts.push_back(open.size());
+    open.clear();
+    open_sizes.clear();
+    held = 0;
+  };
+  for (Py_ssize_t k = 0; k < PyList_GET_SIZE(a[1]); ++k) {
+    PyObject* t = PyList_GET_ITEM(a[1], k);
+    if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 3 || !THPVariable_Check(PyTuple_GET_ITEM(t, 2))) Py_RETURN_FALSE;
+    const Tensor& g = THPVariable_Unpack(PyTuple_GET_ITEM(t, 2));
+    if (!g.is_cuda() || g.scalar_type() != at::kFloat) Py_RETURN_FALSE;
+    if (static_cast<double>(count(g)) > threshold) {
+      ptrs.push_back(raww(g));
+      sizes.push_back(count(g));
+      counts.push_back(1);
+      continue;
+    }
+    open.push_back(raww(g));
+    open_sizes.push_back(count(g));
+    held += count(g);
+    if (static_cast<double>(held) > threshold) flush();
+  }
+  if (!open.empty()) flush();
+  return PyBool_FromLong(
+      sgb_comm_sparse_update_takes(comm(a[0]), ptrs.data(), sizes.data(), counts.data(), counts.size(), topk));
+}
 // (communicator, buckets, residuals, params, moments | None, spars, topk, hyper) -> done?
 PyObject* py_comm_sparse_update(Args a, Py_ssize_t) {
   std::vector<void*> ptrs;
@@ -1265,7 +1301,7 @@ PyMethodDef kMethods[] = {
     METHOD(bn_backward, 9), METHOD(bn_add_relu_backward, 10), METHOD(pool_forward, 5), METHOD(pool_backward, 5),
     METHOD(pool_forward_argmax, 4), METHOD(pool_backward_argmax, 3), METHOD(sgd_multi, 9), METHOD(pack, 3), METHOD(unpack, 4),
     METHOD(comm_synch, 2), METHOD(comm_synch_half, 2), METHOD(comm_fused_synch, 3), METHOD(comm_fused_synch_half, 3),
-    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_update_half, 6), METHOD(comm_sparse_update, 8), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5), METHOD(program_captures, 1),
+    METHOD(comm_sparsify, 5), METHOD(comm_sparsify_begin, 5), METHOD(comm_sparsify_end, 1), METHOD(comm_sparsify_buckets, 4), METHOD(comm_sync_dense, 4), METHOD(comm_update_half, 6), METHOD(comm_sparse_update, 8), METHOD(comm_sparse_update_takes, 4), METHOD(comm_wait, 1), METHOD(program, 2), METHOD(run_program, 5), METHOD(program_captures, 1),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -385,6 +385,11 @@ class DistOpt(object):
         if corr and self.world_size == 1 and type(grad_stream) in _LISTS:
             joint = None if topK else self._whole("joint")
             update = self._with_update("sparse", grad_stream)
+            takes = getattr(self.communicator, "takesSparseUpdate", None)
+            if update is not None and takes is not None:
+                grad_stream = list(grad_stream)
+                if not takes(grad_stream, threshold, topK):
+                    update = None
         updated = False
         try:
             if joint is not None or update is not None:

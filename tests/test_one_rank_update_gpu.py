@@ -160,6 +160,7 @@ def test_joint_selection_of_large_lists(comm, sizes, threshold, spars, mode, val
             for _ in range(2):
                 grads = gradients(values, sizes, threshold, g)
                 triples = [("p%d" % i, p, d) for i, (p, d) in enumerate(zip(params, grads))]
+                assert comm.takesSparseUpdate(triples, threshold, True)
                 opt.backward_and_sparse_update(triples if as_list else (t for t in triples), threshold=threshold,
                                                spars=spars, topK=True)
             sides.append(grads + params + [opt.opt.moments["p%d" % i] for i in range(len(sizes))] + opt.gradAccumulation)
@@ -170,3 +171,16 @@ def test_joint_selection_of_large_lists(comm, sizes, threshold, spars, mode, val
         assert faults.value == 0
     finally:
         comm.set_topk_mode("magnitude")
+
+
+def test_what_is_taken_is_known_ahead(comm):
+    """By size: 2 to 32 buckets of at most 256 pieces, or one.  By threshold: up to 16 million elements."""
+    for sizes, threshold, topk, want in (([300] * 33, 100, True, False), ([300] * 32, 100, True, True),
+                                         ([1 << 20] * 15, 1 << 21, False, True), ([1 << 20] * 16, 1 << 21, False, False),
+                                         ([1 << 22], 1 << 21, True, True), ([8] * 600, 1000, True, True)):
+        flat = torch.zeros(sum(sizes), device="cuda")      # back to back: one piece a bucket
+        grads = list(flat.split(sizes))
+        assert comm.takesSparseUpdate([("p", g, g) for g in grads], threshold, topk) is want, (len(sizes), topk)
+    apart = [torch.zeros(8, device="cuda") for _ in range(257)]
+    assert not comm.takesSparseUpdate([("p", g, g) for g in apart], 1000, True)
+    assert comm.takesSparseUpdate([("p", g, g) for g in apart[:-1]], 1000, True)

@@ -159,3 +159,27 @@ def test_a_function_put_into_the_class_is_called(owner, name, monkeypatch):
         assert called and not any(isinstance(s, tuple) for s in seen)
         called.clear()
         assert run(opt, method, **kw) == both
+
+
+def test_a_communicator_that_declines_by_sizes():
+    class Asked(Comm):
+        """Asked first, before anything is prepared for the call."""
+        answer = False
+
+        def takesSparseUpdate(self, triples, threshold, topK):
+            self.seen.append(("asked", [g.numel() for _, _, g in triples], threshold))
+            return self.answer
+    opt = DistOpt(SGD(lr=0.0), communicator=Asked())
+    opt.opt._moments_of = lambda *a: opt.communicator.seen.append("prepared")
+    with pytest.raises(ValueError):                      # the separate update: no CPU path
+        run(opt, "backward_and_sparse_update", iter(triples()), spars=0.1, topK=True)
+    assert opt.communicator.seen == [("asked", [30, 4, 50, 5], 20), "begin", "begin", "end", "begin", "end", "end",
+                                     "wait", "prepared"]
+    opt.communicator.answer = True
+    assert [s[0] for s in run(opt, "backward_and_sparse_update", iter(triples()), spars=0.1, topK=True)][:3] == \
+        ["asked", "p", "sparse"]
+
+
+def test_no_communicator_takes_nothing():
+    assert _lib.lib().sgb_comm_sparse_update_takes(None, None, None, None, 0, 0) == 0
+    assert _lib.native.comm_sparse_update_takes(None, [("p", 1, 2)], 20, True) is False
