@@ -952,11 +952,18 @@ int sgb_comm_sparsification_buckets(sgb_comm* c, void* const* tensors, const siz
   return threshold_buckets(c, list, threshold, nullptr, sgb::as_stream(compute_stream));
 }
 
-// Which lists of one rank the joint call takes.  Beyond that many elements by threshold
-// the update has enough to read to cover its own latency, and gains nothing from the
-// dense sum's tiles (2.2e6 elements 27.9 -> 23.2 us a pass, 2.56e7 in 11 buckets
-// 180.4 -> 181.4).
-static bool sparse_update_pays(size_t elements, size_t, size_t, int topk) { return topk || elements <= 16000000; }
+// Which lists of one rank the joint call takes.  Several buckets by size: whatever
+// one launch can, since their selections are one launch then (us a pass, a call per
+// bucket and update / joint: 4 buckets of 12 tensors, 2e6 elements in all 70.9 / 32.6, 12
+// of 160, 2.4e7 355.3 / 186.7).  Else only the update is saved a launch and a read of
+// the gradients, for tiles in which a tensor's update waits for its neighbour's and a
+// longer list of arguments: the line is at few tensors and, by threshold, few elements.
+//   by size, one bucket of 1e6: in 1 tensor 30.0 / 21.8, 12 35.5 / 32.7, 50 33.8 / 53.5
+//   by threshold, 1e6:   in 1 tensor 20.6 / 16.4, 5 21.3 / 18.1, 12 22.8 / 24.8, 50 27.1 / 31.3
+//   in 1 tensor 3e6 32.5 / 30.8, 8e6 67.8 / 69.0; in 6 3.4e6 35.4 / 33.2, 5.8e6 54.6 / 55.3
+static bool sparse_update_pays(size_t elements, size_t tensors, size_t nbuckets, int topk) {
+  return topk ? nbuckets > 1 || tensors <= 16 : tensors <= 8 && elements <= 4000000;
+}
 
 int sgb_comm_sparse_update_takes(const sgb_comm* c, void* const* tensors, const size_t* sizes, const size_t* counts,
                                  size_t nbuckets, int topk) {

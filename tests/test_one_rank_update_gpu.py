@@ -174,9 +174,10 @@ def test_joint_selection_of_large_lists(comm, sizes, threshold, spars, mode, val
 
 
 def test_what_is_taken_is_known_ahead(comm):
-    """By size: 2 to 32 buckets of at most 256 pieces, or one.  By threshold: up to 16 million elements."""
+    """By size: 2 to 32 buckets of at most 256 pieces, or one of 16 tensors.  By threshold: at most 8 tensors and 4 million elements."""
     for sizes, threshold, topk, want in (([300] * 33, 100, True, False), ([300] * 32, 100, True, True),
-                                         ([1 << 20] * 15, 1 << 21, False, True), ([1 << 20] * 16, 1 << 21, False, False),
+                                         ([500000] * 8, 1 << 21, False, True), ([400000] * 9, 1 << 21, False, False),
+                                         ([1 << 20] * 4, 1 << 21, False, False), ([50] * 16, 1000, True, True), ([50] * 17, 1000, True, False),
                                          ([1 << 22], 1 << 21, True, True), ([8] * 600, 1000, True, True)):
         flat = torch.zeros(sum(sizes), device="cuda")      # back to back: one piece a bucket
         grads = list(flat.split(sizes))
