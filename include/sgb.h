@@ -394,10 +394,14 @@ int sgb_bn_backward_faults(unsigned *flags);
  * channels that do not fit a thread-block cluster).  mask: 0 none, 1 ReLU
  * input, 2 ReLU bit record. */
 int sgb_bn_backward_stream_plan(int N, int C, int HW, int mask, int *plan6);
-/* 1 if a backward call on 16-byte aligned tensors takes that form (the plane is
- * a multiple of four floats and no cluster holds a channel), else 0.  Such a
- * launch draws one of eight counter tables: a captured one keeps its own. */
+/* 1 if a backward call on 16-byte aligned tensors, whose workspace holds partial
+ * sums only (64 pairs of floats a channel), takes that form (the plane is a multiple
+ * of four floats and no cluster holds a channel), else 0.  Such a launch draws one of
+ * eight counter tables: a captured one keeps its own. */
 int sgb_bn_backward_streams(int N, int C, int HW, int mask);
+/* The same for a workspace of ws_bytes: with what sgb_bn_backward_workspace_bytes
+ * asks for, large calls visit their data twice instead and draw no table. */
+int sgb_bn_backward_draws_table(int N, int C, int HW, int mask, size_t ws_bytes);
 /* Batch-norm backward for callers that can neither allocate device memory nor
  * hand in a workspace.  (No counterpart in the reference: this entry point
  * exists only in this library.)  Typical callers: an operator running inside

@@ -1709,6 +1709,12 @@ int sgb_bn_backward_streams(int N, int C, int HW, int mask) {
   return bn_stream_plan(N, C, HW, mask, &plan) ? 1 : 0;
 }
 
+int sgb_bn_backward_draws_table(int N, int C, int HW, int mask, size_t ws_bytes) {
+  if (!sgb_bn_backward_streams(N, C, HW, mask)) return 0;
+  const size_t need = revisit_pays(N, C, HW, true, false) ? bn_revisit_workspace_bytes(N, C, HW) : 0;
+  return need == 0 || ws_bytes < need;
+}
+
 int sgb_bn_backward_stream_plan(int N, int C, int HW, int mask, int* plan6) {
   if (!plan6) return SGB_ERR_NULL;
   BnStreamPlan p;

@@ -417,13 +417,14 @@ class HotPathGPU(object):
         # made one by one: collectives (a graph that holds them keeps the communicator
         # from closing), the sparse exchange (more ranks wait for counts on the host)
         # and the streaming batch-norm form (each launch draws one of eight counter
-        # tables, a captured one would keep its own).
+        # tables, a captured one would keep its own), where a call takes it.
         single = self.comm is not None and (self.comm.world_size > 1 or self.dist_option not in ("plain", "half"))
         masks = {"bn_bwd": 0, "bn_add_relu_bwd": 0, "bn_relu_bwd": 1, "bn_relu_mask_bwd": 2}
         for op in self.plan["ops"]:
             if op.kind in masks:
                 n, c, h, w = self.t[op.args["x"]].shape
-                single = single or self.lib.sgb_bn_backward_streams(n, c, h * w, masks[op.kind]) != 0
+                single = single or \
+                    self.lib.sgb_bn_backward_draws_table(n, c, h * w, masks[op.kind], self.ws.numel()) != 0
         self._program = _lib.native.program(prog, None if self.comm is None else self.comm._h.value, not single)
 
     def _sgd_call(self, tables, stream):

@@ -34,3 +34,15 @@ def test_the_query_follows_the_capacity_of_a_cluster():
 @pytest.mark.parametrize("args", [(0, 4, 16, 0), (4, 0, 16, 0), (4, 4, 0, 0), (32, 64, 12544, 3), (32, 64, 12544, -1)])
 def test_no_call_no_stream(args):
     assert _lib.lib().sgb_bn_backward_streams(*args) == 0
+
+
+@pytest.mark.parametrize("shape", [(32, 64, 12544), (9, 64, 12544), (64, 8, 3136), (16, 8, 6400), (65, 64, 3136), (32, 256, 3136)])
+def test_a_call_that_visits_its_data_twice_draws_no_table(shape):
+    """From 4 million elements on, given the workspace for it; below, the streaming form is what it was."""
+    lib = _lib.lib()
+    for mask in (0, 1, 2):
+        streams = lib.sgb_bn_backward_streams(*shape, mask)
+        whole, sums = lib.sgb_bn_backward_workspace_bytes(*shape), 64 * shape[1] * 8
+        twice = shape[0] * shape[1] * shape[2] >= 4000000
+        assert lib.sgb_bn_backward_draws_table(*shape, mask, min(sums, whole - 1) if twice else sums) == streams
+        assert lib.sgb_bn_backward_draws_table(*shape, mask, whole) == (0 if twice else streams)

@@ -128,3 +128,17 @@ def test_a_closed_communicator_is_an_error():
     hp.update_on_arrival = False
     assert hp.run_step() > 0
     torch.cuda.synchronize()
+
+
+def test_a_step_with_layers_that_visit_their_data_twice_is_captured():
+    from singa_b200 import _lib
+    from singa_b200.hot_path import HotPathGPU
+    from singa_b200.resnet50_path import build_plan
+    steps = [HotPathGPU(build_plan(batch=9, image=224, fused=True), seed=3) for _ in range(2)]
+    steps[1].profile = True                     # never captured
+    for _ in range(5):
+        for hp in steps:
+            hp.run_step()
+    assert [_lib.native.program_captures(hp._program) for hp in steps] == [1, 0]
+    for a, b in zip(*map(parameters, steps)):
+        assert torch.equal(a, b)
