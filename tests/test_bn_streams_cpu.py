@@ -46,3 +46,14 @@ def test_a_call_that_visits_its_data_twice_draws_no_table(shape):
         twice = shape[0] * shape[1] * shape[2] >= 4000000
         assert lib.sgb_bn_backward_draws_table(*shape, mask, min(sums, whole - 1) if twice else sums) == streams
         assert lib.sgb_bn_backward_draws_table(*shape, mask, whole) == (0 if twice else streams)
+
+
+def test_a_recorded_step_has_room_for_its_largest_call():
+    from singa_b200.hot_path import workspace_bytes
+    from singa_b200.resnet50_path import build_plan
+    plan = build_plan(batch=2, image=64, fused=False)
+    assert workspace_bytes(plan) == 8 << 20
+    op = next(op for op in plan["ops"] if op.kind == "bn_bwd")
+    plan["tensors"][op.args["x"]] = plan["tensors"][op.args["x"]]._replace(shape=(300, 1300, 57, 57))
+    need = _lib.lib().sgb_bn_backward_workspace_bytes(300, 1300, 57 * 57)      # 1.27e9 elements of odd planes
+    assert workspace_bytes(plan) == need > 8 << 20
