@@ -30,8 +30,8 @@
 //              whose workspace is too small for the form below: persistent
 //              small CTAs take 50 KB items of a channel from a ticket counter and
 //              meet through counters in global memory (bn_stream.cu).
-// Ahead of them all, for large calls (revisit_pays): two visits to the data in one
-// kernel, the second out of L2 (bn_revisit.cu).
+// Ahead of them all, for large calls whose channels are not too large (revisit_pays):
+// two visits to the data in one kernel, the second out of L2 (bn_revisit.cu).
 //
 // Two passes (20 bytes of HBM traffic per element when the tensor does not fit
 // L2) for what is left: ragged planes too large for a cluster, misaligned
@@ -1435,10 +1435,27 @@ int takes_cluster(long long per_channel, bool vec, int C, int* per_cta) {
 //   24x64x71x71   (7.7e6)           40.0 / 28.1   27.6 / 23.7
 //   18x256x33x33  (5.0e6)           25.4 / 19.8   16.1 / 17.0
 //   24x1024x15x15 (5.5e6)           28.6 / 22.6   17.9 / 20.2
+// Two costs grow with the items of a channel: the lead of the first visit over the
+// second (what lies between them has to stay in L2), and every CTA's reading of all
+// the channel's sums.  Large channels therefore take the forms below, unless the
+// whole call is small (elements of a channel, of the call):
+//   64x12x224x224   3.2e6, 3.9e7  172.8 / 143.1   117.8 / 103.0
+//   80x20x224x224   4.0e6, 8.0e7  340.9 / 328.8   245.2 / 235.5
+//   1x8x2048x2048   4.2e6, 3.4e7  152.2 / 155.8   107.9 / 107.2
+//   1x4x2828x2828   8.0e6, 3.2e7  173.1 / 182.5   136.7 / 149.2
+//   4x1x4096x4096   6.7e7, 6.7e7  781.8 / 1482.6  695.8 / 1435.5
+//   128x3x224x224   6.4e6, 1.9e7  115.4 / 106.3    94.6 / 83.9
+//   1x1x4096x4096   1.7e7, 1.7e7  201.7 / 151.1   160.3 / 131.3
+// Odd planes have smaller items and a better form of two passes:
+//   16x32x223x223   8.0e5, 2.5e7  115.8 / 83.7     78.7 / 70.1
+//   2x16x723x723    1.0e6, 1.7e7   75.5 / 61.4     51.3 / 54.6
+//   32x16x223x223   1.6e6, 2.5e7  118.9 / 104.8    80.1 / 92.2
+//   6x8x597x599     2.1e6, 1.7e7   81.7 / 95.3     55.1 / 86.3
+//   32x3x397x397    5.0e6, 1.5e7   86.3 / 141.0    58.2 / 128.1
 inline bool revisit_pays(int N, int C, int HW, bool aligned, bool groups) {
-  const long long elements = static_cast<long long>(N) * C * HW;
-  if (HW % 4) return aligned && !groups && HW >= 2500 && elements >= 6000000;
-  return aligned && HW >= 8 && elements >= 4000000;
+  const long long channel = static_cast<long long>(N) * HW, elements = channel * C;
+  if (HW % 4) return aligned && !groups && HW >= 2500 && elements >= 6000000 && channel <= 1000000;
+  return aligned && HW >= 8 && elements >= 4000000 && (channel <= 4000000 || elements <= 20000000);
 }
 
 template <int MASK>

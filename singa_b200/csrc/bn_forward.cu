@@ -568,14 +568,21 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
 
 // One operand is little to overlap with, so only channels that leave clusters with
 // large shares or no place at all gain (us, the forms above and below / this one):
-//   32x64x112x112 61.5 / 41.3   32x256x56x56 44.5 / 42.4   32x64x56x56 14.9 / 14.2
-//   64x100x40x40  19.4 / 19.6   32x512x28x28 25.3 / 26.6   10x256x52x52 15.3 / 15.9
-//   32x64x111x111 99.1 / 53.1   32x128x57x57 37.3 / 28.7   24x64x71x71 24.4 / 18.8
-//   16x1024x13x13 14.1 / 14.5 (2.8e6 elements)
+//   32x64x112x112 61.5 / 41.3   32x64x56x56 14.9 / 14.2    64x100x40x40  19.4 / 19.6
+//   32x512x28x28 25.3 / 26.6    10x256x52x52 15.3 / 15.9   32x64x111x111 99.1 / 53.1
+//   32x128x57x57 37.3 / 28.7    24x64x71x71 24.4 / 18.8    16x1024x13x13 14.1 / 14.5
+// The lower line for whole vectors is from a layer's forward, ReLU and backward in
+// sequence: what the second visit leaves in L2 is x, and what comes next reads y
+// (elements of a channel: 69,000 134.3 / 136.7, 75,000 145.4 / 147.9, 88,000 149.7 /
+// 152.7, 100,000 154.2 / 147.9 and on 64 channels 42.3 / 39.5).
+// The upper lines are those of the backward (batchnorm.cu): 4.0e6 elements a channel,
+// 8.0e7 in all 175.8 / 172.1, 4.2e6 and 6.7e7 132.3 / 137.9, 8.0e6 and 3.2e7 103.8 /
+// 109.7, 1.7e7 and 1.7e7 141.8 / 101.5; odd planes 2.6e6 and 2.1e7 101.5 / 92.0, 2.9e6
+// and 3.5e7 142.0 / 156.5, 4.0e6 and 3.2e7 155.7 / 187.4.
 inline bool fwd_revisit_pays(int N, int C, int HW) {
-  const long long channel = static_cast<long long>(N) * HW;
-  if (HW % 4) return HW >= 2500 && channel * C >= 6000000;
-  return HW >= 2500 && channel >= 65536 && channel * C >= 6000000;
+  const long long channel = static_cast<long long>(N) * HW, elements = channel * C;
+  if (HW % 4) return HW >= 2500 && elements >= 6000000 && channel <= 2600000;
+  return HW >= 2500 && channel >= 96000 && elements >= 6000000 && (channel <= 4000000 || elements <= 20000000);
 }
 
 // SGB_ERR_WORKSPACE and nothing done where the workspace is too small or the problem too large.

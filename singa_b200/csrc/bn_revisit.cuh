@@ -6,8 +6,9 @@
 // i - delay: the sums of that item's channel have been published by then, and its
 // operands come from L2, where the first visit asked for them to be kept.  So HBM
 // sees every operand once, as if a channel were held on the chip, but nothing is
-// staged: thousands of small CTAs overlap loads, sums and stores, every SM slot is
-// used whatever the shape, and no channel is too large.
+// staged: thousands of small CTAs overlap loads, sums and stores, and every SM slot is
+// used whatever the shape.  A channel of very many items puts its visits too far apart
+// (revisit_pays and fwd_revisit_pays have the lines).
 //
 // What bounds it: HBM and the latency of a CTA's life (load, reduce, load again,
 // store), which the number of CTAs in flight has to cover.  A loop of persistent

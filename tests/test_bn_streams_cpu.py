@@ -57,3 +57,17 @@ def test_a_recorded_step_has_room_for_its_largest_call():
     plan["tensors"][op.args["x"]] = plan["tensors"][op.args["x"]]._replace(shape=(300, 1300, 57, 57))
     need = _lib.lib().sgb_bn_backward_workspace_bytes(300, 1300, 57 * 57)      # 1.27e9 elements of odd planes
     assert workspace_bytes(plan) == need > 8 << 20
+
+
+@pytest.mark.parametrize("shape, backward, forward", [
+    ((79, 20, 50176), True, True), ((80, 20, 50176), False, False), ((1, 4, 4000000), True, True), ((2, 2, 4000000), True, True),
+    ((4, 1, 1 << 24), False, False), ((1, 1, 1 << 24), True, True), ((20, 8, 49729), True, True), ((21, 8, 49729), False, True),
+    ((53, 8, 49729), False, False), ((1, 8, 1000001), False, True)])
+def test_very_large_channels_are_not_visited_twice(shape, backward, forward):
+    """Seen in the workspace that is asked for: an entry for each item of 3584 (odd planes: 2304) elements or,
+    where only the forward visits twice, of 6144 (3072)."""
+    n, c, hw = shape
+    whole = _lib.lib().sgb_bn_backward_workspace_bytes(n, c, hw)
+    items = lambda vec, odd: 16 * n * c * hw / (odd if hw % 4 else vec)   # noqa: E731
+    least = items(3584, 2304) if backward else items(6144, 3072) if forward else 64 * 8 * c
+    assert least * 0.99 <= whole <= least * 1.1, (whole, least)
