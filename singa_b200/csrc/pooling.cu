@@ -430,8 +430,11 @@ pool_k3s2p1_kernel(const StripArgs a) {
   // 29 KB in flight per SM where the rate takes 47.  32x64x112x112: forward 27.5 ->
   // 25.7 us, backward 48.1 -> 46.1, with the record 31.9 -> 28.7, average backward
   // 39.8 -> 32.7; two rows further ahead it is 26.7 and more.  The backward pass that
-  // finds its winners again has no registers to spare: not on small problems (8x64x
-  // 112x112 14.9 -> 15.2, 16x512x14x14 7.7 -> 8.2) and odd rows (111x111 49.8 -> 50.9).
+  // finds its winners again has no registers to spare: not on odd rows (111x111 49.8 ->
+  // 50.9) and small problems (16x512x14x14 7.7 -> 8.2; 64 channels of 112x112, 6.4e6
+  // elements 14.8 -> 15.1, 9.6e6 20.6 -> 20.6, 1.28e7 26.6 -> 26.2, 1.45e7 28.1 -> 28.7,
+  // 1.6e7 32.1 -> 31.2, 1.9e7 37.4 -> 36.0; 56x56 1.28e7 26.9 -> 26.3, 1.6e7 32.5 -> 31.3;
+  // 160x160 1.31e7 32.4 -> 34.2; 28x28 1.28e7 27.7 -> 27.8).
   const bool far = MODE != kMaxBwd || (VEC && static_cast<long long>(a.planes) * H * W >= 16000000);
   auto ahead = [&](int m) {
     if (!far || !active || m > last) return;
