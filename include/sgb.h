@@ -267,7 +267,8 @@ int sgb_relu_backward_conv_bias_f32(const float *dy, const float *x, float *dx, 
                                     void *ws, size_t ws_bytes, void *stream);
 /* The same behind a max pooling: sgb_maxpool_backward_f32(pool_x, pool_y, dy ->
  * pool_dx), whose result goes through the call above; one launch for windows of
- * 2x2 with stride 2 and no padding. */
+ * 2x2 with stride 2 and no padding where that is faster.  Neither dx nor db may lie
+ * in pool_x or dy. */
 int sgb_maxpool_relu_backward_conv_bias_f32(const float *pool_x, const float *pool_y, const float *dy, float *pool_dx,
                                             int N, int C, int H, int W, int kh, int kw, int ph, int pw, int sh, int sw,
                                             const float *x, float *dx, float *db, void *ws, size_t ws_bytes,
@@ -316,8 +317,9 @@ int sgb_softmax_cross_entropy_fused_f32(const float *logits, const int32_t *t,
                                         float *prob, float *loss, float *grad,
                                         void *stream);
 /* The same, then *total = the sum of the losses (sgb_sum_all_f32) and bias_grad =
- * the column sums of grad (sgb_sum_rows_f32): one or two launches, the same bits
- * as the three calls.  Workspace: what either sum needs. */
+ * the column sums of grad (sgb_sum_rows_f32): two launches instead of three where
+ * each sum is one, the same bits.  Neither total nor bias_grad may lie in loss or
+ * grad.  Workspace: what either sum needs. */
 int sgb_loss_head_f32(const float *logits, const int32_t *t, size_t batch, size_t dim,
                       float scale, float *prob, float *loss, float *grad, float *total,
                       float *bias_grad, void *ws, size_t ws_bytes, void *stream);
@@ -730,7 +732,9 @@ int sgb_comm_sparsification_buckets(sgb_comm *c, void *const *tensors, const siz
  * kernel that writes the dense gradients.  The update has to run on the
  * communicator's stream, so it is complete behind sgb_comm_wait.  One rank;
  * SGB_ERR_UNSUPPORTED, and nothing done, where it takes separate calls. */
-/* (0 of the next call: it would not take such a list, by sizes and places alone.) */
+/* (0 of the next call: it would not take such a list, by sizes and places alone; nor,
+ * by threshold, one of more than SGB_SPARSE_UPDATE_TENSORS tensors.) */
+#define SGB_SPARSE_UPDATE_TENSORS 8
 int sgb_comm_sparse_update_takes(const sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
                                  size_t nbuckets, int topk);
 int sgb_comm_sparse_update(sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,

@@ -962,7 +962,7 @@ int sgb_comm_sparsification_buckets(sgb_comm* c, void* const* tensors, const siz
 //   by threshold, 1e6:   in 1 tensor 20.6 / 16.4, 5 21.3 / 18.1, 12 22.8 / 24.8, 50 27.1 / 31.3
 //   in 1 tensor 3e6 32.5 / 30.8, 8e6 67.8 / 69.0; in 6 3.4e6 35.4 / 33.2, 5.8e6 54.6 / 55.3
 static bool sparse_update_pays(size_t elements, size_t tensors, size_t nbuckets, int topk) {
-  return topk ? nbuckets > 1 || tensors <= 16 : tensors <= 8 && elements <= 4000000;
+  return topk ? nbuckets > 1 || tensors <= 16 : tensors <= SGB_SPARSE_UPDATE_TENSORS && elements <= 4000000;
 }
 
 int sgb_comm_sparse_update_takes(const sgb_comm* c, void* const* tensors, const size_t* sizes, const size_t* counts,

@@ -831,6 +831,7 @@ PyObject* py_comm_sparse_update_takes(Args a, Py_ssize_t) {
   if (!PyList_Check(a[1])) Py_RETURN_FALSE;
   const double threshold = real(a[2]);
   const int topk = truth(a[3]);
+  if (!topk && PyList_GET_SIZE(a[1]) > SGB_SPARSE_UPDATE_TENSORS) Py_RETURN_FALSE;
   std::vector<void*> ptrs, open;
   std::vector<size_t> sizes, counts, open_sizes;
   size_t held = 0;

@@ -384,12 +384,12 @@ class DistOpt(object):
         joint = update = None
         if corr and self.world_size == 1 and type(grad_stream) in _LISTS:
             joint = None if topK else self._whole("joint")
-            update = self._with_update("sparse", grad_stream)
             takes = getattr(self.communicator, "takesSparseUpdate", None)
-            if update is not None and takes is not None:
+            if takes is not None and type(self.opt) is SGD:
                 grad_stream = list(grad_stream)
-                if not takes(grad_stream, threshold, topK):
-                    update = None
+                takes = takes(grad_stream, threshold, topK)
+            if takes is None or takes:
+                update = self._with_update("sparse", grad_stream)
         updated = False
         try:
             if joint is not None or update is not None:
