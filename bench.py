@@ -27,7 +27,7 @@ METRIC = "resnet50_backward_sync_update_images_per_sec"
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the batch-norm
 # backward kernels, averaged per call over one step, from the ncu capture
 # summarised in profiles/bench_resnet50_launch_list.md (fused / call-pattern plan).
-NCU_BN_TRAFFIC_PER_CALL = {True: 71.8e6, False: 61.6e6}
+NCU_BN_TRAFFIC_PER_CALL = {True: 71.8e6, False: 60.7e6}
 
 
 def _traffic_from_summary():
@@ -824,7 +824,7 @@ def main():
     achieved = bn_bytes / bn_ms / 1e6
     captured_plan = fused and not args.relu_mask
     roofline = {"bound": "hbm",
-                "kernel": "batch-norm backward (cluster, streaming and channel-group kernels: all 53 calls)",
+                "kernel": "batch-norm backward (two-visit, cluster, register and channel-group kernels: all 53 calls)",
                 "achieved": round(achieved, 1),
                 "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
                 "traffic": _traffic_from_summary()[fused] if (captured_plan or not fused) else None,
@@ -841,14 +841,14 @@ def main():
     check = {"max_rel_err": {k: float("%.3e" % max_over_ranks(v)) for k, v in worst.items()}, "ok": ok,
              "tolerance": "1e-5 fp32, 1e-3 x world fp16, relative to the largest expected sum"}
     tl = timeline(torch, path, comm)
-    launches_per_step = kernel_launches(path)
-    # sticky fault word of the streaming batch-norm kernel (bounded waits between its CTAs): 0 on every rank
+    launches_per_step = kernel_launches(path, torch)
+    # sticky fault word of the batch-norm kernels (bounded waits between their CTAs): 0 on every rank
     import ctypes
     flags = ctypes.c_uint(0)
     _lib.call("sgb_bn_backward_faults", ctypes.byref(flags))
     bn_faults = int(max_over_ranks(float(flags.value)))
     if bn_faults:
-        raise SystemExit("bench.py: the streaming batch-norm kernel recorded fault flags %d" % bn_faults)
+        raise SystemExit("bench.py: the batch-norm kernels recorded fault flags %d" % bn_faults)
 
     nvlink = None
     if multi:
@@ -949,41 +949,35 @@ def main():
     faulthandler.cancel_dump_traceback_later()
 
 
-def kernel_launches(path):
-    """Kernels of this library launched per step (NCCL's own are not counted).
-    Batch-norm backward is one launch, except for ragged planes of small calls
-    when a channel (x and dy of all samples) exceeds what a cluster of eight CTAs
-    can stage (8 x 100 KB): then it is the reduce + apply pair."""
-    per = {"sgb_relu_backward_f32": 1, "sgb_add_relu_backward_f32": 1, "sgb_binary_f32": 1,
-           "sgb_relu_backward_mask_f32": 1, "sgb_add_relu_backward_mask_f32": 1,
-           "sgb_maxpool_backward_f32": 1, "sgb_maxpool_backward_argmax_f32": 1,
-           "sgb_avgpool_backward_f32": 1, "sgb_softmax_rows_f32": 1, "sgb_cross_entropy_f32": 1,
-           "sgb_sum_all_f32": 1, "sgb_softmax_cross_entropy_bwd_f32": 1,
-           "sgb_softmax_cross_entropy_grad_f32": 1, "sgb_softmax_cross_entropy_fused_f32": 1,
-           "sgb_scalar_f32": 1, "sgb_sum_rows_f32": 1, "sgb_set_f32": 1, "sgb_conv_bias_backward_f32": 1,
-           "sgb_relu_backward_sum_rows_f32": 1, "sgb_relu_backward_conv_bias_f32": 1,
-           "sgb_maxpool_relu_backward_conv_bias_f32": 1, "sgb_loss_head_f32": 2}
+def kernel_launches(path, torch):
+    """Kernels of this library launched per step (NCCL's own are not counted): the
+    kernel nodes of a capture of the step that carry a name of this library."""
+    import ctypes as C
+
+    class KernelNode(C.Structure):
+        _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("smem", C.c_uint),
+                    ("params", C.c_void_p), ("extra", C.c_void_p)]
+    rt = C.CDLL("libcudart.so.12")               # the runtime that torch and libsgb.so share
+    graph, side = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side, capture_error_mode="thread_local"):
+        path.run_step()
+    torch.cuda.current_stream().wait_stream(side)
+    handle, count = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
+    if rt.cudaGraphGetNodes(handle, None, C.byref(count)):
+        raise SystemExit("bench.py: the step's graph has no list of nodes")
+    nodes = (C.c_void_p * count.value)()
+    rt.cudaGraphGetNodes(handle, nodes, C.byref(count))
     n = 0
-    for name, args in path.launched:
-        if name in ("sgb_bn_backward_f32", "sgb_bn_relu_backward_f32", "sgb_bn_relu_backward_mask_f32",
-                    "sgb_bn_add_relu_backward_f32"):
-            N, c, HW = args[-6:-3]          # (..., N, C, HW, workspace, workspace bytes, stream)
-            n += 2 if N * HW * 8 > 8 * 100 * 1024 and HW % 4 and (HW < 2500 or N * c * HW < 6000000) else 1
-        elif name == "sgb_unpack_f32":       # stand-in weight gradients: one launch per 72 tensors
-            n += (args[4] + 71) // 72
+    for node in nodes:
+        node, kind, k, name = C.c_void_p(node), C.c_int(), KernelNode(), C.c_char_p()
+        if rt.cudaGraphNodeGetType(node, C.byref(kind)) == 0 and kind.value == 0 and \
+                rt.cudaGraphKernelNodeGetParams(node, C.byref(k)) == 0 and \
+                rt.cudaFuncGetName(C.byref(name), C.c_void_p(k.func)) == 0:
+            n += b"3sgb" in (name.value or b"")  # the namespace, as names are mangled
         else:
-            n += per.get(name, 0)
-    if path.comm is not None:
-        for kind, idx in path.events:
-            if kind == "fused" and path.dist_option == "half":
-                n += 2 * ((len(idx) + 71) // 72)  # pack+cast and unpack+cast launches at flush
-            # fp32 buckets are contiguous arena slices: reduced in place, no pack / unpack
-            elif path.dist_option == "half":
-                n += 2                           # cast down, cast up
-    if getattr(path, "update_on_arrival", False):
-        n += sum((len(idx) + 71) // 72 for _, idx in path.events)   # one fused SGD group per bucket
-    else:
-        n += (len(path.plan["params"]) + 71) // 72               # one fused SGD group per step
+            rt.cudaGetLastError()                # a kernel of another runtime (NCCL's), a copy, an event
+    graph.reset()
     return n
 
 
