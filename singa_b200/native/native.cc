@@ -216,9 +216,13 @@ void give_back() {
   for (const auto n : numbers) captured_scratch().erase(n);
 }
 // Buffer of a capture under way: a new one for a request that the capture's others are too small for.
-Tensor capture_workspace(const Tensor& like, size_t bytes, unsigned long long capture, cudaGraph_t graph,
-                         cudaStream_t stream, unsigned long long thread) {
+Tensor capture_workspace(const Tensor& like, size_t bytes, cudaStream_t stream, unsigned long long thread) {
   static unsigned long long last = 0;
+  cudaStreamCaptureStatus status;
+  unsigned long long capture = 0;
+  cudaGraph_t graph = nullptr;
+  cuda_ok(cudaStreamGetCaptureInfo(stream, &status, &capture, &graph, nullptr, nullptr), "cudaStreamGetCaptureInfo");
+  if (status != cudaStreamCaptureStatusActive) fail(PyExc_RuntimeError, "the capture under way has been invalidated");
   for (const auto& [n, c] : captured_scratch())
     if (c.capture == capture && c.stream == stream && c.thread == thread && c.buffer.device() == like.device() &&
         count(c.buffer) >= bytes)
@@ -242,12 +246,10 @@ Tensor workspace(const Tensor& like, size_t bytes) {
   static std::atomic<unsigned long long> threads{0};
   thread_local const unsigned long long thread = ++threads;
   const cudaStream_t s = c10::cuda::getCurrentCUDAStream().stream();
-  unsigned long long capture = 0;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  cudaGraph_t graph = nullptr;
-  cuda_ok(cudaStreamGetCaptureInfo(s, &status, &capture, &graph, nullptr, nullptr), "cudaStreamGetCaptureInfo");
+  cuda_ok(cudaStreamIsCapturing(s, &status), "cudaStreamIsCapturing");   // (the graph's place takes another query)
   give_back();
-  if (status != cudaStreamCaptureStatusNone) return capture_workspace(like, bytes, capture, graph, s, thread);
+  if (status != cudaStreamCaptureStatusNone) return capture_workspace(like, bytes, s, thread);
   auto& list = scratch_of(static_cast<size_t>(like.device().index()));
   size_t k = 0;
   while (k < list.size() && !(list[k].stream == s && list[k].thread == thread)) ++k;
@@ -435,8 +437,10 @@ PyObject* py_row_max(Args a, Py_ssize_t) {
 PyObject* py_sum_all(Args a, Py_ssize_t) {
   const Tensor& t = dev(a[0]);
   Tensor out = fresh({1}, at::kFloat, t);
-  const Ws ws(t, sgb_sum_all_workspace_bytes(count(t)));
-  ISSUE(sgb_sum_all_f32, f32(t), f32w(out), count(t), ws.ptr, ws.bytes, stream());
+  const size_t need = sgb_sum_all_workspace_bytes(count(t));
+  const bool one = need == sizeof(float);          // the only partial sum is the result
+  const Ws ws(t, one ? 0 : need);
+  ISSUE(sgb_sum_all_f32, f32(t), f32w(out), count(t), one ? raww(out) : ws.ptr, one ? need : ws.bytes, stream());
   return wrap(std::move(out));
 }
 PyObject* py_blas1(Args a, Py_ssize_t n) {       // (0 dot | 1 asum | 2 nrm2 | 3 amax | 4 amin, x[, y])

@@ -6,6 +6,7 @@ any iterable of ``(param, grad)`` pairs in the order gradients are produced
 (what ``autograd.backward(loss)`` yields, python/singa/autograd.py:128-224).
 """
 import functools
+import operator
 
 import numpy as np
 
@@ -112,10 +113,30 @@ def _as_defined(cls, names):
     return all(vars(cls).get(f) is defined[f] for f in names if f in defined)
 
 
-# The last argument of these two: what the classes have in place of the functions that
+def _reader(names):
+    """Function of a class: what it has under these names, None where it has nothing."""
+    read = operator.attrgetter(*names)
+
+    def functions(cls):
+        try:
+            return read(cls)
+        except AttributeError:
+            return tuple(getattr(cls, f, None) for f in names)
+    return functions
+
+
+# By exchange: the names that must not be an instance's own (of DistOpt, of the
+# communicator), and what reads the classes' functions.
+_OF_WHOLE = {x: (f + c, operator.attrgetter(*f), operator.attrgetter(name, *c)) for x, (name, f, c) in _WHOLE.items()}
+_OF_UPDATE = {x: (frozenset(_WHOLE[x][1] + _AROUND), frozenset((name,) + c + _WHOLE[x][2]),
+                  _reader(_WHOLE[x][1] + _AROUND), _reader((name, _WHOLE[x][0]) + c + _WHOLE[x][2]))
+              for x, (name, c) in _WITH_UPDATE.items()}
+
+
+# The last arguments of these two: what the classes have in place of the functions that
 # the answer is about, so that a remembered answer is not given for others.
 @functools.lru_cache(maxsize=64)
-def _stands(own, kind, exchange, functions):
+def _stands(own, kind, exchange, *functions):
     """Whether the method of communicators of class `kind` does what `own` (DistOpt
     or a subclass) would do call by call: nobody below the class that defines it
     has a version of its own of a call, and nobody has put one into that class."""
@@ -127,7 +148,7 @@ def _stands(own, kind, exchange, functions):
 
 
 @functools.lru_cache(maxsize=64)
-def _stands_with_update(own, kind, exchange, functions):
+def _stands_with_update(own, kind, exchange, *functions):
     """Whether the method of communicators of class `kind` that also updates does what
     the exchange, wait() and the update of `own` would do one after the other."""
     def owner(name):
@@ -135,7 +156,8 @@ def _stands_with_update(own, kind, exchange, functions):
     name, calls = _WITH_UPDATE[exchange]
     return owner(name) is not None and all(owner(x) in (None, owner(name)) for x in calls) and \
         all(getattr(own, f) is getattr(DistOpt, f) for f in _AROUND) and \
-        _as_defined(DistOpt, _AROUND) and _as_defined(owner(name), calls) and _as_defined(SGD, ("apply_many",))
+        _as_defined(DistOpt, _AROUND) and _as_defined(owner(name), calls) and _as_defined(SGD, ("apply_many",)) and \
+        _stands.__wrapped__(own, kind, exchange)
 
 
 class DistOpt(object):
@@ -190,13 +212,16 @@ class DistOpt(object):
         where it has none, or where a subclass or an instance has its own version
         of one of the calls that it stands for, which then has to be called."""
         c = self.communicator
-        name, (f, g), (x, y) = _WHOLE[exchange]
+        (f, g, x, y), of_mine, of_theirs = _OF_WHOLE[exchange]
         mine, theirs, own, kind = self.__dict__, getattr(c, "__dict__", ()), type(self), type(c)
-        if f in mine or g in mine or x in theirs or y in theirs or \
-                not _stands(own, kind, exchange, (getattr(own, f), getattr(own, g), getattr(kind, x, None),
-                                                  getattr(kind, y, None), getattr(kind, name, None))):
-            return None
-        return getattr(c, name)
+        try:
+            if f in mine or g in mine or x in theirs or y in theirs or \
+                    not _stands(own, kind, exchange, of_mine(own), of_theirs(kind)):
+                return None
+        except AttributeError:                            # a communicator without one of the calls
+            if not _stands.__wrapped__(own, kind, exchange):
+                return None
+        return getattr(c, _WHOLE[exchange][0])
 
     def _with_update(self, exchange, grad_stream):
         """The communicator's method that does the whole `exchange` of gradients that
@@ -205,16 +230,13 @@ class DistOpt(object):
         c, opt = self.communicator, self.opt
         if self.world_size != 1 or type(grad_stream) not in _LISTS or type(opt) is not SGD:
             return None
+        mine, theirs, of_mine, of_theirs = _OF_UPDATE[exchange]
         own, kind = type(self), type(c)
-        (name, calls), mine, theirs = _WITH_UPDATE[exchange], self.__dict__, getattr(c, "__dict__", ())
-        functions = (SGD.apply_many, own.wait, own._update_all, own._sync_dense, getattr(kind, name, None),
-                     *[getattr(kind, x, None) for x in calls])
-        if not _stands_with_update(own, kind, exchange, functions) or self._whole(exchange) is None:
+        if "apply_many" in opt.__dict__ or not (
+                mine.isdisjoint(self.__dict__) and theirs.isdisjoint(getattr(c, "__dict__", ())) and
+                _stands_with_update(own, kind, exchange, SGD.apply_many, of_mine(own), of_theirs(kind))):
             return None
-        if "apply_many" in opt.__dict__ or "wait" in mine or "_update_all" in mine or "_sync_dense" in mine or \
-                name in theirs or any(x in theirs for x in calls):
-            return None
-        return getattr(c, name)
+        return getattr(c, _WITH_UPDATE[exchange][0])
 
     def _hyper(self):
         o = self.opt
@@ -383,13 +405,14 @@ class DistOpt(object):
         # and are updated as they are written.
         joint = update = None
         if corr and self.world_size == 1 and type(grad_stream) in _LISTS:
-            joint = None if topK else self._whole("joint")
             takes = getattr(self.communicator, "takesSparseUpdate", None)
             if takes is not None and type(self.opt) is SGD:
                 grad_stream = list(grad_stream)
                 takes = takes(grad_stream, threshold, topK)
             if takes is None or takes:
                 update = self._with_update("sparse", grad_stream)
+            if not topK and update is None:
+                joint = self._whole("joint")
         updated = False
         try:
             if joint is not None or update is not None:
@@ -406,6 +429,8 @@ class DistOpt(object):
                     updated = len(place) == len(grads) and update(
                         lists, residuals, [params[i] for i in order],
                         None if moments is None else [moments[i] for i in order], spars, topK, self._hyper())
+                if not updated and update is not None and not topK:
+                    joint = self._whole("joint")
                 if not updated and (joint is None or not ready or not joint(lists, residuals, spars)):
                     begin = self._whole("sparse")
                     for b in ready:
