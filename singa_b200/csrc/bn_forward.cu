@@ -481,11 +481,13 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
   if (threadIdx.x >= threads) {
     dependency_wait();
     release_dependents();
+    if (summing) revisit_open(r, item);
     if (!finishing) return;
     const unsigned c = r.parts.quot(mine);
     const float sc = a.scale[c], b = a.bias[c];
     Moments m{0.f, 0.f, 0.f};
-    const bool got = revisit_gather(r, c, [&](unsigned k, float mean, float m2) {
+    unsigned base;
+    const bool got = revisit_gather(r, c, base, [&](unsigned k, float mean, float m2) {
       const unsigned e0 = elements_before<VEC>(r, c, k * r.per), e1 = elements_before<VEC>(r, c, min((k + 1) * r.per, r.total));
       m = merge(m, Moments{static_cast<float>(e1 - e0), mean, m2});
     });
@@ -500,7 +502,7 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
       if (got && mine == c * r.parts.d) finish_channel(a, c, m.mean, var, invstd);
     }
     revisit_arrive(2, blockDim.x);
-    if (got) revisit_leave(r, c);
+    if (got) revisit_leave(r, c, base);
     return;
   }
   Vec4f v[NV];
@@ -543,7 +545,7 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
           q += d * d;
         }
     q = total(q, sm[1]);
-    if (threadIdx.x == 0) revisit_publish(r, item, u.c, u.part, mean, q);
+    if (threadIdx.x == 0) put_entry(r.entries + item, mean, q, r.tag);
   } else {
     dependency_wait();
   }

@@ -32,8 +32,24 @@ __device__ RevisitState g_revisit_state;
 //   32x512x28x28            45.6 / 37.9 / 38.8-41.0            34.1 / 30.3 / 30.1-31.1
 //   32x64x56x56             24.6 / 20.6 / 21.1-21.9            18.3 / 16.4 / 16.8-17.6
 //   32x128x57x57            66.0 / 45.8 / 47.8-53.3            46.6 / 38.5 / 40.4-47.4
+// (Those are from when the exchange had fences, see bn_revisit.cuh; now, with / without:
+// 32x256x56x56 68.0 / 51.2, 32x512x28x28 36.4 / 28.2, 32x64x56x56 19.8 / 15.4, 32x128x57x57
+// 42.0 / 32.5.)
+template <bool MASKED, bool VEC>
+constexpr RevisitShape kBwd = VEC ? RevisitShape{4, 224, 4} : RevisitShape{2, 288, MASKED ? 4 : 5};
+
+// Whether what is to be finished is asked for before the CTA's warps meet to add up, and
+// so is on its way while they do.  Odd planes, whose masked ends make a CTA's reduction
+// long: 32x128x57x57 38.5 -> 35.3 us, with a ReLU (and four CTAs, for the registers) 44.9
+// -> 43.4; 24x64x71x71 23.9 -> 22.6 and 27.9 -> 27.4.  Whole vectors gain nothing (53.3 ->
+// 53.2), and with a ReLU the registers that it takes cost more (69.8 -> 71.9).
+//
+// What did not help either (us, 32x256x56x56 with / without a ReLU, 69.7 / 53.4): the second
+// visit through shared memory by asynchronous copies that start with the first (74.1 /
+// 54.9); a join in front taken into both visits (124.4 with its 24 bytes an element, the
+// join and this kernel apart 110.0: four operands leave too little of them in L2).
 template <bool VEC>
-constexpr RevisitShape kBwd = VEC ? RevisitShape{4, 224, 4} : RevisitShape{2, 288, 5};
+constexpr bool kEarly = !VEC;
 
 struct BwdArgs {
   const float *x, *dy, *relu, *scale, *mean, *invstd;
@@ -46,10 +62,10 @@ struct BwdArgs {
 // The last warp fetches the sums and forms the coefficients of the item to be
 // finished while the others load and add up the item to be summed.
 template <int MASK, bool VEC>
-__global__ void __launch_bounds__(kBwd<VEC>.threads + 32, kBwd<VEC>.per_sm)
+__global__ void __launch_bounds__(kBwd<MASK != 0, VEC>.threads + 32, kBwd<MASK != 0, VEC>.per_sm)
 bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
-  constexpr int NV = kBwd<VEC>.units;
-  __shared__ float2 sm[kBwd<VEC>.threads / 32];
+  constexpr int NV = kBwd<MASK != 0, VEC>.units;
+  __shared__ float2 sm[kBwd<MASK != 0, VEC>.threads / 32];
   __shared__ float4 coef;
   __shared__ bool stopped;
   const unsigned item = blockIdx.x, mine = item - a.r.delay, threads = blockDim.x - 32;
@@ -57,11 +73,13 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
   if (threadIdx.x >= threads) {
     dependency_wait();
     release_dependents();
+    if (summing) revisit_open(a.r, item);
     if (!finishing) return;
     const unsigned c = a.r.parts.quot(mine);
     const float sc = a.scale[c], r = a.invstd[c], mu = a.mean[c];
     float s = 0.f, t = 0.f;
-    const bool got = revisit_gather(a.r, c, [&](unsigned, float p, float q) {
+    unsigned base;
+    const bool got = revisit_gather(a.r, c, base, [&](unsigned, float p, float q) {
       s += p;
       t += q;
     });
@@ -77,7 +95,7 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
       }
     }
     revisit_arrive(2, blockDim.x);
-    if (got) revisit_leave(a.r, c);
+    if (got) revisit_leave(a.r, c, base);
     return;
   }
   // loads of all units at once; what is not there is 0
@@ -100,10 +118,11 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
     if (MASK == 2) return (vm[k].i[0] >> j) & 1 ? g : 0.0f;
     return g;
   };
+  float s = 0.f, t = 0.f;
   if (summing) {
     const RevisitUnits<VEC, NV> u(a.r, item, threads);
     // the first CTAs wait for DRAM while the previous kernel drains; dy may be its output
-    if (first_wave(kBwd<VEC>.per_sm)) {
+    if (first_wave(kBwd<MASK != 0, VEC>.per_sm)) {
 #pragma unroll
       for (int k = 0; k < NV; ++k)
         if (u.valid[k] && (VEC || u.off[k] < a.numel)) {
@@ -114,7 +133,6 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
     dependency_wait();
     load(u, keep_policy());
     const float mu = a.mean[u.c];
-    float s = 0.f, t = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; ++k)
 #pragma unroll
@@ -124,6 +142,14 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
           s += g;
           t += g * (vx[k].f[j] - mu);
         }
+  } else {
+    dependency_wait();
+  }
+  // What is to be finished is asked for before the warps meet: it is on its way while
+  // they add up, and while the slowest of them still waits for its operands.
+  RevisitUnits<VEC, NV> u(a.r, finishing ? mine : item, threads);
+  if (kEarly<VEC> && finishing) load(u, drop_policy());
+  if (summing) {
     s = warp_sum(s);
     t = warp_sum(t);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = make_float2(s, t);
@@ -134,14 +160,11 @@ bn_bwd_revisit_kernel(const __grid_constant__ BwdArgs a) {
         s += sm[w].x;
         t += sm[w].y;
       }
-      revisit_publish(a.r, item, u.c, u.part, s, t);
+      put_entry(a.r.entries + item, s, t, a.r.tag);
     }
-  } else {
-    dependency_wait();
   }
   if (!finishing) return;
-  const RevisitUnits<VEC, NV> u(a.r, mine, threads);
-  load(u, drop_policy());
+  if (!kEarly<VEC>) load(u, drop_policy());
   revisit_sync(2, blockDim.x);
   if (stopped) return;
   const float k_ = coef.x, am = coef.y, bm = coef.z, mu = coef.w;
@@ -186,7 +209,7 @@ int revisit_faults(unsigned* flags) {
 size_t bn_revisit_workspace_bytes(int N, int C, int HW) {
   const int upp = HW % 4 ? ragged_units(HW) : HW / 4;
   RevisitPlan p;
-  return revisit_plan(HW % 4 ? kBwd<false> : kBwd<true>, static_cast<long long>(N) * upp, upp, C, &p) ? p.bytes : 0;
+  return revisit_plan(HW % 4 ? kBwd<false, false> : kBwd<false, true>, static_cast<long long>(N) * upp, upp, C, &p) ? p.bytes : 0;
 }
 
 int bn_revisit_backward(int mask, const float* x, const float* dy, const float* relu, const float* scale,
@@ -195,8 +218,10 @@ int bn_revisit_backward(int mask, const float* x, const float* dy, const float* 
   const bool vec = HW % 4 == 0;
   const int upp = vec ? HW / 4 : ragged_units(HW);
   const long long units = static_cast<long long>(N) * upp;
+  const RevisitShape shape = vec ? (mask ? kBwd<true, true> : kBwd<false, true>)
+                                 : (mask ? kBwd<true, false> : kBwd<false, false>);
   RevisitPlan p;
-  if (!ws || !aligned16(ws) || !revisit_plan(vec ? kBwd<true> : kBwd<false>, units, upp, C, &p) || ws_bytes < p.bytes) return SGB_ERR_WORKSPACE;
+  if (!ws || !aligned16(ws) || !revisit_plan(shape, units, upp, C, &p) || ws_bytes < p.bytes) return SGB_ERR_WORKSPACE;
   int st = SGB_OK;
   RevisitState* state = revisit_state(&st);
   if (!state) return st;
