@@ -972,7 +972,7 @@ int sgb_comm_sparse_update_takes(const sgb_comm* c, void* const* tensors, const 
   for (size_t k = 0; k < nbuckets; ++k) count += counts[k];
   return sparse_update_pays(total_of(sizes, count), count, nbuckets, topk) &&
          (!topk || nbuckets == 1 ||
-          sgb::sparse_topk_buckets_may(reinterpret_cast<float* const*>(tensors), sizes, counts, nbuckets));
+          sgb::sparse_topk_buckets_cut(reinterpret_cast<float* const*>(tensors), sizes, counts, nbuckets, nullptr));
 }
 
 int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* sizes, const size_t* counts,
@@ -995,45 +995,52 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
   if (!topk) return threshold_buckets(c, list, spars, &update, compute);
   for (const sgb::SparseBucket& b : list)
     if (!sgb::sparse_selects_from(b.tensors, b.sizes, b.count, b.acc)) return SGB_ERR_UNSUPPORTED;
-  // all buckets by one launch where they are few and small enough
-  std::vector<size_t> ks;
-  size_t span = 0;
-  for (const sgb::SparseBucket& b : list) {
-    const size_t n = total_of(b.sizes, b.count);
-    ks.push_back(static_cast<size_t>(sgb_topk_count(spars, n)));
-    span += n + 512;
-  }
-  const size_t ws_bytes = sgb::sparse_topk_buckets_bytes(list.data(), ks.data(), list.size(), c->topk_mode);
-  if (ws_bytes) {
-    OK(joint_reserve(c, span, compute, ws_bytes));
+  // several buckets: one launch selects from as many as it can take, the next updates them
+  if (nbuckets > 1) {
+    std::vector<size_t> ends, ks;
+    if (!sgb::sparse_topk_buckets_cut(reinterpret_cast<float* const*>(tensors), sizes, counts, nbuckets, &ends))
+      return SGB_ERR_UNSUPPORTED;
+    size_t widest = 0, ws_bytes = 0, k = 0, tensor = 0;
+    for (const size_t end : ends) {
+      size_t span = 0;
+      const size_t first = k;
+      for (; k < end; ++k) {
+        const size_t n = total_of(list[k].sizes, list[k].count);
+        ks.push_back(static_cast<size_t>(sgb_topk_count(spars, n)));
+        span += n + 512;
+      }
+      const size_t need = sgb::sparse_topk_buckets_bytes(list.data() + first, ks.data() + first, k - first, c->topk_mode);
+      if (!need) return SGB_ERR_UNSUPPORTED;
+      widest = span > widest ? span : widest;
+      ws_bytes = need > ws_bytes ? need : ws_bytes;
+    }
+    OK(joint_reserve(c, widest, compute, ws_bytes));
     OK(emit(c, plan_call(c, sgb::order::kStageCopy).pre, compute));
     Phase ph(c, "Dist_c1c2_fusedSparsification", sgb::order::kStreamC1);
-    int sent = 0;
-    OK(sgb::sparse_topk_buckets(list.data(), ks.data(), list.size(), c->topk_mode, c->joint_pay, &sent, c->joint_ws,
-                                c->joint_ws_bytes, c->c1));
-    return sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data(), list.size(), c->c1, &update);
+    k = 0;
+    for (const size_t end : ends) {
+      int sent = 0;
+      OK(sgb::sparse_topk_buckets(list.data() + k, ks.data() + k, end - k, c->topk_mode, c->joint_pay, &sent,
+                                  c->joint_ws, c->joint_ws_bytes, c->c1));
+      const sgb::SparseUpdate part{&sgd, update.params + tensor, update.moments ? update.moments + tensor : nullptr};
+      OK(sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data() + k, end - k, c->c1, &part));
+      for (; k < end; ++k) tensor += list[k].count;
+    }
+    return SGB_OK;
   }
-  // one bucket; several would follow one another on c1, without the overlap that
-  // separate calls have (72 buckets: 620 us a pass, 867 this way)
-  if (list.size() != 1) return SGB_ERR_UNSUPPORTED;
-  if (!c->dropped_dev && (capturing(compute) || capturing(c->c1))) return SGB_ERR_UNSUPPORTED;
+  if (nbuckets != 1 || (!c->dropped_dev && (capturing(compute) || capturing(c->c1)))) return SGB_ERR_UNSUPPORTED;
   OK(sparse_init(c));
   const sgb::order::Step p = plan_call(c, sgb::order::kSparseUpdate);
   const sgb_comm::Sparse& x = c->sparse[p.slot];
   OK(emit(c, p.pre, compute, p.slot));
   Phase ph(c, "Dist_c1c2_fusedSparsification", sgb::order::kStreamC1);
-  size_t at = 0;
-  for (const sgb::SparseBucket& b : list) {
-    const size_t n = total_of(b.sizes, b.count), k = static_cast<size_t>(sgb_topk_count(spars, n));
-    const int sent[1] = {static_cast<int>(k)};
-    if (k)
-      OK(sgb::sparse_topk(b.tensors, b.sizes, b.count, b.acc, k, c->topk_mode, x.pay_send,
-                          reinterpret_cast<float*>(x.pay_send) + k, c->ws, c->ws_bytes, c->c1));
-    const sgb::SparseUpdate part{&sgd, update.params + at, update.moments ? update.moments + at : nullptr};
-    OK(sgb::sparse_dense_sum(x.pay_send, 0, 0, sent, nullptr, 1, b.tensors, b.sizes, b.count, c->c1, &part));
-    at += b.count;
-  }
-  return SGB_OK;
+  const sgb::SparseBucket& b = list[0];
+  const size_t n = total_of(b.sizes, b.count), k = static_cast<size_t>(sgb_topk_count(spars, n));
+  const int sent[1] = {static_cast<int>(k)};
+  if (k)
+    OK(sgb::sparse_topk(b.tensors, b.sizes, b.count, b.acc, k, c->topk_mode, x.pay_send,
+                        reinterpret_cast<float*>(x.pay_send) + k, c->ws, c->ws_bytes, c->c1));
+  return sgb::sparse_dense_sum(x.pay_send, 0, 0, sent, nullptr, 1, b.tensors, b.sizes, b.count, c->c1, &update);
 }
 
 int sgb_comm_update_half(sgb_comm* c, void* const* params, void* const* grads, void* const* moments,

@@ -1,5 +1,7 @@
 // Internal interface of the sparsifiers, used by the communicator.
 #pragma once
+#include <vector>
+
 #include "sgd.cuh"
 
 namespace sgb {
@@ -46,9 +48,11 @@ struct SparseUpdate {
 };
 // Top-K of several buckets (the first ks[k] of bucket k by size) by one launch, into
 // a payload of the same joint space; *sent: its length.  sparse_topk_buckets_bytes:
-// of workspace, 0 where it takes a launch per bucket (fewer than two, more than 32).
-// sparse_topk_buckets_may: by sizes and places alone, before anything is prepared.
-bool sparse_topk_buckets_may(float* const* tensors, const size_t* sizes, const size_t* counts, size_t nbuckets);
+// of workspace, 0 where one launch does not take them.  sparse_topk_buckets_cut: whether
+// launches of several buckets each take a list, by sizes and places alone, before
+// anything is prepared, and where each ends (`ends` may be null).
+bool sparse_topk_buckets_cut(float* const* tensors, const size_t* sizes, const size_t* counts, size_t nbuckets,
+                             std::vector<size_t>* ends);
 size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode);
 int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
                         void* ws, size_t ws_bytes, cudaStream_t s);
