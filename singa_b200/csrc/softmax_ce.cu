@@ -218,11 +218,15 @@ softmax_ce_long_kernel(const float* __restrict__ x, const int* __restrict__ t, f
   }
 }
 
-// Threads per row and vectors per thread by row length: a warp up to 512
-// elements (no barrier at all), then the smallest CTA whose threads hold the
-// row with four vectors each.  F is called with the two constants.
+// Threads per row and vectors per thread: a warp up to 512 elements (no barrier at
+// all), then the smallest CTA whose threads hold the row with four vectors each.  A CTA of
+// 1024 threads has its SM to itself, so where there are more rows than SMs half the threads
+// take eight vectors each: one row's sums overlap another's loads, and twice the bytes are
+// in flight (us, 517 rows of 12384 24.0 -> 19.1, 149 11.2 -> 9.6, 1000 of 16000 40.4 -> 31.4;
+// shorter rows, of which an SM holds several anyhow, lost: 4096 of 3000 26.5 -> 32.0, 297 of
+// 6000 7.9 -> 10.1).  F is called with the two constants.
 template <typename V, typename F>
-int by_length(size_t ncol, F f) {
+int by_length(size_t nrow, size_t ncol, F f) {
   constexpr size_t kL = 16 / sizeof(V);
   const size_t vecs = ceil_div(ncol, kL);
 #define SGB_ROW(T, NV)                                                            \
@@ -234,6 +238,9 @@ int by_length(size_t ncol, F f) {
   SGB_ROW(128, 4)
   SGB_ROW(256, 4)
   SGB_ROW(512, 4)
+  if constexpr (kL == 4) {
+    if (nrow > static_cast<size_t>(sm_count())) { SGB_ROW(512, 8) }
+  }
   SGB_ROW(1024, 4)
   if constexpr (kL == 4) { SGB_ROW(1024, 8) }
 #undef SGB_ROW
@@ -246,7 +253,7 @@ int softmax_rows(const V* x, V* y, size_t nrow, size_t ncol, void* stream) {
   if (!x || !y) return SGB_ERR_NULL;
   if (nrow > 0x7fffffffu) return SGB_ERR_SIZE;
   const bool vec = ncol % (16 / sizeof(V)) == 0 && aligned16(x) && aligned16(y);
-  const int st = by_length<V>(ncol, [&](auto T, auto NV) {
+  const int st = by_length<V>(nrow, ncol, [&](auto T, auto NV) {
     constexpr int kT = decltype(T)::value, kNV = decltype(NV)::value;
     const unsigned grid = static_cast<unsigned>(kT == 32 ? ceil_div(nrow, 4) : nrow);
     return launch_ex(softmax_rows_kernel<V, kT, kNV>, dim3(grid), dim3(kT == 32 ? 128 : kT), 0, as_stream(stream), 0,
@@ -470,7 +477,7 @@ int sgb_softmax_cross_entropy_fused_f32(const float* logits, const int32_t* t, s
   if (!logits || !t || !loss || !grad) return SGB_ERR_NULL;
   if (batch > 0x7fffffffu) return SGB_ERR_SIZE;
   const bool vec = dim % 4 == 0 && aligned16(logits) && (!prob || aligned16(prob)) && aligned16(grad);
-  const int st = by_length<float>(dim, [&](auto T, auto NV) {
+  const int st = by_length<float>(batch, dim, [&](auto T, auto NV) {
     constexpr int kT = decltype(T)::value, kNV = decltype(NV)::value;
     const unsigned grid = static_cast<unsigned>(kT == 32 ? ceil_div(batch, 4) : batch);
     return launch_ex(softmax_ce_fused_kernel<kT, kNV>, dim3(grid), dim3(kT == 32 ? 128 : kT), 0, as_stream(stream), 0,
