@@ -9,6 +9,8 @@
 // '>' while scanning, padding never wins).
 #include <float.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace sgb {
@@ -336,19 +338,39 @@ struct StripArgs {
 
 constexpr int kNoCell = -1;
 
-// Index 0..8 (raster order) of the window's first maximum; kNoCell if no cell
-// exceeds -FLT_MAX.  NANS: a NaN wins and then sticks, as in cuDNN.
+// The first maximum of a window in raster order, in two steps: of the three cells of
+// each row, which serves every window that holds them, then of the three rows (a row's
+// winner counts only if it is strictly greater than the rows above).  NANS: a NaN wins
+// and then sticks, as in cuDNN; warps that have seen none (nor an infinity) take the
+// plain comparisons.  (us, 32x64x112x112 by 3/2/1, nine comparisons a window -> this:
+// forward 24.7 -> 23.9, with the record 32.0 -> 29.6, backward 45.0 -> 42.2.)
 template <bool NANS>
-__device__ __forceinline__ int first_max(const float (&v)[9], float& best) {
-  best = -FLT_MAX;
-  int at = kNoCell;
+__device__ __forceinline__ bool beats(float v, float best) {
+  return v > best || (NANS && v != v && best == best);
+}
+template <bool NANS>
+__device__ __forceinline__ void first_of_cells(float c0, float c1, float c2, float& best, int& at) {
+  bool p = beats<NANS>(c1, c0);
+  best = p ? c1 : c0;
+  at = p ? 1 : 0;
+  p = beats<NANS>(c2, best);
+  best = p ? c2 : best;
+  at = p ? 2 : at;
+}
+// Index 0..8 of the winner; kNoCell (and -FLT_MAX) if no cell exceeds -FLT_MAX.
+template <bool NANS>
+__device__ __forceinline__ void first_of_rows(const float (&v)[3], const int (&col)[3], float& best, int& at) {
+  best = v[0];
+  at = col[0];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const bool p = NANS ? v[k] > best || (v[k] != v[k] && best == best) : v[k] > best;
-    best = p ? v[k] : best;
-    at = p ? k : at;
+  for (int r = 1; r < 3; ++r) {
+    const bool p = beats<NANS>(v[r], best);
+    best = p ? v[r] : best;
+    at = p ? 3 * r + col[r] : at;
   }
-  return at;
+  const bool some = beats<NANS>(best, -FLT_MAX);
+  best = some ? best : -FLT_MAX;
+  at = some ? at : kNoCell;
 }
 
 template <int MODE, bool VEC>
@@ -458,6 +480,8 @@ pool_k3s2p1_kernel(const StripArgs a) {
   };
 
   float above[4], above_left = kPad, r0[4], r1[4], n0[4], n1[4], g[2] = {0.f, 0.f}, ng[2] = {0.f, 0.f};
+  float top[2] = {kPad, kPad};     // maxima: what the two windows hold in the row above
+  int top_at[2] = {0, 0};
   unsigned code[2] = {0, 0}, ncode[2] = {0, 0};
   bool odd_above = false;          // something in the row above that only the NaN-aware comparison may decide
   auto unordered = [](const float (&v)[4]) {
@@ -470,7 +494,11 @@ pool_k3s2p1_kernel(const StripArgs a) {
     load_row(2 * m0 + 1, n1);
     above_left = __shfl_up_sync(kAll, above[3], 1);
     if (!has_left) above_left = kPad;
-    if (kMax) odd_above = __any_sync(kAll, unordered(above));
+    if (kMax) {
+      odd_above = __any_sync(kAll, unordered(above));
+      first_of_cells<true>(above_left, above[0], above[1], top[0], top_at[0]);
+      first_of_cells<true>(above[1], above[2], above[3], top[1], top_at[1]);
+    }
   }
   load_windows(m0, ng, ncode);
   ahead(m0 + 1);
@@ -499,28 +527,39 @@ pool_k3s2p1_kernel(const StripArgs a) {
     if (kNeedsX) {
       float l0 = __shfl_up_sync(kAll, r0[3], 1), l1 = __shfl_up_sync(kAll, r1[3], 1);
       if (!has_left) l0 = l1 = kPad;
-      const float w0[9] = {above_left, above[0], above[1], l0, r0[0], r0[1], l1, r1[0], r1[1]};
-      const float w1[9] = {above[1], above[2], above[3], r0[1], r0[2], r0[3], r1[1], r1[2], r1[3]};
       if (kMax) {
         const bool odd0 = __any_sync(kAll, unordered(r0)), odd1 = __any_sync(kAll, unordered(r1));
-        if (odd_above || odd0 || odd1) {
-          at0 = first_max<true>(w0, best0);
-          at1 = first_max<true>(w1, best1);
-        } else {
-          at0 = first_max<false>(w0, best0);
-          at1 = first_max<false>(w1, best1);
-        }
+        auto windows = [&](auto nans) {
+          constexpr bool kNans = decltype(nans)::value;
+          float v[2][3] = {{top[0]}, {top[1]}};
+          int col[2][3] = {{top_at[0]}, {top_at[1]}};
+          first_of_cells<kNans>(l0, r0[0], r0[1], v[0][1], col[0][1]);
+          first_of_cells<kNans>(r0[1], r0[2], r0[3], v[1][1], col[1][1]);
+          first_of_cells<kNans>(l1, r1[0], r1[1], v[0][2], col[0][2]);
+          first_of_cells<kNans>(r1[1], r1[2], r1[3], v[1][2], col[1][2]);
+          first_of_rows<kNans>(v[0], col[0], best0, at0);
+          first_of_rows<kNans>(v[1], col[1], best1, at1);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            top[j] = v[j][2];
+            top_at[j] = col[j][2];
+          }
+        };
+        if (odd_above || odd0 || odd1) windows(std::true_type{});
+        else windows(std::false_type{});
         odd_above = odd1;
       } else {
+        const float w0[9] = {above_left, above[0], above[1], l0, r0[0], r0[1], l1, r1[0], r1[1]};
+        const float w1[9] = {above[1], above[2], above[3], r0[1], r0[2], r0[3], r1[1], r1[2], r1[3]};
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
           best0 += w0[k];
           best1 += w1[k];
         }
-      }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) above[j] = r1[j];
-      above_left = l1;
+        for (int j = 0; j < 4; ++j) above[j] = r1[j];
+        above_left = l1;
+      }
     }
     if (MODE == kMaxBwdRecord) {
       at0 = code[0] == 0xffu ? kNoCell : static_cast<int>(code[0] >> 4) * 3 + static_cast<int>(code[0] & 15u);
@@ -648,17 +687,19 @@ inline bool is_k3s2p1(const PoolShape& p) {
 // ------------------------------------------------ 3x3 / stride 1 / pad 1, max passes
 // Same layout: a lane owns four columns and the four windows centred on them.
 // The first maximum of three adjacent cells of a row is worked out once and
-// serves the three windows it belongs to (6 comparisons per window instead of
-// 9; taking a row's winner only if it is strictly greater than the rows above
-// keeps the raster order).  Was 231 us forward and 276 us backward at
-// 32x64x112x112, where the bytes take 31 and 47 us.
+// serves the three windows it belongs to (4 comparisons per window instead of
+// 9).  Was 231 us forward and 276 us backward at 32x64x112x112, where the bytes take
+// 31 and 47 us, and 56.5 and 104.2 when all comparisons looked for NaNs and began at
+// the lowest value; now 47.7 and 90.2.  The backward pass of rows off a vector's
+// boundary has registers for three CTAs an SM only (64x512x14x14 38.0 us with four and
+// spilled ones, 30.1 with three; 64x64x35x35 33.2 and 27.4).
 struct RowBest {
   float v[4];
-  int at[4];               // column offset 0..2 of the winner, kNoCell if none
+  int at[4];               // column offset 0..2 of the winner
 };
 
 template <int MODE, bool VEC>
-__global__ void __launch_bounds__(kBlock, 4)
+__global__ void __launch_bounds__(kBlock, MODE == kMaxBwd && !VEC ? 3 : 4)
 pool_k3s1p1_kernel(const StripArgs a) {
   constexpr bool kBackward = MODE == kMaxBwd || MODE == kMaxBwdRecord;
   constexpr bool kNeedsX = MODE != kMaxBwdRecord;
@@ -712,29 +753,22 @@ pool_k3s1p1_kernel(const StripArgs a) {
         if (c + j < W) r[j] = v[j];
     }
   };
-  auto better = [](bool nans, float v, float best) { return v > best || (nans && v != v && best == best); };
   // the winner of each window's three cells in one row, and whether the row
   // (of the whole warp) holds anything that needs the NaN-aware comparison
   auto row_best = [&](const float (&v)[4], RowBest& b) -> bool {
     float left = __shfl_up_sync(kAll, v[3], 1), right = __shfl_down_sync(kAll, v[0], 1);
     if (!has_left) left = -FLT_MAX;
     if (!has_right) right = -FLT_MAX;
-    const float s = (v[0] + v[1]) + (v[2] + v[3]) + (left + right);
+    const float s = (v[0] + v[1]) + (v[2] + v[3]);
     const bool nans = __any_sync(kAll, s != s);
     const float cell[6] = {left, v[0], v[1], v[2], v[3], right};
+    auto work_out = [&](auto kind) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float best = -FLT_MAX;
-      int at = kNoCell;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const bool p = better(nans, cell[j + k], best);
-        best = p ? cell[j + k] : best;
-        at = p ? k : at;
-      }
-      b.v[j] = best;
-      b.at[j] = at;
-    }
+      for (int j = 0; j < 4; ++j)
+        first_of_cells<decltype(kind)::value>(cell[j], cell[j + 1], cell[j + 2], b.v[j], b.at[j]);
+    };
+    if (nans) work_out(std::true_type{});
+    else work_out(std::false_type{});
     return nans;
   };
 
@@ -789,19 +823,17 @@ pool_k3s1p1_kernel(const StripArgs a) {
     }
     if (kNeedsX) {
       nan_low = row_best(v, low);
-      const bool nans = nan_up || nan_mid || nan_low;
+      auto windows = [&](auto kind) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        best[j] = up.v[j];
-        win[j] = up.at[j];
-        bool p = better(nans, mid.v[j], best[j]);
-        best[j] = p ? mid.v[j] : best[j];
-        win[j] = p ? 3 + mid.at[j] : win[j];
-        p = better(nans, low.v[j], best[j]);
-        best[j] = p ? low.v[j] : best[j];
-        win[j] = p ? 6 + low.at[j] : win[j];
-        if (kBackward && c + j >= W) win[j] = kNoCell;
-      }
+        for (int j = 0; j < 4; ++j) {
+          const float rows[3] = {up.v[j], mid.v[j], low.v[j]};
+          const int col[3] = {up.at[j], mid.at[j], low.at[j]};
+          first_of_rows<decltype(kind)::value>(rows, col, best[j], win[j]);
+          if (kBackward && c + j >= W) win[j] = kNoCell;
+        }
+      };
+      if (nan_up || nan_mid || nan_low) windows(std::true_type{});
+      else windows(std::false_type{});
       up = mid;
       mid = low;
       nan_up = nan_mid;
