@@ -166,6 +166,35 @@ union Vec4f {
   float f[4];
   int i[4];
 };
+// Four floats at an address that need not be a vector's (the same alignment in all
+// lanes): tensors of any length lie back to back in a gradient arena.
+__device__ __forceinline__ Vec4f ld4(const float* p) {
+  Vec4f v;
+  const unsigned at = static_cast<unsigned>(reinterpret_cast<uintptr_t>(p));
+  if ((at & 15u) == 0) {
+    v.u = ld128(p);
+  } else if ((at & 7u) == 0) {
+    const float2 a = *reinterpret_cast<const float2*>(p), b = *reinterpret_cast<const float2*>(p + 2);
+    v.f[0] = a.x; v.f[1] = a.y; v.f[2] = b.x; v.f[3] = b.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v.f[j] = p[j];
+  }
+  return v;
+}
+__device__ __forceinline__ void st4(float* p, const Vec4f& v) {
+  const unsigned at = static_cast<unsigned>(reinterpret_cast<uintptr_t>(p));
+  if ((at & 15u) == 0) {
+    st128(p, v.u);
+  } else if ((at & 7u) == 0) {
+    *reinterpret_cast<float2*>(p) = make_float2(v.f[0], v.f[1]);
+    *reinterpret_cast<float2*>(p + 2) = make_float2(v.f[2], v.f[3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = v.f[j];
+  }
+}
+
 union Vec8h {
   uint4 u;
   __half h[8];

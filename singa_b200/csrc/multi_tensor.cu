@@ -13,6 +13,8 @@
 // only beyond that are several launches made.
 // Every CTA handles one 1024-element tile and finds its tensor with a binary
 // search over the table.
+#include <type_traits>
+
 #include "sgd.cuh"
 
 namespace sgb {
@@ -51,7 +53,12 @@ __device__ __forceinline__ int find_tensor(const Table<N>& t, unsigned tile) {
 // ROUND: the gradient is rounded to fp16 and widened again on the way, and written
 // back: what a one-rank exchange in half precision does to it.  One pass over p, g
 // and m (24 B/element) instead of one over g and one over all three (28).
-template <int N, bool ROUND>
+//
+// ANY: some tensor is off a vector's boundary (tensors of any length lie back to back in
+// a gradient arena), and four elements are still accessed together, as far as they can be.
+// (us, the gradient off by one element: 1.2e6 elements 8.8 element by element, 5.0 so;
+// 1.7e7 84.0 and 49.2.  In a kernel for both kinds the aligned lists took 5.0 instead of 4.4.)
+template <int N, bool ROUND, bool ANY>
 __global__ void __launch_bounds__(kBlock)
 sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
   const int k = find_tensor(t, blockIdx.x);
@@ -60,29 +67,35 @@ sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
   float* p = static_cast<float*>(t.a[k]);
   float* g = static_cast<float*>(t.b[k]);
   float* m = static_cast<float*>(t.c[k]);
-  const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
-                     (a.use_momentum ? reinterpret_cast<uintptr_t>(m) : 0)) & 15u) == 0;
   const size_t i = base + 4 * threadIdx.x;
-  if (vec && i + 4 <= n && first_wave(8)) {
+  auto load = [](const float* from) {
+    if (ANY) return ld4(from);
+    Vec4f v;
+    v.u = ld128(from);
+    return v;
+  };
+  auto store = [](float* to, const Vec4f& v) {
+    if (ANY) st4(to, v);
+    else st128(to, v.u);
+  };
+  if (i + 4 <= n && first_wave(8)) {
     prefetch_l2(p + i);
     if (a.use_momentum) prefetch_l2(m + i);
   }
   dependency_wait();
-  if (vec && i + 4 <= n) {
-    Vec4f vp, vg, vm;
-    vp.u = ld128(p + i);
-    vg.u = ld128(g + i);
-    if (a.use_momentum) vm.u = ld128(m + i);
+  if (i + 4 <= n) {
+    Vec4f vp = load(p + i), vg = load(g + i), vm;
+    if (a.use_momentum) vm = load(m + i);
     release_dependents();
     if (ROUND) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) vg.f[j] = __half2float(__float2half_rn(vg.f[j]));
-      st128(g + i, vg.u);
+      store(g + i, vg);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) sgd_one(vp.f[j], vg.f[j], vm.f[j], a);
-    st128(p + i, vp.u);
-    if (a.use_momentum) st128(m + i, vm.u);
+    store(p + i, vp);
+    if (a.use_momentum) store(m + i, vm);
   } else {
     for (size_t j = i; j < n && j < i + 4; ++j) {
       float pv = p[j], gv = g[j], mv = a.use_momentum ? m[j] : 0.f;
@@ -98,7 +111,8 @@ sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
 // (what packing, a one-rank all-reduce and unpacking do to them).
 enum PackMode { kPackF32 = 0, kPackF32ToF16 = 1, kUnpackF32 = 2, kUnpackF16ToF32 = 3, kRoundF16 = 4 };
 
-template <int MODE, int N>
+// ANY: as in sgd_multi_kernel.
+template <int MODE, int N, bool ANY>
 __global__ void __launch_bounds__(kBlock)
 pack_multi_kernel(const __grid_constant__ Table<N> t, const __grid_constant__ Offsets<N> o,
                   void* flat, float scale, int use_scale) {
@@ -110,13 +124,22 @@ pack_multi_kernel(const __grid_constant__ Table<N> t, const __grid_constant__ Of
   if (i >= n) return;
   float* tensor = static_cast<float*>(t.a[k]);
   const bool full = i + 4 <= n;
+  auto load = [](const float* from) {
+    if (ANY) return ld4(from);
+    Vec4f v;
+    v.u = ld128(from);
+    return v;
+  };
+  auto store = [](float* to, const Vec4f& v) {
+    if (ANY) st4(to, v);
+    else st128(to, v.u);
+  };
   if (MODE == kRoundF16) {
-    if (full && (reinterpret_cast<uintptr_t>(tensor + i) & 15u) == 0) {
-      Vec4f v;
-      v.u = ld128(tensor + i);
+    if (full) {
+      Vec4f v = load(tensor + i);
 #pragma unroll
       for (int j = 0; j < 4; ++j) v.f[j] = __half2float(__float2half_rn(v.f[j]));
-      st128(tensor + i, v.u);
+      store(tensor + i, v);
     } else {
       for (size_t j = 0; j < 4 && i + j < n; ++j) tensor[i + j] = __half2float(__float2half_rn(tensor[i + j]));
     }
@@ -125,19 +148,17 @@ pack_multi_kernel(const __grid_constant__ Table<N> t, const __grid_constant__ Of
   const size_t fo = o.off[k] + i;
   if (MODE == kPackF32 || MODE == kUnpackF32) {
     float* fl = static_cast<float*>(flat) + fo;
-    const bool vec = full && ((reinterpret_cast<uintptr_t>(tensor + i) |
-                               reinterpret_cast<uintptr_t>(fl)) & 15u) == 0;
     if (MODE == kPackF32) {
-      if (vec) st128(fl, ld128(tensor + i));
+      if (full) store(fl, load(tensor + i));
       else for (size_t j = 0; j < 4 && i + j < n; ++j) fl[j] = tensor[i + j];
     } else {
-      if (vec) {
-        Vec4f v; v.u = ld128(fl);
+      if (full) {
+        Vec4f v = load(fl);
         if (use_scale) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) v.f[j] = v.f[j] * scale;
         }
-        st128(tensor + i, v.u);
+        store(tensor + i, v);
       } else {
         for (size_t j = 0; j < 4 && i + j < n; ++j)
           tensor[i + j] = use_scale ? fl[j] * scale : fl[j];
@@ -145,11 +166,10 @@ pack_multi_kernel(const __grid_constant__ Table<N> t, const __grid_constant__ Of
     }
   } else {
     __half* fl = static_cast<__half*>(flat) + fo;
-    const bool vec = full && (reinterpret_cast<uintptr_t>(tensor + i) & 15u) == 0 &&
-                     (reinterpret_cast<uintptr_t>(fl) & 7u) == 0;
+    const bool vec = full && (reinterpret_cast<uintptr_t>(fl) & 7u) == 0;
     if (MODE == kPackF32ToF16) {
       if (vec) {
-        Vec4f v; v.u = ld128(tensor + i);
+        const Vec4f v = load(tensor + i);
         union { uint2 u; __half h[4]; } h;
 #pragma unroll
         for (int j = 0; j < 4; ++j) h.h[j] = __float2half_rn(v.f[j]);
@@ -167,7 +187,7 @@ pack_multi_kernel(const __grid_constant__ Table<N> t, const __grid_constant__ Of
           const float f = __half2float(h.h[j]);
           v.f[j] = use_scale ? f * scale : f;
         }
-        st128(tensor + i, v.u);
+        store(tensor + i, v);
       } else {
         for (size_t j = 0; j < 4 && i + j < n; ++j) {
           const float f = __half2float(fl[j]);
@@ -238,11 +258,17 @@ int pack_list(int mode, void* const* tensors, const size_t* sizes, size_t count,
     if (cnt == 0) continue;
     // offsets inside the chunk are contiguous because empty tensors add 0
     const unsigned tiles = fill_table<N>(t, &o, ptrs, nullptr, nullptr, ns, 0, cnt, chunk_off);
-    auto kernel = mode == kPackF32        ? pack_multi_kernel<kPackF32, N>
-                  : mode == kPackF32ToF16 ? pack_multi_kernel<kPackF32ToF16, N>
-                  : mode == kUnpackF32    ? pack_multi_kernel<kUnpackF32, N>
-                  : mode == kRoundF16     ? pack_multi_kernel<kRoundF16, N>
-                                          : pack_multi_kernel<kUnpackF16ToF32, N>;
+    bool any = mode != kRoundF16 && !aligned16(flat);
+    for (int k = 0; k < cnt; ++k) any = any || !aligned16(ptrs[k]) || (mode != kRoundF16 && (o.off[k] & 3u));
+    auto pick = [&](auto off) {
+      constexpr bool kAny = decltype(off)::value;
+      return mode == kPackF32        ? pack_multi_kernel<kPackF32, N, kAny>
+             : mode == kPackF32ToF16 ? pack_multi_kernel<kPackF32ToF16, N, kAny>
+             : mode == kUnpackF32    ? pack_multi_kernel<kUnpackF32, N, kAny>
+             : mode == kRoundF16     ? pack_multi_kernel<kRoundF16, N, kAny>
+                                     : pack_multi_kernel<kUnpackF16ToF32, N, kAny>;
+    };
+    auto kernel = any ? pick(std::true_type{}) : pick(std::false_type{});
     const int st = launch_ex(kernel, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, o, flat, scale, use_scale);
     if (st != SGB_OK) return st;
   }
@@ -266,6 +292,7 @@ int sgd_list(void* const* params, void* const* grads, void* const* moments, cons
     void *pa[N], *pb[N], *pc[N];
     size_t ns[N];
     int cnt = 0;
+    bool any = false;
     unsigned long long tiles64 = 0;
     while (first < count && cnt < N) {
       const size_t n = sizes[first];
@@ -279,6 +306,7 @@ int sgd_list(void* const* params, void* const* grads, void* const* moments, cons
         pa[cnt] = params[first];
         pb[cnt] = grads[first];
         pc[cnt] = use_m ? moments[first] : nullptr;
+        any = any || !aligned16(pa[cnt]) || !aligned16(pb[cnt]) || !aligned16(pc[cnt]);
         ns[cnt] = n;
         ++cnt;
         tiles64 += tl;
@@ -287,7 +315,8 @@ int sgd_list(void* const* params, void* const* grads, void* const* moments, cons
     }
     if (cnt == 0) continue;
     const unsigned tiles = fill_table<N>(t, nullptr, pa, pb, pc, ns, 0, cnt, 0);
-    const int st = launch_ex(sgd_multi_kernel<N, ROUND>, dim3(tiles), dim3(kBlock), 0, s, 0, true, t, a);
+    const int st = launch_ex(any ? sgd_multi_kernel<N, ROUND, true> : sgd_multi_kernel<N, ROUND, false>, dim3(tiles),
+                             dim3(kBlock), 0, s, 0, true, t, a);
     if (st != SGB_OK) return st;
   }
   return launch_status();
