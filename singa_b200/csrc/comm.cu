@@ -960,9 +960,12 @@ int sgb_comm_sparsification_buckets(sgb_comm* c, void* const* tensors, const siz
 // longer list of arguments: the line is at few tensors and, by threshold, few elements.
 //   by size, one bucket of 1e6: in 1 tensor 30.0 / 21.8, 12 35.5 / 32.7, 50 33.8 / 53.5
 //   by threshold, 1e6:   in 1 tensor 20.6 / 16.4, 5 21.3 / 18.1, 12 22.8 / 24.8, 50 27.1 / 31.3
-//   in 1 tensor 3e6 32.5 / 30.8, 8e6 67.8 / 69.0; in 6 3.4e6 35.4 / 33.2, 5.8e6 54.6 / 55.3
+//   3e6 elements in 1 tensor 36.9 / 33.3, 5e6 53.5 / 45.9, 8e6 70.3 / 66.0, 1.6e7 116 / 109;
+//   in 6 3.4e6 35.4 / 33.2, 4.6e6 54.6 / 53.4, 5.8e6 63.2 / 65.3, 8.2e6 77 / 86; 2.56e7 in 161
+//   182 / 174, but 27 us more of the host
 static bool sparse_update_pays(size_t elements, size_t tensors, size_t nbuckets, int topk) {
-  return topk ? nbuckets > 1 || tensors <= 16 : tensors <= SGB_SPARSE_UPDATE_TENSORS && elements <= 4000000;
+  if (topk) return nbuckets > 1 || tensors <= 16;
+  return tensors == 1 ? elements <= sgb::kMaxBucketSpan : tensors <= SGB_SPARSE_UPDATE_TENSORS && elements <= 4000000;
 }
 
 int sgb_comm_sparse_update_takes(const sgb_comm* c, void* const* tensors, const size_t* sizes, const size_t* counts,

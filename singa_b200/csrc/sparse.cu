@@ -229,6 +229,22 @@ __device__ __forceinline__ void load_pieces(const P& p, const Cursor& c, const f
     load_tile(base, acc, tile, n, true, s);
     return;
   }
+  if (e1 <= p.off[lo + 1] && e1 <= n) {
+    // inside one tensor, but not at a vector's start (a list of odd-sized tensors): single
+    // loads of it, without a look at the list for each
+    float b[kRounds][4];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[r][j] = base[vec_at(tile, r) + j];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) load4(acc, vec_at(tile, r), n, true, b[r]);
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[r][j] += b[r][j];
+    return;
+  }
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
     const unsigned i = static_cast<unsigned>(vec_at(tile, r));
@@ -1341,35 +1357,30 @@ __device__ __forceinline__ unsigned warp_lower_bound(const int* idx, unsigned co
   return lo;
 }
 
-// g = src (in shared memory, at the same offset modulo 16 bytes as `at` in the tile),
-// and the update of p and m with it; by all threads of the CTA.
+// g = src (in shared memory), and the update of p and m with it; by all threads of the
+// CTA: what is not a whole tile of one tensor.  Vectors start where the tensors' addresses
+// are aligned, wherever that is in the tile.
 __device__ __forceinline__ void update_run(const SgdArgs& a, float* p, float* g, float* m, const float* src, int len) {
-  const uintptr_t all = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
-                        static_cast<uintptr_t>(__cvta_generic_to_shared(src));
-  const int nv = (all & 15u) == 0 ? len >> 2 : 0;
-  constexpr int kVecs = 2;                             // loads of two vectors in flight
-  for (int v0 = threadIdx.x; v0 < nv; v0 += kVecs * kBlock) {
-    Vec4f vp[kVecs], vm[kVecs];
+  const uintptr_t at = reinterpret_cast<uintptr_t>(g);
+  const uintptr_t apart = (reinterpret_cast<uintptr_t>(p) ^ at) | (a.use_momentum ? reinterpret_cast<uintptr_t>(m) ^ at : 0);
+  const int lead = static_cast<int>((0u - static_cast<unsigned>(at >> 2)) & 3u);
+  const bool vectors = (apart & 15u) == 0 && lead < len;
+  const int head = vectors ? lead : 0, nv = vectors ? (len - lead) >> 2 : 0;
+  for (int v = threadIdx.x; v < nv; v += kBlock) {
+    const int i = head + 4 * v;
+    Vec4f vp, vg, vm;
+    vp.u = ld128(p + i);
+    if (a.use_momentum) vm.u = ld128(m + i);
 #pragma unroll
-    for (int k = 0; k < kVecs; ++k)
-      if (v0 + k * kBlock < nv) {
-        vp[k].u = ld128(p + 4 * (v0 + k * kBlock));
-        if (a.use_momentum) vm[k].u = ld128(m + 4 * (v0 + k * kBlock));
-      }
+    for (int j = 0; j < 4; ++j) vg.f[j] = src[i + j];
+    st128(g + i, vg.u);
 #pragma unroll
-    for (int k = 0; k < kVecs; ++k) {
-      const int i = 4 * (v0 + k * kBlock);
-      if (v0 + k * kBlock >= nv) break;
-      Vec4f vg;
-      vg.u = *reinterpret_cast<const uint4*>(src + i);
-      st128(g + i, vg.u);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) sgd_one(vp[k].f[j], vg.f[j], vm[k].f[j], a);
-      st128(p + i, vp[k].u);
-      if (a.use_momentum) st128(m + i, vm[k].u);
-    }
+    for (int j = 0; j < 4; ++j) sgd_one(vp.f[j], vg.f[j], vm.f[j], a);
+    st128(p + i, vp.u);
+    if (a.use_momentum) st128(m + i, vm.u);
   }
-  for (int i = 4 * nv + threadIdx.x; i < len; i += kBlock) {
+  for (int e = threadIdx.x; e < len - 4 * nv; e += kBlock) {
+    const int i = e < head ? e : e + 4 * nv;
     float pv = p[i], mv = a.use_momentum ? m[i] : 0.f;
     const float gv = src[i];
     g[i] = gv;
@@ -1390,12 +1401,23 @@ __device__ __forceinline__ void update_run(const SgdArgs& a, float* p, float* g,
 // Update: the tile's parameters and momentum are updated with it on the way, so
 // that the dense gradient is not read back (a pass of 1e8 elements, 1 % sent:
 // 652 -> 644 us; of 3.6e6 62 -> 56, of 4.4e5 34 -> 30).
+constexpr int kUpdateCtas = 4;
+constexpr size_t kMostTiles = 4;
+constexpr size_t kUpdateStage = 2 * kDenseTile * sizeof(float);
+__device__ __forceinline__ void stage16(uint4* to, const float* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(to))),
+               "l"(from)
+               : "memory");
+}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <bool ALONE, typename Update>
-__global__ void __launch_bounds__(kBlock, std::is_same_v<Update, NoUpdate> ? 8 : 5)
+__global__ void __launch_bounds__(kBlock, std::is_same_v<Update, NoUpdate> ? 8 : kUpdateCtas)
 dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_per_cta, const __grid_constant__ Update u) {
   constexpr unsigned kPer = 4, kWindow = kPer * kBlock;
   constexpr bool kUpdate = std::is_same_v<Update, DenseUpdate>;
+  constexpr int kVecs = kDenseTile / (4 * kBlock);     // of a thread and tile
   __shared__ __align__(16) float out[kDenseTile];
+  [[maybe_unused]] extern __shared__ uint4 staged[];   // kUpdate: the tile's parameters, and its momentum
   __shared__ unsigned cursor[kMaxDenseRanks], count[kMaxDenseRanks];
   dependency_wait();
   release_dependents();
@@ -1423,6 +1445,32 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
   bool have = false;                                 // ALONE: the window at cursor[0] is in wi, wv
   for (size_t base = begin; base < end; base += kDenseTile) {
     const size_t stop = base + kDenseTile < end ? base + kDenseTile : end;
+    // A whole tile of one tensor, whose parameters and momentum lie like its gradient
+    // modulo a vector: what its update reads is on its way while the tile is put together.
+    [[maybe_unused]] float *pt = nullptr, *gt = nullptr, *mt = nullptr;
+    [[maybe_unused]] int head = 0;
+    bool whole = false;
+    if constexpr (kUpdate) {
+      if (base + kDenseTile == stop && a.off[target + 1] >= stop && a.ptr[target]) {
+        const size_t in = base - a.off[target];
+        gt = a.ptr[target] + in;
+        pt = u.p[target] + in;
+        mt = u.sgd.use_momentum ? u.m[target] + in : gt;
+        const uintptr_t at = reinterpret_cast<uintptr_t>(gt);
+        whole = (((reinterpret_cast<uintptr_t>(pt) ^ at) | (reinterpret_cast<uintptr_t>(mt) ^ at)) & 15u) == 0;
+        head = static_cast<int>((0u - static_cast<unsigned>(at >> 2)) & 3u);
+      }
+      if (whole) {
+#pragma unroll
+        for (int k = 0; k < kVecs; ++k) {
+          const int i = head + 4 * (k * kBlock + static_cast<int>(threadIdx.x));
+          if (i + 4 <= kDenseTile) {                   // all but the last thread's last vector, if head > 0
+            stage16(staged + k * kBlock + threadIdx.x, pt + i);
+            if (u.sgd.use_momentum) stage16(staged + (kVecs + k) * kBlock + threadIdx.x, mt + i);
+          }
+        }
+      }
+    }
     __syncthreads();                                 // cursors set; the previous tile has been stored
 #pragma unroll
     for (int r = 0; r < kDenseTile / (4 * kBlock); ++r)
@@ -1451,6 +1499,41 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
         c += kWindow;
         have = false;
         if (threadIdx.x == 0) cursor[r] = c;         // read again behind a barrier
+      }
+    }
+    if constexpr (kUpdate) {
+      if (whole) {
+        stage_wait();                                  // a thread reads what it has asked for itself
+#pragma unroll
+        for (int k = 0; k < kVecs; ++k) {
+          const int i = head + 4 * (k * kBlock + static_cast<int>(threadIdx.x));
+          if (i + 4 > kDenseTile) break;
+          Vec4f vp, vg, vm;
+          vp.u = staged[k * kBlock + threadIdx.x];
+          if (u.sgd.use_momentum) vm.u = staged[(kVecs + k) * kBlock + threadIdx.x];
+          if (head == 0) {
+            vg.u = *reinterpret_cast<const uint4*>(out + i);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) vg.f[j] = out[i + j];
+          }
+          st128(gt + i, vg.u);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) sgd_one(vp.f[j], vg.f[j], vm.f[j], u.sgd);
+          st128(pt + i, vp.u);
+          if (u.sgd.use_momentum) st128(mt + i, vm.u);
+        }
+        if (head != 0 && threadIdx.x < 4) {            // the elements ahead of the vectors and behind them
+          const int t = static_cast<int>(threadIdx.x), i = t < head ? t : kDenseTile - 4 + t;
+          float pv = pt[i], mv = u.sgd.use_momentum ? mt[i] : 0.f;
+          const float gv = out[i];
+          gt[i] = gv;
+          sgd_one(pv, gv, mv, u.sgd);
+          pt[i] = pv;
+          if (u.sgd.use_momentum) mt[i] = mv;
+        }
+        if (a.off[target + 1] == stop && target + 1 < a.targets) ++target;
+        continue;
       }
     }
     // store the tile to the tensors it overlaps
@@ -1503,6 +1586,19 @@ int check_common(const float* g, size_t n, const void* idx_out, void* ws, size_t
   if (n > 0x7fffffffu) return SGB_ERR_SIZE;  // 1-based int32 indices on the wire
   if (!ws || ws_bytes < workspace_bytes(n) || (reinterpret_cast<uintptr_t>(ws) & 255u))
     return SGB_ERR_WORKSPACE;
+  return SGB_OK;
+}
+
+// Lets a kernel have `bytes` of dynamic shared memory beside its own, once per device.
+template <typename K>
+int more_shared_memory(K kernel, size_t bytes, std::atomic<bool>* done) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  const bool tracked = dev >= 0 && dev < 64;
+  if (tracked && done[dev].load(std::memory_order_acquire)) return SGB_OK;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e != cudaSuccess) return note_cuda_error(e);
+  if (tracked) done[dev].store(true, std::memory_order_release);
   return SGB_OK;
 }
 
@@ -1895,12 +1991,25 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
     a.last = at;
     a.off[a.targets] = at;
     const size_t tiles = ceil_div(a.last - a.first, kDenseTile);
-    const unsigned per = static_cast<unsigned>(ceil_div(tiles, static_cast<size_t>(sm_count()) * (update ? 5 : 8)));
+    // A CTA's tiles: few enough that those whose entries crowd (the first elements of a
+    // bucket whose keys tie) are spread over the GPU, where they are updated as well.  As many
+    // as fill the GPU once, 16, 8 and 4 of them: 3.1e7 elements, the first 4.8 % sent, 218 / 218 /
+    // 195 / 185 us a pass; 1e8, 1 % anywhere, 629 / 609 / 601 / 594; 2.56e7 in 16 buckets 172 /
+    // 172 / 170 / 165.  Without the update 5e7 elements at 2.6 standard deviations took 323
+    // instead of 317.
+    const size_t even = ceil_div(tiles, static_cast<size_t>(sm_count()) * (update ? kUpdateCtas : 8));
+    const unsigned per = static_cast<unsigned>(update && even > kMostTiles ? kMostTiles : even);
     const dim3 grid(static_cast<unsigned>(ceil_div(tiles, per)));
-    const int st = update ? launch_ex(dense_from_payloads_kernel<true, DenseUpdate>, grid, dim3(kBlock), 0, s, 0, true, a, per, u)
-                          : launch_ex(world == 1 ? dense_from_payloads_kernel<true, NoUpdate>
-                                                 : dense_from_payloads_kernel<false, NoUpdate>,
-                                      grid, dim3(kBlock), 0, s, 0, true, a, per, NoUpdate{});
+    int st;
+    if (update) {
+      static std::atomic<bool> ready[64];
+      st = more_shared_memory(dense_from_payloads_kernel<true, DenseUpdate>, kUpdateStage, ready);
+      if (st == SGB_OK)
+        st = launch_ex(dense_from_payloads_kernel<true, DenseUpdate>, grid, dim3(kBlock), kUpdateStage, s, 0, true, a, per, u);
+    } else {
+      st = launch_ex(world == 1 ? dense_from_payloads_kernel<true, NoUpdate> : dense_from_payloads_kernel<false, NoUpdate>,
+                     grid, dim3(kBlock), 0, s, 0, true, a, per, NoUpdate{});
+    }
     if (st != SGB_OK) return st;
   }
   return launch_status();

@@ -19,6 +19,16 @@ LISTS = [([40000] * 40, 20000, 0), ([30001] * 75, 25000, 0), ([4097] * 300, 6000
          ([1 << 21] * 17 + [5], 1 << 20, 0)]
 
 
+# whole tiles and their ends, on and off a vector's boundary; one tensor by threshold, of any size that one selection takes
+ONE = [(4096, 0), (4097, 0), (8191, 1), (4000001, 0), (5000003, 2), (1 << 25, 0)]
+
+
+@pytest.mark.parametrize("size, offset", ONE)
+@pytest.mark.parametrize("topk, spars", [(False, 2.0), (True, 0.03)])
+def test_one_tensor(size, offset, topk, spars):
+    compare([size], 1 << 22, offset, "magnitude", topk, spars, 1 << 25)
+
+
 @pytest.mark.parametrize("sizes, threshold, offset", LISTS)
 @pytest.mark.parametrize("mode", ["magnitude", "compat"])
 def test_topk_of_long_lists(sizes, threshold, offset, mode):
