@@ -1423,18 +1423,26 @@ int takes_cluster(long long per_channel, bool vec, int C, int* per_cta) {
 // Whether a call takes the form that visits its data twice (bn_revisit.cu).  It
 // overlaps everything but its first loads and last stores, which a call has to be
 // large enough for; the line is the same whatever the mask, so that a fused call
-// and its parts agree bit for bit.  Time of the forms below / of this one, with and
-// without a ReLU:
-//   32x128x28x28  (3.2e6 elements)  14.0 / 11.9    9.9 / 10.2
-//   12x48x80x80   (3.7e6)           14.0 / 13.3   10.1 / 11.3
-//   32x40x56x56   (4.0e6)           16.2 / 13.9   11.3 / 11.3
-//   8x512x32x32   (4.2e6)           18.3 / 15.6   13.8 / 13.2
-//   32x1024x14x14 (6.4e6)           24.1 / 22.0   18.3 / 18.5
-//   12x200x50x50  (6.0e6)           25.4 / 20.0   17.4 / 16.1
+// and its parts agree bit for bit, and lies where a call without a ReLU loses nothing.
+// Time of the forms below / of this one, with and without a ReLU:
+//   16x64x56x56   (3.2e6 elements)  14.0 / 11.2   10.2 /  9.6
+//   32x128x28x28  (3.2e6)           13.7 / 11.1    9.9 /  9.9
+//   32x512x14x14  (3.2e6)           14.0 / 11.8    9.8 /  9.9
+//   8x512x28x28   (3.2e6)           13.8 / 11.6    9.9 /  9.4
+//   12x48x80x80   (3.7e6)           14.1 / 13.2   10.1 / 10.5
+//   32x1024x14x14 (6.4e6)           24.1 / 20.7   18.3 / 16.8
+//   12x200x50x50  (6.0e6)           25.4 / 19.2   17.4 / 15.4
+// smaller ones: 10x256x30x30 (2.3e6) 10.8 / 9.5, 7.8 / 8.2; 8x256x32x32 (2.1e6) 10.3 / 8.9,
+// 7.5 / 8.3; 16x128x28x28 (1.6e6) 8.3 / 6.9, 6.3 / 6.0; and channels that one CTA's
+// registers hold: 4x512x32x32 6.8 / 8.9, 4.9 / 7.5; 24x1024x8x8 5.4 / 7.3, 4.1 / 6.8.
 // Planes that are no multiple of four pay for their masked ends twice:
-//   24x64x71x71   (7.7e6)           40.0 / 28.1   27.6 / 23.7
-//   18x256x33x33  (5.0e6)           25.4 / 19.8   16.1 / 17.0
-//   24x1024x15x15 (5.5e6)           28.6 / 22.6   17.9 / 20.2
+//   24x64x71x71   (7.7e6)           40.0 / 26.4   27.6 / 20.4
+//   12x64x79x79   (4.8e6)           29.8 / 18.0   17.0 / 14.8
+//   18x256x33x33  (5.0e6)           25.1 / 19.0   16.2 / 15.3
+//   16x512x25x25  (5.1e6)           25.7 / 19.6   16.3 / 15.1
+//   24x128x39x39  (4.7e6)           24.3 / 17.8   16.4 / 14.2
+// smaller ones: 24x64x45x45 (3.1e6) 16.0 / 13.6, 10.4 / 11.1; 16x64x51x51 (2.7e6) 14.6 / 12.5,
+// 9.7 / 10.4.
 // Two costs grow with the items of a channel: the lead of the first visit over the
 // second (what lies between them has to stay in L2), and every CTA's reading of all
 // the channel's sums.  Large channels therefore take the forms below, unless the
@@ -1454,8 +1462,12 @@ int takes_cluster(long long per_channel, bool vec, int C, int* per_cta) {
 //   32x3x397x397    5.0e6, 1.5e7   86.3 / 141.0    58.2 / 128.1
 inline bool revisit_pays(int N, int C, int HW, bool aligned, bool groups) {
   const long long channel = static_cast<long long>(N) * HW, elements = channel * C;
-  if (HW % 4) return aligned && !groups && HW >= 2500 && elements >= 6000000 && channel <= 1000000;
-  return aligned && HW >= 8 && elements >= 4000000 && (channel <= 4000000 || elements <= 20000000);
+  const bool shared = channel > 6144;                  // a channel is more than one CTA's registers hold
+  if (HW % 4)
+    return aligned && !groups && channel <= 1000000 &&
+           ((HW >= 400 && elements >= 4400000 && shared) || (HW >= 2500 && elements >= 6000000));
+  return aligned && HW >= 8 && (elements >= 4000000 || (elements >= 3000000 && shared)) &&
+         (channel <= 4000000 || elements <= 20000000);
 }
 
 template <int MASK>

@@ -570,9 +570,13 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
 
 // One operand is little to overlap with, so only channels that leave clusters with
 // large shares or no place at all gain (us, the forms above and below / this one):
-//   32x64x112x112 61.5 / 41.3   32x64x56x56 14.9 / 14.2    64x100x40x40  19.4 / 19.6
-//   32x512x28x28 25.3 / 26.6    10x256x52x52 15.3 / 15.9   32x64x111x111 99.1 / 53.1
-//   32x128x57x57 37.3 / 28.7    24x64x71x71 24.4 / 18.8    16x1024x13x13 14.1 / 14.5
+//   32x64x112x112 61.5 / 40.5   32x64x56x56 14.9 / 13.3    64x100x40x40  19.4 / 18.5
+//   32x512x28x28 25.4 / 24.7    10x256x52x52 15.5 / 14.8   12x200x50x50  12.5 / 13.7
+// and odd planes, whose clusters read with masked ends:
+//   32x128x57x57 37.3 / 28.6    24x64x71x71 24.4 / 18.4    24x64x57x57   18.9 / 14.7
+//   40x32x51x51  13.7 / 10.2    24x64x37x37  9.9 / 8.8     33x128x35x35  16.9 / 15.6
+//   12x64x69x69  12.6 / 11.9    40x64x31x31 10.3 / 10.3    18x100x47x47  12.9 / 13.3
+//   18x256x25x25 11.1 / 11.6 (11,250 elements a channel), 4x128x57x57 8.5 / 8.9 (12,996)
 // The lower line for whole vectors is from a layer's forward, ReLU and backward in
 // sequence: what the second visit leaves in L2 is x, and what comes next reads y
 // (elements of a channel: 69,000 134.3 / 136.7, 75,000 145.4 / 147.9, 88,000 149.7 /
@@ -583,7 +587,9 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
 // and 3.5e7 142.0 / 156.5, 4.0e6 and 3.2e7 155.7 / 187.4.
 inline bool fwd_revisit_pays(int N, int C, int HW) {
   const long long channel = static_cast<long long>(N) * HW, elements = channel * C;
-  if (HW % 4) return HW >= 2500 && elements >= 6000000 && channel <= 2600000;
+  if (HW % 4)
+    return channel <= 2600000 &&
+           ((HW >= 900 && elements >= 2000000 && channel >= 32000) || (HW >= 2500 && elements >= 6000000));
   return HW >= 2500 && channel >= 96000 && elements >= 6000000 && (channel <= 4000000 || elements <= 20000000);
 }
 
