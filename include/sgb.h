@@ -500,6 +500,15 @@ int sgb_sgd_update_multi_f32(void *const *params, void *const *grads,
                              size_t count, float lr, float momentum,
                              float dampening, float weight_decay, int nesterov,
                              float grad_scale, void *stream);
+/* The same results from one thread block per SM, which leaves room for the kernels of
+ * another stream: an update beside the rest of a backward pass.  round_f16: the gradients
+ * are first rounded to fp16 and widened again, where they are (what a one-rank exchange
+ * in half precision makes of them, sgb_comm_update_half). */
+int sgb_sgd_update_beside_f32(void *const *params, void *const *grads,
+                              void *const *moments, const size_t *sizes,
+                              size_t count, float lr, float momentum,
+                              float dampening, float weight_decay, int nesterov,
+                              float grad_scale, int round_f16, void *stream);
 
 /* ------------------------------------------------ bucket pack / unpack */
 /* Gather a HOST list of fp32 tensors into a flat device buffer starting at

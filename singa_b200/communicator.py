@@ -44,6 +44,7 @@ class Communicator(object):
         self.local_rank = int(local_rank)
         self.global_rank = int(local_rank)
         self.world_size = int(world_size)
+        self.buffSize = int(buffSize)
         torch.cuda.set_device(self.local_rank)
         torch.cuda.current_stream().synchronize()   # context exists before NCCL init
         handle = C.c_void_p()

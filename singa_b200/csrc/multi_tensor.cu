@@ -107,6 +107,63 @@ sgd_multi_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
   }
 }
 
+// The same by one CTA an SM that walks the tiles, two at a time: for an update beside a
+// chain of small kernels, which finds room on every SM.  A ResNet-50 step at batch 2 and
+// images of 159, us: the update behind the chain 240, on a branch with all the CTAs that the
+// SMs hold 228, with four an SM 239, three 230, two 227, one 206.
+template <int N, bool ROUND>
+__global__ void __launch_bounds__(kBlock)
+sgd_beside_kernel(const __grid_constant__ Table<N> t, const SgdArgs a) {
+  constexpr int kAbreast = 2;
+  dependency_wait();
+  release_dependents();
+  const unsigned tiles = t.first_tile[t.count];
+  for (unsigned first = blockIdx.x; first < tiles; first += kAbreast * gridDim.x) {
+    float *p[kAbreast], *g[kAbreast], *m[kAbreast];
+    int left[kAbreast];                                // elements from this thread's first on
+    Vec4f vp[kAbreast], vg[kAbreast], vm[kAbreast];
+#pragma unroll
+    for (int k = 0; k < kAbreast; ++k) {
+      const unsigned tile = first + k * gridDim.x;
+      left[k] = 0;
+      if (tile >= tiles) continue;
+      const int j = find_tensor(t, tile);
+      const size_t i = static_cast<size_t>(tile - t.first_tile[j]) * kTile + 4 * threadIdx.x;
+      if (i >= t.n[j]) continue;
+      left[k] = t.n[j] - i < 4 ? static_cast<int>(t.n[j] - i) : 4;
+      p[k] = static_cast<float*>(t.a[j]) + i;
+      g[k] = static_cast<float*>(t.b[j]) + i;
+      m[k] = a.use_momentum ? static_cast<float*>(t.c[j]) + i : nullptr;
+      if (left[k] < 4) continue;
+      vp[k] = ld4(p[k]);
+      vg[k] = ld4(g[k]);
+      if (a.use_momentum) vm[k] = ld4(m[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kAbreast; ++k) {
+      if (left[k] == 4) {
+        if (ROUND) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) vg[k].f[j] = __half2float(__float2half_rn(vg[k].f[j]));
+          st4(g[k], vg[k]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sgd_one(vp[k].f[j], vg[k].f[j], vm[k].f[j], a);
+        st4(p[k], vp[k]);
+        if (a.use_momentum) st4(m[k], vm[k]);
+      } else {
+        for (int j = 0; j < left[k]; ++j) {
+          float pv = p[k][j], gv = g[k][j], mv = a.use_momentum ? m[k][j] : 0.f;
+          if (ROUND) g[k][j] = gv = __half2float(__float2half_rn(gv));
+          sgd_one(pv, gv, mv, a);
+          p[k][j] = pv;
+          if (a.use_momentum) m[k][j] = mv;
+        }
+      }
+    }
+  }
+}
+
 // kRoundF16: the tensors are rounded to fp16 and widened again where they are
 // (what packing, a one-rank all-reduce and unpacking do to them).
 enum PackMode { kPackF32 = 0, kPackF32ToF16 = 1, kUnpackF32 = 2, kUnpackF16ToF32 = 3, kRoundF16 = 4 };
@@ -285,7 +342,7 @@ int pack_common(int mode, void* const* tensors, const size_t* sizes, size_t coun
 // One launch for as many tensors as the table holds.
 template <int N, bool ROUND>
 int sgd_list(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
-             const SgdArgs& a, cudaStream_t s) {
+             const SgdArgs& a, bool beside, cudaStream_t s) {
   const bool use_m = a.use_momentum;
   for (size_t first = 0; first < count;) {
     Table<N> t;
@@ -315,8 +372,11 @@ int sgd_list(void* const* params, void* const* grads, void* const* moments, cons
     }
     if (cnt == 0) continue;
     const unsigned tiles = fill_table<N>(t, nullptr, pa, pb, pc, ns, 0, cnt, 0);
-    const int st = launch_ex(any ? sgd_multi_kernel<N, ROUND, true> : sgd_multi_kernel<N, ROUND, false>, dim3(tiles),
-                             dim3(kBlock), 0, s, 0, true, t, a);
+    const unsigned few = static_cast<unsigned>(sm_count());
+    const int st = launch_ex(beside ? sgd_beside_kernel<N, ROUND>
+                             : any  ? sgd_multi_kernel<N, ROUND, true>
+                                    : sgd_multi_kernel<N, ROUND, false>,
+                             dim3(beside && few < tiles ? few : tiles), dim3(kBlock), 0, s, 0, true, t, a);
     if (st != SGB_OK) return st;
   }
   return launch_status();
@@ -324,16 +384,16 @@ int sgd_list(void* const* params, void* const* grads, void* const* moments, cons
 
 template <bool ROUND>
 int sgd_any(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
-            const SgdArgs& a, cudaStream_t s) {
-  return count <= kSmallTable ? sgd_list<kSmallTable, ROUND>(params, grads, moments, sizes, count, a, s)
-                              : sgd_list<kLargeTable, ROUND>(params, grads, moments, sizes, count, a, s);
+            const SgdArgs& a, bool beside, cudaStream_t s) {
+  return count <= kSmallTable ? sgd_list<kSmallTable, ROUND>(params, grads, moments, sizes, count, a, beside, s)
+                              : sgd_list<kLargeTable, ROUND>(params, grads, moments, sizes, count, a, beside, s);
 }
 
 }  // namespace
 
 int sgd_round_f16_multi(void* const* params, void* const* grads, void* const* moments, const size_t* sizes, size_t count,
                         const SgdArgs& a, cudaStream_t s) {
-  return sgd_any<true>(params, grads, moments, sizes, count, a, s);
+  return sgd_any<true>(params, grads, moments, sizes, count, a, false, s);
 }
 
 int round_f16_multi(void* const* tensors, const size_t* sizes, size_t count, cudaStream_t s) {
@@ -355,7 +415,19 @@ int sgb_sgd_update_multi_f32(void* const* params, void* const* grads, void* cons
   SgdArgs a;
   const int st = sgd_args(&a, moments, lr, momentum, dampening, weight_decay, nesterov, grad_scale);
   if (st != SGB_OK) return st;
-  return sgd_any<false>(params, grads, moments, sizes, count, a, as_stream(stream));
+  return sgd_any<false>(params, grads, moments, sizes, count, a, false, as_stream(stream));
+}
+
+int sgb_sgd_update_beside_f32(void* const* params, void* const* grads, void* const* moments, const size_t* sizes,
+                              size_t count, float lr, float momentum, float dampening, float weight_decay, int nesterov,
+                              float grad_scale, int round_f16, void* stream) {
+  if (count == 0) return SGB_OK;
+  if (!params || !grads || !sizes) return SGB_ERR_NULL;
+  SgdArgs a;
+  const int st = sgd_args(&a, moments, lr, momentum, dampening, weight_decay, nesterov, grad_scale);
+  if (st != SGB_OK) return st;
+  return round_f16 ? sgd_any<true>(params, grads, moments, sizes, count, a, true, as_stream(stream))
+                   : sgd_any<false>(params, grads, moments, sizes, count, a, true, as_stream(stream));
 }
 
 int sgb_sgd_update_f32(float* param, const float* grad, float* moment, size_t n, float lr,

@@ -1093,18 +1093,49 @@ const Callable kCallables[] = {
     CALLABLE(sgb_unpack_f32), CALLABLE(sgb_sgd_update_multi_f32), CALLABLE(sgb_comm_synch),
     CALLABLE(sgb_comm_synch_half), CALLABLE(sgb_comm_fused_synch), CALLABLE(sgb_comm_fused_synch_half),
     CALLABLE(sgb_comm_sparsification), CALLABLE(sgb_comm_wait), CALLABLE(sgb_comm_profile_mark),
-    CALLABLE(sgb_comm_profile_range),
+    CALLABLE(sgb_comm_profile_range), CALLABLE(sgb_comm_update_half), CALLABLE(sgb_sgd_update_beside_f32),
 };
 
-enum Patch { kStream, kResultStream, kResultIndex, kLr, kMomentum, kDecay, kPatches };
-const char* const kPatchNames[kPatches] = {"STREAM", "RESULT_STREAM", "RESULT_INDEX", "LR", "MOMENTUM", "DECAY"};
+enum Patch { kStream, kSideStream, kResultStream, kResultIndex, kLr, kMomentum, kDecay, kPatches };
+const char* const kPatchNames[kPatches] = {"STREAM", "SIDE_STREAM", "RESULT_STREAM", "RESULT_INDEX", "LR", "MOMENTUM", "DECAY"};
+
+// When a call of a program is issued.  A forked run is one into a capture: "fork" and
+// "join" order the side stream behind the main one and back, and what a run does there
+// is a branch of the graph.  (One by one, the two events of a fork cost the host more
+// than the branch saves, and threads that run a program would share them.)
+enum When { kAlways, kProfiled, kForked, kUnforked };
 
 constexpr size_t kMaxArguments = 24;
 struct Call {
-  const Callable* fn;
+  const Callable* fn;                        // null: a fork or a join
   std::vector<Slot> slots;
   std::vector<std::pair<size_t, int>> patches;
-  bool profile_only;
+  int when;
+  bool join = false;
+};
+// The side stream of a program that forks, below the priority of what it runs beside.
+struct Side {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t event = nullptr;
+  Side() = default;
+  Side(const Side&) = delete;
+  Side& operator=(const Side&) = delete;
+  ~Side() {
+    if (event) cudaEventDestroy(event);
+    if (stream) cudaStreamDestroy(stream);
+  }
+  bool open() {
+    int least = 0, greatest = 0;
+    const bool ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
+                    cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, least) == cudaSuccess &&
+                    cudaEventCreateWithFlags(&event, cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  }
+  // Everything of `from` so far, in front of whatever comes to `to`.
+  bool order(cudaStream_t from, cudaStream_t to) const {
+    return cudaEventRecord(event, from) == cudaSuccess && cudaStreamWaitEvent(to, event, 0) == cudaSuccess;
+  }
 };
 // What a recorded step depends on besides its arguments: if this is the same as
 // in the run before, so are its launches.
@@ -1139,7 +1170,8 @@ struct Program {
   unsigned eager = 2;         // of which so many are launched one by one
   unsigned captures = 0;
   cudaGraphExec_t exec = nullptr;
-  std::mutex guard;           // of the five fields above
+  std::unique_ptr<Side> side; // where the program forks
+  std::mutex guard;           // of the six fields above
 };
 constexpr unsigned kEagerRuns = 2, kPaysAfter = 40, kMostEagerRuns = 1u << 16;
 const char kProgramTag[] = "singa_b200.program";
@@ -1152,7 +1184,8 @@ void drop_program(PyObject* capsule) {
   delete p;
 }
 
-// (list of (function name, argument tuple, profile only), communicator | None[, graphable]) -> program
+// (list of (function name, argument tuple, when), communicator | None[, graphable]) -> program;
+// "fork" and "join" stand for themselves
 PyObject* py_program(Args a, Py_ssize_t n) {
   PyObject* seq = PySequence_Fast(a[0], "a list of calls is expected");
   if (!seq) throw PyError{};
@@ -1164,15 +1197,25 @@ PyObject* py_program(Args a, Py_ssize_t n) {
     PyObject* item = PySequence_Fast_GET_ITEM(seq, k);
     const char* name;
     PyObject* args;
-    int profile_only;
-    if (!PyArg_ParseTuple(item, "sO!p", &name, &PyTuple_Type, &args, &profile_only)) throw PyError{};
+    int when;
+    if (!PyArg_ParseTuple(item, "sO!i", &name, &PyTuple_Type, &args, &when)) throw PyError{};
+    if (when < kAlways || when > kUnforked) fail(PyExc_ValueError, "no such time for a call");
+    const bool join = !strcmp(name, "join");
+    if (join || !strcmp(name, "fork")) {
+      prog->calls.push_back(Call{nullptr, {}, {}, kForked, join});
+      if (!prog->side) {
+        prog->side = std::make_unique<Side>();
+        if (!prog->side->open()) fail(PyExc_RuntimeError, "no side stream for a program");
+      }
+      continue;
+    }
     const Callable* fn = nullptr;
     for (const Callable& c : kCallables)
       if (!strcmp(c.name, name)) fn = &c;
     if (!fn) fail(PyExc_ValueError, std::string("no such call in a step: ") + name);
     if (fn->arity > kMaxArguments || static_cast<size_t>(PyTuple_GET_SIZE(args)) != fn->arity)
       fail(PyExc_TypeError, std::string(name) + ": wrong number of arguments");
-    Call call{fn, {}, {}, profile_only != 0};
+    Call call{fn, {}, {}, when};
     for (size_t i = 0; i < fn->arity; ++i) {
       PyObject* v = PyTuple_GET_ITEM(args, i);
       Slot s{};
@@ -1198,17 +1241,25 @@ PyObject* py_program(Args a, Py_ssize_t n) {
   return cap;
 }
 
-// Issues the calls in order on `st`; on a failure `where` names the call.
-int issue_calls(const Program* prog, const Settings& now, bool profile, void* st, const char** where) {
+// Issues the calls in order on `st`, forking to `side` where there is one; on a failure
+// `where` names the call.
+int issue_calls(const Program* prog, const Settings& now, bool profile, void* st, const Side* side, const char** where) {
   Slot scratch_slots[kMaxArguments];
   for (const Call& c : prog->calls) {
-    if (c.profile_only && !profile) continue;
+    if (c.when == kProfiled ? !profile : c.when == kForked ? !side : c.when == kUnforked && side) continue;
+    if (!c.fn) {
+      const cudaStream_t main = static_cast<cudaStream_t>(st);
+      if (c.join ? side->order(side->stream, main) : side->order(main, side->stream)) continue;
+      *where = c.join ? "join" : "fork";
+      return SGB_ERR_CUDA;
+    }
     const Slot* slots = c.slots.data();
     if (!c.patches.empty()) {   // patched copies on this thread's stack: a program can run on several threads
       std::copy(c.slots.begin(), c.slots.end(), scratch_slots);
       for (const auto& [i, what] : c.patches) {
         switch (what) {
           case kStream: scratch_slots[i].p = st; break;
+          case kSideStream: scratch_slots[i].p = side ? side->stream : st; break;
           case kResultStream: scratch_slots[i].p = sgb_comm_result_stream(prog->comm); break;
           case kResultIndex: {
             void* r = sgb_comm_result_stream(prog->comm);
@@ -1242,7 +1293,7 @@ bool capture_calls(Program* prog, const Settings& now) {
   const char* where = "";
   bool ok = cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
-    ok = issue_calls(prog, now, false, side, &where) == SGB_OK;
+    ok = issue_calls(prog, now, false, side, prog->side.get(), &where) == SGB_OK;
     ok = cudaStreamEndCapture(side, &graph) == cudaSuccess && ok && graph;
   }
   cudaGraphExec_t exec = nullptr;
@@ -1267,8 +1318,9 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
   const Settings now{real(a[1]), real(a[2]), real(a[3]), sgb_get_option(SGB_OPT_OVERLAP_LAUNCHES),
                      current.device_index()};
   void* const st = current.stream();
-  const bool may_graph = prog->graphable && !profile && !sgb_comm_profiling(prog->comm) &&
-                         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
+  const bool plain = !profile && !sgb_comm_profiling(prog->comm);
+  const bool captured = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+  const bool may_graph = prog->graphable && plain && !captured;
   int status = SGB_OK;
   const char* where = "";
   Py_BEGIN_ALLOW_THREADS;
@@ -1298,7 +1350,15 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
       }
     }
   }
-  if (!launched) status = issue_calls(prog, now, profile, st, &where);
+  if (captured && plain && prog->side) {
+    // a caller's capture; one at a time, as there is one side stream
+    const std::lock_guard<std::mutex> lock(prog->guard);
+    cudaStreamCaptureStatus other = cudaStreamCaptureStatusActive;
+    const bool ours = cudaStreamIsCapturing(prog->side->stream, &other) == cudaSuccess && other == cudaStreamCaptureStatusNone;
+    status = issue_calls(prog, now, profile, st, ours ? prog->side.get() : nullptr, &where);
+  } else if (!launched) {
+    status = issue_calls(prog, now, profile, st, nullptr, &where);
+  }
   Py_END_ALLOW_THREADS;
   if (status != SGB_OK) fail_status(where, status);
   Py_RETURN_NONE;

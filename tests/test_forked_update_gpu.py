@@ -1,0 +1,81 @@
+"""A captured step without other ranks updates its buckets on a branch beside the
+backward pass: the same bits as the calls one by one, captured by the library or by
+the caller, for one bucket and for many, and whatever the exchange."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def step(sync, threshold, comm, **kw):
+    from singa_b200.hot_path import HotPathGPU
+    from singa_b200.resnet50_path import add_wgrad_refresh, build_mlp_plan, fuse_plan
+    plan = fuse_plan(build_mlp_plan(batch=9, dims=(23, 130, 57, 10)))
+    if sync != "none":
+        plan = add_wgrad_refresh(plan)
+    return HotPathGPU(plan, communicator=comm if sync != "none" else None, seed=5, threshold=threshold,
+                      dist_option=sync if sync != "none" else "plain", **kw)
+
+
+def state(hp):
+    torch.cuda.synchronize()
+    return [hp.t[p] for p in hp.plan["params"]] + [hp.moments[p] for p in hp.plan["params"]] + [hp.grad_arena, hp.t["loss"]]
+
+
+@pytest.mark.parametrize("sync", ["none", "plain", "half"])
+@pytest.mark.parametrize("threshold", [1, 200, 3000, 1 << 20])          # a bucket a tensor ... one bucket
+@pytest.mark.parametrize("on_arrival", [True, False])
+def test_captured_steps_equal_single_calls(sync, threshold, on_arrival):
+    from singa_b200.communicator import Communicator, NcclIdHolder
+    comm = Communicator(torch.cuda.current_device(), 1, NcclIdHolder(), buffSize=1 << 20)
+    make = lambda: step(sync, threshold, comm, update_on_arrival=on_arrival)   # noqa: E731
+    single, library, caller = make(), make(), make()
+    single.profile = True                        # one by one
+    caller.run_step()
+    torch.cuda.synchronize()
+    graph = caller.capture()
+    for k in range(6):
+        single.run_step()
+        library.run_step()
+        if k:
+            graph.replay()
+    for other in (library, caller):
+        assert all(torch.equal(a, b) for a, b in zip(state(single), state(other))), (sync, threshold)
+    caller.release_graph()
+    del graph
+    comm.close()
+
+
+def test_what_does_not_fit_the_communicator_is_still_refused():
+    from singa_b200 import _lib
+    from singa_b200.communicator import Communicator, NcclIdHolder
+    comm = Communicator(torch.cuda.current_device(), 1, NcclIdHolder(), buffSize=64)
+    for sync in ("plain", "half"):
+        hp = step(sync, 1 << 20, comm)
+        for _ in range(4):
+            with pytest.raises(_lib.SgbError):
+                hp.run_step()
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("sizes", [[1, 5, 1023, 1024, 1025], [700001, 3], [7] * 100])    # one walk of the tiles, several; a long table
+@pytest.mark.parametrize("offset", [0, 1, 2])
+@pytest.mark.parametrize("round_f16", [0, 1])
+def test_the_narrow_update_has_the_bits_of_the_wide_one(sizes, offset, round_f16):
+    import ctypes
+    from singa_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(6)
+    make = lambda: [torch.randn(n + 4, device="cuda", generator=g)[offset:offset + n] for n in sizes]   # noqa: E731
+    p, d, m = make(), make(), make()
+    copies = [[t.clone() for t in ts] for ts in (p, d, m)]
+    n, stream = len(sizes), torch.cuda.current_stream().cuda_stream
+    table = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])   # noqa: E731
+    counts = (ctypes.c_size_t * n)(*sizes)
+    rates = (0.1, 0.9, 0.0, 1e-3, 0, 0.5)
+    _lib.call("sgb_sgd_update_beside_f32", table(p), table(d), table(m), counts, n, *rates, round_f16, stream)
+    cp, cd, cm = copies
+    if round_f16:
+        for t in cd:
+            t.copy_(t.half().float())
+    _lib.call("sgb_sgd_update_multi_f32", table(cp), table(cd), table(cm), counts, n, *rates, stream)
+    assert all(torch.equal(a, b) for x, y in ((p, cp), (d, cd), (m, cm)) for a, b in zip(x, y))
