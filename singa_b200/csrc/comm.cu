@@ -90,6 +90,12 @@ struct sgb_comm {
   int *joint_pay = nullptr, *joint_nnz = nullptr;
   void* joint_ws = nullptr;
   size_t joint_elems = 0, joint_ws_bytes = 0;
+  // How many bytes of counters at the start of a workspace the last exchange's dense sum
+  // has set to 0; never again once a graph holds the workspace (its replays use it too).
+  struct Cleared {
+    size_t bytes = 0;
+    bool captured = false;
+  } ws_clear, joint_clear;
   std::vector<void*> joint_retired;
   unsigned sparse_begun = 0, sparse_ended = 0;
   unsigned long long* dropped_dev = nullptr;   // entries the bounded threshold form left for later calls
@@ -738,6 +744,18 @@ int sgb_comm_round_half(sgb_comm* c, void* const* tensors, const size_t* sizes, 
   return sgb::round_f16_multi(tensors, sizes, count, c->c1);
 }
 
+// Whether the first `bytes` of a workspace are clear, which they no longer count as: the
+// selection uses them.  (Two microseconds of a pass went by between the call that cleared
+// them and the selection.)
+static bool take_cleared(sgb_comm* c, sgb_comm::Cleared* w, size_t bytes, cudaStream_t compute) {
+  w->captured = w->captured || capturing(compute) || capturing(c->c1);
+  const bool clear = !w->captured && w->bytes >= bytes;
+  w->bytes = 0;
+  return clear;
+}
+// The dense sum that clears them has been launched.
+static void now_cleared(sgb_comm::Cleared* w, size_t bytes) { w->bytes = w->captured ? 0 : bytes; }
+
 // The selection half.  capacity == 0: the reference's exchange (the payload is
 // as long as the largest count, which the host reads back).  capacity > 0
 // (threshold mode): every rank sends exactly `capacity` slots, no host round trip.
@@ -779,6 +797,7 @@ static int sparse_begin(sgb_comm* c, void* const* tensors, const size_t* sizes, 
       grad_sizes = &x.n;
       ngrads = 1;
     }
+    take_cleared(c, &c->ws_clear, 0, sgb::as_stream(compute_stream));   // (clears for itself, and leaves its own behind)
     if (topk) {
       x.nnz_max = static_cast<size_t>(sgb_topk_count(spars, n));
       for (int r = 0; r < c->world; ++r) x.nnz_host[r] = static_cast<int>(x.nnz_max);
@@ -887,6 +906,7 @@ static int joint_reserve(sgb_comm* c, size_t span, cudaStream_t compute, size_t 
   if (c->joint_ws) c->joint_retired.push_back(c->joint_ws);
   c->joint_ws = ws;
   c->joint_ws_bytes = ws_bytes;
+  c->joint_clear = {};
   c->joint_elems = elems;
   return SGB_OK;
 }
@@ -917,12 +937,15 @@ static int threshold_buckets(sgb_comm* c, const std::vector<sgb::SparseBucket>& 
   Phase ph(c, "Dist_c1c2_fusedSparsification", sgb::order::kStreamC1);
   size_t k = 0, tensor = 0;
   for (const size_t end : ends) {
+    const size_t counters = sgb::sparse_counter_bytes(1);
     OK(sgb::sparse_threshold_buckets(list.data() + k, end - k, threshold, c->joint_pay, c->joint_nnz, c->joint_ws,
-                                     c->joint_ws_bytes, c->c1));
+                                     c->joint_ws_bytes, c->c1, take_cleared(c, &c->joint_clear, counters, compute)));
     sgb::SparseUpdate part{};
     if (update)
       part = {update->sgd, update->params + tensor, update->moments ? update->moments + tensor : nullptr};
-    OK(sgb::sparse_dense_buckets(c->joint_pay, 0, c->joint_nnz, list.data() + k, end - k, c->c1, update ? &part : nullptr));
+    OK(sgb::sparse_dense_buckets(c->joint_pay, 0, c->joint_nnz, list.data() + k, end - k, c->c1, update ? &part : nullptr,
+                                 {c->joint_ws, counters}));
+    now_cleared(&c->joint_clear, counters);
     for (; k < end; ++k) tensor += list[k].count;
   }
   return SGB_OK;
@@ -1023,10 +1046,14 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
     k = 0;
     for (const size_t end : ends) {
       int sent = 0;
+      const size_t counters = sgb::sparse_counter_bytes(end - k);
       OK(sgb::sparse_topk_buckets(list.data() + k, ks.data() + k, end - k, c->topk_mode, c->joint_pay, &sent,
-                                  c->joint_ws, c->joint_ws_bytes, c->c1));
+                                  c->joint_ws, c->joint_ws_bytes, c->c1,
+                                  take_cleared(c, &c->joint_clear, counters, compute)));
       const sgb::SparseUpdate part{&sgd, update.params + tensor, update.moments ? update.moments + tensor : nullptr};
-      OK(sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data() + k, end - k, c->c1, &part));
+      OK(sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data() + k, end - k, c->c1, &part,
+                                   {c->joint_ws, counters}));
+      now_cleared(&c->joint_clear, counters);
       for (; k < end; ++k) tensor += list[k].count;
     }
     return SGB_OK;
@@ -1040,10 +1067,15 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
   const sgb::SparseBucket& b = list[0];
   const size_t n = total_of(b.sizes, b.count), k = static_cast<size_t>(sgb_topk_count(spars, n));
   const int sent[1] = {static_cast<int>(k)};
+  const size_t counters = sgb::sparse_counter_bytes(1);
   if (k)
     OK(sgb::sparse_topk(b.tensors, b.sizes, b.count, b.acc, k, c->topk_mode, x.pay_send,
-                        reinterpret_cast<float*>(x.pay_send) + k, c->ws, c->ws_bytes, c->c1));
-  return sgb::sparse_dense_sum(x.pay_send, 0, 0, sent, nullptr, 1, b.tensors, b.sizes, b.count, c->c1, &update);
+                        reinterpret_cast<float*>(x.pay_send) + k, c->ws, c->ws_bytes, c->c1,
+                        take_cleared(c, &c->ws_clear, counters, compute)));
+  OK(sgb::sparse_dense_sum(x.pay_send, 0, 0, sent, nullptr, 1, b.tensors, b.sizes, b.count, c->c1, &update,
+                           {c->ws, k ? counters : 0}));
+  if (k) now_cleared(&c->ws_clear, counters);
+  return SGB_OK;
 }
 
 int sgb_comm_update_half(sgb_comm* c, void* const* params, void* const* grads, void* const* moments,

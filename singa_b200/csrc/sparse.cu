@@ -1324,6 +1324,8 @@ struct DenseArgs {
   int world;
   int counts[kMaxDenseRanks];
   size_t first, last;          // element range of this launch
+  uint4* clear;                // set to 0 on the way, for the next selection
+  unsigned clear_vecs;
   int targets;
   size_t off[kDenseTargets + 1];   // first element of each target tensor; off[targets] == last
   float* ptr[kDenseTargets];
@@ -1421,6 +1423,8 @@ dense_from_payloads_kernel(const __grid_constant__ DenseArgs a, unsigned tiles_p
   __shared__ unsigned cursor[kMaxDenseRanks], count[kMaxDenseRanks];
   dependency_wait();
   release_dependents();
+  for (unsigned i = blockIdx.x * kBlock + threadIdx.x; i < a.clear_vecs; i += gridDim.x * kBlock)
+    a.clear[i] = make_uint4(0, 0, 0, 0);
   const size_t begin = a.first + static_cast<size_t>(blockIdx.x) * tiles_per_cta * kDenseTile;
   const size_t end = begin + static_cast<size_t>(tiles_per_cta) * kDenseTile < a.last
                          ? begin + static_cast<size_t>(tiles_per_cta) * kDenseTile : a.last;
@@ -1719,7 +1723,7 @@ inline unsigned sample_target(size_t n, size_t k, int mode, const Work& work) {
 }
 
 int topk_launch(const Gradient& source, float* acc, size_t k, int mode, int* idx_out, float* val_out, void* ws,
-                size_t ws_bytes, cudaStream_t s) {
+                size_t ws_bytes, cudaStream_t s, bool cleared = false) {
   const size_t n = source.n;
   if (n == 0 || k == 0) return SGB_OK;
   if (mode != 0 && mode != 1) return SGB_ERR_UNSUPPORTED;
@@ -1731,8 +1735,10 @@ int topk_launch(const Gradient& source, float* acc, size_t k, int mode, int* idx
   const Work work = work_for(n);
   TopkArgs a{g, acc, n, static_cast<unsigned>(k), sample_target(n, k, mode, work), work, carve(ws, work), idx_out, val_out,
              aligned16(g) && (!acc || aligned16(acc)), 0};
-  cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
-  if (e != cudaSuccess) return note_cuda_error(e);
+  if (!cleared) {
+    const cudaError_t e = cudaMemsetAsync(a.ws.counters, 0, sizeof(Counters), s);
+    if (e != cudaSuccess) return note_cuda_error(e);
+  }
   if (!source.flat)
     return mode == 0 ? launch_cooperative(topk_select_kernel<0, Pieces>, work.grid, a, source.pieces, s)
                      : launch_cooperative(topk_select_kernel<1, Pieces>, work.grid, a, source.pieces, s);
@@ -1749,8 +1755,10 @@ size_t sparse_buckets_span(const SparseBucket* buckets, size_t count) {
   return gather_buckets(&b, buckets, count, &span) ? span : 0;
 }
 
+size_t sparse_counter_bytes(size_t buckets) { return buckets * align256(sizeof(Counters)); }
+
 int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float thr, int* payload, int* nnz_dev, void* ws,
-                             size_t ws_bytes, cudaStream_t s) {
+                             size_t ws_bytes, cudaStream_t s, bool cleared) {
   Buckets b;
   size_t n = 0;
   if (!gather_buckets(&b, buckets, count, &n)) return SGB_ERR_UNSUPPORTED;
@@ -1758,7 +1766,7 @@ int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float th
   if (st != SGB_OK) return st;
   const Work work = work_for(n);
   ThrArgs a{nullptr, nullptr, n, thr, work, carve(ws, work), payload, nullptr, nnz_dev, 0, nullptr, true};
-  if (work.dynamic) {
+  if (work.dynamic && !cleared) {
     cudaError_t e = cudaMemsetAsync(a.ws.counters->ticket, 0, sizeof(a.ws.counters->ticket), s);
     if (e != cudaSuccess) return note_cuda_error(e);
   }
@@ -1863,7 +1871,7 @@ size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, 
 }
 
 int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
-                        void* ws, size_t ws_bytes, cudaStream_t s) {
+                        void* ws, size_t ws_bytes, cudaStream_t s, bool cleared) {
   TopkBuckets b;
   size_t bytes = 0, total = 0;
   if (!topk_plan(buckets, ks, count, mode, &b, &bytes, &total)) return SGB_ERR_UNSUPPORTED;
@@ -1873,7 +1881,7 @@ int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t co
   b.ws = static_cast<char*>(ws);
   b.idx_out = payload;
   b.val_out = reinterpret_cast<float*>(payload) + total;
-  cudaError_t e = cudaMemsetAsync(ws, 0, b.count * align256(sizeof(Counters)), s);
+  cudaError_t e = cleared ? cudaSuccess : cudaMemsetAsync(ws, 0, sparse_counter_bytes(b.count), s);
   if (e != cudaSuccess) return note_cuda_error(e);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(b.first_cta[b.count]);
@@ -1889,7 +1897,7 @@ int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t co
 }
 
 int sparse_dense_buckets(const int* payload, int known, const int* nnz_dev, const SparseBucket* buckets, size_t count,
-                         cudaStream_t s, const SparseUpdate* update) {
+                         cudaStream_t s, const SparseUpdate* update, const SparseClear& clear) {
   std::vector<float*> tensors, params, moments;
   std::vector<size_t> sizes;
   const int none[1] = {known};
@@ -1910,7 +1918,7 @@ int sparse_dense_buckets(const int* payload, int known, const int* nnz_dev, cons
   }
   const SparseUpdate joint{update ? update->sgd : nullptr, params.data(), moments.data()};
   return sparse_dense_sum(payload, 0, 0, none, nnz_dev, 1, tensors.data(), sizes.data(), tensors.size(), s,
-                          update ? &joint : nullptr);
+                          update ? &joint : nullptr, clear);
 }
 
 int sparse_faults(unsigned* flags) {
@@ -1940,20 +1948,22 @@ int sparse_threshold_bounded(float* const* tensors, const size_t* sizes, size_t 
 }
 
 int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float* acc, size_t k, int mode, int* idx_out,
-                float* val_out, void* ws, size_t ws_bytes, cudaStream_t s) {
+                float* val_out, void* ws, size_t ws_bytes, cudaStream_t s, bool cleared) {
   Gradient g;
   if (!gather(&g, tensors, sizes, count, acc)) return SGB_ERR_UNSUPPORTED;
-  return topk_launch(g, acc, k, mode, idx_out, val_out, ws, ws_bytes, s);
+  return topk_launch(g, acc, k, mode, idx_out, val_out, ws, ws_bytes, s, cleared);
 }
 
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
                      int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s,
-                     const SparseUpdate* update) {
+                     const SparseUpdate* update, const SparseClear& clear) {
   DenseArgs a;
   DenseUpdate u;
   if (update && world != 1) return SGB_ERR_UNSUPPORTED;
   if (update) u.sgd = *update->sgd;
   if (world < 1 || world > kMaxDenseRanks) return SGB_ERR_UNSUPPORTED;
+  a.clear = static_cast<uint4*>(clear.at);
+  a.clear_vecs = static_cast<unsigned>(clear.bytes / sizeof(uint4));
   a.payload = payload;
   a.stride = stride;
   a.val_off = val_off;
@@ -2011,6 +2021,7 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
                      grid, dim3(kBlock), 0, s, 0, true, a, per, NoUpdate{});
     }
     if (st != SGB_OK) return st;
+    a.clear_vecs = 0;
   }
   return launch_status();
 }

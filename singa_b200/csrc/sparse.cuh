@@ -38,7 +38,15 @@ struct SparseBucket {
 constexpr size_t kMaxBucketSpan = size_t{1} << 25;
 size_t sparse_buckets_span(const SparseBucket* buckets, size_t count);
 int sparse_threshold_buckets(const SparseBucket* buckets, size_t count, float thr, int* payload, int* nnz_dev, void* ws,
-                             size_t ws_bytes, cudaStream_t s);
+                             size_t ws_bytes, cudaStream_t s, bool cleared = false);
+// The counters of a selection are the first bytes of its workspace and are 0 when it
+// starts: set so ahead of it, unless the caller says that they are (`cleared`).  A dense
+// sum behind the selection does that for the next one on its way (`clear`).
+size_t sparse_counter_bytes(size_t buckets);
+struct SparseClear {
+  void* at = nullptr;
+  size_t bytes = 0;      // a multiple of 256
+};
 // The SGD update that a dense sum ends in: parameters (and momentum buffers) of the
 // tensors, in their order.
 struct SparseUpdate {
@@ -55,15 +63,15 @@ bool sparse_topk_buckets_cut(float* const* tensors, const size_t* sizes, const s
                              std::vector<size_t>* ends);
 size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode);
 int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
-                        void* ws, size_t ws_bytes, cudaStream_t s);
+                        void* ws, size_t ws_bytes, cudaStream_t s, bool cleared = false);
 // The dense gradients of such a payload, back into the buckets' tensors; its length
 // is on the device, or (nnz_dev null) `known`.
 int sparse_dense_buckets(const int* payload, int known, const int* nnz_dev, const SparseBucket* buckets, size_t count,
-                         cudaStream_t s, const SparseUpdate* update = nullptr);
+                         cudaStream_t s, const SparseUpdate* update = nullptr, const SparseClear& clear = {});
 
 // Top-K selection (see sgb_sparse_topk_f32) from a tensor list.
 int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float* acc, size_t k, int mode, int* idx_out,
-                float* val_out, void* ws, size_t ws_bytes, cudaStream_t s);
+                float* val_out, void* ws, size_t ws_bytes, cudaStream_t s, bool cleared = false);
 
 // Dense sum of `world` payloads (ascending indices, rank r at payload + r *
 // stride words) into the tensors, which cover the index space in list order.
@@ -72,7 +80,7 @@ int sparse_topk(float* const* tensors, const size_t* sizes, size_t count, float*
 // (then clamped to val_off, or to the size of the index space).  update: one rank only.
 int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const int* counts, const int* counts_dev,
                      int world, float* const* tensors, const size_t* sizes, size_t ntensors, cudaStream_t s,
-                     const SparseUpdate* update = nullptr);
+                     const SparseUpdate* update = nullptr, const SparseClear& clear = {});
 
 // Rounds the tensors to fp16 and back, in place (multi_tensor.cu).
 int round_f16_multi(void* const* tensors, const size_t* sizes, size_t count, cudaStream_t s);
