@@ -131,9 +131,9 @@ def _recorded(name):
     return property(read, write)
 
 
-# When a recorded call is issued: in every run, in timed ones, in runs into a capture
-# (which fork), in those that are not.
-_ALWAYS, _PROFILED, _FORKED, _UNFORKED = range(4)
+# When a recorded call is issued: in every run, in timed ones, in runs into a capture, in
+# those that are not.
+_ALWAYS, _PROFILED, _CAPTURED, _SINGLE = range(4)
 
 
 class HotPathGPU(object):
@@ -419,16 +419,16 @@ class HotPathGPU(object):
         for name, args in self.launched:
             if name == "grad_ready":
                 idx = order_index[args]
-                self.calls_per_step += self._record_exchange(prog, idx, _UNFORKED if forks else _ALWAYS)
+                self.calls_per_step += self._record_exchange(prog, idx, _SINGLE if forks else _ALWAYS)
                 if idx in beside:
-                    prog += [("fork", (), _FORKED), beside[idx]]
+                    prog += [("fork", (), _CAPTURED), beside[idx]]
             elif name == "sync_and_update":
-                when = _UNFORKED if forks else _ALWAYS
+                when = _SINGLE if forks else _ALWAYS
                 if self.comm is not None:
                     prog.append(("sgb_comm_wait", (self.comm._h.value, "STREAM"), when))
                 prog += behind or []
                 if beside:
-                    prog.append(("join", (), _FORKED))
+                    prog.append(("join", (), _CAPTURED))
                 if self.update_on_arrival:
                     continue                  # every bucket was updated as it arrived
                 prog.append(self._sgd_call(self.sgd_tables, "STREAM", when))
@@ -485,14 +485,15 @@ class HotPathGPU(object):
             pp, gp, mp, sizes, n = tables
             return C.addressof(pp), C.addressof(gp), C.addressof(mp), C.addressof(sizes), n
 
-        # when each gradient is ready, in us: a call takes 2.5, or what its tensors take at 6 TB/s
+        # when each gradient is ready, in us: a call takes 2.5, or what its tensors (three of
+        # the result's size, about) take at 6 TB/s
         now, ready, order = 0.0, {}, {n: i for i, n in enumerate(self.plan["grad_order"])}
         for op in self.plan["ops"]:
             if op.kind == "grad_ready":
                 ready[order[op.args["param"]]] = now
             elif op.kind != "sync_and_update":
-                names = [v for v in op.args.values() if isinstance(v, str)]
-                now += max(2.5, sum(4e-6 * self.t[v].numel() for v in names if v in self.t) / 6)
+                result = self.t.get(op.args.get("dx"))
+                now += 2.5 if result is None else max(2.5, 2e-6 * result.numel())
         beside, late, free = {}, [], 0.0
         for idx in sorted(self.flush_after):
             bucket = self.flush_after[idx][1]
@@ -501,7 +502,7 @@ class HotPathGPU(object):
             if done <= now:
                 free = done
                 beside[idx] = ("sgb_sgd_update_beside_f32",
-                               addresses(self.bucket_sgd[idx]) + rates + (int(half), "SIDE_STREAM"), _FORKED)
+                               addresses(self.bucket_sgd[idx]) + rates + (int(half), "SIDE_STREAM"), _CAPTURED)
             else:
                 late += bucket
         if not late:
@@ -512,8 +513,8 @@ class HotPathGPU(object):
         tables = addresses(self._late_tables)
         if half:
             return beside, [("sgb_comm_update_half", (self.comm._h.value,) + tables + (max(p.numel() for p in ps),) + rates +
-                             ("STREAM",), _FORKED)]
-        return beside, [("sgb_sgd_update_multi_f32", tables + rates + ("STREAM",), _FORKED)]
+                             ("STREAM",), _CAPTURED)]
+        return beside, [("sgb_sgd_update_multi_f32", tables + rates + ("STREAM",), _CAPTURED)]
 
     def _sgd_call(self, tables, stream, when=_ALWAYS):
         pp, gp, mp, sizes, n = tables

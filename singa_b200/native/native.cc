@@ -1099,11 +1099,11 @@ const Callable kCallables[] = {
 enum Patch { kStream, kSideStream, kResultStream, kResultIndex, kLr, kMomentum, kDecay, kPatches };
 const char* const kPatchNames[kPatches] = {"STREAM", "SIDE_STREAM", "RESULT_STREAM", "RESULT_INDEX", "LR", "MOMENTUM", "DECAY"};
 
-// When a call of a program is issued.  A forked run is one into a capture: "fork" and
-// "join" order the side stream behind the main one and back, and what a run does there
-// is a branch of the graph.  (One by one, the two events of a fork cost the host more
-// than the branch saves, and threads that run a program would share them.)
-enum When { kAlways, kProfiled, kForked, kUnforked };
+// When a call of a program is issued: in every run, in timed ones, in runs into a capture,
+// in those that are not.  In a capture "fork" and "join" order a side stream behind the main
+// one and back, and what a run does there is a branch of the graph.  (One by one, the two
+// events of a fork cost the host more than the branch saves.)
+enum When { kAlways, kProfiled, kCaptured, kSingle };
 
 constexpr size_t kMaxArguments = 24;
 struct Call {
@@ -1113,28 +1113,69 @@ struct Call {
   int when;
   bool join = false;
 };
-// The side stream of a program that forks, below the priority of what it runs beside.
+// A side stream, below the priority of what it runs beside, and the event that orders it.
+// A few are kept per device for all programs (one costs more than a millisecond); one that
+// takes part in a capture is not lent again before that ends.
 struct Side {
   cudaStream_t stream = nullptr;
   cudaEvent_t event = nullptr;
-  Side() = default;
-  Side(const Side&) = delete;
-  Side& operator=(const Side&) = delete;
-  ~Side() {
-    if (event) cudaEventDestroy(event);
-    if (stream) cudaStreamDestroy(stream);
-  }
-  bool open() {
-    int least = 0, greatest = 0;
-    const bool ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
-                    cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, least) == cudaSuccess &&
-                    cudaEventCreateWithFlags(&event, cudaEventDisableTiming) == cudaSuccess;
-    if (!ok) cudaGetLastError();
-    return ok;
-  }
+  bool lent = false;
   // Everything of `from` so far, in front of whatever comes to `to`.
   bool order(cudaStream_t from, cudaStream_t to) const {
     return cudaEventRecord(event, from) == cudaSuccess && cudaStreamWaitEvent(to, event, 0) == cudaSuccess;
+  }
+};
+class Sides {
+ public:
+  // On the current device; null where all are in use.
+  static Side* lend() {
+    const std::lock_guard<std::mutex> lock(guard());
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return failed();
+    auto& sides = all()[device];
+    for (const auto& side : sides) {
+      cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+      if (side->lent) continue;
+      if (cudaStreamIsCapturing(side->stream, &status) != cudaSuccess) return failed();
+      if (status == cudaStreamCaptureStatusNone) return lent(side.get());
+    }
+    if (sides.size() == kMost) return nullptr;
+    int least = 0, greatest = 0;
+    auto side = std::make_unique<Side>();
+    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+        cudaEventCreateWithFlags(&side->event, cudaEventDisableTiming) != cudaSuccess)
+      return failed();
+    if (cudaStreamCreateWithPriority(&side->stream, cudaStreamNonBlocking, least) != cudaSuccess) {
+      cudaEventDestroy(side->event);
+      return failed();
+    }
+    sides.push_back(std::move(side));
+    return lent(sides.back().get());
+  }
+  static void give_back(Side* side) {
+    if (!side) return;
+    const std::lock_guard<std::mutex> lock(guard());
+    side->lent = false;
+  }
+
+ private:
+  static constexpr size_t kMost = 8;
+  static std::mutex& guard() {
+    static auto* m = new std::mutex;
+    return *m;
+  }
+  // Never destroyed: the CUDA context may be gone by then.
+  static std::map<int, std::vector<std::unique_ptr<Side>>>& all() {
+    static auto* m = new std::map<int, std::vector<std::unique_ptr<Side>>>;
+    return *m;
+  }
+  static Side* lent(Side* side) {
+    side->lent = true;
+    return side;
+  }
+  static Side* failed() {
+    cudaGetLastError();
+    return nullptr;
   }
 };
 // What a recorded step depends on besides its arguments: if this is the same as
@@ -1170,8 +1211,8 @@ struct Program {
   unsigned eager = 2;         // of which so many are launched one by one
   unsigned captures = 0;
   cudaGraphExec_t exec = nullptr;
-  std::unique_ptr<Side> side; // where the program forks
-  std::mutex guard;           // of the six fields above
+  bool forks = false;         // needs a side stream in a capture
+  std::mutex guard;           // of streak, eager, captures, exec, seen
 };
 constexpr unsigned kEagerRuns = 2, kPaysAfter = 40, kMostEagerRuns = 1u << 16;
 const char kProgramTag[] = "singa_b200.program";
@@ -1199,14 +1240,12 @@ PyObject* py_program(Args a, Py_ssize_t n) {
     PyObject* args;
     int when;
     if (!PyArg_ParseTuple(item, "sO!i", &name, &PyTuple_Type, &args, &when)) throw PyError{};
-    if (when < kAlways || when > kUnforked) fail(PyExc_ValueError, "no such time for a call");
+    if (when < kAlways || when > kSingle) fail(PyExc_ValueError, "no such time for a call");
     const bool join = !strcmp(name, "join");
     if (join || !strcmp(name, "fork")) {
-      prog->calls.push_back(Call{nullptr, {}, {}, kForked, join});
-      if (!prog->side) {
-        prog->side = std::make_unique<Side>();
-        if (!prog->side->open()) fail(PyExc_RuntimeError, "no side stream for a program");
-      }
+      prog->calls.push_back(Call{nullptr, {}, {}, kCaptured, join});
+      if (!prog->forks) Sides::give_back(Sides::lend());    // made outside captures
+      prog->forks = true;
       continue;
     }
     const Callable* fn = nullptr;
@@ -1241,12 +1280,13 @@ PyObject* py_program(Args a, Py_ssize_t n) {
   return cap;
 }
 
-// Issues the calls in order on `st`, forking to `side` where there is one; on a failure
-// `where` names the call.
-int issue_calls(const Program* prog, const Settings& now, bool profile, void* st, const Side* side, const char** where) {
+// Issues the calls in order on `st`, in a capture with forks to `side`; on a failure `where`
+// names the call.
+int issue_calls(const Program* prog, const Settings& now, bool profile, void* st, bool captured, const Side* side,
+                const char** where) {
   Slot scratch_slots[kMaxArguments];
   for (const Call& c : prog->calls) {
-    if (c.when == kProfiled ? !profile : c.when == kForked ? !side : c.when == kUnforked && side) continue;
+    if (c.when == kProfiled ? !profile : c.when == kCaptured ? !captured : c.when == kSingle && captured) continue;
     if (!c.fn) {
       const cudaStream_t main = static_cast<cudaStream_t>(st);
       if (c.join ? side->order(side->stream, main) : side->order(main, side->stream)) continue;
@@ -1287,19 +1327,21 @@ int issue_calls(const Program* prog, const Settings& now, bool profile, void* st
 // Captures one run on a stream of its own (nothing executes) and instantiates
 // it.  False: not possible here; the program then stays with single launches.
 bool capture_calls(Program* prog, const Settings& now) {
-  cudaStream_t side;
-  if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
+  cudaStream_t main;
+  if (cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking) != cudaSuccess) return false;
+  Side* const side = prog->forks ? Sides::lend() : nullptr;
   cudaGraph_t graph = nullptr;
   const char* where = "";
-  bool ok = cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  bool ok = cudaStreamBeginCapture(main, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
-    ok = issue_calls(prog, now, false, side, prog->side.get(), &where) == SGB_OK;
-    ok = cudaStreamEndCapture(side, &graph) == cudaSuccess && ok && graph;
+    ok = issue_calls(prog, now, false, main, !prog->forks || side, side, &where) == SGB_OK;
+    ok = cudaStreamEndCapture(main, &graph) == cudaSuccess && ok && graph;
   }
+  Sides::give_back(side);
   cudaGraphExec_t exec = nullptr;
   if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
   if (graph) cudaGraphDestroy(graph);
-  cudaStreamDestroy(side);
+  cudaStreamDestroy(main);
   if (!ok) {
     cudaGetLastError();      // a refused capture is not an error of the step
     return false;
@@ -1350,14 +1392,12 @@ PyObject* py_run_program(Args a, Py_ssize_t) {
       }
     }
   }
-  if (captured && plain && prog->side) {
-    // a caller's capture; one at a time, as there is one side stream
-    const std::lock_guard<std::mutex> lock(prog->guard);
-    cudaStreamCaptureStatus other = cudaStreamCaptureStatusActive;
-    const bool ours = cudaStreamIsCapturing(prog->side->stream, &other) == cudaSuccess && other == cudaStreamCaptureStatusNone;
-    status = issue_calls(prog, now, profile, st, ours ? prog->side.get() : nullptr, &where);
+  if (captured && plain) {                             // a caller's capture
+    Side* const side = prog->forks ? Sides::lend() : nullptr;
+    status = issue_calls(prog, now, profile, st, !prog->forks || side, side, &where);
+    Sides::give_back(side);
   } else if (!launched) {
-    status = issue_calls(prog, now, profile, st, nullptr, &where);
+    status = issue_calls(prog, now, profile, st, false, nullptr, &where);
   }
   Py_END_ALLOW_THREADS;
   if (status != SGB_OK) fail_status(where, status);

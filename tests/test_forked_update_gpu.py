@@ -46,6 +46,26 @@ def test_captured_steps_equal_single_calls(sync, threshold, on_arrival):
     comm.close()
 
 
+@pytest.mark.parametrize("count", [2, 11])      # more than there are side streams
+def test_several_steps_in_one_capture(count):
+    single, together = [[step("none", 200, None) for _ in range(count)] for _ in range(2)]
+    for hp in single:
+        hp.profile = True                        # one by one
+    for hp in together:
+        hp.run_step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        for hp in together:
+            hp.run_step()
+    for _ in range(3):
+        graph.replay()
+    for a, b in zip(single, together):
+        for _ in range(4):
+            a.run_step()
+        assert all(torch.equal(x, y) for x, y in zip(state(a), state(b)))
+
+
 def test_what_does_not_fit_the_communicator_is_still_refused():
     from singa_b200 import _lib
     from singa_b200.communicator import Communicator, NcclIdHolder
