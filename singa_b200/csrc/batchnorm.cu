@@ -516,10 +516,15 @@ bn_bwd_cluster_kernel(const float* __restrict__ x, const float* __restrict__ dy,
 // ADJACENT channels of one sample form a contiguous, 16-byte aligned run of
 // G*HW floats.  One CTA stages the G channels of all N samples (G*N*HW*8
 // bytes of shared memory) with 16-byte copies, reduces every channel with a
-// sub-group of its threads from shared memory, overwrites the staged dy with
-// dx in place and streams it back with 16-byte stores.
+// sub-group of its threads from shared memory and forms dx from the staged
+// copies on the way out: four elements belong to two channels at most.  Such a
+// call is one wave that loads, reduces and stores, so each step between counts: with
+// the channel's scalars fetched behind the copies and dx formed in place by a pass
+// of its own 32x2048x7x7 took 12.8 us (now 10.6), 64x512x7x7 9.8 (7.2); with the
+// masked gradient brought in through registers, four units a round, 13.1 (9.7).
+constexpr int kGroupBytes = 100 * 1024;               // the two staged operands of a group at most
 template <int MASK, int G>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 4)
 bn_bwd_group_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                     const float* __restrict__ relu_in, const float* __restrict__ scale,
                     const float* __restrict__ mean, const float* __restrict__ invstd,
@@ -528,7 +533,7 @@ bn_bwd_group_kernel(const float* __restrict__ x, const float* __restrict__ dy,
   extern __shared__ __align__(16) float stage[];
   constexpr int kSub = kBlock / G;                    // threads per channel
   __shared__ float red[2][kBlock / 32];
-  __shared__ float coef[G][4];
+  __shared__ float4 coef[G];
   const int c0 = blockIdx.x * G;
   const int run = G * sh.HW;                          // floats per sample, multiple of 4
   const int run4 = run >> 2;
@@ -537,65 +542,89 @@ bn_bwd_group_kernel(const float* __restrict__ x, const float* __restrict__ dy,
   float* sg = stage + static_cast<size_t>(sh.N) * run;
   const size_t sample_stride = static_cast<size_t>(sh.C) * sh.HW;
   const size_t base = static_cast<size_t>(c0) * sh.HW;
-  UnitWalk wl(threadIdx.x, kBlock, run4);
+  const UnitWalk start(threadIdx.x, kBlock, run4);
+  UnitWalk wl = start;
   if (first_wave(2)) prefetch_share(x, MASK == 1 ? relu_in : nullptr, threadIdx.x, units, kBlock, run4, sample_stride, base);
-  dependency_wait();
-  if (MASK) {
-    // x by asynchronous copy; dy and the ReLU input through registers, four
-    // units (eight independent 16-byte loads) per round
-    for (int u = threadIdx.x; u < units;) {
-      Vec4f vg[4], vm[4];
-      unsigned bits[4];
-      int us[4], cnt = 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (u < units) {
-          const size_t off = wl.n * sample_stride + base + 4 * static_cast<size_t>(wl.q);
-          cp_async16(sx + 4 * u, x + off);
-          vg[j].u = ld128(dy + off);
-          if (MASK == 1) vm[j].u = ld128(relu_in + off);
-          if (MASK == 2) bits[j] = keep4<2>(relu_in, off);
-          us[j] = u;
-          u += kBlock;
-          wl.next();
-          cnt = j + 1;
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j < cnt) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (MASK == 1) vg[j].f[k] = vm[j].f[k] > 0 ? vg[j].f[k] : 0.0f;
-            if (MASK == 2) vg[j].f[k] = (bits[j] >> k) & 1u ? vg[j].f[k] : 0.0f;
-          }
-          *reinterpret_cast<uint4*>(sg + 4 * us[j]) = vg[j].u;
-        }
-      }
-    }
-  } else {
-    for (int u = threadIdx.x; u < units; u += kBlock, wl.next()) {
-      const size_t off = wl.n * sample_stride + base + 4 * static_cast<size_t>(wl.q);
-      cp_async16(sx + 4 * u, x + off);
-      cp_async16(sg + 4 * u, dy + off);
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  // channel g is handled by threads [g*kSub, (g+1)*kSub): element (n, i) of the
-  // channel sits at staged offset n*run + g*HW + i
+  // channel g is handled by threads [g*kSub, (g+1)*kSub)
   const int g = threadIdx.x / kSub, t = threadIdx.x - g * kSub;
   const int c = c0 + g;
-  const float mu = mean[c];
+  UnitWalk w(t, kSub, sh.HW);                         // (sample, position) without a division per step
+  dependency_wait();
+  const float mu = mean[c], r = invstd[c], gain = scale[c];     // on their way with the operands
+  for (int u = threadIdx.x; u < units; u += kBlock, wl.next()) {
+    const size_t off = wl.n * sample_stride + base + 4 * static_cast<size_t>(wl.q);
+    cp_async16(sx + 4 * u, x + off);
+    cp_async16(sg + 4 * u, dy + off);
+  }
+  if (MASK) {
+    // what the ReLU keeps of the thread's own units, four bits each, eight loads at a
+    // time while the copies are on their way
+    constexpr int kWords = (kGroupBytes / 32 + 8 * kBlock - 1) / (8 * kBlock);
+    unsigned keep[kWords];
+    wl = start;
+    int u = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < kWords; ++k) {
+      keep[k] = 0;
+      if (8 * k * kBlock >= units) break;
+      Vec4f vm[8];
+      unsigned bits[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j, u += kBlock, wl.next()) {
+        if (u >= units) continue;
+        const size_t off = wl.n * sample_stride + base + 4 * static_cast<size_t>(wl.q);
+        if (MASK == 1) vm[j].u = ld128(relu_in + off);
+        if (MASK == 2) bits[j] = keep4<2>(relu_in, off);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (static_cast<int>(threadIdx.x) + (8 * k + j) * kBlock >= units) continue;
+        if (MASK == 1) {
+          bits[j] = 0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) bits[j] |= (vm[j].f[i] > 0 ? 1u : 0u) << i;
+        }
+        keep[k] |= (bits[j] & 15u) << (4 * j);
+      }
+    }
+    cp_async_wait_all();
+#pragma unroll
+    for (int j = 0; j < 8 * kWords; ++j) {
+      const int own = threadIdx.x + j * kBlock;
+      if (own >= units) break;
+      uint4* const at = reinterpret_cast<uint4*>(sg + 4 * own);
+      Vec4f v;
+      v.u = *at;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v.f[i] = (keep[j / 8] >> (4 * (j % 8) + i)) & 1u ? v.f[i] : 0.0f;
+      *at = v.u;
+    }
+  } else {
+    cp_async_wait_all();
+  }
+  __syncthreads();
+  // element (n, i) of the channel sits at staged offset n*run + g*HW + i
   const int per = sh.N * sh.HW;
   float s_dy = 0.f, s_dyx = 0.f;
-  {
-    UnitWalk w(t, kSub, sh.HW);                       // (sample, position) without a division per step
-    for (int e = t; e < per; e += kSub, w.next()) {
+  int e = t;
+  for (constexpr int kAhead = 4; e + (kAhead - 1) * kSub < per; e += kAhead * kSub) {
+    float vg[kAhead], vx[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j, w.next()) {
       const int l = w.n * run + g * sh.HW + w.q;
-      s_dy += sg[l];
-      s_dyx += sg[l] * (sx[l] - mu);
+      vg[j] = sg[l];
+      vx[j] = sx[l];
     }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      s_dy += vg[j];
+      s_dyx += vg[j] * (vx[j] - mu);
+    }
+  }
+  for (; e < per; e += kSub, w.next()) {
+    const int l = w.n * run + g * sh.HW + w.q;
+    s_dy += sg[l];
+    s_dyx += sg[l] * (sx[l] - mu);
   }
   // reduce inside the sub-group (kSub is a multiple of 32: whole warps per channel)
   s_dy = warp_sum(s_dy);
@@ -613,33 +642,32 @@ bn_bwd_group_kernel(const float* __restrict__ x, const float* __restrict__ dy,
       a += red[0][g * kWarpsPer + w];
       b += red[1][g * kWarpsPer + w];
     }
-    const float r = invstd[c];
     const float inv_m = 1.0f / (static_cast<float>(sh.N) * static_cast<float>(sh.HW));
     const float ds = b * r;
-    coef[g][0] = scale[c] * r;
-    coef[g][1] = a * inv_m;
-    coef[g][2] = ds * r * inv_m;
-    coef[g][3] = mu;
+    coef[g] = make_float4(gain * r, a * inv_m, ds * r * inv_m, mu);
     dscale[c] = ds;
     dbias[c] = a;
   }
   __syncthreads();
-  const float k_ = coef[g][0], am = coef[g][1], bm = coef[g][2];
-  {
-    UnitWalk w(t, kSub, sh.HW);
-    for (int e = t; e < per; e += kSub, w.next()) {
-      const int l = w.n * run + g * sh.HW + w.q;
-      sg[l] = k_ * (sg[l] - am - (sx[l] - mu) * bm);        // dx in place
-    }
-  }
-  __syncthreads();
   release_dependents();
-  {
-    UnitWalk w(threadIdx.x, kBlock, run4);
-    for (int u = threadIdx.x; u < units; u += kBlock, w.next()) {
-      const size_t off = w.n * sample_stride + base + 4 * static_cast<size_t>(w.q);
-      st128(dx + off, *reinterpret_cast<const uint4*>(sg + 4 * u));
+  wl = start;
+  for (int u = threadIdx.x; u < units; u += kBlock, wl.next()) {
+    const size_t off = wl.n * sample_stride + base + 4 * static_cast<size_t>(wl.q);
+    const int i = 4 * wl.q;
+    int first = 0;                                    // the channel of element i
+#pragma unroll
+    for (int j = 1; j < G; ++j) first += i >= j * sh.HW;
+    const int next = (first + 1) * sh.HW - i;         // so many elements are its own
+    const float4 k0 = coef[first], k1 = coef[first + 1 < G ? first + 1 : first];
+    Vec4f vx, vg, o;
+    vx.u = *reinterpret_cast<const uint4*>(sx + 4 * u);
+    vg.u = *reinterpret_cast<const uint4*>(sg + 4 * u);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool own = j < next;
+      o.f[j] = (own ? k0.x : k1.x) * (vg.f[j] - (own ? k0.y : k1.y) - (vx.f[j] - (own ? k0.w : k1.w)) * (own ? k0.z : k1.z));
     }
+    st128(dx + off, o.u);
   }
 }
 
@@ -1494,27 +1522,36 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
   // groups of G adjacent channels make 16-byte runs of odd planes (7x7 layers)
   const int G = (HW % 2) ? 4 : 2;
   const bool groups = !vec && HW > 1 && bases_aligned && (HW * G) % 4 == 0 && C % G == 0 &&
-                      static_cast<long long>(G) * per_channel * 8 <= 100 * 1024;
+                      static_cast<long long>(G) * per_channel * 8 <= kGroupBytes;
   if (revisit_pays(N, C, HW, bases_aligned, groups)) {
     const int st = bn_revisit_backward(MASK, x, dy, relu_in, scale, mean, invstd, dx, dscale, dbias, N, C, HW, ws,
                                        ws_bytes, s);
     if (st != SGB_ERR_WORKSPACE) return st;            // a smaller workspace: the forms below
   }
   // Channels that fit a CTA's registers need no staging.  Where that means scalar
-  // accesses and no mask has to be formed, the group form takes over above 2e6
-  // elements, where the call is bound by bytes and no longer by latency.  Time in
-  // groups over time in registers (odd planes of 9 to 225, cold inputs), by how
-  // many of the threads' 1024, 2048 or 3072 slots a channel fills:
-  //   elements of a channel   1.5e6      2.2e6      4.5e6      12e6
-  //   1125-1215 (of 2048)    .95-1.01   .89-.95    .80-.83    .67-.70
-  //   567-605 (of 1024)     1.07-1.17   .99-1.09   .89-.96    -
-  //   1450-1575 (of 2048)   1.11-1.18  1.03-1.11   .93-1.01   .82-.87
-  //   2050-2110 (of 3072)   1.23-1.27   .98-1.00   .93-.96    .82-.85
-  //   845-900, 1780-2030, 2475-3040 (nearly all)
-  //                         1.12-1.46  1.18-1.55  1.08-1.37   .93-1.21
-  // So the line is right for channels that leave a quarter of the slots empty, and
-  // on the group form's side by up to half of the time for those that fill them.
-  if (!(groups && MASK == 0 && per_channel * C > 2000000LL)) {
+  // accesses the group form takes over above 2e6 elements, where the call is bound by
+  // bytes and no longer by latency, unless a channel nearly fills the threads' 1024 or
+  // 2048 slots.  Cold inputs, us in registers / in groups, (plain; with the ReLU's
+  // input; with its bits), 2.1e6 to 3.2e6 elements if not said:
+  //   elements of a channel   plain                   input                 bits
+  //   567 (of 1024)           9.7 /  9.2             12.0 / 10.8           13.8 / 10.3
+  //   882                     7.8 / 10.0             10.4 / 11.5           12.1 / 11.0
+  //   1014                    6.8 /  9.1              8.6 / 10.9           12.7 / 10.1
+  //   980, 5.9e6             15.9 / 19.3             21.1 / 22.4           29.4 / 21.7
+  //   1125 (of 2048)         12.1 /  8.5             15.0 / 10.6           17.6 / 10.2
+  //   1568                   13.0 / 10.8             16.5 / 14.5           20.6 / 12.9
+  //   1715                    9.9 /  9.5             12.7 / 12.6           16.5 / 10.7
+  //   2025                    7.7 /  9.1             10.3 / 11.7           13.1 / 10.1
+  //   2160 (of 3072)         10.0 /  8.5             15.6 / 10.8           19.3 /  9.9
+  //   2997                   11.1 / 10.8             17.3 / 15.0           24.5 / 12.8
+  // Up to 1.6e6 elements registers are the better or within a tenth.  A ReLU's input
+  // and its bits take the same side, so that they have the same bits; a plain call's
+  // full channels come back to groups above 6e6.
+  const long long elements = per_channel * C;
+  const bool full = per_channel <= 1024 ? per_channel > 768 : per_channel > 1600 && per_channel <= 2048;
+  const bool grouped = groups && elements > 2000000LL &&
+                       (MASK == 0 ? !full || elements > 6000000LL : !full && per_channel > 1024);
+  if (!grouped) {
     int st = SGB_OK;
     auto go = [&](auto g, auto nv, auto v) {
       st = launch_small<MASK, decltype(g)::value, decltype(nv)::value, decltype(v)::value>(
