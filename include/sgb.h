@@ -531,6 +531,11 @@ int sgb_unpack_f16_to_f32(const void *flat_f16, size_t flat_offset,
 /* ------------------------------------------------- sparsification kernels */
 /* Workspace (256-byte aligned) for the two selectors below. */
 size_t sgb_sparse_workspace_bytes(size_t n);
+/* How a joint top-K selection (sgb_comm_sparse_update) of ks[k] out of sizes[k] elements
+ * each lays out its workspace: the bytes it needs, 0 where one launch does not take the
+ * buckets, and in *counters how many of them, at the start, are counters, which the call
+ * leaves clear.  Host arithmetic only. */
+size_t sgb_sparse_topk_plan(const size_t *sizes, const size_t *ks, size_t nbuckets, int mode, size_t *counters);
 /* Diagnostic: the sticky fault word of the current device's joint top-K selections
  * (sgb_comm_sparse_update), whose CTAs meet with bounded waits: 0 = none, 1 a wait
  * ran out.  Such a launch stops early; its gradients, parameters, momenta and

@@ -944,7 +944,7 @@ static int threshold_buckets(sgb_comm* c, const std::vector<sgb::SparseBucket>& 
     if (update)
       part = {update->sgd, update->params + tensor, update->moments ? update->moments + tensor : nullptr};
     OK(sgb::sparse_dense_buckets(c->joint_pay, 0, c->joint_nnz, list.data() + k, end - k, c->c1, update ? &part : nullptr,
-                                 {c->joint_ws, counters}));
+                                 {c->joint_ws, counters, c->joint_ws_bytes}));
     now_cleared(&c->joint_clear, counters);
     for (; k < end; ++k) tensor += list[k].count;
   }
@@ -1023,7 +1023,7 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
     if (!sgb::sparse_selects_from(b.tensors, b.sizes, b.count, b.acc)) return SGB_ERR_UNSUPPORTED;
   // several buckets: one launch selects from as many as it can take, the next updates them
   if (nbuckets > 1) {
-    std::vector<size_t> ends, ks;
+    std::vector<size_t> ends, ks, counters;            // counters: bytes of them, per launch
     if (!sgb::sparse_topk_buckets_cut(reinterpret_cast<float* const*>(tensors), sizes, counts, nbuckets, &ends))
       return SGB_ERR_UNSUPPORTED;
     size_t widest = 0, ws_bytes = 0, k = 0, tensor = 0;
@@ -1035,8 +1035,11 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
         ks.push_back(static_cast<size_t>(sgb_topk_count(spars, n)));
         span += n + 512;
       }
-      const size_t need = sgb::sparse_topk_buckets_bytes(list.data() + first, ks.data() + first, k - first, c->topk_mode);
+      size_t of_these = 0;
+      const size_t need =
+          sgb::sparse_topk_buckets_bytes(list.data() + first, ks.data() + first, k - first, c->topk_mode, &of_these);
       if (!need) return SGB_ERR_UNSUPPORTED;
+      counters.push_back(of_these);
       widest = span > widest ? span : widest;
       ws_bytes = need > ws_bytes ? need : ws_bytes;
     }
@@ -1044,16 +1047,16 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
     OK(emit(c, plan_call(c, sgb::order::kStageCopy).pre, compute));
     Phase ph(c, "Dist_c1c2_fusedSparsification", sgb::order::kStreamC1);
     k = 0;
-    for (const size_t end : ends) {
+    for (size_t part = 0; part < ends.size(); ++part) {
+      const size_t end = ends[part], used = counters[part];
       int sent = 0;
-      const size_t counters = sgb::sparse_counter_bytes(end - k);
       OK(sgb::sparse_topk_buckets(list.data() + k, ks.data() + k, end - k, c->topk_mode, c->joint_pay, &sent,
                                   c->joint_ws, c->joint_ws_bytes, c->c1,
-                                  take_cleared(c, &c->joint_clear, counters, compute)));
-      const sgb::SparseUpdate part{&sgd, update.params + tensor, update.moments ? update.moments + tensor : nullptr};
-      OK(sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data() + k, end - k, c->c1, &part,
-                                   {c->joint_ws, counters}));
-      now_cleared(&c->joint_clear, counters);
+                                  take_cleared(c, &c->joint_clear, used, compute)));
+      const sgb::SparseUpdate behind{&sgd, update.params + tensor, update.moments ? update.moments + tensor : nullptr};
+      OK(sgb::sparse_dense_buckets(c->joint_pay, sent, nullptr, list.data() + k, end - k, c->c1, &behind,
+                                   {c->joint_ws, used, c->joint_ws_bytes}));
+      now_cleared(&c->joint_clear, used);
       for (; k < end; ++k) tensor += list[k].count;
     }
     return SGB_OK;
@@ -1073,7 +1076,7 @@ int sgb_comm_sparse_update(sgb_comm* c, void* const* tensors, const size_t* size
                         reinterpret_cast<float*>(x.pay_send) + k, c->ws, c->ws_bytes, c->c1,
                         take_cleared(c, &c->ws_clear, counters, compute)));
   OK(sgb::sparse_dense_sum(x.pay_send, 0, 0, sent, nullptr, 1, b.tensors, b.sizes, b.count, c->c1, &update,
-                           {c->ws, k ? counters : 0}));
+                           {c->ws, k ? counters : 0, c->ws_bytes}));
   if (k) now_cleared(&c->ws_clear, counters);
   return SGB_OK;
 }

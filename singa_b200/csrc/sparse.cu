@@ -1822,7 +1822,7 @@ static bool topk_plan(const SparseBucket* buckets, const size_t* ks, size_t coun
   }
   if (index > kMaxBucketSpan || ctas > most) return false;
   b->first_cta[b->count] = static_cast<unsigned>(ctas);
-  const size_t counters = b->count * align256(sizeof(Counters));
+  const size_t counters = sparse_counter_bytes(b->count);
   for (int i = 0; i < b->count; ++i) b->ws_off[i] += counters;
   *bytes = counters + lists;
   *sent = payload;
@@ -1864,10 +1864,12 @@ bool sparse_topk_buckets_cut(float* const* tensors, const size_t* sizes, const s
   return cuts == 0 || total >= kLeastCut;
 }
 
-size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode) {
+size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, size_t* counters) {
   TopkBuckets b;
   size_t bytes = 0, sent = 0;
-  return topk_plan(buckets, ks, count, mode, &b, &bytes, &sent) ? bytes + 256 : 0;
+  if (!topk_plan(buckets, ks, count, mode, &b, &bytes, &sent)) return 0;
+  *counters = sparse_counter_bytes(b.count);
+  return bytes + 256;
 }
 
 int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
@@ -1962,6 +1964,7 @@ int sparse_dense_sum(const int* payload, size_t stride, size_t val_off, const in
   if (update && world != 1) return SGB_ERR_UNSUPPORTED;
   if (update) u.sgd = *update->sgd;
   if (world < 1 || world > kMaxDenseRanks) return SGB_ERR_UNSUPPORTED;
+  if (clear.bytes > clear.room) return SGB_ERR_WORKSPACE;
   a.clear = static_cast<uint4*>(clear.at);
   a.clear_vecs = static_cast<unsigned>(clear.bytes / sizeof(uint4));
   a.payload = payload;
@@ -2033,6 +2036,14 @@ using namespace sgb;
 extern "C" {
 
 size_t sgb_sparse_workspace_bytes(size_t n) { return n ? workspace_bytes(n) : 256; }
+
+size_t sgb_sparse_topk_plan(const size_t* sizes, const size_t* ks, size_t nbuckets, int mode, size_t* counters) {
+  if (!sizes || !ks || !counters) return 0;
+  float* const somewhere = reinterpret_cast<float*>(static_cast<uintptr_t>(256));   // never followed
+  std::vector<SparseBucket> buckets;
+  for (size_t k = 0; k < nbuckets; ++k) buckets.push_back({&somewhere, sizes + k, 1, somewhere});
+  return sparse_topk_buckets_bytes(buckets.data(), ks, nbuckets, mode, counters);
+}
 
 int sgb_topk_count(float ratio, size_t n) {
   // (int)ceil(threshold * num) evaluated in fp32, as the reference does

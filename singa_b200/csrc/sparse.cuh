@@ -46,6 +46,7 @@ size_t sparse_counter_bytes(size_t buckets);
 struct SparseClear {
   void* at = nullptr;
   size_t bytes = 0;      // a multiple of 256
+  size_t room = 0;       // what there is at `at`; more than that is refused
 };
 // The SGD update that a dense sum ends in: parameters (and momentum buffers) of the
 // tensors, in their order.
@@ -56,12 +57,14 @@ struct SparseUpdate {
 };
 // Top-K of several buckets (the first ks[k] of bucket k by size) by one launch, into
 // a payload of the same joint space; *sent: its length.  sparse_topk_buckets_bytes:
-// of workspace, 0 where one launch does not take them.  sparse_topk_buckets_cut: whether
+// of workspace, 0 where one launch does not take them, and how much of its start is
+// counters: those of the buckets that it selects from (one without elements, or of
+// which nothing is sent, has none).  sparse_topk_buckets_cut: whether
 // launches of several buckets each take a list, by sizes and places alone, before
 // anything is prepared, and where each ends (`ends` may be null).
 bool sparse_topk_buckets_cut(float* const* tensors, const size_t* sizes, const size_t* counts, size_t nbuckets,
                              std::vector<size_t>* ends);
-size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode);
+size_t sparse_topk_buckets_bytes(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, size_t* counters);
 int sparse_topk_buckets(const SparseBucket* buckets, const size_t* ks, size_t count, int mode, int* payload, int* sent,
                         void* ws, size_t ws_bytes, cudaStream_t s, bool cleared = false);
 // The dense gradients of such a payload, back into the buckets' tensors; its length
