@@ -38,11 +38,28 @@ __device__ __forceinline__ float row_reduce(float v, float* sm) {
   v = lane < kWarps ? sm[lane] : (MAX ? -INFINITY : 0.0f);
   return MAX ? warp_max(v) : warp_sum(v);
 }
+// The sum over twice as many threads: this one stands for itself (a) and for the one T
+// further on (b).
+template <int T>
+__device__ __forceinline__ float row_sum_of_two(float a, float b, float* sm) {
+  static_assert(T == 512, "32 partial sums");
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if ((threadIdx.x & 31) == 0) {
+    sm[threadIdx.x >> 5] = a;
+    sm[(threadIdx.x >> 5) + T / 32] = b;
+  }
+  __syncthreads();
+  return warp_sum(sm[threadIdx.x & 31]);
+}
 
 // One row in registers: NV vectors of kL elements per thread.
 template <typename V, int T, int NV>
 struct Row {
   static constexpr int kL = 16 / sizeof(V);
+  // 512 threads with eight vectors add up in the order of 1024 with four, which have the
+  // same row where there are fewer (by_length): a row's bits do not depend on the others.
+  static constexpr bool kOfTwo = T == 512 && NV == 8;
   float v[NV][kL];
   float sum;
 
@@ -87,9 +104,25 @@ struct Row {
 #pragma unroll
       for (int j = 0; j < kL; ++j) {
         v[k][j] = at(k, j, t, vec) < ncol ? expf(v[k][j] - m) : 0.0f;
-        s += v[k][j];
+        if (!kOfTwo) s += v[k][j];
       }
-    sum = row_reduce<T, false>(s, sm + 32);
+    if constexpr (kOfTwo) {
+      float of[2] = {0.f, 0.f};
+      if (vec) {                                   // every second vector is the other thread's
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+#pragma unroll
+          for (int j = 0; j < kL; ++j) of[k & 1] += v[k][j];
+      } else {                                     // every second element
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+#pragma unroll
+          for (int j = 0; j < kL; ++j) of[j & 1] += v[k][j];
+      }
+      sum = row_sum_of_two<T>(of[0], of[1], sm + 32);
+    } else {
+      sum = row_reduce<T, false>(s, sm + 32);
+    }
   }
   __device__ __forceinline__ static void store(V* __restrict__ y, size_t ncol, bool vec, int k, int t,
                                                const float (&e)[kL]) {
@@ -222,9 +255,10 @@ softmax_ce_long_kernel(const float* __restrict__ x, const int* __restrict__ t, f
 // all), then the smallest CTA whose threads hold the row with four vectors each.  A CTA of
 // 1024 threads has its SM to itself, so where there are more rows than SMs half the threads
 // take eight vectors each: one row's sums overlap another's loads, and twice the bytes are
-// in flight (us, 517 rows of 12384 24.0 -> 19.1, 149 11.2 -> 9.6, 1000 of 16000 40.4 -> 31.4;
-// shorter rows, of which an SM holds several anyhow, lost: 4096 of 3000 26.5 -> 32.0, 297 of
-// 6000 7.9 -> 10.1).  F is called with the two constants.
+// in flight, with the same additions in the same order (us, 517 rows of 12384 24.0 -> 17.9, with
+// loss and gradient 29.5 -> 24.4, 149 11.4 -> 9.0, 1000 of 16000 40.6 -> 31.6, 400 of 8194 16.9 ->
+// 13.5; shorter rows, of which an SM holds several anyhow, lost: 4096 of 3000 26.5 -> 32.0, 297
+// of 6000 7.9 -> 10.1).  F is called with the two constants.
 template <typename V, typename F>
 int by_length(size_t nrow, size_t ncol, F f) {
   constexpr size_t kL = 16 / sizeof(V);
