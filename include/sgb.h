@@ -674,6 +674,10 @@ int sgb_comm_set_topk_mode(sgb_comm *c, int mode);
 /* Communicator::wait (communicator.cc:169-186): the compute stream waits for
  * the three side streams. */
 int sgb_comm_wait(sgb_comm *c, void *compute_stream);
+/* The same for work behind it that uses none of the three streams: while the compute
+ * stream is being captured, those of them are waited for that take part in that capture.
+ * What was queued before it stays for the next sgb_comm_wait. */
+int sgb_comm_wait_captured(sgb_comm *c, void *compute_stream);
 /* Communicator::synch (communicator.cc:304-328): in-place all-reduce(sum) on
  * stream s after the compute stream's work so far. */
 int sgb_comm_synch(sgb_comm *c, void *data, size_t n, int is_half,

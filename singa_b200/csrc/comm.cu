@@ -458,6 +458,38 @@ int sgb_comm_wait(sgb_comm* c, void* compute_stream) {
   return emit(c, plan_call(c, sgb::order::kWait).before, sgb::as_stream(compute_stream));
 }
 
+// The capture that a stream takes part in; 0 where it takes part in none.
+static unsigned long long capture_of(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &st, &id) == cudaSuccess && st == cudaStreamCaptureStatusActive) return id;
+  cudaGetLastError();
+  return 0;
+}
+
+int sgb_comm_wait_captured(sgb_comm* c, void* compute_stream) {
+  if (!c) return SGB_ERR_NULL;
+  const cudaStream_t compute = sgb::as_stream(compute_stream);
+  const unsigned long long mine = capture_of(compute);
+  if (!mine) return sgb_comm_wait(c, compute_stream);
+  if (c->sparse_begun != c->sparse_ended) return SGB_ERR_STATE;
+  // what was queued before the capture stays as it is noted
+  sgb::order::State before;
+  before.dirty_s = c->order.dirty_s && capture_of(c->s) != mine;
+  before.dirty_c1 = c->order.dirty_c1 && capture_of(c->c1) != mine;
+  before.dirty_c2 = c->order.dirty_c2 && capture_of(c->c2) != mine;
+  if (before.dirty_c2) {
+    before.c2_reads_recv = c->order.c2_reads_recv;
+    before.sparse = c->order.sparse;
+  }
+  c->order.dirty_s &= !before.dirty_s;
+  c->order.dirty_c1 &= !before.dirty_c1;
+  c->order.dirty_c2 &= !before.dirty_c2;
+  const int st = emit(c, plan_call(c, sgb::order::kWait).before, compute);
+  c->order = before;
+  return st;
+}
+
 void* sgb_comm_result_stream(const sgb_comm* c) { return c ? side(c, c->result_stream) : nullptr; }
 
 int sgb_comm_order_plan(unsigned char* state, int call, unsigned* edges, int* result_stream) {
@@ -1092,7 +1124,7 @@ int sgb_comm_update_half(sgb_comm* c, void* const* params, void* const* grads, v
   sgb::SgdArgs sgd;
   OK(sgb::sgd_args(&sgd, moments, lr, momentum, dampening, weight_decay, nesterov, grad_scale));
   // no buffer of the communicator takes part: behind what its streams still do, on the caller's
-  OK(sgb_comm_wait(c, compute_stream));
+  OK(sgb_comm_wait_captured(c, compute_stream));
   return sgb::sgd_round_f16_multi(params, grads, moments, sizes, count, sgd, sgb::as_stream(compute_stream));
 }
 

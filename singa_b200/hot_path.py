@@ -416,6 +416,9 @@ class HotPathGPU(object):
         order_index = {n: i for i, n in enumerate(self.plan["grad_order"])}
         beside, behind = self._forked_update()
         forks = behind is not None
+        if forks and self.comm is not None:
+            # the captured step exchanges nothing itself: behind what the caller has in the capture
+            prog.append(("sgb_comm_wait_captured", (self.comm._h.value, "STREAM"), _CAPTURED))
         for name, args in self.launched:
             if name == "grad_ready":
                 idx = order_index[args]

@@ -1094,6 +1094,7 @@ const Callable kCallables[] = {
     CALLABLE(sgb_comm_synch_half), CALLABLE(sgb_comm_fused_synch), CALLABLE(sgb_comm_fused_synch_half),
     CALLABLE(sgb_comm_sparsification), CALLABLE(sgb_comm_wait), CALLABLE(sgb_comm_profile_mark),
     CALLABLE(sgb_comm_profile_range), CALLABLE(sgb_comm_update_half), CALLABLE(sgb_sgd_update_beside_f32),
+    CALLABLE(sgb_comm_wait_captured),
 };
 
 enum Patch { kStream, kSideStream, kResultStream, kResultIndex, kLr, kMomentum, kDecay, kPatches };
