@@ -119,14 +119,17 @@ def workspace_bytes(plan):
     return max(need)
 
 
-def _recorded(name):
+def _recorded(name, *with_it):
     """An attribute that the recorded program of a step holds (the communicator by
-    its address): setting it has the program recorded anew at the next run."""
+    its address): setting it has the program recorded anew at the next run.  Setting it
+    sets those `with_it` to the same truth value."""
     def read(self):
         return getattr(self, "_" + name)
 
     def write(self, value):
         setattr(self, "_" + name, value)
+        for other in with_it:
+            setattr(self, other, bool(value))
         self._program = None
     return property(read, write)
 
@@ -138,7 +141,9 @@ _ALWAYS, _PROFILED, _CAPTURED, _SINGLE = range(4)
 
 class HotPathGPU(object):
     comm, world, dist_option = _recorded("comm"), _recorded("world"), _recorded("dist_option")
-    spars, update_on_arrival = _recorded("spars"), _recorded("update_on_arrival")
+    # _branch: without a communicator nothing arrives, but a captured step may update its
+    # buckets before the pass is over, unless it was asked not to.
+    spars, update_on_arrival = _recorded("spars"), _recorded("update_on_arrival", "_branch")
 
     def __init__(self, plan, communicator=None, world=1, seed=0, lr=0.1, momentum=0.9,
                  weight_decay=1e-5, threshold=2097152, dist_option="plain", spars=0.05,
@@ -150,9 +155,9 @@ class HotPathGPU(object):
         # communicator's side stream as soon as that bucket's reduced gradients
         # have landed, overlapped with the rest of the backward pass (same
         # results as updating everything after the final wait).
-        self._on_arrival = bool(update_on_arrival)
         self.update_on_arrival = bool(update_on_arrival) and communicator is not None \
             and dist_option in ("plain", "half")
+        self._branch = bool(update_on_arrival)
         # pool_argmax: max-pool backward consumes the arg-max record of the forward
         # partner (produced once at set-up: the forward pass is outside this path)
         # instead of recomputing the winners from x and y.  Same dx bit for bit.
@@ -414,7 +419,7 @@ class HotPathGPU(object):
         prog, self.calls_per_step = [], 0
         self.launched = merge_calls(self.calls)
         order_index = {n: i for i, n in enumerate(self.plan["grad_order"])}
-        beside, behind = self._forked_update()
+        beside, behind, self._late_tables = self._forked_update()
         forks = behind is not None
         if forks and self.comm is not None:
             # the captured step exchanges nothing itself: behind what the caller has in the capture
@@ -432,7 +437,7 @@ class HotPathGPU(object):
                 prog += behind or []
                 if beside:
                     prog.append(("join", (), _CAPTURED))
-                if self.update_on_arrival:
+                if self._arrives():
                     continue                  # every bucket was updated as it arrived
                 prog.append(self._sgd_call(self.sgd_tables, "STREAM", when))
                 self.calls_per_step += 1
@@ -453,12 +458,16 @@ class HotPathGPU(object):
                     self.lib.sgb_bn_backward_draws_table(n, c, h * w, masks[op.kind], self.ws.numel()) != 0
         self._program = _lib.native.program(prog, None if self.comm is None else self.comm._h.value, not single)
 
+    def _arrives(self):
+        """Whether buckets are updated where their reduced gradients land."""
+        return self.update_on_arrival and self.comm is not None and self.dist_option in ("plain", "half")
+
     def _forked_update(self):
         """The update in a captured step without other ranks: what goes on a branch of
         its own beside the rest of the backward pass, as {gradient that completes a
-        bucket: call}, and the calls behind the pass.  ({}, None) where the update stays
-        as it is: several ranks, the sparse exchanges, or one update behind the whole
-        pass was asked for.
+        bucket: call}, the calls behind the pass, and the tables that these read.  ({}, None,
+        None) where the update stays as it is: several ranks, the sparse exchanges, or one
+        update behind the whole pass was asked for.
 
         A step of small layers leaves most of the memory's rate unused, and the update
         is nothing but memory traffic.  A bucket goes on the branch if that gets done
@@ -475,13 +484,13 @@ class HotPathGPU(object):
             return max((sum(self.grads[i].numel() for i in ev[1]) for ev in self.events if ev[0] in kinds), default=0)
 
         if self.comm is None:
-            if not self._on_arrival:
-                return {}, None
+            if not self._branch:
+                return {}, None, None
         # one rank: the sum over the ranks is the gradient (rounded, in half precision);
         # what does not fit the communicator's buffers is refused by its own calls
-        elif self.comm.world_size != 1 or not self.update_on_arrival or \
+        elif self.comm.world_size != 1 or not self._arrives() or \
                 largest(("direct", "fused") if half else ("fused",)) > getattr(self.comm, "buffSize", 0):
-            return {}, None
+            return {}, None, None
         rates = ("LR", "MOMENTUM", 0.0, "DECAY", 0, float(np.float32(1.0) / np.float32(self.world)))
 
         def addresses(tables):
@@ -509,15 +518,15 @@ class HotPathGPU(object):
             else:
                 late += bucket
         if not late:
-            return beside, []
+            return beside, [], None
         names = [self.plan["grad_order"][i] for i in late]
         ps, gs, ms = ([t[n] for n in names] for t in (self.t, {n: self.t["d:" + n] for n in names}, self.moments))
-        self._late_tables = (_table(ps)[0], _table(gs)[0], _table(ms)[0], _table(ps)[1], len(names))
-        tables = addresses(self._late_tables)
+        keep = (_table(ps)[0], _table(gs)[0], _table(ms)[0], _table(ps)[1], len(names))
+        tables = addresses(keep)
         if half:
             return beside, [("sgb_comm_update_half", (self.comm._h.value,) + tables + (max(p.numel() for p in ps),) + rates +
-                             ("STREAM",), _CAPTURED)]
-        return beside, [("sgb_sgd_update_multi_f32", tables + rates + ("STREAM",), _CAPTURED)]
+                             ("STREAM",), _CAPTURED)], keep
+        return beside, [("sgb_sgd_update_multi_f32", tables + rates + ("STREAM",), _CAPTURED)], keep
 
     def _sgd_call(self, tables, stream, when=_ALWAYS):
         pp, gp, mp, sizes, n = tables
@@ -573,7 +582,7 @@ class HotPathGPU(object):
         """The bucket's parameters are updated on the side stream on which its
         reduced gradients land (never on the NCCL stream: the next bucket's
         all-reduce does not wait for this update)."""
-        if not self.update_on_arrival:
+        if not self._arrives():
             return
         h = self.comm._h.value
         prog.append(("sgb_comm_profile_range", (h, b"sgd_update_bucket", "RESULT_INDEX", 1), when))

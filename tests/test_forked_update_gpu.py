@@ -46,6 +46,56 @@ def test_captured_steps_equal_single_calls(sync, threshold, on_arrival):
     comm.close()
 
 
+def replayed(hp, runs=3):
+    hp.run_step()
+    torch.cuda.synchronize()
+    graph = hp.capture()
+    for _ in range(runs - 1):
+        graph.replay()
+    out = [t.clone() for t in state(hp)]
+    hp.release_graph()
+    return out
+
+
+def branches(hp):
+    """What the recorded step does on a branch of its own."""
+    return hp._forked_update()[0]
+
+
+def test_the_branch_can_be_turned_off():
+    on, off, built_off = step("none", 200, None), step("none", 200, None), step("none", 200, None, update_on_arrival=False)
+    assert branches(on) and not branches(built_off)
+    off.update_on_arrival = False
+    assert not branches(off)
+    assert all(torch.equal(a, b) for a, b in zip(replayed(on), replayed(off)))
+
+
+@pytest.mark.parametrize("change", ["no communicator", "sparse"])
+def test_what_arrives_follows_what_is_set(change):
+    """Captured steps and single ones do the same after the exchange has been changed."""
+    from singa_b200.communicator import Communicator, NcclIdHolder
+    comm = Communicator(torch.cuda.current_device(), 1, NcclIdHolder(), buffSize=1 << 20)
+    single, captured = step("plain", 200, comm), step("plain", 200, comm)
+    reference = step("plain", 200, comm)
+    reference.update_on_arrival = False
+    for hp in (single, captured, reference):
+        if change == "sparse":
+            hp.dist_option, hp.spars = "sparseTopK", 0.4
+            hp.residuals = {i: torch.zeros(sum(hp.grads[k].numel() for k in ev[1]), device="cuda") for i, ev in hp.flush_after.items()}
+        else:
+            hp.comm = None
+    assert not (change == "sparse" and branches(captured))
+    for _ in range(3):
+        single.run_step()
+        reference.run_step()
+    want = state(reference)
+    assert all(torch.equal(a, b) for a, b in zip(state(single), want))
+    assert any(bool(m.any()) for m in single.moments.values())
+    if change != "sparse":                       # (a captured sparse step is not replayed here: the host takes part)
+        assert all(torch.equal(a, b) for a, b in zip(replayed(captured), want))
+    comm.close()
+
+
 @pytest.mark.parametrize("count", [2, 11])      # more than there are side streams
 def test_several_steps_in_one_capture(count):
     single, together = [[step("none", 200, None) for _ in range(count)] for _ in range(2)]
