@@ -119,6 +119,28 @@ def workspace_bytes(plan):
     return max(need)
 
 
+def leaves_what_is_ready(plan):
+    """Whether the parameters can be updated before the pass is over, with the results of
+    one update at its end: each gradient is reported ready once, in the order of the
+    buckets, no op behind that touches it or its parameter, and the one update comes
+    behind all of them and is of them all."""
+    order, done = list(plan["grad_order"]), set()
+    ready = [op.args["param"] for op in plan["ops"] if op.kind == "grad_ready"]
+    if ready != order or sorted(order) != sorted(plan["params"]) or \
+            sum(op.kind == "sync_and_update" for op in plan["ops"]) != 1:
+        return False
+    for op in plan["ops"]:
+        if op.kind == "sync_and_update":
+            break
+        if op.kind == "grad_ready":
+            done |= {op.args["param"], "d:" + op.args["param"]}
+            continue
+        for value in op.args.values():
+            if not done.isdisjoint(value if isinstance(value, (tuple, list)) else (value,)):
+                return False
+    return len(done) == 2 * len(order)
+
+
 def _recorded(name, *with_it):
     """An attribute that the recorded program of a step holds (the communicator by
     its address): setting it has the program recorded anew at the next run.  Setting it
@@ -466,8 +488,8 @@ class HotPathGPU(object):
         """The update in a captured step without other ranks: what goes on a branch of
         its own beside the rest of the backward pass, as {gradient that completes a
         bucket: call}, the calls behind the pass, and the tables that these read.  ({}, None,
-        None) where the update stays as it is: several ranks, the sparse exchanges, or one
-        update behind the whole pass was asked for.
+        None) where the update stays as it is: several ranks, the sparse exchanges, one
+        update behind the whole pass was asked for, or `leaves_what_is_ready` does not hold.
 
         A step of small layers leaves most of the memory's rate unused, and the update
         is nothing but memory traffic.  A bucket goes on the branch if that gets done
@@ -479,6 +501,8 @@ class HotPathGPU(object):
         in half precision 35 -> 21, the CNN of 53 channels at batch 49 44 -> 35.  All of
         the 4096 MLP's update on the branch: 76 -> 111, so its rate matters."""
         half = self.comm is not None and self.dist_option == "half"
+        if not leaves_what_is_ready(self.plan):
+            return {}, None, None
 
         def largest(kinds):
             return max((sum(self.grads[i].numel() for i in ev[1]) for ev in self.events if ev[0] in kinds), default=0)

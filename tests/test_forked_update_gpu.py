@@ -96,6 +96,22 @@ def test_what_arrives_follows_what_is_set(change):
     comm.close()
 
 
+@pytest.mark.parametrize("kind", ["no update", "a gradient changed behind its report"])
+def test_plans_of_other_forms(kind):
+    from singa_b200.hot_path import HotPathGPU
+    from singa_b200.resnet50_path import Op, build_mlp_plan, fuse_plan
+    plan = fuse_plan(build_mlp_plan(batch=9, dims=(23, 130, 57, 10)))
+    if kind == "no update":
+        ops = [op for op in plan["ops"] if op.kind != "sync_and_update"]
+    else:
+        ops = plan["ops"][:-1] + [Op("scale", dict(x="d:" + plan["grad_order"][0], c=0.5))] + plan["ops"][-1:]
+    single, captured = [HotPathGPU(dict(plan, ops=ops), seed=5, threshold=200) for _ in range(2)]
+    single.profile = True                        # one by one
+    for _ in range(3):
+        single.run_step()
+    assert all(torch.equal(a, b) for a, b in zip(replayed(captured), state(single)))
+
+
 @pytest.mark.parametrize("count", [2, 11])      # more than there are side streams
 def test_several_steps_in_one_capture(count):
     single, together = [[step("none", 200, None) for _ in range(count)] for _ in range(2)]
