@@ -1498,6 +1498,45 @@ inline bool revisit_pays(int N, int C, int HW, bool aligned, bool groups) {
          (channel <= 4000000 || elements <= 20000000);
 }
 
+// Whether channels that fit a CTA's registers, read one float an access, go through groups of
+// G all the same: above 2e6 elements, where the call is bound by bytes and no longer by
+// latency, unless a channel nearly fills the threads' 512, 1024 or 2048 slots, or is so small
+// that a group's threads find little to do.  Cold inputs, us in registers / in groups, 2.3e6
+// elements if not said:
+//   elements of a channel   plain                   ReLU's input          its bits
+//     49                   13.2 / 36.1             13.9 / 49.9           13.7 / 49.7
+//    294 (of 512)          10.9 / 12.1             13.9 / 14.5           14.2 / 14.1
+//    441, 1e7              30.0 / 33.4             39.6 / 41.2           43.9 / 40.8
+//    567 (of 1024)          9.8 /  9.2             12.2 / 10.9           14.7 / 10.3
+//    637                    9.0 /  9.4             11.4 / 11.1           13.8 / 10.6
+//    686                    8.7 /  9.3             10.7 / 10.9           14.3 / 10.2
+//    735, 3.6e6 and 5e6    12.1 / 12.6, 16.2 / 16.0  15.6 / 15.2, 20.8 / 19.4  19.8 / 14.5, 27.1 / 18.4
+//    833, 5e6 and 7.5e6    15.2 / 16.4, 21.6 / 22.3  19.3 / 19.5, 28.2 / 26.8  26.3 / 18.8, 37.1 / 26.1
+//   1014, 1.3e7            30.9 / 34.7             40.7 / 41.8           58.7 / 40.7
+//   1617 (of 2048)          9.8 /  9.1             12.5 / 12.2           16.0 / 10.3
+//   1764, and 3.6e6         9.6 /  9.6, 13.4 / 12.4  11.0 / 13.1, 17.1 / 17.0  16.2 / 10.9, 22.4 / 14.4
+//   1960, 3.6e6 and 7.5e6  12.7 / 13.3, 24.0 / 21.5  16.9 / 17.4, 31.9 / 28.6  23.4 / 15.6, 41.8 / 26.3
+//   2025, 5e6 and 7.5e6    16.1 / 17.1, 22.8 / 22.2  21.4 / 21.8, 31.2 / 28.9  29.9 / 19.7, 42.2 / 26.5
+//   2997 (of 3072)         11.1 / 10.8             17.3 / 15.0           24.5 / 12.8
+// and in groups of two, which are half as large:
+//    600, 5e6              18.3 / 21.9             22.4 / 28.1           28.0 / 27.3
+//    900, 5e6              14.2 / 19.3             18.4 / 24.0           26.3 / 22.6
+//   1050                   12.1 /  9.2             14.8 / 11.2           16.6 / 10.6
+//   1800, 5e6              17.1 / 16.0             22.6 / 20.1           28.7 / 18.3
+//   3000                    8.1 /  8.8             12.0 / 11.8           17.1 / 10.0
+// A ReLU's input and its bits take the same side, so that they have the same bits; it is
+// the side of the input.
+inline bool groups_pay(long long channel, long long elements, int G, bool masked) {
+  if (channel <= 512 || (G == 2 && channel <= 1024)) return false;
+  if (channel <= 640) return elements > 2000000;
+  if (channel <= 768) return elements > 4000000;
+  if (channel <= 1024) return masked && channel <= 960 && elements > 6000000;
+  if (channel <= 1680) return elements > 2000000;
+  if (channel <= 1920) return elements > 3500000;
+  if (channel <= 2048) return elements > 6000000;
+  return elements > 2000000;
+}
+
 template <int MASK>
 int bn_backward(const float* x, const float* dy, const float* relu_in, const float* scale,
                 const float* mean, const float* invstd, float* dx, float* dscale,
@@ -1528,29 +1567,8 @@ int bn_backward(const float* x, const float* dy, const float* relu_in, const flo
                                        ws_bytes, s);
     if (st != SGB_ERR_WORKSPACE) return st;            // a smaller workspace: the forms below
   }
-  // Channels that fit a CTA's registers need no staging.  Where that means scalar
-  // accesses the group form takes over above 2e6 elements, where the call is bound by
-  // bytes and no longer by latency, unless a channel nearly fills the threads' 1024 or
-  // 2048 slots.  Cold inputs, us in registers / in groups, (plain; with the ReLU's
-  // input; with its bits), 2.1e6 to 3.2e6 elements if not said:
-  //   elements of a channel   plain                   input                 bits
-  //   567 (of 1024)           9.7 /  9.2             12.0 / 10.8           13.8 / 10.3
-  //   882                     7.8 / 10.0             10.4 / 11.5           12.1 / 11.0
-  //   1014                    6.8 /  9.1              8.6 / 10.9           12.7 / 10.1
-  //   980, 5.9e6             15.9 / 19.3             21.1 / 22.4           29.4 / 21.7
-  //   1125 (of 2048)         12.1 /  8.5             15.0 / 10.6           17.6 / 10.2
-  //   1568                   13.0 / 10.8             16.5 / 14.5           20.6 / 12.9
-  //   1715                    9.9 /  9.5             12.7 / 12.6           16.5 / 10.7
-  //   2025                    7.7 /  9.1             10.3 / 11.7           13.1 / 10.1
-  //   2160 (of 3072)         10.0 /  8.5             15.6 / 10.8           19.3 /  9.9
-  //   2997                   11.1 / 10.8             17.3 / 15.0           24.5 / 12.8
-  // Up to 1.6e6 elements registers are the better or within a tenth.  A ReLU's input
-  // and its bits take the same side, so that they have the same bits; a plain call's
-  // full channels come back to groups above 6e6.
-  const long long elements = per_channel * C;
-  const bool full = per_channel <= 1024 ? per_channel > 768 : per_channel > 1600 && per_channel <= 2048;
-  const bool grouped = groups && elements > 2000000LL &&
-                       (MASK == 0 ? !full || elements > 6000000LL : !full && per_channel > 1024);
+  // Channels that fit a CTA's registers need no staging.
+  const bool grouped = groups && groups_pay(per_channel, per_channel * C, G, MASK != 0);
   if (!grouped) {
     int st = SGB_OK;
     auto go = [&](auto g, auto nv, auto v) {

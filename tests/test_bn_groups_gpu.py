@@ -15,6 +15,12 @@ SHAPES = [(11, 20000, 3, 3), (17, 21000, 1, 6), (400, 2600, 1, 2), (350, 2048, 1
           (32, 1300, 7, 7), (32, 1276, 7, 7),                                                  # 2e6 elements, both sides
           (9, 3000, 9, 9), (16, 3000, 7, 7), (6, 2200, 13, 13), (50, 1600, 5, 5), (33, 1300, 7, 7), (23, 3500, 9, 9),
           (25, 1024, 9, 9), (33, 1024, 9, 9), (65, 640, 7, 7), (128, 512, 5, 5), (14, 700, 15, 15), (42, 340, 10, 15)]
+# both sides of each line in elements of a channel (512, 640, 768, 960, 1024, 1680, 1920, 2048)
+# and in all (2e6, 3.5e6, 4e6, 6e6); groups of two: 1024
+SHAPES += [(10, 4200, 3, 17), (9, 4000, 3, 19), (128, 3300, 1, 5), (129, 3200, 1, 5), (129, 6300, 1, 5), (256, 5300, 1, 3),
+           (257, 5300, 1, 3), (64, 6400, 3, 5), (64, 6200, 3, 5), (65, 6400, 3, 5), (341, 2000, 1, 3), (205, 2000, 1, 5),
+           (336, 1200, 1, 5), (561, 1200, 1, 3), (384, 1840, 1, 5), (384, 1800, 1, 5), (641, 1840, 1, 3), (641, 3124, 1, 3),
+           (683, 1000, 1, 3), (102, 2000, 1, 10), (103, 2000, 1, 10)]
 
 
 def rel(got, want):
