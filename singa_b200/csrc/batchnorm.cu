@@ -1451,13 +1451,18 @@ int takes_cluster(long long per_channel, bool vec, int C, int* per_cta) {
 // Whether a call takes the form that visits its data twice (bn_revisit.cu).  It
 // overlaps everything but its first loads and last stores, which a call has to be
 // large enough for; the line is the same whatever the mask, so that a fused call
-// and its parts agree bit for bit, and lies where a call without a ReLU loses nothing.
+// and its parts agree bit for bit, and lies where a call with a ReLU gains a microsecond or
+// more, and one without at best as much and at worst loses 0.4.
 // Time of the forms below / of this one, with and without a ReLU:
-//   16x64x56x56   (3.2e6 elements)  14.0 / 11.2   10.2 /  9.6
-//   32x128x28x28  (3.2e6)           13.7 / 11.1    9.9 /  9.9
-//   32x512x14x14  (3.2e6)           14.0 / 11.8    9.8 /  9.9
-//   8x512x28x28   (3.2e6)           13.8 / 11.6    9.9 /  9.4
-//   12x48x80x80   (3.7e6)           14.1 / 13.2   10.1 / 10.5
+//   24x40x56x56   (3.0e6 elements)  12.9 / 10.8    9.2 /  9.6
+//   16x64x56x56   (3.2e6)           14.2 / 11.1   10.4 /  9.6
+//   32x128x28x28  (3.2e6)           14.2 / 11.4   10.0 /  9.9
+//   32x512x14x14  (3.2e6)           13.8 / 11.9    9.5 /  9.9
+//   8x512x28x28   (3.2e6)           13.9 / 11.7    9.9 /  9.4
+//   32x256x20x20  (3.3e6)           14.5 / 12.0   10.0 /  9.8
+//   9x30x112x112  (3.4e6)           21.6 / 12.0   16.0 /  9.9
+//   6x48x112x112  (3.6e6)           14.1 / 13.0   10.3 / 10.5
+//   12x48x80x80   (3.7e6)           13.9 / 13.1   10.5 / 10.3
 //   32x1024x14x14 (6.4e6)           24.1 / 20.7   18.3 / 16.8
 //   12x200x50x50  (6.0e6)           25.4 / 19.2   17.4 / 15.4
 // smaller ones: 10x256x30x30 (2.3e6) 10.8 / 9.5, 7.8 / 8.2; 8x256x32x32 (2.1e6) 10.3 / 8.9,

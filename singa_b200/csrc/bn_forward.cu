@@ -573,10 +573,13 @@ bn_fwd_revisit_kernel(const __grid_constant__ FwdArgs a, const __grid_constant__
 //   32x64x112x112 61.5 / 40.5   32x64x56x56 14.9 / 13.3    64x100x40x40  19.4 / 18.5
 //   32x512x28x28 25.4 / 24.7    10x256x52x52 15.5 / 14.8   12x200x50x50  12.5 / 13.7
 // and odd planes, whose clusters read with masked ends:
-//   32x128x57x57 37.3 / 28.6    24x64x71x71 24.4 / 18.4    24x64x57x57   18.9 / 14.7
-//   40x32x51x51  13.7 / 10.2    24x64x37x37  9.9 / 8.8     33x128x35x35  16.9 / 15.6
-//   12x64x69x69  12.6 / 11.9    40x64x31x31 10.3 / 10.3    18x100x47x47  12.9 / 13.3
+//   32x128x57x57 37.3 / 28.6    24x64x71x71 24.4 / 18.4    24x64x57x57   19.1 / 14.8
+//   40x32x51x51  13.5 / 10.4    24x64x37x37 10.2 / 9.4     33x128x35x35  17.0 / 15.3
+//   12x64x69x69  12.6 / 11.9    40x64x31x31 11.0 / 10.1    18x100x47x47  12.9 / 12.8
+//   20x100x47x47 13.7 / 13.7    4x100x99x99 12.7 / 12.1    16x96x49x49   12.6 / 13.2
 //   18x256x25x25 11.1 / 11.6 (11,250 elements a channel), 4x128x57x57 8.5 / 8.9 (12,996)
+// (the last two are on the other side; of the 22 shapes in this range that were looked at,
+// 16x96x49x49 alone lost more than a percent)
 // The lower line for whole vectors is from a layer's forward, ReLU and backward in
 // sequence: what the second visit leaves in L2 is x, and what comes next reads y
 // (elements of a channel: 69,000 134.3 / 136.7, 75,000 145.4 / 147.9, 88,000 149.7 /
