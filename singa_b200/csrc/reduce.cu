@@ -335,7 +335,7 @@ chansum_kernel(const float* __restrict__ dy, const float* __restrict__ x, float*
   // (sample, position) of the unit is advanced without a division per step
   int n = (i0 + static_cast<int>(threadIdx.x)) / hwu, q = (i0 + static_cast<int>(threadIdx.x)) - n * hwu;
   const int dn = kBlock / hwu, dq = kBlock - dn * hwu;
-  if (RELU && first_wave(8)) {
+  if (RELU && first_wave(4)) {      // (8 asked ahead for CTAs that start later: 64x256x14x14 from L2 8.6 us, 8.2 so)
     int pn = n, pq = q;
     for (int k = 0, i = i0 + threadIdx.x; k < 4 && i < i1; ++k, i += kBlock) {
       const size_t at = (static_cast<size_t>(pn) * C + c) * HW + static_cast<size_t>(pq) * kW;
@@ -642,15 +642,19 @@ int sgb_maxpool_relu_backward_conv_bias_f32(const float* pool_x, const float* po
   // whole rows.  It pays while a CTA's threads have their few vectors in flight at once
   // and the grid is one wave (elements per CTA, CTAs: the two calls / one, with the
   // operands in L2, as a step of small layers has them, and from DRAM):
-  //   1024, 64     16x64x8x8     3.0 / 2.2    2.9 / 2.0
-  //   2304, 256    32x32x24x24   5.8 / 4.8    6.3 / 6.4
-  //   4608, 256    64x32x24x24   7.7 / 6.5    8.9 / 9.5
-  //   4608, 512    256x64x12x12 11.6 / 9.5   11.9 / 11.7
-  //   2304, 1024   32x128x24x24  9.0 / 11.8   9.9 / 14.2
-  //   9216, 64     128x8x24x24   7.7 / 8.0    9.4 / 13.6
-  //   9216, 256    128x32x24x24 13.7 / 9.5   13.7 / 16.3
-  //   36864, 96    512x12x24x24 19.1 / 25.6  29.4 / 49.8
-  // and not with single accesses (64x32x13x13 8.1 / 10.2, 256x8x15x15 13.5 / 21.9).
+  //   1024, 64     16x64x8x8     3.0 / 1.8    3.0 / 1.8
+  //   2304, 256    32x32x24x24   5.2 / 4.5    5.5 / 5.6
+  //   2304, 512    32x64x24x24   6.9 / 5.7    7.6 / 6.7
+  //   4608, 64     64x8x24x24    4.7 / 5.0    5.5 / 6.6
+  //   4608, 128    64x16x24x24   5.6 / 5.4    6.5 / 7.2
+  //   4608, 256    64x32x24x24   7.2 / 6.1    7.6 / 8.3
+  //   4608, 512    256x64x12x12  9.4 / 8.2   10.7 / 10.8
+  //   2304, 1024   32x128x24x24 10.7 / 11.0  11.8 / 13.0
+  //   9216, 64     128x8x24x24   6.6 / 7.4    7.6 / 10.7
+  //   9216, 256    128x32x24x24 10.0 / 9.3   11.3 / 13.5
+  //   36864, 96    512x12x24x24 15.1 / 27.8  19.1 / 37.8
+  // (64x8x24x24 is the one shape on this side that loses from L2.)  A form with single
+  // accesses, for other widths, lost (64x32x13x13 8.1 / 10.2, 256x8x15x15 13.5 / 21.9).
   bool clustered, pays = kh == 2 && kw == 2 && sh == 2 && sw == 2 && ph == 0 && pw == 0 && N > 0 && C > 0 && H >= 2 &&
                          HW && W % 4 == 0 && pool_x && dy && pool_dx && x && dx && db && aligned16(pool_x) &&
                          aligned16(pool_dx) && aligned16(x) && aligned16(dx) && C <= 65535;
