@@ -750,8 +750,11 @@ int sgb_comm_sparsification_buckets(sgb_comm *c, void *const *tensors, const siz
  * kernel that writes the dense gradients.  The update has to run on the
  * communicator's stream, so it is complete behind sgb_comm_wait.  One rank;
  * SGB_ERR_UNSUPPORTED, and nothing done, where it takes separate calls. */
-/* (0 of the next call: it would not take such a list, by sizes and places alone; nor,
- * by threshold, one of more than SGB_SPARSE_UPDATE_TENSORS tensors.) */
+/* What it takes, besides the limits above: by threshold one tensor of up to 2^25
+ * elements, or up to SGB_SPARSE_UPDATE_TENSORS tensors of 4,000,000 in all; the largest
+ * share of one bucket of up to 16 tensors, or of several buckets, if one launch holds them
+ * (32 buckets, 256 runs of tensors, 2^25 elements) or they have 2^20 elements or more.
+ * (0 of the next call: it would not take such a list, by sizes and places alone.) */
 #define SGB_SPARSE_UPDATE_TENSORS 8
 int sgb_comm_sparse_update_takes(const sgb_comm *c, void *const *tensors, const size_t *sizes, const size_t *counts,
                                  size_t nbuckets, int topk);

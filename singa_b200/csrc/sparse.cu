@@ -1831,8 +1831,8 @@ static bool topk_plan(const SparseBucket* buckets, const size_t* ks, size_t coun
 
 // A list that one launch cannot take goes through several, of about as many buckets
 // each (2.56e7 elements, the largest 1.8 % of 35 buckets: 1105 us a pass with a call per
-// bucket, 270 in two groups).  Below a million elements a list that one launch does not
-// take keeps its calls, as the interface says.
+// bucket, 270 in two groups).  Below 2^20 elements a list that one launch does not take
+// keeps its calls, as sgb.h says.
 constexpr size_t kLeastCut = size_t{1} << 20;
 bool sparse_topk_buckets_cut(float* const* tensors, const size_t* sizes, const size_t* counts, size_t nbuckets,
                              std::vector<size_t>* ends) {

@@ -494,12 +494,16 @@ class HotPathGPU(object):
         A step of small layers leaves most of the memory's rate unused, and the update
         is nothing but memory traffic.  A bucket goes on the branch if that gets done
         while the pass lasts; what does not is updated behind it, by all of the GPU at
-        once.  Before -> with it, us a step: ResNet-50, batch 3 at 160^2 279 -> 253, 2 at
-        159^2 240 -> 213, 9 at 97^2 322 -> 303; on one rank, where the communicator's
-        streams had the update, plain 10 at 85^2 363 -> 336 and in half precision 2 at
-        190^2 365 -> 333; the MLP of 2035 at batch 5, plain, 45 -> 36, of 748 at batch 177
-        in half precision 35 -> 21, the CNN of 53 channels at batch 49 44 -> 35.  All of
-        the 4096 MLP's update on the branch: 76 -> 111, so its rate matters."""
+        once.  Launched one by one (the first runs of a program and those after its rates
+        have changed) the step stays as it is.  All figures here are of one B200 and of
+        graphs, as are the rates below, from which it follows which buckets go where.
+
+        Without -> with it, us a step: ResNet-50, batch 3 at 160^2 277 -> 249, 2 at 159^2
+        241 -> 211, 9 at 97^2 321 -> 302; on one rank, where the communicator's streams had
+        the update, plain 10 at 85^2 314 -> 300 and in half precision 2 at 190^2 313 -> 304;
+        the MLP of 2035 at batch 5, plain, 41 -> 31, of 748 at batch 177 in half precision
+        35 -> 19, the CNN of 53 channels at batch 49 35 -> 23.  All of the 4096 MLP's update
+        on the branch: 76 -> 111, so its rate matters."""
         half = self.comm is not None and self.dist_option == "half"
         if not leaves_what_is_ready(self.plan):
             return {}, None, None

@@ -1114,8 +1114,9 @@ struct Call {
   int when;
   bool join = false;
 };
-// A side stream, below the priority of what it runs beside, and the event that orders it.
-// A few are kept per device for all programs (one costs more than a millisecond); one that
+// A side stream and the event that orders it.  It has the priority of ordinary streams,
+// which is the lowest there is: what leaves room for the kernels that it runs beside is that
+// its own have one block an SM.  A few are kept per device for all programs (one costs more than a millisecond); one that
 // takes part in a capture is not lent again before that ends.
 struct Side {
   cudaStream_t stream = nullptr;
@@ -1141,12 +1142,9 @@ class Sides {
       if (status == cudaStreamCaptureStatusNone) return lent(side.get());
     }
     if (sides.size() == kMost) return nullptr;
-    int least = 0, greatest = 0;
     auto side = std::make_unique<Side>();
-    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
-        cudaEventCreateWithFlags(&side->event, cudaEventDisableTiming) != cudaSuccess)
-      return failed();
-    if (cudaStreamCreateWithPriority(&side->stream, cudaStreamNonBlocking, least) != cudaSuccess) {
+    if (cudaEventCreateWithFlags(&side->event, cudaEventDisableTiming) != cudaSuccess) return failed();
+    if (cudaStreamCreateWithFlags(&side->stream, cudaStreamNonBlocking) != cudaSuccess) {
       cudaEventDestroy(side->event);
       return failed();
     }

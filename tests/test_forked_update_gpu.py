@@ -113,7 +113,8 @@ def test_plans_of_other_forms(kind):
 
 
 @pytest.mark.parametrize("count", [2, 11])      # more than there are side streams
-def test_several_steps_in_one_capture(count):
+@pytest.mark.parametrize("mode", ["thread_local", "global"])
+def test_several_steps_in_one_capture(count, mode):
     single, together = [[step("none", 200, None) for _ in range(count)] for _ in range(2)]
     for hp in single:
         hp.profile = True                        # one by one
@@ -121,7 +122,7 @@ def test_several_steps_in_one_capture(count):
         hp.run_step()
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+    with torch.cuda.graph(graph, capture_error_mode=mode):
         for hp in together:
             hp.run_step()
     for _ in range(3):
