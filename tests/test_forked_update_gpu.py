@@ -106,6 +106,7 @@ def test_plans_of_other_forms(kind):
     else:
         ops = plan["ops"][:-1] + [Op("scale", dict(x="d:" + plan["grad_order"][0], c=0.5))] + plan["ops"][-1:]
     single, captured = [HotPathGPU(dict(plan, ops=ops), seed=5, threshold=200) for _ in range(2)]
+    assert not branches(captured)
     single.profile = True                        # one by one
     for _ in range(3):
         single.run_step()
