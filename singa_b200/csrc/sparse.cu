@@ -2038,7 +2038,7 @@ extern "C" {
 size_t sgb_sparse_workspace_bytes(size_t n) { return n ? workspace_bytes(n) : 256; }
 
 size_t sgb_sparse_topk_plan(const size_t* sizes, const size_t* ks, size_t nbuckets, int mode, size_t* counters) {
-  if (!sizes || !ks || !counters) return 0;
+  if (!sizes || !ks || !counters || nbuckets > kBuckets) return 0;
   float* const somewhere = reinterpret_cast<float*>(static_cast<uintptr_t>(256));   // never followed
   std::vector<SparseBucket> buckets;
   for (size_t k = 0; k < nbuckets; ++k) buckets.push_back({&somewhere, sizes + k, 1, somewhere});
