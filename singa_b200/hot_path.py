@@ -136,7 +136,8 @@ def leaves_what_is_ready(plan):
             done |= {op.args["param"], "d:" + op.args["param"]}
             continue
         for value in op.args.values():
-            if not done.isdisjoint(value if isinstance(value, (tuple, list)) else (value,)):
+            names = value if isinstance(value, (tuple, list)) else (value,)
+            if any(isinstance(name, str) and name in done for name in names):
                 return False
     return len(done) == 2 * len(order)
 
