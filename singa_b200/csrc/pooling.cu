@@ -689,10 +689,11 @@ inline bool is_k3s2p1(const PoolShape& p) {
 // The first maximum of three adjacent cells of a row is worked out once and
 // serves the three windows it belongs to (5 comparisons per window instead of
 // 9: two for a row's winner, two between the rows, one against the lowest value).
-// Was 231 us forward and 276 us backward at 32x64x112x112, where the bytes take 31 and 47 us, and 56.5 and 104.2 when all comparisons looked for NaNs and began at
-// the lowest value; now 47.7 and 90.2.  The backward pass of rows off a vector's
-// boundary has registers for three CTAs an SM only (64x512x14x14 38.0 us with four and
-// spilled ones, 30.1 with three; 64x64x35x35 33.2 and 27.4).
+// Was 231 us forward and 276 us backward at 32x64x112x112, where the bytes take 31 and 47 us,
+// and 56.5 and 104.2 when all comparisons looked for NaNs and began at the lowest value; now
+// 47.7 and 90.2.  The backward pass of rows off a vector's boundary has registers for three
+// CTAs an SM only (64x512x14x14 38.0 us with four and spilled ones, 30.1 with three;
+// 64x64x35x35 33.2 and 27.4).
 struct RowBest {
   float v[4];
   int at[4];               // column offset 0..2 of the winner
